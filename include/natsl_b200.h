@@ -222,6 +222,33 @@ int natsl_attn_fwd_fp32(int dtype, const void* q, const void* k, const void* v, 
                         float* lse, int B, int T, int HQ, int HKV, int HN, int DK, int DV, int nbs, float scale,
                         int flags, void* stream);
 
+/* One decoding token of a whole layer (projections, short convolutions, linear-branch step, softmax attention over the
+ * cached keys, mixing, output projection) in four launches; state is updated in place.  All tensors bf16 and contiguous
+ * unless noted.  B <= 64, hidden and H*V multiples of 32, K a multiple of 32 up to 256, V a multiple of 32, softmax head
+ * dims H*K/HQ and H*V/HQ 64 or 128 each, convolution width 4.
+ *   x, out [B,hidden];  w_q, w_k [H*K,hidden], w_v, w_g [H*V,hidden], w_a, w_b [H,hidden] (w_b: delta rule only),
+ *   w_o [hidden,H*V], w_mix [2*HQ,H*K] or NULL;  cw_* [channels,4] convolution weights, cb_* biases or NULL;
+ *   qn_w, kn_w [H*K/HQ] query / key norm weights of the softmax branch or NULL; A_log, dt_bias [H]; w1, w2 [H*V/HQ] or
+ *   NULL (each fp32 or bf16: the *_f32 fields);  conv_* [B,channels,4] = the last four inputs of each convolution;
+ *   state, start [B,H,K,V] fp32 = current state, state at the start of the current block; g_block [B,H] fp32 = log decay
+ *   of the current block so far; pool_sum [B,hidden] fp32 += x, or NULL; k_cache, v_cache [B,cap,HQ,.]: rows [0,pos) hold
+ *   the keys and values so far, row pos is written; types [B,n_done,HN,2] = 0/1 types of the n_done = pos / nbs finished
+ *   blocks; types_new [B,1,HN,2] = type of the block this token completes (NULL when it completes none).
+ * workspace: natsl_decode_workspace_bytes(args) bytes (depends on the shapes only; stays valid as pos grows).
+ * Replaces: one token of src/nats/layers/natsl_attn_gdn.py:389-666 / natsl_attn_mamba2.py:330-599 with a cache. */
+typedef struct natsl_decode_args {
+    int32_t B, hidden, H, K, V, HQ, HN, nbs, pos, cap, n_done, rule;
+    int32_t attn_conv, silu, own_chunk, decay, neg_eigval, mix_sigmoid;
+    int32_t qn_f32, kn_f32, alog_f32, dt_f32, w12_f32, types_f32;
+    float norm_eps, l2_eps, mix_eps, scale_attn, scale_lin, reserved;
+    const void *x, *w_q, *w_k, *w_v, *w_a, *w_b, *w_g, *w_o, *w_mix;
+    const void *cw_q, *cw_k, *cw_v, *cb_q, *cb_k, *cb_v, *qn_w, *kn_w, *A_log, *dt_bias, *w1, *w2, *types, *types_new;
+    void *conv_q, *conv_k, *conv_v, *state, *start, *g_block, *pool_sum, *k_cache, *v_cache, *out, *workspace;
+    int64_t workspace_bytes;
+} natsl_decode_args;
+int64_t natsl_decode_workspace_bytes(const natsl_decode_args* args);
+int natsl_decode_step(const natsl_decode_args* args, void* stream);
+
 /* Sequence-parallel helpers (no reference counterpart; the recurrence they split is
  * src/nats/ops/mamba/chunk_h.py:139-218).
  * natsl_sp_segment_decay: a [B,H] = exp(total log decay the carried state sees over this segment);

@@ -47,6 +47,8 @@ PROTOTYPES = {
     "natsl_linear_recurrent_fwd": [_i, _i, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _f, _i, _i, _p],
     "natsl_linear_recurrent_step": [_i, _i, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _f,
                                     _i, _i, _p],
+    "natsl_decode_workspace_bytes": [_p],
+    "natsl_decode_step": [_p, _p],
     "natsl_attn_fwd_fp32": [_i, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _i, _f, _i, _p],
     "natsl_norm_gate_mix": [_p, _p, _p, _p, _i, _p, _p, _i, _p, C.c_long, _i, _f, _i, _p],
     "natsl_attn_bwd": [_p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _i, _f, _i, _p],
@@ -70,6 +72,19 @@ PROTOTYPES = {
 }
 NOALLOC_SCRATCH_BYTES = 32 << 20
 
+
+class DecodeArgs(C.Structure):
+    """``natsl_decode_args`` of the public header, field for field."""
+    _fields_ = ([(n, C.c_int32) for n in (
+        "B hidden H K V HQ HN nbs pos cap n_done rule attn_conv silu own_chunk decay neg_eigval mix_sigmoid "
+        "qn_f32 kn_f32 alog_f32 dt_f32 w12_f32 types_f32").split()]
+        + [(n, C.c_float) for n in "norm_eps l2_eps mix_eps scale_attn scale_lin reserved".split()]
+        + [(n, C.c_void_p) for n in (
+            "x w_q w_k w_v w_a w_b w_g w_o w_mix cw_q cw_k cw_v cb_q cb_k cb_v qn_w kn_w A_log dt_bias w1 w2 types types_new "
+            "conv_q conv_k conv_v state start g_block pool_sum k_cache v_cache out workspace").split()]
+        + [("workspace_bytes", C.c_int64)])
+
+
 _lib = None
 
 
@@ -90,14 +105,15 @@ def load() -> C.CDLL:
     lib.natsl_last_error.argtypes = []
     for name, args in PROTOTYPES.items():
         fn = getattr(lib, name)
-        fn.restype = C.c_int
+        fn.restype = C.c_int64 if name == "natsl_decode_workspace_bytes" else C.c_int
         fn.argtypes = args
     _lib = lib
     return lib
 
 
 # kernels one successful call of an entry point launches (for launch accounting; entry points not listed launch one)
-KERNELS_PER_CALL = {"natsl_build_tables": 2, "natsl_attn_bwd": 2, "natsl_gdn_fwd_noalloc": 3, "natsl_abi_version": 0,
+KERNELS_PER_CALL = {"natsl_build_tables": 2, "natsl_attn_bwd": 2, "natsl_gdn_fwd_noalloc": 3, "natsl_decode_step": 4,
+                    "natsl_abi_version": 0,
                     "natsl_device_status": 0}
 _launches = 0
 

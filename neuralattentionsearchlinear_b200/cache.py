@@ -8,8 +8,12 @@ arrived).  This is a compact restatement of the same bookkeeping for batches wit
 * keys / values of every token are kept together with the 0/1 types of the finished blocks; visibility of a key for a
   query is evaluated from the types (``generate_msk``), the same object the reference's ``generate_msk`` (:209-287) builds.
   (The reference additionally drops the keys of unselected blocks to save memory; outputs do not depend on that.)
+  The rows live in buffers that grow by a quarter at a time, so that a decoding token writes its own row only.
 * ``state`` / ``state_block_start`` / ``g_block``: the current recurrent state, the state the current block started from
   and the log decay accumulated in the current block (re-roll at the block end needs all three).
+
+Single-token steps update these tensors in place.  ``copy.copy`` of a layer cache gives an independent continuation (one
+prompt, several completions): the small tensors are cloned, the key/value rows are shared until either side appends.
 """
 from __future__ import annotations
 
@@ -22,14 +26,46 @@ class NAtSLayerCache:
     def __init__(self, nats_block_size: int = 64):
         self.nats_block_size = nats_block_size
         self.n_tokens = 0                               # tokens seen so far
-        self.k_attn: Optional[torch.Tensor] = None      # [B, n_tokens, HKV, DK]
-        self.v_attn: Optional[torch.Tensor] = None      # [B, n_tokens, HKV, DV]
+        self._k_buf: Optional[torch.Tensor] = None      # [B, capacity, HKV, DK]
+        self._v_buf: Optional[torch.Tensor] = None      # [B, capacity, HKV, DV]
+        self._n_kv = 0                                  # rows of the buffers in use
+        self._kv_shared = False                         # another cache reads the same buffers
+        self._workspace: Optional[torch.Tensor] = None  # intermediates of a single-token step
         self.block_types: Optional[torch.Tensor] = None  # [B, finished blocks, HN, 2] sampled types
         self.state: Optional[torch.Tensor] = None        # [B, H, K, V] fp32: current state
         self.state_block_start: Optional[torch.Tensor] = None
         self.g_block: Optional[torch.Tensor] = None      # [B, H] fp32: log decay of the current block so far
         self.pool_sum: Optional[torch.Tensor] = None     # [B, D] fp32: sum of the layer input over the current block
         self.conv_state = None                           # (q, k, v) tails of the short convolutions
+
+    def __copy__(self):
+        new = type(self).__new__(type(self))
+        new.__dict__.update(self.__dict__)
+        for name in ("state", "state_block_start", "g_block", "pool_sum"):
+            t = getattr(self, name)
+            setattr(new, name, None if t is None else t.clone())
+        new.conv_state = None if self.conv_state is None else tuple(None if t is None else t.clone() for t in self.conv_state)
+        new._workspace = None
+        self._kv_shared = new._kv_shared = True
+        return new
+
+    @property
+    def k_attn(self) -> Optional[torch.Tensor]:
+        """Keys of every token so far [B, n_tokens, HKV, DK]."""
+        return None if self._k_buf is None else self._k_buf[:, :self._n_kv]
+
+    @k_attn.setter
+    def k_attn(self, k: Optional[torch.Tensor]) -> None:
+        self._k_buf, self._n_kv = k, 0 if k is None else k.shape[1]
+
+    @property
+    def v_attn(self) -> Optional[torch.Tensor]:
+        """Values of every token so far [B, n_tokens, HKV, DV]."""
+        return None if self._v_buf is None else self._v_buf[:, :self._n_kv]
+
+    @v_attn.setter
+    def v_attn(self, v: Optional[torch.Tensor]) -> None:
+        self._v_buf, self._n_kv = v, 0 if v is None else v.shape[1]
 
     @property
     def n_tokens_in_nats_block(self) -> int:
@@ -39,9 +75,30 @@ class NAtSLayerCache:
     def n_finished_blocks(self) -> int:
         return self.n_tokens // self.nats_block_size
 
+    def reserve_kv(self, n: int) -> None:
+        """Makes room for ``n`` more key/value rows that nobody else reads."""
+        cap = self._k_buf.shape[1]
+        if (self._n_kv + n <= cap and cap == self._v_buf.shape[1] and not self._kv_shared and self._k_buf.is_contiguous()
+                and self._v_buf.is_contiguous()):
+            return
+        need = self._n_kv + n
+        cap = -(-(need + max(256, need // 4)) // 64) * 64
+        for name in ("_k_buf", "_v_buf"):
+            old = getattr(self, name)
+            buf = old.new_empty((old.shape[0], cap) + tuple(old.shape[2:]))
+            buf[:, :self._n_kv].copy_(old[:, :self._n_kv])
+            setattr(self, name, buf)
+        self._kv_shared = False
+
     def append_kv(self, k: torch.Tensor, v: torch.Tensor) -> None:
-        self.k_attn = k if self.k_attn is None else torch.cat([self.k_attn, k], 1)
-        self.v_attn = v if self.v_attn is None else torch.cat([self.v_attn, v], 1)
+        if self._k_buf is None:
+            self._k_buf, self._v_buf, self._n_kv = k, v, k.shape[1]
+            return
+        n = k.shape[1]
+        self.reserve_kv(n)
+        self._k_buf[:, self._n_kv:self._n_kv + n].copy_(k)
+        self._v_buf[:, self._n_kv:self._n_kv + n].copy_(v)
+        self._n_kv += n
 
     def append_types(self, types: torch.Tensor) -> None:
         self.block_types = types if self.block_types is None else torch.cat([self.block_types, types], 1)

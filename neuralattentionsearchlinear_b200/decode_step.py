@@ -1,0 +1,212 @@
+"""Single-token decoding of a whole layer through ``natsl_decode_step`` (four launches, state updated in place) for the
+configurations the kernel is built for; everything else takes the general path of ``decoding.forward_cached``
+(src/nats/layers/natsl_attn_gdn.py:389-666, src/nats/layers/natsl_attn_mamba2.py:330-599 with one new token)."""
+from __future__ import annotations
+
+import ctypes
+import threading
+import weakref
+
+import torch
+import torch.nn as nn
+
+from . import _lib
+from .modules import FusedMultiInputRMSNormGated, L2Norm, RMSNorm, ShortConvolution
+from .nats_util import current_stream_ptr
+
+BF16 = torch.bfloat16
+MAX_BATCH = 64
+_tls = threading.local()                     # one argument block per thread: a call in flight is never rewritten
+
+
+class _Plan:
+    """Argument block of one layer: shapes, options and weight pointers, valid while ``current()`` holds."""
+
+    def __init__(self, layer):
+        self.ok = False
+        mods = {n: type_ for n, type_ in (
+            ("q_proj", nn.Linear), ("k_proj", nn.Linear), ("v_proj", nn.Linear), ("a_proj", nn.Linear),
+            ("g_proj", nn.Linear), ("o_proj", nn.Linear), ("q_conv1d", ShortConvolution), ("k_conv1d", ShortConvolution),
+            ("v_conv1d", ShortConvolution), ("o_norm", FusedMultiInputRMSNormGated))}
+        gdn = hasattr(layer, "b_proj")
+        weighted = layer.outputs_are_weighted if gdn else layer.outputs_are_wighted
+        if gdn:
+            mods["b_proj"] = nn.Linear
+        else:
+            mods["q_norm2"] = mods["k_norm2"] = L2Norm
+        if weighted:
+            mods["nats_out_weights_layer"] = nn.Linear
+        if layer.attn_qk_norm:
+            mods["q_norm"] = mods["k_norm"] = RMSNorm
+        self.mods = []
+        for n, type_ in mods.items():
+            m = layer._modules.get(n)
+            self.mods.append((layer._modules, n, m))
+            if type(m) is not type_:
+                return
+        self.hooks = [h for _, _, m in self.mods for h in (m._forward_hooks, m._forward_pre_hooks)]
+        a = self.args = _lib.DecodeArgs()
+        self.params = []
+
+        def weight(field, owner, name="weight", any_float=None):
+            p = owner._parameters.get(name)
+            self.params.append((owner._parameters, name, p, 0 if p is None else p.data_ptr()))
+            if p is None:
+                return True
+            if any_float is not None and p.dtype == torch.float32:
+                setattr(a, any_float, 1)
+            elif p.dtype != BF16:
+                return False
+            setattr(a, field, p.data_ptr())
+            return p.is_cuda and p.is_contiguous() and p.device == layer.q_proj.weight.device
+
+        m = layer
+        good = all([weight("w_q", m.q_proj), weight("w_k", m.k_proj), weight("w_v", m.v_proj), weight("w_a", m.a_proj),
+                    weight("w_g", m.g_proj), weight("w_o", m.o_proj), weight("cw_q", m.q_conv1d), weight("cw_k", m.k_conv1d),
+                    weight("cw_v", m.v_conv1d), weight("cb_q", m.q_conv1d, "bias"), weight("cb_k", m.k_conv1d, "bias"),
+                    weight("cb_v", m.v_conv1d, "bias"), weight("A_log", m, "A_log", "alog_f32"),
+                    weight("dt_bias", m, "dt_bias", "dt_f32"), weight("w1", m.o_norm, "weight1", "w12_f32"),
+                    weight("w2", m.o_norm, "weight2", "w12_f32")])
+        if gdn:
+            good = good and weight("w_b", m.b_proj)
+        if weighted:
+            good = good and weight("w_mix", m.nats_out_weights_layer)
+        if m.attn_qk_norm:
+            good = good and weight("qn_w", m.q_norm, "weight", "qn_f32") and weight("kn_w", m.k_norm, "weight", "kn_f32")
+            good = good and m.q_norm.eps == m.k_norm.eps
+            a.norm_eps = m.q_norm.eps
+        if not gdn:
+            good = good and m.q_norm2.eps == m.k_norm2.eps
+            a.l2_eps = m.q_norm2.eps
+        w1, w2 = m.o_norm.weight1, m.o_norm.weight2
+        DK, DV = m.head_attn_k_dim, m.head_attn_v_dim
+        self.ok = bool(
+            good and all(mod.bias is None for mod in (m.q_proj, m.k_proj, m.v_proj, m.a_proj, m.g_proj, m.o_proj))
+            and (w1 is None) == (w2 is None) and (w1 is None or w1.dtype == w2.dtype)
+            and m.num_v_heads == m.num_heads and m.n_ops == 2 and m.o_norm.hidden_size == DV
+            and all(c.kernel_size == (4,) and c.activation == m.q_conv1d.activation for c in (m.q_conv1d, m.k_conv1d, m.v_conv1d))
+            and m.hidden_size % 32 == 0 and m.value_dim % 32 == 0 and m.head_k_dim % 32 == 0 and m.head_k_dim <= 256
+            and m.head_v_dim % 32 == 0 and DK in (64, 128) and DV in (64, 128) and m.key_dim <= 10240
+            and m.num_heads % m.num_nats_head == 0 and m.num_attn_heads % m.num_nats_head == 0)
+        a.hidden, a.H, a.K, a.V, a.HQ, a.HN = (m.hidden_size, m.num_heads, m.head_k_dim, m.head_v_dim, m.num_attn_heads,
+                                               m.num_nats_head)
+        a.nbs, a.rule = m.nats_block_size, _lib.RULE_GDN if gdn else _lib.RULE_MAMBA
+        a.silu = int(m.q_conv1d.activation in ("silu", "swish"))
+        a.mix_sigmoid, a.mix_eps = int(m.o_norm.activation == "sigmoid"), m.o_norm.eps
+        a.scale_attn, a.scale_lin = DK ** -0.5, m.head_k_dim ** -0.5 if gdn else 1.0
+        self.options = ()
+        self.ws_bytes = {}
+
+    def current(self) -> bool:
+        for d, n, m in self.mods:
+            if d.get(n) is not m:
+                return False
+        if not self.ok:
+            return True                      # nothing else to check: the general path runs
+        for h in self.hooks:
+            if h:
+                return False
+        for d, n, p, ptr in self.params:
+            if d.get(n) is not p or (p is not None and p.data_ptr() != ptr):
+                return False
+        return True
+
+
+def _plan(layer):
+    plans = getattr(_tls, "plans", None)
+    if plans is None:
+        plans = _tls.plans = weakref.WeakKeyDictionary()
+    p = plans.get(layer)
+    if p is None or not p.current():
+        p = plans[layer] = _Plan(layer)
+        if p.ok and any(p.hooks):
+            p.ok = False
+            p.mods = [(layer._modules, "q_proj", None)]      # looked at again with the next token
+    return p
+
+
+@torch.no_grad()
+def decode_token(layer, x: torch.Tensor, container):
+    """The layer's output [B, 1, hidden] for one new token, or None where the general path has to run (which also raises
+    what there is to raise).  Updates the layer's cache."""
+    if (x.dim() != 3 or x.shape[1] != 1 or x.dtype != BF16 or not x.is_cuda or x.shape[0] > MAX_BATCH or layer.layer_idx is None
+            or layer.ops_for_incomplete_chunks == 'attn' or not layer.incomplete_block_start_with_ht
+            or not (layer.use_short_conv and layer.use_gate) or torch.is_autocast_enabled() or not hasattr(container, "layer")):
+        return None
+    plan = _plan(layer)
+    if not plan.ok or torch.nn.modules.module._has_any_global_hook():
+        return None
+    a = plan.args
+    B, _, D = x.shape
+    dev = x.device
+    if D != a.hidden or dev != layer.q_proj.weight.device:
+        return None
+    nbs = layer.nats_block_size
+    cache = container.layer(layer.layer_idx, nbs)
+    pos = cache.n_tokens
+    if pos == 0:                                             # a prompt of one token: start from empty states
+        f32 = dict(dtype=torch.float32, device=dev)
+        cache.state = torch.zeros(B, a.H, a.K, a.V, **f32)
+        cache.state_block_start = torch.zeros(B, a.H, a.K, a.V, **f32)
+        cache.g_block, cache.pool_sum = torch.zeros(B, a.H, **f32), torch.zeros(B, D, **f32)
+        cache.conv_state = tuple(torch.zeros(B, n, 4, dtype=BF16, device=dev)
+                                 for n in (layer.key_dim, layer.key_dim, layer.value_dim))
+        cache._k_buf = torch.empty(B, 256, a.HQ, layer.head_attn_k_dim, dtype=BF16, device=dev)
+        cache._v_buf = torch.empty(B, 256, a.HQ, layer.head_attn_v_dim, dtype=BF16, device=dev)
+        cache._n_kv, cache._kv_shared = 0, False
+    elif cache._k_buf is None or cache._n_kv != pos or cache.state.shape[0] != B or cache.conv_state is None:
+        return None
+    cq, ck, cv = cache.conv_state
+    n_done, types = pos // nbs, cache.block_types
+    if n_done and (types is None or types.shape[1] != n_done or types.dtype not in (BF16, torch.float32)):
+        return None
+    for t in (cq, ck, cv, cache._k_buf, cache._v_buf):
+        if t is None or t.dtype != BF16 or t.device != dev:
+            return None
+    completes = (pos + 1) % nbs == 0
+    types_new = None
+    x = x.contiguous()
+    if completes:                                            # a block's type is decided once its last token is known
+        pooled = ((cache.pool_sum + x[:, 0].float()) / nbs).to(x.dtype)[:, None, :]
+        types_new = layer.select(pooled).contiguous()
+        if types_new.dtype not in (BF16, torch.float32) or (types is not None and types.dtype != types_new.dtype):
+            return None
+    cache.reserve_kv(1)
+    for name in ("state", "state_block_start", "g_block", "pool_sum"):
+        t = getattr(cache, name)
+        if t.dtype != torch.float32 or not t.is_contiguous():
+            setattr(cache, name, t.float().contiguous())
+    if not (cq.is_contiguous() and ck.is_contiguous() and cv.is_contiguous()):
+        cache.conv_state = cq, ck, cv = cq.contiguous(), ck.contiguous(), cv.contiguous()
+    if n_done and not types.is_contiguous():
+        types = cache.block_types = types.contiguous()
+    ws = cache._workspace
+    need = plan.ws_bytes.get(B)
+    a.B = B
+    if need is None:
+        need = plan.ws_bytes[B] = _lib.load().natsl_decode_workspace_bytes(ctypes.byref(a))
+        if need < 0:
+            raise _lib.NatslError(_lib.load().natsl_last_error().decode())
+    if ws is None or ws.numel() < need or ws.device != dev:
+        ws = cache._workspace = torch.empty(need, dtype=torch.uint8, device=dev)
+    out = torch.empty_like(x)
+    a.own_chunk = int(layer.ops_for_incomplete_chunks == 'all')
+    gdn = a.rule == _lib.RULE_GDN
+    a.decay = int(layer.decay_for_non_gdn_blocks if gdn else layer.decay_for_non_mamba_blocks)
+    a.neg_eigval = int(gdn and layer.allow_neg_eigval)
+    a.attn_conv = int(layer.attn_with_short_conv)
+    a.pos, a.cap, a.n_done = pos, cache._k_buf.shape[1], n_done
+    a.types_f32 = int((types_new if types is None else types).dtype == torch.float32) if (n_done or completes) else 0
+    a.x, a.out = x.data_ptr(), out.data_ptr()
+    a.types, a.types_new = (types.data_ptr() if n_done else None), (types_new.data_ptr() if completes else None)
+    a.conv_q, a.conv_k, a.conv_v = cq.data_ptr(), ck.data_ptr(), cv.data_ptr()
+    a.state, a.start, a.g_block = cache.state.data_ptr(), cache.state_block_start.data_ptr(), cache.g_block.data_ptr()
+    a.pool_sum = None if completes else cache.pool_sum.data_ptr()
+    a.k_cache, a.v_cache = cache._k_buf.data_ptr(), cache._v_buf.data_ptr()
+    a.workspace, a.workspace_bytes = ws.data_ptr(), need
+    _lib.call("natsl_decode_step", ctypes.byref(a), current_stream_ptr(dev))
+    cache._n_kv = cache.n_tokens = pos + 1
+    if completes:
+        cache.append_types(types_new)
+        cache.pool_sum = torch.zeros_like(cache.pool_sum)
+    return out

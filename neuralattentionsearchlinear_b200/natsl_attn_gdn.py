@@ -17,6 +17,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from .mixed_attn_gdn import nats_mixed_attn_gdn, nats_mixed_attn_gdn_chunk_inference, nats_mixed_attn_gdn_recurrent
+from .decode_step import decode_token
 from .decoding import forward_cached
 from .modules import FusedMultiInputRMSNormGated, RMSNorm, ShortConvolution, hard_softmax, mean_pooling
 
@@ -299,6 +300,10 @@ class NeuralAttentionSearchLinearAttnGDN(nn.Module):
     def _forward_cached(self, hidden_states: torch.Tensor, past_key_values):
         """Prefill into an empty cache (64 tokens or more, chunk kernels) or a decoding step of fewer than 64 tokens
         (token recurrence with re-roll + masked attention over the cached keys), natsl_attn_gdn.py:389-410, 576-650."""
+        if hidden_states.shape[1] == 1 and type(self) is NeuralAttentionSearchLinearAttnGDN:
+            y = decode_token(self, hidden_states, past_key_values)
+            if y is not None:
+                return y, None, past_key_values
         o_gd, o_attn, o_w = forward_cached(self, hidden_states, past_key_values)
         with torch.no_grad():
             return self.mix(hidden_states, o_gd, o_attn, o_w), None, past_key_values

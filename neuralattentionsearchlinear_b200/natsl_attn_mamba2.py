@@ -15,6 +15,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from .decode_step import decode_token
 from .decoding import forward_cached
 from .mixed_attn_mamba import (nats_mixed_attn_mamba, nats_mixed_attn_mamba_chunk_inference,
                                nats_mixed_attn_mamba_recurrent)
@@ -236,6 +237,10 @@ class NeuralAttentionSearchLinearAttnMamba(nn.Module):
             raise NotImplementedError("variable-length batches are not built")
         B, T, _ = hidden_states.shape
         if cache_params is not None:                        # prefill into / decode from a NAtSCache
+            if T == 1 and type(self) is NeuralAttentionSearchLinearAttnMamba:
+                y = decode_token(self, hidden_states, cache_params)
+                if y is not None:
+                    return y
             o_m, o_attn, o_w = forward_cached(self, hidden_states, cache_params)
             with torch.no_grad():
                 return self.mix(hidden_states, o_m, o_attn, o_w)
