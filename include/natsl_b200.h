@@ -174,6 +174,24 @@ int natsl_gdn_walk_fused(const void* q, const void* k, const void* w, const void
                          const int32_t* indices, const int32_t* n_blocks, const float* h0, void* o, float* ht, int B,
                          int T, int H, int HN, int K, int V, int nbs, float scale, int flags, void* stream);
 
+/* natsl_gdn_walk_fused that also writes hstart [B,H,K,V] fp32 (or NULL) = the state a decoder rolls back to: the state in
+ * front of the last block with its carried decay, or, when the last block is complete (T % nbs == 0), the state behind it
+ * where last_types [B,HN,2] (last_dtype fp32 or bf16: that block's own types) says linear, else the state in front of it
+ * decayed over it (NATSL_FLAG_DECAY_SKIPPED) or as it is.
+ * Replaces in addition: src/nats/ops/gated_delta_rule/chunk_fwd.py:178-206. */
+int natsl_gdn_walk_fused_ex(const void* q, const void* k, const void* w, const void* u, const void* pmat,
+                            const float* gcs, const float* k_rstd, const float* q_rstd, const int32_t* types_i,
+                            const int32_t* indices, const int32_t* n_blocks, const float* h0, void* o, float* ht,
+                            float* hstart, const void* last_types, int last_dtype, int B, int T, int H, int HN, int K, int V,
+                            int nbs, float scale, int flags, void* stream);
+
+/* The same recurrence + output walk on mma.sync for K in {64, 128, 192}, V a multiple of 32 (64 and up) and any
+ * nats_block_size; same arguments.  It cuts the value dim into slices of 32 or 64 columns per CTA. */
+int natsl_gdn_walk(const void* q, const void* k, const void* w, const void* u, const void* pmat, const float* gcs,
+                   const float* k_rstd, const float* q_rstd, const int32_t* types_i, const int32_t* indices,
+                   const int32_t* n_blocks, const float* h0, void* o, float* ht, float* hstart, const void* last_types,
+                   int last_dtype, int B, int T, int H, int HN, int K, int V, int nbs, float scale, int flags, void* stream);
+
 /* The same walk with the value dimension split over two CTAs per (batch, head): 256 tensor-memory columns and about
  * 107 KB of shared memory per CTA, so that two of them, or one of them and one attention CTA, share an SM (the two
  * branches of the layer then overlap).  Same arguments and results; T <= 8192. */
@@ -194,6 +212,12 @@ int natsl_gdn_walk_fused_vsplit(const void* q, const void* k, const void* w, con
 int natsl_mamba_walk_fused(const void* q, const void* k, const void* v, const float* gcs, const int32_t* types_i,
                            const int32_t* indices, const int32_t* n_blocks, const float* h0, void* o, float* ht, int B,
                            int T, int H, int HN, int K, int V, int nbs, float scale, int flags, void* stream);
+
+/* natsl_mamba_walk_fused that also writes hstart (see natsl_gdn_walk_fused_ex). */
+int natsl_mamba_walk_fused_ex(const void* q, const void* k, const void* v, const float* gcs, const int32_t* types_i,
+                              const int32_t* indices, const int32_t* n_blocks, const float* h0, void* o, float* ht,
+                              float* hstart, const void* last_types, int last_dtype, int B, int T, int H, int HN, int K, int V,
+                              int nbs, float scale, int flags, void* stream);
 
 /* Reference-precision (fp32 math, CUDA cores) path for fp32 or bf16 tensors (dtype = NATSL_DT_F32 / _BF16 for
  * q, k, v, beta, o): token-by-token linear recurrence with re-roll to the block-start state, and plain masked

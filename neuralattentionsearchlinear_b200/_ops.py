@@ -10,7 +10,10 @@ from .nats_util import SelectionTables, cdiv, current_stream_ptr
 
 BF16 = torch.bfloat16
 USE_MAMBA_WALK = os.environ.get("NATSL_MAMBA_WALK", "1") != "0"    # natsl_mamba_walk_fused (K = 128, V = 64)
-USE_FUSED_WALK = True        # K = V = 128, block 64: recurrence + output fused on tcgen05 (natsl_gdn_walk_fused)
+# recurrence + output in one walk: on tcgen05 (natsl_gdn_walk_fused, K = V = 128, block 64) or mma.sync (natsl_gdn_walk)
+USE_FUSED_WALK = True
+# (K, V) with a chunk preparation; all of them have a walk for every block size
+GDN_HEAD_DIMS = {(64, 64), (64, 128), (128, 64), (128, 128), (128, 256), (192, 384)}
 # value dimension of the fused walk split over two CTAs (natsl_gdn_walk_fused_vsplit, T <= 8192): half an SM per CTA.
 # Off by default: measured alone it is no faster than the one-CTA walk (0.204 vs 0.189 ms at B=8, T=4096, H=16), and
 # the kernels of the two branches do not overlap in practice (the block scheduler drains one grid before the next).
@@ -23,6 +26,12 @@ PREP_TC = os.environ.get("NATSL_PREP_TC", "1") != "0"
 # Off by default: parity-green but measured slower (0.43 vs 0.29 ms at B=8, T=4096, H=16).
 ATTN_PERSISTENT = os.environ.get("NATSL_ATTN_PERSISTENT", "0") == "1"
 
+# (batch, head) pairs up to which the delta rule takes the mma.sync walk also where the tcgen05 one is built (K = V = 128,
+# block 64): its slices of the value dim fill four SMs per pair, and a chunk takes 1.6 instead of 2.8 us.  Measured at
+# T = 2048: 32 pairs 51 against 90 us, 48 and 64 pairs 78 against 91 us, 128 pairs (T = 4096) 283 against 174 us.  The line
+# is drawn at 31 so that from 32 pairs on a sequence's result does not depend, bit for bit, on the batch around it.
+WALK_MMA_MAX_HEADS = 31
+
 
 def _attn_flags(own_chunk: bool) -> int:
     return (_lib.FLAG_ATTN_OWN_CHUNK if own_chunk else 0) | (_lib.FLAG_ATTN_PERSISTENT if ATTN_PERSISTENT else 0)
@@ -31,6 +40,13 @@ def _attn_flags(own_chunk: bool) -> int:
 def prep_entry(K: int, V: int) -> str:
     """Name of the chunk-preparation entry point for these head dims (both take the arguments of ``..._prep_ex``)."""
     return "natsl_gdn_chunk_prep_tc" if (PREP_TC and K == 128 and V == 128) else "natsl_gdn_chunk_prep_ex"
+
+
+def walks_with_state(rule: int, K: int, V: int, T: int) -> bool:
+    """Whether ``linear_fwd`` can hand over the block-start state of these head dims without chunk intermediates."""
+    if rule == _lib.RULE_GDN:
+        return USE_FUSED_WALK and (K, V) in GDN_HEAD_DIMS and T <= 65536
+    return USE_MAMBA_WALK and K == 128 and V == 64 and T <= 65536
 
 
 def _need(cond: bool, msg: str, exc=ValueError):
@@ -119,12 +135,14 @@ def attn_dense_mask(tables: SelectionTables, HQ: int, own_chunk: bool) -> torch.
 
 def linear_fwd(rule: int, q, k, v, g, beta, tables: SelectionTables, scale: float, h0, decay: bool,
                use_l2norm: bool, output_final_state: bool, trailing_quirk: bool = True,
-               return_intermediates: bool = False, skip_out: bool = False, own_chunk: bool = True, tables_event=None):
+               return_intermediates: bool = False, skip_out: bool = False, own_chunk: bool = True, tables_event=None,
+               want_start: bool = False, last_types=None):
     """Linear branch forward (prep -> state recurrence -> output).  Returns (o, ht, inter); with ``skip_out``
     only the recurrence runs (o is None).  ``own_chunk=False``: the output keeps only the state term (the mode
     in which the softmax branch alone covers the current chunk); ``tables`` must then be per 64-token chunk.
     ``tables_event``: CUDA event after which the tables (built on another stream) are valid; the chunk preparation
-    does not read them and is launched before the wait."""
+    does not read them and is launched before the wait.  ``want_start`` (head dims of ``walks_with_state``): inter is
+    dict(start=...), the state a decoder rolls back to, with ``last_types`` [B,HN,2] the own types of a complete last block."""
     _need(q.dtype == BF16 and k.dtype == BF16 and v.dtype == BF16, "linear branch needs bf16 q/k/v", TypeError)
     _check_qkv(q, k, v, tables, "linear branch", same_heads=True)
     q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
@@ -140,10 +158,10 @@ def linear_fwd(rule: int, q, k, v, g, beta, tables: SelectionTables, scale: floa
     _need(H % HN == 0, f"{H} heads over {HN} selection heads")
     NT = cdiv(T, 64)
     nbs = tables.nats_block_size
-    if K not in (64, 128) or V not in (64, 128, 256):
-        # head dims the chunk kernels have no tiles for (the 760M configuration: K = 192, V = 384): the token recurrence
-        # with re-roll computes the same function for any K in {32, 64, 96, 128, 192, 256} and V a multiple of 8 --
-        # correct, not fast, forward only
+    walk = (rule == _lib.RULE_GDN and walks_with_state(rule, K, V, T) and not return_intermediates and not skip_out and own_chunk)
+    if not walk and (K not in (64, 128) or V not in (64, 128, 256)):
+        # head dims the chunk kernels have no tiles for: the token recurrence with re-roll computes the same function for
+        # any K in {32, 64, 96, 128, 192, 256} and V a multiple of 8 -- correct, not fast, forward only
         if return_intermediates or skip_out or not own_chunk:
             raise NotImplementedError(f"head dims K={K}, V={V} run the token recurrence, which has no chunk intermediates "
                                       "(backward pass, state-only and mode 'attn' need K in {64,128}, V in {64,128,256})")
@@ -154,8 +172,8 @@ def linear_fwd(rule: int, q, k, v, g, beta, tables: SelectionTables, scale: floa
     st = current_stream_ptr(dev)
     g = g.float().contiguous()
     gcs = torch.empty(B, T, H, dtype=torch.float32, device=dev)
-    fused = (rule == _lib.RULE_GDN and K == 128 and V == 128 and nbs == 64 and NT <= 1024 and not return_intermediates
-             and not skip_out and own_chunk and USE_FUSED_WALK)
+    fused = walk
+    tc_walk = walk and K == 128 and V == 128 and nbs == 64 and B * H > WALK_MMA_MAX_HEADS
     # Mamba2 with state dim 128 and head dim 64: recurrence + output (or the recurrence alone) in one tcgen05 walk
     mamba_fused = (rule == _lib.RULE_MAMBA and K == 128 and V == 64 and NT <= 1024 and not return_intermediates
                    and own_chunk and USE_MAMBA_WALK and (not skip_out or output_final_state))
@@ -180,21 +198,37 @@ def linear_fwd(rule: int, q, k, v, g, beta, tables: SelectionTables, scale: floa
         h0 = h0.float().contiguous()
         _need(tuple(h0.shape) == (B, H, K, V), f"initial state must be [B,H,K,V], got {tuple(h0.shape)}")
     flags = (_lib.FLAG_DECAY_SKIPPED if decay else 0) | (0 if trailing_quirk else _lib.FLAG_NO_TRAILING_QUIRK)
+    start, last_code = None, _lib.DT_F32
+    if want_start:
+        _need(fused or mamba_fused, "the block-start state needs head dims with a fused walk", NotImplementedError)
+        start = torch.empty(B, H, K, V, dtype=torch.float32, device=dev)
+        if T % nbs == 0:
+            _need(last_types is not None and tuple(last_types.shape) == (B, HN, 2), "a complete last block needs its types [B,HN,2]")
+            last_types = (last_types if last_types.dtype in (BF16, torch.float32) else last_types.float()).contiguous()
+            last_code = _dt_code(last_types)
+        else:
+            last_types = None
+    inter = dict(start=start) if want_start else None
     if fused:
-        # recurrence + output in one tcgen05 walk; the per-chunk states are never materialised
+        # recurrence + output in one walk; the per-chunk states are never materialised
         o = torch.empty(B, T, H, V, dtype=BF16, device=dev)
-        entry = "natsl_gdn_walk_fused_vsplit" if (WALK_VSPLIT and NT <= 128) else "natsl_gdn_walk_fused"
-        _lib.call(entry, q.data_ptr(), k.data_ptr(), w.data_ptr(), u.data_ptr(), pmat.data_ptr(),
-                  gcs.data_ptr(), krstd.data_ptr(), qrstd.data_ptr(), tables.types_i.data_ptr(),
-                  tables.indices.data_ptr(), tables.n_blocks.data_ptr(), _lib.ptr(h0), o.data_ptr(), _lib.ptr(ht),
-                  B, T, H, HN, K, V, nbs, float(scale), flags, st)
-        return o, ht, None
+        args = (q.data_ptr(), k.data_ptr(), w.data_ptr(), u.data_ptr(), pmat.data_ptr(), gcs.data_ptr(), krstd.data_ptr(),
+                qrstd.data_ptr(), tables.types_i.data_ptr(), tables.indices.data_ptr(), tables.n_blocks.data_ptr(),
+                _lib.ptr(h0), o.data_ptr(), _lib.ptr(ht))
+        dims = (B, T, H, HN, K, V, nbs, float(scale), flags, st)
+        if WALK_VSPLIT and tc_walk and NT <= 128 and not want_start:
+            _lib.call("natsl_gdn_walk_fused_vsplit", *args, *dims)
+        else:
+            _lib.call("natsl_gdn_walk_fused_ex" if tc_walk else "natsl_gdn_walk", *args, _lib.ptr(start),
+                      _lib.ptr(last_types if want_start else None), last_code, *dims)
+        return o, ht, inter
     if mamba_fused:
         o = None if skip_out else torch.empty(B, T, H, V, dtype=BF16, device=dev)
-        _lib.call("natsl_mamba_walk_fused", None if skip_out else q.data_ptr(), k.data_ptr(), v.data_ptr(), gcs.data_ptr(),
+        _lib.call("natsl_mamba_walk_fused_ex", None if skip_out else q.data_ptr(), k.data_ptr(), v.data_ptr(), gcs.data_ptr(),
                   tables.types_i.data_ptr(), tables.indices.data_ptr(), tables.n_blocks.data_ptr(), _lib.ptr(h0),
-                  _lib.ptr(o), _lib.ptr(ht), B, T, H, HN, K, V, nbs, float(scale), flags, st)
-        return o, ht, (dict(gcs=gcs) if skip_out else None)
+                  _lib.ptr(o), _lib.ptr(ht), _lib.ptr(start), _lib.ptr(last_types if want_start else None), last_code,
+                  B, T, H, HN, K, V, nbs, float(scale), flags, st)
+        return o, ht, (dict(gcs=gcs) if skip_out else inter)
     state_only = skip_out and ht is not None and not return_intermediates
     h = None if state_only else torch.empty(B, NT, H, K, V, dtype=BF16, device=dev)
     carry = None if state_only else torch.empty(B, NT, H, dtype=torch.float32, device=dev)

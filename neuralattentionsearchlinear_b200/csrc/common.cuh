@@ -48,11 +48,11 @@ __device__ __forceinline__ void cp_async_wait() {
 }
 
 // Byte offset of 16-byte chunk `chunk` of row `row` in a swizzled tile whose rows are
-// ROW_BYTES long (64, 128 or 256).  The XOR keeps the eight rows touched by one
+// ROW_BYTES long (64 or a multiple of 128).  The XOR keeps the eight rows touched by one
 // ldmatrix 8x8 load in eight different 16-byte bank groups.
 template <int ROW_BYTES>
 __device__ __forceinline__ uint32_t swz(int row, int chunk) {
-    static_assert(ROW_BYTES == 64 || ROW_BYTES == 128 || ROW_BYTES == 256 || ROW_BYTES == 512, "row size");
+    static_assert(ROW_BYTES == 64 || ROW_BYTES % 128 == 0, "row size");
     if (ROW_BYTES == 64) return row * 64 + ((chunk ^ ((row >> 1) & 3)) << 4);
     return row * ROW_BYTES + ((chunk ^ (row & 7)) << 4);
 }

@@ -45,8 +45,8 @@ gdn_walk_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                    const __grid_constant__ CUtensorMap map_p, const float* __restrict__ gcs,
                    const float* __restrict__ krstd, const float* __restrict__ qrstd, const int* __restrict__ types_i,
                    const int* __restrict__ indices, const int* __restrict__ n_blocks, const float* __restrict__ h0,
-                   __nv_bfloat16* __restrict__ o, float* __restrict__ ht, int T, int H, int HN, int TN, float scale,
-                   int decay, int trailing_quirk, int* status) {
+                   __nv_bfloat16* __restrict__ o, float* __restrict__ ht, float* hstart, const void* __restrict__ last_types,
+                   int last_f32, int T, int H, int HN, int TN, float scale, int decay, int trailing_quirk, int* status) {
     using L = WkSmem;
     constexpr int K = 128, V = 128;
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -218,8 +218,23 @@ gdn_walk_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         const int tr = row & 63;                          // token row inside the chunk
         bool ok = true;
 
+        // the state in front of the last chunk (with its carried decay), for a decoder that continues the sequence: it is
+        // the one published when no chunk from `c` up to the last one updates the state
+        float* hs_row = hstart ? hstart + (((long)b * H + h) * K + row) * V : nullptr;
+        auto starts_last = [&](int c) -> bool {
+            if (!hs_row) return false;
+            for (int j = c; j < NT - 1; ++j)
+                if (m_sel[j]) return false;
+            return true;
+        };
+        auto store_row = [&](float* dst, int c0, const uint32_t (&r)[32], float f) {
+#pragma unroll
+            for (int i = 0; i < 32; i += 4)
+                *reinterpret_cast<float4*>(dst + c0 + i) = make_float4(__uint_as_float(r[i]) * f, __uint_as_float(r[i + 1]) * f,
+                                                                      __uint_as_float(r[i + 2]) * f, __uint_as_float(r[i + 3]) * f);
+        };
         // copies columns [cb, cb+64) of this lane's S row as bf16 into the shared copy and leaves S * mul in TMEM
-        auto publish_state = [&](float mul, const float* init_row) {
+        auto publish_state = [&](float mul, const float* init_row, bool hs) {
 #pragma unroll 1
             for (int c0 = cb; c0 < cb + 64; c0 += 32) {
                 uint32_t r[32];
@@ -240,6 +255,7 @@ gdn_walk_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     *reinterpret_cast<uint4*>(smem + L::sbf + (col >> 6) * 16384 + swz<128>(row, (col & 63) >> 3)) =
                         make_uint4(w4[0], w4[1], w4[2], w4[3]);
                 }
+                if (hs) store_row(hs_row, c0, r, __expf(m_carry[NT - 1]));
                 if (mul != 1.f || init_row) {
 #pragma unroll
                     for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * mul);
@@ -257,14 +273,16 @@ gdn_walk_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         {   // initial state
             const float* init = h0 ? h0 + (((long)b * H + h) * K + row) * V : nullptr;
             if (init) {
-                publish_state(next_dec(0), init);
+                publish_state(next_dec(0), init, starts_last(0));
             } else {
+                const bool hs = starts_last(0);
 #pragma unroll 1
                 for (int c0 = cb; c0 < cb + 64; c0 += 32) {
                     uint32_t r[32];
 #pragma unroll
                     for (int i = 0; i < 32; ++i) r[i] = 0u;
                     tmem_st32(t_lane + WK_S + c0, r);
+                    if (hs) store_row(hs_row, c0, r, 1.f);
                 }
                 tmem_st_wait();
                 for (int i = 0; i < 8; ++i)
@@ -340,7 +358,7 @@ gdn_walk_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 ok = __all_sync(0xffffffffu, mbar_wait(bar_s3, c & 1, status));
                 if (ok) {
                     tc_fence_after();
-                    publish_state(next_dec(c + 1), nullptr);
+                    publish_state(next_dec(c + 1), nullptr, c < NT - 1 && starts_last(c + 1));
                     fence_async_smem();
                 }
             }
@@ -383,19 +401,32 @@ gdn_walk_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             g_cur = g_nxt;
             r_cur = r_nxt;
         }
-        if (ok && ht) {
-            // every update's decay was pre-applied except after the last one: TMEM holds the final state
+        // every update's decay was pre-applied except after the last one: TMEM holds the final state.  A complete last
+        // block: the decoder continues from it if that block's own type is linear, else from the state in front of the
+        // block, decayed over it.
+        bool last_lin = false, last_roll = false;
+        if (hs_row && T % 64 == 0) {
+            const long li = ((long)b * HN + hn) * 2 + 1;
+            last_lin = (last_f32 ? reinterpret_cast<const float*>(last_types)[li]
+                                 : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(last_types)[li])) > 0.f;
+            last_roll = !last_lin && decay;
+        }
+        if (ok && (ht || last_lin || last_roll)) {
             tc_fence_after();
-            float* hrow = ht + (((long)b * H + h) * K + row) * V;
+            float* hrow = ht ? ht + (((long)b * H + h) * K + row) * V : nullptr;
+            const float f = last_roll ? __expf(m_gl[NT - 1]) : 1.f;
 #pragma unroll 1
             for (int c0 = cb; c0 < cb + 64; c0 += 32) {
                 uint32_t r[32];
                 tmem_ld32(t_lane + WK_S + c0, r);
                 tmem_ld_wait();
+                if (hrow) store_row(hrow, c0, r, 1.f);
+                if (last_lin) store_row(hs_row, c0, r, 1.f);
+                if (last_roll) {
 #pragma unroll
-                for (int i = 0; i < 32; i += 4)
-                    *reinterpret_cast<float4*>(hrow + c0 + i) = make_float4(__uint_as_float(r[i]), __uint_as_float(r[i + 1]),
-                                                                           __uint_as_float(r[i + 2]), __uint_as_float(r[i + 3]));
+                    for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(hs_row[c0 + i]);
+                    store_row(hs_row, c0, r, f);
+                }
             }
         }
     }
@@ -407,11 +438,11 @@ gdn_walk_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 
 }  // namespace natsl
 
-extern "C" int natsl_gdn_walk_fused(const void* q, const void* k, const void* w, const void* u, const void* pmat,
+extern "C" int natsl_gdn_walk_fused_ex(const void* q, const void* k, const void* w, const void* u, const void* pmat,
                                     const float* gcs, const float* k_rstd, const float* q_rstd, const int32_t* types_i,
                                     const int32_t* indices, const int32_t* n_blocks, const float* h0, void* o, float* ht,
-                                    int B, int T, int H, int HN, int K, int V, int nbs, float scale, int flags,
-                                    void* stream) {
+                                    float* hstart, const void* last_types, int last_dtype, int B, int T, int H, int HN, int K,
+                                    int V, int nbs, float scale, int flags, void* stream) {
     using namespace natsl;
     NATSL_REQUIRE(q && k && w && u && pmat && gcs && k_rstd && q_rstd && types_i && indices && n_blocks && o, NATSL_ERR_NULL,
                   "natsl_gdn_walk_fused: null pointer");
@@ -421,6 +452,8 @@ extern "C" int natsl_gdn_walk_fused(const void* q, const void* k, const void* w,
                   "natsl_linear_fwd_h + natsl_linear_fwd_o", K, V, nbs);
     NATSL_REQUIRE((T + 63) / 64 <= WK_MAX_NT, NATSL_ERR_TOO_LARGE, "natsl_gdn_walk_fused: T <= 65536");
     NATSL_REQUIRE(H <= 65535 && B <= 65535, NATSL_ERR_TOO_LARGE, "natsl_gdn_walk_fused: B, H <= 65535");
+    NATSL_REQUIRE(!hstart || T % nbs != 0 || (last_types && (last_dtype == NATSL_DT_F32 || last_dtype == NATSL_DT_BF16)),
+                  NATSL_ERR_NULL, "natsl_gdn_walk_fused: the block-start state of a complete last block needs that block's types");
     auto kern = gdn_walk_tc_kernel<true>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, WkSmem::total);
     if (e != cudaSuccess) {
@@ -439,7 +472,16 @@ extern "C" int natsl_gdn_walk_fused(const void* q, const void* k, const void* w,
     const int TN = (T + nbs - 1) / nbs;
     dim3 grid(H, B);
     kern<<<grid, WK_THREADS, WkSmem::total, reinterpret_cast<cudaStream_t>(stream)>>>(
-        mw, mq, mk, mu, mp, gcs, k_rstd, q_rstd, types_i, indices, n_blocks, h0, reinterpret_cast<__nv_bfloat16*>(o), ht, T, H,
-        HN, TN, scale, (flags & NATSL_FLAG_DECAY_SKIPPED) ? 1 : 0, (flags & NATSL_FLAG_NO_TRAILING_QUIRK) ? 0 : 1, status);
+        mw, mq, mk, mu, mp, gcs, k_rstd, q_rstd, types_i, indices, n_blocks, h0, reinterpret_cast<__nv_bfloat16*>(o), ht, hstart,
+        last_types, last_dtype == NATSL_DT_F32, T, H, HN, TN, scale, (flags & NATSL_FLAG_DECAY_SKIPPED) ? 1 : 0, (flags & NATSL_FLAG_NO_TRAILING_QUIRK) ? 0 : 1, status);
     return check_launch("natsl_gdn_walk_fused");
+}
+
+extern "C" int natsl_gdn_walk_fused(const void* q, const void* k, const void* w, const void* u, const void* pmat,
+                                    const float* gcs, const float* k_rstd, const float* q_rstd, const int32_t* types_i,
+                                    const int32_t* indices, const int32_t* n_blocks, const float* h0, void* o, float* ht,
+                                    int B, int T, int H, int HN, int K, int V, int nbs, float scale, int flags,
+                                    void* stream) {
+    return natsl_gdn_walk_fused_ex(q, k, w, u, pmat, gcs, k_rstd, q_rstd, types_i, indices, n_blocks, h0, o, ht, nullptr, nullptr,
+                                   0, B, T, H, HN, K, V, nbs, scale, flags, stream);
 }

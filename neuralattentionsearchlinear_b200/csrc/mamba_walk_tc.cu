@@ -70,8 +70,9 @@ __global__ void __launch_bounds__(MW_THREADS, 1)
 mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                      const __grid_constant__ CUtensorMap map_v, const float* __restrict__ gcs,
                      const int* __restrict__ types_i, const int* __restrict__ indices, const int* __restrict__ n_blocks,
-                     const float* __restrict__ h0, __nv_bfloat16* __restrict__ o, float* __restrict__ ht, int T, int H,
-                     int HN, int TN, int nbs, float scale, int decay, int trailing_quirk, int* status) {
+                     const float* __restrict__ h0, __nv_bfloat16* __restrict__ o, float* __restrict__ ht, float* hstart,
+                     const void* __restrict__ last_types, int last_f32, int T, int H, int HN, int TN, int nbs, float scale,
+                     int decay, int trailing_quirk, int* status) {
     using L = MwSmem;
     constexpr int K = 128, V = 64;
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -327,7 +328,22 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         // Publishes this thread's state row: bf16 copy into shared memory, optionally a raw copy into the saved-state
         // region, and `value * mul` as the state in TMEM.  The value comes from the state in TMEM (src 0), the saved
         // state (src 1), the initial state (src 2, init_row) or is zero (src 3).
-        auto publish_state = [&](float mul, int src, const float* init_row, bool save) {
+        // With hs the value is also what the last block starts from: it goes to hstart with that block's carried decay.
+        const int c_last = (TN - 1) * cpb;
+        float* hs_row = hstart ? hstart + (((long)b * H + h) * K + row) * V : nullptr;
+        auto starts_last = [&](int c) -> bool {            // no chunk from c up to the last block updates the state
+            if (!hs_row || c > c_last) return false;
+            for (int j = c; j < c_last; ++j)
+                if (m_fl[j] & MW_ACTIVE) return false;
+            return true;
+        };
+        auto store_row = [&](float* dst, int c0, const uint32_t (&r)[32], float f) {
+#pragma unroll
+            for (int i = 0; i < 32; i += 4)
+                *reinterpret_cast<float4*>(dst + c0 + i) = make_float4(__uint_as_float(r[i]) * f, __uint_as_float(r[i + 1]) * f,
+                                                                      __uint_as_float(r[i + 2]) * f, __uint_as_float(r[i + 3]) * f);
+        };
+        auto publish_state = [&](float mul, int src, const float* init_row, bool save, bool hs) {
             // copy pubs & 1: MMA 1 of the chunks that read its previous content must be complete
             if (want_o && pubs >= 2) {
                 ok = __all_sync(0xffffffffu, mbar_wait(bar_cempty + (pubs & 1) * 8, ((pubs >> 1) - 1) & 1, status));
@@ -356,6 +372,7 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                     *reinterpret_cast<uint4*>(dst + swz<128>(row, (c0 >> 3) + cc)) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
                 }
                 if (save) tmem_st32(t_lane + MW_BK + c0, r);
+                if (hs) store_row(hs_row, c0, r, __expf(m_carry[c_last]));
                 if (mul != 1.f || src != 0) {
 #pragma unroll
                     for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * mul);
@@ -375,7 +392,7 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         };
         {   // initial state
             const float* init = h0 ? h0 + (((long)b * H + h) * K + row) * V : nullptr;
-            publish_state(next_dec(0), init ? 2 : 3, init, (m_fl[0] & MW_SAVE) != 0);
+            publish_state(next_dec(0), init ? 2 : 3, init, (m_fl[0] & MW_SAVE) != 0, starts_last(0));
             fence_async_smem();
             tc_fence_before();
             mbar_arrive(bar_sready);
@@ -392,7 +409,7 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 tc_fence_after();
                 const bool restore = (fl & MW_RESTORE) != 0;
                 const bool save = !restore && c + 1 < NT && (m_fl[c + 1] & MW_SAVE) != 0;
-                publish_state(next_dec(c + 1), restore ? 1 : 0, nullptr, save);
+                publish_state(next_dec(c + 1), restore ? 1 : 0, nullptr, save, starts_last(c + 1));
                 fence_async_smem();
             }
             if (ok) {
@@ -401,19 +418,34 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             }
             if (warp == 2) MW_ACC(9);
         }
-        if (ok && ht) {
-            // every update's decay was pre-applied except after the last one: TMEM holds the final state
+        // every update's decay was pre-applied except after the last one: TMEM holds the final state.  A complete last
+        // block: the decoder continues from it if that block's own type is linear, else from the state in front of the
+        // block, decayed over it.
+        bool last_lin = false, last_roll = false;
+        if (hs_row && T % nbs == 0) {
+            const long li = ((long)b * HN + hn) * 2 + 1;
+            last_lin = (last_f32 ? reinterpret_cast<const float*>(last_types)[li]
+                                 : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(last_types)[li])) > 0.f;
+            last_roll = !last_lin && decay;
+        }
+        if (ok && (ht || last_lin || last_roll)) {
             tc_fence_after();
-            float* hrow = ht + (((long)b * H + h) * K + row) * V;
+            float* hrow = ht ? ht + (((long)b * H + h) * K + row) * V : nullptr;
+            float blk_g = 0.f;
+            for (int c = c_last; c < NT; ++c) blk_g += m_gl[c];
+            const float f = __expf(blk_g);
 #pragma unroll 1
             for (int c0 = 0; c0 < 64; c0 += 32) {
                 uint32_t r[32];
                 tmem_ld32(t_lane + MW_S + c0, r);
                 tmem_ld_wait();
+                if (hrow) store_row(hrow, c0, r, 1.f);
+                if (last_lin) store_row(hs_row, c0, r, 1.f);
+                if (last_roll) {
 #pragma unroll
-                for (int i = 0; i < 32; i += 4)
-                    *reinterpret_cast<float4*>(hrow + c0 + i) = make_float4(__uint_as_float(r[i]), __uint_as_float(r[i + 1]),
-                                                                           __uint_as_float(r[i + 2]), __uint_as_float(r[i + 3]));
+                    for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(hs_row[c0 + i]);
+                    store_row(hs_row, c0, r, f);
+                }
             }
         }
     } else if (warp == 8 || warp == 9) {
@@ -561,10 +593,11 @@ extern "C" int natsl_mw_timing(long long* out, int reset) {
 }
 #endif
 
-extern "C" int natsl_mamba_walk_fused(const void* q, const void* k, const void* v, const float* gcs,
+extern "C" int natsl_mamba_walk_fused_ex(const void* q, const void* k, const void* v, const float* gcs,
                                       const int32_t* types_i, const int32_t* indices, const int32_t* n_blocks,
-                                      const float* h0, void* o, float* ht, int B, int T, int H, int HN, int K, int V,
-                                      int nbs, float scale, int flags, void* stream) {
+                                      const float* h0, void* o, float* ht, float* hstart, const void* last_types,
+                                      int last_dtype, int B, int T, int H, int HN, int K, int V, int nbs, float scale, int flags,
+                                      void* stream) {
     using namespace natsl;
     NATSL_REQUIRE(k && v && gcs && types_i && indices && n_blocks, NATSL_ERR_NULL, "natsl_mamba_walk_fused: null pointer");
     NATSL_REQUIRE((o && q) || (!o && ht), NATSL_ERR_NULL,
@@ -575,6 +608,8 @@ extern "C" int natsl_mamba_walk_fused(const void* q, const void* k, const void* 
                   "nbs=%d); use natsl_linear_fwd_h + natsl_linear_fwd_o", K, V, nbs);
     NATSL_REQUIRE((T + 63) / 64 <= MW_MAX_NT, NATSL_ERR_TOO_LARGE, "natsl_mamba_walk_fused: T <= 65536");
     NATSL_REQUIRE(H <= 65535 && B <= 65535, NATSL_ERR_TOO_LARGE, "natsl_mamba_walk_fused: B, H <= 65535");
+    NATSL_REQUIRE(!hstart || T % nbs != 0 || (last_types && (last_dtype == NATSL_DT_F32 || last_dtype == NATSL_DT_BF16)),
+                  NATSL_ERR_NULL, "natsl_mamba_walk_fused: the block-start state of a complete last block needs that block's types");
     auto kern = mamba_walk_tc_kernel;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MwSmem::total);
     if (e != cudaSuccess) {
@@ -592,7 +627,16 @@ extern "C" int natsl_mamba_walk_fused(const void* q, const void* k, const void* 
     const int TN = (T + nbs - 1) / nbs;
     dim3 grid(H, B);
     kern<<<grid, MW_THREADS, MwSmem::total, reinterpret_cast<cudaStream_t>(stream)>>>(
-        mq, mk, mv, gcs, types_i, indices, n_blocks, h0, reinterpret_cast<__nv_bfloat16*>(o), ht, T, H, HN, TN, nbs, scale,
+        mq, mk, mv, gcs, types_i, indices, n_blocks, h0, reinterpret_cast<__nv_bfloat16*>(o), ht, hstart, last_types,
+        last_dtype == NATSL_DT_F32, T, H, HN, TN, nbs, scale,
         (flags & NATSL_FLAG_DECAY_SKIPPED) ? 1 : 0, (flags & NATSL_FLAG_NO_TRAILING_QUIRK) ? 0 : 1, status);
     return check_launch("natsl_mamba_walk_fused");
+}
+
+extern "C" int natsl_mamba_walk_fused(const void* q, const void* k, const void* v, const float* gcs,
+                                      const int32_t* types_i, const int32_t* indices, const int32_t* n_blocks,
+                                      const float* h0, void* o, float* ht, int B, int T, int H, int HN, int K, int V,
+                                      int nbs, float scale, int flags, void* stream) {
+    return natsl_mamba_walk_fused_ex(q, k, v, gcs, types_i, indices, n_blocks, h0, o, ht, nullptr, nullptr, 0, B, T, H, HN, K, V,
+                                     nbs, scale, flags, stream);
 }

@@ -52,22 +52,23 @@ static EncodeTiledFn encode_fn() {
     return fn;
 }
 
-int encode_bthd_map(CUtensorMap* out, const void* base, int B, int T, int H, int D, int box_rows, const char* who) {
+int encode_bthd_map(CUtensorMap* out, const void* base, int B, int T, int H, int D, int box_rows, const char* who, int box_cols) {
     EncodeTiledFn enc = encode_fn();
     if (!enc) {
         set_error("%s: the driver does not provide cuTensorMapEncodeTiled", who);
         return NATSL_ERR_CUDA;
     }
-    if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || D % 64 != 0) {
-        set_error("%s: TMA needs a 16-byte aligned base and a head dim multiple of 64 (D=%d)", who, D);
+    if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || D % box_cols != 0) {
+        set_error("%s: TMA needs a 16-byte aligned base and a head dim multiple of %d (D=%d)", who, box_cols, D);
         return NATSL_ERR_UNSUPPORTED;
     }
     cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)H, (cuuint64_t)T, (cuuint64_t)B};
     cuuint64_t strides[3] = {(cuuint64_t)D * 2, (cuuint64_t)H * D * 2, (cuuint64_t)T * H * D * 2};
-    cuuint32_t box[4] = {64, 1, (cuuint32_t)box_rows, 1};
+    cuuint32_t box[4] = {(cuuint32_t)box_cols, 1, (cuuint32_t)box_rows, 1};
     cuuint32_t estr[4] = {1, 1, 1, 1};
     CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE,
+                     box_cols == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
         set_error("%s: cuTensorMapEncodeTiled failed (%d) for [B=%d,T=%d,H=%d,D=%d]", who, (int)r, B, T, H, D);

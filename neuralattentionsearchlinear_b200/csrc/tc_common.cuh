@@ -209,7 +209,9 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
 
 // ------------------------------------------------------------------ host: tensor maps
 // bf16 tensor [B][T][H][D] (token-major, contiguous) viewed as a 4-D TMA tensor (D, H, T, B) with
-// boxes of 64 elements x `box_rows` tokens of one head, 128-byte swizzle, zero fill out of range.
-int encode_bthd_map(CUtensorMap* out, const void* base, int B, int T, int H, int D, int box_rows, const char* who);
+// boxes of `box_cols` (64 or 32) elements x `box_rows` tokens of one head, swizzle over the box row (128 or 64 bytes: the
+// layout of swz<128> / swz<64>), zero fill out of range.
+int encode_bthd_map(CUtensorMap* out, const void* base, int B, int T, int H, int D, int box_rows, const char* who,
+                    int box_cols = 64);
 
 }  // namespace natsl

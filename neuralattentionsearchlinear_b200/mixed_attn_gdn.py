@@ -307,10 +307,18 @@ def nats_mixed_attn_gdn_chunk_inference(
     with torch.no_grad():
         tables = build_selection_tables(nats_block_types, T, nats_block_size)
         o_attn, _ = _ops.attn_fwd(q_attn, k_attn, v_attn, tables, scale_attn, own_chunk=strategy['attn'])
+        want = bool(output_final_state_gated_delta)
+        if _ops.walks_with_state(_lib.RULE_GDN, q_lattn.shape[-1], v_lattn.shape[-1], T):
+            assert not want or T % nats_block_size or op_type_last_chunk is not None
+            o_gdn, ht, inter = _ops.linear_fwd(_lib.RULE_GDN, q_lattn, k_lattn, v_lattn, g, beta, tables, scale_lattn,
+                                               initial_state_gated_delta_chunk_start, decay_for_non_gdn_blocks,
+                                               lattn_use_qk_l2norm_in_kernel, want, want_start=want,
+                                               last_types=op_type_last_chunk)
+            return o_gdn, o_attn, ht, (inter['start'] if want else None)
         o_gdn, ht, inter = _ops.linear_fwd(_lib.RULE_GDN, q_lattn, k_lattn, v_lattn, g, beta, tables, scale_lattn,
                                            initial_state_gated_delta_chunk_start, decay_for_non_gdn_blocks,
                                            lattn_use_qk_l2norm_in_kernel, True, return_intermediates=True)
-        if not output_final_state_gated_delta:
+        if not want:
             return o_gdn, o_attn, None, None
         start = _chunk_start_state(inter, ht, inter['gcs'], tables, op_type_last_chunk, T, nats_block_size,
                                    decay_for_non_gdn_blocks)

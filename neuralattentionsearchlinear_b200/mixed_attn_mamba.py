@@ -135,10 +135,17 @@ def nats_mixed_attn_mamba_chunk_inference(
     with torch.no_grad():
         tables = build_selection_tables(nats_block_types, T, nats_block_size)
         o_attn, _ = _ops.attn_fwd(q_attn, k_attn, v_attn, tables, scale_attn, own_chunk=strategy['attn'])
+        want = bool(output_final_state_mamba)
+        if _ops.walks_with_state(_lib.RULE_MAMBA, q_lattn.shape[-1], v_lattn.shape[-1], T):
+            assert not want or T % nats_block_size or op_type_last_chunk is not None
+            o_m, ht, inter = _ops.linear_fwd(_lib.RULE_MAMBA, q_lattn, k_lattn, v_lattn, g, None, tables, scale_lattn,
+                                             initial_state_mamba_start, decay_for_non_mamba_blocks, False, want,
+                                             want_start=want, last_types=op_type_last_chunk)
+            return o_m, o_attn, ht, (inter['start'] if want else None)
         o_m, ht, inter = _ops.linear_fwd(_lib.RULE_MAMBA, q_lattn, k_lattn, v_lattn, g, None, tables, scale_lattn,
                                          initial_state_mamba_start, decay_for_non_mamba_blocks, False, True,
                                          return_intermediates=True)
-        if not output_final_state_mamba:
+        if not want:
             return o_m, o_attn, None, None
         start = _chunk_start_state(inter, ht, inter['gcs'], tables, op_type_last_chunk, T, nats_block_size,
                                    decay_for_non_mamba_blocks)
