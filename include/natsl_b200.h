@@ -176,13 +176,14 @@ int natsl_gdn_walk_fused(const void* q, const void* k, const void* w, const void
 
 /* natsl_gdn_walk_fused that also writes hstart [B,H,K,V] fp32 (or NULL) = the state a decoder rolls back to: the state in
  * front of the last block with its carried decay, or, when the last block is complete (T % nbs == 0), the state behind it
- * where last_types [B,HN,2] (last_dtype fp32 or bf16: that block's own types) says linear, else the state in front of it
+ * where last_types (last_dtype fp32 or bf16: that block's own types [HN,2], last_stride elements from one
+ * batch entry to the next) says linear, else the state in front of it
  * decayed over it (NATSL_FLAG_DECAY_SKIPPED) or as it is.
  * Replaces in addition: src/nats/ops/gated_delta_rule/chunk_fwd.py:178-206. */
 int natsl_gdn_walk_fused_ex(const void* q, const void* k, const void* w, const void* u, const void* pmat,
                             const float* gcs, const float* k_rstd, const float* q_rstd, const int32_t* types_i,
                             const int32_t* indices, const int32_t* n_blocks, const float* h0, void* o, float* ht,
-                            float* hstart, const void* last_types, int last_dtype, int B, int T, int H, int HN, int K, int V,
+                            float* hstart, const void* last_types, int last_dtype, int last_stride, int B, int T, int H, int HN, int K, int V,
                             int nbs, float scale, int flags, void* stream);
 
 /* The same recurrence + output walk on mma.sync for K in {64, 128, 192}, V a multiple of 32 (64 and up) and any
@@ -190,7 +191,7 @@ int natsl_gdn_walk_fused_ex(const void* q, const void* k, const void* w, const v
 int natsl_gdn_walk(const void* q, const void* k, const void* w, const void* u, const void* pmat, const float* gcs,
                    const float* k_rstd, const float* q_rstd, const int32_t* types_i, const int32_t* indices,
                    const int32_t* n_blocks, const float* h0, void* o, float* ht, float* hstart, const void* last_types,
-                   int last_dtype, int B, int T, int H, int HN, int K, int V, int nbs, float scale, int flags, void* stream);
+                   int last_dtype, int last_stride, int B, int T, int H, int HN, int K, int V, int nbs, float scale, int flags, void* stream);
 
 /* The same walk with the value dimension split over two CTAs per (batch, head): 256 tensor-memory columns and about
  * 107 KB of shared memory per CTA, so that two of them, or one of them and one attention CTA, share an SM (the two
@@ -216,7 +217,7 @@ int natsl_mamba_walk_fused(const void* q, const void* k, const void* v, const fl
 /* natsl_mamba_walk_fused that also writes hstart (see natsl_gdn_walk_fused_ex). */
 int natsl_mamba_walk_fused_ex(const void* q, const void* k, const void* v, const float* gcs, const int32_t* types_i,
                               const int32_t* indices, const int32_t* n_blocks, const float* h0, void* o, float* ht,
-                              float* hstart, const void* last_types, int last_dtype, int B, int T, int H, int HN, int K, int V,
+                              float* hstart, const void* last_types, int last_dtype, int last_stride, int B, int T, int H, int HN, int K, int V,
                               int nbs, float scale, int flags, void* stream);
 
 /* Reference-precision (fp32 math, CUDA cores) path for fp32 or bf16 tensors (dtype = NATSL_DT_F32 / _BF16 for
@@ -245,6 +246,58 @@ int natsl_linear_recurrent_step(int rule, int dtype, const void* q, const void* 
 int natsl_attn_fwd_fp32(int dtype, const void* q, const void* k, const void* v, const int32_t* types_i, void* o,
                         float* lse, int B, int T, int HQ, int HKV, int HN, int DK, int DV, int nbs, float scale,
                         int flags, void* stream);
+
+/* Both branches of the op in one call, forward: selection tables, softmax branch, linear branch (preparation or cumsum, then
+ * the recurrence + output walk), the linear branch on a high-priority side stream of the library's own that forks from and
+ * joins `stream` inside the call.  Shapes as in natsl_attn_fwd_ex / natsl_gdn_walk(_fused_ex) / natsl_mamba_walk_fused_ex;
+ * gcs: chunk-local cumsum of g if the caller has it (Mamba2), else NULL; tables as in natsl_build_tables (starting_h_idx may
+ * be NULL; without the compact list).  ht, hstart, h0, last_types may be NULL. */
+#define NATSL_HYBRID_PREP_MMA 1        /* mma.sync chunk preparation also where the tcgen05 one is built */
+#define NATSL_HYBRID_WALK_MMA 2        /* mma.sync walk also where the tcgen05 one is built (few (batch, head) pairs) */
+#define NATSL_HYBRID_ATTN_PERSISTENT 4
+typedef struct natsl_hybrid_args {
+    int32_t B, T, H, HN, K, V, HQ, HKV, DK, DV, nbs, rule;
+    int32_t types_dtype, beta_dtype, last_dtype, last_stride, own_attn, decay, use_l2norm, options;
+    float scale_attn, scale_lin;
+    const void *q_attn, *k_attn, *v_attn, *q, *k, *v;
+    const float *g, *gcs;
+    const void *beta, *types;
+    const float* h0;
+    const void* last_types;
+    void* o_attn;
+    float* lse;
+    void* o_lin;
+    float *ht, *hstart;
+    int32_t *types_i, *indices, *n_blocks, *n_chunks_lin, *starting_h_idx, *attn_n_iters;
+    void* workspace;
+    int64_t workspace_bytes;
+} natsl_hybrid_args;
+int64_t natsl_hybrid_workspace_bytes(const natsl_hybrid_args* args);
+int natsl_hybrid_forward(const natsl_hybrid_args* args, void* stream);
+
+/* A layer's forward between its projections and its output projection (no gradients): decays and betas, short convolutions
+ * with both branches' norms, hard selection + tables, both branches, mixing weights, and the state a decoding cache keeps.
+ * Inputs (bf16): x [B,T,hidden]; logits [B,TN,HN,2]; q_raw, k_raw [B,T,H*K], v_raw [B,T,H*V] = projections; w_a, w_b
+ * [H,hidden] (w_b: delta rule); w_mix [2*HQ,H*K] or NULL; convolution and norm weights as in natsl_decode_args.
+ * Outputs: o_lin [B,T,H,V], o_attn [B,T,HQ,DV], mix [B,T,HQ,2] bf16; lse [B,T,HQ] fp32; types_raw [B,TN,HN,2] bf16 = sampled
+ * types; tables: 2*B*TN*HN*2 + 3*B*HN + B*cdiv(T,128)*HN int32 (types, indices, block counts [B,HN,2], scratch);
+ * k_attn, v_attn = keys and values of the softmax branch (v_attn also holds the linear branch's values when attn_conv and the
+ * rule is the delta rule; with attn_conv = 0 they are k_raw / v_raw themselves unless normed, and the delta rule then needs
+ * v_lin [B,T,H*V]).  Optional (NULL): ht, hstart [B,H,K,V] fp32; tail_* [B,channels,4]; g_block [B,H] and pool_sum [B,hidden]
+ * fp32 = log decay and summed input of the tokens behind the last complete block.
+ * Replaces: src/nats/layers/natsl_attn_gdn.py:411-650, src/nats/layers/natsl_attn_mamba2.py:352-590 under eval. */
+typedef struct natsl_layer_args {
+    int32_t B, T, hidden, H, K, V, HQ, HN, nbs, rule, options;
+    int32_t attn_conv, silu, own_chunk, decay, neg_eigval, qn_f32, kn_f32, alog_f32, dt_f32, reserved;
+    float norm_eps, l2_eps, scale_attn, scale_lin;
+    const void *x, *logits, *q_raw, *k_raw, *v_raw, *w_a, *w_b, *w_mix;
+    const void *cw_q, *cw_k, *cw_v, *cb_q, *cb_k, *cb_v, *qn_w, *kn_w, *A_log, *dt_bias;
+    void *o_lin, *o_attn, *mix, *lse, *types_raw, *tables, *k_attn, *v_attn, *v_lin;
+    void *ht, *hstart, *tail_q, *tail_k, *tail_v, *g_block, *pool_sum, *workspace;
+    int64_t workspace_bytes;
+} natsl_layer_args;
+int64_t natsl_layer_workspace_bytes(const natsl_layer_args* args);
+int natsl_layer_forward(const natsl_layer_args* args, void* stream);
 
 /* One decoding token of a whole layer (projections, short convolutions, linear-branch step, softmax attention over the
  * cached keys, mixing, output projection) in four launches; state is updated in place.  All tensors bf16 and contiguous

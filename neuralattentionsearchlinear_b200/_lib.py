@@ -42,14 +42,18 @@ PROTOTYPES = {
     "natsl_gdn_chunk_prep_ex": [_p, _p, _p, _p, _p, _i, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _p],
     "natsl_gdn_chunk_prep_tc": [_p, _p, _p, _p, _p, _i, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _p],
     "natsl_gdn_walk_fused": [_p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _f, _i, _p],
-    "natsl_gdn_walk_fused_ex": [_p] * 16 + [_i] * 8 + [_f, _i, _p],
-    "natsl_gdn_walk": [_p] * 16 + [_i] * 8 + [_f, _i, _p],
-    "natsl_mamba_walk_fused_ex": [_p] * 12 + [_i] * 8 + [_f, _i, _p],
+    "natsl_gdn_walk_fused_ex": [_p] * 16 + [_i] * 9 + [_f, _i, _p],
+    "natsl_gdn_walk": [_p] * 16 + [_i] * 9 + [_f, _i, _p],
+    "natsl_mamba_walk_fused_ex": [_p] * 12 + [_i] * 9 + [_f, _i, _p],
     "natsl_gdn_walk_fused_vsplit": [_p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _f, _i, _p],
     "natsl_mamba_walk_fused": [_p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _f, _i, _p],
     "natsl_linear_recurrent_fwd": [_i, _i, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _f, _i, _i, _p],
     "natsl_linear_recurrent_step": [_i, _i, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _f,
                                     _i, _i, _p],
+    "natsl_hybrid_workspace_bytes": [_p],
+    "natsl_hybrid_forward": [_p, _p],
+    "natsl_layer_workspace_bytes": [_p],
+    "natsl_layer_forward": [_p, _p],
     "natsl_decode_workspace_bytes": [_p],
     "natsl_decode_step": [_p, _p],
     "natsl_attn_fwd_fp32": [_i, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _i, _f, _i, _p],
@@ -88,6 +92,33 @@ class DecodeArgs(C.Structure):
         + [("workspace_bytes", C.c_int64)])
 
 
+class HybridArgs(C.Structure):
+    """``natsl_hybrid_args``."""
+    _fields_ = ([(n, C.c_int32) for n in (
+        "B T H HN K V HQ HKV DK DV nbs rule types_dtype beta_dtype last_dtype last_stride own_attn decay use_l2norm options").split()]
+        + [(n, C.c_float) for n in "scale_attn scale_lin".split()]
+        + [(n, C.c_void_p) for n in (
+            "q_attn k_attn v_attn q k v g gcs beta types h0 last_types o_attn lse o_lin ht hstart types_i indices n_blocks "
+            "n_chunks_lin starting_h_idx attn_n_iters workspace").split()]
+        + [("workspace_bytes", C.c_int64)])
+
+
+class LayerArgs(C.Structure):
+    """``natsl_layer_args``."""
+    _fields_ = ([(n, C.c_int32) for n in (
+        "B T hidden H K V HQ HN nbs rule options attn_conv silu own_chunk decay neg_eigval qn_f32 kn_f32 alog_f32 dt_f32 "
+        "reserved").split()]
+        + [(n, C.c_float) for n in "norm_eps l2_eps scale_attn scale_lin".split()]
+        + [(n, C.c_void_p) for n in (
+            "x logits q_raw k_raw v_raw w_a w_b w_mix cw_q cw_k cw_v cb_q cb_k cb_v qn_w kn_w A_log dt_bias "
+            "o_lin o_attn mix lse types_raw tables k_attn v_attn v_lin ht hstart tail_q tail_k tail_v g_block pool_sum "
+            "workspace").split()]
+        + [("workspace_bytes", C.c_int64)])
+
+
+HYBRID_PREP_MMA, HYBRID_WALK_MMA, HYBRID_ATTN_PERSISTENT = 1, 2, 4
+
+
 _lib = None
 
 
@@ -108,7 +139,7 @@ def load() -> C.CDLL:
     lib.natsl_last_error.argtypes = []
     for name, args in PROTOTYPES.items():
         fn = getattr(lib, name)
-        fn.restype = C.c_int64 if name == "natsl_decode_workspace_bytes" else C.c_int
+        fn.restype = C.c_int64 if name.endswith("_workspace_bytes") else C.c_int
         fn.argtypes = args
     _lib = lib
     return lib
@@ -116,6 +147,7 @@ def load() -> C.CDLL:
 
 # kernels one successful call of an entry point launches (for launch accounting; entry points not listed launch one)
 KERNELS_PER_CALL = {"natsl_build_tables": 2, "natsl_attn_bwd": 2, "natsl_gdn_fwd_noalloc": 3, "natsl_decode_step": 4,
+                    "natsl_hybrid_forward": 4, "natsl_layer_forward": 7,
                     "natsl_abi_version": 0,
                     "natsl_device_status": 0}
 _launches = 0

@@ -1,12 +1,13 @@
 """Thin launch wrappers: allocate outputs with torch, pass raw pointers to the C ABI."""
 from __future__ import annotations
 
+import ctypes
 import os
 
 import torch
 
 from . import _lib
-from .nats_util import SelectionTables, cdiv, current_stream_ptr
+from .nats_util import _TYPE_CODES, SelectionTables, cdiv, current_stream_ptr
 
 BF16 = torch.bfloat16
 USE_MAMBA_WALK = os.environ.get("NATSL_MAMBA_WALK", "1") != "0"    # natsl_mamba_walk_fused (K = 128, V = 64)
@@ -220,14 +221,14 @@ def linear_fwd(rule: int, q, k, v, g, beta, tables: SelectionTables, scale: floa
             _lib.call("natsl_gdn_walk_fused_vsplit", *args, *dims)
         else:
             _lib.call("natsl_gdn_walk_fused_ex" if tc_walk else "natsl_gdn_walk", *args, _lib.ptr(start),
-                      _lib.ptr(last_types if want_start else None), last_code, *dims)
+                      _lib.ptr(last_types if want_start else None), last_code, 2 * HN, *dims)
         return o, ht, inter
     if mamba_fused:
         o = None if skip_out else torch.empty(B, T, H, V, dtype=BF16, device=dev)
         _lib.call("natsl_mamba_walk_fused_ex", None if skip_out else q.data_ptr(), k.data_ptr(), v.data_ptr(), gcs.data_ptr(),
                   tables.types_i.data_ptr(), tables.indices.data_ptr(), tables.n_blocks.data_ptr(), _lib.ptr(h0),
                   _lib.ptr(o), _lib.ptr(ht), _lib.ptr(start), _lib.ptr(last_types if want_start else None), last_code,
-                  B, T, H, HN, K, V, nbs, float(scale), flags, st)
+                  2 * HN, B, T, H, HN, K, V, nbs, float(scale), flags, st)
         return o, ht, (dict(gcs=gcs) if skip_out else inter)
     state_only = skip_out and ht is not None and not return_intermediates
     h = None if state_only else torch.empty(B, NT, H, K, V, dtype=BF16, device=dev)
@@ -243,6 +244,98 @@ def linear_fwd(rule: int, q, k, v, g, beta, tables: SelectionTables, scale: floa
               _lib.ptr(krstd), h.data_ptr(), carry.data_ptr(), o.data_ptr(), B, T, H, K, V, float(scale),
               int(use_l2norm and rule == _lib.RULE_GDN) | (0 if own_chunk else 2), st)
     return o, ht, inter
+
+
+def tables_from_flat(flat, B: int, TN: int, HN: int, T: int, nbs: int) -> SelectionTables:
+    """Views of the tables ``hybrid_fwd`` built into one buffer (without the compact chunk list and its offsets)."""
+    NT, NTq = cdiv(T, 64), cdiv(T, _lib.ATTN_BT)
+    sizes = [B * TN * HN * 2, B * TN * HN * 2, B * HN * 2, B * HN, B * NT * HN, B * NTq * HN]
+    ti, ix, nb, nc, sh, an = torch.split(flat, sizes)
+    return SelectionTables(types_i=ti.view(B, TN, HN, 2), indices=ix.view(B, TN, HN, 2), n_blocks=nb.view(B, HN, 2), n_chunks_lin=nc,
+                           offsets=None, chunk_indices=None, starting_h_idx=sh.view(B, NT, HN), attn_n_iters=an.view(B, NTq, HN),
+                           T=T, nats_block_size=nbs)
+
+
+_hybrid_ws: dict = {}
+
+
+def hybrid_fwd(rule: int, q_attn, k_attn, v_attn, q, k, v, g, beta, types, nbs: int, scale_attn: float, scale_lin: float, h0,
+               own_attn: bool, decay: bool, use_l2norm: bool, want_ht: bool, want_start: bool = False, last_types=None):
+    """Tables and both branches in one native call (bf16 tensors, head dims of ``walks_with_state``, own-block linear
+    attention).  -> (o_lin, o_attn, lse, ht, start, flat tables for ``tables_from_flat``)."""
+    for t_ in (q_attn, k_attn, v_attn, q, k, v):
+        _need(t_.dim() == 4, "q, k, v must be [B, T, H, D]")
+        _need(t_.is_cuda and t_.device == q.device, "q, k, v of both branches must be on one CUDA device")
+        _need(t_.dtype == BF16, "the branches need q, k, v in one dtype: bf16", TypeError)
+    q_attn, k_attn, v_attn, q, k, v = (t_.contiguous() for t_ in (q_attn, k_attn, v_attn, q, k, v))
+    B, T, H, K = q.shape
+    V, HQ, DK, HKV, DV = v.shape[3], q_attn.shape[2], q_attn.shape[3], k_attn.shape[2], v_attn.shape[3]
+    dev = q.device
+    TN, HN = types.shape[1], types.shape[2]
+    _need(tuple(k.shape) == (B, T, H, K), f"linear branch: q {tuple(q.shape)} and k {tuple(k.shape)} differ")
+    _need(tuple(v.shape) == (B, T, H, V), f"linear branch: k {tuple(k.shape)} and v {tuple(v.shape)} differ in length or heads")
+    _need(tuple(q_attn.shape) == (B, T, HQ, DK) and tuple(k_attn.shape) == (B, T, HKV, DK) and tuple(v_attn.shape) == (B, T, HKV, DV),
+          f"softmax branch: q {tuple(q_attn.shape)}, k {tuple(k_attn.shape)}, v {tuple(v_attn.shape)} do not match")
+    _need(HQ % HKV == 0, f"softmax branch: {HQ} query heads over {HKV} key/value heads")
+    _need(tuple(g.shape) == (B, T, H) and g.device == dev, f"g must be [B,T,H] = {(B, T, H)} on {dev}, got {tuple(g.shape)}")
+    if not types.is_cuda:
+        raise ValueError("nats_block_types must be a CUDA tensor (there is no CPU path)")
+    if types.dtype not in _TYPE_CODES:
+        raise TypeError(f"unsupported nats_block_types dtype {types.dtype}")
+    if types.shape[3] != 2:
+        raise NotImplementedError("selection tables are specified for n_ops == 2")
+    _need(types.shape[0] == B and types.device == dev, "the block types were made for another batch or device")
+    _need(TN == cdiv(T, nbs), f"{TN} blocks of {nbs} tokens do not cover T={T}")
+    _need(H % HN == 0 and HQ % HN == 0, f"{H} / {HQ} heads over {HN} selection heads")
+    g = g.float().contiguous()
+    types = types.contiguous()
+    a = _lib.HybridArgs()
+    if rule == _lib.RULE_GDN:
+        _need(beta is not None, "the gated delta rule needs beta")
+        _need(tuple(beta.shape) == (B, T, H) and beta.device == dev, f"beta must be [B,T,H] = {(B, T, H)} on {dev}")
+        _need(beta.dtype in (BF16, torch.float32), "beta must be bf16 or fp32", TypeError)
+        beta = beta.contiguous()
+        a.beta, a.beta_dtype = beta.data_ptr(), _dt_code(beta)
+    if h0 is not None:
+        h0 = h0.float().contiguous()
+        _need(tuple(h0.shape) == (B, H, K, V), f"initial state must be [B,H,K,V], got {tuple(h0.shape)}")
+        a.h0 = h0.data_ptr()
+    o_lin = torch.empty(B, T, H, V, dtype=BF16, device=dev)
+    o_attn = torch.empty(B, T, HQ, DV, dtype=BF16, device=dev)
+    lse = torch.empty(B, T, HQ, dtype=torch.float32, device=dev)
+    ht = torch.empty(B, H, K, V, dtype=torch.float32, device=dev) if want_ht else None
+    start = torch.empty(B, H, K, V, dtype=torch.float32, device=dev) if want_start else None
+    if want_start and T % nbs == 0:
+        _need(last_types is not None and tuple(last_types.shape) == (B, HN, 2), "a complete last block needs its types [B,HN,2]")
+        last_types = (last_types if last_types.dtype in (BF16, torch.float32) else last_types.float()).contiguous()
+        a.last_types, a.last_dtype, a.last_stride = last_types.data_ptr(), _dt_code(last_types), 2 * HN
+    NT, NTq = cdiv(T, 64), cdiv(T, _lib.ATTN_BT)
+    nt = B * TN * HN * 2
+    flat = torch.empty(2 * nt + 3 * B * HN + B * (NT + NTq) * HN, dtype=torch.int32, device=dev)
+    p = flat.data_ptr()
+    a.types_i, a.indices, a.n_blocks = p, p + 4 * nt, p + 8 * nt
+    a.n_chunks_lin = a.n_blocks + 8 * B * HN
+    a.starting_h_idx = a.n_chunks_lin + 4 * B * HN
+    a.attn_n_iters = a.starting_h_idx + 4 * B * NT * HN
+    a.B, a.T, a.H, a.HN, a.K, a.V, a.HQ, a.HKV, a.DK, a.DV, a.nbs, a.rule = B, T, H, HN, K, V, HQ, HKV, DK, DV, nbs, rule
+    a.types_dtype = _TYPE_CODES[types.dtype]
+    a.own_attn, a.decay, a.use_l2norm = int(own_attn), int(decay), int(use_l2norm)
+    a.options = ((0 if PREP_TC else _lib.HYBRID_PREP_MMA) | (_lib.HYBRID_WALK_MMA if B * H <= WALK_MMA_MAX_HEADS else 0)
+                 | (_lib.HYBRID_ATTN_PERSISTENT if ATTN_PERSISTENT else 0))
+    a.scale_attn, a.scale_lin = scale_attn, scale_lin
+    a.q_attn, a.k_attn, a.v_attn, a.q, a.k, a.v = (t_.data_ptr() for t_ in (q_attn, k_attn, v_attn, q, k, v))
+    a.g, a.types, a.o_attn, a.lse, a.o_lin = g.data_ptr(), types.data_ptr(), o_attn.data_ptr(), lse.data_ptr(), o_lin.data_ptr()
+    a.ht, a.hstart = _lib.ptr(ht), _lib.ptr(start)
+    key = (rule, B, T, H, K, V)
+    need = _hybrid_ws.get(key)
+    if need is None:
+        if len(_hybrid_ws) > 1024:
+            _hybrid_ws.clear()
+        need = _hybrid_ws[key] = _lib.load().natsl_hybrid_workspace_bytes(ctypes.byref(a))
+    ws = torch.empty(need, dtype=torch.uint8, device=dev)
+    a.workspace, a.workspace_bytes = ws.data_ptr(), need
+    _lib.call("natsl_hybrid_forward", ctypes.byref(a), current_stream_ptr(dev))
+    return o_lin, o_attn, lse, ht, start, flat
 
 
 def _dt_code(t):

@@ -55,7 +55,7 @@ gdn_walk_mma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                     const float* __restrict__ krstd, const float* __restrict__ qrstd, const int* __restrict__ types_i,
                     const int* __restrict__ indices, const int* __restrict__ n_blocks, const float* __restrict__ h0,
                     __nv_bfloat16* __restrict__ o, float* __restrict__ ht, float* hstart, const void* __restrict__ last_types,
-                    int last_f32, int T, int H, int HN, int V, int TN, int nbs, float scale, int decay, int trailing_quirk,
+                    int last_f32, int last_stride, int T, int H, int HN, int V, int TN, int nbs, float scale, int decay, int trailing_quirk,
                     int* status) {
     using L = GwSmem<K, BV>;
     constexpr int MT = K / 64, NTL = BV / 8, NSUB = K / 64;
@@ -361,7 +361,7 @@ gdn_walk_mma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     if (hstart && T % nbs == 0) {
         // the last block is complete: the decoder starts from the state behind it if its own type is linear, else from
         // the state in front of it, decayed over it
-        const long li = ((long)b * HN + hn) * 2 + 1;
+        const long li = (long)b * last_stride + hn * 2 + 1;
         const float lt = last_f32 ? reinterpret_cast<const float*>(last_types)[li]
                                   : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(last_types)[li]);
         if (lt > 0.f) {
@@ -385,7 +385,7 @@ gdn_walk_mma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 template <int K, int BV>
 static int launch_walk_mma(const void* q, const void* k, const void* w, const void* u, const void* pmat, const float* gcs,
                            const float* krstd, const float* qrstd, const int* types_i, const int* indices, const int* n_blocks,
-                           const float* h0, void* o, float* ht, float* hstart, const void* last_types, int last_f32, int B, int T,
+                           const float* h0, void* o, float* ht, float* hstart, const void* last_types, int last_f32, int last_stride, int B, int T,
                            int H, int HN, int V, int nbs, float scale, int flags, cudaStream_t st) {
     using L = GwSmem<K, BV>;
     const char* who = "natsl_gdn_walk";
@@ -410,7 +410,7 @@ static int launch_walk_mma(const void* q, const void* k, const void* w, const vo
     if (rc != NATSL_OK) return rc;
     kern<<<dim3(V / BV, H, B), gw_threads<BV>, smem, st>>>(
         mw, mq, mk, mu, mp, gcs, krstd, qrstd, types_i, indices, n_blocks, h0, reinterpret_cast<__nv_bfloat16*>(o), ht, hstart,
-        last_types, last_f32, T, H, HN, V, (T + nbs - 1) / nbs, nbs, scale, (flags & NATSL_FLAG_DECAY_SKIPPED) ? 1 : 0,
+        last_types, last_f32, last_stride, T, H, HN, V, (T + nbs - 1) / nbs, nbs, scale, (flags & NATSL_FLAG_DECAY_SKIPPED) ? 1 : 0,
         (flags & NATSL_FLAG_NO_TRAILING_QUIRK) ? 0 : 1, status);
     return check_launch(who);
 }
@@ -420,7 +420,7 @@ static int launch_walk_mma(const void* q, const void* k, const void* w, const vo
 extern "C" int natsl_gdn_walk(const void* q, const void* k, const void* w, const void* u, const void* pmat, const float* gcs,
                               const float* k_rstd, const float* q_rstd, const int32_t* types_i, const int32_t* indices,
                               const int32_t* n_blocks, const float* h0, void* o, float* ht, float* hstart,
-                              const void* last_types, int last_dtype, int B, int T, int H, int HN, int K, int V, int nbs,
+                              const void* last_types, int last_dtype, int last_stride, int B, int T, int H, int HN, int K, int V, int nbs,
                               float scale, int flags, void* stream) {
     using namespace natsl;
     NATSL_REQUIRE(q && k && w && u && pmat && gcs && k_rstd && q_rstd && types_i && indices && n_blocks && o, NATSL_ERR_NULL,
@@ -435,7 +435,7 @@ extern "C" int natsl_gdn_walk(const void* q, const void* k, const void* w, const
     const int f32 = last_dtype == NATSL_DT_F32;
 #define NATSL_GW(KK, BB) \
     return launch_walk_mma<KK, BB>(q, k, w, u, pmat, gcs, k_rstd, q_rstd, types_i, indices, n_blocks, h0, o, ht, hstart, \
-                                   last_types, f32, B, T, H, HN, V, nbs, scale, flags, st)
+                                   last_types, f32, last_stride, B, T, H, HN, V, nbs, scale, flags, st)
     // 32 value columns per CTA while that still leaves no second wave, 64 otherwise (the w, q, k and P tiles are then read
     // half as often).
     const bool narrow = V % 64 != 0 || (long)B * H * (V / 32) <= 148;

@@ -46,7 +46,7 @@ gdn_walk_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                    const float* __restrict__ krstd, const float* __restrict__ qrstd, const int* __restrict__ types_i,
                    const int* __restrict__ indices, const int* __restrict__ n_blocks, const float* __restrict__ h0,
                    __nv_bfloat16* __restrict__ o, float* __restrict__ ht, float* hstart, const void* __restrict__ last_types,
-                   int last_f32, int T, int H, int HN, int TN, float scale, int decay, int trailing_quirk, int* status) {
+                   int last_f32, int last_stride, int T, int H, int HN, int TN, float scale, int decay, int trailing_quirk, int* status) {
     using L = WkSmem;
     constexpr int K = 128, V = 128;
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -406,7 +406,7 @@ gdn_walk_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         // block, decayed over it.
         bool last_lin = false, last_roll = false;
         if (hs_row && T % 64 == 0) {
-            const long li = ((long)b * HN + hn) * 2 + 1;
+            const long li = (long)b * last_stride + hn * 2 + 1;
             last_lin = (last_f32 ? reinterpret_cast<const float*>(last_types)[li]
                                  : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(last_types)[li])) > 0.f;
             last_roll = !last_lin && decay;
@@ -441,7 +441,7 @@ gdn_walk_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 extern "C" int natsl_gdn_walk_fused_ex(const void* q, const void* k, const void* w, const void* u, const void* pmat,
                                     const float* gcs, const float* k_rstd, const float* q_rstd, const int32_t* types_i,
                                     const int32_t* indices, const int32_t* n_blocks, const float* h0, void* o, float* ht,
-                                    float* hstart, const void* last_types, int last_dtype, int B, int T, int H, int HN, int K,
+                                    float* hstart, const void* last_types, int last_dtype, int last_stride, int B, int T, int H, int HN, int K,
                                     int V, int nbs, float scale, int flags, void* stream) {
     using namespace natsl;
     NATSL_REQUIRE(q && k && w && u && pmat && gcs && k_rstd && q_rstd && types_i && indices && n_blocks && o, NATSL_ERR_NULL,
@@ -473,7 +473,7 @@ extern "C" int natsl_gdn_walk_fused_ex(const void* q, const void* k, const void*
     dim3 grid(H, B);
     kern<<<grid, WK_THREADS, WkSmem::total, reinterpret_cast<cudaStream_t>(stream)>>>(
         mw, mq, mk, mu, mp, gcs, k_rstd, q_rstd, types_i, indices, n_blocks, h0, reinterpret_cast<__nv_bfloat16*>(o), ht, hstart,
-        last_types, last_dtype == NATSL_DT_F32, T, H, HN, TN, scale, (flags & NATSL_FLAG_DECAY_SKIPPED) ? 1 : 0, (flags & NATSL_FLAG_NO_TRAILING_QUIRK) ? 0 : 1, status);
+        last_types, last_dtype == NATSL_DT_F32, last_stride, T, H, HN, TN, scale, (flags & NATSL_FLAG_DECAY_SKIPPED) ? 1 : 0, (flags & NATSL_FLAG_NO_TRAILING_QUIRK) ? 0 : 1, status);
     return check_launch("natsl_gdn_walk_fused");
 }
 
@@ -483,5 +483,5 @@ extern "C" int natsl_gdn_walk_fused(const void* q, const void* k, const void* w,
                                     int B, int T, int H, int HN, int K, int V, int nbs, float scale, int flags,
                                     void* stream) {
     return natsl_gdn_walk_fused_ex(q, k, w, u, pmat, gcs, k_rstd, q_rstd, types_i, indices, n_blocks, h0, o, ht, nullptr, nullptr,
-                                   0, B, T, H, HN, K, V, nbs, scale, flags, stream);
+                                   0, 0, B, T, H, HN, K, V, nbs, scale, flags, stream);
 }

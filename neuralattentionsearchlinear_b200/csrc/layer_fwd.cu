@@ -1,0 +1,628 @@
+// The steps of a NAtSL layer between its projection GEMMs and its output GEMM, forward without gradients, as one call:
+// selection (hard softmax of the block logits), decays, short convolutions with the norms of both branches, mixing weights,
+// selection tables, both attention branches on two streams, and what a decoding cache keeps
+// (src/nats/layers/natsl_attn_gdn.py:411-650, src/nats/layers/natsl_attn_mamba2.py:352-590).
+// Why one call: a prompt of a thousand tokens is some 200 us of device work in 46 launches that took the host 900 us to
+// issue from Python (about 30 of them torch elementwise kernels over small tensors); the large-batch case read and wrote
+// every projection two or three times (convolution, norm, cast) on its way.  What each kernel is bound by stands beside it.
+#include <mutex>
+
+#include "layer_fwd.cuh"
+#include "tc_common.cuh"
+#include "../../include/natsl_b200.h"
+
+namespace natsl {
+
+namespace {
+
+using bf16 = __nv_bfloat16;
+
+__device__ __forceinline__ float bf(const bf16* p, long i) { return __bfloat162float(p[i]); }
+__device__ __forceinline__ float rb(float x) { return __bfloat162float(__float2bfloat16(x)); }
+__device__ __forceinline__ float ldw(const void* p, int f32, long i) {
+    return f32 ? reinterpret_cast<const float*>(p)[i] : __bfloat162float(reinterpret_cast<const bf16*>(p)[i]);
+}
+
+// ------------------------------------------------------------------------------------------------ narrow projections
+// y[t, n] = x[t, :] . W[n, :] for a few rows n (2 H decays and betas, or 2 HQ mixing logits) with the pointwise steps
+// behind it.  Bound by reading x once; the torch form read it once per GEMM and took seven more kernels over the results.
+// One CTA = one 64-token chunk: eight warps = 2 groups of 32 tokens x 4 slices of the contraction, fragments loaded
+// straight from global memory (a lane's 16 bytes are the fragment pairs of a 32-wide k group under a permuted k order).
+struct NarrowArgs {
+    const bf16 *x, *w0, *w1;                  // x [B,T,Kdim]; w0 [n0,Kdim], w1 [n1,Kdim] or NULL
+    int n0, n1, T, Kdim, mode;                // mode 0: decays (w0) and betas (w1); mode 1: softmax over pairs of rows
+    const void *A_log, *dt_bias;
+    int alog_f32, dt_f32, neg_eigval;
+    float *g, *gcs, *dt;                      // [B,T,n0]; gcs, dt or NULL
+    bf16* out;                                // mode 0: beta [B,T,n1]; mode 1: weights [B,T,n0]
+};
+
+template <int NB>
+__global__ void __launch_bounds__(256) narrow_kernel(const NarrowArgs a) {
+    constexpr int N = NB * 8, LD = N + 1;
+    extern __shared__ float red[];            // [4][64][LD]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    const int mg = warp & 1, wk = warp >> 1;
+    const int c = blockIdx.x, b = blockIdx.y, valid = min(64, a.T - c * 64);
+    const int n_all = a.n0 + a.n1, n_base = blockIdx.z * N;
+    const bf16* x = a.x + ((long)b * a.T + (long)c * 64) * a.Kdim;
+    const int nc = a.Kdim / 32, c0 = nc * wk / 4, c1 = nc * (wk + 1) / 4;
+    const bf16* xr[4];
+    const bf16* wr[NB];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) xr[i] = x + (long)min(mg * 32 + i * 8 + g, valid - 1) * a.Kdim + t * 8;
+#pragma unroll
+    for (int n = 0; n < NB; ++n) {
+        const int row = min(n_base + n * 8 + g, n_all - 1);
+        wr[n] = (row < a.n0 ? a.w0 + (long)row * a.Kdim : a.w1 + (long)(row - a.n0) * a.Kdim) + t * 8;
+    }
+    float acc[2][NB][4];
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int n = 0; n < NB; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[m][n][e] = 0.f;
+    constexpr int UN = NB >= 8 ? 1 : 2;
+    for (int k = c0; k < c1; k += UN) {
+        uint4 xv[UN][4], wv[UN][NB];
+#pragma unroll
+        for (int u = 0; u < UN; ++u) {
+            const int kk = min(k + u, c1 - 1) * 32;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) xv[u][i] = *reinterpret_cast<const uint4*>(xr[i] + kk);
+#pragma unroll
+            for (int n = 0; n < NB; ++n) wv[u][n] = __ldg(reinterpret_cast<const uint4*>(wr[n] + kk));
+        }
+#pragma unroll
+        for (int u = 0; u < UN; ++u) {
+            if (k + u >= c1) break;
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+                const uint4 p = xv[u][2 * m], q = xv[u][2 * m + 1];
+                const uint32_t f0[4] = {p.x, q.x, p.y, q.y}, f1[4] = {p.z, q.z, p.w, q.w};
+#pragma unroll
+                for (int n = 0; n < NB; ++n) {
+                    mma_bf16(acc[m][n], f0, wv[u][n].x, wv[u][n].y);
+                    mma_bf16(acc[m][n], f1, wv[u][n].z, wv[u][n].w);
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int n = 0; n < NB; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                red[(wk * 64 + mg * 32 + m * 16 + g + 8 * (e >> 1)) * LD + n * 8 + 2 * t + (e & 1)] = acc[m][n][e];
+    __syncthreads();
+    const long tok0 = (long)b * a.T + (long)c * 64;
+    auto total = [&](int r, int n) {
+        return rb(((red[r * LD + n] + red[(64 + r) * LD + n]) + red[(128 + r) * LD + n]) + red[(192 + r) * LD + n]);
+    };
+    if (a.mode == 1) {
+        for (int i = tid; i < 64 * (N / 2); i += 256) {
+            const int r = i / (N / 2), n = (i % (N / 2)) * 2;
+            if (r < valid && n_base + n < a.n0) {
+                const float l0 = total(r, n), l1 = total(r, n + 1), mx = fmaxf(l0, l1);
+                const float e0 = expf(l0 - mx), e1 = expf(l1 - mx), s = e0 + e1;
+                *reinterpret_cast<__nv_bfloat162*>(a.out + (tok0 + r) * a.n0 + n_base + n) = __floats2bfloat162_rn(e0 / s, e1 / s);
+            }
+        }
+        return;
+    }
+    for (int i = tid; i < 64 * N; i += 256) {
+        const int r = i / N, nn = i % N, n = n_base + nn;
+        float gt = 0.f;
+        if (r < valid && n < n_all) {
+            const float y = total(r, nn);
+            if (n < a.n0) {
+                const float z = y + ldw(a.dt_bias, a.dt_f32, n);
+                const float sp = z > 20.f ? z : log1pf(expf(z));
+                gt = -expf(ldw(a.A_log, a.alog_f32, n)) * sp;
+                a.g[(tok0 + r) * a.n0 + n] = gt;
+                if (a.dt) a.dt[(tok0 + r) * a.n0 + n] = sp;
+            } else {
+                float be = rb(1.f / (1.f + expf(-y)));
+                if (a.neg_eigval) be *= 2.f;
+                a.out[(tok0 + r) * a.n1 + n - a.n0] = __float2bfloat16(be);
+            }
+        }
+        if (a.gcs) red[r * LD + nn] = gt;                  // this thread's own entry: nobody else reads it before the barrier
+    }
+    if (a.gcs) {                                           // chunk-local cumsum, one warp per head
+        __syncthreads();
+        for (int nn = warp; nn < N && n_base + nn < a.n0; nn += 8) {
+            float lo = red[lane * LD + nn], hi = red[(lane + 32) * LD + nn];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const float u = __shfl_up_sync(0xffffffffu, lo, o), v = __shfl_up_sync(0xffffffffu, hi, o);
+                if (lane >= o) { lo += u; hi += v; }
+            }
+            hi += __shfl_sync(0xffffffffu, lo, 31);
+            if (lane < valid) a.gcs[(tok0 + lane) * a.n0 + n_base + nn] = lo;
+            if (lane + 32 < valid) a.gcs[(tok0 + lane + 32) * a.n0 + n_base + nn] = hi;
+        }
+    }
+}
+
+int launch_narrow(const NarrowArgs& a, int B, cudaStream_t st) {
+    const int n = a.n0 + a.n1;
+    const int NB = n <= 16 ? 2 : n <= 32 ? 4 : 8;
+    const size_t smem = (size_t)4 * 64 * (NB * 8 + 1) * 4;
+    dim3 grid((a.T + 63) / 64, B, (n + NB * 8 - 1) / (NB * 8));
+    cudaError_t e = cudaSuccess;
+    if (NB == 8) e = cudaFuncSetAttribute(narrow_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) {
+        set_error("natsl_layer_forward: cannot reserve %d B of shared memory (%s)", (int)smem, cudaGetErrorString(e));
+        return NATSL_ERR_CUDA;
+    }
+    if (NB == 2) narrow_kernel<2><<<grid, 256, smem, st>>>(a);
+    else if (NB == 4) narrow_kernel<4><<<grid, 256, smem, st>>>(a);
+    else narrow_kernel<8><<<grid, 256, smem, st>>>(a);
+    return check_launch("natsl_layer_forward (narrow projection)");
+}
+
+// ------------------------------------------------------------------------------------------------ convolutions + norms
+// Short causal convolution + SiLU of the q, k and v projections with the row norms behind it, each projection read once:
+//   lin  = conv, conv / ||conv|| (Mamba2 q, k) or conv * dt (Mamba2 v);   attn = RMS norm of conv or of the raw projection;
+//   conv = the convolution itself where the mixing weights or the softmax branch need it beside a normed copy.
+// Bandwidth: a lane owns 8 channels (16-byte accesses, 256 channels per warp) and slides over TT tokens with the next four
+// rows in flight; a norm group (a head) is 8, 16 or 32 neighbouring lanes.  The three convolutions and two norms as kernels
+// of their own took 402 us at B = 16, T = 4096, 1024 channels; the sigmoid's division is the approximate one (2 ulp in
+// fp32, rounded to bf16 right behind it), which is what keeps the kernel off the instruction roof.
+struct ConvSeg {
+    const bf16 *x, *w, *bias;
+    bf16 *lin, *attn, *conv, *tail;
+    const void* nw;                           // norm weights [DK] (attn)
+    int nw_f32, D, lin_mode, attn_mode;       // lin 0 plain 1 l2 norm 2 times dt; attn 0 none 1 norm of conv 2 norm of raw
+    int lin_lanes, attn_lanes, head, blk0;    // lanes of a norm group; channels per head (dt); first grid block
+};
+struct ConvArgs {
+    ConvSeg seg[3];
+    const float* dt;
+    int T, H, silu, TT;
+    float l2_eps, norm_eps;
+};
+
+__global__ void __launch_bounds__(128) conv_norm_kernel(const ConvArgs a) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, b = blockIdx.z;
+    const int si = (int)blockIdx.x >= a.seg[2].blk0 ? 2 : (int)blockIdx.x >= a.seg[1].blk0 ? 1 : 0;
+    const ConvSeg& s = a.seg[si];
+    const int D = s.D, d0 = ((int)blockIdx.x - s.blk0) * 256 + lane * 8;
+    const bool ok = d0 < D;
+    const int dd = ok ? d0 : D - 8;                        // idle lanes stay in the shuffles
+    const int t0 = ((int)blockIdx.y * 4 + warp) * a.TT, t1 = min(a.T, t0 + a.TT);
+    if (t0 >= a.T) return;
+    float w[8][4], bs[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        const uint2 u = *reinterpret_cast<const uint2*>(s.w + (long)(dd + c) * 4);
+        const float2 lo = unpack_bf16(u.x), hi = unpack_bf16(u.y);
+        w[c][0] = lo.x; w[c][1] = lo.y; w[c][2] = hi.x; w[c][3] = hi.y;
+        bs[c] = s.bias ? bf(s.bias, dd + c) : 0.f;
+    }
+    float nw[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) nw[c] = s.attn_mode ? ldw(s.nw, s.nw_f32, (dd + c) & (s.attn_lanes * 8 - 1)) : 0.f;
+    const float* dt = s.lin_mode == 2 ? a.dt + (long)b * a.T * a.H + dd / s.head : nullptr;
+    const bf16* x = s.x + (long)b * a.T * D + dd;
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+    auto ld = [&](int t) { return t >= 0 && t < a.T ? *reinterpret_cast<const uint4*>(x + (long)t * D) : zero; };
+    auto open = [](const uint4& v, float (&f)[8]) {
+        const uint32_t* u = reinterpret_cast<const uint32_t*>(&v);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float2 p = unpack_bf16(u[i]);
+            f[2 * i] = p.x;
+            f[2 * i + 1] = p.y;
+        }
+    };
+    float h0[8], h1[8], h2[8];                             // inputs of the three tokens before
+    open(ld(t0 - 3), h0);
+    open(ld(t0 - 2), h1);
+    open(ld(t0 - 1), h2);
+    uint4 nxt[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) nxt[i] = ld(t0 + i);
+    auto group_sum = [&](const float (&f)[8], int lanes) {
+        float ss = 0.f;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) ss += f[c] * f[c];
+        for (int o = lanes >> 1; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        return ss;
+    };
+    auto st = [&](bf16* p, int t, const float (&f)[8]) {
+        if (ok) *reinterpret_cast<uint4*>(p + ((long)b * a.T + t) * D + d0) =
+            make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
+    };
+    for (int tb = t0; tb < t1; tb += 4) {
+        uint4 cur[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) cur[i] = nxt[i];
+        if (tb + 4 < t1)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) nxt[i] = ld(tb + 4 + i);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int t = tb + i;
+            if (t >= t1) break;
+            float r[8], y[8];
+            open(cur[i], r);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                float v = bs[c];
+                v += w[c][0] * h0[c];
+                v += w[c][1] * h1[c];
+                v += w[c][2] * h2[c];
+                v += w[c][3] * r[c];
+                y[c] = rb(a.silu ? __fdividef(v, 1.f + __expf(-v)) : v);
+                h0[c] = h1[c];
+                h1[c] = h2[c];
+                h2[c] = r[c];
+            }
+            if (s.conv) st(s.conv, t, y);
+            if (s.attn_mode) {
+                float z[8];
+                const float rs = rsqrtf(group_sum(s.attn_mode == 1 ? y : r, s.attn_lanes) / (s.attn_lanes * 8) + a.norm_eps);
+#pragma unroll
+                for (int c = 0; c < 8; ++c)
+                    z[c] = (s.attn_mode == 1 ? y[c] : r[c]) * rs * nw[c];
+                st(s.attn, t, z);
+            }
+            if (s.lin_mode == 1) {
+                const float rs = rsqrtf(group_sum(y, s.lin_lanes) + a.l2_eps);
+#pragma unroll
+                for (int c = 0; c < 8; ++c) y[c] *= rs;
+            } else if (s.lin_mode == 2) {
+                const float d = dt[(long)t * a.H];
+#pragma unroll
+                for (int c = 0; c < 8; ++c) y[c] *= d;
+            }
+            st(s.lin, t, y);
+        }
+    }
+    if (s.tail && t1 == a.T && ok) {                       // the last four inputs, oldest first
+#pragma unroll
+        for (int i = 0; i < 4; ++i) nxt[i] = ld(a.T - 4 + i);
+        const bf16* n0 = reinterpret_cast<const bf16*>(&nxt[0]);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            bf16 o4[4] = {n0[c], n0[8 + c], n0[16 + c], n0[24 + c]};
+            *reinterpret_cast<uint2*>(s.tail + ((long)b * D + d0 + c) * 4) = *reinterpret_cast<const uint2*>(o4);
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------------------------ decoding state
+// log decay and pooled layer input of the tokens behind the last complete block: g_block [B,H], pool_sum [B,hidden]
+__global__ void __launch_bounds__(256)
+block_rest_kernel(const float* __restrict__ g, const bf16* __restrict__ x, float* __restrict__ g_block, float* __restrict__ pool,
+                  int T, int H, int hidden, int rest) {
+    const int i = blockIdx.x * 256 + threadIdx.x, b = blockIdx.y;
+    if (i < hidden) {
+        float s = 0.f;
+        for (int t = T - rest; t < T; ++t) s += bf(x, ((long)b * T + t) * hidden + i);
+        pool[(long)b * hidden + i] = s;
+    }
+    if (i < H) {
+        float s = 0.f;
+        for (int t = T - rest; t < T; ++t) s += g[((long)b * T + t) * H + i];
+        g_block[(long)b * H + i] = s;
+    }
+}
+
+// ------------------------------------------------------------------------------------------------ two streams
+// The linear branch runs on a side stream of high priority (one per device; events per thread), so that its CTAs are placed
+// ahead of the softmax branch's remaining ones whenever an SM frees up: the serial walk starts earlier and the attention CTAs
+// fill in around it (0.621 - 0.633 against 0.640 - 0.644 ms for the whole op at B = 8, T = 4096, H = 16).  The caller's stream
+// forks to it and joins again before the call returns, so every buffer may belong to the caller's stream alone.
+struct ThreadEvents {
+    cudaEvent_t ev[64][3] = {};
+    ~ThreadEvents() {
+        for (auto& e : ev)
+            for (auto& x : e)
+                if (x) cudaEventDestroy(x);
+    }
+};
+thread_local ThreadEvents t_events;
+
+int side_stream(cudaStream_t* side, cudaEvent_t** ev) {
+    static std::mutex mu;
+    static cudaStream_t streams[64] = {};
+    int dev = -1;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess && dev >= 0 && dev < 64) {
+        std::lock_guard<std::mutex> lock(mu);
+        int lo = 0, hi = 0;
+        if (!streams[dev]) {
+            e = cudaDeviceGetStreamPriorityRange(&lo, &hi);
+            if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&streams[dev], cudaStreamNonBlocking, hi < 0 ? -1 : 0);
+        }
+        *side = streams[dev];
+    } else if (e == cudaSuccess) {
+        e = cudaErrorInvalidDevice;
+    }
+    for (int i = 0; i < 3 && e == cudaSuccess; ++i)
+        if (!t_events.ev[dev][i]) e = cudaEventCreateWithFlags(&t_events.ev[dev][i], cudaEventDisableTiming);
+    if (e != cudaSuccess) {
+        set_error("cannot create the side stream: %s", cudaGetErrorString(e));
+        return NATSL_ERR_CUDA;
+    }
+    *ev = t_events.ev[dev];
+    return NATSL_OK;
+}
+
+int stream_after(cudaStream_t waiter, cudaStream_t done, cudaEvent_t ev) {
+    cudaError_t e = cudaEventRecord(ev, done);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(waiter, ev, 0);
+    if (e != cudaSuccess) {
+        set_error("cannot order two streams: %s", cudaGetErrorString(e));
+        return NATSL_ERR_CUDA;
+    }
+    return NATSL_OK;
+}
+
+long up256(long x) { return (x + 255) / 256 * 256; }
+
+struct HybridLayout {
+    long w, u, p, gcs, kr, qr, total;
+};
+HybridLayout hybrid_layout(const natsl_hybrid_args& a) {
+    HybridLayout l = {};
+    const long n = (long)a.B * a.T * a.H;
+    const bool gdn = a.rule == NATSL_RULE_GDN;
+    l.gcs = 0;
+    l.kr = up256(l.gcs + 4 * n);
+    l.qr = up256(l.kr + (gdn ? 4 * n : 0));
+    l.w = up256(l.qr + (gdn ? 4 * n : 0));
+    l.u = up256(l.w + (gdn ? 2 * n * a.K : 0));
+    l.p = up256(l.u + (gdn ? 2 * n * a.V : 0));
+    l.total = up256(l.p + (gdn ? 2 * n * 64 : 0));
+    return l;
+}
+
+int check_hybrid(const natsl_hybrid_args& a) {
+    NATSL_REQUIRE(a.q_attn && a.k_attn && a.v_attn && a.q && a.k && a.v && a.g && a.types && a.o_attn && a.lse && a.o_lin &&
+                      a.types_i && a.indices && a.n_blocks && a.n_chunks_lin && a.attn_n_iters && a.workspace &&
+                      (a.rule != NATSL_RULE_GDN || a.beta),
+                  NATSL_ERR_NULL, "natsl_hybrid_forward: null pointer");
+    NATSL_REQUIRE(a.B > 0 && a.T > 0 && a.H > 0 && a.HN > 0 && a.H % a.HN == 0 && a.HQ > 0 && a.HQ % a.HN == 0 && a.HKV > 0 &&
+                      a.HQ % a.HKV == 0 && a.nbs >= 64 && a.nbs % 64 == 0,
+                  NATSL_ERR_BAD_SHAPE, "natsl_hybrid_forward: bad shape");
+    NATSL_REQUIRE(a.rule == NATSL_RULE_GDN || (a.rule == NATSL_RULE_MAMBA && a.K == 128 && a.V == 64), NATSL_ERR_UNSUPPORTED,
+                  "natsl_hybrid_forward: Mamba2 is built for K = 128, V = 64 (got K=%d V=%d)", a.K, a.V);
+    NATSL_REQUIRE(a.workspace_bytes >= hybrid_layout(a).total, NATSL_ERR_TOO_LARGE, "natsl_hybrid_forward: workspace of %ld bytes, %ld needed",
+                  (long)a.workspace_bytes, hybrid_layout(a).total);
+    return NATSL_OK;
+}
+
+// Both branches.  types_dtype TBL_LOGITS: a.types are logits, types_raw receives the sampled types.  `before_attn` is launched
+// on the caller's stream beside the linear branch.
+template <typename F>
+int hybrid_forward(const natsl_hybrid_args& a, void* types_raw, cudaStream_t st, F before_attn) {
+    cudaStream_t side = st;
+    cudaEvent_t* ev = nullptr;
+    int rc = side_stream(&side, &ev);
+    if (rc != NATSL_OK) return rc;
+    const HybridLayout l = hybrid_layout(a);
+    unsigned char* ws = reinterpret_cast<unsigned char*>(a.workspace);
+    float* gcs = reinterpret_cast<float*>(ws + l.gcs);
+    const int TN = (a.T + a.nbs - 1) / a.nbs;
+    const bool gdn = a.rule == NATSL_RULE_GDN;
+    rc = stream_after(side, st, ev[0]);
+    // the preparation reads no tables: it starts while they are built
+    if (rc == NATSL_OK && gdn) {
+        auto prep = (a.K == 128 && a.V == 128 && !(a.options & NATSL_HYBRID_PREP_MMA)) ? natsl_gdn_chunk_prep_tc : natsl_gdn_chunk_prep_ex;
+        rc = prep(a.q, a.k, a.v, a.g, a.beta, a.beta_dtype, ws + l.w, ws + l.u, gcs, reinterpret_cast<float*>(ws + l.kr),
+                  reinterpret_cast<float*>(ws + l.qr), ws + l.p, a.B, a.T, a.H, a.K, a.V, a.use_l2norm, side);
+    } else if (rc == NATSL_OK && !a.gcs) {
+        rc = natsl_chunk_local_cumsum(a.g, gcs, a.B, a.T, a.H, side);
+    }
+    if (rc == NATSL_OK)
+        rc = launch_tables(a.types, a.types_dtype, types_raw, a.B, TN, a.HN, a.T, a.nbs, a.types_i, a.indices, a.n_blocks,
+                           a.n_chunks_lin, a.starting_h_idx, a.attn_n_iters, st);
+    if (rc == NATSL_OK) rc = stream_after(side, st, ev[1]);
+    const int flags = (a.decay ? NATSL_FLAG_DECAY_SKIPPED : 0);
+    const void* last = types_raw ? (const void*)(reinterpret_cast<bf16*>(types_raw) + (long)(TN - 1) * a.HN * 2) : a.last_types;
+    const int last_dtype = types_raw ? NATSL_DT_BF16 : a.last_dtype;
+    if (rc == NATSL_OK && gdn) {
+        auto walk = (a.K == 128 && a.V == 128 && a.nbs == 64 && a.T <= 65536 && !(a.options & NATSL_HYBRID_WALK_MMA))
+                        ? natsl_gdn_walk_fused_ex : natsl_gdn_walk;
+        rc = walk(a.q, a.k, ws + l.w, ws + l.u, ws + l.p, gcs, reinterpret_cast<float*>(ws + l.kr), reinterpret_cast<float*>(ws + l.qr),
+                  a.types_i, a.indices, a.n_blocks, a.h0, a.o_lin, a.ht, a.hstart, last, last_dtype, a.last_stride, a.B, a.T, a.H, a.HN,
+                  a.K, a.V, a.nbs, a.scale_lin, flags, side);
+    } else if (rc == NATSL_OK) {
+        rc = natsl_mamba_walk_fused_ex(a.q, a.k, a.v, a.gcs ? a.gcs : gcs, a.types_i, a.indices, a.n_blocks, a.h0, a.o_lin, a.ht,
+                                       a.hstart, last, last_dtype, a.last_stride, a.B, a.T, a.H, a.HN, a.K, a.V, a.nbs, a.scale_lin,
+                                       flags, side);
+    }
+    if (rc == NATSL_OK) rc = before_attn(st);
+    if (rc == NATSL_OK)
+        rc = natsl_attn_fwd_ex(a.q_attn, a.k_attn, a.v_attn, a.types_i, a.indices, a.attn_n_iters, a.o_attn, a.lse, a.B, a.T, a.T, 0,
+                               a.HQ, a.HKV, a.HN, a.DK, a.DV, a.nbs, a.scale_attn,
+                               (a.own_attn ? NATSL_FLAG_ATTN_OWN_CHUNK : 0) |
+                                   ((a.options & NATSL_HYBRID_ATTN_PERSISTENT) ? NATSL_FLAG_ATTN_PERSISTENT : 0), st);
+    const int join = stream_after(st, side, ev[2]);          // also after an error: the side stream may hold work of this call
+    return rc != NATSL_OK ? rc : join;
+}
+
+}  // namespace
+}  // namespace natsl
+
+extern "C" int64_t natsl_hybrid_workspace_bytes(const natsl_hybrid_args* args) {
+    using namespace natsl;
+    NATSL_REQUIRE(args, NATSL_ERR_NULL, "natsl_hybrid_workspace_bytes: null argument block");
+    return hybrid_layout(*args).total;
+}
+
+extern "C" int natsl_hybrid_forward(const natsl_hybrid_args* args, void* stream) {
+    using namespace natsl;
+    NATSL_REQUIRE(args, NATSL_ERR_NULL, "natsl_hybrid_forward: null argument block");
+    NATSL_REQUIRE(args->types_dtype >= 0 && args->types_dtype <= NATSL_DT_I32, NATSL_ERR_UNSUPPORTED, "natsl_hybrid_forward: bad types dtype");
+    const int rc = check_hybrid(*args);
+    if (rc != NATSL_OK) return rc;
+    return hybrid_forward(*args, nullptr, reinterpret_cast<cudaStream_t>(stream), [](cudaStream_t) { return (int)NATSL_OK; });
+}
+
+namespace natsl {
+namespace {
+
+struct LayerLayout {
+    long q, k, v, qa, ka, qc, vc, g, beta, dt, hybrid, total;
+};
+// Intermediates of a layer's forward.  Tensors the caller keeps (k_attn, v_attn) are outputs and not listed here.
+LayerLayout layer_layout(const natsl_layer_args& a, const natsl_hybrid_args& h) {
+    LayerLayout l = {};
+    const long n = (long)a.B * a.T, HK = (long)a.H * a.K, HV = (long)a.H * a.V;
+    const bool mamba = a.rule == NATSL_RULE_MAMBA;
+    long at = 0;
+    auto take = [&](long& slot, long bytes) { slot = at; at = up256(at + bytes); };
+    take(l.q, 2 * n * HK);
+    take(l.k, 2 * n * HK);
+    take(l.v, mamba ? 2 * n * HV : 0);
+    take(l.qa, a.qn_w || (mamba && a.attn_conv) ? 2 * n * HK : 0);
+    take(l.ka, 0);
+    take(l.qc, mamba ? 2 * n * HK : 0);
+    take(l.vc, 0);
+    take(l.g, 4 * n * a.H);
+    take(l.beta, mamba ? 0 : 2 * n * a.H);
+    take(l.dt, mamba ? 8 * n * a.H : 0);
+    take(l.hybrid, hybrid_layout(h).total);
+    l.total = at;
+    return l;
+}
+void hybrid_dims(const natsl_layer_args& a, natsl_hybrid_args& h) {
+    h.B = a.B; h.T = a.T; h.H = a.H; h.HN = a.HN; h.K = a.K; h.V = a.V; h.HQ = h.HKV = a.HQ;
+    h.DK = a.H * a.K / a.HQ; h.DV = a.H * a.V / a.HQ;
+    h.nbs = a.nbs; h.rule = a.rule; h.options = a.options;
+}
+
+}  // namespace
+}  // namespace natsl
+
+extern "C" int64_t natsl_layer_workspace_bytes(const natsl_layer_args* args) {
+    using namespace natsl;
+    NATSL_REQUIRE(args, NATSL_ERR_NULL, "natsl_layer_workspace_bytes: null argument block");
+    natsl_hybrid_args h = {};
+    hybrid_dims(*args, h);
+    return layer_layout(*args, h).total;
+}
+
+extern "C" int natsl_layer_forward(const natsl_layer_args* args, void* stream) {
+    using namespace natsl;
+    NATSL_REQUIRE(args, NATSL_ERR_NULL, "natsl_layer_forward: null argument block");
+    const natsl_layer_args& a = *args;
+    const bool mamba = a.rule == NATSL_RULE_MAMBA;
+    NATSL_REQUIRE(a.x && a.logits && a.q_raw && a.k_raw && a.v_raw && a.w_a && (mamba || a.w_b) && a.cw_q && a.cw_k && a.cw_v && a.A_log &&
+                      a.dt_bias && a.o_lin && a.o_attn && a.k_attn && a.v_attn && a.types_raw && a.tables && a.workspace && a.lse,
+                  NATSL_ERR_NULL, "natsl_layer_forward: null pointer");
+    NATSL_REQUIRE(a.B > 0 && a.T >= 4 && a.hidden % 32 == 0 && a.H > 0 && a.HQ > 0 && (a.H * a.K) % a.HQ == 0 && (a.H * a.V) % a.HQ == 0 &&
+                      (a.H * a.K) % 32 == 0 && a.B <= 65535,
+                  NATSL_ERR_BAD_SHAPE, "natsl_layer_forward: bad shape");
+    natsl_hybrid_args h = {};
+    hybrid_dims(a, h);
+    NATSL_REQUIRE(!a.qn_w || h.DK == 64 || h.DK == 128, NATSL_ERR_UNSUPPORTED, "natsl_layer_forward: norm width %d (64 or 128)", h.DK);
+    NATSL_REQUIRE(!mamba || a.K == 128, NATSL_ERR_UNSUPPORTED, "natsl_layer_forward: Mamba2 is built for K = 128");
+    const LayerLayout l = layer_layout(a, h);
+    NATSL_REQUIRE(a.workspace_bytes >= l.total, NATSL_ERR_TOO_LARGE, "natsl_layer_forward: workspace of %ld bytes, %ld needed",
+                  (long)a.workspace_bytes, l.total);
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    unsigned char* ws = reinterpret_cast<unsigned char*>(a.workspace);
+    auto cb = [](const void* p) { return reinterpret_cast<const bf16*>(p); };
+    auto mb = [](void* p) { return reinterpret_cast<bf16*>(p); };
+    const int HK = a.H * a.K, HV = a.H * a.V, TN = (a.T + a.nbs - 1) / a.nbs, NT = (a.T + 63) / 64;
+
+    NarrowArgs n = {};
+    n.x = cb(a.x); n.w0 = cb(a.w_a); n.w1 = mamba ? nullptr : cb(a.w_b);
+    n.n0 = a.H; n.n1 = mamba ? 0 : a.H; n.T = a.T; n.Kdim = a.hidden; n.mode = 0;
+    n.A_log = a.A_log; n.dt_bias = a.dt_bias; n.alog_f32 = a.alog_f32; n.dt_f32 = a.dt_f32; n.neg_eigval = a.neg_eigval;
+    n.g = reinterpret_cast<float*>(ws + l.g);
+    n.dt = mamba ? reinterpret_cast<float*>(ws + l.dt) : nullptr;
+    n.gcs = mamba ? n.dt + (long)a.B * a.T * a.H : nullptr;
+    n.out = mb(ws + l.beta);
+    int rc = launch_narrow(n, a.B, st);
+    if (rc != NATSL_OK) return rc;
+
+    // where each tensor of the two branches lives: the delta rule's k and v convolutions double as the softmax branch's
+    // tensors where nothing lies between them
+    const bool conv_attn = a.attn_conv, normed = a.qn_w != nullptr;
+    ConvArgs c = {};
+    c.dt = n.dt; c.T = a.T; c.H = a.H; c.silu = a.silu; c.l2_eps = a.l2_eps; c.norm_eps = a.norm_eps;
+    bf16 *q = mb(ws + l.q), *k = mb(ws + l.k), *v = mamba ? mb(ws + l.v) : mb(a.v_attn);
+    const bf16 *qa = nullptr, *q_mix = q;
+    c.seg[0] = {cb(a.q_raw), cb(a.cw_q), cb(a.cb_q), q, nullptr, nullptr, mb(a.tail_q), a.qn_w, a.qn_f32, HK, mamba ? 1 : 0, 0, a.K / 8, h.DK / 8, a.K, 0};
+    c.seg[1] = {cb(a.k_raw), cb(a.cw_k), cb(a.cb_k), k, nullptr, nullptr, mb(a.tail_k), a.kn_w, a.kn_f32, HK, mamba ? 1 : 0, 0, a.K / 8, h.DK / 8, a.K, 0};
+    c.seg[2] = {cb(a.v_raw), cb(a.cw_v), cb(a.cb_v), v, nullptr, nullptr, mb(a.tail_v), nullptr, 0, HV, mamba ? 2 : 0, 0, 1, 1, a.V, 0};
+    if (mamba) {
+        c.seg[0].conv = mb(ws + l.qc);                       // the mixing weights read the query in front of its l2 norm
+        q_mix = c.seg[0].conv;
+    }
+    if (normed) {
+        c.seg[0].attn = mb(ws + l.qa);
+        c.seg[1].attn = mb(a.k_attn);
+        c.seg[0].attn_mode = c.seg[1].attn_mode = conv_attn ? 1 : 2;
+        qa = c.seg[0].attn;
+    } else if (conv_attn) {
+        if (mamba) {
+            c.seg[1].conv = mb(a.k_attn);
+            qa = c.seg[0].conv;
+        } else {
+            k = mb(a.k_attn);
+            c.seg[1].lin = k;
+            qa = q;
+        }
+    } else {
+        qa = cb(a.q_raw);                                    // k_attn, v_attn are the raw projections (the caller passes them)
+    }
+    if (conv_attn && mamba) c.seg[2].conv = mb(a.v_attn);
+    if (!conv_attn && !mamba) {
+        v = mb(a.v_lin);
+        NATSL_REQUIRE(v, NATSL_ERR_NULL, "natsl_layer_forward: v_lin is needed beside a raw v_attn");
+        c.seg[2].lin = v;
+    }
+    const int kb = (HK + 255) / 256, vb = (HV + 255) / 256;
+    c.seg[1].blk0 = kb;
+    c.seg[2].blk0 = 2 * kb;
+    // tokens per warp: long runs amortise the three halo rows, short ones keep enough warps in flight (about 16 per SM)
+    const long rows = (long)a.B * a.T * (2 * kb + vb);
+    c.TT = rows / 64 >= 148 * 16 ? 64 : rows / 32 >= 148 * 16 ? 32 : rows / 16 >= 148 * 16 ? 16 : 8;
+    conv_norm_kernel<<<dim3(2 * kb + vb, (a.T + 4 * c.TT - 1) / (4 * c.TT), a.B), 128, 0, st>>>(c);
+    rc = check_launch("natsl_layer_forward (convolutions)");
+    if (rc != NATSL_OK) return rc;
+    if (a.g_block) {
+        const int rest = a.T % a.nbs;
+        const int width = a.hidden > a.H ? a.hidden : a.H;
+        block_rest_kernel<<<dim3((width + 255) / 256, a.B), 256, 0, st>>>(n.g, cb(a.x), reinterpret_cast<float*>(a.g_block),
+                                                                         reinterpret_cast<float*>(a.pool_sum), a.T, a.H, a.hidden, rest);
+        rc = check_launch("natsl_layer_forward (state)");
+        if (rc != NATSL_OK) return rc;
+    }
+
+    h.types_dtype = NATSL_DT_BF16;
+    h.beta_dtype = NATSL_DT_BF16;
+    h.own_attn = a.own_chunk; h.decay = a.decay; h.use_l2norm = mamba ? 0 : 1;
+    h.scale_attn = a.scale_attn; h.scale_lin = a.scale_lin;
+    h.q_attn = qa; h.k_attn = a.k_attn; h.v_attn = a.v_attn;
+    h.q = q; h.k = k; h.v = v; h.g = n.g; h.gcs = n.gcs; h.beta = n.out; h.types = a.logits;
+    h.o_attn = a.o_attn; h.lse = reinterpret_cast<float*>(a.lse); h.o_lin = a.o_lin;
+    h.ht = reinterpret_cast<float*>(a.ht); h.hstart = reinterpret_cast<float*>(a.hstart);
+    h.last_stride = TN * a.HN * 2;
+    int32_t* tb = reinterpret_cast<int32_t*>(a.tables);
+    const long nt = (long)a.B * TN * a.HN * 2;
+    h.types_i = tb; h.indices = tb + nt; h.n_blocks = tb + 2 * nt; h.n_chunks_lin = h.n_blocks + 2l * a.B * a.HN;
+    h.attn_n_iters = h.n_chunks_lin + (long)a.B * a.HN;
+    (void)NT;
+    h.workspace = ws + l.hybrid;
+    h.workspace_bytes = a.workspace_bytes - l.hybrid;
+    rc = check_hybrid(h);
+    if (rc != NATSL_OK) return rc;
+    h.types_dtype = TBL_LOGITS;
+    return hybrid_forward(h, a.types_raw, st, [&](cudaStream_t s) {
+        if (!a.w_mix) return (int)NATSL_OK;
+        NarrowArgs m = {};
+        m.x = q_mix; m.w0 = cb(a.w_mix); m.n0 = 2 * a.HQ; m.T = a.T; m.Kdim = HK; m.mode = 1; m.out = mb(a.mix);
+        return launch_narrow(m, a.B, s);
+    });
+}

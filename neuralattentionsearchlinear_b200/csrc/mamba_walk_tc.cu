@@ -71,7 +71,7 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                      const __grid_constant__ CUtensorMap map_v, const float* __restrict__ gcs,
                      const int* __restrict__ types_i, const int* __restrict__ indices, const int* __restrict__ n_blocks,
                      const float* __restrict__ h0, __nv_bfloat16* __restrict__ o, float* __restrict__ ht, float* hstart,
-                     const void* __restrict__ last_types, int last_f32, int T, int H, int HN, int TN, int nbs, float scale,
+                     const void* __restrict__ last_types, int last_f32, int last_stride, int T, int H, int HN, int TN, int nbs, float scale,
                      int decay, int trailing_quirk, int* status) {
     using L = MwSmem;
     constexpr int K = 128, V = 64;
@@ -423,7 +423,7 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         // block, decayed over it.
         bool last_lin = false, last_roll = false;
         if (hs_row && T % nbs == 0) {
-            const long li = ((long)b * HN + hn) * 2 + 1;
+            const long li = (long)b * last_stride + hn * 2 + 1;
             last_lin = (last_f32 ? reinterpret_cast<const float*>(last_types)[li]
                                  : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(last_types)[li])) > 0.f;
             last_roll = !last_lin && decay;
@@ -596,7 +596,7 @@ extern "C" int natsl_mw_timing(long long* out, int reset) {
 extern "C" int natsl_mamba_walk_fused_ex(const void* q, const void* k, const void* v, const float* gcs,
                                       const int32_t* types_i, const int32_t* indices, const int32_t* n_blocks,
                                       const float* h0, void* o, float* ht, float* hstart, const void* last_types,
-                                      int last_dtype, int B, int T, int H, int HN, int K, int V, int nbs, float scale, int flags,
+                                      int last_dtype, int last_stride, int B, int T, int H, int HN, int K, int V, int nbs, float scale, int flags,
                                       void* stream) {
     using namespace natsl;
     NATSL_REQUIRE(k && v && gcs && types_i && indices && n_blocks, NATSL_ERR_NULL, "natsl_mamba_walk_fused: null pointer");
@@ -628,7 +628,7 @@ extern "C" int natsl_mamba_walk_fused_ex(const void* q, const void* k, const voi
     dim3 grid(H, B);
     kern<<<grid, MW_THREADS, MwSmem::total, reinterpret_cast<cudaStream_t>(stream)>>>(
         mq, mk, mv, gcs, types_i, indices, n_blocks, h0, reinterpret_cast<__nv_bfloat16*>(o), ht, hstart, last_types,
-        last_dtype == NATSL_DT_F32, T, H, HN, TN, nbs, scale,
+        last_dtype == NATSL_DT_F32, last_stride, T, H, HN, TN, nbs, scale,
         (flags & NATSL_FLAG_DECAY_SKIPPED) ? 1 : 0, (flags & NATSL_FLAG_NO_TRAILING_QUIRK) ? 0 : 1, status);
     return check_launch("natsl_mamba_walk_fused");
 }
@@ -637,6 +637,6 @@ extern "C" int natsl_mamba_walk_fused(const void* q, const void* k, const void* 
                                       const int32_t* types_i, const int32_t* indices, const int32_t* n_blocks,
                                       const float* h0, void* o, float* ht, int B, int T, int H, int HN, int K, int V,
                                       int nbs, float scale, int flags, void* stream) {
-    return natsl_mamba_walk_fused_ex(q, k, v, gcs, types_i, indices, n_blocks, h0, o, ht, nullptr, nullptr, 0, B, T, H, HN, K, V,
+    return natsl_mamba_walk_fused_ex(q, k, v, gcs, types_i, indices, n_blocks, h0, o, ht, nullptr, nullptr, 0, 0, B, T, H, HN, K, V,
                                      nbs, scale, flags, stream);
 }

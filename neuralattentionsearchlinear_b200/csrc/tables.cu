@@ -11,11 +11,13 @@
 // head) compacts the selected block ids with a block-wide prefix sum; the "sort" of
 // the reference is that compaction (selected ids are already ascending).
 #include "common.cuh"
+#include "layer_fwd.cuh"
 #include "../../include/natsl_b200.h"
 
 namespace natsl {
 
 constexpr int TBL_THREADS = 256;
+constexpr int TBL_MAX_TN = 4096;           // blocks whose prefix counts fit the shared table (longer sequences search)
 
 __device__ __forceinline__ float load_type(const void* p, int dtype, long i) {
     switch (dtype) {
@@ -36,10 +38,19 @@ __device__ __forceinline__ int count_below(const int* idx, long stride, int n, i
     return lo;
 }
 
+// The hard softmax of two bf16 logits as torch computes it on the device (softmax rounded to bf16, first maximum): 0 or 1.
+__device__ __forceinline__ int pick_logit(float l0, float l1) {
+    const float mx = fmaxf(l0, l1), e0 = expf(l0 - mx), e1 = expf(l1 - mx), s = e0 + e1;
+    return __bfloat162float(__float2bfloat16(e1 / s)) > __bfloat162float(__float2bfloat16(e0 / s)) ? 1 : 0;
+}
+
+// dtype TBL_LOGITS: `types` holds the selection logits (bf16); the type of a block is their hard softmax, written to
+// types_raw (bf16 0/1), and the last block takes both columns (src/nats/layers/natsl_attn_gdn.py:47-61, 420, 553).
 __global__ void __launch_bounds__(TBL_THREADS)
-tables_kernel(const void* __restrict__ types, int dtype, int B, int TN, int HN, int T, int nbs, int attn_bt,
-              int* __restrict__ types_i, int* __restrict__ indices, int* __restrict__ n_blocks,
+tables_kernel(const void* __restrict__ types, int dtype, __nv_bfloat16* __restrict__ types_raw, int B, int TN, int HN, int T,
+              int nbs, int attn_bt, int* __restrict__ types_i, int* __restrict__ indices, int* __restrict__ n_blocks,
               int* __restrict__ n_chunks_lin, int* __restrict__ starting_h_idx, int* __restrict__ attn_n_iters) {
+    __shared__ int s_cnt[2][TBL_MAX_TN + 1];               // selected blocks before block j
     __shared__ int warp_tot[TBL_THREADS / 32];
     __shared__ int s_n[2];
     const int bh = blockIdx.x, b = bh / HN, hn = bh % HN;
@@ -52,7 +63,15 @@ tables_kernel(const void* __restrict__ types, int dtype, int B, int TN, int HN, 
             int i = i0 + tid;
             int flag = 0;
             if (i < TN) {
-                flag = (rintf(load_type(types, dtype, base + (long)i * stride)) == 1.0f) ? 1 : 0;
+                if (dtype == TBL_LOGITS) {
+                    const uint32_t l = reinterpret_cast<const uint32_t*>(types)[((long)b * TN + i) * HN + hn];
+                    const float2 f = unpack_bf16(l);
+                    const int raw = pick_logit(f.x, f.y) == op;
+                    types_raw[base + (long)i * stride] = __float2bfloat16((float)raw);
+                    flag = raw | (i == TN - 1);
+                } else {
+                    flag = (rintf(load_type(types, dtype, base + (long)i * stride)) == 1.0f) ? 1 : 0;
+                }
                 types_i[base + (long)i * stride] = flag;
             }
             unsigned bal = __ballot_sync(0xffffffffu, flag);
@@ -67,9 +86,11 @@ tables_kernel(const void* __restrict__ types, int dtype, int B, int TN, int HN, 
                 tot += v;
             }
             if (flag) indices[base + (long)(running + off + excl) * stride] = i;
+            if (i <= TN && i <= TBL_MAX_TN) s_cnt[op][i] = running + off + excl;
             running += tot;
             __syncthreads();
         }
+        if (tid == 0 && TN <= TBL_MAX_TN) s_cnt[op][TN] = running;
         for (int j = running + tid; j < TN; j += TBL_THREADS) indices[base + (long)j * stride] = TN;
         if (tid == 0) {
             n_blocks[(long)bh * 2 + op] = running;
@@ -80,17 +101,18 @@ tables_kernel(const void* __restrict__ types, int dtype, int B, int TN, int HN, 
     __syncthreads();   // indices written by this CTA are visible to it from here on
     const int NT = (T + NATSL_CHUNK - 1) / NATSL_CHUNK;
     const int* lin = indices + ((long)b * TN * HN + hn) * 2 + 1;
-    for (int i = tid; i < NT; i += TBL_THREADS) {
+    const bool table = TN <= TBL_MAX_TN;
+    for (int i = tid; i < NT && starting_h_idx; i += TBL_THREADS) {
         // #selected linear blocks with idx*nbs < i*64  <=>  idx < ceil(i*64 / nbs)
         int x = (i * NATSL_CHUNK + nbs - 1) / nbs;
-        starting_h_idx[((long)b * NT + i) * HN + hn] = count_below(lin, stride, s_n[1], x);
+        starting_h_idx[((long)b * NT + i) * HN + hn] = table ? s_cnt[1][min(x, TN)] : count_below(lin, stride, s_n[1], x);
     }
     const int NTq = (T + attn_bt - 1) / attn_bt;
     const int* att = indices + ((long)b * TN * HN + hn) * 2;
     for (int i = tid; i < NTq; i += TBL_THREADS) {
         // #selected attention blocks with (idx+1)*nbs <= i*attn_bt  <=>  idx < floor(i*attn_bt / nbs)
         int x = (i * attn_bt) / nbs;
-        attn_n_iters[((long)b * NTq + i) * HN + hn] = count_below(att, stride, s_n[0], x);
+        attn_n_iters[((long)b * NTq + i) * HN + hn] = table ? s_cnt[0][min(x, TN)] : count_below(att, stride, s_n[0], x);
     }
 }
 
@@ -135,6 +157,14 @@ __global__ void chunk_indices_kernel(const int* __restrict__ offsets, int* __res
     }
 }
 
+int launch_tables(const void* types, int dtype, void* types_raw, int B, int TN, int HN, int T, int nbs, int* types_i, int* indices,
+                  int* n_blocks, int* n_chunks_lin, int* starting_h_idx, int* attn_n_iters, cudaStream_t st) {
+    tables_kernel<<<B * HN, TBL_THREADS, 0, st>>>(types, dtype, reinterpret_cast<__nv_bfloat16*>(types_raw), B, TN, HN, T, nbs,
+                                                  NATSL_ATTN_BT, types_i, indices, n_blocks, n_chunks_lin, starting_h_idx,
+                                                  attn_n_iters);
+    return check_launch("selection tables");
+}
+
 }  // namespace natsl
 
 extern "C" int natsl_build_tables(const void* types, int types_dtype, int B, int TN, int HN, int T, int nbs,
@@ -152,7 +182,7 @@ extern "C" int natsl_build_tables(const void* types, int types_dtype, int B, int
     NATSL_REQUIRE(attn_bt > 0 && types_dtype >= 0 && types_dtype <= NATSL_DT_I32, NATSL_ERR_UNSUPPORTED,
                   "natsl_build_tables: bad attn_bt/dtype");
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    tables_kernel<<<B * HN, TBL_THREADS, 0, st>>>(types, types_dtype, B, TN, HN, T, nbs, attn_bt, types_i, indices,
+    tables_kernel<<<B * HN, TBL_THREADS, 0, st>>>(types, types_dtype, nullptr, B, TN, HN, T, nbs, attn_bt, types_i, indices,
                                                   n_blocks, n_chunks_lin, starting_h_idx, attn_n_iters);
     offsets_kernel<<<1, TBL_THREADS, 0, st>>>(n_chunks_lin, B * HN, offsets);
     if (chunk_indices) chunk_indices_kernel<<<B * HN, 128, 0, st>>>(offsets, chunk_indices);

@@ -94,8 +94,12 @@ class _Plan:
         a.silu = int(m.q_conv1d.activation in ("silu", "swish"))
         a.mix_sigmoid, a.mix_eps = int(m.o_norm.activation == "sigmoid"), m.o_norm.eps
         a.scale_attn, a.scale_lin = DK ** -0.5, m.head_k_dim ** -0.5 if gdn else 1.0
-        self.options = ()
         self.ws_bytes = {}
+        b = self.layer_args = _lib.LayerArgs()
+        for n in ("hidden H K V HQ HN nbs rule silu qn_f32 kn_f32 alog_f32 dt_f32 norm_eps l2_eps scale_attn scale_lin w_a w_b "
+                  "w_mix cw_q cw_k cw_v cb_q cb_k cb_v qn_w kn_w A_log dt_bias").split():
+            setattr(b, n, getattr(a, n))
+        self.layer_ws = {}
 
     def current(self) -> bool:
         for d, n, m in self.mods:
@@ -112,7 +116,8 @@ class _Plan:
         return True
 
 
-def _plan(layer):
+def layer_plan(layer) -> _Plan:
+    """This thread's plan of the layer, rebuilt when a module, a parameter or its storage has changed."""
     plans = getattr(_tls, "plans", None)
     if plans is None:
         plans = _tls.plans = weakref.WeakKeyDictionary()
@@ -133,7 +138,7 @@ def decode_token(layer, x: torch.Tensor, container):
             or layer.ops_for_incomplete_chunks == 'attn' or not layer.incomplete_block_start_with_ht
             or not (layer.use_short_conv and layer.use_gate) or torch.is_autocast_enabled() or not hasattr(container, "layer")):
         return None
-    plan = _plan(layer)
+    plan = layer_plan(layer)
     if not plan.ok or torch.nn.modules.module._has_any_global_hook():
         return None
     a = plan.args

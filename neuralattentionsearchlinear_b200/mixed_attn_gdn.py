@@ -91,8 +91,16 @@ def reference_compat_bwd(enabled: bool = True):
         REFERENCE_COMPAT_BWD = old
 
 
-def _zeros_like_or_none(t):
-    return None if t is None else torch.zeros_like(t)
+class NoGrad:
+    """Stands in for an autograd context where no input needs a gradient (saves ``Function.apply``'s bookkeeping)."""
+
+    @staticmethod
+    def save_for_backward(*tensors):
+        pass
+
+
+def wants_grad(*tensors) -> bool:
+    return torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in tensors)
 
 
 def hybrid_backward(ctx, rule, do_lin, do_attn, dht):
@@ -101,7 +109,7 @@ def hybrid_backward(ctx, rule, do_lin, do_attn, dht):
     if not ctx.bwd_ok:
         raise NotImplementedError(ctx.bwd_why)
     q_attn, k_attn, v_attn, o_attn, lse, q, k, v, g, beta, h0 = ctx.saved_tensors
-    tables = ctx.tables
+    tables = ctx.tables if ctx.tables is not None else _ops.tables_from_flat(*ctx.flat_tables)
     if do_attn is None:
         do_attn = torch.zeros_like(o_attn)
     if do_lin is None:
@@ -115,6 +123,21 @@ def hybrid_backward(ctx, rule, do_lin, do_attn, dht):
     dbeta = None if r['dbeta'] is None else r['dbeta'].to(beta.dtype)
     dh0 = None if (h0 is None or r['dh0'] is None) else r['dh0'].to(h0.dtype)
     return dqa, dka, dva, r['dq'], r['dk'], r['dv'], dh0, dg, dbeta, dnats
+
+
+def save_hybrid(ctx, tensors, flat, types, T, nbs, scale_attn, scale_lattn, own_attn, decay, use_l2norm, invalid_dnats):
+    """What ``hybrid_backward`` needs from a forward of ``_ops.hybrid_fwd``."""
+    K, V = tensors[5].shape[-1], tensors[7].shape[-1]
+    if nbs != CHUNK_SIZE:
+        ctx.bwd_ok, ctx.bwd_why = False, "the backward pass is built for nats_block_size = 64"
+    elif K not in (64, 128) or V not in (64, 128):
+        ctx.bwd_ok, ctx.bwd_why = False, "the backward pass is built for linear-branch head dims 64 and 128"
+    ctx.save_for_backward(*tensors)
+    ctx.tables, ctx.flat_tables = None, (flat, types.shape[0], types.shape[1], types.shape[2], T, nbs)
+    ctx.scale_attn, ctx.scale_lattn, ctx.own_attn = float(scale_attn), float(scale_lattn), own_attn
+    ctx.decay, ctx.use_l2norm, ctx.invalid_dnats_linear = bool(decay), bool(use_l2norm), bool(invalid_dnats)
+    ctx.compat = REFERENCE_COMPAT_BWD
+    ctx.types_dtype = types.dtype
 
 
 class NAtSMixedAttentionGDN(torch.autograd.Function):
@@ -146,6 +169,16 @@ class NAtSMixedAttentionGDN(torch.autograd.Function):
                                                  lattn_use_qk_l2norm_in_kernel)
             ctx.bwd_ok, ctx.bwd_why = False, "the backward pass is built for bf16 tensors (fp32 tensors run forward only)"
             return o_gdn, o_attn, (ht if output_final_state_gated_delta else None)
+        if own_linear and _ops.walks_with_state(_lib.RULE_GDN, q_lattn.shape[-1], v_lattn.shape[-1], T):
+            # both branches and the tables in one native call, the linear branch on a stream of its own
+            o_gdn, o_attn, lse, ht, _, flat = _ops.hybrid_fwd(
+                _lib.RULE_GDN, q_attn, k_attn, v_attn, q_lattn, k_lattn, v_lattn, g, beta, nats_block_types, nats_block_size,
+                scale_attn, scale_lattn, initial_state_gated_delta, strategy['attn'], decay_for_non_gdn_blocks,
+                lattn_use_qk_l2norm_in_kernel, output_final_state_gated_delta)
+            save_hybrid(ctx, (q_attn, k_attn, v_attn, o_attn, lse, q_lattn, k_lattn, v_lattn, g, beta, initial_state_gated_delta),
+                        flat, nats_block_types, T, nats_block_size, scale_attn, scale_lattn, strategy['attn'],
+                        decay_for_non_gdn_blocks, lattn_use_qk_l2norm_in_kernel, compute_dnats_for_invalid_blocks_linear_att)
+            return o_gdn, o_attn, ht
         # The two branches are independent: the softmax branch runs on a side stream (as the reference does for
         # its Mamba2 / DeltaNet ops, src/nats/ops/mixed_ops/mixed_attn_mamba.py:114-124) and joins before returning.
         # The selection tables are built on the side stream too: the chunk preparation of the linear branch does not
@@ -238,13 +271,15 @@ def nats_mixed_attn_gdn(
         scale_attn = k_attn.shape[-1] ** -0.5
     if scale_lattn is None:
         scale_lattn = k_lattn.shape[-1] ** -0.5
-    return NAtSMixedAttentionGDN.apply(
-        q_attn, k_attn, v_attn, q_lattn, k_lattn, v_lattn, initial_state_gated_delta, g, beta,
-        nats_block_types, n_nats_blocks, scale_attn, scale_lattn, cu_seqlens, cu_seqlens_nats,
-        nats_block_size, attn_sw_size, ops_for_incomplete_chunks, output_final_state_gated_delta,
-        compute_dnats_for_invalid_blocks_attn, compute_dnats_for_invalid_blocks_linear_att,
-        decay_for_non_gdn_blocks, incomplete_block_start_with_ht, use_g_for_attn,
-        lattn_use_qk_l2norm_in_kernel)
+    args = (q_attn, k_attn, v_attn, q_lattn, k_lattn, v_lattn, initial_state_gated_delta, g, beta,
+            nats_block_types, n_nats_blocks, scale_attn, scale_lattn, cu_seqlens, cu_seqlens_nats,
+            nats_block_size, attn_sw_size, ops_for_incomplete_chunks, output_final_state_gated_delta,
+            compute_dnats_for_invalid_blocks_attn, compute_dnats_for_invalid_blocks_linear_att,
+            decay_for_non_gdn_blocks, incomplete_block_start_with_ht, use_g_for_attn,
+            lattn_use_qk_l2norm_in_kernel)
+    if not wants_grad(*args[:10]):
+        return NAtSMixedAttentionGDN.forward(NoGrad(), *args)
+    return NAtSMixedAttentionGDN.apply(*args)
 
 
 def _chunk_start_state(inter, ht, gcs, tables, op_type_last_chunk, T, nbs, decay):
@@ -304,17 +339,17 @@ def nats_mixed_attn_gdn_chunk_inference(
     if scale_lattn is None:
         scale_lattn = k_lattn.shape[-1] ** -0.5
     T = q_lattn.shape[1]
+    want = bool(output_final_state_gated_delta)
     with torch.no_grad():
-        tables = build_selection_tables(nats_block_types, T, nats_block_size)
-        o_attn, _ = _ops.attn_fwd(q_attn, k_attn, v_attn, tables, scale_attn, own_chunk=strategy['attn'])
-        want = bool(output_final_state_gated_delta)
         if _ops.walks_with_state(_lib.RULE_GDN, q_lattn.shape[-1], v_lattn.shape[-1], T):
             assert not want or T % nats_block_size or op_type_last_chunk is not None
-            o_gdn, ht, inter = _ops.linear_fwd(_lib.RULE_GDN, q_lattn, k_lattn, v_lattn, g, beta, tables, scale_lattn,
-                                               initial_state_gated_delta_chunk_start, decay_for_non_gdn_blocks,
-                                               lattn_use_qk_l2norm_in_kernel, want, want_start=want,
-                                               last_types=op_type_last_chunk)
-            return o_gdn, o_attn, ht, (inter['start'] if want else None)
+            o_gdn, o_attn, _, ht, start, _ = _ops.hybrid_fwd(
+                _lib.RULE_GDN, q_attn, k_attn, v_attn, q_lattn, k_lattn, v_lattn, g, beta, nats_block_types, nats_block_size,
+                scale_attn, scale_lattn, initial_state_gated_delta_chunk_start, strategy['attn'], decay_for_non_gdn_blocks,
+                lattn_use_qk_l2norm_in_kernel, want, want, op_type_last_chunk)
+            return o_gdn, o_attn, ht, start
+        tables = build_selection_tables(nats_block_types, T, nats_block_size)
+        o_attn, _ = _ops.attn_fwd(q_attn, k_attn, v_attn, tables, scale_attn, own_chunk=strategy['attn'])
         o_gdn, ht, inter = _ops.linear_fwd(_lib.RULE_GDN, q_lattn, k_lattn, v_lattn, g, beta, tables, scale_lattn,
                                            initial_state_gated_delta_chunk_start, decay_for_non_gdn_blocks,
                                            lattn_use_qk_l2norm_in_kernel, True, return_intermediates=True)

@@ -36,6 +36,17 @@ class NAtSMixedAttentionMamba(torch.autograd.Function):
         if own_linear and not incomplete_block_start_with_ht:
             raise NotImplementedError("incomplete_block_start_with_ht=False is not built")
         T = q_lattn.shape[1]
+        if (own_linear and q_lattn.dtype != torch.float32
+                and _ops.walks_with_state(_lib.RULE_MAMBA, q_lattn.shape[-1], v_lattn.shape[-1], T)):
+            ctx.bwd_ok, ctx.bwd_why = True, ""
+            o_m, o_attn, lse, ht, _, flat = _ops.hybrid_fwd(
+                _lib.RULE_MAMBA, q_attn, k_attn, v_attn, q_lattn, k_lattn, v_lattn, g, None, nats_block_types, nats_block_size,
+                scale_attn, scale_lattn, initial_state_mamba, strategy['attn'], decay_for_non_mamba_blocks, False,
+                output_final_state_mamba)
+            gdn_ops.save_hybrid(ctx, (q_attn, k_attn, v_attn, o_attn, lse, q_lattn, k_lattn, v_lattn, g, None, initial_state_mamba),
+                                flat, nats_block_types, T, nats_block_size, scale_attn, scale_lattn, strategy['attn'],
+                                decay_for_non_mamba_blocks, False, compute_dnats_for_invalid_blocks_linear_att)
+            return o_m, o_attn, ht
         tables = build_selection_tables(nats_block_types, T, nats_block_size)
         lin_tables = tables if own_linear else per_chunk_tables(nats_block_types, T, nats_block_size)
         ctx.bwd_ok, ctx.bwd_why = True, ""
@@ -95,11 +106,13 @@ def nats_mixed_attn_mamba(
         scale_attn = k_attn.shape[-1] ** -0.5
     if scale_lattn is None:
         scale_lattn = 1                                                     # mixed_attn_mamba.py:318-319
-    return NAtSMixedAttentionMamba.apply(
-        q_attn, k_attn, v_attn, q_lattn, k_lattn, v_lattn, initial_state_mamba, g, nats_block_types, n_nats_blocks,
-        scale_attn, scale_lattn, cu_seqlens, cu_seqlens_nats, nats_block_size, attn_sw_size, ops_for_incomplete_chunks,
-        output_final_state_mamba, compute_dnats_for_invalid_blocks_attn, compute_dnats_for_invalid_blocks_linear_att,
-        decay_for_non_mamba_blocks, incomplete_block_start_with_ht, use_g_for_attn)
+    args = (q_attn, k_attn, v_attn, q_lattn, k_lattn, v_lattn, initial_state_mamba, g, nats_block_types, n_nats_blocks,
+            scale_attn, scale_lattn, cu_seqlens, cu_seqlens_nats, nats_block_size, attn_sw_size, ops_for_incomplete_chunks,
+            output_final_state_mamba, compute_dnats_for_invalid_blocks_attn, compute_dnats_for_invalid_blocks_linear_att,
+            decay_for_non_mamba_blocks, incomplete_block_start_with_ht, use_g_for_attn)
+    if not gdn_ops.wants_grad(*args[:9]):
+        return NAtSMixedAttentionMamba.forward(gdn_ops.NoGrad(), *args)
+    return NAtSMixedAttentionMamba.apply(*args)
 
 
 def nats_mixed_attn_mamba_chunk_inference(
@@ -132,16 +145,17 @@ def nats_mixed_attn_mamba_chunk_inference(
     if scale_lattn is None:
         scale_lattn = k_lattn.shape[-1] ** -0.5                             # mixed_attn_mamba.py:389-390
     T = q_lattn.shape[1]
+    want = bool(output_final_state_mamba)
     with torch.no_grad():
-        tables = build_selection_tables(nats_block_types, T, nats_block_size)
-        o_attn, _ = _ops.attn_fwd(q_attn, k_attn, v_attn, tables, scale_attn, own_chunk=strategy['attn'])
-        want = bool(output_final_state_mamba)
         if _ops.walks_with_state(_lib.RULE_MAMBA, q_lattn.shape[-1], v_lattn.shape[-1], T):
             assert not want or T % nats_block_size or op_type_last_chunk is not None
-            o_m, ht, inter = _ops.linear_fwd(_lib.RULE_MAMBA, q_lattn, k_lattn, v_lattn, g, None, tables, scale_lattn,
-                                             initial_state_mamba_start, decay_for_non_mamba_blocks, False, want,
-                                             want_start=want, last_types=op_type_last_chunk)
-            return o_m, o_attn, ht, (inter['start'] if want else None)
+            o_m, o_attn, _, ht, start, _ = _ops.hybrid_fwd(
+                _lib.RULE_MAMBA, q_attn, k_attn, v_attn, q_lattn, k_lattn, v_lattn, g, None, nats_block_types, nats_block_size,
+                scale_attn, scale_lattn, initial_state_mamba_start, strategy['attn'], decay_for_non_mamba_blocks, False, want, want,
+                op_type_last_chunk)
+            return o_m, o_attn, ht, start
+        tables = build_selection_tables(nats_block_types, T, nats_block_size)
+        o_attn, _ = _ops.attn_fwd(q_attn, k_attn, v_attn, tables, scale_attn, own_chunk=strategy['attn'])
         o_m, ht, inter = _ops.linear_fwd(_lib.RULE_MAMBA, q_lattn, k_lattn, v_lattn, g, None, tables, scale_lattn,
                                          initial_state_mamba_start, decay_for_non_mamba_blocks, False, True,
                                          return_intermediates=True)

@@ -19,6 +19,7 @@ import torch.nn.functional as F
 from .mixed_attn_gdn import nats_mixed_attn_gdn, nats_mixed_attn_gdn_chunk_inference, nats_mixed_attn_gdn_recurrent
 from .decode_step import decode_token
 from .decoding import forward_cached
+from .layer_forward import layer_forward
 from .modules import FusedMultiInputRMSNormGated, RMSNorm, ShortConvolution, hard_softmax, mean_pooling
 
 
@@ -151,9 +152,22 @@ class NeuralAttentionSearchLinearAttnGDN(nn.Module):
         else:
             self.o_norm = nn.ModuleList([RMSNorm(self.head_v_dim, eps=norm_eps), RMSNorm(self.head_attn_v_dim, eps=norm_eps)])
         self.o_proj = nn.Linear(self.value_dim, hidden_size, bias=False)
+        self.attn_blocks = None            # (block counts [B, HN, 2], blocks) of the last forward, behind attn_fraction
         self.attn_fraction = torch.zeros(1)
 
     # ------------------------------------------------------------------------------------------------
+    @property
+    def attn_fraction(self) -> torch.Tensor:
+        """Share of the blocks of the last forward that took the softmax branch, per selection head."""
+        if self.attn_blocks is not None:
+            counts, n = self.attn_blocks
+            self.attn_fraction = (counts[..., 0].float() / n).mean(0)
+        return self._attn_fraction
+
+    @attn_fraction.setter
+    def attn_fraction(self, value: torch.Tensor) -> None:
+        self._attn_fraction, self.attn_blocks = value, None
+
     def select(self, pooled: torch.Tensor) -> torch.Tensor:
         """Block-mean layer input [B, NB, D] -> sampled 0/1 block types [B, NB, HN, n_ops] (natsl_attn_gdn.py:411-420)."""
         logits = self.nats_layer(pooled).unflatten(-1, (self.num_nats_head, self.n_ops))
@@ -250,6 +264,10 @@ class NeuralAttentionSearchLinearAttnGDN(nn.Module):
             return self._forward_cached(hidden_states, past_key_values)
         if T < 64 or self.mode != 'chunk':
             raise NotImplementedError("fewer than 64 tokens (decoding) need a NAtSCache in past_key_values")
+        if not self.training and type(self) is NeuralAttentionSearchLinearAttnGDN and not torch.is_grad_enabled():
+            y = layer_forward(self, hidden_states)
+            if y is not None:
+                return y, None, past_key_values
         p = self.project(hidden_states)
         common = dict(scale_attn=p['k_attn'].shape[-1] ** -0.5, scale_lattn=p['k'].shape[-1] ** -0.5,
                       cu_seqlens=None, cu_seqlens_nats=None, nats_block_size=self.nats_block_size,
@@ -302,6 +320,11 @@ class NeuralAttentionSearchLinearAttnGDN(nn.Module):
         (token recurrence with re-roll + masked attention over the cached keys), natsl_attn_gdn.py:389-410, 576-650."""
         if hidden_states.shape[1] == 1 and type(self) is NeuralAttentionSearchLinearAttnGDN:
             y = decode_token(self, hidden_states, past_key_values)
+            if y is not None:
+                return y, None, past_key_values
+        elif self.layer_idx is not None and type(self) is NeuralAttentionSearchLinearAttnGDN:
+            cache = past_key_values.layer(self.layer_idx, self.nats_block_size)
+            y = layer_forward(self, hidden_states, cache) if cache.n_tokens == 0 else None
             if y is not None:
                 return y, None, past_key_values
         o_gd, o_attn, o_w = forward_cached(self, hidden_states, past_key_values)

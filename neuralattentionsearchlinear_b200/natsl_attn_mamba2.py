@@ -17,6 +17,7 @@ import torch.nn.functional as F
 
 from .decode_step import decode_token
 from .decoding import forward_cached
+from .layer_forward import layer_forward
 from .mixed_attn_mamba import (nats_mixed_attn_mamba, nats_mixed_attn_mamba_chunk_inference,
                                nats_mixed_attn_mamba_recurrent)
 from .modules import FusedMultiInputRMSNormGated, L2Norm, RMSNorm, ShortConvolution, hard_softmax, mean_pooling
@@ -128,7 +129,20 @@ class NeuralAttentionSearchLinearAttnMamba(nn.Module):
         else:
             raise NotImplementedError("use_gate=False is not built for the Mamba2 layer")
         self.o_proj = nn.Linear(self.value_dim, hidden_size, bias=False)
+        self.attn_blocks = None            # (block counts [B, HN, 2], blocks) of the last forward, behind attn_fraction
         self.attn_fraction = torch.zeros(1)
+
+    @property
+    def attn_fraction(self) -> torch.Tensor:
+        """Share of the blocks of the last forward that took the softmax branch, per selection head."""
+        if self.attn_blocks is not None:
+            counts, n = self.attn_blocks
+            self.attn_fraction = (counts[..., 0].float() / n).mean(0)
+        return self._attn_fraction
+
+    @attn_fraction.setter
+    def attn_fraction(self, value: torch.Tensor) -> None:
+        self._attn_fraction, self.attn_blocks = value, None
 
     def select(self, pooled: torch.Tensor) -> torch.Tensor:
         """Block-mean layer input [B, NB, D] -> sampled 0/1 block types [B, NB, HN, n_ops] (natsl_attn_mamba2.py:352-365)."""
@@ -241,11 +255,20 @@ class NeuralAttentionSearchLinearAttnMamba(nn.Module):
                 y = decode_token(self, hidden_states, cache_params)
                 if y is not None:
                     return y
+            elif self.layer_idx is not None and type(self) is NeuralAttentionSearchLinearAttnMamba:
+                cache = cache_params.layer(self.layer_idx, self.nats_block_size)
+                y = layer_forward(self, hidden_states, cache) if cache.n_tokens == 0 else None
+                if y is not None:
+                    return y
             o_m, o_attn, o_w = forward_cached(self, hidden_states, cache_params)
             with torch.no_grad():
                 return self.mix(hidden_states, o_m, o_attn, o_w)
         if T < 64 or self.mode != 'chunk':
             raise NotImplementedError("fewer than 64 tokens (decoding) need a NAtSCache in cache_params")
+        if not self.training and type(self) is NeuralAttentionSearchLinearAttnMamba and not torch.is_grad_enabled():
+            y = layer_forward(self, hidden_states)
+            if y is not None:
+                return y
         p = self.project(hidden_states)
         common = dict(scale_attn=p['k_attn'].shape[-1] ** -0.5, scale_lattn=1, cu_seqlens=None, cu_seqlens_nats=None,
                       nats_block_size=self.nats_block_size, ops_for_incomplete_chunks=self.ops_for_incomplete_chunks,
