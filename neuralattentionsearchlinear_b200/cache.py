@@ -30,7 +30,7 @@ class NAtSLayerCache:
         self._v_buf: Optional[torch.Tensor] = None      # [B, capacity, HKV, DV]
         self._n_kv = 0                                  # rows of the buffers in use
         self._kv_shared = False                         # another cache reads the same buffers
-        self._workspace: Optional[torch.Tensor] = None  # intermediates of a single-token step
+        self._step = None                               # argument block and workspace of the single-token steps
         self.block_types: Optional[torch.Tensor] = None  # [B, finished blocks, HN, 2] sampled types
         self.state: Optional[torch.Tensor] = None        # [B, H, K, V] fp32: current state
         self.state_block_start: Optional[torch.Tensor] = None
@@ -45,9 +45,12 @@ class NAtSLayerCache:
             t = getattr(self, name)
             setattr(new, name, None if t is None else t.clone())
         new.conv_state = None if self.conv_state is None else tuple(None if t is None else t.clone() for t in self.conv_state)
-        new._workspace = None
+        new._step = None
         self._kv_shared = new._kv_shared = True
         return new
+
+    def __getstate__(self):
+        return dict(self.__dict__, _step=None)             # holds addresses: not for another process
 
     @property
     def k_attn(self) -> Optional[torch.Tensor]:

@@ -13,7 +13,8 @@
 //     both operands leaves the sum unchanged).  Weight loads do not depend on the previous kernel and are issued before
 //     the programmatic-launch wait.
 //   * core: three kinds of CTA in one grid.  Every CTA recomputes the short convolution of the channels it needs (four
-//     taps), which costs less than a launch in between.  The recurrence reads the state once: S^T k and S^T q are formed
+//     taps), which costs less than a launch in between, and loads everything but the projections (states, tails, weights,
+//     the first keys) before it waits for them.  The recurrence reads the state once: S^T k and S^T q are formed
 //     together (o = e^g S^T q + (q.k) v').  Attention splits the 64-key units of the finished blocks over CTAs; a warp
 //     takes 16 keys of a unit, K and V loads of all of them in flight.
 //   * merge: combines the splits, both RMS norms, mixing weights and gate; extra CTAs shift the convolution tails.
@@ -27,9 +28,8 @@ namespace {
 
 using bf16 = __nv_bfloat16;
 constexpr int DS_THREADS = 128;               // core CTAs
-constexpr int DS_VS = 32;                     // value columns per recurrence CTA
 constexpr int DS_MAXK = 256;
-constexpr int DS_WROWS = 8;                   // mixing-weight rows per CTA
+constexpr int DS_MIX = 512;                   // channels per CTA of the mixing logits
 constexpr float kLog2e = 1.4426950408889634f;
 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -73,7 +73,7 @@ struct SkinnyArgs {
 // NB groups of 8 batch rows; WM warps side by side over weight rows (16 each), WK warps over the contraction.
 template <int NB, int WM, int WK>
 __global__ void __launch_bounds__(256) skinny_kernel(const SkinnyArgs a) {
-    constexpr int R = 16 * WM, UN = NB >= 4 ? 2 : 4;
+    constexpr int R = 16 * WM, UN = NB > 4 ? 2 : 4;
     __shared__ float red[WK][R][NB * 8 + 1];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int wm = warp % WM, wk = warp / WM, g = lane >> 2, t = lane & 3;
@@ -110,16 +110,21 @@ __global__ void __launch_bounds__(256) skinny_kernel(const SkinnyArgs a) {
 #pragma unroll
         for (int u = 0; u < UN; ++u) { ca[u] = wa[u]; cb[u] = wb[u]; }
         if (c + UN < c1) load_w(c + UN);
+        uint4 xv[UN][NB];                                 // all activation fragments of these steps in flight at once
 #pragma unroll
-        for (int u = 0; u < UN; ++u) {
-            if (c + u >= c1) break;
-            const uint32_t f0[4] = {ca[u].x, cb[u].x, ca[u].y, cb[u].y}, f1[4] = {ca[u].z, cb[u].z, ca[u].w, cb[u].w};
+        for (int u = 0; u < UN; ++u)
 #pragma unroll
             for (int n = 0; n < NB; ++n) {
                 const int row = n * 8 + g;
-                const uint4 xb = row < a.B ? *(reinterpret_cast<const uint4*>(a.x + (long)row * a.Kdim) + (c + u) * 4 + t) : zero;
-                mma_bf16(acc[n], f0, xb.x, xb.y);
-                mma_bf16(acc[n], f1, xb.z, xb.w);
+                xv[u][n] = row < a.B && c + u < c1 ? *(reinterpret_cast<const uint4*>(a.x + (long)row * a.Kdim) + (c + u) * 4 + t) : zero;
+            }
+#pragma unroll
+        for (int u = 0; u < UN; ++u) {
+            const uint32_t f0[4] = {ca[u].x, cb[u].x, ca[u].y, cb[u].y}, f1[4] = {ca[u].z, cb[u].z, ca[u].w, cb[u].w};
+#pragma unroll
+            for (int n = 0; n < NB; ++n) {
+                mma_bf16(acc[n], f0, xv[u][n].x, xv[u][n].y);
+                mma_bf16(acc[n], f1, xv[u][n].z, xv[u][n].w);
             }
         }
     }
@@ -145,23 +150,33 @@ struct CoreArgs {
     Args a;
     const bf16* raw;                          // [B, NR]: q | k | v | gate | a | b
     bf16* o_lin;                              // [B, H*V]
-    bf16* wlog;                               // [B, 2*HQ]
+    float* wlog;                              // [B, n_slices, 2*HQ] partial mixing logits
     float* part;                              // [B, HQ, S, DV + 2]
     float* gnew;                              // [B, H]
-    int NR, S, n_attn, n_rec;
+    int NR, S, n_attn, n_rec, vs, n_slices;
 };
 
-// Convolved channel (rounded to bf16 like the layer's own convolution output): tail = the last four inputs.
-__device__ __forceinline__ float conv1(const bf16* tail, const bf16* w, const bf16* bias, float x_new, int d, int silu) {
-    const uint2 tw = *reinterpret_cast<const uint2*>(tail), ww = *reinterpret_cast<const uint2*>(w + (long)d * 4);
-    const float2 t0 = unpack_bf16(tw.x), t1 = unpack_bf16(tw.y), w0 = unpack_bf16(ww.x), w1 = unpack_bf16(ww.y);
-    float acc = bias ? bf(bias, d) : 0.f;
-    acc += w0.x * t0.y;
-    acc += w0.y * t1.x;
-    acc += w1.x * t1.y;
-    acc += w1.y * x_new;
-    return rb(silu ? acc * (1.f / (1.f + __expf(-acc))) : acc);
-}
+// What a convolution needs besides the new input: the tail (the last four inputs), weights, bias.  None of it is written by
+// the kernels in front of this one in the step, so it is loaded before the programmatic-launch wait.
+struct Conv {
+    uint2 tail, w;
+    float bias;
+    __device__ __forceinline__ void load(const bf16* tails, const bf16* weights, const bf16* biases, long row, int d) {
+        tail = *reinterpret_cast<const uint2*>(tails + row * 4);
+        w = *reinterpret_cast<const uint2*>(weights + (long)d * 4);
+        bias = biases ? bf(biases, d) : 0.f;
+    }
+    // rounded to bf16 like the layer's own convolution output
+    __device__ __forceinline__ float operator()(float x_new, int silu) const {
+        const float2 t0 = unpack_bf16(tail.x), t1 = unpack_bf16(tail.y), w0 = unpack_bf16(w.x), w1 = unpack_bf16(w.y);
+        float acc = bias;
+        acc += w0.x * t0.y;
+        acc += w0.y * t1.x;
+        acc += w1.x * t1.y;
+        acc += w1.y * x_new;
+        return rb(silu ? acc * (1.f / (1.f + __expf(-acc))) : acc);
+    }
+};
 
 template <int NTHR>
 __device__ __forceinline__ float block_sum(float v, float* s_red, int tid) {
@@ -175,43 +190,65 @@ __device__ __forceinline__ float block_sum(float v, float* s_red, int tid) {
     return r;
 }
 
+// VS value columns (32 or 64) per CTA: rows of the state rg + RP i, four columns per thread.
+template <int VS>
 __device__ void core_recurrence(const CoreArgs& c, int idx, float* sm) {
+    constexpr int TPR = VS / 4, RP = DS_THREADS / TPR;    // threads per state row, rows per pass
     const Args& a = c.a;
     const int tid = threadIdx.x, K = a.K, V = a.V, H = a.H, HK = H * K, HV = H * V;
-    const int nvs = V / DS_VS, vs = idx % nvs, h = (idx / nvs) % H, b = idx / (nvs * H);
+    const int nvs = V / VS, vs = idx % nvs, h = (idx / nvs) % H, b = idx / (nvs * H);
     const bool gdn = a.rule == NATSL_RULE_GDN;
     float* s_q = sm;                           // [256]
     float* s_k = sm + DS_MAXK;                 // [256]
-    float* s_v = s_k + DS_MAXK;                // [32]
-    float* s_red = s_v + DS_VS;                // [8]
-    float* s_dot = s_red + 8;                  // [2][16][32]
+    float* s_v = s_k + DS_MAXK;                // [VS]
+    float* s_red = s_v + VS;                // [8]
+    float* s_dot = s_red + 8;                  // [2][RP][VS]
     const bf16* raw = c.raw + (long)b * c.NR;
-    // state rows of this thread: rg + 16 i, four columns
-    const int rg = tid >> 3, col = vs * DS_VS + (tid & 7) * 4;
+    const int rg = tid / TPR, c4 = (tid % TPR) * 4, col = vs * VS + c4;
     float* Sp = a.state + (((long)b * H + h) * K) * V + col;
     constexpr int NREG = 8;
     float4 S[NREG];
-    pdl_wait();
 #pragma unroll
     for (int i = 0; i < NREG; ++i)
-        if (rg + 16 * i < K) S[i] = *reinterpret_cast<const float4*>(Sp + (long)(rg + 16 * i) * V);
+        if (rg + RP * i < K) S[i] = *reinterpret_cast<const float4*>(Sp + (long)(rg + RP * i) * V);
+    Conv cq[2], ck[2], cv;
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+        if (tid + j * DS_THREADS < K) {
+            const int d = h * K + tid + j * DS_THREADS;
+            cq[j].load(a.conv_q, a.cw_q, a.cb_q, (long)b * HK + d, d);
+            ck[j].load(a.conv_k, a.cw_k, a.cb_k, (long)b * HK + d, d);
+        }
+    const int dv = h * V + vs * VS + (tid & (VS - 1));
+    cv.load(a.conv_v, a.cw_v, a.cb_v, (long)b * HV + dv, dv);
+    const float dtb = ldw(a.dt_bias, a.dt_f32, h), alog = expf(ldw(a.A_log, a.alog_f32, h));
+    const float gsum = a.types_new ? a.g_block[(long)b * H + h] : 0.f;
+    pdl_wait();
+    float rq2[2], rk2[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+        if (tid + j * DS_THREADS < K) {
+            rq2[j] = bf(raw, h * K + tid + j * DS_THREADS);
+            rk2[j] = bf(raw, HK + h * K + tid + j * DS_THREADS);
+        }
+    const float rv = bf(raw, 2 * HK + dv), z = bf(raw, 2 * HK + 2 * HV + h) + dtb;
+    const float braw = gdn ? bf(raw, 2 * HK + 2 * HV + H + h) : 0.f;
     float sq = 0.f, sk = 0.f;
-    for (int i = tid; i < K; i += DS_THREADS) {
-        const int d = h * K + i;
-        const float qv = conv1(a.conv_q + ((long)b * HK + d) * 4, a.cw_q, a.cb_q, bf(raw, d), d, a.silu);
-        const float kv = conv1(a.conv_k + ((long)b * HK + d) * 4, a.cw_k, a.cb_k, bf(raw, HK + d), d, a.silu);
-        s_q[i] = qv;
-        s_k[i] = kv;
-        sq += qv * qv;
-        sk += kv * kv;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const int i = tid + j * DS_THREADS;
+        if (i < K) {
+            const float qv = cq[j](rq2[j], a.silu), kv = ck[j](rk2[j], a.silu);
+            s_q[i] = qv;
+            s_k[i] = kv;
+            sq += qv * qv;
+            sk += kv * kv;
+        }
     }
-    const float araw = bf(raw, 2 * HK + 2 * HV + h);
-    const float z = araw + ldw(a.dt_bias, a.dt_f32, h);
     const float sp = z > 20.f ? z : log1pf(expf(z));
-    const float gt = -expf(ldw(a.A_log, a.alog_f32, h)) * sp;
-    if (tid < DS_VS) {
-        const int d = h * V + vs * DS_VS + tid;
-        float vv = conv1(a.conv_v + ((long)b * HV + d) * 4, a.cw_v, a.cb_v, bf(raw, 2 * HK + d), d, a.silu);
+    const float gt = -alog * sp;
+    if (tid < VS) {
+        float vv = cv(rv, a.silu);
         if (!gdn) vv = rb(vv * sp);
         s_v[tid] = vv;
     }
@@ -236,29 +273,29 @@ __device__ void core_recurrence(const CoreArgs& c, int idx, float* sm) {
     };
 #pragma unroll
     for (int i = 0; i < NREG; ++i)
-        if (rg + 16 * i < K) add(S[i], rg + 16 * i);
-    for (int r = rg + 16 * NREG; r < K; r += 16) add(*reinterpret_cast<const float4*>(Sp + (long)r * V), r);
-    float* d0 = s_dot + rg * DS_VS + (tid & 7) * 4;
+        if (rg + RP * i < K) add(S[i], rg + RP * i);
+    for (int r = rg + RP * NREG; r < K; r += RP) add(*reinterpret_cast<const float4*>(Sp + (long)r * V), r);
+    float* d0 = s_dot + rg * VS + c4;
     *reinterpret_cast<float4*>(d0) = dk;
-    *reinterpret_cast<float4*>(d0 + 16 * DS_VS) = dq;
+    *reinterpret_cast<float4*>(d0 + RP * VS) = dq;
     __syncthreads();
-    if (tid < DS_VS) {
+    if (tid < VS) {
         float tk = 0.f, tq = 0.f;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) { tk += s_dot[i * DS_VS + tid]; tq += s_dot[(16 + i) * DS_VS + tid]; }
+        for (int i = 0; i < RP; ++i) { tk += s_dot[i * VS + tid]; tq += s_dot[(RP + i) * VS + tid]; }
         const float eg = __expf(gt);
         float vv = s_v[tid];
         if (gdn) {
-            float beta = rb(1.f / (1.f + expf(-bf(raw, 2 * HK + 2 * HV + H + h))));
+            float beta = rb(1.f / (1.f + expf(-braw)));
             if (a.neg_eigval) beta *= 2.f;
             vv = beta * (vv - eg * tk);
         }
         s_v[tid] = vv;
-        c.o_lin[(long)b * HV + h * V + vs * DS_VS + tid] = __float2bfloat16((eg * tq + qk * vv) * a.scale_lin);
+        c.o_lin[(long)b * HV + h * V + vs * VS + tid] = __float2bfloat16((eg * tq + qk * vv) * a.scale_lin);
     }
     __syncthreads();
     const float eg = __expf(gt);
-    const float4 vn = *reinterpret_cast<const float4*>(s_v + (tid & 7) * 4);
+    const float4 vn = *reinterpret_cast<const float4*>(s_v + c4);
     const bool ends = a.types_new != nullptr;
     float* Bp = a.start + (((long)b * H + h) * K) * V + col;
     float roll = 1.f;
@@ -266,7 +303,7 @@ __device__ void core_recurrence(const CoreArgs& c, int idx, float* sm) {
     if (ends) {
         const int hn = h / (H / a.HN);
         sel = rintf(ldw(a.types_new, a.types_f32, ((long)b * a.HN + hn) * 2 + 1)) == 1.f;
-        roll = a.decay ? __expf(a.g_block[(long)b * H + h] + gt) : 1.f;
+        roll = a.decay ? __expf(gsum + gt) : 1.f;
     }
     auto upd = [&](float4 s, int r) {
         const float kk = s_k[r];
@@ -283,8 +320,8 @@ __device__ void core_recurrence(const CoreArgs& c, int idx, float* sm) {
     };
 #pragma unroll
     for (int i = 0; i < NREG; ++i)
-        if (rg + 16 * i < K) upd(S[i], rg + 16 * i);
-    for (int r = rg + 16 * NREG; r < K; r += 16) upd(*reinterpret_cast<const float4*>(Sp + (long)r * V), r);
+        if (rg + RP * i < K) upd(S[i], rg + RP * i);
+    for (int r = rg + RP * NREG; r < K; r += RP) upd(*reinterpret_cast<const float4*>(Sp + (long)r * V), r);
     if (vs == 0 && tid == 0) c.gnew[(long)b * H + h] = gt;
 }
 
@@ -302,26 +339,94 @@ __device__ void core_attention(const CoreArgs& c, int idx, float* sm) {
     float* s_ml = s_p + 64;                            // [4][2]
     float* s_red = s_ml + 8;                           // [8]
     float* s_acc = s_red + 8;                          // [4][DV]
-    pdl_wait();
-    const bf16* raw = c.raw + (long)b * c.NR;
     const bool last = s == c.S - 1;
+    float m = -INFINITY, l = 0.f, acc[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc[e] = 0.f;
+    const bf16* kb = a.k_cache + ((long)b * a.cap * a.HQ + hq) * DK + (lane % LK) * 8;
+    const bf16* vb = a.v_cache + ((long)b * a.cap * a.HQ + hq) * DV + (lane % LV) * 8;
+    float* my_p = s_p + warp * 16;
+    // A step of a warp = KS keys, four 16-byte K loads and as many V loads as their width takes, with the next step's loads
+    // in flight while this one is computed.  Steps: the warp's quarter of every selected 64-key unit of this split (32 units'
+    // selection bits per load, by ballot), then of the current block.
+    constexpr int KM = KG < VG ? KG : VG, KS = 4 * KM < 16 ? 4 * KM : 16, NK = KS / KG, NV = KS / VG;
+    static_assert(NK >= 1 && NV >= 1, "lanes per row");
+    const int hn = hq / (a.HQ / a.HN), upb = a.nbs / 64;
+    const int n_units = a.n_done * upb;
+    const int u0 = (int)((long)n_units * s / c.S), u1 = (int)((long)n_units * (s + 1) / c.S);
+    const int own0 = (last && a.own_chunk) ? a.pos / a.nbs * a.nbs : a.pos;     // keys of the current block before the new token
+    const long tstride = (long)a.HN * 2;
+    const long tbase = ((long)b * a.n_done * a.HN + hn) * 2;
+    unsigned mask = 0;
+    int base = u0 - 32, sub = 0, unit = -1, own = own0 + warp * 16;
+    auto next = [&](int& key0, int& n) -> bool {
+        if (unit >= 0 && sub + KS < 16) {                                       // rest of the warp's 16 keys of this unit
+            sub += KS;
+            key0 = unit * 64 + warp * 16 + sub;
+            n = KS;
+            return true;
+        }
+        while (mask == 0 && base + 32 < u1) {
+            base += 32;
+            const int u = base + lane;
+            mask = __ballot_sync(0xffffffffu, u < u1 && ldw(a.types, a.types_f32, tbase + (long)(u / upb) * tstride) > 0.5f);
+        }
+        if (mask) {
+            unit = base + __ffs(mask) - 1;
+            mask &= mask - 1;
+            sub = 0;
+            key0 = unit * 64 + warp * 16;
+            n = KS;
+            return true;
+        }
+        unit = -1;
+        if (own >= a.pos) return false;
+        key0 = own;
+        n = min(KS, a.pos - own);
+        const int in = (own - own0) & 15;
+        own += in + KS < 16 ? KS : 64 - in;
+        return true;
+    };
+    auto fetch = [&](int key0, int n, uint4 (&kr)[NK], uint4 (&vr)[NV]) {
+#pragma unroll
+        for (int i = 0; i < NK; ++i)
+            kr[i] = *reinterpret_cast<const uint4*>(kb + (long)(key0 + min(i * KG + lane / LK, n - 1)) * a.HQ * DK);
+#pragma unroll
+        for (int i = 0; i < NV; ++i)
+            vr[i] = *reinterpret_cast<const uint4*>(vb + (long)(key0 + min(i * VG + lane / LV, n - 1)) * a.HQ * DV);
+    };
+    uint4 k0[NK], v0[NV], k1[NK], v1[NV];
+    int key0 = 0, n0 = 0, n1 = 0;
+    bool more0 = next(key0, n0), more1 = false;
+    if (more0) fetch(key0, n0, k0, v0);
+
+    // ---- query of this head, and (last split) the new token's key and value: they wait for the projections
     {
-        float qv = 0.f, kv = 0.f;
-        if (tid < DK) {
-            const int d = hq * DK + tid;
-            qv = bf(raw, d);
-            kv = bf(raw, HK + d);
-            if (a.attn_conv) {
-                qv = conv1(a.conv_q + ((long)b * HK + d) * 4, a.cw_q, a.cb_q, qv, d, a.silu);
-                kv = conv1(a.conv_k + ((long)b * HK + d) * 4, a.cw_k, a.cb_k, kv, d, a.silu);
-            }
+        const int dk = hq * DK + (tid & (DK - 1)), dv = hq * DV + (tid & (DV - 1));
+        Conv cq, ck, cv;
+        float wq = 1.f, wk = 1.f;
+        if (a.attn_conv) {
+            cq.load(a.conv_q, a.cw_q, a.cb_q, (long)b * HK + dk, dk);
+            ck.load(a.conv_k, a.cw_k, a.cb_k, (long)b * HK + dk, dk);
+            cv.load(a.conv_v, a.cw_v, a.cb_v, (long)b * HV + dv, dv);
         }
         if (a.qn_w) {
-            const float sq = block_sum<DS_THREADS>(qv * qv, s_red, tid), sk = block_sum<DS_THREADS>(kv * kv, s_red + 4, tid);
-            if (tid < DK) {
-                qv = rb(qv * rsqrtf(sq / DK + a.norm_eps) * ldw(a.qn_w, a.qn_f32, tid));
-                kv = rb(kv * rsqrtf(sk / DK + a.norm_eps) * ldw(a.kn_w, a.kn_f32, tid));
-            }
+            wq = ldw(a.qn_w, a.qn_f32, tid & (DK - 1));
+            wk = ldw(a.kn_w, a.kn_f32, tid & (DK - 1));
+        }
+        pdl_wait();
+        const bf16* raw = c.raw + (long)b * c.NR;
+        float qv = bf(raw, dk), kv = bf(raw, HK + dk), vv = bf(raw, 2 * HK + dv);
+        if (a.attn_conv) {
+            qv = cq(qv, a.silu);
+            kv = ck(kv, a.silu);
+            vv = cv(vv, a.silu);
+        }
+        if (a.qn_w) {
+            const float sq = block_sum<DS_THREADS>(tid < DK ? qv * qv : 0.f, s_red, tid);
+            const float sk = block_sum<DS_THREADS>(tid < DK ? kv * kv : 0.f, s_red + 4, tid);
+            qv = rb(qv * rsqrtf(sq / DK + a.norm_eps) * wq);
+            kv = rb(kv * rsqrtf(sk / DK + a.norm_eps) * wk);
         }
         if (tid < DK) {
             s_q[tid] = qv * (a.scale_attn * kLog2e);
@@ -329,9 +434,6 @@ __device__ void core_attention(const CoreArgs& c, int idx, float* sm) {
             if (last) a.k_cache[(((long)b * a.cap + a.pos) * a.HQ + hq) * DK + tid] = __float2bfloat16(kv);
         }
         if (last && tid < DV) {
-            const int d = hq * DV + tid;
-            float vv = bf(raw, 2 * HK + d);
-            if (a.attn_conv) vv = conv1(a.conv_v + ((long)b * HV + d) * 4, a.cw_v, a.cb_v, vv, d, a.silu);
             s_vn[tid] = vv;
             a.v_cache[(((long)b * a.cap + a.pos) * a.HQ + hq) * DV + tid] = __float2bfloat16(vv);
         }
@@ -343,25 +445,7 @@ __device__ void core_attention(const CoreArgs& c, int idx, float* sm) {
 #pragma unroll
         for (int e = 0; e < 8; ++e) q8[e] = s_q[d0 + e];
     }
-    float m = -INFINITY, l = 0.f, acc[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) acc[e] = 0.f;
-    const bf16* kb = a.k_cache + ((long)b * a.cap * a.HQ + hq) * DK + (lane % LK) * 8;
-    const bf16* vb = a.v_cache + ((long)b * a.cap * a.HQ + hq) * DV + (lane % LV) * 8;
-    float* my_p = s_p + warp * 16;
-    auto unit = [&](int key0, int n_keys) {            // this warp's 16 keys from key0, the first n_keys of them valid
-        constexpr int NK = 16 / KG, NV = 16 / VG;
-        uint4 kr[NK], vr[NV];
-#pragma unroll
-        for (int i = 0; i < NK; ++i) {
-            const int j = min(i * KG + lane / LK, n_keys - 1);
-            kr[i] = *reinterpret_cast<const uint4*>(kb + (long)(key0 + j) * a.HQ * DK);
-        }
-#pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            const int j = min(i * VG + lane / LV, n_keys - 1);
-            vr[i] = *reinterpret_cast<const uint4*>(vb + (long)(key0 + j) * a.HQ * DV);
-        }
+    auto step = [&](const uint4 (&kr)[NK], const uint4 (&vr)[NV], int n_keys) {
 #pragma unroll
         for (int i = 0; i < NK; ++i) {
             const uint32_t* w = reinterpret_cast<const uint32_t*>(&kr[i]);
@@ -377,25 +461,22 @@ __device__ void core_attention(const CoreArgs& c, int idx, float* sm) {
             if (lane % LK == 0) my_p[i * KG + lane / LK] = d;
         }
         __syncwarp();
-        const float sc = (lane & 15) < n_keys ? my_p[lane & 15] : -INFINITY;
+        const float sc = (lane & (KS - 1)) < n_keys ? my_p[lane & (KS - 1)] : -INFINITY;
         float mx = sc;
 #pragma unroll
-        for (int o = 8; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        for (int o = KS / 2; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         const float mn = fmaxf(m, mx), al = exp2f(m - mn);
         const float p = exp2f(sc - mn);
         float ps = p;
 #pragma unroll
-        for (int o = 8; o > 0; o >>= 1) ps += __shfl_xor_sync(0xffffffffu, ps, o);
+        for (int o = KS / 2; o > 0; o >>= 1) ps += __shfl_xor_sync(0xffffffffu, ps, o);
         l = l * al + ps;
         m = mn;
-        __syncwarp();
-        if (lane < 16) my_p[lane] = p;
-        __syncwarp();
 #pragma unroll
         for (int e = 0; e < 8; ++e) acc[e] *= al;
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
-            const float pj = my_p[i * VG + lane / LV];
+            const float pj = __shfl_sync(0xffffffffu, p, i * VG + lane / LV);
             const uint32_t* w = reinterpret_cast<const uint32_t*>(&vr[i]);
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
@@ -406,16 +487,15 @@ __device__ void core_attention(const CoreArgs& c, int idx, float* sm) {
         }
         __syncwarp();
     };
-    const int hn = hq / (a.HQ / a.HN), upb = a.nbs / 64;
-    const int n_units = a.n_done * upb;
-    const int u0 = (int)((long)n_units * s / c.S), u1 = (int)((long)n_units * (s + 1) / c.S);
-    for (int u = u0; u < u1; ++u) {
-        const int blk = u / upb;
-        if (ldw(a.types, a.types_f32, (((long)b * a.n_done + blk) * a.HN + hn) * 2) > 0.5f) unit(u * 64 + warp * 16, 16);
-    }
-    if (last && a.own_chunk) {
-        const int own0 = a.pos / a.nbs * a.nbs;         // keys of the current block before the new token
-        for (int k0 = own0 + warp * 16; k0 < a.pos; k0 += 64) unit(k0, min(16, a.pos - k0));
+    // two register buffers in turn (a copy from one to the other would wait for its loads before the next ones are issued)
+    while (more0) {
+        more1 = next(key0, n1);
+        if (more1) fetch(key0, n1, k1, v1);
+        step(k0, v0, n0);
+        if (!more1) break;
+        more0 = next(key0, n0);
+        if (more0) fetch(key0, n0, k0, v0);
+        step(k1, v1, n1);
     }
     // sum the key groups of a warp, then the warps
 #pragma unroll
@@ -426,10 +506,10 @@ __device__ void core_attention(const CoreArgs& c, int idx, float* sm) {
 #pragma unroll
         for (int e = 0; e < 8; ++e) s_acc[warp * DV + lane * 8 + e] = acc[e];
     if (lane == 0) { s_ml[warp * 2] = m; s_ml[warp * 2 + 1] = l; }
-    float own = -INFINITY;                              // score of the new token
-    if (last && a.own_chunk) own = block_sum<DS_THREADS>(tid < DK ? s_q[tid] * s_kn[tid] : 0.f, s_red, tid);
+    float s_new = -INFINITY;                            // score of the new token
+    if (last && a.own_chunk) s_new = block_sum<DS_THREADS>(tid < DK ? s_q[tid] * s_kn[tid] : 0.f, s_red, tid);
     __syncthreads();
-    float M = own;
+    float M = s_new;
 #pragma unroll
     for (int w = 0; w < 4; ++w) M = fmaxf(M, s_ml[w * 2]);
     float* part = c.part + (((long)b * a.HQ + hq) * c.S + s) * (DV + 2);
@@ -442,8 +522,8 @@ __device__ void core_attention(const CoreArgs& c, int idx, float* sm) {
                 L += f * s_ml[w * 2 + 1];
                 o += f * s_acc[w * DV + tid];
             }
-            if (own != -INFINITY) {
-                const float p = exp2f(own - M);
+            if (s_new != -INFINITY) {
+                const float p = exp2f(s_new - M);
                 L += p;
                 o += p * s_vn[tid];
             }
@@ -453,69 +533,99 @@ __device__ void core_attention(const CoreArgs& c, int idx, float* sm) {
     }
 }
 
-// logits of the mixing weights: rows of w_mix [2 HQ, H K] times the convolved query of one batch row
-__device__ void core_mix_logits(const CoreArgs& c, int idx) {
+// Partial logits of the mixing weights: all rows of w_mix [2 HQ, H K] times one slice of DS_MIX channels of the convolved
+// query of one batch row (the merge adds the slices up; whole rows per CTA took 16 us at H K = 4096, a chain of 32
+// convolutions per thread).
+__device__ void core_mix_logits(const CoreArgs& c, int idx, float* sm) {
     const Args& a = c.a;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int rows = 2 * a.HQ, groups = (rows + DS_WROWS - 1) / DS_WROWS;
-    const int b = idx / groups, row0 = (idx % groups) * DS_WROWS, HK = a.H * a.K;
-    extern __shared__ float s_dyn[];                   // [HK] convolved query
-    pdl_wait();
-    const bf16* raw = c.raw + (long)b * c.NR;
-    for (int d = tid; d < HK; d += DS_THREADS)
-        s_dyn[d] = conv1(a.conv_q + ((long)b * HK + d) * 4, a.cw_q, a.cb_q, bf(raw, d), d, a.silu);
-    __syncthreads();
-    for (int r = row0 + warp; r < min(row0 + DS_WROWS, rows); r += 4) {
-        float acc = 0.f;
-        for (int d = lane * 8; d < HK; d += 256) {
-            const uint4 v = *reinterpret_cast<const uint4*>(a.w_mix + (long)r * HK + d);
-            const uint32_t* w = reinterpret_cast<const uint32_t*>(&v);
+    const int HK = a.H * a.K, rows = 2 * a.HQ, slice = idx % c.n_slices, b = idx / c.n_slices, d0 = slice * DS_MIX;
+    constexpr int PER = DS_MIX / DS_THREADS;
+    Conv cq[PER];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float2 f = unpack_bf16(w[e]);
-                acc += f.x * s_dyn[d + 2 * e];
-                acc += f.y * s_dyn[d + 2 * e + 1];
+    for (int j = 0; j < PER; ++j) {
+        const int d = min(d0 + tid + j * DS_THREADS, HK - 1);
+        cq[j].load(a.conv_q, a.cw_q, a.cb_q, (long)b * HK + d, d);
+    }
+    pdl_wait();
+    float x[PER];
+#pragma unroll
+    for (int j = 0; j < PER; ++j) x[j] = bf(c.raw + (long)b * c.NR, min(d0 + tid + j * DS_THREADS, HK - 1));
+#pragma unroll
+    for (int j = 0; j < PER; ++j) sm[tid + j * DS_THREADS] = d0 + tid + j * DS_THREADS < HK ? cq[j](x[j], a.silu) : 0.f;
+    __syncthreads();
+    float q[DS_MIX / 32];                                   // channels (lane + 32 i) * 8 .. + 7
+#pragma unroll
+    for (int i = 0; i < DS_MIX / 256; ++i)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) q[i * 8 + e] = sm[(lane + 32 * i) * 8 + e];
+#pragma unroll 4
+    for (int r = warp; r < rows; r += DS_THREADS / 32) {
+        float acc = 0.f;
+#pragma unroll
+        for (int i = 0; i < DS_MIX / 256; ++i) {
+            const int d = d0 + (lane + 32 * i) * 8;
+            if (d < HK) {
+                const uint4 v = *reinterpret_cast<const uint4*>(a.w_mix + (long)r * HK + d);
+                const uint32_t* w = reinterpret_cast<const uint32_t*>(&v);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float2 f = unpack_bf16(w[e]);
+                    acc += f.x * q[i * 8 + 2 * e];
+                    acc += f.y * q[i * 8 + 2 * e + 1];
+                }
             }
         }
         acc = warp_sum(acc);
-        if (lane == 0) c.wlog[(long)b * rows + r] = __float2bfloat16(acc);
+        if (lane == 0) c.wlog[((long)b * c.n_slices + slice) * rows + r] = acc;
     }
 }
 
 template <int DK, int DV>
-__global__ void __launch_bounds__(DS_THREADS) decode_core_kernel(const CoreArgs c) {
-    __shared__ __align__(16) float sm[2 * DS_MAXK + DS_VS + 8 + 2 * 16 * DS_VS];
-    static_assert(2 * DK + DV + 64 + 16 + 4 * DV <= 2 * DS_MAXK + DS_VS + 8 + 2 * 16 * DS_VS, "attention scratch");
+__global__ void __launch_bounds__(DS_THREADS, 4) decode_core_kernel(const CoreArgs c) {
+    __shared__ __align__(16) float sm[2 * DS_MAXK + 64 + 8 + 2 * DS_THREADS * 4];
+    static_assert(2 * DK + DV + 64 + 16 + 4 * DV <= 2 * DS_MAXK + 64 + 8 + 2 * DS_THREADS * 4, "attention scratch");
     pdl_trigger();
     int idx = blockIdx.x;
     if (idx < c.n_attn) {
         core_attention<DK, DV>(c, idx, sm);
     } else if (idx < c.n_attn + c.n_rec) {
-        core_recurrence(c, idx - c.n_attn, sm);
+        if (c.vs == 64) core_recurrence<64>(c, idx - c.n_attn, sm);
+        else core_recurrence<32>(c, idx - c.n_attn, sm);
     } else {
-        core_mix_logits(c, idx - c.n_attn - c.n_rec);
+        core_mix_logits(c, idx - c.n_attn - c.n_rec, sm);
     }
 }
 
 // ------------------------------------------------------------------------------------------------ merge
 struct MergeArgs {
     Args a;
-    const bf16 *raw, *o_lin, *wlog;
-    const float *part, *gnew;
+    const bf16 *raw, *o_lin;
+    const float *wlog, *part, *gnew;
     bf16* y;                                  // [B, H*V]
-    int NR, S, n_heads;                       // n_heads = B * HQ CTAs of the merge itself, then the tail CTAs
+    int NR, S, n_slices, n_heads;             // n_heads = B * HQ, four to a CTA, then the CTAs of the tails
 };
 
+// One warp per (batch, head), DV / 32 channels per lane: nothing but warp shuffles between the loads, which are issued up front.
 template <int DV>
-__global__ void __launch_bounds__(DV) decode_merge_kernel(const MergeArgs c) {
+__global__ void __launch_bounds__(128) decode_merge_kernel(const MergeArgs c) {
+    constexpr int E = DV / 32;
     const Args& a = c.a;
-    const int tid = threadIdx.x, HK = a.H * a.K, HV = a.H * a.V;
-    __shared__ float s_red[8];
+    const int tid = threadIdx.x, lane = tid & 31, HK = a.H * a.K, HV = a.H * a.V;
+    const int n_cta = (c.n_heads + 3) / 4;
+    float w1[E], w2[E];
+    const bool tails = (int)blockIdx.x >= n_cta;
+    if (!tails)
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            w1[e] = a.w1 ? ldw(a.w1, a.w12_f32, lane * E + e) : 1.f;
+            w2[e] = a.w2 ? ldw(a.w2, a.w12_f32, lane * E + e) : 1.f;
+        }
     pdl_wait();
     pdl_trigger();
-    if ((int)blockIdx.x >= c.n_heads) {
+    if (tails) {
         // convolution tails: drop the oldest input, append the new one; decay sums of the current block
-        const long i = (long)(blockIdx.x - c.n_heads) * DV + tid;
+        const long i = (long)(blockIdx.x - n_cta) * 128 + tid;
         const int per = 2 * HK + HV;
         if (i < (long)a.B * per) {
             const int b = (int)(i / per);
@@ -533,67 +643,96 @@ __global__ void __launch_bounds__(DV) decode_merge_kernel(const MergeArgs c) {
         if (i < a.B * a.H) a.g_block[i] = a.types_new ? 0.f : a.g_block[i] + c.gnew[i];
         return;
     }
-    const int hq = blockIdx.x % a.HQ, b = blockIdx.x / a.HQ;
-    const float* part = c.part + ((long)b * a.HQ + hq) * c.S * (DV + 2);
-    float M = -INFINITY;
-    for (int s = 0; s < c.S; ++s) M = fmaxf(M, part[(long)s * (DV + 2)]);
-    float L = 0.f, o = 0.f;
-    if (M != -INFINITY)
-        for (int s = 0; s < c.S; ++s) {
-            const float* p = part + (long)s * (DV + 2);
-            const float f = exp2f(p[0] - M);
-            L += f * p[1];
-            o += f * p[2 + tid];
-        }
-    const float x2 = rb(L > 0.f ? o / L : 0.f);
-    const int d = hq * DV + tid;
-    const float x1 = bf(c.o_lin, (long)b * HV + d);
-    const float s1 = block_sum<DV>(x1 * x1, s_red, tid), s2 = block_sum<DV>(x2 * x2, s_red + 4, tid);
-    const float r1 = rsqrtf(s1 / DV + a.mix_eps), r2 = rsqrtf(s2 / DV + a.mix_eps);
-    float m1 = 1.f, m2 = 1.f;
-    if (a.w_mix) {
-        const float l1 = bf(c.wlog, ((long)b * a.HQ + hq) * 2), l2 = bf(c.wlog, ((long)b * a.HQ + hq) * 2 + 1);
-        const float mx = fmaxf(l1, l2), e1 = expf(l1 - mx), e2 = expf(l2 - mx);
-        m1 = rb(e1 / (e1 + e2));
-        m2 = rb(e2 / (e1 + e2));
+    const int unit = blockIdx.x * 4 + (tid >> 5);
+    if (unit >= c.n_heads) return;
+    const int hq = unit % a.HQ, b = unit / a.HQ;
+    const float* part = c.part + (long)unit * c.S * (DV + 2);
+    const int d0 = hq * DV + lane * E;
+    float x1[E], gg[E], o[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        x1[e] = bf(c.o_lin, (long)b * HV + d0 + e);
+        gg[e] = bf(c.raw, (long)b * c.NR + 2 * HK + HV + d0 + e);
+        o[e] = 0.f;
     }
-    const float gg = bf(c.raw, (long)b * c.NR + 2 * HK + HV + d);
-    const float v = x1 * r1 * (a.w1 ? ldw(a.w1, a.w12_f32, tid) : 1.f) * m1 + x2 * r2 * (a.w2 ? ldw(a.w2, a.w12_f32, tid) : 1.f) * m2;
-    const float sg = 1.f / (1.f + __expf(-gg));
-    c.y[(long)b * HV + d] = __float2bfloat16(a.mix_sigmoid ? v * sg : v * gg * sg);
+    float l1 = 0.f, l2 = 0.f;
+    if (a.w_mix) {
+        for (int k = 0; k < c.n_slices; ++k) {
+            const float2 w = *reinterpret_cast<const float2*>(c.wlog + (((long)b * c.n_slices + k) * a.HQ + hq) * 2);
+            l1 += w.x;
+            l2 += w.y;
+        }
+        l1 = rb(l1);
+        l2 = rb(l2);
+    }
+    // splits s = lane, lane + 32 (at most 64)
+    float m0 = -INFINITY, m1 = -INFINITY, s0 = 0.f, s1 = 0.f;
+    if (lane < c.S) { m0 = part[(long)lane * (DV + 2)]; s0 = part[(long)lane * (DV + 2) + 1]; }
+    if (lane + 32 < c.S) { m1 = part[(long)(lane + 32) * (DV + 2)]; s1 = part[(long)(lane + 32) * (DV + 2) + 1]; }
+    float M = fmaxf(m0, m1);
+#pragma unroll
+    for (int k = 16; k > 0; k >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, k));
+    const float f0 = M == -INFINITY ? 0.f : exp2f(m0 - M), f1 = M == -INFINITY ? 0.f : exp2f(m1 - M);
+    const float L = warp_sum(f0 * s0 + f1 * s1);
+#pragma unroll 4
+    for (int s = 0; s < c.S; ++s) {
+        const float f = __shfl_sync(0xffffffffu, s < 32 ? f0 : f1, s & 31);
+        const float* p = part + (long)s * (DV + 2) + 2 + lane * E;
+#pragma unroll
+        for (int e = 0; e < E; ++e) o[e] += f * p[e];
+    }
+    float q1 = 0.f, q2 = 0.f;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        o[e] = rb(L > 0.f ? o[e] / L : 0.f);
+        q1 += x1[e] * x1[e];
+        q2 += o[e] * o[e];
+    }
+    const float r1 = rsqrtf(warp_sum(q1) / DV + a.mix_eps), r2 = rsqrtf(warp_sum(q2) / DV + a.mix_eps);
+    float m_1 = 1.f, m_2 = 1.f;
+    if (a.w_mix) {
+        const float mx = fmaxf(l1, l2), e1 = expf(l1 - mx), e2 = expf(l2 - mx);
+        m_1 = rb(e1 / (e1 + e2));
+        m_2 = rb(e2 / (e1 + e2));
+    }
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const float v = x1[e] * r1 * w1[e] * m_1 + o[e] * r2 * w2[e] * m_2;
+        const float sg = 1.f / (1.f + __expf(-gg[e]));
+        c.y[(long)b * HV + d0 + e] = __float2bfloat16(a.mix_sigmoid ? v * sg : v * gg[e] * sg);
+    }
 }
 
 // ------------------------------------------------------------------------------------------------ host
 template <typename Arg>
-cudaError_t launch_pdl(void (*kern)(const Arg), unsigned grid, unsigned block, size_t smem, cudaStream_t st, const Arg& arg) {
+cudaError_t launch_pdl(void (*kern)(const Arg), unsigned grid, unsigned block, cudaStream_t st, const Arg& arg, bool overlap = true) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = overlap ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kern, arg);
 }
 
-// Row tiles of every segment, then the launch.  The split between weight rows and contraction per CTA follows the batch:
-// few batch rows -> all warps on the contraction of 16 weight rows (most CTAs, most loads in flight); more rows -> warps
-// side by side over weight rows, so that a CTA reads the activations once for 64 of them.
-cudaError_t launch_skinny(SkinnyArgs& a, cudaStream_t st) {
+// Row tiles of every segment, then the launch.  Up to 32 batch rows all eight warps share the contraction of 16 weight rows
+// (most CTAs, most loads in flight; 64-row tiles left 16 CTAs for the output product at hidden 1024: 15 us a product); above
+// that, warps side by side over 64 weight rows read the activations a quarter as often.
+cudaError_t launch_skinny(SkinnyArgs& a, cudaStream_t st, bool overlap) {
     const int nb = (a.B + 7) / 8;
-    const int R = nb == 1 ? 16 : nb == 2 ? 32 : 64;
+    const int R = nb <= 4 ? 16 : 64;
     int tiles = 0;
     for (int i = 0; i < a.nseg; ++i) {
         a.seg[i].tile0 = tiles;
         tiles += (a.seg[i].rows + R - 1) / R;
     }
-    if (nb == 1) return launch_pdl(skinny_kernel<1, 1, 8>, tiles, 256, 0, st, a);
-    if (nb == 2) return launch_pdl(skinny_kernel<2, 2, 4>, tiles, 256, 0, st, a);
-    if (nb <= 4) return launch_pdl(skinny_kernel<4, 4, 2>, tiles, 256, 0, st, a);
-    return launch_pdl(skinny_kernel<8, 4, 2>, tiles, 256, 0, st, a);
+    if (nb == 1) return launch_pdl(skinny_kernel<1, 1, 8>, tiles, 256, st, a, overlap);
+    if (nb == 2) return launch_pdl(skinny_kernel<2, 1, 8>, tiles, 256, st, a, overlap);
+    if (nb <= 4) return launch_pdl(skinny_kernel<4, 1, 8>, tiles, 256, st, a, overlap);
+    return launch_pdl(skinny_kernel<8, 4, 2>, tiles, 256, st, a, overlap);
 }
 
 // Splits of the finished keys of one (batch, head) over CTAs: enough CTAs for four per SM, at least two 64-key units each.
@@ -605,7 +744,7 @@ int attn_splits(int B, int HQ, int units) {
 
 struct Layout {
     long raw, olin, wlog, y, part, gnew, total;
-    int NR, S;
+    int NR, S, slices;
 };
 Layout layout(const Args& a) {
     Layout l;
@@ -617,7 +756,8 @@ Layout layout(const Args& a) {
     l.raw = 0;
     l.olin = up(l.raw + 2l * a.B * l.NR);
     l.wlog = up(l.olin + 2l * a.B * HV);
-    l.y = up(l.wlog + 2l * a.B * 2 * a.HQ);
+    l.slices = (int)((HK + DS_MIX - 1) / DS_MIX);
+    l.y = up(l.wlog + 4l * a.B * l.slices * 2 * a.HQ);
     l.gnew = up(l.y + 2l * a.B * HV);
     l.part = up(l.gnew + 4l * a.B * a.H);
     // sized for the most splits this batch can get, so that one workspace serves a request from its first token on
@@ -631,7 +771,7 @@ int check(const Args* a) {
     NATSL_REQUIRE(a->B > 0 && a->B <= 64 && a->hidden > 0 && a->hidden % 32 == 0 && a->H > 0 && a->HQ > 0 && a->HN > 0 &&
                       a->H % a->HN == 0 && a->HQ % a->HN == 0 && a->nbs >= 64 && a->nbs % 64 == 0,
                   NATSL_ERR_BAD_SHAPE, "natsl_decode_step: bad shape (1 <= B <= 64, hidden a multiple of 32)");
-    NATSL_REQUIRE(a->K % 32 == 0 && a->K <= DS_MAXK && a->V % DS_VS == 0 && (a->H * a->K) % a->HQ == 0 && (a->H * a->V) % a->HQ == 0,
+    NATSL_REQUIRE(a->K % 32 == 0 && a->K <= DS_MAXK && a->V % 32 == 0 && (a->H * a->K) % a->HQ == 0 && (a->H * a->V) % a->HQ == 0,
                   NATSL_ERR_UNSUPPORTED, "natsl_decode_step: head dims K=%d V=%d (multiples of 32, K <= 256)", a->K, a->V);
     const int DK = a->H * a->K / a->HQ, DV = a->H * a->V / a->HQ;
     NATSL_REQUIRE((DK == 64 || DK == 128) && (DV == 64 || DV == 128), NATSL_ERR_UNSUPPORTED,
@@ -684,25 +824,28 @@ extern "C" int natsl_decode_step(const natsl_decode_args* args, void* stream) {
     p.x = a.x;
     p.y = raw;
     p.pool = a.pool_sum;
-    cudaError_t e = launch_skinny(p, st);
+    // the first launch waits for everything in front of it (its early weight loads must not overtake a kernel that writes
+    // them), the other three overlap their prologues with the one before
+    cudaError_t e = launch_skinny(p, st, false);
 
     CoreArgs c = {};
     c.a = a;
     c.raw = raw;
     c.o_lin = reinterpret_cast<bf16*>(ws + l.olin);
-    c.wlog = reinterpret_cast<bf16*>(ws + l.wlog);
+    c.wlog = reinterpret_cast<float*>(ws + l.wlog);
     c.part = reinterpret_cast<float*>(ws + l.part);
     c.gnew = reinterpret_cast<float*>(ws + l.gnew);
     c.NR = l.NR;
     c.S = l.S;
     c.n_attn = a.B * a.HQ * l.S;
-    c.n_rec = a.B * a.H * (a.V / DS_VS);
-    const int n_mix = a.w_mix ? a.B * ((2 * a.HQ + DS_WROWS - 1) / DS_WROWS) : 0;
-    const size_t dyn = a.w_mix ? (size_t)HK * 4 : 0;
-    NATSL_REQUIRE(dyn <= 40 * 1024, NATSL_ERR_TOO_LARGE, "natsl_decode_step: H*K = %d is too large", HK);
+    // 64 columns per recurrence CTA (half the convolution work) once 32 would take more than one wave
+    c.vs = a.K <= 64 && a.V % 64 == 0 && (long)a.B * a.H * (a.V / 32) > 148 * 4 ? 64 : 32;
+    c.n_rec = a.B * a.H * (a.V / c.vs);
+    c.n_slices = l.slices;
+    const int n_mix = a.w_mix ? a.B * l.slices : 0;
     auto core = DK == 64 ? (DV == 64 ? decode_core_kernel<64, 64> : decode_core_kernel<64, 128>)
                          : (DV == 64 ? decode_core_kernel<128, 64> : decode_core_kernel<128, 128>);
-    if (e == cudaSuccess) e = launch_pdl(core, c.n_attn + c.n_rec + n_mix, DS_THREADS, dyn, st, c);
+    if (e == cudaSuccess) e = launch_pdl(core, c.n_attn + c.n_rec + n_mix, DS_THREADS, st, c);
 
     MergeArgs g = {};
     g.a = a;
@@ -714,9 +857,11 @@ extern "C" int natsl_decode_step(const natsl_decode_args* args, void* stream) {
     g.y = reinterpret_cast<bf16*>(ws + l.y);
     g.NR = l.NR;
     g.S = l.S;
+    g.n_slices = l.slices;
     g.n_heads = a.B * a.HQ;
-    const unsigned tails = (unsigned)(((long)a.B * (2 * HK + HV) + DV - 1) / DV);
-    if (e == cudaSuccess) e = launch_pdl(DV == 64 ? decode_merge_kernel<64> : decode_merge_kernel<128>, g.n_heads + tails, DV, 0, st, g);
+    const unsigned tails = (unsigned)(((long)a.B * (2 * HK + HV) + 127) / 128);
+    if (e == cudaSuccess)
+        e = launch_pdl(DV == 64 ? decode_merge_kernel<64> : decode_merge_kernel<128>, (g.n_heads + 3) / 4 + tails, 128, st, g);
 
     SkinnyArgs o = {};
     o.seg[0] = {a.w_o, a.hidden, 0, 0};
@@ -726,7 +871,7 @@ extern "C" int natsl_decode_step(const natsl_decode_args* args, void* stream) {
     o.y_stride = a.hidden;
     o.x = g.y;
     o.y = a.out;
-    if (e == cudaSuccess) e = launch_skinny(o, st);
+    if (e == cudaSuccess) e = launch_skinny(o, st, true);
     if (e != cudaSuccess) {
         set_error("natsl_decode_step: CUDA error %d (%s)", (int)e, cudaGetErrorString(e));
         return NATSL_ERR_CUDA;

@@ -4,6 +4,7 @@ configurations the kernel is built for; everything else takes the general path o
 from __future__ import annotations
 
 import ctypes
+import operator
 import threading
 import weakref
 
@@ -43,7 +44,7 @@ class _Plan:
             m = layer._modules.get(n)
             self.mods.append((layer._modules, n, m))
             if type(m) is not type_:
-                return
+                return                       # ok stays False
         self.hooks = [h for _, _, m in self.mods for h in (m._forward_hooks, m._forward_pre_hooks)]
         a = self.args = _lib.DecodeArgs()
         self.params = []
@@ -101,19 +102,79 @@ class _Plan:
             setattr(b, n, getattr(a, n))
         self.layer_ws = {}
 
+        # what current() compares, as flat sequences for one pass in C each
+        self._mod_d, self._mod_n, self._mod_v = zip(*self.mods)
+        self._par_d, self._par_n, self._par_v, _ = zip(*self.params)
+        self._tensors = [t for t in self._par_v if t is not None]
+        self._ptrs = [t.data_ptr() for t in self._tensors]
+
     def current(self) -> bool:
-        for d, n, m in self.mods:
-            if d.get(n) is not m:
-                return False
         if not self.ok:
-            return True                      # nothing else to check: the general path runs
-        for h in self.hooks:
-            if h:
+            return all(d.get(n) is m for d, n, m in self.mods)    # nothing else to check: the general path runs
+        return (all(map(operator.is_, map(dict.get, self._mod_d, self._mod_n), self._mod_v)) and not any(self.hooks)
+                and all(map(operator.is_, map(dict.get, self._par_d, self._par_n), self._par_v))
+                and list(map(torch.Tensor.data_ptr, self._tensors)) == self._ptrs)
+
+
+class _Step:
+    """Argument block of one layer's decoding steps on one cache: everything that stays the same from token to token."""
+
+    def __init__(self, plan, layer, cache, B, dev):
+        self.plan, self.cache_tensors = plan, None
+        a = self.args = _lib.DecodeArgs()
+        ctypes.memmove(ctypes.byref(a), ctypes.byref(plan.args), ctypes.sizeof(a))
+        a.B = B
+        need = plan.ws_bytes.get(B)
+        if need is None:
+            need = plan.ws_bytes[B] = _lib.load().natsl_decode_workspace_bytes(ctypes.byref(a))
+            if need < 0:
+                raise _lib.NatslError(_lib.load().natsl_last_error().decode())
+        self.workspace = torch.empty(need, dtype=torch.uint8, device=dev)
+        a.workspace, a.workspace_bytes = self.workspace.data_ptr(), need
+        self.ref = ctypes.byref(a)
+        gdn = a.rule == _lib.RULE_GDN
+        a.own_chunk = int(layer.ops_for_incomplete_chunks == 'all')
+        a.decay = int(layer.decay_for_non_gdn_blocks if gdn else layer.decay_for_non_mamba_blocks)
+        a.neg_eigval = int(gdn and layer.allow_neg_eigval)
+        a.attn_conv = int(layer.attn_with_short_conv)
+        self.options = (layer.ops_for_incomplete_chunks, layer.attn_with_short_conv)
+
+    def bind(self, cache) -> bool:
+        """Takes over the cache's tensors (made contiguous where they are not); False if they are not the kernel's kind."""
+        a = self.args
+        B, dev = a.B, self.workspace.device
+        if cache.conv_state is None or any(t is None or t.dtype != BF16 or t.device != dev or t.shape[0] != B for t in
+                                           (*cache.conv_state, cache._k_buf, cache._v_buf)):
+            return False
+        for name in ("state", "state_block_start", "g_block", "pool_sum"):
+            t = getattr(cache, name)
+            if t is None or t.shape[0] != B or t.device != dev:
                 return False
-        for d, n, p, ptr in self.params:
-            if d.get(n) is not p or (p is not None and p.data_ptr() != ptr):
+            if t.dtype != torch.float32 or not t.is_contiguous():
+                setattr(cache, name, t.float().contiguous())
+        if not all(t.is_contiguous() for t in cache.conv_state):
+            cache.conv_state = tuple(t.contiguous() for t in cache.conv_state)
+        if cache.block_types is not None and not cache.block_types.is_contiguous():
+            cache.block_types = cache.block_types.contiguous()
+        types = cache.block_types
+        if types is not None:
+            if types.dtype not in (BF16, torch.float32):
                 return False
+            a.types_f32 = int(types.dtype == torch.float32)
+        a.conv_q, a.conv_k, a.conv_v = (t.data_ptr() for t in cache.conv_state)
+        a.state, a.start, a.g_block = cache.state.data_ptr(), cache.state_block_start.data_ptr(), cache.g_block.data_ptr()
+        a.k_cache, a.v_cache, a.cap = cache._k_buf.data_ptr(), cache._v_buf.data_ptr(), cache._k_buf.shape[1]
+        a.types = None if types is None else types.data_ptr()
+        self.cache_tensors = (cache.state, cache.state_block_start, cache.g_block, cache.pool_sum, cache.conv_state, cache._k_buf,
+                              cache._v_buf, types)
+        self.pool = cache.pool_sum.data_ptr()
         return True
+
+    def bound(self, cache) -> bool:
+        t = self.cache_tensors
+        return (t is not None and t[0] is cache.state and t[1] is cache.state_block_start and t[2] is cache.g_block
+                and t[3] is cache.pool_sum and t[4] is cache.conv_state and t[5] is cache._k_buf and t[6] is cache._v_buf
+                and t[7] is cache.block_types)
 
 
 def layer_plan(layer) -> _Plan:
@@ -130,25 +191,35 @@ def layer_plan(layer) -> _Plan:
     return p
 
 
-@torch.no_grad()
 def decode_token(layer, x: torch.Tensor, container):
     """The layer's output [B, 1, hidden] for one new token, or None where the general path has to run (which also raises
     what there is to raise).  Updates the layer's cache."""
-    if (x.dim() != 3 or x.shape[1] != 1 or x.dtype != BF16 or not x.is_cuda or x.shape[0] > MAX_BATCH or layer.layer_idx is None
-            or layer.ops_for_incomplete_chunks == 'attn' or not layer.incomplete_block_start_with_ht
-            or not (layer.use_short_conv and layer.use_gate) or torch.is_autocast_enabled() or not hasattr(container, "layer")):
+    if x.dim() != 3 or x.shape[1] != 1 or x.dtype != BF16 or not x.is_cuda or layer.layer_idx is None or not hasattr(container, "layer"):
         return None
     plan = layer_plan(layer)
-    if not plan.ok or torch.nn.modules.module._has_any_global_hook():
-        return None
-    a = plan.args
-    B, _, D = x.shape
-    dev = x.device
-    if D != a.hidden or dev != layer.q_proj.weight.device:
+    if not plan.ok:
         return None
     nbs = layer.nats_block_size
     cache = container.layer(layer.layer_idx, nbs)
     pos = cache.n_tokens
+    B = x.shape[0]
+    step = cache._step
+    if (step is None or step.plan is not plan or step.args.B != B
+            or step.options != (layer.ops_for_incomplete_chunks, layer.attn_with_short_conv)):
+        if (B > MAX_BATCH or x.shape[2] != plan.args.hidden or x.device != layer.q_proj.weight.device
+                or layer.ops_for_incomplete_chunks == 'attn' or not layer.incomplete_block_start_with_ht
+                or not (layer.use_short_conv and layer.use_gate)):
+            return None
+        step = _Step(plan, layer, cache, B, x.device)
+    if torch.is_autocast_enabled() or torch.nn.modules.module._has_any_global_hook():
+        return None
+    with torch.no_grad():
+        return _decode(layer, x, cache, step, pos, nbs)
+
+
+def _decode(layer, x, cache, step, pos: int, nbs: int):
+    a = step.args
+    B, D, dev = a.B, a.hidden, step.workspace.device
     if pos == 0:                                             # a prompt of one token: start from empty states
         f32 = dict(dtype=torch.float32, device=dev)
         cache.state = torch.zeros(B, a.H, a.K, a.V, **f32)
@@ -159,59 +230,32 @@ def decode_token(layer, x: torch.Tensor, container):
         cache._k_buf = torch.empty(B, 256, a.HQ, layer.head_attn_k_dim, dtype=BF16, device=dev)
         cache._v_buf = torch.empty(B, 256, a.HQ, layer.head_attn_v_dim, dtype=BF16, device=dev)
         cache._n_kv, cache._kv_shared = 0, False
-    elif cache._k_buf is None or cache._n_kv != pos or cache.state.shape[0] != B or cache.conv_state is None:
+    elif cache._k_buf is None or cache._n_kv != pos:
         return None
-    cq, ck, cv = cache.conv_state
-    n_done, types = pos // nbs, cache.block_types
-    if n_done and (types is None or types.shape[1] != n_done or types.dtype not in (BF16, torch.float32)):
+    n_done = pos // nbs
+    if n_done and (cache.block_types is None or cache.block_types.shape[1] != n_done):
         return None
-    for t in (cq, ck, cv, cache._k_buf, cache._v_buf):
-        if t is None or t.dtype != BF16 or t.device != dev:
-            return None
-    completes = (pos + 1) % nbs == 0
-    types_new = None
     x = x.contiguous()
-    if completes:                                            # a block's type is decided once its last token is known
+    types_new = None
+    if (pos + 1) % nbs == 0:                                 # a block's type is decided once its last token is known
         pooled = ((cache.pool_sum + x[:, 0].float()) / nbs).to(x.dtype)[:, None, :]
         types_new = layer.select(pooled).contiguous()
-        if types_new.dtype not in (BF16, torch.float32) or (types is not None and types.dtype != types_new.dtype):
+        if types_new.dtype not in (BF16, torch.float32) or (cache.block_types is not None and cache.block_types.dtype != types_new.dtype):
             return None
     cache.reserve_kv(1)
-    for name in ("state", "state_block_start", "g_block", "pool_sum"):
-        t = getattr(cache, name)
-        if t.dtype != torch.float32 or not t.is_contiguous():
-            setattr(cache, name, t.float().contiguous())
-    if not (cq.is_contiguous() and ck.is_contiguous() and cv.is_contiguous()):
-        cache.conv_state = cq, ck, cv = cq.contiguous(), ck.contiguous(), cv.contiguous()
-    if n_done and not types.is_contiguous():
-        types = cache.block_types = types.contiguous()
-    ws = cache._workspace
-    need = plan.ws_bytes.get(B)
-    a.B = B
-    if need is None:
-        need = plan.ws_bytes[B] = _lib.load().natsl_decode_workspace_bytes(ctypes.byref(a))
-        if need < 0:
-            raise _lib.NatslError(_lib.load().natsl_last_error().decode())
-    if ws is None or ws.numel() < need or ws.device != dev:
-        ws = cache._workspace = torch.empty(need, dtype=torch.uint8, device=dev)
+    if not step.bound(cache) and not step.bind(cache):
+        return None
+    cache._step = step
     out = torch.empty_like(x)
-    a.own_chunk = int(layer.ops_for_incomplete_chunks == 'all')
-    gdn = a.rule == _lib.RULE_GDN
-    a.decay = int(layer.decay_for_non_gdn_blocks if gdn else layer.decay_for_non_mamba_blocks)
-    a.neg_eigval = int(gdn and layer.allow_neg_eigval)
-    a.attn_conv = int(layer.attn_with_short_conv)
-    a.pos, a.cap, a.n_done = pos, cache._k_buf.shape[1], n_done
-    a.types_f32 = int((types_new if types is None else types).dtype == torch.float32) if (n_done or completes) else 0
+    a.pos, a.n_done = pos, n_done
     a.x, a.out = x.data_ptr(), out.data_ptr()
-    a.types, a.types_new = (types.data_ptr() if n_done else None), (types_new.data_ptr() if completes else None)
-    a.conv_q, a.conv_k, a.conv_v = cq.data_ptr(), ck.data_ptr(), cv.data_ptr()
-    a.state, a.start, a.g_block = cache.state.data_ptr(), cache.state_block_start.data_ptr(), cache.g_block.data_ptr()
-    a.pool_sum = None if completes else cache.pool_sum.data_ptr()
-    a.k_cache, a.v_cache = cache._k_buf.data_ptr(), cache._v_buf.data_ptr()
-    a.workspace, a.workspace_bytes = ws.data_ptr(), need
-    _lib.call("natsl_decode_step", ctypes.byref(a), current_stream_ptr(dev))
+    if types_new is None:
+        a.types_new, a.pool_sum = None, step.pool
+    else:
+        a.types_new, a.pool_sum, a.types_f32 = types_new.data_ptr(), None, int(types_new.dtype == torch.float32)
+    _lib.call("natsl_decode_step", step.ref, current_stream_ptr(dev))
     cache._n_kv = cache.n_tokens = pos + 1
-    if completes:
+    if types_new is not None:
         cache.append_types(types_new)
         cache.pool_sum = torch.zeros_like(cache.pool_sum)
     return out
