@@ -261,12 +261,14 @@ _hybrid_ws: dict = {}
 
 def hybrid_fwd(rule: int, q_attn, k_attn, v_attn, q, k, v, g, beta, types, nbs: int, scale_attn: float, scale_lin: float, h0,
                own_attn: bool, decay: bool, use_l2norm: bool, want_ht: bool, want_start: bool = False, last_types=None):
-    """Tables and both branches in one native call (bf16 tensors, head dims of ``walks_with_state``, own-block linear
-    attention).  -> (o_lin, o_attn, lse, ht, start, flat tables for ``tables_from_flat``)."""
+    """Tables and both branches in one native call (bf16 tensors with head dims of ``walks_with_state``, or fp32 tensors;
+    own-block linear attention).  -> (o_lin, o_attn, lse, ht, start, flat tables for ``tables_from_flat``)."""
     for t_ in (q_attn, k_attn, v_attn, q, k, v):
         _need(t_.dim() == 4, "q, k, v must be [B, T, H, D]")
         _need(t_.is_cuda and t_.device == q.device, "q, k, v of both branches must be on one CUDA device")
-        _need(t_.dtype == BF16, "the branches need q, k, v in one dtype: bf16", TypeError)
+        _need(t_.dtype == q.dtype, "q, k, v of both branches must share a dtype", TypeError)
+    fp32 = q.dtype == torch.float32
+    _need(fp32 or q.dtype == BF16, f"unsupported dtype {q.dtype} (fp32 or bf16)", TypeError)
     q_attn, k_attn, v_attn, q, k, v = (t_.contiguous() for t_ in (q_attn, k_attn, v_attn, q, k, v))
     B, T, H, K = q.shape
     V, HQ, DK, HKV, DV = v.shape[3], q_attn.shape[2], q_attn.shape[3], k_attn.shape[2], v_attn.shape[3]
@@ -293,15 +295,15 @@ def hybrid_fwd(rule: int, q_attn, k_attn, v_attn, q, k, v, g, beta, types, nbs: 
     if rule == _lib.RULE_GDN:
         _need(beta is not None, "the gated delta rule needs beta")
         _need(tuple(beta.shape) == (B, T, H) and beta.device == dev, f"beta must be [B,T,H] = {(B, T, H)} on {dev}")
+        beta = beta.float().contiguous() if fp32 else beta.contiguous()
         _need(beta.dtype in (BF16, torch.float32), "beta must be bf16 or fp32", TypeError)
-        beta = beta.contiguous()
         a.beta, a.beta_dtype = beta.data_ptr(), _dt_code(beta)
     if h0 is not None:
         h0 = h0.float().contiguous()
         _need(tuple(h0.shape) == (B, H, K, V), f"initial state must be [B,H,K,V], got {tuple(h0.shape)}")
         a.h0 = h0.data_ptr()
-    o_lin = torch.empty(B, T, H, V, dtype=BF16, device=dev)
-    o_attn = torch.empty(B, T, HQ, DV, dtype=BF16, device=dev)
+    o_lin = torch.empty(B, T, H, V, dtype=q.dtype, device=dev)
+    o_attn = torch.empty(B, T, HQ, DV, dtype=q.dtype, device=dev)
     lse = torch.empty(B, T, HQ, dtype=torch.float32, device=dev)
     ht = torch.empty(B, H, K, V, dtype=torch.float32, device=dev) if want_ht else None
     start = torch.empty(B, H, K, V, dtype=torch.float32, device=dev) if want_start else None
@@ -326,6 +328,10 @@ def hybrid_fwd(rule: int, q_attn, k_attn, v_attn, q, k, v, g, beta, types, nbs: 
     a.q_attn, a.k_attn, a.v_attn, a.q, a.k, a.v = (t_.data_ptr() for t_ in (q_attn, k_attn, v_attn, q, k, v))
     a.g, a.types, a.o_attn, a.lse, a.o_lin = g.data_ptr(), types.data_ptr(), o_attn.data_ptr(), lse.data_ptr(), o_lin.data_ptr()
     a.ht, a.hstart = _lib.ptr(ht), _lib.ptr(start)
+    if fp32:
+        a.options |= _lib.HYBRID_FP32
+        _lib.call("natsl_hybrid_forward", ctypes.byref(a), current_stream_ptr(dev))
+        return o_lin, o_attn, lse, ht, start, flat
     key = (rule, B, T, H, K, V)
     need = _hybrid_ws.get(key)
     if need is None:
@@ -402,23 +408,6 @@ def linear_recurrent_step(rule: int, q, k, v, g, beta, block_types, state, state
               new_state.data_ptr(), new_start.data_ptr(), B, T, H, types_i.shape[2], K, V, int(nbs), float(scale),
               _lib.FLAG_DECAY_SKIPPED if decay else 0, int(use_l2norm), current_stream_ptr(dev))
     return o, new_state, new_start
-
-
-def attn_fwd_fp32(q, k, v, tables: SelectionTables, scale: float, own_chunk: bool):
-    """Reference-precision softmax branch (fp32 math; fp32 or bf16 tensors).  Returns (o, lse base-2)."""
-    _need(q.dtype == k.dtype == v.dtype, "q, k, v must share a dtype", TypeError)
-    code = _dt_code(q)
-    _check_qkv(q, k, v, tables, "softmax branch (fp32 form)", same_heads=False)
-    _need(k.shape[1] == q.shape[1] and tables.T == q.shape[1], "q, k and the tables must cover the same sequence")
-    q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-    B, T, HQ, DK = q.shape
-    HKV, DV = k.shape[2], v.shape[3]
-    o = torch.empty(B, T, HQ, DV, dtype=q.dtype, device=q.device)
-    lse = torch.empty(B, T, HQ, dtype=torch.float32, device=q.device)
-    _lib.call("natsl_attn_fwd_fp32", code, q.data_ptr(), k.data_ptr(), v.data_ptr(), tables.types_i.data_ptr(),
-              o.data_ptr(), lse.data_ptr(), B, T, HQ, HKV, tables.types_i.shape[2], DK, DV, tables.nats_block_size,
-              float(scale), _lib.FLAG_ATTN_OWN_CHUNK if own_chunk else 0, current_stream_ptr(q.device))
-    return o, lse
 
 
 # ------------------------------------------------------------------------------------------------ backward

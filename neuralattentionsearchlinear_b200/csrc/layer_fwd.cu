@@ -373,6 +373,7 @@ HybridLayout hybrid_layout(const natsl_hybrid_args& a) {
     HybridLayout l = {};
     const long n = (long)a.B * a.T * a.H;
     const bool gdn = a.rule == NATSL_RULE_GDN;
+    if (a.options & NATSL_HYBRID_FP32) return l;
     l.gcs = 0;
     l.kr = up256(l.gcs + 4 * n);
     l.qr = up256(l.kr + (gdn ? 4 * n : 0));
@@ -385,13 +386,14 @@ HybridLayout hybrid_layout(const natsl_hybrid_args& a) {
 
 int check_hybrid(const natsl_hybrid_args& a) {
     NATSL_REQUIRE(a.q_attn && a.k_attn && a.v_attn && a.q && a.k && a.v && a.g && a.types && a.o_attn && a.lse && a.o_lin &&
-                      a.types_i && a.indices && a.n_blocks && a.n_chunks_lin && a.attn_n_iters && a.workspace &&
+                      a.types_i && a.indices && a.n_blocks && a.n_chunks_lin && a.attn_n_iters && (a.workspace || (a.options & NATSL_HYBRID_FP32)) &&
                       (a.rule != NATSL_RULE_GDN || a.beta),
                   NATSL_ERR_NULL, "natsl_hybrid_forward: null pointer");
     NATSL_REQUIRE(a.B > 0 && a.T > 0 && a.H > 0 && a.HN > 0 && a.H % a.HN == 0 && a.HQ > 0 && a.HQ % a.HN == 0 && a.HKV > 0 &&
                       a.HQ % a.HKV == 0 && a.nbs >= 64 && a.nbs % 64 == 0,
                   NATSL_ERR_BAD_SHAPE, "natsl_hybrid_forward: bad shape");
-    NATSL_REQUIRE(a.rule == NATSL_RULE_GDN || (a.rule == NATSL_RULE_MAMBA && a.K == 128 && a.V == 64), NATSL_ERR_UNSUPPORTED,
+    NATSL_REQUIRE(a.rule == NATSL_RULE_GDN || (a.rule == NATSL_RULE_MAMBA && ((a.K == 128 && a.V == 64) || (a.options & NATSL_HYBRID_FP32))),
+                  NATSL_ERR_UNSUPPORTED,
                   "natsl_hybrid_forward: Mamba2 is built for K = 128, V = 64 (got K=%d V=%d)", a.K, a.V);
     NATSL_REQUIRE(a.workspace_bytes >= hybrid_layout(a).total, NATSL_ERR_TOO_LARGE, "natsl_hybrid_forward: workspace of %ld bytes, %ld needed",
                   (long)a.workspace_bytes, hybrid_layout(a).total);
@@ -411,6 +413,21 @@ int hybrid_forward(const natsl_hybrid_args& a, void* types_raw, cudaStream_t st,
     float* gcs = reinterpret_cast<float*>(ws + l.gcs);
     const int TN = (a.T + a.nbs - 1) / a.nbs;
     const bool gdn = a.rule == NATSL_RULE_GDN;
+    if (a.options & NATSL_HYBRID_FP32) {
+        // reference-precision kernels; the recurrence is the longer chain and starts first
+        rc = launch_tables(a.types, a.types_dtype, types_raw, a.B, TN, a.HN, a.T, a.nbs, a.types_i, a.indices, a.n_blocks,
+                           a.n_chunks_lin, a.starting_h_idx, a.attn_n_iters, st);
+        if (rc == NATSL_OK) rc = stream_after(side, st, ev[0]);
+        if (rc == NATSL_OK)
+            rc = natsl_linear_recurrent_fwd(a.rule, NATSL_DT_F32, a.q, a.k, a.v, a.g, a.beta, a.types_i, a.h0, a.o_lin, a.ht, a.hstart, a.B,
+                                            a.T, a.H, a.HN, a.K, a.V, a.nbs, a.scale_lin, a.decay ? NATSL_FLAG_DECAY_SKIPPED : 0,
+                                            a.use_l2norm, side);
+        if (rc == NATSL_OK)
+            rc = natsl_attn_fwd_fp32(NATSL_DT_F32, a.q_attn, a.k_attn, a.v_attn, a.types_i, a.o_attn, a.lse, a.B, a.T, a.HQ, a.HKV, a.HN,
+                                     a.DK, a.DV, a.nbs, a.scale_attn, a.own_attn ? NATSL_FLAG_ATTN_OWN_CHUNK : 0, st);
+        const int join = stream_after(st, side, ev[2]);
+        return rc != NATSL_OK ? rc : join;
+    }
     rc = stream_after(side, st, ev[0]);
     // the preparation reads no tables: it starts while they are built
     if (rc == NATSL_OK && gdn) {

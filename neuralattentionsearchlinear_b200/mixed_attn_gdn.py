@@ -162,13 +162,12 @@ class NAtSMixedAttentionGDN(torch.autograd.Function):
             if not own_linear:
                 raise NotImplementedError("ops_for_incomplete_chunks='attn' is built for bf16 tensors only")
             # fp32 tensors take the reference-precision kernels (token recurrence with re-roll, fp32 softmax)
-            tables = build_selection_tables(nats_block_types, T, nats_block_size)
-            o_attn, lse = _ops.attn_fwd_fp32(q_attn, k_attn, v_attn, tables, scale_attn, own_chunk=strategy['attn'])
-            o_gdn, ht, _ = _ops.linear_recurrent(_lib.RULE_GDN, q_lattn, k_lattn, v_lattn, g, beta, tables, scale_lattn,
-                                                 initial_state_gated_delta, decay_for_non_gdn_blocks,
-                                                 lattn_use_qk_l2norm_in_kernel)
+            o_gdn, o_attn, _, ht, _, _ = _ops.hybrid_fwd(
+                _lib.RULE_GDN, q_attn, k_attn, v_attn, q_lattn, k_lattn, v_lattn, g, beta, nats_block_types, nats_block_size,
+                scale_attn, scale_lattn, initial_state_gated_delta, strategy['attn'], decay_for_non_gdn_blocks,
+                lattn_use_qk_l2norm_in_kernel, output_final_state_gated_delta)
             ctx.bwd_ok, ctx.bwd_why = False, "the backward pass is built for bf16 tensors (fp32 tensors run forward only)"
-            return o_gdn, o_attn, (ht if output_final_state_gated_delta else None)
+            return o_gdn, o_attn, ht
         if own_linear and _ops.walks_with_state(_lib.RULE_GDN, q_lattn.shape[-1], v_lattn.shape[-1], T):
             # both branches and the tables in one native call, the linear branch on a stream of its own
             o_gdn, o_attn, lse, ht, _, flat = _ops.hybrid_fwd(

@@ -47,17 +47,18 @@ class NAtSMixedAttentionMamba(torch.autograd.Function):
                                 flat, nats_block_types, T, nats_block_size, scale_attn, scale_lattn, strategy['attn'],
                                 decay_for_non_mamba_blocks, False, compute_dnats_for_invalid_blocks_linear_att)
             return o_m, o_attn, ht
-        tables = build_selection_tables(nats_block_types, T, nats_block_size)
-        lin_tables = tables if own_linear else per_chunk_tables(nats_block_types, T, nats_block_size)
         ctx.bwd_ok, ctx.bwd_why = True, ""
         if q_lattn.dtype == torch.float32:
             if not own_linear:
                 raise NotImplementedError("ops_for_incomplete_chunks='attn' is built for bf16 tensors only")
-            o_attn, _ = _ops.attn_fwd_fp32(q_attn, k_attn, v_attn, tables, scale_attn, own_chunk=strategy['attn'])
-            o_m, ht, _ = _ops.linear_recurrent(_lib.RULE_MAMBA, q_lattn, k_lattn, v_lattn, g, None, tables, scale_lattn,
-                                               initial_state_mamba, decay_for_non_mamba_blocks, False)
+            o_m, o_attn, _, ht, _, _ = _ops.hybrid_fwd(
+                _lib.RULE_MAMBA, q_attn, k_attn, v_attn, q_lattn, k_lattn, v_lattn, g, None, nats_block_types, nats_block_size,
+                scale_attn, scale_lattn, initial_state_mamba, strategy['attn'], decay_for_non_mamba_blocks, False,
+                output_final_state_mamba)
             ctx.bwd_ok, ctx.bwd_why = False, "the backward pass is built for bf16 tensors (fp32 tensors run forward only)"
-            return o_m, o_attn, (ht if output_final_state_mamba else None)
+            return o_m, o_attn, ht
+        tables = build_selection_tables(nats_block_types, T, nats_block_size)
+        lin_tables = tables if own_linear else per_chunk_tables(nats_block_types, T, nats_block_size)
         o_attn, lse = _ops.attn_fwd(q_attn, k_attn, v_attn, tables, scale_attn, own_chunk=strategy['attn'])
         o_m, ht, _ = _ops.linear_fwd(_lib.RULE_MAMBA, q_lattn, k_lattn, v_lattn, g, None, lin_tables, scale_lattn,
                                      initial_state_mamba, decay_for_non_mamba_blocks, False,
