@@ -4,350 +4,890 @@
 //     p = exp2(scale*log2(e) * q.k - lse),   delta = rowsum(o * do),   ds = p * (do.v - delta)
 // the gradients are dq = scale * ds k, dk = scale * ds^T q, dv = p^T do.
 //
-// Two kernels, both on mma.sync with bf16 operands and fp32 accumulation, both deterministic (no atomics; every
-// reduction has a fixed order):
-//   attn_bwd_dq_kernel    one CTA per (64 queries, query head): walks the visible 64-key tiles, keeps dq in
-//                         registers; also writes delta (the preprocess kernel of the reference folded in).
-//   attn_bwd_dkdv_kernel  one CTA per (64 keys, key/value head): walks the query tiles that see these keys
-//                         (rest of the own block, and every later block when the keys' block is selected) for
-//                         every query head of the group, keeps dk and dv in registers, and sums ds over the
-//                         later blocks' queries: the reference's `dnats` column for the softmax branch
-//                         (attns.py:922, 975-978), written per (64-key tile, query head).
+// Two kernels on the 5th-generation tensor cores, both deterministic (no atomics; every reduction has a fixed order).
+// Warp roles as in the forward (320 threads): warp 0 TMA producer, warp 1 MMA issuer, warps 2-9 softmax with 16 query
+// rows each, four threads per row.  All score tiles are 128 queries x 64 keys with the queries in the TMEM lanes.
+//   attn_bwd_dq_kernel    one CTA per (128 queries, query head), two per SM: walks the visible 64-key tiles, dq stays in
+//                         TMEM; also writes delta (the preprocess kernel of the reference folded in).  ds goes back to
+//                         TMEM (over do.v) as the A operand of ds k.
+//   attn_bwd_dkdv_kernel  one CTA per two selected 64-key tiles of a key/value head (walks the 128-query tiles that see
+//                         either) or per eight unselected ones (own blocks only); accumulates dk^T and dv^T (head dim in
+//                         the lanes, keys in the columns) of two key tiles in TMEM; p and ds go to shared memory as the B
+//                         operands of do^T p and q^T ds.  It also sums ds over the later blocks' queries: the reference's
+//                         `dnats` column for the softmax branch (attns.py:922, 975-978), per (64-key tile, query head).
 // `compat` reproduces the reference's default backward, which drops every own-block entry of ds and p
 // (attns.py:590-591, 631-633, 842, 884 with the flag passed at mixed_attn_gdn.py:237) while lse and delta still
 // come from the full forward.
-#include "warp_gemm.cuh"
+// Every mbarrier wait has an iteration limit; on expiry the CTA records a status, stops issuing work, still frees its
+// TMEM and returns.
+#include "attn_tc.cuh"
 #include "../../include/natsl_b200.h"
 
 namespace natsl {
 
-constexpr int AB_THREADS = 128;
 constexpr float kLog2e = 1.4426950408889634f;
-
-template <int DK, int DV>
-struct AttnBwdSmem {
-    static constexpr int fixed_a = 0;                         // dq: Q tile     dkdv: K tile
-    static constexpr int fixed_b = fixed_a + 64 * DK * 2;     // dq: dO tile    dkdv: V tile
-    static constexpr int ring_a = fixed_b + 64 * DV * 2;      // 2 x [64][DK]   dq: K tiles   dkdv: Q tiles
-    static constexpr int ring_b = ring_a + 2 * 64 * DK * 2;   // 2 x [64][DV]   dq: V tiles   dkdv: dO tiles
-    static constexpr int vec = ring_b + 2 * 64 * DV * 2;      // lse, delta: 2 x 2 x 64 floats
-    static constexpr int list = vec + 4 * 64 * 4;             // dq: visible key tiles (ints), NT entries
-    static int total(int NT) { return list + NT * 4; }
-};
 
 // ------------------------------------------------------------------------------------------------- dq
 template <int DK, int DV>
-__global__ void __launch_bounds__(AB_THREADS)
-attn_bwd_dq_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
-                   const __nv_bfloat16* __restrict__ v, const __nv_bfloat16* __restrict__ o,
-                   const __nv_bfloat16* __restrict__ d_o, const float* __restrict__ lse, const int* __restrict__ types_i,
-                   __nv_bfloat16* __restrict__ dq, float* __restrict__ delta_out, int T, int HQ, int HKV, int HN, int TN,
-                   int nbs, float scale, int own_chunk, int compat) {
-    using L = AttnBwdSmem<DK, DV>;
-    extern __shared__ __align__(128) unsigned char smem[];
+struct DqSmem {
+    // 128 / 128: one V stage (its tile is free as soon as do.v is done) keeps the CTA at half an SM's shared memory
+    static constexpr int VST = DK + DV == 256 ? 1 : 2;
+    static constexpr int q = 0;                               // DK/64 sub-tiles [128][64]; at the end the dq staging
+    static constexpr int dos = q + 128 * DK * 2;              // DV/64 sub-tiles [128][64]
+    static constexpr int k = dos + 128 * DV * 2;              // 2 stages x DK/64 sub-tiles [64][64]
+    static constexpr int v = k + 2 * 64 * DK * 2;             // VST stages x DV/64 sub-tiles [64][64]
+    static constexpr int bars = v + VST * 64 * DV * 2;
+    static constexpr int list = bars + 160;                   // visible key tiles (16 bits each), NT entries
+    static int total(int NT) { return list + ((NT * 2 + 15) & ~15); }
+};
+
+template <int DK, int DV>
+__global__ void __launch_bounds__(TC_THREADS, 2)
+attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+                   const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
+                   const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o, const float* __restrict__ lse,
+                   const int* __restrict__ types_i, __nv_bfloat16* __restrict__ dq, float* __restrict__ delta_out, int T, int HQ,
+                   int HKV, int HN, int TN, int nbs, float scale, int own, int* status) {
+    using L = DqSmem<DK, DV>;
+    constexpr int VST = L::VST;
+    constexpr uint32_t C_S = 0, C_DP = 64, C_DQ = 128;        // TMEM columns: scores; do.v, then ds; dq
+    extern __shared__ __align__(1024) unsigned char smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int gq = lane >> 2, qd = lane & 3;
-    const int NT = (T + 63) / 64;
-    const int qt = NT - 1 - blockIdx.x;                      // heavy (late) query tiles first
+    const uint32_t sbase = smem_u32(smem);
+    if ((sbase & 1023u) != 0) {
+        if (tid == 0) atomicExch(status, 2);
+        return;
+    }
+    const int it = (int)gridDim.x - 1 - (int)blockIdx.x;      // heavy (late) query tiles first
     const int hq = blockIdx.y, b = blockIdx.z;
     const int hkv = hq / (HQ / HKV), hn = hq / (HQ / HN);
+    const int q0 = it * ATT_BM;
+    const int* selp = types_i + ((long)b * TN * HN + hn) * 2;  // column 0
+    const long tstride = (long)HN * 2;
+    const uint32_t s_q = sbase + L::q, s_do = sbase + L::dos, s_k = sbase + L::k, s_v = sbase + L::v;
+    const uint32_t bar0 = sbase + L::bars;
+    const uint32_t bar_q = bar0, bar_k_full = bar0 + 8, bar_k_empty = bar0 + 24, bar_v_full = bar0 + 40, bar_v_empty = bar0 + 56,
+                   bar_s = bar0 + 72, bar_dp = bar0 + 80, bar_s_free = bar0 + 88, bar_ds = bar0 + 96, bar_done = bar0 + 104;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::bars + 112);
+    int* s_count = reinterpret_cast<int*>(smem + L::bars + 116);
+    uint16_t* s_list = reinterpret_cast<uint16_t*>(smem + L::list);
+    const int span0 = (q0 / nbs) * nbs / 64;                  // first key tile of the own span
     const int cpb = nbs / 64;
-    const int bq = qt / cpb;                                 // block of the queries
-    const int valid_q = min(64, T - qt * 64);
-    const long tokq = (long)b * T + (long)qt * 64;
 
-    unsigned char* qs_p = smem + L::fixed_a;
-    unsigned char* dos_p = smem + L::fixed_b;
-    const uint32_t qs = smem_u32(qs_p), dos = smem_u32(dos_p);
-    const uint32_t kring = smem_u32(smem + L::ring_a), vring = smem_u32(smem + L::ring_b);
-    float* s_lse = reinterpret_cast<float*>(smem + L::vec);
-    float* s_delta = s_lse + 64;
-    int* s_list = reinterpret_cast<int*>(smem + L::list);
-    __shared__ int s_count;
-
-    // ---- Q, dO, and O (staged in the first V buffer) of the query tile
-    load_tile_async<64, DK, AB_THREADS>(qs, q + (tokq * HQ + hq) * DK, (long)HQ * DK, valid_q, tid);
-    load_tile_async<64, DV, AB_THREADS>(dos, d_o + (tokq * HQ + hq) * DV, (long)HQ * DV, valid_q, tid);
-    load_tile_async<64, DV, AB_THREADS>(vring, o + (tokq * HQ + hq) * DV, (long)HQ * DV, valid_q, tid);
-    cp_async_commit();
-    if (tid < 64) s_lse[tid] = tid < valid_q ? lse[(tokq + tid) * HQ + hq] : 0.f;
-
-    // ---- visible key tiles: sub-tiles of the selected blocks before the query's block, then the own block's
-    // sub-tiles up to the query tile (warp 0 compacts with ballots)
-    if (warp == 0) {
-        const int* sel_p = types_i + ((long)b * TN * HN + hn) * 2;           // column 0, stride HN * 2 per block
+    if (tid == 0) {
+        mbar_init(bar_q, 1);
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(bar_k_full + 8 * i, 1);
+            mbar_init(bar_k_empty + 8 * i, 1);
+            mbar_init(bar_v_full + 8 * i, 1);
+            mbar_init(bar_v_empty + 8 * i, 1);
+        }
+        mbar_init(bar_s, 1);
+        mbar_init(bar_dp, 1);
+        mbar_init(bar_s_free, 8);                             // one arrival per softmax warp
+        mbar_init(bar_ds, 8);
+        mbar_init(bar_done, 1);
+        mbar_fence_init();
+        mbar_expect_tx(bar_q, 128 * (DK + DV) * 2);
+#pragma unroll
+        for (int sub = 0; sub < DK / 64; ++sub) tma_load_4d(s_q + sub * 16384, &map_q, sub * 64, hq, q0, b, bar_q);
+#pragma unroll
+        for (int sub = 0; sub < DV / 64; ++sub) tma_load_4d(s_do + sub * 16384, &map_do, sub * 64, hq, q0, b, bar_q);
+    }
+    if (warp == 1) tmem_alloc(smem_u32(tmem_slot), TC_TMEM_COLS);
+    if (warp == 2) {
+        // visible key tiles in ascending order: sub-tiles of selected blocks before the own span, then the own span
+        // (whose entries are masked per element)
+        const int n_cand = min((q0 + ATT_BM + 63) / 64, (T + 63) / 64);
         int count = 0;
-        const int n_cand = qt + 1;
         for (int base = 0; base < n_cand; base += 32) {
             const int kt = base + lane;
-            bool vis = false;
-            if (kt < n_cand) {
-                const int c = kt / cpb;
-                vis = (c == bq) ? (own_chunk && !compat) : (sel_p[(long)c * HN * 2] != 0);
-            }
+            const bool vis = kt < n_cand && (kt >= span0 || selp[(long)(kt / cpb) * tstride] != 0);
             const unsigned m = __ballot_sync(0xffffffffu, vis);
-            if (vis) s_list[count + __popc(m & ((1u << lane) - 1))] = kt;
+            if (vis) s_list[count + __popc(m & ((1u << lane) - 1))] = (uint16_t)kt;
             count += __popc(m);
         }
-        if (lane == 0) s_count = count;
+        if (lane == 0) *s_count = count;
     }
-    cp_async_wait<0>();
+    tc_fence_before();
     __syncthreads();
-    const int n_tiles = s_count;
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    const int n_tiles = *s_count;                             // >= 1: the own span is never empty
 
-    // ---- delta = rowsum(o * do)
-    {
-        const unsigned char* os_p = smem + L::ring_b;
-        constexpr int CPR = DV / 8;
-        for (int r = warp * 16; r < warp * 16 + 16; ++r) {
-            float s = 0.f;
-            for (int cc = lane; cc < CPR; cc += 32) {
-                const uint4 a = *reinterpret_cast<const uint4*>(os_p + swz<DV * 2>(r, cc));
-                const uint4 d = *reinterpret_cast<const uint4*>(dos_p + swz<DV * 2>(r, cc));
-                const uint32_t* aw = reinterpret_cast<const uint32_t*>(&a);
-                const uint32_t* dw = reinterpret_cast<const uint32_t*>(&d);
+    if (warp == 0) {
+        // ------------------------------------------------------------ TMA producer
+        bool ok = true;
+        for (int j = 0; ok && j < n_tiles; ++j) {
+            const int ks = j & 1, vs = j % VST, t0 = s_list[j] * 64;
+            if (j >= 2) ok = __all_sync(0xffffffffu, mbar_wait(bar_k_empty + ks * 8, ((j >> 1) - 1) & 1, status));
+            if (!ok) break;
+            if (lane == 0) {
+                mbar_expect_tx(bar_k_full + ks * 8, 64 * DK * 2);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const float2 x = unpack_bf16(aw[j]), y = unpack_bf16(dw[j]);
-                    s += x.x * y.x + x.y * y.y;
+                for (int sub = 0; sub < DK / 64; ++sub)
+                    tma_load_4d(s_k + ks * (64 * DK * 2) + sub * 8192, &map_k, sub * 64, hkv, t0, b, bar_k_full + ks * 8);
+#pragma unroll
+                for (int sub = 0; sub < DV / 64; ++sub) tma_prefetch_4d(&map_v, sub * 64, hkv, t0, b);
+            }
+            __syncwarp();
+            if (j >= VST) ok = __all_sync(0xffffffffu, mbar_wait(bar_v_empty + vs * 8, ((j / VST) - 1) & 1, status));
+            if (!ok) break;
+            if (lane == 0) {
+                mbar_expect_tx(bar_v_full + vs * 8, 64 * DV * 2);
+#pragma unroll
+                for (int sub = 0; sub < DV / 64; ++sub)
+                    tma_load_4d(s_v + vs * (64 * DV * 2) + sub * 8192, &map_v, sub * 64, hkv, t0, b, bar_v_full + vs * 8);
+            }
+            __syncwarp();
+        }
+    } else if (warp == 1) {
+        // ------------------------------------------------------------ MMA issuer
+        constexpr uint32_t id_s = umma_idesc_bf16(128, 64, false);
+        constexpr uint32_t id_dq = umma_idesc_bf16(128, DK, true);
+        auto issue_s = [&](int j) {                           // S = Q K_j^T
+            const uint32_t kt = s_k + (j & 1) * (64 * DK * 2);
+#pragma unroll
+            for (int kk = 0; kk < DK / 16; ++kk)
+                umma_ss(tmem + C_S, umma_desc(s_q + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
+                        umma_desc(kt + (kk >> 2) * 8192 + (kk & 3) * 32, 16, 1024), id_s, kk > 0);
+            umma_commit(bar_s);
+        };
+        auto issue_dp = [&](int j) {                          // dO V_j^T
+            const uint32_t vt = s_v + (j % VST) * (64 * DV * 2);
+#pragma unroll
+            for (int kk = 0; kk < DV / 16; ++kk)
+                umma_ss(tmem + C_DP, umma_desc(s_do + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
+                        umma_desc(vt + (kk >> 2) * 8192 + (kk & 3) * 32, 16, 1024), id_s, kk > 0);
+            umma_commit(bar_dp);
+            umma_commit(bar_v_empty + (j % VST) * 8);
+        };
+        bool ok = __all_sync(0xffffffffu, mbar_wait(bar_q, 0, status));
+        if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_k_full, 0, status));
+        if (ok && lane == 0) {
+            tc_fence_after();
+            issue_s(0);
+        }
+        __syncwarp();
+        if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_v_full, 0, status));
+        if (ok && lane == 0) {
+            tc_fence_after();
+            issue_dp(0);
+        }
+        __syncwarp();
+        for (int j = 0; ok && j < n_tiles; ++j) {
+            const int jn = j + 1;
+            if (jn < n_tiles) {                               // the next scores as soon as these have been read
+                ok = __all_sync(0xffffffffu, mbar_wait(bar_k_full + (jn & 1) * 8, (jn >> 1) & 1, status));
+                if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_s_free, j & 1, status));
+                if (!ok) break;
+                if (lane == 0) {
+                    tc_fence_after();
+                    issue_s(jn);
+                }
+                __syncwarp();
+            }
+            ok = __all_sync(0xffffffffu, mbar_wait(bar_ds, j & 1, status));
+            if (!ok) break;
+            if (lane == 0) {
+                tc_fence_after();
+                const uint32_t kt = s_k + (j & 1) * (64 * DK * 2);
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk)
+                    umma_ts(tmem + C_DQ, tmem + C_DP + kk * 8, umma_desc(kt + kk * 2048, 8192, 1024), id_dq, (j > 0 || kk > 0) ? 1u : 0u);
+                umma_commit(jn < n_tiles ? bar_k_empty + (j & 1) * 8 : bar_done);
+            }
+            __syncwarp();
+            if (jn < n_tiles) {
+                ok = __all_sync(0xffffffffu, mbar_wait(bar_v_full + (jn % VST) * 8, (jn / VST) & 1, status));
+                if (!ok) break;
+                if (lane == 0) {
+                    tc_fence_after();
+                    issue_dp(jn);                             // behind ds k in the tensor pipe: ds may be overwritten
+                }
+                __syncwarp();
+            }
+        }
+    } else {
+        // ------------------------------------------------------------ softmax (8 warps)
+        const int quad = warp & 3, half = (warp - 2) >> 2;
+        const int row_a = quad * 32 + half * 16 + (lane >> 2), row_b = row_a + 8;
+        const int cq = (lane & 3) * 2;
+        const int t_a = q0 + row_a, t_b = q0 + row_b;
+        const uint32_t t_rows = tmem + ((uint32_t)(quad * 32 + half * 16) << 16);
+        const float sl2 = scale * kLog2e;
+        // delta = rowsum(o * do): four threads per row
+        auto row_delta = [&](int t) -> float {
+            float s = 0.f;
+            if (t < T) {
+                const long off = (((long)b * T + t) * HQ + hq) * DV + (lane & 3) * 8;
+#pragma unroll
+                for (int c = 0; c < DV / 32; ++c) {
+                    const uint4 x = *reinterpret_cast<const uint4*>(o + off + c * 32);
+                    const uint4 y = *reinterpret_cast<const uint4*>(d_o + off + c * 32);
+                    const uint32_t* xw = reinterpret_cast<const uint32_t*>(&x);
+                    const uint32_t* yw = reinterpret_cast<const uint32_t*>(&y);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const float2 u = unpack_bf16(xw[e]), w = unpack_bf16(yw[e]);
+                        s += u.x * w.x + u.y * w.y;
+                    }
                 }
             }
-            s = warp_sum(s);
-            if (lane == 0) {
-                s_delta[r] = s;
-                if (r < valid_q) delta_out[(tokq + r) * HQ + hq] = s;
+            s += __shfl_xor_sync(0xffffffffu, s, 1);
+            s += __shfl_xor_sync(0xffffffffu, s, 2);
+            return s;
+        };
+        const float del_a = row_delta(t_a), del_b = row_delta(t_b);
+        float lse_a = 0.f, lse_b = 0.f;
+        if (t_a < T) lse_a = lse[((long)b * T + t_a) * HQ + hq];
+        if (t_b < T) lse_b = lse[((long)b * T + t_b) * HQ + hq];
+        if ((lane & 3) == 0) {
+            if (t_a < T) delta_out[((long)b * T + t_a) * HQ + hq] = del_a;
+            if (t_b < T) delta_out[((long)b * T + t_b) * HQ + hq] = del_b;
+        }
+        bool ok = true;
+        for (int j = 0; j < n_tiles; ++j) {
+            ok = __all_sync(0xffffffffu, mbar_wait(bar_s, j & 1, status));
+            if (!ok) break;
+            tc_fence_after();
+            uint32_t sr[32], pr[16];
+            tmem_ld_16x256b_x8(t_rows + C_S, sr);
+            tmem_ld_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_s_free);
+            const int kt = s_list[j];
+            if (kt >= span0) {
+                // own-span tile: per row the visible keys are columns [0, limit] (attn_walk.cuh: visible()); an invisible
+                // score becomes -inf, its p zero
+                const int s0 = kt * 64, blk = s0 / nbs, blk_end = (blk + 1) * nbs;
+                const bool selb = selp[(long)blk * tstride] != 0;
+                int lim_a = T - 1 - s0, lim_b = lim_a;
+                if (t_a < blk_end) lim_a = own ? min(lim_a, t_a - s0) : -1;
+                else if (!selb) lim_a = -1;
+                if (t_b < blk_end) lim_b = own ? min(lim_b, t_b - s0) : -1;
+                else if (!selb) lim_b = -1;
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const int c = 8 * k + cq + e;
+                        if (c > lim_a) sr[4 * k + e] = 0xff800000u;
+                        if (c > lim_b) sr[4 * k + 2 + e] = 0xff800000u;
+                    }
+            }
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    sr[4 * k + e] = __float_as_uint(ex2(fmaf(__uint_as_float(sr[4 * k + e]), sl2, (e >> 1) ? -lse_b : -lse_a)));
+            ok = __all_sync(0xffffffffu, mbar_wait(bar_dp, j & 1, status));
+            if (!ok) break;
+            tc_fence_after();
+            uint32_t dr[32];
+            tmem_ld_16x256b_x8(t_rows + C_DP, dr);
+            tmem_ld_wait();
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                pr[2 * k] = pack_bf16(__uint_as_float(sr[4 * k]) * (__uint_as_float(dr[4 * k]) - del_a),
+                                      __uint_as_float(sr[4 * k + 1]) * (__uint_as_float(dr[4 * k + 1]) - del_a));
+                pr[2 * k + 1] = pack_bf16(__uint_as_float(sr[4 * k + 2]) * (__uint_as_float(dr[4 * k + 2]) - del_b),
+                                          __uint_as_float(sr[4 * k + 3]) * (__uint_as_float(dr[4 * k + 3]) - del_b));
+            }
+            tmem_st_16x128b_x8(t_rows + C_DP, pr);            // ds over the first 32 columns of do.v
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_ds);
+        }
+        if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_done, 0, status));
+        unsigned char* stage = smem + L::q;
+        if (ok) {
+            tc_fence_after();
+#pragma unroll 1
+            for (int c0 = 0; c0 < DK; c0 += 64) {
+                uint32_t r[32];
+                tmem_ld_16x256b_x8(t_rows + C_DQ + c0, r);
+                tmem_ld_wait();
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const int chunk = (c0 >> 3) + k;
+                    *reinterpret_cast<uint32_t*>(stage + swz<DK * 2>(row_a, chunk) + (lane & 3) * 4) =
+                        pack_bf16(__uint_as_float(r[4 * k]) * scale, __uint_as_float(r[4 * k + 1]) * scale);
+                    *reinterpret_cast<uint32_t*>(stage + swz<DK * 2>(row_b, chunk) + (lane & 3) * 4) =
+                        pack_bf16(__uint_as_float(r[4 * k + 2]) * scale, __uint_as_float(r[4 * k + 3]) * scale);
+                }
             }
         }
+        asm volatile("bar.sync 1, 256;" ::: "memory");       // every softmax warp reaches it, also after a failed wait
+        if (ok)
+            store_tile<128, DK, 256>(stage, dq + (((long)b * T + q0) * HQ + hq) * DK, (long)HQ * DK, min(128, T - q0), tid - 64);
     }
-    __syncthreads();                                          // the O staging buffer is free again
-
-    auto issue = [&](int i) {
-        if (i < n_tiles) {
-            const int kt = s_list[i];
-            const int valid_k = min(64, T - kt * 64);
-            const long tokk = (long)b * T + (long)kt * 64;
-            load_tile_async<64, DK, AB_THREADS>(kring + (i & 1) * 64 * DK * 2, k + (tokk * HKV + hkv) * DK, (long)HKV * DK,
-                                                valid_k, tid);
-            load_tile_async<64, DV, AB_THREADS>(vring + (i & 1) * 64 * DV * 2, v + (tokk * HKV + hkv) * DV, (long)HKV * DV,
-                                                valid_k, tid);
-        }
-        cp_async_commit();
-    };
-
-    float acc_dq[DK / 8][4];
-    zero_acc(acc_dq);
-    const int r0 = warp * 16;
-    const int ia = r0 + gq, ib = ia + 8;
-    const float lse_a = s_lse[ia], lse_b = s_lse[ib], del_a = s_delta[ia], del_b = s_delta[ib];
-    const float sl2 = scale * kLog2e;
-
-    issue(0);
-    for (int i = 0; i < n_tiles; ++i) {
-        issue(i + 1);
-        cp_async_wait<1>();
-        __syncthreads();
-        const int kt = s_list[i];
-        const uint32_t ks = kring + (i & 1) * 64 * DK * 2, vs = vring + (i & 1) * 64 * DV * 2;
-        float acc_s[8][4], acc_p[8][4];
-        zero_acc(acc_s);
-        zero_acc(acc_p);
-        warp_gemm<DK * 2, A_ROW, DK * 2, B_NK, 8>(acc_s, qs, r0, ks, 0, 0, DK, lane);
-        warp_gemm<DV * 2, A_ROW, DV * 2, B_NK, 8>(acc_p, dos, r0, vs, 0, 0, DV, lane);
-        const bool diag = kt == qt;
-        const int kmax = T - kt * 64;                         // keys j >= kmax do not exist
-#pragma unroll
-        for (int nt = 0; nt < 8; ++nt)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int i_row = (e >> 1) ? ib : ia;
-                const int j = nt * 8 + qd * 2 + (e & 1);
-                const bool ok = j < kmax && (!diag || j <= i_row);
-                const float p = exp2f(acc_s[nt][e] * sl2 - ((e >> 1) ? lse_b : lse_a));
-                acc_s[nt][e] = ok ? p * (acc_p[nt][e] - ((e >> 1) ? del_b : del_a)) : 0.f;
-            }
-        uint32_t dsf[4][4];
-        acc_to_afrag<8>(acc_s, dsf);
-        warp_gemm_ra<4, DK * 2, B_KN, DK / 8>(acc_dq, dsf, ks, 0, 0, lane);
-        __syncthreads();                                      // every warp is done with this stage before it is refilled
-    }
-    cp_async_wait<0>();
-
-    // ---- dq = scale * acc, staged through the Q tile
-#pragma unroll
-    for (int nt = 0; nt < DK / 8; ++nt)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) acc_dq[nt][e] *= scale;
-    store_acc_bf16<DK * 2, DK / 8>(qs_p, acc_dq, r0, 0, lane);
+    tc_fence_before();
     __syncthreads();
-    store_tile<64, DK, AB_THREADS>(qs_p, dq + (tokq * HQ + hq) * DK, (long)HQ * DK, valid_q, tid);
+    if (warp == 1) tmem_dealloc(tmem, TC_TMEM_COLS);
 }
 
 // ------------------------------------------------------------------------------------------------- dk, dv
+constexpr int BKV_MAXG = 16;
 template <int DK, int DV>
-__global__ void __launch_bounds__(AB_THREADS)
-attn_bwd_dkdv_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
-                     const __nv_bfloat16* __restrict__ v, const __nv_bfloat16* __restrict__ d_o,
-                     const float* __restrict__ lse, const float* __restrict__ delta, const int* __restrict__ types_i,
-                     __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv, float* __restrict__ dnats_part, int T,
-                     int HQ, int HKV, int HN, int TN, int nbs, float scale, int own_chunk, int compat) {
-    using L = AttnBwdSmem<DK, DV>;
-    extern __shared__ __align__(128) unsigned char smem[];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int gq = lane >> 2, qd = lane & 3;
-    const int NT = (T + 63) / 64;
-    const int kt = blockIdx.x;                               // early key tiles are seen by the most queries: first
-    const int hkv = blockIdx.y, b = blockIdx.z;
-    const int G = HQ / HKV;
-    const int cpb = nbs / 64;
-    const int c = kt / cpb;                                  // block of the keys
-    const int valid_k = min(64, T - kt * 64);
-    const long tokk = (long)b * T + (long)kt * 64;
-    const int own_end = min((c + 1) * cpb, NT);              // query tiles [kt, own_end) share the keys' block
-    const int n_own = (own_chunk && !compat) ? own_end - kt : 0;
+struct DkvSmem {
+    // A stage is [do | q], both as [128][64] sub-tiles.  With a head dim of 64 the M = 128 products read the 64 columns
+    // behind the tile as well (the next sub-tile, always inside the buffers) and those result rows are never used.
+    static constexpr int stage_bytes = 128 * (DK + DV) * 2;
+    static constexpr int stage = 0;                           // 2 stages
+    static constexpr int kv = stage + 2 * stage_bytes;        // per key tile: DK/64 + DV/64 sub-tiles [64][64]
+    static constexpr int kv_bytes = 64 * (DK + DV) * 2;
+    static constexpr int p = kv + 2 * kv_bytes;               // p [128 queries][64 keys]
+    static constexpr int ds = p + 16384;                      // ds, same layout
+    static constexpr int dn = ds + 16384;                     // dnats parts [2 tiles][16 heads][8 warps]
+    static constexpr int last = dn + 2 * BKV_MAXG * 8 * 4;    // last query tile [2 tiles][16 heads]
+    static constexpr int tiles = last + 2 * BKV_MAXG * 4;     // key tiles of this CTA [8]
+    static constexpr int bars = tiles + 32;
+    static constexpr int total = bars + 96;
+    static_assert(total <= 227 * 1024, "one CTA per SM");
+};
 
-    unsigned char* ks_p = smem + L::fixed_a;
-    unsigned char* vs_p = smem + L::fixed_b;
-    const uint32_t ks = smem_u32(ks_p), vs = smem_u32(vs_p);
-    const uint32_t qring = smem_u32(smem + L::ring_a), doring = smem_u32(smem + L::ring_b);
-    float* s_vec = reinterpret_cast<float*>(smem + L::vec);  // [stage][lse 64 | delta 64]
-    __shared__ float s_dn[16][4];                            // per query head of the group and warp: fixed summation order
-    __shared__ int s_npast[16];
-
-    load_tile_async<64, DK, AB_THREADS>(ks, k + (tokk * HKV + hkv) * DK, (long)HKV * DK, valid_k, tid);
-    load_tile_async<64, DV, AB_THREADS>(vs, v + (tokk * HKV + hkv) * DV, (long)HKV * DV, valid_k, tid);
-    cp_async_commit();
-    if (tid < 16) {
-#pragma unroll
-        for (int wv = 0; wv < 4; ++wv) s_dn[tid][wv] = 0.f;
-        int np = 0;
-        if (tid < G) {
-            const int hq = hkv * G + tid;
-            const int hn = hq / (HQ / HN);
-            const bool sel = types_i[(((long)b * TN + c) * HN + hn) * 2] != 0;
-            np = sel ? max(0, NT - own_end) : 0;
-        }
-        s_npast[tid] = np;
+// What a CTA walks: for every query head of the group the query tiles that see either key tile, and inside a query
+// tile the key tiles that it sees.  All roles step through the same sequence.
+struct DkvWalk {
+    const int* last;                                          // shared memory [2][16]; -1: no query tile
+    int first[2];
+    int G;
+    int gi, qt, u;
+    __device__ __forceinline__ bool active(int uu) const { return qt >= first[uu] && qt <= last[uu * BKV_MAXG + gi]; }
+    __device__ __forceinline__ void enter() {                 // first query tile of head gi
+        const int l0 = last[gi], l1 = last[BKV_MAXG + gi];
+        qt = min(l0 >= first[0] ? first[0] : 0x7fffffff, l1 >= first[1] ? first[1] : 0x7fffffff);
+        u = 0;
     }
-    __syncthreads();
-    int total = 0;
-    for (int gi = 0; gi < G; ++gi) total += n_own + s_npast[gi];
-
-    // flat iteration index -> (query head of the group, query tile, own-block flag)
-    auto decode = [&](int idx, int& gi, int& qt, bool& own) {
+    // moves to the first (gi, qt, u) at or after the current one; false at the end
+    __device__ __forceinline__ bool settle() {
+        while (gi < G) {
+            const int hi = max(last[gi], last[BKV_MAXG + gi]);
+            for (; qt <= hi; ++qt, u = 0) {
+                if (u == 0 && active(0)) return true;
+                if (u <= 1 && active(1)) {
+                    u = 1;
+                    return true;
+                }
+            }
+            if (++gi < G) enter();
+        }
+        return false;
+    }
+    __device__ __forceinline__ bool begin() {
         gi = 0;
-        while (true) {
-            const int n = n_own + s_npast[gi];
-            if (idx < n) break;
-            idx -= n;
-            ++gi;
-        }
-        own = idx < n_own;
-        qt = own ? kt + idx : own_end + (idx - n_own);
-    };
-    auto issue = [&](int i) {
-        if (i < total) {
-            int gi, qt;
-            bool own;
-            decode(i, gi, qt, own);
-            const int hq = hkv * G + gi;
-            const int valid_q = min(64, T - qt * 64);
-            const long tokq = (long)b * T + (long)qt * 64;
-            load_tile_async<64, DK, AB_THREADS>(qring + (i & 1) * 64 * DK * 2, q + (tokq * HQ + hq) * DK, (long)HQ * DK,
-                                                valid_q, tid);
-            load_tile_async<64, DV, AB_THREADS>(doring + (i & 1) * 64 * DV * 2, d_o + (tokq * HQ + hq) * DV, (long)HQ * DV,
-                                                valid_q, tid);
-            if (tid < 64) {
-                const bool okr = tid < valid_q;
-                const long gi_ = (tokq + (okr ? tid : 0)) * HQ + hq;
-                float* dst = s_vec + (i & 1) * 128;
-                dst[tid] = okr ? lse[gi_] : 0.f;
-                dst[64 + tid] = okr ? delta[gi_] : 0.f;
-            }
-        }
-        cp_async_commit();
-    };
-
-    float acc_dk[DK / 8][4], acc_dv[DV / 8][4];
-    zero_acc(acc_dk);
-    zero_acc(acc_dv);
-    const int r0 = warp * 16;
-    const int ja = r0 + gq, jb = ja + 8;                      // key rows of this lane
-    const float sl2 = scale * kLog2e;
-    float dn_acc = 0.f;
-    int dn_gi = 0;
-
-    issue(0);
-    for (int i = 0; i < total; ++i) {
-        issue(i + 1);
-        cp_async_wait<1>();
-        __syncthreads();
-        int gi, qt;
-        bool own;
-        decode(i, gi, qt, own);
-        if (gi != dn_gi) {                                    // uniform over the CTA
-            dn_acc = warp_sum(dn_acc);
-            if (lane == 0) s_dn[dn_gi][warp] += dn_acc;
-            dn_acc = 0.f;
-            dn_gi = gi;
-        }
-        const uint32_t qs = qring + (i & 1) * 64 * DK * 2, dos = doring + (i & 1) * 64 * DV * 2;
-        const float* v_lse = s_vec + (i & 1) * 128;
-        const float* v_del = v_lse + 64;
-        // transposed score tile: rows = keys, columns = queries
-        float acc_s[8][4], acc_p[8][4];
-        zero_acc(acc_s);
-        zero_acc(acc_p);
-        warp_gemm<DK * 2, A_ROW, DK * 2, B_NK, 8>(acc_s, ks, r0, qs, 0, 0, DK, lane);
-        warp_gemm<DV * 2, A_ROW, DV * 2, B_NK, 8>(acc_p, vs, r0, dos, 0, 0, DV, lane);
-        const bool diag = qt == kt;
-        const int qmax = T - qt * 64;
-#pragma unroll
-        for (int nt = 0; nt < 8; ++nt)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int j = (e >> 1) ? jb : ja;             // key
-                const int iq = nt * 8 + qd * 2 + (e & 1);     // query
-                const bool ok = iq < qmax && j < valid_k && (!diag || j <= iq);
-                const float p = ok ? exp2f(acc_s[nt][e] * sl2 - v_lse[iq]) : 0.f;
-                const float ds = p * (acc_p[nt][e] - v_del[iq]);
-                acc_s[nt][e] = p;
-                acc_p[nt][e] = ds;
-                if (!own) dn_acc += ds;
-            }
-        uint32_t pf[4][4], dsf[4][4];
-        acc_to_afrag<8>(acc_s, pf);
-        acc_to_afrag<8>(acc_p, dsf);
-        warp_gemm_ra<4, DV * 2, B_KN, DV / 8>(acc_dv, pf, dos, 0, 0, lane);
-        warp_gemm_ra<4, DK * 2, B_KN, DK / 8>(acc_dk, dsf, qs, 0, 0, lane);
-        __syncthreads();
+        enter();
+        return settle();
     }
-    cp_async_wait<0>();
-    dn_acc = warp_sum(dn_acc);
-    if (lane == 0 && total > 0) s_dn[dn_gi][warp] += dn_acc;
+    __device__ __forceinline__ bool next() {
+        ++u;
+        return settle();
+    }
+    __device__ __forceinline__ bool next_query() {
+        u = 2;
+        return settle();
+    }
+    __device__ __forceinline__ bool first_of_query() const { return u == 0 || !active(0); }
+    __device__ __forceinline__ bool last_of_query() const { return u == 1 || !active(1); }
+};
 
-    // ---- stores: dk = scale * acc, dv; staged through the (idle) ring buffers
-    unsigned char* st_k = smem + L::ring_a;
-    unsigned char* st_v = smem + L::ring_b;
+// The key tiles of unselected blocks, one after the other: only queries of their own block see them.
+constexpr int BKV_OWN = 8;                                    // tiles per CTA
+struct OwnWalk {
+    const volatile int* tiles;
+    int n, G, nbs, NTq;
+    int u, gi, qt, last;
+    __device__ __forceinline__ void enter() {
+        const int k0 = tiles[u] * 64;
+        qt = k0 / ATT_BM;
+        last = min(((k0 / nbs + 1) * nbs - 1) / ATT_BM, NTq - 1);
+    }
+    __device__ __forceinline__ bool begin() {
+        u = gi = 0;
+        if (n > 0) enter();
+        return n > 0;
+    }
+    __device__ __forceinline__ bool next() {
+        if (++qt > last) {
+            if (++gi == G) {
+                gi = 0;
+                if (++u == n) return false;
+            }
+            enter();
+        }
+        return true;
+    }
+    __device__ __forceinline__ bool first_of_tile() const { return gi == 0 && qt == tiles[u] * 64 / ATT_BM; }
+};
+
+// Heads whose CTAs are interleaved, heaviest first: the last CTAs to start are then light ones, and q and do of that many
+// heads (2 MB each at 4096 x 128) stay in L2 for the CTAs of a head that run at the same time.
+constexpr int BKV_HEADS = 32;
+
+template <int DK, int DV>
+__global__ void __launch_bounds__(TC_THREADS, 1)
+attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+                     const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
+                     const float* __restrict__ lse, const float* __restrict__ delta, const int* __restrict__ types_i,
+                     __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv, float* __restrict__ dnats_part, int T, int HQ,
+                     int HKV, int HN, int TN, int nbs, float scale, int own, int heads, int ctas_per_head, int* status) {
+    using L = DkvSmem<DK, DV>;
+    // TMEM: scores 2 x 64 columns, do.v 2 x 64, then two accumulator pairs dv^T (64), dk^T (64)
+    constexpr uint32_t C_S = 0, C_DP = 128, C_ACC = 256;
+    extern __shared__ __align__(1024) unsigned char smem[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t sbase = smem_u32(smem);
+    if ((sbase & 1023u) != 0) {
+        if (tid == 0) atomicExch(status, 2);
+        return;
+    }
+    const int hbase = (int)blockIdx.x / (BKV_HEADS * ctas_per_head) * BKV_HEADS, hcount = min(BKV_HEADS, heads - hbase);
+    const int within = (int)blockIdx.x - hbase * ctas_per_head;
+    const int item = within / hcount, head = hbase + within % hcount;
+    const int hkv = head % HKV, b = head / HKV;
+    const int G = HQ / HKV, cpb = nbs / 64;
+    const int NT = (T + 63) / 64, NTq = (T + ATT_BM - 1) / ATT_BM;
+    float* s_dn = reinterpret_cast<float*>(smem + L::dn);
+    int* s_last = reinterpret_cast<int*>(smem + L::last);
+    volatile int* s_tile = reinterpret_cast<volatile int*>(smem + L::tiles);
+    const uint32_t bar0 = sbase + L::bars;
+    const uint32_t bar_full = bar0, bar_empty = bar0 + 16, bar_kv = bar0 + 32, bar_s = bar0 + 48, bar_p = bar0 + 64, bar_acc = bar0 + 72;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::bars + 80);
+    volatile int* s_nsel = reinterpret_cast<volatile int*>(smem + L::bars + 84);
+
+    if (tid == 0) {
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(bar_full + 8 * i, 1);
+            mbar_init(bar_empty + 8 * i, 1);
+            mbar_init(bar_kv + 8 * i, 1);
+            mbar_init(bar_s + 8 * i, 1);
+        }
+        mbar_init(bar_p, 8);                                  // one arrival per softmax warp
+        mbar_init(bar_acc, 1);
+        mbar_fence_init();
+    }
+    for (int i = tid; i < 2 * BKV_MAXG * 8; i += TC_THREADS) s_dn[i] = 0.f;
+    if (warp == 2) {
+        // Key tiles in the order: those of selected blocks (of any head of the group), then the others.  The first
+        // ceil(n / 2) CTAs of a head take two selected tiles each: neighbours see nearly the same queries, so the pair
+        // shares the loads of q and do (64 KB per 128 x 64 scores of one tile).  The next ones take eight unselected
+        // tiles, the rest of the CTAs have nothing to do.
+        auto selected = [&](int kt) -> bool {
+            bool s = false;
+            for (int gi = 0; gi < G; ++gi) s |= types_i[(((long)b * TN + kt / cpb) * HN + (hkv * G + gi) / (HQ / HN)) * 2] != 0;
+            return s;
+        };
+        constexpr int KEEP = 4;                               // ballots kept from the counting pass (8192 tokens)
+        unsigned kept[KEEP];
+        int n_sel = 0;
 #pragma unroll
-    for (int nt = 0; nt < DK / 8; ++nt)
+        for (int i = 0; i < KEEP; ++i) {
+            kept[i] = __ballot_sync(0xffffffffu, i * 32 + lane < NT && selected(i * 32 + lane));
+            n_sel += __popc(kept[i]);
+        }
+        for (int base = KEEP * 32; base < NT; base += 32)
+            n_sel += __popc(__ballot_sync(0xffffffffu, base + lane < NT && selected(base + lane)));
+        const int n_pairs = (n_sel + 1) / 2;
+        const bool mine_sel = item < n_pairs;
+        const int r0 = mine_sel ? 2 * item : (item - n_pairs) * BKV_OWN;
+        const int want = mine_sel ? 2 : BKV_OWN;              // ranks [r0, r0 + want) among the tiles of that kind
+        if (lane < BKV_OWN) s_tile[lane] = -1;
+        __syncwarp();
+        int cnt = 0;
+        auto place = [&](int base, unsigned ms) {
+            const unsigned in = base + 32 <= NT ? 0xffffffffu : (1u << (NT - base)) - 1;
+            const unsigned m = mine_sel ? ms : in & ~ms;
+            const int r = cnt + __popc(m & ((1u << lane) - 1)) - r0;
+            if (((m >> lane) & 1) && r >= 0 && r < want) s_tile[r] = base + lane;
+            cnt += __popc(m);
+        };
 #pragma unroll
-        for (int e = 0; e < 4; ++e) acc_dk[nt][e] *= scale;
-    store_acc_bf16<DK * 2, DK / 8>(st_k, acc_dk, r0, 0, lane);
-    store_acc_bf16<DV * 2, DV / 8>(st_v, acc_dv, r0, 0, lane);
+        for (int i = 0; i < KEEP; ++i)
+            if (i * 32 < NT) place(i * 32, kept[i]);
+        for (int base = KEEP * 32; base < NT && cnt < r0 + want; base += 32)
+            place(base, __ballot_sync(0xffffffffu, base + lane < NT && selected(base + lane)));
+        __syncwarp();
+        if (lane == 0) *s_nsel = n_sel;
+        // query tiles [first, last] of every (selected tile, head): the own block's from the keys on, the later ones if the
+        // head selected the block
+        for (int i = lane; mine_sel && i < 2 * BKV_MAXG; i += 32) {
+            const int kt = s_tile[i / BKV_MAXG], gi = i % BKV_MAXG;
+            int last = -1;
+            if (kt >= 0 && gi < G) {
+                const int blk = kt / cpb, blk_end = (blk + 1) * nbs;
+                const bool s = G == 1 || types_i[(((long)b * TN + blk) * HN + (hkv * G + gi) / (HQ / HN)) * 2] != 0;
+                if (s && blk_end < T) last = NTq - 1;
+                else if (own) last = min((blk_end - 1) / ATT_BM, NTq - 1);
+            }
+            s_last[i] = last;
+        }
+    }
     __syncthreads();
-    store_tile<64, DK, AB_THREADS>(st_k, dk + (tokk * HKV + hkv) * DK, (long)HKV * DK, valid_k, tid);
-    store_tile<64, DV, AB_THREADS>(st_v, dv + (tokk * HKV + hkv) * DV, (long)HKV * DV, valid_k, tid);
-    if (tid < G) dnats_part[((long)b * NT + kt) * HQ + hkv * G + tid] = (s_dn[tid][0] + s_dn[tid][1]) + (s_dn[tid][2] + s_dn[tid][3]);
+    const int n_pairs = (*s_nsel + 1) / 2;
+    const bool paired = item < n_pairs;
+    if (s_tile[0] < 0) return;                                // no tile of either kind is left for this CTA
+    if (warp == 1) tmem_alloc(smem_u32(tmem_slot), 512);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    const int tile[2] = {s_tile[0], s_tile[1]};
+    int n_own = 0;
+    while (n_own < BKV_OWN && s_tile[n_own] >= 0) ++n_own;
+    DkvWalk w;
+    w.last = s_last;
+    w.G = G;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) w.first[u] = tile[u] < 0 ? NTq : own ? tile[u] * 64 / ATT_BM : ((tile[u] / cpb + 1) * nbs) / ATT_BM;
+    auto has_items = [&](int u) -> bool {
+        for (int gi = 0; gi < G; ++gi)
+            if (s_last[u * BKV_MAXG + gi] >= w.first[u]) return true;
+        return false;
+    };
+    OwnWalk ow;
+    ow.tiles = s_tile;
+    ow.n = own ? n_own : 0;
+    ow.G = G;
+    ow.nbs = nbs;
+    ow.NTq = NTq;
+
+    if (warp == 0) {
+        // ------------------------------------------------------------ TMA producer
+        auto load_kv = [&](int slot, int kt, uint32_t bar) {
+            const uint32_t dst = sbase + L::kv + slot * L::kv_bytes;
+#pragma unroll
+            for (int sub = 0; sub < DK / 64; ++sub) tma_load_4d(dst + sub * 8192, &map_k, sub * 64, hkv, kt * 64, b, bar);
+#pragma unroll
+            for (int sub = 0; sub < DV / 64; ++sub)
+                tma_load_4d(dst + 64 * DK * 2 + sub * 8192, &map_v, sub * 64, hkv, kt * 64, b, bar);
+        };
+        auto load_q = [&](int stg, int gi, int qt) {
+            const uint32_t base = sbase + L::stage + stg * L::stage_bytes;
+#pragma unroll
+            for (int sub = 0; sub < DK / 64; ++sub)
+                tma_load_4d(base + 128 * DV * 2 + sub * 16384, &map_q, sub * 64, hkv * G + gi, qt * ATT_BM, b, bar_full + stg * 8);
+#pragma unroll
+            for (int sub = 0; sub < DV / 64; ++sub)
+                tma_load_4d(base + sub * 16384, &map_do, sub * 64, hkv * G + gi, qt * ATT_BM, b, bar_full + stg * 8);
+        };
+        bool ok = true;
+        int n = 0;
+        if (paired) {
+            if (lane == 0)
+                for (int u = 0; u < 2; ++u)
+                    if (has_items(u)) {
+                        mbar_expect_tx(bar_kv + u * 8, L::kv_bytes);
+                        load_kv(u, tile[u], bar_kv + u * 8);
+                    }
+            __syncwarp();
+            for (bool more = w.begin(); more; more = w.next_query(), ++n) {
+                const int stg = n & 1;
+                if (n >= 2) ok = __all_sync(0xffffffffu, mbar_wait(bar_empty + stg * 8, ((n >> 1) - 1) & 1, status));
+                if (!ok) break;
+                if (lane == 0) {
+                    mbar_expect_tx(bar_full + stg * 8, L::stage_bytes);
+                    load_q(stg, w.gi, w.qt);
+                    if (w.qt + 2 < NTq) {                     // warm L2 for the tile this stage most likely receives next
+#pragma unroll
+                        for (int sub = 0; sub < DK / 64; ++sub)
+                            tma_prefetch_4d(&map_q, sub * 64, hkv * G + w.gi, (w.qt + 2) * ATT_BM, b);
+#pragma unroll
+                        for (int sub = 0; sub < DV / 64; ++sub)
+                            tma_prefetch_4d(&map_do, sub * 64, hkv * G + w.gi, (w.qt + 2) * ATT_BM, b);
+                    }
+                }
+                __syncwarp();
+            }
+        } else {
+            for (bool more = ow.begin(); more; more = ow.next(), ++n) {
+                const int stg = n & 1;
+                if (n >= 2) ok = __all_sync(0xffffffffu, mbar_wait(bar_empty + stg * 8, ((n >> 1) - 1) & 1, status));
+                if (!ok) break;
+                if (lane == 0) {                              // every item brings its own copy of k and v
+                    mbar_expect_tx(bar_full + stg * 8, L::stage_bytes + L::kv_bytes);
+                    load_kv(stg, s_tile[ow.u], bar_full + stg * 8);
+                    load_q(stg, ow.gi, ow.qt);
+                }
+                __syncwarp();
+            }
+        }
+    } else if (warp == 1) {
+        // ------------------------------------------------------------ MMA issuer
+        constexpr uint32_t id_s = umma_idesc_bf16(128, 64, false);
+        constexpr uint32_t id_acc = umma_idesc_bf16(128, 64, true) | (1u << 15);         // A MN-major too
+        auto scores = [&](int n, int stg, int kv) {           // S and dO V^T of item n into buffer n & 1
+            if (lane == 0) {
+                tc_fence_after();
+                const uint32_t dos = sbase + L::stage + stg * L::stage_bytes, qs = dos + 128 * DV * 2;
+                const uint32_t kt = sbase + L::kv + kv * L::kv_bytes, vt = kt + 64 * DK * 2;
+#pragma unroll
+                for (int kk = 0; kk < DK / 16; ++kk)
+                    umma_ss(tmem + C_S + (n & 1) * 64, umma_desc(qs + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
+                            umma_desc(kt + (kk >> 2) * 8192 + (kk & 3) * 32, 16, 1024), id_s, kk > 0);
+#pragma unroll
+                for (int kk = 0; kk < DV / 16; ++kk)
+                    umma_ss(tmem + C_DP + (n & 1) * 64, umma_desc(dos + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
+                            umma_desc(vt + (kk >> 2) * 8192 + (kk & 3) * 32, 16, 1024), id_s, kk > 0);
+                umma_commit(bar_s + (n & 1) * 8);
+            }
+            __syncwarp();
+        };
+        auto accumulate = [&](int stg, int slot, bool cont, bool release) {
+            if (lane == 0) {
+                tc_fence_after();
+                const uint32_t dos = sbase + L::stage + stg * L::stage_bytes, qs = dos + 128 * DV * 2;
+                const uint32_t acc = tmem + C_ACC + slot * 128;
+#pragma unroll
+                for (int kk = 0; kk < 8; ++kk)                // dv^T += do^T p
+                    umma_ss(acc, umma_desc(dos + kk * 2048, 16384, 1024), umma_desc(sbase + L::p + kk * 2048, 8192, 1024), id_acc,
+                            (cont || kk > 0) ? 1u : 0u);
+#pragma unroll
+                for (int kk = 0; kk < 8; ++kk)                // dk^T += q^T ds
+                    umma_ss(acc + 64, umma_desc(qs + kk * 2048, 16384, 1024), umma_desc(sbase + L::ds + kk * 2048, 8192, 1024), id_acc,
+                            (cont || kk > 0) ? 1u : 0u);
+                umma_commit(bar_acc);
+                if (release) umma_commit(bar_empty + stg * 8);
+            }
+            __syncwarp();
+        };
+        bool ok = true;
+        if (paired) {
+            DkvWalk a = w;                                    // one item ahead: scores
+            bool more = w.begin(), ahead = a.begin();
+            int na = 0, nq_a = -1, nq = -1;                   // items issued; query tiles entered by a / w
+            bool kv_seen[2] = {false, false}, started[2] = {false, false};
+            auto step_ahead = [&]() {
+                if (a.first_of_query()) {
+                    ++nq_a;
+                    ok = __all_sync(0xffffffffu, mbar_wait(bar_full + (nq_a & 1) * 8, (nq_a >> 1) & 1, status));
+                }
+                if (ok && !kv_seen[a.u]) ok = __all_sync(0xffffffffu, mbar_wait(bar_kv + a.u * 8, 0, status));
+                kv_seen[a.u] = true;
+                if (ok) scores(na, nq_a & 1, a.u);
+                ++na;
+                ahead = a.next();
+            };
+            if (ahead) step_ahead();
+            // The scores of the next item go ahead of this item's products (their buffer was read before bar_p of item
+            // i - 1) unless their tiles are still on the way: the stage that the producer fills after them is the one
+            // that these products release.
+            auto ready = [&]() {
+                return __all_sync(0xffffffffu, !a.first_of_query() || mbar_test_wait(bar_full + ((nq_a + 1) & 1) * 8, ((nq_a + 1) >> 1) & 1));
+            };
+            for (int i = 0; ok && more; ++i) {
+                const bool first = ahead && ready();
+                if (first) step_ahead();
+                if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_p, i & 1, status));
+                if (!ok) break;
+                if (w.first_of_query()) ++nq;
+                accumulate(nq & 1, w.u, started[w.u], w.last_of_query());
+                started[w.u] = true;
+                more = w.next();
+                if (more && !first) step_ahead();
+            }
+        } else {
+            OwnWalk a = ow;
+            bool more = ow.begin(), ahead = a.begin();
+            int na = 0;
+            auto step_ahead = [&]() {
+                ok = __all_sync(0xffffffffu, mbar_wait(bar_full + (na & 1) * 8, (na >> 1) & 1, status));
+                if (ok) scores(na, na & 1, na & 1);
+                ++na;
+                ahead = a.next();
+            };
+            if (ahead) step_ahead();
+            for (int i = 0; ok && more; ++i) {
+                const bool first = ahead && __all_sync(0xffffffffu, mbar_test_wait(bar_full + (na & 1) * 8, (na >> 1) & 1));
+                if (first) step_ahead();
+                // the accumulators of tile u - 2 were read before the softmax warps arrived here for this item
+                if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_p, i & 1, status));
+                if (!ok) break;
+                accumulate(i & 1, ow.u & 1, !ow.first_of_tile(), true);
+                more = ow.next();
+                if (more && !first) step_ahead();
+            }
+        }
+    } else {
+        // ------------------------------------------------------------ softmax (8 warps)
+        const int quad = warp & 3, half = (warp - 2) >> 2, sw = warp - 2;
+        const int row_a = quad * 32 + half * 16 + (lane >> 2), row_b = row_a + 8;
+        const int cq = (lane & 3) * 2;
+        const uint32_t t_rows = tmem + ((uint32_t)(quad * 32 + half * 16) << 16);
+        const float sl2 = scale * kLog2e;
+        unsigned char* p_t = smem + L::p;
+        unsigned char* ds_t = smem + L::ds;
+        float lse_a = 0.f, lse_b = 0.f, del_a = 0.f, del_b = 0.f;
+        auto load_rows = [&](int gi, int qt) {
+            const int t_a = qt * ATT_BM + row_a, t_b = t_a + 8;
+            const long r = ((long)b * T + t_a) * HQ + hkv * G + gi;
+            lse_a = t_a < T ? lse[r] : 0.f;
+            del_a = t_a < T ? delta[r] : 0.f;
+            lse_b = t_b < T ? lse[r + 8L * HQ] : 0.f;
+            del_b = t_b < T ? delta[r + 8L * HQ] : 0.f;
+        };
+        // p and ds of item i (key tile kt, query tile qt; `sel`: later blocks see the keys) into shared memory; adds the ds
+        // of later blocks' queries to dn
+        auto item_p = [&](int i, int kt, int qt, bool sel, float& dn) -> bool {
+            bool ok = __all_sync(0xffffffffu, mbar_wait(bar_s + (i & 1) * 8, (i >> 1) & 1, status));
+            if (!ok) return false;
+            tc_fence_after();
+            uint32_t sr[32], dr[32];
+            tmem_ld_16x256b_x8(t_rows + C_S + (i & 1) * 64, sr);
+            tmem_ld_16x256b_x8(t_rows + C_DP + (i & 1) * 64, dr);
+            tmem_ld_wait();
+            const int t_a = qt * ATT_BM + row_a, t_b = t_a + 8;
+            const int s0 = kt * 64, blk_end = (kt / cpb + 1) * nbs;
+            if (qt * ATT_BM < blk_end) {
+                // rows of the own block see columns [0, t - s0], rows behind it all or none
+                const int lim_a = t_a >= blk_end ? (sel ? 63 : -1) : (own ? t_a - s0 : -1);
+                const int lim_b = t_b >= blk_end ? (sel ? 63 : -1) : (own ? t_b - s0 : -1);
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const int c = 8 * k + cq + e;
+                        if (c > lim_a) sr[4 * k + e] = 0xff800000u;
+                        if (c > lim_b) sr[4 * k + 2 + e] = 0xff800000u;
+                    }
+            }
+            float sum_a = 0.f, sum_b = 0.f;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const float p0 = ex2(fmaf(__uint_as_float(sr[4 * k]), sl2, -lse_a));
+                const float p1 = ex2(fmaf(__uint_as_float(sr[4 * k + 1]), sl2, -lse_a));
+                const float p2 = ex2(fmaf(__uint_as_float(sr[4 * k + 2]), sl2, -lse_b));
+                const float p3 = ex2(fmaf(__uint_as_float(sr[4 * k + 3]), sl2, -lse_b));
+                const float d0 = p0 * (__uint_as_float(dr[4 * k]) - del_a), d1 = p1 * (__uint_as_float(dr[4 * k + 1]) - del_a);
+                const float d2 = p2 * (__uint_as_float(dr[4 * k + 2]) - del_b), d3 = p3 * (__uint_as_float(dr[4 * k + 3]) - del_b);
+                sum_a += d0 + d1;
+                sum_b += d2 + d3;
+                sr[4 * k] = pack_bf16(p0, p1);
+                sr[4 * k + 1] = pack_bf16(p2, p3);
+                sr[4 * k + 2] = pack_bf16(d0, d1);
+                sr[4 * k + 3] = pack_bf16(d2, d3);
+            }
+            dn += (t_a >= blk_end ? sum_a : 0.f) + (t_b >= blk_end ? sum_b : 0.f);
+            // the products of the previous item have read p and ds
+            if (i > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar_acc, (i - 1) & 1, status));
+            if (!ok) return false;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const uint32_t oa = swz<128>(row_a, k) + (lane & 3) * 4, ob = swz<128>(row_b, k) + (lane & 3) * 4;
+                *reinterpret_cast<uint32_t*>(p_t + oa) = sr[4 * k];
+                *reinterpret_cast<uint32_t*>(p_t + ob) = sr[4 * k + 1];
+                *reinterpret_cast<uint32_t*>(ds_t + oa) = sr[4 * k + 2];
+                *reinterpret_cast<uint32_t*>(ds_t + ob) = sr[4 * k + 3];
+            }
+            fence_async_smem();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_p);
+            return true;
+        };
+        // dk, dv of key tile kt from accumulator pair `slot` (zeros without `any`): lane = head-dim index, columns = keys, a
+        // warp writes 64 contiguous bytes per key
+        auto finish = [&](int kt, int slot, bool any) {
+            const int d = quad * 32 + lane;
+            const long tok = (long)b * T + kt * 64 + half * 32;
+            const int n_valid = min(32, T - kt * 64 - half * 32);
+            const uint32_t acc = tmem + ((uint32_t)(quad * 32) << 16) + C_ACC + slot * 128 + half * 32;
+            tc_fence_after();
+            uint32_t r[32];
+            if (quad * 32 < DV) {
+                tmem_ld32(acc, r);
+                tmem_ld_wait();
+#pragma unroll
+                for (int c = 0; c < 32; ++c)
+                    if (c < n_valid) dv[((tok + c) * HKV + hkv) * DV + d] = __float2bfloat16(any ? __uint_as_float(r[c]) : 0.f);
+            }
+            if (quad * 32 < DK) {
+                tmem_ld32(acc + 64, r);
+                tmem_ld_wait();
+#pragma unroll
+                for (int c = 0; c < 32; ++c)
+                    if (c < n_valid) dk[((tok + c) * HKV + hkv) * DK + d] = __float2bfloat16(any ? __uint_as_float(r[c]) * scale : 0.f);
+            }
+        };
+        bool ok = true;
+        int i = 0;
+        if (paired) {
+            float dn[2] = {0.f, 0.f};
+            auto flush = [&](int gi) {                        // one slot per (key tile, head, warp): a fixed order of summation
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    dn[u] = warp_sum(dn[u]);
+                    if (lane == 0) s_dn[(u * BKV_MAXG + gi) * 8 + sw] = dn[u];
+                    dn[u] = 0.f;
+                }
+            };
+            int gi = 0;
+            for (bool more = w.begin(); more; more = w.next(), ++i) {
+                if (w.gi != gi) {
+                    flush(gi);
+                    gi = w.gi;
+                }
+                if (w.first_of_query()) load_rows(gi, w.qt);
+                const int kt = w.u ? tile[1] : tile[0];
+                // rows behind the own block are in the walk only where the head selected the block; in a tile that holds
+                // both, the flag decides
+                bool sel = true;
+                if (G > 1 && w.qt * ATT_BM < (kt / cpb + 1) * nbs)
+                    sel = types_i[(((long)b * TN + kt / cpb) * HN + (hkv * G + gi) / (HQ / HN)) * 2] != 0;
+                float add = 0.f;
+                ok = item_p(i, kt, w.qt, sel, add);
+                if (!ok) break;
+                if (w.u) dn[1] += add; else dn[0] += add;
+            }
+            flush(gi);
+            if (ok && i > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar_acc, (i - 1) & 1, status));
+            if (ok) {
+                finish(tile[0], 0, has_items(0));
+                if (tile[1] >= 0) finish(tile[1], 1, has_items(1));
+            }
+        } else if (!own) {
+            for (int u = 0; u < n_own; ++u) finish(s_tile[u], 0, false);
+        } else {
+            int done = 0;                                     // tiles written
+            float unused = 0.f;
+            for (bool more = ow.begin(); more; more = ow.next(), ++i) {
+                load_rows(ow.gi, ow.qt);
+                ok = item_p(i, s_tile[ow.u], ow.qt, false, unused);
+                if (!ok) break;
+                // item_p has waited for the products of the previous item: a tile that ended there is complete
+                if (ow.u > done) {
+                    finish(s_tile[done], done & 1, true);
+                    tc_fence_before();
+                    ++done;
+                }
+            }
+            if (ok && i > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar_acc, (i - 1) & 1, status));
+            if (ok && done < n_own) finish(s_tile[done], done & 1, true);
+        }
+        asm volatile("bar.sync 1, 256;" ::: "memory");       // every softmax warp reaches it, also after a failed wait
+        const int n_tiles = paired ? 2 : n_own;
+        for (int e = tid - 64; e < n_tiles * G; e += 256) {
+            const int u = e / G, gi = e % G;
+            if (s_tile[u] < 0) continue;
+            const float* p = s_dn + (u * BKV_MAXG + gi) * 8;
+            dnats_part[((long)b * NT + s_tile[u]) * HQ + hkv * G + gi] =
+                paired ? ((p[0] + p[1]) + (p[2] + p[3])) + ((p[4] + p[5]) + (p[6] + p[7])) : 0.f;
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) tmem_dealloc(tmem, 512);
 }
 
 template <int DK, int DV>
 static int launch_attn_bwd(const void* q, const void* k, const void* v, const void* o, const void* d_o, const float* lse,
                            const int* types_i, void* dq, void* dk, void* dv, float* delta, float* dnats_part, int B, int T,
                            int HQ, int HKV, int HN, int nbs, float scale, int own_chunk, int compat, cudaStream_t st) {
-    using L = AttnBwdSmem<DK, DV>;
-    const int NT = (T + 63) / 64;
+    const int NT = (T + 63) / 64, NTq = (T + ATT_BM - 1) / ATT_BM;
     const int TN = (T + nbs - 1) / nbs;
-    const int smem = L::total(NT);
+    const int smem = DqSmem<DK, DV>::total(NT);
     if (smem > 227 * 1024) {
         set_error("natsl_attn_bwd: T=%d needs %d B of shared memory (max %d)", T, smem, 227 * 1024);
         return NATSL_ERR_TOO_LARGE;
@@ -355,20 +895,30 @@ static int launch_attn_bwd(const void* q, const void* k, const void* v, const vo
     auto k1 = attn_bwd_dq_kernel<DK, DV>;
     auto k2 = attn_bwd_dkdv_kernel<DK, DV>;
     cudaError_t e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, DkvSmem<DK, DV>::total);
     if (e != cudaSuccess) {
         set_error("natsl_attn_bwd: cannot reserve %d B of shared memory (%s)", smem, cudaGetErrorString(e));
         return NATSL_ERR_CUDA;
     }
-    auto bf = [](const void* p) { return reinterpret_cast<const __nv_bfloat16*>(p); };
-    k1<<<dim3(NT, HQ, B), AB_THREADS, smem, st>>>(bf(q), bf(k), bf(v), bf(o), bf(d_o), lse, types_i,
-                                                 reinterpret_cast<__nv_bfloat16*>(dq), delta, T, HQ, HKV, HN, TN, nbs, scale,
-                                                 own_chunk, compat);
-    int rc = check_launch("natsl_attn_bwd (dq)");
+    CUtensorMap mq, mk, mv, mdo;
+    int* status = nullptr;
+    int rc = encode_bthd_map(&mq, q, B, T, HQ, DK, 128, "natsl_attn_bwd(q)");
+    if (rc == NATSL_OK) rc = encode_bthd_map(&mk, k, B, T, HKV, DK, 64, "natsl_attn_bwd(k)");
+    if (rc == NATSL_OK) rc = encode_bthd_map(&mv, v, B, T, HKV, DV, 64, "natsl_attn_bwd(v)");
+    if (rc == NATSL_OK) rc = encode_bthd_map(&mdo, d_o, B, T, HQ, DV, 128, "natsl_attn_bwd(do)");
+    if (rc == NATSL_OK) rc = status_word_ptr(&status);
     if (rc != NATSL_OK) return rc;
-    k2<<<dim3(NT, HKV, B), AB_THREADS, smem, st>>>(bf(q), bf(k), bf(v), bf(d_o), lse, delta, types_i,
-                                                  reinterpret_cast<__nv_bfloat16*>(dk), reinterpret_cast<__nv_bfloat16*>(dv),
-                                                  dnats_part, T, HQ, HKV, HN, TN, nbs, scale, own_chunk, compat);
+    auto bf = [](const void* p) { return reinterpret_cast<const __nv_bfloat16*>(p); };
+    const int own = own_chunk && !compat;
+    k1<<<dim3(NTq, HQ, B), TC_THREADS, smem, st>>>(mq, mk, mv, mdo, bf(o), bf(d_o), lse, types_i, reinterpret_cast<__nv_bfloat16*>(dq),
+                                                  delta, T, HQ, HKV, HN, TN, nbs, scale, own, status);
+    rc = check_launch("natsl_attn_bwd (dq)");
+    if (rc != NATSL_OK) return rc;
+    // ceil(n / 2) + ceil((NT - n) / 8) CTAs per head for n selected tiles, known on the device only
+    const int per_head = NT / 2 + 1, heads = HKV * B;
+    k2<<<per_head * heads, TC_THREADS, DkvSmem<DK, DV>::total, st>>>(
+        mq, mk, mv, mdo, lse, delta, types_i, reinterpret_cast<__nv_bfloat16*>(dk), reinterpret_cast<__nv_bfloat16*>(dv), dnats_part, T,
+        HQ, HKV, HN, TN, nbs, scale, own, heads, per_head, status);
     return check_launch("natsl_attn_bwd (dk, dv)");
 }
 

@@ -1,0 +1,46 @@
+"""GPU test (-m gpu) of the tcgen05 softmax backward at the edges of its tiles: 128-query tiles, pairs of 64-key tiles
+(one key tile in all, an odd number, pairs far apart, none or every block selected), query heads of a group with
+selections of their own, against the CPU oracle in float64."""
+import pytest
+import torch
+
+from oracle import grad as ograd
+from oracle import tables as otab
+from tests.test_gpu_backward import close_scaled
+
+pytestmark = pytest.mark.gpu
+
+CASES = [  # T, query heads, key/value heads, selection heads, DK, DV, block, share of softmax blocks, own block, compat
+    (1, 2, 2, 2, 128, 128, 64, 0.5, True, False), (63, 2, 2, 2, 64, 64, 64, 0.5, True, False),
+    (64, 2, 2, 2, 128, 64, 64, 0.5, False, False), (65, 2, 2, 2, 64, 128, 64, 0.5, True, False),
+    (129, 2, 2, 2, 128, 128, 64, 1.0, True, False), (191, 4, 1, 4, 128, 128, 64, 0.4, True, False),
+    (320, 4, 2, 4, 64, 64, 64, 0.0, True, False), (577, 4, 2, 2, 128, 64, 128, 0.5, True, True),
+    (832, 2, 2, 2, 128, 128, 192, 0.3, False, False), (1000, 16, 1, 8, 64, 128, 64, 0.2, True, False),
+    (2112, 1, 1, 1, 128, 128, 64, 0.1, True, False),
+]
+
+
+@pytest.mark.parametrize("T,HQ,HKV,HN,DK,DV,nbs,p,own,compat", CASES)
+def test_softmax_backward_tiles(T, HQ, HKV, HN, DK, DV, nbs, p, own, compat):
+    import neuralattentionsearchlinear_b200 as nat
+    from neuralattentionsearchlinear_b200 import _lib, _ops
+    B = 2
+    gen = torch.Generator().manual_seed(T + DK + DV)
+    rnd = lambda *s: torch.randn(*s, generator=gen).bfloat16()
+    q, k, v, do = rnd(B, T, HQ, DK), rnd(B, T, HKV, DK), rnd(B, T, HKV, DV), rnd(B, T, HQ, DV)
+    types = otab.synth_types(B, -(-T // nbs), HN, p, seed=T)
+    tb = nat.build_selection_tables(types.cuda(), T, nbs)
+    scale = DK ** -0.5
+    c = [x.cuda() for x in (q, k, v)]
+    o, lse = _ops.attn_fwd(*c, tb, scale, own)
+    got = _ops.attn_bwd(*c, o, lse, do.cuda(), tb, scale, own, reference_compat=compat)
+    ref = ograd.attn_grads(q.double(), k.double(), v.double(), types[..., 0], do.double(), nbs=nbs, scale=scale, own_chunk=own,
+                           reference_compat=compat)
+    # dq: delta = rowsum(o do) is summed from o rounded to bf16 (2^-9 of an entry at most, 2^-9 / sqrt(3) in the mean), so
+    # it is off by 0.0011 sqrt(128) = 0.0128 in the mean for normal o and do, and dq by that times scale |k|: 0.0064 with
+    # DK = 64 and |k| = 4; three times that, over the millions of entries here, is 2e-2
+    for x, name in zip(got, ("dq", "dk", "dv", "dnats")):
+        close_scaled(x, ref[name], name, tol=2e-2 if name == "dq" else 1e-2, scale="max" if name == "dnats" else "auto")
+    assert _lib.load().natsl_device_status() == 0
+    again = _ops.attn_bwd(*c, o, lse, do.cuda(), tb, scale, own, reference_compat=compat)
+    assert all(torch.equal(x, y) for x, y in zip(got, again))
