@@ -168,26 +168,26 @@ linear_bwd_pre_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* 
 }
 
 // ================================================================================================ dh (reverse walk)
-constexpr int DH_THREADS = 128;
-
+// Serial over the chunks, so what bounds it is the latency of one step times NT.  A step has two products with a barrier
+// before each; the tiles of product 1 (k, do, dv'_loc, decays) are requested when product 2 of the previous step begins
+// and those of product 2 (q, w) when product 1 begins, so that every load runs behind a product.  do and dv'_loc
+// alternate between two buffers and are overwritten in place by the scaled copies that product 2 reads.
 template <int K, int BV, bool GDN>
 struct DhSmem {
     static constexpr int ks = 0;
     static constexpr int qs = ks + 64 * K * 2;
     static constexpr int ws = qs + 64 * K * 2;
-    static constexpr int dob = ws + (GDN ? 64 * K * 2 : 0);   // do slice
-    static constexpr int dvl = dob + 64 * BV * 2;             // dv'_loc slice
-    static constexpr int dsb = dvl + 64 * BV * 2;             // dS as bf16 [K][BV]
-    static constexpr int dos = dsb + K * BV * 2;              // s e^{g+car} do
-    static constexpr int dvs = dos + 64 * BV * 2;             // -e^{car} dv'
-    static constexpr int dvo = dvs + 64 * BV * 2;             // dv' (store staging)
-    static constexpr int vec = dvo + 64 * BV * 2;             // g[64]
-    static constexpr int meta = vec + 64 * 4;                 // per chunk: g_last, carry, act
+    static constexpr int dob = ws + (GDN ? 64 * K * 2 : 0);   // 2 x do slice, then s e^{g+car} do
+    static constexpr int dvl = dob + 2 * 64 * BV * 2;         // 2 x dv'_loc slice, then -e^{car} dv'
+    static constexpr int dsb = dvl + 2 * 64 * BV * 2;         // dS as bf16 [K][BV]
+    static constexpr int dvo = dsb + K * BV * 2;              // dv' (store staging)
+    static constexpr int vec = dvo + 64 * BV * 2;             // 2 x g[64]
+    static constexpr int meta = vec + 2 * 64 * 4;             // per chunk: g_last, carry, act
     static int total(int NT) { return meta + NT * 12; }
 };
 
 template <int K, int BV, bool GDN>
-__global__ void __launch_bounds__(DH_THREADS)
+__global__ void __launch_bounds__(BV * 4)
 linear_bwd_dh_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat16* __restrict__ kn,
                      const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ d_o,
                      const __nv_bfloat16* __restrict__ dvl_in, const float* __restrict__ gcs,
@@ -195,10 +195,12 @@ linear_bwd_dh_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat16* 
                      const int* __restrict__ n_blocks, const float* __restrict__ dht, __nv_bfloat16* __restrict__ dS_all,
                      __nv_bfloat16* __restrict__ dvp_out, float* __restrict__ dh0, int T, int H, int HN, int V, float scale) {
     using L = DhSmem<K, BV, GDN>;
+    constexpr int DH_THREADS = BV * 4;                      // a warp: 16 tokens (K / 4 rows of dS) x 32 value columns
     constexpr int MT = K / 64;
-    constexpr int NTL = BV / 8;
+    constexpr int NTL = 4;
     extern __shared__ __align__(128) unsigned char smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int rw = warp & 3, n0 = (warp >> 2) * 32;         // row group, first column
     const int gq = lane >> 2, qd = lane & 3;
     const int vsplit = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
     const int v0 = vsplit * BV;
@@ -209,14 +211,9 @@ linear_bwd_dh_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat16* 
     const int last_sel = nsel > 0 ? indices[(((long)b * TN + (nsel - 1)) * HN + hn) * 2 + 1] : -1;
 
     unsigned char* dsb_p = smem + L::dsb;
-    unsigned char* dos_p = smem + L::dos;
-    unsigned char* dvs_p = smem + L::dvs;
     unsigned char* dvo_p = smem + L::dvo;
-    const unsigned char* dob_p = smem + L::dob;
-    const unsigned char* dvl_p = smem + L::dvl;
     const uint32_t ks = smem_u32(smem + L::ks), qs = smem_u32(smem + L::qs), ws = smem_u32(smem + L::ws);
-    const uint32_t dsb = smem_u32(dsb_p), dos = smem_u32(dos_p), dvs = smem_u32(dvs_p);
-    float* s_g = reinterpret_cast<float*>(smem + L::vec);
+    const uint32_t dsb = smem_u32(dsb_p);
     float* s_gl = reinterpret_cast<float*>(smem + L::meta);
     float* s_car = s_gl + NT;
     int* s_act = reinterpret_cast<int*>(s_car + NT);
@@ -230,7 +227,7 @@ linear_bwd_dh_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat16* 
     __syncthreads();
 
     float dS[MT][NTL][4];
-    const int krow0 = warp * (K / 4);
+    const int krow0 = rw * (K / 4);
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt) zero_acc(dS[mt]);
 
@@ -242,61 +239,83 @@ linear_bwd_dh_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat16* 
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const int r = krow0 + mt * 16 + gq + ((e >> 1) << 3);
-                    const int cidx = v0 + nt * 8 + qd * 2 + (e & 1);
+                    const int cidx = v0 + n0 + nt * 8 + qd * 2 + (e & 1);
                     dS[mt][nt][e] += dht[(((long)b * H + h) * K + r) * V + cidx];
                 }
     };
+    auto issue_a = [&](int c) {                             // what product 1 of chunk c reads
+        if (c >= 0) {
+            const int valid = min(64, T - c * 64), stg = c & 1;
+            const long tok0 = (long)b * T + (long)c * 64;
+            if (s_act[c]) load_tile_async<64, K, DH_THREADS>(ks, kn + (tok0 * H + h) * K, (long)H * K, valid, tid);
+            load_tile_async<64, BV, DH_THREADS>(smem_u32(smem + L::dob + stg * 64 * BV * 2), d_o + (tok0 * H + h) * V + v0, (long)H * V,
+                                                valid, tid);
+            load_tile_async<64, BV, DH_THREADS>(smem_u32(smem + L::dvl + stg * 64 * BV * 2), dvl_in + (tok0 * H + h) * V + v0,
+                                                (long)H * V, valid, tid);
+            if (tid < 64)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(smem_u32(smem + L::vec) + (stg * 64 + tid) * 4),
+                             "l"(gcs + (tok0 + min(tid, valid - 1)) * H + h));
+        }
+        cp_async_commit();
+    };
+    auto issue_b = [&](int c) {                             // ... product 2
+        const int valid = min(64, T - c * 64);
+        const long tok0 = (long)b * T + (long)c * 64;
+        load_tile_async<64, K, DH_THREADS>(qs, qn + (tok0 * H + h) * K, (long)H * K, valid, tid);
+        if (GDN) load_tile_async<64, K, DH_THREADS>(ws, w + (tok0 * H + h) * K, (long)H * K, valid, tid);
+        cp_async_commit();
+    };
 
-    const int r0 = warp * 16;
+    const int r0 = rw * 16;
     const int ia = r0 + gq, ib = ia + 8;
+    issue_a(NT - 1);
     for (int c = NT - 1; c >= 0; --c) {
         const int valid = min(64, T - c * 64);
         const long tok0 = (long)b * T + (long)c * 64;
         const bool act = s_act[c] != 0;
         const float gl = s_gl[c], car = s_car[c];
-        if (act) load_tile_async<64, K, DH_THREADS>(ks, kn + (tok0 * H + h) * K, (long)H * K, valid, tid);
-        load_tile_async<64, K, DH_THREADS>(qs, qn + (tok0 * H + h) * K, (long)H * K, valid, tid);
-        if (GDN) load_tile_async<64, K, DH_THREADS>(ws, w + (tok0 * H + h) * K, (long)H * K, valid, tid);
-        load_tile_async<64, BV, DH_THREADS>(smem_u32(smem + L::dob), d_o + (tok0 * H + h) * V + v0, (long)H * V, valid, tid);
-        load_tile_async<64, BV, DH_THREADS>(smem_u32(smem + L::dvl), dvl_in + (tok0 * H + h) * V + v0, (long)H * V, valid, tid);
-        cp_async_commit();
-        if (tid < 64) s_g[tid] = gcs[(tok0 + min(tid, valid - 1)) * H + h];
+        unsigned char* dob_p = smem + L::dob + (c & 1) * 64 * BV * 2;
+        unsigned char* dvl_p = smem + L::dvl + (c & 1) * 64 * BV * 2;
+        const float* s_g = reinterpret_cast<const float*>(smem + L::vec) + (c & 1) * 64;
         if (dht && c == last_sel) add_dht();
         if (act) {
 #pragma unroll
-            for (int mt = 0; mt < MT; ++mt) store_acc_bf16<BV * 2, NTL>(dsb_p, dS[mt], krow0 + mt * 16, 0, lane);
+            for (int mt = 0; mt < MT; ++mt) store_acc_bf16<BV * 2, NTL>(dsb_p, dS[mt], krow0 + mt * 16, n0, lane);
         }
         cp_async_wait<0>();
-        __syncthreads();
+        __syncthreads();                                    // also: every warp is done with product 2 of the previous chunk
+        issue_b(c);
         if (act) store_tile<K, BV, DH_THREADS>(dsb_p, dS_all + ((((long)b * NT + c) * H + h) * K) * V + v0, V, K, tid);
 
         // ---- dv' = act (kn dS) kd + dv'_loc
         float acc[NTL][4];
         zero_acc(acc);
-        if (act) warp_gemm<K * 2, A_ROW, BV * 2, B_KN, NTL>(acc, ks, r0, dsb, 0, 0, K, lane);
+        if (act) warp_gemm<K * 2, A_ROW, BV * 2, B_KN, NTL>(acc, ks, r0, dsb, n0, 0, K, lane);
         const float kda = kdecay(gl, s_g[ia], GDN), kdb = kdecay(gl, s_g[ib], GDN);
         const float ec = __expf(car);
         const float ea = scale * __expf(s_g[ia] + car), eb = scale * __expf(s_g[ib] + car);
 #pragma unroll
         for (int nt = 0; nt < NTL; ++nt) {
-            const int col = nt * 8 + qd * 2;
+            const int col = n0 + nt * 8 + qd * 2;
             const float2 la = load_pair_bf16<BV * 2>(dvl_p, ia, col), lb = load_pair_bf16<BV * 2>(dvl_p, ib, col);
             const float2 da = load_pair_bf16<BV * 2>(dob_p, ia, col), db = load_pair_bf16<BV * 2>(dob_p, ib, col);
             const float a0 = acc[nt][0] * kda + la.x, a1 = acc[nt][1] * kda + la.y;
             const float b0 = acc[nt][2] * kdb + lb.x, b1 = acc[nt][3] * kdb + lb.y;
-            const uint32_t offa = swz<BV * 2>(ia, nt) + qd * 4, offb = swz<BV * 2>(ib, nt) + qd * 4;
+            const uint32_t offa = swz<BV * 2>(ia, col >> 3) + qd * 4, offb = swz<BV * 2>(ib, col >> 3) + qd * 4;
             *reinterpret_cast<uint32_t*>(dvo_p + offa) = pack_bf16(a0, a1);
             *reinterpret_cast<uint32_t*>(dvo_p + offb) = pack_bf16(b0, b1);
             if (GDN) {
                 // the rounded dv' is what the other kernels read: use it here too
                 const float2 ra = unpack_bf16(pack_bf16(a0, a1)), rb = unpack_bf16(pack_bf16(b0, b1));
-                *reinterpret_cast<uint32_t*>(dvs_p + offa) = pack_bf16(-ec * ra.x, -ec * ra.y);
-                *reinterpret_cast<uint32_t*>(dvs_p + offb) = pack_bf16(-ec * rb.x, -ec * rb.y);
+                *reinterpret_cast<uint32_t*>(dvl_p + offa) = pack_bf16(-ec * ra.x, -ec * ra.y);
+                *reinterpret_cast<uint32_t*>(dvl_p + offb) = pack_bf16(-ec * rb.x, -ec * rb.y);
             }
-            *reinterpret_cast<uint32_t*>(dos_p + offa) = pack_bf16(ea * da.x, ea * da.y);
-            *reinterpret_cast<uint32_t*>(dos_p + offb) = pack_bf16(eb * db.x, eb * db.y);
+            *reinterpret_cast<uint32_t*>(dob_p + offa) = pack_bf16(ea * da.x, ea * da.y);
+            *reinterpret_cast<uint32_t*>(dob_p + offb) = pack_bf16(eb * db.x, eb * db.y);
         }
+        cp_async_wait<0>();
         __syncthreads();
+        issue_a(c - 1);
         store_tile<64, BV, DH_THREADS>(dvo_p, dvp_out + (tok0 * H + h) * V + v0, (long)H * V, valid, tid);
 
         // ---- dS <- (act ? e^{g_L+car} : 1) dS + qn^T (s e^{g+car} do) + w^T (-e^{car} dv')
@@ -311,10 +330,9 @@ linear_bwd_dh_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat16* 
         }
 #pragma unroll
         for (int mt = 0; mt < MT; ++mt) {
-            warp_gemm<K * 2, A_TRANS, BV * 2, B_KN, NTL>(dS[mt], qs, krow0 + mt * 16, dos, 0, 0, 64, lane);
-            if (GDN) warp_gemm<K * 2, A_TRANS, BV * 2, B_KN, NTL>(dS[mt], ws, krow0 + mt * 16, dvs, 0, 0, 64, lane);
+            warp_gemm<K * 2, A_TRANS, BV * 2, B_KN, NTL>(dS[mt], qs, krow0 + mt * 16, smem_u32(dob_p), n0, 0, 64, lane);
+            if (GDN) warp_gemm<K * 2, A_TRANS, BV * 2, B_KN, NTL>(dS[mt], ws, krow0 + mt * 16, smem_u32(dvl_p), n0, 0, 64, lane);
         }
-        __syncthreads();                                    // tiles are overwritten by the next chunk's loads
     }
     if (dht && last_sel < 0) add_dht();                     // no chunk updated the state: the final state is h0
     if (dh0) {
@@ -323,7 +341,7 @@ linear_bwd_dh_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat16* 
 #pragma unroll
             for (int nt = 0; nt < NTL; ++nt) {
                 const int r = krow0 + mt * 16 + gq;
-                const int cidx = v0 + nt * 8 + qd * 2;
+                const int cidx = v0 + n0 + nt * 8 + qd * 2;
                 float* p = dh0 + (((long)b * H + h) * K + r) * V + cidx;
                 *reinterpret_cast<float2*>(p) = make_float2(dS[mt][nt][0], dS[mt][nt][1]);
                 *reinterpret_cast<float2*>(p + 8L * V) = make_float2(dS[mt][nt][2], dS[mt][nt][3]);
@@ -545,26 +563,28 @@ linear_bwd_state_kernel(const __nv_bfloat16* __restrict__ kn, const __nv_bfloat1
 }
 
 // ================================================================================================ intra
+// Six tile buffers hold what each phase needs, loaded behind the products of the phase before, so that two CTAs share an
+// SM: alone, a CTA is a chain of short phases that leaves the SM waiting at its barriers and loads.
+//     c: do, then dv' -> dzu -> dv      d: v', then dw -> dzw
+//     e: H, then u, then dq1 (later dq staging)      f: A, then w, then dk1 (later dk staging)
+//     m: dqk, then the diagonal blocks X, then dkk
 template <int K, int V, bool GDN>
 struct InSmem {
+    static constexpr int cmax(int x, int y) { return x > y ? x : y; }
+    static constexpr int KB = 64 * K * 2, VB = 64 * V * 2;
     static constexpr int qns = 0;
-    static constexpr int kns = qns + 64 * K * 2;
-    static constexpr int ws = kns + 64 * K * 2;               // w; later dq staging
-    static constexpr int dws = ws + 64 * K * 2;               // dw -> dzw; later dk staging
-    static constexpr int vps = dws + 64 * K * 2;              // v'
-    static constexpr int dos = vps + 64 * V * 2;
-    static constexpr int m1 = dos + 64 * V * 2;               // dqk (bf16 64x64)
-    static constexpr int us = m1 + 64 * 64 * 2;
-    static constexpr int dvs = us + (GDN ? 64 * V * 2 : 0);   // dv' -> dzu -> dv
-    static constexpr int vs = dvs + (GDN ? 64 * V * 2 : 0);
-    static constexpr int m2 = vs + (GDN ? 64 * V * 2 : 0);    // dkk (bf16 64x64)
-    static constexpr int hs = m2 + (GDN ? 64 * 64 * 2 : 0);   // H (bf16 64x64)
-    static constexpr int As = hs + (GDN ? 64 * 64 * 2 : 0);   // A fp32 [64][68]
-    static constexpr int Xs = As + (GDN ? 64 * LB_A_LD * 4 : 0);
-    static constexpr int vec = Xs + (GDN ? 4 * 16 * LB_X_LD * 4 : 0);
+    static constexpr int kns = qns + KB;
+    static constexpr int c = kns + KB;
+    static constexpr int d = c + VB;
+    static constexpr int e = d + (GDN ? cmax(KB, VB) : VB);
+    static constexpr int f = e + (GDN ? cmax(KB, cmax(VB, 64 * 64 * 2)) : KB);
+    static constexpr int m = f + (GDN ? cmax(KB, 64 * LB_A_LD * 4) : KB);     // A: fp32 [64][68]
+    static constexpr int vec = m + 64 * 64 * 2;
     // g, beta, zk, dE, dotq, dotk (6 x 64); decay-gradient row sums [2 phases][2 halves][64] and column sums
     // [2 phases][4 row blocks][64]; dbeta parts [2 halves + value part][64]; + 16
     static constexpr int total = vec + ((6 + 4 + 8 + 3) * 64 + 16) * 4;
+    static_assert(4 * 16 * LB_X_LD * 4 <= 64 * 64 * 2, "the X blocks fit over dqk");
+    static_assert(total <= 115712, "two CTAs per SM");
 };
 
 // In-place solve of (I + A)^T X = R for 32 columns [col0, col0+32) of a [64][COLS] bf16 tile by one warp:
@@ -595,7 +615,7 @@ __device__ __forceinline__ void solve_t_group(uint32_t htile, uint32_t ztile, un
 }
 
 template <int K, int V, bool GDN>
-__global__ void __launch_bounds__(LB_THREADS)
+__global__ void __launch_bounds__(LB_THREADS, 2)
 linear_bwd_intra_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat16* __restrict__ kn,
                         const __nv_bfloat16* __restrict__ v, const __nv_bfloat16* __restrict__ w,
                         const __nv_bfloat16* __restrict__ u, const __nv_bfloat16* __restrict__ vp,
@@ -620,18 +640,15 @@ linear_bwd_intra_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat1
 
     unsigned char* qns_p = smem + L::qns;
     unsigned char* kns_p = smem + L::kns;
-    unsigned char* ws_p = smem + L::ws;
-    unsigned char* dws_p = smem + L::dws;
-    unsigned char* m1_p = smem + L::m1;
-    unsigned char* m2_p = smem + L::m2;
-    unsigned char* hs_p = smem + L::hs;
-    unsigned char* dvs_p = smem + L::dvs;
-    const unsigned char* vs_p = smem + L::vs;
-    const uint32_t qns = smem_u32(qns_p), kns = smem_u32(kns_p), ws = smem_u32(ws_p), dws = smem_u32(dws_p),
-                   vps = smem_u32(smem + L::vps), dos = smem_u32(smem + L::dos), m1 = smem_u32(m1_p), us = smem_u32(smem + L::us),
-                   dvs = smem_u32(dvs_p), m2 = smem_u32(m2_p), hs = smem_u32(hs_p);
-    float* As = reinterpret_cast<float*>(smem + L::As);
-    float* Xs = reinterpret_cast<float*>(smem + L::Xs);
+    unsigned char* c_p = smem + L::c;
+    unsigned char* d_p = smem + L::d;
+    unsigned char* e_p = smem + L::e;
+    unsigned char* f_p = smem + L::f;
+    unsigned char* m_p = smem + L::m;
+    const uint32_t qns = smem_u32(qns_p), kns = smem_u32(kns_p), ct = smem_u32(c_p), dt = smem_u32(d_p), et = smem_u32(e_p),
+                   ft = smem_u32(f_p), mt = smem_u32(m_p);
+    float* As = reinterpret_cast<float*>(f_p);
+    float* Xs = reinterpret_cast<float*>(m_p);
     float* s_g = reinterpret_cast<float*>(smem + L::vec);
     float* s_b = s_g + 64;
     float* s_zk = s_b + 64;
@@ -645,15 +662,13 @@ linear_bwd_intra_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat1
 
     load_tile_async<64, K, LB_THREADS>(qns, qn + (tok0 * H + h) * K, (long)H * K, valid, tid);
     load_tile_async<64, K, LB_THREADS>(kns, kn + (tok0 * H + h) * K, (long)H * K, valid, tid);
-    load_tile_async<64, V, LB_THREADS>(vps, vp + (tok0 * H + h) * V, (long)H * V, valid, tid);
-    load_tile_async<64, V, LB_THREADS>(dos, d_o + (tok0 * H + h) * V, (long)H * V, valid, tid);
-    if (GDN) {
-        load_tile_async<64, K, LB_THREADS>(ws, w + (tok0 * H + h) * K, (long)H * K, valid, tid);
-        load_tile_async<64, K, LB_THREADS>(dws, dw_in + (tok0 * H + h) * K, (long)H * K, valid, tid);
-        load_tile_async<64, V, LB_THREADS>(us, u + (tok0 * H + h) * V, (long)H * V, valid, tid);
-        load_tile_async<64, V, LB_THREADS>(dvs, dvp + (tok0 * H + h) * V, (long)H * V, valid, tid);
-        load_tile_async<64, V, LB_THREADS>(smem_u32(smem + L::vs), v + (tok0 * H + h) * V, (long)H * V, valid, tid);
-    }
+    load_tile_async<64, V, LB_THREADS>(dt, vp + (tok0 * H + h) * V, (long)H * V, valid, tid);
+    load_tile_async<64, V, LB_THREADS>(ct, d_o + (tok0 * H + h) * V, (long)H * V, valid, tid);
+    auto load_state_parts = [&]() {                          // dk1 exists for updating chunks only
+        load_tile_async<64, K, LB_THREADS>(et, dq1 + (tok0 * H + h) * K, (long)H * K, valid, tid);
+        if (act) load_tile_async<64, K, LB_THREADS>(ft, dk1 + (tok0 * H + h) * K, (long)H * K, valid, tid);
+    };
+    if (!GDN) load_state_parts();
     cp_async_commit();
     if (tid < 64) {
         const long gi = (tok0 + min(tid, valid - 1)) * H + h;
@@ -684,7 +699,7 @@ linear_bwd_intra_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat1
         zero_acc(dpr);
         warp_gemm<K * 2, A_ROW, K * 2, B_NK, 4>(qk, qns, r0, kns, c0, 0, K, lane);
         if (GDN) warp_gemm<K * 2, A_ROW, K * 2, B_NK, 4>(kk, kns, r0, kns, c0, 0, K, lane);
-        warp_gemm<V * 2, A_ROW, V * 2, B_NK, 4>(dpr, dos, r0, vps, c0, 0, V, lane);
+        warp_gemm<V * 2, A_ROW, V * 2, B_NK, 4>(dpr, ct, r0, dt, c0, 0, V, lane);
         float rs_a = 0.f, rs_b = 0.f;
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) {
@@ -715,9 +730,14 @@ linear_bwd_intra_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat1
             s_dgr[(0 * 2 + half) * 64 + ia] = rs_a;
             s_dgr[(0 * 2 + half) * 64 + ib] = rs_b;
         }
-        store_acc_bf16<128, 4>(m1_p, dpr, r0, c0, lane);
+        store_acc_bf16<128, 4>(m_p, dpr, r0, c0, lane);
     }
     __syncthreads();
+    if (GDN) {                                               // do and v' are done with
+        load_tile_async<64, V, LB_THREADS>(ct, dvp + (tok0 * H + h) * V, (long)H * V, valid, tid);
+        load_tile_async<64, K, LB_THREADS>(dt, dw_in + (tok0 * H + h) * K, (long)H * K, valid, tid);
+        cp_async_commit();
+    }
 
     // ---- phase 2: dqn = dqk kn, dkn = dqk^T qn
     constexpr int NK = K / 16;
@@ -725,11 +745,12 @@ linear_bwd_intra_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat1
     float acc_q[NK][4], acc_k[NK][4];
     zero_acc(acc_q);
     zero_acc(acc_k);
-    warp_gemm<128, A_ROW, K * 2, B_KN, NK>(acc_q, m1, r0, kns, nk0, 0, 64, lane);
-    warp_gemm<128, A_TRANS, K * 2, B_KN, NK>(acc_k, m1, r0, qns, nk0, 0, 64, lane);
+    warp_gemm<128, A_ROW, K * 2, B_KN, NK>(acc_q, mt, r0, kns, nk0, 0, 64, lane);
+    warp_gemm<128, A_TRANS, K * 2, B_KN, NK>(acc_k, mt, r0, qns, nk0, 0, 64, lane);
 
     if (GDN) {
         // ---- phase 3: X_dd = (I + A_dd)^-1 (forward substitution, one warp per diagonal block), then H
+        __syncthreads();                                     // dqk has been read: X goes over it
         if (warp < 4 && lane < 16) {
             const int d0 = warp * 16, cidx = lane;
             float xcol[16];
@@ -747,7 +768,7 @@ linear_bwd_intra_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat1
         for (int e = tid; e < 4 * 16 * 16; e += LB_THREADS) {          // diagonal blocks: H_dd = X_dd
             const int d = e >> 8, r = (e >> 4) & 15, cc = e & 15;
             const int row = d * 16 + r, col = d * 16 + cc;
-            reinterpret_cast<__nv_bfloat16*>(hs_p + swz<128>(row, col >> 3))[col & 7] =
+            reinterpret_cast<__nv_bfloat16*>(e_p + swz<128>(row, col >> 3))[col & 7] =
                 __float2bfloat16(Xs[(d * 16 + r) * LB_X_LD + cc]);
         }
         for (int e = tid; e < 6 * 16 * 16; e += LB_THREADS) {          // below the diagonal: H_ji = -A_ji X_ii
@@ -759,22 +780,30 @@ linear_bwd_intra_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat1
 #pragma unroll
             for (int m = 0; m < 16; ++m) a -= As[(bj * 16 + r) * LB_A_LD + bi * 16 + m] * Xs[(bi * 16 + m) * LB_X_LD + cc];
             const int row = bj * 16 + r, col = bi * 16 + cc;
-            reinterpret_cast<__nv_bfloat16*>(hs_p + swz<128>(row, col >> 3))[col & 7] = __float2bfloat16(a);
+            reinterpret_cast<__nv_bfloat16*>(e_p + swz<128>(row, col >> 3))[col & 7] = __float2bfloat16(a);
         }
-        __syncthreads();
+        cp_async_wait<0>();
+        __syncthreads();                                     // H, dv', dw in place; A is done with
+        load_tile_async<64, K, LB_THREADS>(ft, w + (tok0 * H + h) * K, (long)H * K, valid, tid);
+        cp_async_commit();
         // ---- phase 4: [dzu | dzw] = (I + A)^-T [dv' | dw], in place, 32 columns per warp
         constexpr int NCG = (K + V) / 32;
         for (int cg = warp; cg < NCG; cg += 8) {
-            if (cg < V / 32) solve_t_group<V>(hs, dvs, dvs_p, cg * 32, lane);
-            else solve_t_group<K>(hs, dws, dws_p, (cg - V / 32) * 32, lane);
+            if (cg < V / 32) solve_t_group<V>(et, ct, c_p, cg * 32, lane);
+            else solve_t_group<K>(et, dt, d_p, (cg - V / 32) * 32, lane);
         }
-        __syncthreads();
+        cp_async_wait<0>();
+        __syncthreads();                                     // dzu, dzw and w in place; H is done with
+        load_tile_async<64, V, LB_THREADS>(et, u + (tok0 * H + h) * V, (long)H * V, valid, tid);
+        cp_async_commit();
         // ---- phase 5: dA = -strictLower(dzu u^T + dzw w^T); dkk = dA beta Gam; gradients of beta and the decays
         {
             float dar[4][4];
             zero_acc(dar);
-            warp_gemm<V * 2, A_ROW, V * 2, B_NK, 4>(dar, dvs, r0, us, c0, 0, V, lane);
-            warp_gemm<K * 2, A_ROW, K * 2, B_NK, 4>(dar, dws, r0, ws, c0, 0, K, lane);
+            warp_gemm<K * 2, A_ROW, K * 2, B_NK, 4>(dar, dt, r0, ft, c0, 0, K, lane);
+            cp_async_wait<0>();
+            __syncthreads();
+            warp_gemm<V * 2, A_ROW, V * 2, B_NK, 4>(dar, ct, r0, et, c0, 0, V, lane);
             float rs_a = 0.f, rs_b = 0.f, db_a = 0.f, db_b = 0.f;
 #pragma unroll
             for (int nt = 0; nt < 4; ++nt) {
@@ -807,12 +836,14 @@ linear_bwd_intra_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat1
                 s_dbp[half * 64 + ia] = db_a;
                 s_dbp[half * 64 + ib] = db_b;
             }
-            store_acc_bf16<128, 4>(m2_p, dar, r0, c0, lane);
+            store_acc_bf16<128, 4>(m_p, dar, r0, c0, lane);
         }
-        __syncthreads();
+        __syncthreads();                                     // u and w are done with
+        load_state_parts();
+        cp_async_commit();
         // ---- phase 6: dkn += dkk kn + dkk^T kn
-        warp_gemm<128, A_ROW, K * 2, B_KN, NK>(acc_k, m2, r0, kns, nk0, 0, 64, lane);
-        warp_gemm<128, A_TRANS, K * 2, B_KN, NK>(acc_k, m2, r0, kns, nk0, 0, 64, lane);
+        warp_gemm<128, A_ROW, K * 2, B_KN, NK>(acc_k, mt, r0, kns, nk0, 0, 64, lane);
+        warp_gemm<128, A_TRANS, K * 2, B_KN, NK>(acc_k, mt, r0, kns, nk0, 0, 64, lane);
         // ---- dv = dzu beta (in place), dbeta += <dzu, v>
         {
             constexpr int CPR = V / 8;
@@ -821,9 +852,10 @@ linear_bwd_intra_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat1
             const int sub = lane / CPR, cc = lane % CPR;
             for (int rr = 0; rr < 8; rr += RPP) {
                 const int r = warp * 8 + rr + sub;
-                uint4* pz = reinterpret_cast<uint4*>(dvs_p + swz<V * 2>(r, cc));
+                uint4* pz = reinterpret_cast<uint4*>(c_p + swz<V * 2>(r, cc));
                 uint4 z = *pz;
-                const uint4 vv = *reinterpret_cast<const uint4*>(vs_p + swz<V * 2>(r, cc));
+                uint4 vv = make_uint4(0, 0, 0, 0);
+                if (r < valid) vv = *reinterpret_cast<const uint4*>(v + ((tok0 + r) * H + h) * V + cc * 8);
                 uint32_t* zw = reinterpret_cast<uint32_t*>(&z);
                 const uint32_t* vw = reinterpret_cast<const uint32_t*>(&vv);
                 const float bt = s_b[r];
@@ -840,45 +872,33 @@ linear_bwd_intra_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat1
                 if (cc == 0) s_dbp[2 * 64 + r] = s;
             }
         }
+        cp_async_wait<0>();
+        __syncthreads();
     }
     // ---- phase 7: per-element epilogue in the accumulator layout of dqn / dkn
     {
         const float ega = __expf(s_g[ia]), egb = __expf(s_g[ib]);
         const float fa = s_b[ia] * ega, fb = s_b[ib] * egb;
         float zk_a = 0.f, zk_b = 0.f, dE_a = 0.f, dE_b = 0.f;
-        const __nv_bfloat16* dq1_a = dq1 + ((tok0 + ia) * H + h) * K;
-        const __nv_bfloat16* dq1_b = dq1 + ((tok0 + ib) * H + h) * K;
-        const __nv_bfloat16* dk1_a = dk1 + ((tok0 + ia) * H + h) * K;
-        const __nv_bfloat16* dk1_b = dk1 + ((tok0 + ib) * H + h) * K;
 #pragma unroll
         for (int nt = 0; nt < NK; ++nt) {
             const int col = nk0 + nt * 8 + qd * 2;
             const float2 kna = load_pair_bf16<K * 2>(kns_p, ia, col), knb = load_pair_bf16<K * 2>(kns_p, ib, col);
             const float2 qna = load_pair_bf16<K * 2>(qns_p, ia, col), qnb = load_pair_bf16<K * 2>(qns_p, ib, col);
             if (GDN) {
-                const float2 za = load_pair_bf16<K * 2>(dws_p, ia, col), zb = load_pair_bf16<K * 2>(dws_p, ib, col);
+                const float2 za = load_pair_bf16<K * 2>(d_p, ia, col), zb = load_pair_bf16<K * 2>(d_p, ib, col);
                 zk_a += za.x * kna.x + za.y * kna.y;
                 zk_b += zb.x * knb.x + zb.y * knb.y;
                 acc_k[nt][0] += za.x * fa; acc_k[nt][1] += za.y * fa;
                 acc_k[nt][2] += zb.x * fb; acc_k[nt][3] += zb.y * fb;
             }
-            if (ia < valid) {
-                const float2 x = unpack_bf16(*reinterpret_cast<const uint32_t*>(dq1_a + col));
-                acc_q[nt][0] += x.x; acc_q[nt][1] += x.y;
-                dE_a += x.x * qna.x + x.y * qna.y;
-                if (act) {
-                    const float2 y = unpack_bf16(*reinterpret_cast<const uint32_t*>(dk1_a + col));
-                    acc_k[nt][0] += y.x; acc_k[nt][1] += y.y;
-                }
-            }
-            if (ib < valid) {
-                const float2 x = unpack_bf16(*reinterpret_cast<const uint32_t*>(dq1_b + col));
-                acc_q[nt][2] += x.x; acc_q[nt][3] += x.y;
-                dE_b += x.x * qnb.x + x.y * qnb.y;
-                if (act) {
-                    const float2 y = unpack_bf16(*reinterpret_cast<const uint32_t*>(dk1_b + col));
-                    acc_k[nt][2] += y.x; acc_k[nt][3] += y.y;
-                }
+            const float2 xa = load_pair_bf16<K * 2>(e_p, ia, col), xb = load_pair_bf16<K * 2>(e_p, ib, col);
+            acc_q[nt][0] += xa.x; acc_q[nt][1] += xa.y; acc_q[nt][2] += xb.x; acc_q[nt][3] += xb.y;
+            dE_a += xa.x * qna.x + xa.y * qna.y;
+            dE_b += xb.x * qnb.x + xb.y * qnb.y;
+            if (act) {
+                const float2 ya = load_pair_bf16<K * 2>(f_p, ia, col), yb = load_pair_bf16<K * 2>(f_p, ib, col);
+                acc_k[nt][0] += ya.x; acc_k[nt][1] += ya.y; acc_k[nt][2] += yb.x; acc_k[nt][3] += yb.y;
             }
         }
         // dot products of the l2-norm backward, over the finished dqn / dkn
@@ -904,7 +924,7 @@ linear_bwd_intra_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat1
             atomicAdd(&s_dotk[ia], dk_a); atomicAdd(&s_dotk[ib], dk_b);
         }
     }
-    __syncthreads();                                         // row sums complete; w and dzw tiles are free
+    __syncthreads();                                         // row sums complete; dq1 and dk1 have been read
     // ---- phase 8: l2-norm backward, staging, stores
     {
         float qra = 1.f, qrb = 1.f, kra = 1.f, krb = 1.f;
@@ -926,8 +946,8 @@ linear_bwd_intra_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat1
             acc_k[nt][0] = kra * (acc_k[nt][0] - kna.x * pk_a); acc_k[nt][1] = kra * (acc_k[nt][1] - kna.y * pk_a);
             acc_k[nt][2] = krb * (acc_k[nt][2] - knb.x * pk_b); acc_k[nt][3] = krb * (acc_k[nt][3] - knb.y * pk_b);
         }
-        store_acc_bf16<K * 2, NK>(ws_p, acc_q, r0, nk0, lane);
-        store_acc_bf16<K * 2, NK>(dws_p, acc_k, r0, nk0, lane);
+        store_acc_bf16<K * 2, NK>(e_p, acc_q, r0, nk0, lane);
+        store_acc_bf16<K * 2, NK>(f_p, acc_k, r0, nk0, lane);
     }
     if (tid < 64) {
         const float eg = __expf(s_g[tid]);
@@ -949,9 +969,9 @@ linear_bwd_intra_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat1
         if (lane == 0) atomicAdd(&s_red[0], se);
     }
     __syncthreads();
-    store_tile<64, K, LB_THREADS>(ws_p, dq + (tok0 * H + h) * K, (long)H * K, valid, tid);
-    store_tile<64, K, LB_THREADS>(dws_p, dk + (tok0 * H + h) * K, (long)H * K, valid, tid);
-    if (GDN) store_tile<64, V, LB_THREADS>(dvs_p, dv + (tok0 * H + h) * V, (long)H * V, valid, tid);
+    store_tile<64, K, LB_THREADS>(e_p, dq + (tok0 * H + h) * K, (long)H * K, valid, tid);
+    store_tile<64, K, LB_THREADS>(f_p, dk + (tok0 * H + h) * K, (long)H * K, valid, tid);
+    if (GDN) store_tile<64, V, LB_THREADS>(c_p, dv + (tok0 * H + h) * V, (long)H * V, valid, tid);
     if (tid == 0) scal[(((long)b * NT + c) * H + h) * 4 + 3] = s_red[0];
 }
 
@@ -1051,7 +1071,7 @@ static int launch_dh(const void* qn, const void* kn, const void* w, const void* 
     const int smem = DhSmem<K, BV, GDN>::total(NT);
     int rc = reserve_smem(kern, smem, "natsl_linear_bwd_dh");
     if (rc != NATSL_OK) return rc;
-    kern<<<dim3(V / BV, H, B), DH_THREADS, smem, st>>>(bfc(qn), bfc(kn), bfc(w), bfc(d_o), bfc(dvl), gcs, carry, types_i,
+    kern<<<dim3(V / BV, H, B), BV * 4, smem, st>>>(bfc(qn), bfc(kn), bfc(w), bfc(d_o), bfc(dvl), gcs, carry, types_i,
                                                        indices, n_blocks, dht, bfm(dS_all), bfm(dvp), dh0, T, H, HN, V, scale);
     return check_launch("natsl_linear_bwd_dh");
 }
@@ -1120,13 +1140,17 @@ extern "C" int natsl_linear_bwd_dh(int rule, const void* qn, const void* kn, con
     NATSL_REQUIRE(V % 32 == 0, NATSL_ERR_UNSUPPORTED, "natsl_linear_bwd_dh: V must be a multiple of 32");
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
 #define NATSL_ARGS qn, kn, w, d_o, dvl, gcs, carry, types_i, indices, n_blocks, dht, dS_all, dvp, dh0, B, T, H, HN, V, scale, st
+    // slices of 64 value columns read q, k and w half as often; slices of 32 keep more SMs busy when there are few heads
+    const bool wide = V % 64 == 0 && (long)B * H * (V / 64) >= 148;
+#define NATSL_DH(KK, GDN) return wide ? launch_dh<KK, 64, GDN>(NATSL_ARGS) : launch_dh<KK, 32, GDN>(NATSL_ARGS)
     if (rule == NATSL_RULE_GDN) {
-        if (K == 64) return launch_dh<64, 32, true>(NATSL_ARGS);
-        if (K == 128) return launch_dh<128, 32, true>(NATSL_ARGS);
+        if (K == 64) NATSL_DH(64, true);
+        if (K == 128) NATSL_DH(128, true);
     } else {
-        if (K == 64) return launch_dh<64, 32, false>(NATSL_ARGS);
-        if (K == 128) return launch_dh<128, 32, false>(NATSL_ARGS);
+        if (K == 64) NATSL_DH(64, false);
+        if (K == 128) NATSL_DH(128, false);
     }
+#undef NATSL_DH
 #undef NATSL_ARGS
     set_error("natsl_linear_bwd_dh: unsupported key dim K=%d (64 or 128)", K);
     return NATSL_ERR_UNSUPPORTED;
