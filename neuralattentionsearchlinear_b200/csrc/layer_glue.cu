@@ -515,25 +515,30 @@ extern "C" int natsl_short_conv_fwd(const void* x, const void* w, const void* bi
 
 // The same backward for span = 64 with the tiles staged in shared memory: one CTA = 128 channels x 64 tokens, all loads
 // of the x tile (64 + 6 halo rows) and the dy tile (64 + 3) are issued at once with cp.async (the sliding-window form
-// above has two loads in flight per thread and is bound by their latency), warp s computes the tokens 8 s .. 8 s + 7 for
-// 32 groups of 8 channels, and the eight warps' weight-gradient partials are summed in shared memory in a fixed order:
-// one partial per CTA.
-constexpr int CB_TT = 64, CB_CG = 32, CB_CH = 4;      // tokens per CTA, threads across channels, channels per thread
-__global__ void __launch_bounds__(256, 3)
+// above has two loads in flight per thread and is bound by their latency).  What bounds it then is instruction issue, so
+// a warp (64 channels, two per lane: four would need 90 registers and leave two CTAs on an SM) slides over 16 tokens with
+// the window of x and of the pre-activation gradients in registers: each row is read and unpacked once and three of
+// nineteen gradients are computed twice.  The weight-gradient partials of the four warps of a channel group are summed in
+// shared memory in a fixed order: one partial per CTA.
+constexpr int CB_TT = 64, CB_CG = 32, CB_CH = 2;      // tokens per CTA, threads across channels, channels per thread
+constexpr int CB_GR = 2, CB_WT = 16;                  // channel groups per CTA, tokens per warp
+__global__ void __launch_bounds__(256, 4)
 short_conv_bwd_tile_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                            const __nv_bfloat16* __restrict__ bias, const __nv_bfloat16* __restrict__ dy,
                            __nv_bfloat16* __restrict__ dx, float* __restrict__ dw_part, int T, int D, int silu) {
     constexpr int W = CONV_W;
     constexpr int XR = CB_TT + 2 * (W - 1), YR = CB_TT + (W - 1);            // rows of the two tiles
-    constexpr int ROWB = CB_CG * CB_CH * 2;                                  // bytes per tile row
+    constexpr int ROWB = CB_GR * CB_CG * CB_CH * 2;                          // bytes per tile row
     constexpr int CPR = ROWB / 16;                                          // 16-byte chunks per tile row
+    static_assert(CB_TT / CB_WT * CB_GR == 8 && W == 4 && CB_CH == 2, "eight warps; a lane reads 4 bytes per row");
     extern __shared__ __align__(16) unsigned char smem_cb[];
     unsigned char* xs = smem_cb;
     unsigned char* ys = smem_cb + XR * ROWB;
-    const int tid = threadIdx.x, lane = tid & 31, sr = tid >> 5;
-    const int d_cta = blockIdx.x * CB_CG * CB_CH;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int grp = warp & (CB_GR - 1), sr = warp / CB_GR;
+    const int d_cta = blockIdx.x * CB_GR * CB_CG * CB_CH;
     const int t0 = blockIdx.y * CB_TT, b = blockIdx.z;
-    const int d0 = d_cta + lane * CB_CH;
+    const int d0 = d_cta + (grp * CB_CG + lane) * CB_CH;
     const bool ch_ok = d0 < D;
     {
         const uint32_t xs_a = smem_u32(xs), ys_a = smem_u32(ys);
@@ -562,21 +567,21 @@ short_conv_bwd_tile_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloa
     }
     cp_async_wait<0>();
     __syncthreads();
-    static_assert(CB_CH == 4, "a thread reads 8 bytes per row");
-    auto row8 = [&](const unsigned char* tile, int r, float (&f)[CB_CH]) {
-        const uint2 v = *reinterpret_cast<const uint2*>(tile + r * ROWB + lane * 8);
-        const float2 t0_ = unpack_bf16(v.x), t1_ = unpack_bf16(v.y);
-        f[0] = t0_.x; f[1] = t0_.y; f[2] = t1_.x; f[3] = t1_.y;
+    auto row = [&](const unsigned char* tile, int r, float (&f)[CB_CH]) {
+        const float2 v = unpack_bf16(*reinterpret_cast<const uint32_t*>(tile + r * ROWB + (grp * CB_CG + lane) * 4));
+        f[0] = v.x; f[1] = v.y;
     };
-    // token tt of the tile (0 .. 63 + halo): x rows tt .. tt + 3 of the x tile are its window, dy row tt its gradient.
-    // With `own` (a token of this warp's range, inside the sequence) its weight-gradient terms are added while the
-    // window is in registers.
-    auto dpre_at = [&](int tt, bool own, float (&dp)[CB_CH]) {
-        float xw[W][CB_CH];
+    // Step i of this warp: the pre-activation gradient of token ts + i (rows ts + i .. ts + i + 3 of the x tile are its
+    // window; dy is zero outside the sequence) and, from the third step on, dx of token ts + i - 3, which needs the
+    // gradients of tokens ts + i - 3 .. ts + i.  The weight gradients take the warp's own tokens only.
+    const int ts = sr * CB_WT;
+    float xw[W][CB_CH], dps[W][CB_CH];
 #pragma unroll
-        for (int j = 0; j < W; ++j) row8(xs, tt + j, xw[j]);
+    for (int j = 0; j < W - 1; ++j) row(xs, ts + j, xw[j]);
+    auto step = [&](int i, bool own) {
+        row(xs, ts + i + W - 1, xw[W - 1]);
         float g[CB_CH];
-        row8(ys, tt, g);                                   // zero outside the sequence
+        row(ys, ts + i, g);
 #pragma unroll
         for (int c = 0; c < CB_CH; ++c) {
             float a = bs[c];
@@ -584,30 +589,32 @@ short_conv_bwd_tile_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloa
             for (int j = 0; j < W; ++j) a += wt[c][j] * xw[j][c];
             if (silu) {
                 const float sg = sigmoidf_(a);
-                dp[c] = g[c] * sg * (1.f + a * (1.f - sg));
-            } else {
-                dp[c] = g[c];
+                g[c] = g[c] * sg * (1.f + a * (1.f - sg));
             }
             if (own) {
 #pragma unroll
-                for (int j = 0; j < W; ++j) dwa[c][j] += dp[c] * xw[j][c];
-                dwa[c][W] += dp[c];
+                for (int j = 0; j < W; ++j) dwa[c][j] += g[c] * xw[j][c];
+                dwa[c][W] += g[c];
             }
+#pragma unroll
+            for (int k = 0; k < W - 1; ++k) {
+                dps[k][c] = dps[k + 1][c];
+                xw[k][c] = xw[k + 1][c];
+            }
+            dps[W - 1][c] = g[c];
         }
     };
-    const int ts = sr * 8;                                  // first token of this warp inside the tile
-    float dps[W][CB_CH];                                        // dpre[tt .. tt + 3]
 #pragma unroll
-    for (int i = 1; i < W; ++i) dpre_at(ts + i - 1, true, dps[i]);        // dps[1..3] = dpre[ts .. ts+2] (dy = 0 past T)
-#pragma unroll 1
-    for (int i = 0; i < 8; ++i) {
-        const int tt = ts + i;
+    for (int c = 0; c < CB_CH; ++c)
 #pragma unroll
-        for (int k = 0; k < W - 1; ++k)
+        for (int k = 0; k < W; ++k) dps[k][c] = 0.f;
 #pragma unroll
-            for (int c = 0; c < CB_CH; ++c) dps[k][c] = dps[k + 1][c];
-        dpre_at(tt + W - 1, i + W - 1 < 8, dps[W - 1]);
-        if (t0 + tt < T) {
+    for (int i = 0; i < W - 1; ++i) step(i, true);
+#pragma unroll 4
+    for (int i = W - 1; i < CB_WT + W - 1; ++i) {
+        step(i, i < CB_WT);
+        const int t = t0 + ts + i - (W - 1);
+        if (t < T && ch_ok) {
             float o[CB_CH];
 #pragma unroll
             for (int c = 0; c < CB_CH; ++c) {
@@ -616,24 +623,25 @@ short_conv_bwd_tile_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloa
                 for (int j = 0; j < W; ++j) a += wt[c][j] * dps[W - 1 - j][c];
                 o[c] = a;
             }
-            if (ch_ok)
-                *reinterpret_cast<uint2*>(dx + ((long)b * T + t0 + tt) * D + d0) = make_uint2(pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]));
+            *reinterpret_cast<uint32_t*>(dx + ((long)b * T + t) * D + d0) = pack_bf16(o[0], o[1]);
         }
     }
-    // ---- the eight warps' partials -> one per CTA (fixed order)
+    // ---- the warps' partials -> one per CTA (fixed order)
     __syncthreads();
-    float* red = reinterpret_cast<float*>(smem_cb);          // [8 warps][CB_CH * (W + 1)][32 lanes]
+    constexpr int NW = CB_TT / CB_WT, PER = CB_CH * (W + 1) * CB_CG;
+    float* red = reinterpret_cast<float*>(smem_cb);          // [group][token warps][CB_CH * (W + 1)][32 lanes]
 #pragma unroll
     for (int c = 0; c < CB_CH; ++c)
 #pragma unroll
-        for (int j = 0; j <= W; ++j) red[(sr * CB_CH * (W + 1) + c * (W + 1) + j) * CB_CG + lane] = dwa[c][j];
+        for (int j = 0; j <= W; ++j) red[(grp * NW + sr) * PER + (c * (W + 1) + j) * CB_CG + lane] = dwa[c][j];
     __syncthreads();
-    for (int o = tid; o < CB_CH * (W + 1) * CB_CG; o += 256) {
+    for (int e = tid; e < CB_GR * PER; e += 256) {
+        const int gr = e / PER, o = e % PER;
         float a = 0.f;
 #pragma unroll
-        for (int s8 = 0; s8 < 8; ++s8) a += red[s8 * CB_CH * (W + 1) * CB_CG + o];
+        for (int k = 0; k < NW; ++k) a += red[(gr * NW + k) * PER + o];
         const int i = o / CB_CG, cgp = o % CB_CG;
-        const int dd = d_cta + cgp * CB_CH + i / (W + 1);
+        const int dd = d_cta + (gr * CB_CG + cgp) * CB_CH + i / (W + 1);
         if (dd < D) dw_part[(((long)b * gridDim.y + blockIdx.y) * D + dd) * (W + 1) + i % (W + 1)] = a;
     }
 }
@@ -646,14 +654,14 @@ extern "C" int natsl_short_conv_bwd(const void* x, const void* w, const void* bi
     NATSL_REQUIRE(W == CONV_W, NATSL_ERR_UNSUPPORTED, "natsl_short_conv_bwd: kernel size %d is not built (4)", W);
     const int groups = D / 8;
     if (span == CB_TT) {
-        constexpr int smem = ((CB_TT + 2 * (CONV_W - 1)) + (CB_TT + CONV_W - 1)) * CB_CG * CB_CH * 2;
+        constexpr int smem = ((CB_TT + 2 * (CONV_W - 1)) + (CB_TT + CONV_W - 1)) * CB_GR * CB_CG * CB_CH * 2;
         static_assert(smem >= 8 * CB_CH * (CONV_W + 1) * CB_CG * 4, "the partial sums are reduced over the tiles");
         cudaError_t e = cudaFuncSetAttribute(short_conv_bwd_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) {
             set_error("natsl_short_conv_bwd: cannot reserve %d B of shared memory (%s)", smem, cudaGetErrorString(e));
             return NATSL_ERR_CUDA;
         }
-        dim3 grid((D + CB_CG * CB_CH - 1) / (CB_CG * CB_CH), (T + CB_TT - 1) / CB_TT, B);
+        dim3 grid((D + CB_GR * CB_CG * CB_CH - 1) / (CB_GR * CB_CG * CB_CH), (T + CB_TT - 1) / CB_TT, B);
         short_conv_bwd_tile_kernel<<<grid, 256, smem, reinterpret_cast<cudaStream_t>(stream)>>>(
             bfc(x), bfc(w), bfc(bias), bfc(dy), bfm(dx), dw_part, T, D, silu);
         return check_launch("natsl_short_conv_bwd");
