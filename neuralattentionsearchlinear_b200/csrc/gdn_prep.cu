@@ -34,7 +34,7 @@ struct PrepSmem {
     static constexpr int Gs = Xs + 4 * 16 * X_LD * 4;          // bf16 [64][64] swizzled (128-byte rows)
     static constexpr int vec = Gs + 64 * 64 * 2;               // gcs, beta, rstd, wscale, q rstd: 5 x 64 floats
     static constexpr int total = vec + 5 * 64 * 4;
-    static constexpr int ctas = 3 * (total + 1024) <= 227 * 1024 ? 3 : 2;      // resident CTAs the register budget is set for
+    static constexpr int ctas = 4 * (total + 1024) <= 228 * 1024 ? 4 : 3 * (total + 1024) <= 227 * 1024 ? 3 : 2;      // resident CTAs the register budget is set for
     static_assert(Gs % 128 == 0, "G tile alignment");
 };
 
