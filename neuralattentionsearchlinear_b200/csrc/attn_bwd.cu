@@ -149,63 +149,52 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             const uint32_t kt = s_k + (j & 1) * (64 * DK * 2);
 #pragma unroll
             for (int kk = 0; kk < DK / 16; ++kk)
-                umma_ss(tmem + C_S, umma_desc(s_q + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
+                umma_ss_warp(tmem + C_S, umma_desc(s_q + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
                         umma_desc(kt + (kk >> 2) * 8192 + (kk & 3) * 32, 16, 1024), id_s, kk > 0);
-            umma_commit(bar_s);
+            umma_commit_warp(bar_s);
         };
         auto issue_dp = [&](int j) {                          // dO V_j^T
             const uint32_t vt = s_v + (j % VST) * (64 * DV * 2);
 #pragma unroll
             for (int kk = 0; kk < DV / 16; ++kk)
-                umma_ss(tmem + C_DP, umma_desc(s_do + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
+                umma_ss_warp(tmem + C_DP, umma_desc(s_do + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
                         umma_desc(vt + (kk >> 2) * 8192 + (kk & 3) * 32, 16, 1024), id_s, kk > 0);
-            umma_commit(bar_dp);
-            umma_commit(bar_v_empty + (j % VST) * 8);
+            umma_commit_warp(bar_dp);
+            umma_commit_warp(bar_v_empty + (j % VST) * 8);
         };
         bool ok = __all_sync(0xffffffffu, mbar_wait(bar_q, 0, status));
         if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_k_full, 0, status));
-        if (ok && lane == 0) {
+        if (ok) {
             tc_fence_after();
             issue_s(0);
         }
-        __syncwarp();
         if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_v_full, 0, status));
-        if (ok && lane == 0) {
+        if (ok) {
             tc_fence_after();
             issue_dp(0);
         }
-        __syncwarp();
         for (int j = 0; ok && j < n_tiles; ++j) {
             const int jn = j + 1;
             if (jn < n_tiles) {                               // the next scores as soon as these have been read
                 ok = __all_sync(0xffffffffu, mbar_wait(bar_k_full + (jn & 1) * 8, (jn >> 1) & 1, status));
                 if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_s_free, j & 1, status));
                 if (!ok) break;
-                if (lane == 0) {
-                    tc_fence_after();
-                    issue_s(jn);
-                }
-                __syncwarp();
+                tc_fence_after();
+                issue_s(jn);
             }
             ok = __all_sync(0xffffffffu, mbar_wait(bar_ds, j & 1, status));
             if (!ok) break;
-            if (lane == 0) {
-                tc_fence_after();
-                const uint32_t kt = s_k + (j & 1) * (64 * DK * 2);
+            tc_fence_after();
+            const uint32_t kt = s_k + (j & 1) * (64 * DK * 2);
 #pragma unroll
-                for (int kk = 0; kk < 4; ++kk)
-                    umma_ts(tmem + C_DQ, tmem + C_DP + kk * 8, umma_desc(kt + kk * 2048, 8192, 1024), id_dq, (j > 0 || kk > 0) ? 1u : 0u);
-                umma_commit(jn < n_tiles ? bar_k_empty + (j & 1) * 8 : bar_done);
-            }
-            __syncwarp();
+            for (int kk = 0; kk < 4; ++kk)
+                umma_ts_warp(tmem + C_DQ, tmem + C_DP + kk * 8, umma_desc(kt + kk * 2048, 8192, 1024), id_dq, (j > 0 || kk > 0) ? 1u : 0u);
+            umma_commit_warp(jn < n_tiles ? bar_k_empty + (j & 1) * 8 : bar_done);
             if (jn < n_tiles) {
                 ok = __all_sync(0xffffffffu, mbar_wait(bar_v_full + (jn % VST) * 8, (jn / VST) & 1, status));
                 if (!ok) break;
-                if (lane == 0) {
-                    tc_fence_after();
-                    issue_dp(jn);                             // behind ds k in the tensor pipe: ds may be overwritten
-                }
-                __syncwarp();
+                tc_fence_after();
+                issue_dp(jn);                                 // behind ds k in the tensor pipe: ds may be overwritten
             }
         }
     } else {
@@ -619,39 +608,38 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         constexpr uint32_t id_s = umma_idesc_bf16(128, 64, false);
         constexpr uint32_t id_acc = umma_idesc_bf16(128, 64, true) | (1u << 15);         // A MN-major too
         auto scores = [&](int n, int stg, int kv) {           // S and dO V^T of item n into buffer n & 1
-            if (lane == 0) {
-                tc_fence_after();
-                const uint32_t dos = sbase + L::stage + stg * L::stage_bytes, qs = dos + 128 * DV * 2;
-                const uint32_t kt = sbase + L::kv + kv * L::kv_bytes, vt = kt + 64 * DK * 2;
+            stg = __shfl_sync(0xffffffffu, stg, 0);
+            kv = __shfl_sync(0xffffffffu, kv, 0);
+            n = __shfl_sync(0xffffffffu, n, 0) & 1;
+            tc_fence_after();
+            const uint32_t dos = sbase + L::stage + stg * L::stage_bytes, qs = dos + 128 * DV * 2;
+            const uint32_t kt = sbase + L::kv + kv * L::kv_bytes, vt = kt + 64 * DK * 2;
 #pragma unroll
-                for (int kk = 0; kk < DK / 16; ++kk)
-                    umma_ss(tmem + C_S + (n & 1) * 64, umma_desc(qs + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
-                            umma_desc(kt + (kk >> 2) * 8192 + (kk & 3) * 32, 16, 1024), id_s, kk > 0);
+            for (int kk = 0; kk < DK / 16; ++kk)
+                umma_ss_warp(tmem + C_S + n * 64, umma_desc(qs + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
+                             umma_desc(kt + (kk >> 2) * 8192 + (kk & 3) * 32, 16, 1024), id_s, kk > 0);
 #pragma unroll
-                for (int kk = 0; kk < DV / 16; ++kk)
-                    umma_ss(tmem + C_DP + (n & 1) * 64, umma_desc(dos + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
-                            umma_desc(vt + (kk >> 2) * 8192 + (kk & 3) * 32, 16, 1024), id_s, kk > 0);
-                umma_commit(bar_s + (n & 1) * 8);
-            }
-            __syncwarp();
+            for (int kk = 0; kk < DV / 16; ++kk)
+                umma_ss_warp(tmem + C_DP + n * 64, umma_desc(dos + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
+                             umma_desc(vt + (kk >> 2) * 8192 + (kk & 3) * 32, 16, 1024), id_s, kk > 0);
+            umma_commit_warp(bar_s + n * 8);
         };
         auto accumulate = [&](int stg, int slot, bool cont, bool release) {
-            if (lane == 0) {
-                tc_fence_after();
-                const uint32_t dos = sbase + L::stage + stg * L::stage_bytes, qs = dos + 128 * DV * 2;
-                const uint32_t acc = tmem + C_ACC + slot * 128;
+            stg = __shfl_sync(0xffffffffu, stg, 0);
+            slot = __shfl_sync(0xffffffffu, slot, 0);
+            tc_fence_after();
+            const uint32_t dos = sbase + L::stage + stg * L::stage_bytes, qs = dos + 128 * DV * 2;
+            const uint32_t acc = tmem + C_ACC + slot * 128;
 #pragma unroll
-                for (int kk = 0; kk < 8; ++kk)                // dv^T += do^T p
-                    umma_ss(acc, umma_desc(dos + kk * 2048, 16384, 1024), umma_desc(sbase + L::p + kk * 2048, 8192, 1024), id_acc,
-                            (cont || kk > 0) ? 1u : 0u);
+            for (int kk = 0; kk < 8; ++kk)                    // dv^T += do^T p
+                umma_ss_warp(acc, umma_desc(dos + kk * 2048, 16384, 1024), umma_desc(sbase + L::p + kk * 2048, 8192, 1024), id_acc,
+                             (cont || kk > 0) ? 1u : 0u);
 #pragma unroll
-                for (int kk = 0; kk < 8; ++kk)                // dk^T += q^T ds
-                    umma_ss(acc + 64, umma_desc(qs + kk * 2048, 16384, 1024), umma_desc(sbase + L::ds + kk * 2048, 8192, 1024), id_acc,
-                            (cont || kk > 0) ? 1u : 0u);
-                umma_commit(bar_acc);
-                if (release) umma_commit(bar_empty + stg * 8);
-            }
-            __syncwarp();
+            for (int kk = 0; kk < 8; ++kk)                    // dk^T += q^T ds
+                umma_ss_warp(acc + 64, umma_desc(qs + kk * 2048, 16384, 1024), umma_desc(sbase + L::ds + kk * 2048, 8192, 1024), id_acc,
+                             (cont || kk > 0) ? 1u : 0u);
+            umma_commit_warp(bar_acc);
+            if (release) umma_commit_warp(bar_empty + stg * 8);
         };
         bool ok = true;
         if (paired) {
@@ -702,7 +690,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             for (int i = 0; ok && more; ++i) {
                 const bool first = ahead && __all_sync(0xffffffffu, mbar_test_wait(bar_full + (na & 1) * 8, (na >> 1) & 1));
                 if (first) step_ahead();
-                // the accumulators of tile u - 2 were read before the softmax warps arrived here for this item
+                // the accumulators of tile u - 2 were read before the softmax warps arrived here for the item before
                 if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_p, i & 1, status));
                 if (!ok) break;
                 accumulate(i & 1, ow.u & 1, !ow.first_of_tile(), true);
@@ -728,13 +716,14 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             lse_b = t_b < T ? lse[r + 8L * HQ] : 0.f;
             del_b = t_b < T ? delta[r + 8L * HQ] : 0.f;
         };
-        // p and ds of item i (key tile kt, query tile qt; `sel`: later blocks see the keys) into shared memory; adds the ds
-        // of later blocks' queries to dn
+        // p and ds of item i (key tile kt, query tile qt; `sel`: later blocks see the keys) into registers, bf16 pairs; adds
+        // the ds of later blocks' queries to dn.  Returns once the products of the previous item have read p and ds.
+        uint32_t sr[32];
         auto item_p = [&](int i, int kt, int qt, bool sel, float& dn) -> bool {
             bool ok = __all_sync(0xffffffffu, mbar_wait(bar_s + (i & 1) * 8, (i >> 1) & 1, status));
             if (!ok) return false;
             tc_fence_after();
-            uint32_t sr[32], dr[32];
+            uint32_t dr[32];
             tmem_ld_16x256b_x8(t_rows + C_S + (i & 1) * 64, sr);
             tmem_ld_16x256b_x8(t_rows + C_DP + (i & 1) * 64, dr);
             tmem_ld_wait();
@@ -770,9 +759,10 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 sr[4 * k + 3] = pack_bf16(d2, d3);
             }
             dn += (t_a >= blk_end ? sum_a : 0.f) + (t_b >= blk_end ? sum_b : 0.f);
-            // the products of the previous item have read p and ds
             if (i > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar_acc, (i - 1) & 1, status));
-            if (!ok) return false;
+            return ok;
+        };
+        auto item_write = [&]() {
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
                 const uint32_t oa = swz<128>(row_a, k) + (lane & 3) * 4, ob = swz<128>(row_b, k) + (lane & 3) * 4;
@@ -785,31 +775,39 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_p);
-            return true;
         };
-        // dk, dv of key tile kt from accumulator pair `slot` (zeros without `any`): lane = head-dim index, columns = keys, a
-        // warp writes 64 contiguous bytes per key
-        auto finish = [&](int kt, int slot, bool any) {
+        // dk, dv of key tile kt from accumulator pair `slot` (zeros without `any`): lane = head-dim index, columns = keys.
+        // Transposed through the p and ds tiles, which no product reads at that time, so that the rows leave in 16-byte
+        // pieces (two-byte stores straight from the registers took 8000 clocks a tile, most of an unselected tile's time).
+        // Every softmax warp calls it, also after a failed wait (`good` false: nothing is read or stored).
+        auto finish = [&](int kt, int slot, bool any, bool good) {
             const int d = quad * 32 + lane;
-            const long tok = (long)b * T + kt * 64 + half * 32;
-            const int n_valid = min(32, T - kt * 64 - half * 32);
             const uint32_t acc = tmem + ((uint32_t)(quad * 32) << 16) + C_ACC + slot * 128 + half * 32;
             tc_fence_after();
             uint32_t r[32];
-            if (quad * 32 < DV) {
+            if (good && quad * 32 < DV) {
                 tmem_ld32(acc, r);
                 tmem_ld_wait();
 #pragma unroll
                 for (int c = 0; c < 32; ++c)
-                    if (c < n_valid) dv[((tok + c) * HKV + hkv) * DV + d] = __float2bfloat16(any ? __uint_as_float(r[c]) : 0.f);
+                    *reinterpret_cast<__nv_bfloat16*>(p_t + swz<DV * 2>(half * 32 + c, d >> 3) + (d & 7) * 2) =
+                        __float2bfloat16(any ? __uint_as_float(r[c]) : 0.f);
             }
-            if (quad * 32 < DK) {
+            if (good && quad * 32 < DK) {
                 tmem_ld32(acc + 64, r);
                 tmem_ld_wait();
 #pragma unroll
                 for (int c = 0; c < 32; ++c)
-                    if (c < n_valid) dk[((tok + c) * HKV + hkv) * DK + d] = __float2bfloat16(any ? __uint_as_float(r[c]) * scale : 0.f);
+                    *reinterpret_cast<__nv_bfloat16*>(ds_t + swz<DK * 2>(half * 32 + c, d >> 3) + (d & 7) * 2) =
+                        __float2bfloat16(any ? __uint_as_float(r[c]) * scale : 0.f);
             }
+            tc_fence_before();
+            asm volatile("bar.sync 2, 256;" ::: "memory");
+            const long tok = (long)b * T + kt * 64;
+            const int n_valid = good ? min(64, T - kt * 64) : 0;
+            store_tile<64, DV, 256>(p_t, dv + (tok * HKV + hkv) * DV, (long)HKV * DV, n_valid, tid - 64);
+            store_tile<64, DK, 256>(ds_t, dk + (tok * HKV + hkv) * DK, (long)HKV * DK, n_valid, tid - 64);
+            asm volatile("bar.sync 2, 256;" ::: "memory");
         };
         bool ok = true;
         int i = 0;
@@ -839,32 +837,29 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 float add = 0.f;
                 ok = item_p(i, kt, w.qt, sel, add);
                 if (!ok) break;
+                item_write();
                 if (w.u) dn[1] += add; else dn[0] += add;
             }
             flush(gi);
             if (ok && i > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar_acc, (i - 1) & 1, status));
-            if (ok) {
-                finish(tile[0], 0, has_items(0));
-                if (tile[1] >= 0) finish(tile[1], 1, has_items(1));
-            }
+            finish(tile[0], 0, has_items(0), ok);
+            if (tile[1] >= 0) finish(tile[1], 1, has_items(1), ok);
         } else if (!own) {
-            for (int u = 0; u < n_own; ++u) finish(s_tile[u], 0, false);
+            for (int u = 0; u < n_own; ++u) finish(s_tile[u], 0, false, true);
         } else {
             int done = 0;                                     // tiles written
             float unused = 0.f;
             for (bool more = ow.begin(); more; more = ow.next(), ++i) {
                 load_rows(ow.gi, ow.qt);
-                ok = item_p(i, s_tile[ow.u], ow.qt, false, unused);
-                if (!ok) break;
-                // item_p has waited for the products of the previous item: a tile that ended there is complete
-                if (ow.u > done) {
-                    finish(s_tile[done], done & 1, true);
-                    tc_fence_before();
+                if (ok) ok = item_p(i, s_tile[ow.u], ow.qt, false, unused);
+                if (ow.u > done) {                            // the previous item was its tile's last
+                    finish(s_tile[done], done & 1, true, ok);
                     ++done;
                 }
+                if (ok) item_write();
             }
             if (ok && i > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar_acc, (i - 1) & 1, status));
-            if (ok && done < n_own) finish(s_tile[done], done & 1, true);
+            finish(s_tile[done], done & 1, true, ok);
         }
         asm volatile("bar.sync 1, 256;" ::: "memory");       // every softmax warp reaches it, also after a failed wait
         const int n_tiles = paired ? 2 : n_own;
