@@ -149,18 +149,18 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             const uint32_t kt = s_k + (j & 1) * (64 * DK * 2);
 #pragma unroll
             for (int kk = 0; kk < DK / 16; ++kk)
-                umma_ss_warp(tmem + C_S, umma_desc(s_q + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
+                umma_ss(tmem + C_S, umma_desc(s_q + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
                         umma_desc(kt + (kk >> 2) * 8192 + (kk & 3) * 32, 16, 1024), id_s, kk > 0);
-            umma_commit_warp(bar_s);
+            umma_commit(bar_s);
         };
         auto issue_dp = [&](int j) {                          // dO V_j^T
             const uint32_t vt = s_v + (j % VST) * (64 * DV * 2);
 #pragma unroll
             for (int kk = 0; kk < DV / 16; ++kk)
-                umma_ss_warp(tmem + C_DP, umma_desc(s_do + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
+                umma_ss(tmem + C_DP, umma_desc(s_do + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
                         umma_desc(vt + (kk >> 2) * 8192 + (kk & 3) * 32, 16, 1024), id_s, kk > 0);
-            umma_commit_warp(bar_dp);
-            umma_commit_warp(bar_v_empty + (j % VST) * 8);
+            umma_commit(bar_dp);
+            umma_commit(bar_v_empty + (j % VST) * 8);
         };
         bool ok = __all_sync(0xffffffffu, mbar_wait(bar_q, 0, status));
         if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_k_full, 0, status));
@@ -188,8 +188,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             const uint32_t kt = s_k + (j & 1) * (64 * DK * 2);
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk)
-                umma_ts_warp(tmem + C_DQ, tmem + C_DP + kk * 8, umma_desc(kt + kk * 2048, 8192, 1024), id_dq, (j > 0 || kk > 0) ? 1u : 0u);
-            umma_commit_warp(jn < n_tiles ? bar_k_empty + (j & 1) * 8 : bar_done);
+                umma_ts(tmem + C_DQ, tmem + C_DP + kk * 8, umma_desc(kt + kk * 2048, 8192, 1024), id_dq, (j > 0 || kk > 0) ? 1u : 0u);
+            umma_commit(jn < n_tiles ? bar_k_empty + (j & 1) * 8 : bar_done);
             if (jn < n_tiles) {
                 ok = __all_sync(0xffffffffu, mbar_wait(bar_v_full + (jn % VST) * 8, (jn / VST) & 1, status));
                 if (!ok) break;
@@ -616,13 +616,13 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             const uint32_t kt = sbase + L::kv + kv * L::kv_bytes, vt = kt + 64 * DK * 2;
 #pragma unroll
             for (int kk = 0; kk < DK / 16; ++kk)
-                umma_ss_warp(tmem + C_S + n * 64, umma_desc(qs + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
+                umma_ss(tmem + C_S + n * 64, umma_desc(qs + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
                              umma_desc(kt + (kk >> 2) * 8192 + (kk & 3) * 32, 16, 1024), id_s, kk > 0);
 #pragma unroll
             for (int kk = 0; kk < DV / 16; ++kk)
-                umma_ss_warp(tmem + C_DP + n * 64, umma_desc(dos + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
+                umma_ss(tmem + C_DP + n * 64, umma_desc(dos + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
                              umma_desc(vt + (kk >> 2) * 8192 + (kk & 3) * 32, 16, 1024), id_s, kk > 0);
-            umma_commit_warp(bar_s + n * 8);
+            umma_commit(bar_s + n * 8);
         };
         auto accumulate = [&](int stg, int slot, bool cont, bool release) {
             stg = __shfl_sync(0xffffffffu, stg, 0);
@@ -632,14 +632,14 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             const uint32_t acc = tmem + C_ACC + slot * 128;
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk)                    // dv^T += do^T p
-                umma_ss_warp(acc, umma_desc(dos + kk * 2048, 16384, 1024), umma_desc(sbase + L::p + kk * 2048, 8192, 1024), id_acc,
+                umma_ss(acc, umma_desc(dos + kk * 2048, 16384, 1024), umma_desc(sbase + L::p + kk * 2048, 8192, 1024), id_acc,
                              (cont || kk > 0) ? 1u : 0u);
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk)                    // dk^T += q^T ds
-                umma_ss_warp(acc + 64, umma_desc(qs + kk * 2048, 16384, 1024), umma_desc(sbase + L::ds + kk * 2048, 8192, 1024), id_acc,
+                umma_ss(acc + 64, umma_desc(qs + kk * 2048, 16384, 1024), umma_desc(sbase + L::ds + kk * 2048, 8192, 1024), id_acc,
                              (cont || kk > 0) ? 1u : 0u);
-            umma_commit_warp(bar_acc);
-            if (release) umma_commit_warp(bar_empty + stg * 8);
+            umma_commit(bar_acc);
+            if (release) umma_commit(bar_empty + stg * 8);
         };
         bool ok = true;
         if (paired) {

@@ -5,7 +5,7 @@
 //   warp 0    TMA producer: Q once, then the K and V tiles of the key-tile walk into a 3- or 4-stage and a
 //             2-stage ring (cp.async.bulk.tensor, 128-byte swizzle, zero fill past the sequence end), in the
 //             order in which the tensor core frees the stages;
-//   warp 1    MMA issuer (one thread): S_j = Q K_j^T into one of two (DV = 128) or three (DV = 64) TMEM score
+//   warp 1    MMA issuer (one elected lane): S_j = Q K_j^T into one of two (DV = 128) or three (DV = 64) TMEM score
 //             buffers, issued that many tiles ahead, and O += P_j V_j with P read straight from TMEM;
 //             completion is signalled with tcgen05.commit on mbarriers;
 //   warps 2-9 softmax, 16 query rows per warp, four threads per row (tcgen05.ld.16x256b fragments):
@@ -210,7 +210,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         // ------------------------------------------------------------ MMA issuer
         constexpr uint32_t idesc_qk = umma_idesc_bf16(128, 64, false);
         constexpr uint32_t idesc_pv = umma_idesc_bf16(128, DV, true);
-        auto issue_qk = [&](int j) {                  // S_{j&1} = Q K_j^T   (lane 0 only)
+        auto issue_qk = [&](int j) {                  // S_{j&1} = Q K_j^T   (the whole warp)
             const int sb = j % NSB, stg = j % TC_KST;
             const uint32_t kt = s_k + stg * (64 * DK * 2);
 #pragma unroll
@@ -225,7 +225,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         bool ok = __all_sync(0xffffffffu, mbar_wait(bar_q, 0, status));
         for (int j = 0; ok && j < min(NSB, n_tiles); ++j) {
             ok = __all_sync(0xffffffffu, mbar_wait(bar_k_full + (j % TC_KST) * 8, (j / TC_KST) & 1, status));
-            if (ok && lane == 0) {
+            if (ok) {
                 tc_fence_after();
                 issue_qk(j);
             }
@@ -236,7 +236,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             ok = __all_sync(0xffffffffu, mbar_wait(bar_v_full + vstg * 8, (j / TC_VST) & 1, status));
             if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_p_full + sb * 8, (j / NSB) & 1, status));
             if (!ok) break;
-            if (lane == 0) {
+            {
                 tc_fence_after();
                 const uint32_t vt = s_v + vstg * (64 * DV * 2);
 #pragma unroll
@@ -252,7 +252,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 const int jn = j + NSB;
                 ok = __all_sync(0xffffffffu, mbar_wait(bar_k_full + (jn % TC_KST) * 8, (jn / TC_KST) & 1, status));
                 if (!ok) break;
-                if (lane == 0) {
+                {
                     tc_fence_after();
                     issue_qk(jn);
                 }

@@ -346,7 +346,7 @@ attn_fwd_tc_persist_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                 }
                 if (!ok) break;
                 AT_T0();
-                if (lane == 0) {
+                {
                     tc_fence_after();
                     const uint32_t kt = s_k + stg * (64 * DK * 2);
 #pragma unroll
@@ -390,7 +390,7 @@ attn_fwd_tc_persist_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                 AT_ADD(0);
             }
             if (!ok) break;
-            if (lane == 0) {
+            {
                 tc_fence_after();
                 const uint32_t vt = s_v + vstg * (64 * DV * 2);
 #pragma unroll

@@ -225,7 +225,8 @@ gdn_prep_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         }
         __syncwarp();
         mbar_wait(bar_load, 0, status);
-        if (lane == 0) {
+        __syncwarp();
+        {
             constexpr uint32_t id_1 = umma_idesc_bf16(128, 64, false);
             tc_fence_after();
 #pragma unroll
@@ -237,12 +238,16 @@ gdn_prep_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         }
         __syncwarp();
         mbar_wait(bar_ai, 0, status);
-        if (lane == 0) {
+        __syncwarp();
+        {
             constexpr uint32_t id_2 = umma_idesc_bf16(128, 64, false) | (1u << 15);      // A MN-major (features x tokens)
             // every thread has finished with A (and fenced): the v tile may land on it
-            mbar_expect_tx(bar_v, 16384);
-            tma_load_4d(sbase + L::v, &map_v, 0, h, t0, b, bar_v);
-            tma_load_4d(sbase + L::v + 8192, &map_v, 64, h, t0, b, bar_v);
+            if (lane == 0) {
+                mbar_expect_tx(bar_v, 16384);
+                tma_load_4d(sbase + L::v, &map_v, 0, h, t0, b, bar_v);
+                tma_load_4d(sbase + L::v + 8192, &map_v, 64, h, t0, b, bar_v);
+            }
+            __syncwarp();
             tc_fence_after();
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk) {
@@ -254,7 +259,8 @@ gdn_prep_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         }
         __syncwarp();
         mbar_wait(bar_v, 0, status);
-        if (lane == 0) {
+        __syncwarp();
+        {
             constexpr uint32_t id_2 = umma_idesc_bf16(128, 64, false) | (1u << 15);
             tc_fence_after();
 #pragma unroll

@@ -188,7 +188,7 @@ gdn_walk_half_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
             if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_sready, c & 1, status));
             if (!ok) break;
             const uint32_t d1 = tmem + ((c & 1) ? WH_D1B : WH_D1);
-            if (lane == 0) {
+            {
                 tc_fence_after();
 #pragma unroll
                 for (int kk = 0; kk < 8; ++kk) {
@@ -202,7 +202,7 @@ gdn_walk_half_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
             ok = __all_sync(0xffffffffu, mbar_wait(bar_pv, c & 1, status));
             if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_fk, c & 1, status));
             if (!ok) break;
-            if (lane == 0) {
+            {
                 // the state update first: the next chunk's products wait for it, the output does not
                 tc_fence_after();
                 if (m_sel[c]) {
@@ -219,7 +219,7 @@ gdn_walk_half_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
             ok = __all_sync(0xffffffffu, mbar_wait(bar_pfull, c & 1, status));
             if (ok && c > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar_odone, (c - 1) & 1, status));   // D2 is free
             if (!ok) break;
-            if (lane == 0) {
+            {
                 tc_fence_after();
 #pragma unroll
                 for (int kk = 0; kk < 4; ++kk) {

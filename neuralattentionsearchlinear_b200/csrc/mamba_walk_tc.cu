@@ -228,7 +228,7 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_pv, c & 1, status));
             MW_ACC(1);
             if (!ok) break;
-            if (lane == 0) {
+            {
                 // the update of the last chunk of an unselected block would be thrown away: it is not issued
                 tc_fence_after();
                 if ((fl & MW_ACTIVE) && !(fl & MW_RESTORE)) {
@@ -251,7 +251,7 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             constexpr uint32_t id_1 = umma_idesc_bf16(128, 64, true);                   // [0;q] S
             constexpr uint32_t id_2 = umma_idesc_bf16(128, 64, true);                   // P v
             bool ok = __all_sync(0xffffffffu, mbar_wait(bar_full, 0, status));
-            if (ok && lane == 0) {                     // q k^T of chunk 0
+            if (ok) {                     // q k^T of chunk 0
                 tc_fence_after();
 #pragma unroll
                 for (int kk = 0; kk < 8; ++kk) {
@@ -277,7 +277,7 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 const bool ahead = c + 1 < NT;
                 if (ok && ahead) ok = __all_sync(0xffffffffu, mbar_wait(bar_full + nstg * 8, ((c + 1) / L::nstage) & 1, status));
                 MW_ACC(4);
-                if (ok && lane == 0) {
+                if (ok) {
                     // q S of this chunk and q k^T of the next one, K-step by K-step in turn
                     tc_fence_after();
                     const uint32_t d1 = tmem + ((c & 1) ? MW_D1B : MW_D1);
@@ -304,7 +304,7 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 if (ok && c > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar_odone, (c - 1) & 1, status));   // D2 is free
                 MW_ACC(6);
                 if (!ok) break;
-                if (lane == 0) {
+                {
                     tc_fence_after();
 #pragma unroll
                     for (int kk = 0; kk < 4; ++kk) {
