@@ -1,0 +1,46 @@
+"""GPU test (-m gpu) of the fp32 kernels at the edges of their tiles (groups of 32 or 16 tokens, 16 value columns; 16
+queries x 64 keys) against the CPU oracle in float64.  Sums of at most a few hundred fp32 products: 1e-4 as in the parity
+tests of the op."""
+import pytest
+import torch
+
+from oracle import attn as oattn
+from oracle import gdn as ogdn
+from oracle import tables as otab
+from tests.helpers import assert_close, synth_gdn_inputs
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("T,K,V,nbs", [(1, 64, 64, 64), (31, 32, 32, 64), (33, 96, 48, 64), (64, 128, 64, 64), (65, 192, 16, 64),
+                                       (161, 256, 64, 128), (130, 64, 128, 128)])
+def test_token_recurrence(T, K, V, nbs):
+    import neuralattentionsearchlinear_b200 as nat
+    from neuralattentionsearchlinear_b200 import _lib, _ops
+    B, H = 2, 3
+    q, k, v, g, beta, h0 = synth_gdn_inputs(B, T, H, K, V, seed=T + K, dtype=torch.float32)
+    types = otab.synth_types(B, -(-T // nbs), H, 0.5, seed=T)
+    cu = lambda x: x.cuda()
+    tb = nat.build_selection_tables(cu(types), T, nbs)
+    for rule in ("gdn", "mamba"):
+        gdn = rule == "gdn"
+        scale = K ** -0.5 if gdn else 1.0
+        o, ht, _ = _ops.linear_recurrent(_lib.RULE_GDN if gdn else _lib.RULE_MAMBA, cu(q), cu(k), cu(v), cu(g), cu(beta) if gdn else None,
+                                         tb, scale, cu(h0), True, gdn)
+        ref, s = ogdn.linear_recurrent(q.double(), k.double(), v.double(), g.double(), beta.double() if gdn else None, types[..., 1],
+                                       nbs=nbs, scale=scale, h0=h0.double(), decay=True, use_l2norm=gdn, rule=rule)
+        assert_close(o, ref.float(), 1e-4, f"o {rule}")
+        assert_close(ht, s.float(), 1e-4, f"state {rule}")
+
+
+@pytest.mark.parametrize("T,D,nbs", [(1, 64, 64), (17, 32, 64), (65, 64, 64), (200, 128, 128)])
+def test_fp32_attention(T, D, nbs):
+    import neuralattentionsearchlinear_b200 as nat
+    B, H = 2, 2
+    q, k, v, g, beta, _ = synth_gdn_inputs(B, T, H, D, D, seed=T + D, dtype=torch.float32)
+    types = otab.synth_types(B, -(-T // nbs), H, 0.5, seed=T)
+    cu = lambda x: x.cuda()
+    _, o, _ = nat.nats_mixed_attn_gdn(cu(q), cu(k), cu(v), cu(q), cu(k), cu(v), None, cu(g), cu(beta), cu(types), None,
+                                      nats_block_size=nbs, ops_for_incomplete_chunks="all", decay_for_non_gdn_blocks=True)
+    ref, _ = oattn.attn_sdpa(q.double(), k.double(), v.double(), oattn.attn_mask(types[..., 0], T, nbs, H))
+    assert_close(o, ref.float(), 1e-4, "o")
