@@ -269,6 +269,7 @@ def hybrid_fwd(rule: int, q_attn, k_attn, v_attn, q, k, v, g, beta, types, nbs: 
         _need(t_.dtype == q.dtype, "q, k, v of both branches must share a dtype", TypeError)
     fp32 = q.dtype == torch.float32
     _need(fp32 or q.dtype == BF16, f"unsupported dtype {q.dtype} (fp32 or bf16)", TypeError)
+    _need(not (fp32 and want_start), "the block-start state needs bf16 tensors", TypeError)
     q_attn, k_attn, v_attn, q, k, v = (t_.contiguous() for t_ in (q_attn, k_attn, v_attn, q, k, v))
     B, T, H, K = q.shape
     V, HQ, DK, HKV, DV = v.shape[3], q_attn.shape[2], q_attn.shape[3], k_attn.shape[2], v_attn.shape[3]

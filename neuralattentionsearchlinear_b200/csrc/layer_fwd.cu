@@ -395,6 +395,10 @@ int check_hybrid(const natsl_hybrid_args& a) {
     NATSL_REQUIRE(a.rule == NATSL_RULE_GDN || (a.rule == NATSL_RULE_MAMBA && ((a.K == 128 && a.V == 64) || (a.options & NATSL_HYBRID_FP32))),
                   NATSL_ERR_UNSUPPORTED,
                   "natsl_hybrid_forward: Mamba2 is built for K = 128, V = 64 (got K=%d V=%d)", a.K, a.V);
+    // the token recurrence behind this option steps over the end of an unfinished last block and knows no types of its own
+    // for a finished one: its block-start state is not the one a decoder rolls back to
+    NATSL_REQUIRE(!((a.options & NATSL_HYBRID_FP32) && a.hstart), NATSL_ERR_UNSUPPORTED,
+                  "natsl_hybrid_forward: no block-start state of fp32 tensors");
     NATSL_REQUIRE(a.workspace_bytes >= hybrid_layout(a).total, NATSL_ERR_TOO_LARGE, "natsl_hybrid_forward: workspace of %ld bytes, %ld needed",
                   (long)a.workspace_bytes, hybrid_layout(a).total);
     return NATSL_OK;

@@ -340,7 +340,7 @@ def nats_mixed_attn_gdn_chunk_inference(
     T = q_lattn.shape[1]
     want = bool(output_final_state_gated_delta)
     with torch.no_grad():
-        if _ops.walks_with_state(_lib.RULE_GDN, q_lattn.shape[-1], v_lattn.shape[-1], T):
+        if q_lattn.dtype != torch.float32 and _ops.walks_with_state(_lib.RULE_GDN, q_lattn.shape[-1], v_lattn.shape[-1], T):
             assert not want or T % nats_block_size or op_type_last_chunk is not None
             o_gdn, o_attn, _, ht, start, _ = _ops.hybrid_fwd(
                 _lib.RULE_GDN, q_attn, k_attn, v_attn, q_lattn, k_lattn, v_lattn, g, beta, nats_block_types, nats_block_size,
