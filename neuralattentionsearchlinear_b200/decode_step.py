@@ -59,9 +59,10 @@ class _Plan:
             elif p.dtype != BF16:
                 return False
             setattr(a, field, p.data_ptr())
-            return p.is_cuda and p.is_contiguous() and p.device == layer.q_proj.weight.device
+            return p.is_cuda and p.is_contiguous() and p.device == self.device
 
         m = layer
+        self.device = m.q_proj.weight.device
         good = all([weight("w_q", m.q_proj), weight("w_k", m.k_proj), weight("w_v", m.v_proj), weight("w_a", m.a_proj),
                     weight("w_g", m.g_proj), weight("w_o", m.o_proj), weight("cw_q", m.q_conv1d), weight("cw_k", m.k_conv1d),
                     weight("cw_v", m.v_conv1d), weight("cb_q", m.q_conv1d, "bias"), weight("cb_k", m.k_conv1d, "bias"),
@@ -197,7 +198,8 @@ def decode_token(layer, x: torch.Tensor, container):
     if x.dim() != 3 or x.shape[1] != 1 or x.dtype != BF16 or not x.is_cuda or layer.layer_idx is None or not hasattr(container, "layer"):
         return None
     plan = layer_plan(layer)
-    if not plan.ok:
+    # the kernel reads and writes batch * hidden entries of x and the output: every token's width and device count
+    if not plan.ok or x.shape[2] != plan.args.hidden or x.device != plan.device:
         return None
     nbs = layer.nats_block_size
     cache = container.layer(layer.layer_idx, nbs)
@@ -206,8 +208,7 @@ def decode_token(layer, x: torch.Tensor, container):
     step = cache._step
     if (step is None or step.plan is not plan or step.args.B != B
             or step.options != (layer.ops_for_incomplete_chunks, layer.attn_with_short_conv)):
-        if (B > MAX_BATCH or x.shape[2] != plan.args.hidden or x.device != layer.q_proj.weight.device
-                or layer.ops_for_incomplete_chunks == 'attn' or not layer.incomplete_block_start_with_ht
+        if (B > MAX_BATCH or layer.ops_for_incomplete_chunks == 'attn' or not layer.incomplete_block_start_with_ht
                 or not (layer.use_short_conv and layer.use_gate)):
             return None
         step = _Step(plan, layer, cache, B, x.device)
