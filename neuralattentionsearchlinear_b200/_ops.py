@@ -7,7 +7,7 @@ import os
 import torch
 
 from . import _lib
-from .nats_util import _TYPE_CODES, SelectionTables, cdiv, current_stream_ptr
+from .nats_util import _TYPE_CODES, SelectionTables, aligned, cdiv, current_stream_ptr
 
 BF16 = torch.bfloat16
 USE_MAMBA_WALK = os.environ.get("NATSL_MAMBA_WALK", "1") != "0"    # natsl_mamba_walk_fused (K = 128, V = 64)
@@ -196,7 +196,7 @@ def linear_fwd(rule: int, q, k, v, g, beta, tables: SelectionTables, scale: floa
         torch.cuda.current_stream(dev).wait_event(tables_event)
     ht = torch.empty(B, H, K, V, dtype=torch.float32, device=dev) if output_final_state else None
     if h0 is not None:
-        h0 = h0.float().contiguous()
+        h0 = aligned(h0.float().contiguous())
         _need(tuple(h0.shape) == (B, H, K, V), f"initial state must be [B,H,K,V], got {tuple(h0.shape)}")
     flags = (_lib.FLAG_DECAY_SKIPPED if decay else 0) | (0 if trailing_quirk else _lib.FLAG_NO_TRAILING_QUIRK)
     start, last_code = None, _lib.DT_F32
@@ -300,7 +300,7 @@ def hybrid_fwd(rule: int, q_attn, k_attn, v_attn, q, k, v, g, beta, types, nbs: 
         _need(beta.dtype in (BF16, torch.float32), "beta must be bf16 or fp32", TypeError)
         a.beta, a.beta_dtype = beta.data_ptr(), _dt_code(beta)
     if h0 is not None:
-        h0 = h0.float().contiguous()
+        h0 = aligned(h0.float().contiguous())
         _need(tuple(h0.shape) == (B, H, K, V), f"initial state must be [B,H,K,V], got {tuple(h0.shape)}")
         a.h0 = h0.data_ptr()
     o_lin = torch.empty(B, T, H, V, dtype=q.dtype, device=dev)

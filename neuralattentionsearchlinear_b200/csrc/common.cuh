@@ -23,6 +23,12 @@ int check_launch(const char* what);
         }                                       \
     } while (0)
 
+// Whether every pointer starts on a multiple of `n` bytes (NULL does): kernels with wide accesses take it on trust.
+template <typename... P>
+inline bool aligned_to(uintptr_t n, const P*... p) {
+    return ((... | reinterpret_cast<uintptr_t>(p)) & (n - 1)) == 0;
+}
+
 enum : int {
     NATSL_OK = 0,
     NATSL_ERR_BAD_SHAPE = -1,

@@ -798,6 +798,10 @@ extern "C" int natsl_decode_step(const natsl_decode_args* args, void* stream) {
                       a.dt_bias && a.conv_q && a.conv_k && a.conv_v && a.state && a.start && a.g_block && a.k_cache &&
                       a.v_cache && a.workspace && (a.n_done == 0 || a.types) && (a.rule != NATSL_RULE_GDN || a.w_b),
                   NATSL_ERR_NULL, "natsl_decode_step: null pointer");
+    NATSL_REQUIRE(aligned_to(16, a.x, a.w_q, a.w_k, a.w_v, a.w_a, a.w_b, a.w_g, a.w_o, a.w_mix, a.state, a.start, a.k_cache, a.v_cache,
+                             a.workspace) &&
+                      aligned_to(8, a.cw_q, a.cw_k, a.cw_v, a.conv_q, a.conv_k, a.conv_v),
+                  NATSL_ERR_UNSUPPORTED, "natsl_decode_step: a tensor does not start on 16 bytes (convolution weights and tails: 8)");
     NATSL_REQUIRE(a.pos >= 0 && a.pos < a.cap && a.n_done >= 0 && a.n_done == a.pos / a.nbs, NATSL_ERR_BAD_SHAPE,
                   "natsl_decode_step: pos=%d cap=%d finished blocks=%d", a.pos, a.cap, a.n_done);
     NATSL_REQUIRE((a.types_new != nullptr) == ((a.pos + 1) % a.nbs == 0), NATSL_ERR_BAD_SHAPE,

@@ -395,6 +395,9 @@ int check_hybrid(const natsl_hybrid_args& a) {
     NATSL_REQUIRE(a.rule == NATSL_RULE_GDN || (a.rule == NATSL_RULE_MAMBA && ((a.K == 128 && a.V == 64) || (a.options & NATSL_HYBRID_FP32))),
                   NATSL_ERR_UNSUPPORTED,
                   "natsl_hybrid_forward: Mamba2 is built for K = 128, V = 64 (got K=%d V=%d)", a.K, a.V);
+    NATSL_REQUIRE((a.options & NATSL_HYBRID_FP32) || aligned_to(16, a.q_attn, a.k_attn, a.v_attn, a.q, a.k, a.v, a.h0, a.o_attn, a.o_lin, a.ht,
+                                                                a.hstart, a.workspace),
+                  NATSL_ERR_UNSUPPORTED, "natsl_hybrid_forward: q, k, v, states, outputs and workspace must start on 16 bytes");
     // the token recurrence behind this option steps over the end of an unfinished last block and knows no types of its own
     // for a finished one: its block-start state is not the one a decoder rolls back to
     NATSL_REQUIRE(!((a.options & NATSL_HYBRID_FP32) && a.hstart), NATSL_ERR_UNSUPPORTED,
@@ -549,6 +552,10 @@ extern "C" int natsl_layer_forward(const natsl_layer_args* args, void* stream) {
     const LayerLayout l = layer_layout(a, h);
     NATSL_REQUIRE(a.workspace_bytes >= l.total, NATSL_ERR_TOO_LARGE, "natsl_layer_forward: workspace of %ld bytes, %ld needed",
                   (long)a.workspace_bytes, l.total);
+    NATSL_REQUIRE(aligned_to(16, a.x, a.q_raw, a.k_raw, a.v_raw, a.w_a, a.w_b, a.w_mix, a.o_lin, a.o_attn, a.k_attn, a.v_attn, a.v_lin,
+                             a.workspace) &&
+                      aligned_to(8, a.cw_q, a.cw_k, a.cw_v, a.tail_q, a.tail_k, a.tail_v) && aligned_to(4, a.logits, a.mix),
+                  NATSL_ERR_UNSUPPORTED, "natsl_layer_forward: a tensor does not start on 16 bytes (convolution weights and tails: 8)");
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     unsigned char* ws = reinterpret_cast<unsigned char*>(a.workspace);
     auto cb = [](const void* p) { return reinterpret_cast<const bf16*>(p); };

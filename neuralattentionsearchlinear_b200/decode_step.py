@@ -13,7 +13,7 @@ import torch.nn as nn
 
 from . import _lib
 from .modules import FusedMultiInputRMSNormGated, L2Norm, RMSNorm, ShortConvolution
-from .nats_util import current_stream_ptr
+from .nats_util import aligned, current_stream_ptr
 
 BF16 = torch.bfloat16
 MAX_BATCH = 64
@@ -59,7 +59,9 @@ class _Plan:
             elif p.dtype != BF16:
                 return False
             setattr(a, field, p.data_ptr())
-            return p.is_cuda and p.is_contiguous() and p.device == self.device
+            # products read 16 bytes at a time, convolutions 8: a parameter that is a view into a flat buffer may start anywhere
+            align = 16 if field.startswith("w_") else 8 if field.startswith("cw_") else 1
+            return p.is_cuda and p.is_contiguous() and p.device == self.device and p.data_ptr() % align == 0
 
         m = layer
         self.device = m.q_proj.weight.device
@@ -157,6 +159,8 @@ class _Step:
             cache.conv_state = tuple(t.contiguous() for t in cache.conv_state)
         if cache.block_types is not None and not cache.block_types.is_contiguous():
             cache.block_types = cache.block_types.contiguous()
+        if any(t.data_ptr() % 16 for t in (cache.state, cache.state_block_start, cache._k_buf, cache._v_buf, *cache.conv_state)):
+            return False
         types = cache.block_types
         if types is not None:
             if types.dtype not in (BF16, torch.float32):
@@ -236,7 +240,7 @@ def _decode(layer, x, cache, step, pos: int, nbs: int):
     n_done = pos // nbs
     if n_done and (cache.block_types is None or cache.block_types.shape[1] != n_done):
         return None
-    x = x.contiguous()
+    x = aligned(x.contiguous())
     types_new = None
     if (pos + 1) % nbs == 0:                                 # a block's type is decided once its last token is known
         pooled = ((cache.pool_sum + x[:, 0].float()) / nbs).to(x.dtype)[:, None, :]

@@ -12,7 +12,7 @@ import torch.nn.functional as F
 from . import _lib, _ops
 from .decode_step import layer_plan
 from .modules import hard_softmax
-from .nats_util import cdiv, current_stream_ptr
+from .nats_util import aligned, cdiv, current_stream_ptr
 
 BF16 = torch.bfloat16
 
@@ -42,7 +42,7 @@ def layer_forward(layer, x: torch.Tensor, cache=None):
         return None
     gdn = rule == _lib.RULE_GDN
     dev = x.device
-    x = x.contiguous()
+    x = aligned(x.contiguous())
     st = current_stream_ptr(dev)
     TN = cdiv(T, nbs)
     bf = dict(dtype=BF16, device=dev)

@@ -29,6 +29,11 @@ def current_stream_ptr(device) -> int:
     return torch.cuda.current_stream(device).cuda_stream
 
 
+def aligned(t: torch.Tensor) -> torch.Tensor:
+    """A contiguous tensor as one that starts on 16 bytes: itself, or a copy where it is a view that does not."""
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 @dataclass
 class SelectionTables:
     """All int32, on the device.  Shapes: types_i / indices [B,TN,HN,2]; n_blocks [B,HN,2];

@@ -77,3 +77,74 @@ def test_token_of_another_width_raises(nat, rule):
             assert cache[0].n_tokens == t and torch.equal(cache[0].state, state)
             call(layer, x[:, t:t + 1], cache)
     assert cache[0].n_tokens == 72
+
+
+def shift(t):
+    """The same values in a tensor that starts one element behind a 16-byte boundary."""
+    buf = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)
+    out = buf[1:].view(t.shape)
+    out.copy_(t.detach())
+    assert out.data_ptr() % 16 == t.element_size()
+    return out
+
+
+def prompt_and_tokens(nat, layer, x, T):
+    cache = nat.NAtSCache()
+    with torch.no_grad():
+        ys = [call(layer, x[:, :T].contiguous(), cache)] + [call(layer, x[:, t:t + 1], cache) for t in range(T, x.shape[1])]
+    return torch.cat(ys, 1)
+
+
+@pytest.mark.parametrize("rule,name", [("gdn", n) for n in ("q_proj", "a_proj", "b_proj", "o_proj", "nats_out_weights_layer", "k_conv1d")]
+                         + [("mamba", n) for n in ("v_proj", "g_proj", "v_conv1d")])
+def test_unaligned_parameters_take_the_general_path(nat, rule, name, monkeypatch):
+    """Views into a flat buffer: the fast paths decline them and the results are the general path's."""
+    from neuralattentionsearchlinear_b200 import natsl_attn_gdn, natsl_attn_mamba2
+    from neuralattentionsearchlinear_b200.decode_step import layer_plan
+    layer, x = make_layer(nat, rule), tokens(2, 130)
+    m = getattr(layer, name)
+    m.weight.data = shift(m.weight)
+    assert not layer_plan(layer).ok
+    got = prompt_and_tokens(nat, layer, x, 126)
+    for mod in (natsl_attn_gdn, natsl_attn_mamba2):
+        monkeypatch.setattr(mod, "layer_forward", lambda *a: None)
+        monkeypatch.setattr(mod, "decode_token", lambda *a: None)
+    assert torch.equal(got, prompt_and_tokens(nat, layer, x, 126))
+
+
+@pytest.mark.parametrize("rule", ["gdn", "mamba"])
+def test_unaligned_inputs(nat, rule):
+    """Prompt, tokens and initial state of any address give what aligned ones give."""
+    layer, x = make_layer(nat, rule), tokens(1, 130)
+    with torch.no_grad():
+        a, b = nat.NAtSCache(), nat.NAtSCache()
+        assert torch.equal(call(layer, x[:, :128], a), call(layer, shift(x[:, :128]), b))
+        for t in (128, 129):
+            assert torch.equal(call(layer, x[:, t:t + 1].contiguous(), a), call(layer, shift(x[:, t:t + 1]), b))
+        K, V = (64, 64) if rule == "gdn" else (128, 64)
+        args, types, _ = op_inputs(rule, 1, 100, 2, K, V, 64)
+        h0 = torch.randn(1, 2, K, V, device="cuda")
+        op = nat.nats_mixed_attn_gdn if rule == "gdn" else nat.nats_mixed_attn_mamba
+        run = lambda h: op(*args[:6], h, *args[7:], types, None, nats_block_size=64, ops_for_incomplete_chunks="all")[0]
+        assert torch.equal(run(h0), run(shift(h0)))
+
+
+def test_entry_points_refuse_unaligned_pointers(nat):
+    """The library itself: an error code before any launch."""
+    import ctypes
+
+    from neuralattentionsearchlinear_b200 import _lib
+    layer, x = make_layer(nat), tokens(1, 66)
+    cache = nat.NAtSCache()
+    with torch.no_grad():
+        call(layer, x[:, :64], cache)
+        call(layer, x[:, 64:65], cache)
+    st = torch.cuda.current_stream().cuda_stream
+    args = cache[0]._step.args
+    for field in ("x", "w_q", "w_mix", "cw_v", "state", "k_cache"):
+        bad = _lib.DecodeArgs()
+        ctypes.memmove(ctypes.byref(bad), ctypes.byref(args), ctypes.sizeof(bad))
+        bad.pos, bad.types_new = 65, None
+        setattr(bad, field, getattr(bad, field) + 2)
+        with pytest.raises(_lib.NatslError, match="start on 16 bytes"):
+            _lib.call("natsl_decode_step", ctypes.byref(bad), st)
