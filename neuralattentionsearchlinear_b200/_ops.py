@@ -7,7 +7,7 @@ import os
 import torch
 
 from . import _lib
-from .nats_util import _TYPE_CODES, SelectionTables, aligned, cdiv, current_stream_ptr
+from .nats_util import _TYPE_CODES, SelectionTables, aligned, cdiv, current_stream_ptr, device_guard
 
 BF16 = torch.bfloat16
 USE_MAMBA_WALK = os.environ.get("NATSL_MAMBA_WALK", "1") != "0"    # natsl_mamba_walk_fused (K = 128, V = 64)
@@ -331,7 +331,8 @@ def hybrid_fwd(rule: int, q_attn, k_attn, v_attn, q, k, v, g, beta, types, nbs: 
     a.ht, a.hstart = _lib.ptr(ht), _lib.ptr(start)
     if fp32:
         a.options |= _lib.HYBRID_FP32
-        _lib.call("natsl_hybrid_forward", ctypes.byref(a), current_stream_ptr(dev))
+        with device_guard(dev):
+            _lib.call("natsl_hybrid_forward", ctypes.byref(a), current_stream_ptr(dev))
         return o_lin, o_attn, lse, ht, start, flat
     key = (rule, B, T, H, K, V)
     need = _hybrid_ws.get(key)
@@ -341,7 +342,8 @@ def hybrid_fwd(rule: int, q_attn, k_attn, v_attn, q, k, v, g, beta, types, nbs: 
         need = _hybrid_ws[key] = _lib.load().natsl_hybrid_workspace_bytes(ctypes.byref(a))
     ws = torch.empty(need, dtype=torch.uint8, device=dev)
     a.workspace, a.workspace_bytes = ws.data_ptr(), need
-    _lib.call("natsl_hybrid_forward", ctypes.byref(a), current_stream_ptr(dev))
+    with device_guard(dev):
+        _lib.call("natsl_hybrid_forward", ctypes.byref(a), current_stream_ptr(dev))
     return o_lin, o_attn, lse, ht, start, flat
 
 

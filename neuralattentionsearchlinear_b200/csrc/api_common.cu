@@ -27,6 +27,23 @@ int check_launch(const char* what) {
     return NATSL_OK;
 }
 
+int check_device(const void* p, const char* what) {
+    int dev = -1;
+    cudaPointerAttributes at = {};
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaPointerGetAttributes(&at, p);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        set_error("%s: CUDA error %d (%s)", what, (int)e, cudaGetErrorString(e));
+        return NATSL_ERR_CUDA;
+    }
+    NATSL_REQUIRE(at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged, NATSL_ERR_UNSUPPORTED,
+                  "%s: a tensor is not in device memory", what);
+    NATSL_REQUIRE(at.type == cudaMemoryTypeManaged || at.device == dev, NATSL_ERR_UNSUPPORTED,
+                  "%s: the tensors are on device %d, the current device is %d", what, at.device, dev);
+    return NATSL_OK;
+}
+
 }  // namespace natsl
 
 extern "C" const char* natsl_last_error(void) { return natsl::g_err; }

@@ -791,7 +791,7 @@ extern "C" int64_t natsl_decode_workspace_bytes(const natsl_decode_args* args) {
 
 extern "C" int natsl_decode_step(const natsl_decode_args* args, void* stream) {
     using namespace natsl;
-    const int rc = check(reinterpret_cast<const Args*>(args));
+    int rc = check(reinterpret_cast<const Args*>(args));
     if (rc != NATSL_OK) return rc;
     const Args& a = *reinterpret_cast<const Args*>(args);
     NATSL_REQUIRE(a.x && a.out && a.w_q && a.w_k && a.w_v && a.w_a && a.w_g && a.w_o && a.cw_q && a.cw_k && a.cw_v && a.A_log &&
@@ -809,6 +809,8 @@ extern "C" int natsl_decode_step(const natsl_decode_args* args, void* stream) {
     const Layout l = layout(a);
     NATSL_REQUIRE(a.workspace_bytes >= l.total, NATSL_ERR_TOO_LARGE, "natsl_decode_step: workspace of %ld bytes, %ld needed",
                   (long)a.workspace_bytes, l.total);
+    rc = check_device(a.x, "natsl_decode_step");
+    if (rc != NATSL_OK) return rc;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     unsigned char* ws = a.workspace;
     const int HK = a.H * a.K, HV = a.H * a.V, DK = HK / a.HQ, DV = HV / a.HQ;

@@ -485,7 +485,8 @@ extern "C" int natsl_hybrid_forward(const natsl_hybrid_args* args, void* stream)
     using namespace natsl;
     NATSL_REQUIRE(args, NATSL_ERR_NULL, "natsl_hybrid_forward: null argument block");
     NATSL_REQUIRE(args->types_dtype >= 0 && args->types_dtype <= NATSL_DT_I32, NATSL_ERR_UNSUPPORTED, "natsl_hybrid_forward: bad types dtype");
-    const int rc = check_hybrid(*args);
+    int rc = check_hybrid(*args);
+    if (rc == NATSL_OK) rc = check_device(args->q, "natsl_hybrid_forward");
     if (rc != NATSL_OK) return rc;
     return hybrid_forward(*args, nullptr, reinterpret_cast<cudaStream_t>(stream), [](cudaStream_t) { return (int)NATSL_OK; });
 }
@@ -570,7 +571,8 @@ extern "C" int natsl_layer_forward(const natsl_layer_args* args, void* stream) {
     n.dt = mamba ? reinterpret_cast<float*>(ws + l.dt) : nullptr;
     n.gcs = mamba ? n.dt + (long)a.B * a.T * a.H : nullptr;
     n.out = mb(ws + l.beta);
-    int rc = launch_narrow(n, a.B, st);
+    int rc = check_device(a.x, "natsl_layer_forward");
+    if (rc == NATSL_OK) rc = launch_narrow(n, a.B, st);
     if (rc != NATSL_OK) return rc;
 
     // where each tensor of the two branches lives: the delta rule's k and v convolutions double as the softmax branch's

@@ -13,7 +13,7 @@ import torch.nn as nn
 
 from . import _lib
 from .modules import FusedMultiInputRMSNormGated, L2Norm, RMSNorm, ShortConvolution
-from .nats_util import aligned, current_stream_ptr
+from .nats_util import aligned, current_stream_ptr, device_guard
 
 BF16 = torch.bfloat16
 MAX_BATCH = 64
@@ -218,7 +218,7 @@ def decode_token(layer, x: torch.Tensor, container):
         step = _Step(plan, layer, cache, B, x.device)
     if torch.is_autocast_enabled() or torch.nn.modules.module._has_any_global_hook():
         return None
-    with torch.no_grad():
+    with torch.no_grad(), device_guard(plan.device):
         return _decode(layer, x, cache, step, pos, nbs)
 
 

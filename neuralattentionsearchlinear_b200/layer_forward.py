@@ -12,7 +12,7 @@ import torch.nn.functional as F
 from . import _lib, _ops
 from .decode_step import layer_plan
 from .modules import hard_softmax
-from .nats_util import aligned, cdiv, current_stream_ptr
+from .nats_util import aligned, cdiv, current_stream_ptr, device_guard
 
 BF16 = torch.bfloat16
 
@@ -34,12 +34,19 @@ def layer_forward(layer, x: torch.Tensor, cache=None):
         return None
     B, T, D = x.shape
     d = plan.args
-    H, K, V, HQ, HN, nbs, rule = d.H, d.K, d.V, d.HQ, d.HN, d.nbs, d.rule
     sel = layer.nats_layer
-    if (D != d.hidden or x.device != layer.q_proj.weight.device or not _ops.walks_with_state(rule, K, V, T) or B > 65535
+    if (D != d.hidden or x.device != plan.device or not _ops.walks_with_state(d.rule, d.K, d.V, T) or B > 65535
             or type(sel) is not nn.Linear or sel.bias is not None or sel.weight.dtype != BF16 or sel._forward_hooks
             or sel._forward_pre_hooks or not sel.weight.is_cuda):
         return None
+    with device_guard(x.device):
+        return _forward(layer, plan, x, cache)
+
+
+def _forward(layer, plan, x, cache):
+    B, T, D = x.shape
+    d, sel = plan.args, layer.nats_layer
+    H, K, V, HQ, HN, nbs, rule = d.H, d.K, d.V, d.HQ, d.HN, d.nbs, d.rule
     gdn = rule == _lib.RULE_GDN
     dev = x.device
     x = aligned(x.contiguous())

@@ -7,6 +7,7 @@ tensor (a device-to-host sync, nats_util.py:29-32).  Here one C-ABI call
 """
 from __future__ import annotations
 
+import contextlib
 from dataclasses import dataclass
 
 import torch
@@ -27,6 +28,14 @@ def cdiv(a: int, b: int) -> int:
 
 def current_stream_ptr(device) -> int:
     return torch.cuda.current_stream(device).cuda_stream
+
+
+_SAME_DEVICE = contextlib.nullcontext()
+
+
+def device_guard(device: torch.device):
+    """Context in which ``device`` is the current one: the library launches on the current device's streams."""
+    return _SAME_DEVICE if device.index == torch.cuda.current_device() else torch.cuda.device(device)
 
 
 def aligned(t: torch.Tensor) -> torch.Tensor:

@@ -148,3 +148,56 @@ def test_entry_points_refuse_unaligned_pointers(nat):
         setattr(bad, field, getattr(bad, field) + 2)
         with pytest.raises(_lib.NatslError, match="start on 16 bytes"):
             _lib.call("natsl_decode_step", ctypes.byref(bad), st)
+
+
+# ------------------------------------------------------------------------------------------------ the current device
+@pytest.mark.parametrize("what", ["gdn op", "mamba op", "fp32 op", "prompt", "token"])
+def test_work_runs_with_the_tensors_device_current(nat, what, monkeypatch):
+    """With another device current, the op and the layers switch to the tensors' device around their launches."""
+    layer, x = make_layer(nat), tokens(1, 66)
+    cache = nat.NAtSCache()
+    with torch.no_grad():
+        call(layer, x[:, :64], cache)
+    args, types, _ = op_inputs("mamba" if what == "mamba op" else "gdn", 1, 64, 2, 128 if what == "mamba op" else 64, 64, 64,
+                               dtype=torch.float32 if what == "fp32 op" else torch.bfloat16)
+    op = nat.nats_mixed_attn_mamba if what == "mamba op" else nat.nats_mixed_attn_gdn
+    entered = []
+
+    class Guard:
+        def __init__(self, device):
+            self.index = torch.device(device).index if not isinstance(device, int) else device
+
+        def __enter__(self):
+            entered.append(self.index)
+
+        def __exit__(self, *exc):
+            pass
+
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 1)
+    monkeypatch.setattr(torch.cuda, "device", Guard)
+    with torch.no_grad():
+        if what == "prompt":
+            call(layer, x[:, :64])
+        elif what == "token":
+            call(layer, x[:, 64:65], cache)
+        else:
+            op(*args, types, None, nats_block_size=64, ops_for_incomplete_chunks="all")
+    assert entered and set(entered) == {0}
+
+
+def test_library_refuses_memory_of_another_place(nat):
+    """A host address in place of a tensor of the current device: an error code before any launch."""
+    import ctypes
+
+    from neuralattentionsearchlinear_b200 import _lib
+    layer, x = make_layer(nat), tokens(1, 66)
+    cache = nat.NAtSCache()
+    with torch.no_grad():
+        call(layer, x[:, :64], cache)
+        call(layer, x[:, 64:65], cache)
+    bad = _lib.DecodeArgs()
+    ctypes.memmove(ctypes.byref(bad), ctypes.byref(cache[0]._step.args), ctypes.sizeof(bad))
+    host = torch.zeros(256, dtype=torch.bfloat16, pin_memory=True)
+    bad.pos, bad.types_new, bad.x = 65, None, host.data_ptr()
+    with pytest.raises(_lib.NatslError, match="device memory"):
+        _lib.call("natsl_decode_step", ctypes.byref(bad), torch.cuda.current_stream().cuda_stream)
