@@ -12,7 +12,7 @@ import torch
 import torch.nn as nn
 
 from . import _lib
-from .modules import FusedMultiInputRMSNormGated, L2Norm, RMSNorm, ShortConvolution
+from .modules import FusedMultiInputRMSNormGated, L2Norm, RMSNorm, ShortConvolution, mean_pooling
 from .nats_util import aligned, current_stream_ptr, device_guard
 
 BF16 = torch.bfloat16
@@ -20,8 +20,17 @@ MAX_BATCH = 64
 _tls = threading.local()                     # one argument block per thread: a call in flight is never rewritten
 
 
+# Attributes of a layer that the plan's argument blocks or its choice of path are made from; hooks of the general path that an
+# instance may have replaced (normally absent from its __dict__).
+_LAYER_ATTRS = ("num_heads num_v_heads num_attn_heads num_nats_head n_ops hidden_size key_dim value_dim head_k_dim head_v_dim "
+                "head_attn_k_dim head_attn_v_dim nats_block_size attn_qk_norm attn_with_short_conv use_short_conv use_gate "
+                "ops_for_incomplete_chunks incomplete_block_start_with_ht usg_for_attn outputs_are_weighted outputs_are_wighted "
+                "decay_for_non_gdn_blocks decay_for_non_mamba_blocks allow_neg_eigval pooling_func").split()
+_LAYER_HOOKS = ("select", "project", "project_qkv", "mix", "_ops_for_cache")
+
+
 class _Plan:
-    """Argument block of one layer: shapes, options and weight pointers, valid while ``current()`` holds."""
+    """Argument blocks of one layer: shapes, options and weight pointers, valid while ``current()`` holds."""
 
     def __init__(self, layer):
         self.ok = False
@@ -39,19 +48,28 @@ class _Plan:
             mods["nats_out_weights_layer"] = nn.Linear
         if layer.attn_qk_norm:
             mods["q_norm"] = mods["k_norm"] = RMSNorm
-        self.mods = []
-        for n, type_ in mods.items():
-            m = layer._modules.get(n)
-            self.mods.append((layer._modules, n, m))
-            if type(m) is not type_:
-                return                       # ok stays False
-        self.hooks = [h for _, _, m in self.mods for h in (m._forward_hooks, m._forward_pre_hooks)]
+        self.mods = [(layer._modules, n, layer._modules.get(n)) for n in mods]
+        attrs = [(layer.__dict__, n) for n in (*_LAYER_ATTRS, *_LAYER_HOOKS)]
+        attrs += [(m.__dict__, n) for _, _, m in self.mods if m is not None and not isinstance(m, nn.Linear)
+                  for n in ("eps", "activation", "kernel_size", "hidden_size")]
+        self.hooks, self.params, self.device = [], [], None
+        if all(type(m) is mods[n] for _, n, m in self.mods):
+            self.hooks = [h for _, _, m in self.mods for h in (m._forward_hooks, m._forward_pre_hooks)]
+            self.ok = self._fill(layer, gdn, weighted) and not any(h in layer.__dict__ for h in _LAYER_HOOKS)
+        # what current() compares, as flat sequences for one pass in C each
+        self._mod_d, self._mod_n, self._mod_v = zip(*self.mods)
+        self._att_d, self._att_n = zip(*attrs)
+        self._att_v = list(map(dict.get, self._att_d, self._att_n))
+        self._par_d, self._par_n, self._par_v = zip(*self.params) if self.params else ((), (), ())
+        self._tensors = [t for t in self._par_v if t is not None]
+        self._ptrs = [t.data_ptr() for t in self._tensors]
+
+    def _fill(self, layer, gdn: bool, weighted: bool) -> bool:
         a = self.args = _lib.DecodeArgs()
-        self.params = []
 
         def weight(field, owner, name="weight", any_float=None):
             p = owner._parameters.get(name)
-            self.params.append((owner._parameters, name, p, 0 if p is None else p.data_ptr()))
+            self.params.append((owner._parameters, name, p))
             if p is None:
                 return True
             if any_float is not None and p.dtype == torch.float32:
@@ -65,56 +83,55 @@ class _Plan:
 
         m = layer
         self.device = m.q_proj.weight.device
-        good = all([weight("w_q", m.q_proj), weight("w_k", m.k_proj), weight("w_v", m.v_proj), weight("w_a", m.a_proj),
-                    weight("w_g", m.g_proj), weight("w_o", m.o_proj), weight("cw_q", m.q_conv1d), weight("cw_k", m.k_conv1d),
-                    weight("cw_v", m.v_conv1d), weight("cb_q", m.q_conv1d, "bias"), weight("cb_k", m.k_conv1d, "bias"),
-                    weight("cb_v", m.v_conv1d, "bias"), weight("A_log", m, "A_log", "alog_f32"),
-                    weight("dt_bias", m, "dt_bias", "dt_f32"), weight("w1", m.o_norm, "weight1", "w12_f32"),
-                    weight("w2", m.o_norm, "weight2", "w12_f32")])
+        checks = [weight("w_q", m.q_proj), weight("w_k", m.k_proj), weight("w_v", m.v_proj), weight("w_a", m.a_proj),
+                  weight("w_g", m.g_proj), weight("w_o", m.o_proj), weight("cw_q", m.q_conv1d), weight("cw_k", m.k_conv1d),
+                  weight("cw_v", m.v_conv1d), weight("cb_q", m.q_conv1d, "bias"), weight("cb_k", m.k_conv1d, "bias"),
+                  weight("cb_v", m.v_conv1d, "bias"), weight("A_log", m, "A_log", "alog_f32"),
+                  weight("dt_bias", m, "dt_bias", "dt_f32"), weight("w1", m.o_norm, "weight1", "w12_f32"),
+                  weight("w2", m.o_norm, "weight2", "w12_f32")]
         if gdn:
-            good = good and weight("w_b", m.b_proj)
-        if weighted:
-            good = good and weight("w_mix", m.nats_out_weights_layer)
-        if m.attn_qk_norm:
-            good = good and weight("qn_w", m.q_norm, "weight", "qn_f32") and weight("kn_w", m.k_norm, "weight", "kn_f32")
-            good = good and m.q_norm.eps == m.k_norm.eps
-            a.norm_eps = m.q_norm.eps
-        if not gdn:
-            good = good and m.q_norm2.eps == m.k_norm2.eps
+            checks.append(weight("w_b", m.b_proj))
+        else:
+            checks.append(m.q_norm2.eps == m.k_norm2.eps)
             a.l2_eps = m.q_norm2.eps
+        if weighted:
+            checks.append(weight("w_mix", m.nats_out_weights_layer))
+        if m.attn_qk_norm:
+            checks += [weight("qn_w", m.q_norm, "weight", "qn_f32"), weight("kn_w", m.k_norm, "weight", "kn_f32"),
+                       m.q_norm.eps == m.k_norm.eps]
+            a.norm_eps = m.q_norm.eps
         w1, w2 = m.o_norm.weight1, m.o_norm.weight2
         DK, DV = m.head_attn_k_dim, m.head_attn_v_dim
-        self.ok = bool(
-            good and all(mod.bias is None for mod in (m.q_proj, m.k_proj, m.v_proj, m.a_proj, m.g_proj, m.o_proj))
+        ok = bool(
+            all(checks) and all(mod.bias is None for mod in (m.q_proj, m.k_proj, m.v_proj, m.a_proj, m.g_proj, m.o_proj))
             and (w1 is None) == (w2 is None) and (w1 is None or w1.dtype == w2.dtype)
             and m.num_v_heads == m.num_heads and m.n_ops == 2 and m.o_norm.hidden_size == DV
             and all(c.kernel_size == (4,) and c.activation == m.q_conv1d.activation for c in (m.q_conv1d, m.k_conv1d, m.v_conv1d))
             and m.hidden_size % 32 == 0 and m.value_dim % 32 == 0 and m.head_k_dim % 32 == 0 and m.head_k_dim <= 256
             and m.head_v_dim % 32 == 0 and DK in (64, 128) and DV in (64, 128) and m.key_dim <= 10240
-            and m.num_heads % m.num_nats_head == 0 and m.num_attn_heads % m.num_nats_head == 0)
+            and m.num_heads % m.num_nats_head == 0 and m.num_attn_heads % m.num_nats_head == 0
+            and m.use_short_conv and m.use_gate and m.ops_for_incomplete_chunks != 'attn' and m.incomplete_block_start_with_ht
+            and not m.usg_for_attn and m.pooling_func is mean_pooling)
         a.hidden, a.H, a.K, a.V, a.HQ, a.HN = (m.hidden_size, m.num_heads, m.head_k_dim, m.head_v_dim, m.num_attn_heads,
                                                m.num_nats_head)
         a.nbs, a.rule = m.nats_block_size, _lib.RULE_GDN if gdn else _lib.RULE_MAMBA
         a.silu = int(m.q_conv1d.activation in ("silu", "swish"))
         a.mix_sigmoid, a.mix_eps = int(m.o_norm.activation == "sigmoid"), m.o_norm.eps
         a.scale_attn, a.scale_lin = DK ** -0.5, m.head_k_dim ** -0.5 if gdn else 1.0
+        a.own_chunk, a.attn_conv = int(m.ops_for_incomplete_chunks == 'all'), int(m.attn_with_short_conv)
+        a.decay = int(m.decay_for_non_gdn_blocks if gdn else m.decay_for_non_mamba_blocks)
+        a.neg_eigval = int(gdn and m.allow_neg_eigval)
         self.ws_bytes = {}
         b = self.layer_args = _lib.LayerArgs()
-        for n in ("hidden H K V HQ HN nbs rule silu qn_f32 kn_f32 alog_f32 dt_f32 norm_eps l2_eps scale_attn scale_lin w_a w_b "
-                  "w_mix cw_q cw_k cw_v cb_q cb_k cb_v qn_w kn_w A_log dt_bias").split():
+        for n in ("hidden H K V HQ HN nbs rule attn_conv silu own_chunk decay neg_eigval qn_f32 kn_f32 alog_f32 dt_f32 norm_eps l2_eps "
+                  "scale_attn scale_lin w_a w_b w_mix cw_q cw_k cw_v cb_q cb_k cb_v qn_w kn_w A_log dt_bias").split():
             setattr(b, n, getattr(a, n))
         self.layer_ws = {}
-
-        # what current() compares, as flat sequences for one pass in C each
-        self._mod_d, self._mod_n, self._mod_v = zip(*self.mods)
-        self._par_d, self._par_n, self._par_v, _ = zip(*self.params)
-        self._tensors = [t for t in self._par_v if t is not None]
-        self._ptrs = [t.data_ptr() for t in self._tensors]
+        return ok
 
     def current(self) -> bool:
-        if not self.ok:
-            return all(d.get(n) is m for d, n, m in self.mods)    # nothing else to check: the general path runs
-        return (all(map(operator.is_, map(dict.get, self._mod_d, self._mod_n), self._mod_v)) and not any(self.hooks)
+        return (all(map(operator.is_, map(dict.get, self._mod_d, self._mod_n), self._mod_v))
+                and list(map(dict.get, self._att_d, self._att_n)) == self._att_v and not any(self.hooks)
                 and all(map(operator.is_, map(dict.get, self._par_d, self._par_n), self._par_v))
                 and list(map(torch.Tensor.data_ptr, self._tensors)) == self._ptrs)
 
@@ -122,7 +139,7 @@ class _Plan:
 class _Step:
     """Argument block of one layer's decoding steps on one cache: everything that stays the same from token to token."""
 
-    def __init__(self, plan, layer, cache, B, dev):
+    def __init__(self, plan, B, dev):
         self.plan, self.cache_tensors = plan, None
         a = self.args = _lib.DecodeArgs()
         ctypes.memmove(ctypes.byref(a), ctypes.byref(plan.args), ctypes.sizeof(a))
@@ -135,12 +152,6 @@ class _Step:
         self.workspace = torch.empty(need, dtype=torch.uint8, device=dev)
         a.workspace, a.workspace_bytes = self.workspace.data_ptr(), need
         self.ref = ctypes.byref(a)
-        gdn = a.rule == _lib.RULE_GDN
-        a.own_chunk = int(layer.ops_for_incomplete_chunks == 'all')
-        a.decay = int(layer.decay_for_non_gdn_blocks if gdn else layer.decay_for_non_mamba_blocks)
-        a.neg_eigval = int(gdn and layer.allow_neg_eigval)
-        a.attn_conv = int(layer.attn_with_short_conv)
-        self.options = (layer.ops_for_incomplete_chunks, layer.attn_with_short_conv)
 
     def bind(self, cache) -> bool:
         """Takes over the cache's tensors (made contiguous where they are not); False if they are not the kernel's kind."""
@@ -183,16 +194,14 @@ class _Step:
 
 
 def layer_plan(layer) -> _Plan:
-    """This thread's plan of the layer, rebuilt when a module, a parameter or its storage has changed."""
+    """This thread's plan of the layer, rebuilt when a module, an attribute, a parameter or its storage has changed."""
     plans = getattr(_tls, "plans", None)
     if plans is None:
         plans = _tls.plans = weakref.WeakKeyDictionary()
     p = plans.get(layer)
     if p is None or not p.current():
         p = plans[layer] = _Plan(layer)
-        if p.ok and any(p.hooks):
-            p.ok = False
-            p.mods = [(layer._modules, "q_proj", None)]      # looked at again with the next token
+        p.ok = p.ok and not any(p.hooks)                     # a plan with hooks is never current: looked at again next time
     return p
 
 
@@ -210,12 +219,10 @@ def decode_token(layer, x: torch.Tensor, container):
     pos = cache.n_tokens
     B = x.shape[0]
     step = cache._step
-    if (step is None or step.plan is not plan or step.args.B != B
-            or step.options != (layer.ops_for_incomplete_chunks, layer.attn_with_short_conv)):
-        if (B > MAX_BATCH or layer.ops_for_incomplete_chunks == 'attn' or not layer.incomplete_block_start_with_ht
-                or not (layer.use_short_conv and layer.use_gate)):
+    if step is None or step.plan is not plan or step.args.B != B:
+        if B > MAX_BATCH:
             return None
-        step = _Step(plan, layer, cache, B, x.device)
+        step = _Step(plan, B, x.device)
     if torch.is_autocast_enabled() or torch.nn.modules.module._has_any_global_hook():
         return None
     with torch.no_grad(), device_guard(plan.device):

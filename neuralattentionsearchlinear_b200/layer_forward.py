@@ -25,9 +25,8 @@ def _r256(n: int) -> int:
 def layer_forward(layer, x: torch.Tensor, cache=None):
     """The layer's output [B, T, hidden] for a whole sequence, or None where the general path has to run.  ``cache``: an empty
     ``NAtSLayerCache`` that receives the state a decoder continues from."""
-    if (x.dim() != 3 or x.dtype != BF16 or not x.is_cuda or x.shape[1] < 64 or not (layer.use_short_conv and layer.use_gate)
-            or layer.ops_for_incomplete_chunks == 'attn' or not layer.incomplete_block_start_with_ht
-            or layer.nats_sample_func is not hard_softmax or torch.is_autocast_enabled()):
+    if (x.dim() != 3 or x.dtype != BF16 or not x.is_cuda or x.shape[1] < 64 or layer.nats_sample_func is not hard_softmax
+            or torch.is_autocast_enabled()):
         return None
     plan = layer_plan(layer)
     if not plan.ok or torch.nn.modules.module._has_any_global_hook():
@@ -60,9 +59,6 @@ def _forward(layer, plan, x, cache):
     q_raw, k_raw, v_raw = (F.linear(x, m.weight) for m in (layer.q_proj, layer.k_proj, layer.v_proj))
     a = plan.layer_args
     a.B, a.T = B, T
-    a.attn_conv, a.own_chunk = int(layer.attn_with_short_conv), int(layer.ops_for_incomplete_chunks == 'all')
-    a.decay = int(layer.decay_for_non_gdn_blocks if gdn else layer.decay_for_non_mamba_blocks)
-    a.neg_eigval = int(gdn and layer.allow_neg_eigval)
     a.options = ((0 if _ops.PREP_TC else _lib.HYBRID_PREP_MMA) | (_lib.HYBRID_WALK_MMA if B * H <= _ops.WALK_MMA_MAX_HEADS else 0)
                  | (_lib.HYBRID_ATTN_PERSISTENT if _ops.ATTN_PERSISTENT else 0))
     normed = bool(d.qn_w)
@@ -72,7 +68,7 @@ def _forward(layer, plan, x, cache):
     types_raw = torch.empty(B, TN, HN, 2, **bf)
     nt = B * TN * HN * 2
     tables = torch.empty(2 * nt + 3 * B * HN + B * cdiv(T, 128) * HN, dtype=torch.int32, device=dev)
-    key = (B, T, a.attn_conv)
+    key = (B, T)
     need = plan.layer_ws.get(key)
     if need is None:
         if len(plan.layer_ws) > 256:

@@ -201,3 +201,85 @@ def test_library_refuses_memory_of_another_place(nat):
     bad.pos, bad.types_new, bad.x = 65, None, host.data_ptr()
     with pytest.raises(_lib.NatslError, match="device memory"):
         _lib.call("natsl_decode_step", ctypes.byref(bad), torch.cuda.current_stream().cuda_stream)
+
+
+# ------------------------------------------------------------------------------------------------ changed layers
+# Both paths round the same tensors to bf16 and differ in the order of fp32 sums: 2^-8 of the largest entry for each of about
+# four roundings that do not cancel (as in tests/test_gpu_decode_step.py).
+TOL = 4 * 2.0 ** -8
+
+
+def general_path(monkeypatch):
+    from neuralattentionsearchlinear_b200 import natsl_attn_gdn, natsl_attn_mamba2
+    for mod in (natsl_attn_gdn, natsl_attn_mamba2):
+        monkeypatch.setattr(mod, "layer_forward", lambda *a: None)
+        monkeypatch.setattr(mod, "decode_token", lambda *a: None)
+
+
+def close(got, want, what):
+    bound = TOL * max(float(want.float().abs().max()), 1e-3)
+    err = float((got.float() - want.float()).abs().max())
+    assert err <= bound, f"{what} off by {err:.3g} (bound {bound:.3g})"
+
+
+def set_conv(layer, activation):
+    for c in (layer.q_conv1d, layer.k_conv1d, layer.v_conv1d):
+        c.activation = activation
+
+
+def scaled_mix(layer):
+    mix = layer.mix
+    layer.mix = lambda *a: 2 * mix(*a)
+
+
+CHANGES = [
+    ("gdn", "block size", lambda m: setattr(m, "nats_block_size", 128)),
+    ("gdn", "q/k norm eps", lambda m: [setattr(n, "eps", 3.0) for n in (m.q_norm, m.k_norm)]),
+    ("gdn", "output norm eps", lambda m: setattr(m.o_norm, "eps", 3.0)),
+    ("gdn", "gate activation", lambda m: setattr(m.o_norm, "activation", "sigmoid")),
+    ("gdn", "convolution activation", lambda m: set_conv(m, None)),
+    ("gdn", "negative eigenvalues", lambda m: setattr(m, "allow_neg_eigval", True)),
+    ("gdn", "decay over skipped blocks", lambda m: setattr(m, "decay_for_non_gdn_blocks", False)),
+    ("gdn", "own chunk", lambda m: setattr(m, "ops_for_incomplete_chunks", "gated_delta_net")),
+    ("gdn", "another mix", scaled_mix),
+    ("mamba", "l2 norm eps", lambda m: [setattr(n, "eps", 3.0) for n in (m.q_norm2, m.k_norm2)]),
+    ("mamba", "decay over skipped blocks", lambda m: setattr(m, "decay_for_non_mamba_blocks", False)),
+]
+
+
+@pytest.mark.parametrize("rule,what,change", CHANGES, ids=[f"{r}-{w}" for r, w, _ in CHANGES])
+def test_changed_attributes_take_effect(nat, rule, what, change, monkeypatch):
+    """An attribute changed after the first calls counts from the next call on: prompt, and tokens of a cache in use."""
+    layer, x = make_layer(nat, rule), tokens(2, 140)
+
+    def run():
+        cache = nat.NAtSCache()
+        with torch.no_grad():
+            y = [call(layer, x[:, :120], cache), call(layer, x[:, 120:121], cache)]
+            old = {n: getattr(layer, n) for n in ("nats_block_size", "ops_for_incomplete_chunks")}
+            if what == "block size":                         # of a new sequence: a cache keeps the one it was begun with
+                cache = nat.NAtSCache()
+                layer.nats_block_size = 128
+                y += [call(layer, x[:, :130], cache)]
+                t0 = 130
+            else:
+                undo = {m: dict(m.__dict__) for m in layer.modules()}
+                change(layer)
+                t0 = 121
+            y += [call(layer, x[:, t:t + 1], cache) for t in range(t0, 140)] + [call(layer, x[:, :120])]
+            if what == "block size":
+                for n, v in old.items():
+                    setattr(layer, n, v)
+            else:
+                for m, d in undo.items():
+                    for n in ("eps", "activation", "allow_neg_eigval", "decay_for_non_gdn_blocks", "decay_for_non_mamba_blocks",
+                              "ops_for_incomplete_chunks"):
+                        if n in d:
+                            setattr(m, n, d[n])
+                layer.__dict__.pop("mix", None)
+        return y
+
+    got = run()
+    general_path(monkeypatch)
+    for i, (a, b) in enumerate(zip(got, run())):
+        close(a, b, f"call {i}")
