@@ -83,6 +83,8 @@ class _Plan:
 
         m = layer
         self.device = m.q_proj.weight.device
+        linears = [mod for _, _, mod in self.mods if type(mod) is nn.Linear]
+        self.params += [(mod._parameters, "bias", mod.bias) for mod in linears]          # the products add none
         checks = [weight("w_q", m.q_proj), weight("w_k", m.k_proj), weight("w_v", m.v_proj), weight("w_a", m.a_proj),
                   weight("w_g", m.g_proj), weight("w_o", m.o_proj), weight("cw_q", m.q_conv1d), weight("cw_k", m.k_conv1d),
                   weight("cw_v", m.v_conv1d), weight("cb_q", m.q_conv1d, "bias"), weight("cb_k", m.k_conv1d, "bias"),
@@ -103,7 +105,7 @@ class _Plan:
         w1, w2 = m.o_norm.weight1, m.o_norm.weight2
         DK, DV = m.head_attn_k_dim, m.head_attn_v_dim
         ok = bool(
-            all(checks) and all(mod.bias is None for mod in (m.q_proj, m.k_proj, m.v_proj, m.a_proj, m.g_proj, m.o_proj))
+            all(checks) and all(mod.bias is None for mod in linears)
             and (w1 is None) == (w2 is None) and (w1 is None or w1.dtype == w2.dtype)
             and m.num_v_heads == m.num_heads and m.n_ops == 2 and m.o_norm.hidden_size == DV
             and all(c.kernel_size == (4,) and c.activation == m.q_conv1d.activation for c in (m.q_conv1d, m.k_conv1d, m.v_conv1d))

@@ -283,3 +283,22 @@ def test_changed_attributes_take_effect(nat, rule, what, change, monkeypatch):
     general_path(monkeypatch)
     for i, (a, b) in enumerate(zip(got, run())):
         close(a, b, f"call {i}")
+
+
+@pytest.mark.parametrize("rule,name", [("gdn", "b_proj"), ("gdn", "nats_out_weights_layer"), ("mamba", "nats_out_weights_layer"),
+                                       ("gdn", "q_proj"), ("gdn", "nats_layer")])
+@pytest.mark.parametrize("replaced", [False, True])
+def test_projections_with_a_bias(nat, rule, name, replaced, monkeypatch):
+    """A projection that has got a bias (another module, or the same one given a bias) takes the general path."""
+    layer, x = make_layer(nat, rule), tokens(2, 140)
+    got = [prompt_and_tokens(nat, layer, x, 130)]
+    old = getattr(layer, name)
+    m = torch.nn.Linear(old.in_features, old.out_features, bias=True).cuda().bfloat16() if replaced else old
+    m.weight.data.copy_(old.weight.data)
+    m.bias = torch.nn.Parameter(torch.linspace(-2, 2, old.out_features, device="cuda").bfloat16())
+    setattr(layer, name, m)
+    got.append(prompt_and_tokens(nat, layer, x, 130))
+    general_path(monkeypatch)
+    want = prompt_and_tokens(nat, layer, x, 130)
+    close(got[1], want, "with the bias")
+    assert float((got[0] - want).abs().max()) > TOL * float(want.abs().max()), "the bias makes no difference here"
