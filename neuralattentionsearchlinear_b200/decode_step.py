@@ -17,6 +17,7 @@ from .nats_util import aligned, current_stream_ptr, device_guard
 
 BF16 = torch.bfloat16
 MAX_BATCH = 64
+_kind = operator.attrgetter("dtype", "shape")
 _tls = threading.local()                     # one argument block per thread: a call in flight is never rewritten
 
 
@@ -63,15 +64,25 @@ class _Plan:
         self._par_d, self._par_n, self._par_v = zip(*self.params) if self.params else ((), (), ())
         self._tensors = [t for t in self._par_v if t is not None]
         self._ptrs = [t.data_ptr() for t in self._tensors]
+        self._kinds = list(map(_kind, self._tensors))
 
     def _fill(self, layer, gdn: bool, weighted: bool) -> bool:
         a = self.args = _lib.DecodeArgs()
 
-        def weight(field, owner, name="weight", any_float=None):
+        m = layer
+        self.device = m.q_proj.weight.device
+        linears = [mod for _, _, mod in self.mods if type(mod) is nn.Linear]
+        self.params += [(mod._parameters, "bias", mod.bias) for mod in linears]          # the products add none
+        H, HQ, K, V, DK, DV, D = (m.num_heads, m.num_attn_heads, m.head_k_dim, m.head_v_dim, m.head_attn_k_dim, m.head_attn_v_dim,
+                                  m.hidden_size)
+
+        def weight(field, owner, *shape, name="weight", any_float=None, optional=False):
             p = owner._parameters.get(name)
             self.params.append((owner._parameters, name, p))
             if p is None:
-                return True
+                return optional
+            if type(p) not in (nn.Parameter, torch.Tensor) or tuple(p.shape) != shape:
+                return False
             if any_float is not None and p.dtype == torch.float32:
                 setattr(a, any_float, 1)
             elif p.dtype != BF16:
@@ -81,45 +92,41 @@ class _Plan:
             align = 16 if field.startswith("w_") else 8 if field.startswith("cw_") else 1
             return p.is_cuda and p.is_contiguous() and p.device == self.device and p.data_ptr() % align == 0
 
-        m = layer
-        self.device = m.q_proj.weight.device
-        linears = [mod for _, _, mod in self.mods if type(mod) is nn.Linear]
-        self.params += [(mod._parameters, "bias", mod.bias) for mod in linears]          # the products add none
-        checks = [weight("w_q", m.q_proj), weight("w_k", m.k_proj), weight("w_v", m.v_proj), weight("w_a", m.a_proj),
-                  weight("w_g", m.g_proj), weight("w_o", m.o_proj), weight("cw_q", m.q_conv1d), weight("cw_k", m.k_conv1d),
-                  weight("cw_v", m.v_conv1d), weight("cb_q", m.q_conv1d, "bias"), weight("cb_k", m.k_conv1d, "bias"),
-                  weight("cb_v", m.v_conv1d, "bias"), weight("A_log", m, "A_log", "alog_f32"),
-                  weight("dt_bias", m, "dt_bias", "dt_f32"), weight("w1", m.o_norm, "weight1", "w12_f32"),
-                  weight("w2", m.o_norm, "weight2", "w12_f32")]
+        checks = [weight("w_q", m.q_proj, H * K, D), weight("w_k", m.k_proj, H * K, D), weight("w_v", m.v_proj, H * V, D),
+                  weight("w_a", m.a_proj, H, D), weight("w_g", m.g_proj, H * V, D), weight("w_o", m.o_proj, D, H * V),
+                  weight("A_log", m, H, name="A_log", any_float="alog_f32"),
+                  weight("dt_bias", m, H, name="dt_bias", any_float="dt_f32")]
+        for n, conv, width in (("q", m.q_conv1d, H * K), ("k", m.k_conv1d, H * K), ("v", m.v_conv1d, H * V)):
+            checks += [weight("cw_" + n, conv, width, 1, 4), weight("cb_" + n, conv, width, name="bias", optional=True)]
+        checks += [weight(f"w{i}", m.o_norm, DV, name=f"weight{i}", any_float="w12_f32", optional=True) for i in (1, 2)]
         if gdn:
-            checks.append(weight("w_b", m.b_proj))
+            checks.append(weight("w_b", m.b_proj, H, D))
         else:
             checks.append(m.q_norm2.eps == m.k_norm2.eps)
             a.l2_eps = m.q_norm2.eps
         if weighted:
-            checks.append(weight("w_mix", m.nats_out_weights_layer))
+            checks.append(weight("w_mix", m.nats_out_weights_layer, 2 * HQ, H * K))
         if m.attn_qk_norm:
-            checks += [weight("qn_w", m.q_norm, "weight", "qn_f32"), weight("kn_w", m.k_norm, "weight", "kn_f32"),
+            checks += [weight("qn_w", m.q_norm, DK, any_float="qn_f32"), weight("kn_w", m.k_norm, DK, any_float="kn_f32"),
                        m.q_norm.eps == m.k_norm.eps]
             a.norm_eps = m.q_norm.eps
         w1, w2 = m.o_norm.weight1, m.o_norm.weight2
-        DK, DV = m.head_attn_k_dim, m.head_attn_v_dim
         ok = bool(
             all(checks) and all(mod.bias is None for mod in linears)
             and (w1 is None) == (w2 is None) and (w1 is None or w1.dtype == w2.dtype)
-            and m.num_v_heads == m.num_heads and m.n_ops == 2 and m.o_norm.hidden_size == DV
+            and m.num_v_heads == H and m.n_ops == 2 and m.o_norm.hidden_size == DV
+            and m.key_dim == H * K == HQ * DK and m.value_dim == H * V == HQ * DV
             and all(c.kernel_size == (4,) and c.activation == m.q_conv1d.activation for c in (m.q_conv1d, m.k_conv1d, m.v_conv1d))
-            and m.hidden_size % 32 == 0 and m.value_dim % 32 == 0 and m.head_k_dim % 32 == 0 and m.head_k_dim <= 256
-            and m.head_v_dim % 32 == 0 and DK in (64, 128) and DV in (64, 128) and m.key_dim <= 10240
+            and D % 32 == 0 and m.value_dim % 32 == 0 and K % 32 == 0 and K <= 256 and V % 32 == 0 and DK in (64, 128)
+            and DV in (64, 128) and m.key_dim <= 10240
             and m.num_heads % m.num_nats_head == 0 and m.num_attn_heads % m.num_nats_head == 0
             and m.use_short_conv and m.use_gate and m.ops_for_incomplete_chunks != 'attn' and m.incomplete_block_start_with_ht
             and not m.usg_for_attn and m.pooling_func is mean_pooling)
-        a.hidden, a.H, a.K, a.V, a.HQ, a.HN = (m.hidden_size, m.num_heads, m.head_k_dim, m.head_v_dim, m.num_attn_heads,
-                                               m.num_nats_head)
+        a.hidden, a.H, a.K, a.V, a.HQ, a.HN = D, H, K, V, HQ, m.num_nats_head
         a.nbs, a.rule = m.nats_block_size, _lib.RULE_GDN if gdn else _lib.RULE_MAMBA
         a.silu = int(m.q_conv1d.activation in ("silu", "swish"))
         a.mix_sigmoid, a.mix_eps = int(m.o_norm.activation == "sigmoid"), m.o_norm.eps
-        a.scale_attn, a.scale_lin = DK ** -0.5, m.head_k_dim ** -0.5 if gdn else 1.0
+        a.scale_attn, a.scale_lin = DK ** -0.5, K ** -0.5 if gdn else 1.0
         a.own_chunk, a.attn_conv = int(m.ops_for_incomplete_chunks == 'all'), int(m.attn_with_short_conv)
         a.decay = int(m.decay_for_non_gdn_blocks if gdn else m.decay_for_non_mamba_blocks)
         a.neg_eigval = int(gdn and m.allow_neg_eigval)
@@ -135,7 +142,8 @@ class _Plan:
         return (all(map(operator.is_, map(dict.get, self._mod_d, self._mod_n), self._mod_v))
                 and list(map(dict.get, self._att_d, self._att_n)) == self._att_v and not any(self.hooks)
                 and all(map(operator.is_, map(dict.get, self._par_d, self._par_n), self._par_v))
-                and list(map(torch.Tensor.data_ptr, self._tensors)) == self._ptrs)
+                and list(map(torch.Tensor.data_ptr, self._tensors)) == self._ptrs and list(map(_kind, self._tensors)) == self._kinds
+                and all(map(torch.Tensor.is_contiguous, self._tensors)))
 
 
 class _Step:

@@ -36,7 +36,7 @@ def layer_forward(layer, x: torch.Tensor, cache=None):
     sel = layer.nats_layer
     if (D != d.hidden or x.device != plan.device or not _ops.walks_with_state(d.rule, d.K, d.V, T) or B > 65535
             or type(sel) is not nn.Linear or sel.bias is not None or sel.weight.dtype != BF16 or sel._forward_hooks
-            or sel._forward_pre_hooks or not sel.weight.is_cuda):
+            or sel._forward_pre_hooks or not sel.weight.is_cuda or tuple(sel.weight.shape) != (2 * d.HN, d.hidden)):
         return None
     with device_guard(x.device):
         return _forward(layer, plan, x, cache)

@@ -302,3 +302,33 @@ def test_projections_with_a_bias(nat, rule, name, replaced, monkeypatch):
     want = prompt_and_tokens(nat, layer, x, 130)
     close(got[1], want, "with the bias")
     assert float((got[0] - want).abs().max()) > TOL * float(want.abs().max()), "the bias makes no difference here"
+
+
+@pytest.mark.parametrize("what", ["wider output", "narrower projection", "missing", "transposed", "other dtype"])
+def test_replaced_weights(nat, what):
+    """Weights of other shapes, layouts or types than the plan was made for: the fast paths see it before any launch."""
+    from neuralattentionsearchlinear_b200.decode_step import layer_plan
+    layer, x = make_layer(nat), tokens(2, 130)
+    prompt_and_tokens(nat, layer, x, 128)
+    assert layer_plan(layer).ok
+    if what == "wider output":                               # the general path serves it: another width out
+        layer.o_proj = torch.nn.Linear(256, 320, bias=False).cuda().bfloat16()
+        want = layer.o_proj.weight
+        assert not layer_plan(layer).ok
+        y = prompt_and_tokens(nat, layer, x, 128)
+        assert y.shape[-1] == want.shape[0] and bool(y.isfinite().all())
+    elif what == "narrower projection":
+        layer.k_proj.weight.data = layer.k_proj.weight.data[:192]
+        assert not layer_plan(layer).ok
+    elif what == "missing":
+        w = layer.a_proj.weight.data
+        del layer.a_proj.weight
+        layer.a_proj.weight = w                              # a plain attribute in place of the parameter
+        assert not layer_plan(layer).ok
+        assert bool(prompt_and_tokens(nat, layer, x, 128).isfinite().all())
+    elif what == "transposed":
+        layer.q_proj.weight.data = layer.q_proj.weight.data.t()
+        assert not layer_plan(layer).ok
+    else:
+        layer.v_proj.weight.data = layer.v_proj.weight.data.view(torch.float16)
+        assert not layer_plan(layer).ok
