@@ -12,8 +12,10 @@ arrived).  This is a compact restatement of the same bookkeeping for batches wit
 * ``state`` / ``state_block_start`` / ``g_block``: the current recurrent state, the state the current block started from
   and the log decay accumulated in the current block (re-roll at the block end needs all three).
 
-Single-token steps update these tensors in place.  ``copy.copy`` of a layer cache gives an independent continuation (one
-prompt, several completions): the small tensors are cloned, the key/value rows are shared until either side appends.
+Single-token steps update these tensors in place, but never one that a caller has seen: reading or setting ``state`` and the
+like hands the tensor out, and the next step works on copies.  ``copy.copy`` of a layer cache gives an independent
+continuation (one prompt, several completions): the small tensors are cloned, the key/value rows are shared until either
+side appends.
 """
 from __future__ import annotations
 
@@ -22,7 +24,33 @@ from typing import List, Optional
 import torch
 
 
+_IN_PLACE = ("_state", "_state_block_start", "_g_block", "_pool_sum", "_conv_state")
+
+
+def _seen(name: str, doc: str) -> property:
+    """Attribute whose tensor belongs to the caller as well once it has been read or set."""
+    def get(self):
+        self._handed_out = True
+        return getattr(self, name)
+
+    def put(self, value):
+        self._handed_out = True
+        setattr(self, name, value)
+
+    return property(get, put, doc=doc)
+
+
+def _copy(t):
+    return None if t is None else tuple(map(_copy, t)) if isinstance(t, tuple) else t.clone()
+
+
 class NAtSLayerCache:
+    state = _seen("_state", "[B, H, K, V] fp32: current state")
+    state_block_start = _seen("_state_block_start", "[B, H, K, V] fp32: state the current block started from")
+    g_block = _seen("_g_block", "[B, H] fp32: log decay accumulated in the current block")
+    pool_sum = _seen("_pool_sum", "[B, D] fp32: sum of the layer input over the current block")
+    conv_state = _seen("_conv_state", "(q, k, v) tails of the short convolutions")
+
     def __init__(self, nats_block_size: int = 64):
         self.nats_block_size = nats_block_size
         self.n_tokens = 0                               # tokens seen so far
@@ -32,25 +60,34 @@ class NAtSLayerCache:
         self._kv_shared = False                         # another cache reads the same buffers
         self._step = None                               # argument block and workspace of the single-token steps
         self.block_types: Optional[torch.Tensor] = None  # [B, finished blocks, HN, 2] sampled types
-        self.state: Optional[torch.Tensor] = None        # [B, H, K, V] fp32: current state
-        self.state_block_start: Optional[torch.Tensor] = None
-        self.g_block: Optional[torch.Tensor] = None      # [B, H] fp32: log decay of the current block so far
-        self.pool_sum: Optional[torch.Tensor] = None     # [B, D] fp32: sum of the layer input over the current block
-        self.conv_state = None                           # (q, k, v) tails of the short convolutions
+        for name in _IN_PLACE:
+            setattr(self, name, None)
+        self._handed_out = False                         # a caller may hold one of these tensors
 
     def __copy__(self):
         new = type(self).__new__(type(self))
         new.__dict__.update(self.__dict__)
-        for name in ("state", "state_block_start", "g_block", "pool_sum"):
-            t = getattr(self, name)
-            setattr(new, name, None if t is None else t.clone())
-        new.conv_state = None if self.conv_state is None else tuple(None if t is None else t.clone() for t in self.conv_state)
+        new._handed_out = True
+        new.own_state()
         new._step = None
         self._kv_shared = new._kv_shared = True
         return new
 
     def __getstate__(self):
         return dict(self.__dict__, _step=None)             # holds addresses: not for another process
+
+    def own_state(self) -> None:
+        """Makes the tensors that a step updates in place this cache's own: copies them if they have been handed out."""
+        if self._handed_out:
+            for name in _IN_PLACE:
+                setattr(self, name, _copy(getattr(self, name)))
+            self._handed_out = False
+
+    def set_state(self, state, state_block_start, g_block, pool_sum, conv_state) -> None:
+        """Takes over tensors that nobody else holds."""
+        self._state, self._state_block_start, self._g_block, self._pool_sum, self._conv_state = (state, state_block_start, g_block,
+                                                                                                pool_sum, conv_state)
+        self._handed_out = False
 
     @property
     def k_attn(self) -> Optional[torch.Tensor]:

@@ -167,39 +167,39 @@ class _Step:
         """Takes over the cache's tensors (made contiguous where they are not); False if they are not the kernel's kind."""
         a = self.args
         B, dev = a.B, self.workspace.device
-        if cache.conv_state is None or any(t is None or t.dtype != BF16 or t.device != dev or t.shape[0] != B for t in
-                                           (*cache.conv_state, cache._k_buf, cache._v_buf)):
+        if cache._conv_state is None or any(t is None or t.dtype != BF16 or t.device != dev or t.shape[0] != B for t in
+                                           (*cache._conv_state, cache._k_buf, cache._v_buf)):
             return False
-        for name in ("state", "state_block_start", "g_block", "pool_sum"):
+        for name in ("_state", "_state_block_start", "_g_block", "_pool_sum"):
             t = getattr(cache, name)
             if t is None or t.shape[0] != B or t.device != dev:
                 return False
             if t.dtype != torch.float32 or not t.is_contiguous():
                 setattr(cache, name, t.float().contiguous())
-        if not all(t.is_contiguous() for t in cache.conv_state):
-            cache.conv_state = tuple(t.contiguous() for t in cache.conv_state)
+        if not all(t.is_contiguous() for t in cache._conv_state):
+            cache._conv_state = tuple(t.contiguous() for t in cache._conv_state)
         if cache.block_types is not None and not cache.block_types.is_contiguous():
             cache.block_types = cache.block_types.contiguous()
-        if any(t.data_ptr() % 16 for t in (cache.state, cache.state_block_start, cache._k_buf, cache._v_buf, *cache.conv_state)):
+        if any(t.data_ptr() % 16 for t in (cache._state, cache._state_block_start, cache._k_buf, cache._v_buf, *cache._conv_state)):
             return False
         types = cache.block_types
         if types is not None:
             if types.dtype not in (BF16, torch.float32):
                 return False
             a.types_f32 = int(types.dtype == torch.float32)
-        a.conv_q, a.conv_k, a.conv_v = (t.data_ptr() for t in cache.conv_state)
-        a.state, a.start, a.g_block = cache.state.data_ptr(), cache.state_block_start.data_ptr(), cache.g_block.data_ptr()
+        a.conv_q, a.conv_k, a.conv_v = (t.data_ptr() for t in cache._conv_state)
+        a.state, a.start, a.g_block = cache._state.data_ptr(), cache._state_block_start.data_ptr(), cache._g_block.data_ptr()
         a.k_cache, a.v_cache, a.cap = cache._k_buf.data_ptr(), cache._v_buf.data_ptr(), cache._k_buf.shape[1]
         a.types = None if types is None else types.data_ptr()
-        self.cache_tensors = (cache.state, cache.state_block_start, cache.g_block, cache.pool_sum, cache.conv_state, cache._k_buf,
+        self.cache_tensors = (cache._state, cache._state_block_start, cache._g_block, cache._pool_sum, cache._conv_state, cache._k_buf,
                               cache._v_buf, types)
-        self.pool = cache.pool_sum.data_ptr()
+        self.pool = cache._pool_sum.data_ptr()
         return True
 
     def bound(self, cache) -> bool:
         t = self.cache_tensors
-        return (t is not None and t[0] is cache.state and t[1] is cache.state_block_start and t[2] is cache.g_block
-                and t[3] is cache.pool_sum and t[4] is cache.conv_state and t[5] is cache._k_buf and t[6] is cache._v_buf
+        return (t is not None and t[0] is cache._state and t[1] is cache._state_block_start and t[2] is cache._g_block
+                and t[3] is cache._pool_sum and t[4] is cache._conv_state and t[5] is cache._k_buf and t[6] is cache._v_buf
                 and t[7] is cache.block_types)
 
 
@@ -244,11 +244,9 @@ def _decode(layer, x, cache, step, pos: int, nbs: int):
     B, D, dev = a.B, a.hidden, step.workspace.device
     if pos == 0:                                             # a prompt of one token: start from empty states
         f32 = dict(dtype=torch.float32, device=dev)
-        cache.state = torch.zeros(B, a.H, a.K, a.V, **f32)
-        cache.state_block_start = torch.zeros(B, a.H, a.K, a.V, **f32)
-        cache.g_block, cache.pool_sum = torch.zeros(B, a.H, **f32), torch.zeros(B, D, **f32)
-        cache.conv_state = tuple(torch.zeros(B, n, 4, dtype=BF16, device=dev)
-                                 for n in (layer.key_dim, layer.key_dim, layer.value_dim))
+        cache.set_state(torch.zeros(B, a.H, a.K, a.V, **f32), torch.zeros(B, a.H, a.K, a.V, **f32), torch.zeros(B, a.H, **f32),
+                        torch.zeros(B, D, **f32), tuple(torch.zeros(B, n, 4, dtype=BF16, device=dev)
+                                                        for n in (layer.key_dim, layer.key_dim, layer.value_dim)))
         cache._k_buf = torch.empty(B, 256, a.HQ, layer.head_attn_k_dim, dtype=BF16, device=dev)
         cache._v_buf = torch.empty(B, 256, a.HQ, layer.head_attn_v_dim, dtype=BF16, device=dev)
         cache._n_kv, cache._kv_shared = 0, False
@@ -260,11 +258,12 @@ def _decode(layer, x, cache, step, pos: int, nbs: int):
     x = aligned(x.contiguous())
     types_new = None
     if (pos + 1) % nbs == 0:                                 # a block's type is decided once its last token is known
-        pooled = ((cache.pool_sum + x[:, 0].float()) / nbs).to(x.dtype)[:, None, :]
+        pooled = ((cache._pool_sum + x[:, 0].float()) / nbs).to(x.dtype)[:, None, :]
         types_new = layer.select(pooled).contiguous()
         if types_new.dtype not in (BF16, torch.float32) or (cache.block_types is not None and cache.block_types.dtype != types_new.dtype):
             return None
     cache.reserve_kv(1)
+    cache.own_state()
     if not step.bound(cache) and not step.bind(cache):
         return None
     cache._step = step
@@ -279,5 +278,5 @@ def _decode(layer, x, cache, step, pos: int, nbs: int):
     cache._n_kv = cache.n_tokens = pos + 1
     if types_new is not None:
         cache.append_types(types_new)
-        cache.pool_sum = torch.zeros_like(cache.pool_sum)
+        cache._pool_sum = torch.zeros_like(cache._pool_sum)
     return out

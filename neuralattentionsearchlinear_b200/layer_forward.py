@@ -107,6 +107,6 @@ def _forward(layer, plan, x, cache):
         cache.append_kv(k_attn, v_attn)
         if n_done:
             cache.append_types(types_raw if n_done == TN else types_raw[:, :n_done].contiguous())
-        cache.state_block_start, cache.state = start, (start.clone() if r == 0 else ht)
-        cache.g_block, cache.pool_sum, cache.conv_state, cache.n_tokens = g_block, pool_sum, tails, T
+        cache.set_state(start.clone() if r == 0 else ht, start, g_block, pool_sum, tails)
+        cache.n_tokens = T
     return F.linear(y, layer.o_proj.weight)

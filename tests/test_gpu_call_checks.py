@@ -332,3 +332,29 @@ def test_replaced_weights(nat, what):
     else:
         layer.v_proj.weight.data = layer.v_proj.weight.data.view(torch.float16)
         assert not layer_plan(layer).ok
+
+
+# ------------------------------------------------------------------------------------------------ what a caller keeps of a cache
+CACHE_STATE = ("state", "state_block_start", "g_block", "pool_sum", "conv_state", "k_attn", "v_attn", "block_types", "n_tokens")
+
+
+@pytest.mark.parametrize("rule", ["gdn", "mamba"])
+@pytest.mark.parametrize("T0", [70, 126])
+def test_snapshot_of_a_cache_by_reference(nat, rule, T0):
+    """Tensors read from a cache stay as they are while it decodes on (also over a block's end), and setting them again takes
+    it back to that token."""
+    layer, x = make_layer(nat, rule), tokens(2, 140)
+    cache = nat.NAtSCache()
+    with torch.no_grad():
+        call(layer, x[:, :T0], cache)
+        call(layer, x[:, T0:T0 + 1], cache)
+        snap = {n: getattr(cache[0], n) for n in CACHE_STATE}
+        flat = lambda: [t for n in CACHE_STATE[:-1] for t in (snap[n] if n == "conv_state" else [snap[n]])]
+        values = [t.clone() for t in flat()]
+        first = [call(layer, x[:, t:t + 1], cache) for t in range(T0 + 1, T0 + 5)]
+        assert all(map(torch.equal, flat(), values))
+        for n in CACHE_STATE:
+            setattr(cache[0], n, snap[n])
+        again = [call(layer, x[:, t:t + 1], cache) for t in range(T0 + 1, T0 + 5)]
+        assert all(map(torch.equal, flat(), values))
+    assert all(map(torch.equal, first, again))
