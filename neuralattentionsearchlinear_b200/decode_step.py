@@ -166,41 +166,46 @@ class _Step:
     def bind(self, cache) -> bool:
         """Takes over the cache's tensors (made contiguous where they are not); False if they are not the kernel's kind."""
         a = self.args
-        B, dev = a.B, self.workspace.device
-        if cache._conv_state is None or any(t is None or t.dtype != BF16 or t.device != dev or t.shape[0] != B for t in
-                                           (*cache._conv_state, cache._k_buf, cache._v_buf)):
-            return False
-        for name in ("_state", "_state_block_start", "_g_block", "_pool_sum"):
+        B, dev, HK, HV = a.B, self.workspace.device, a.H * a.K, a.H * a.V
+        state = (B, a.H, a.K, a.V)
+        for name, shape in (("_state", state), ("_state_block_start", state), ("_g_block", (B, a.H)), ("_pool_sum", (B, a.hidden))):
             t = getattr(cache, name)
-            if t is None or t.shape[0] != B or t.device != dev:
+            if t is None or tuple(t.shape) != shape or t.device != dev:
                 return False
             if t.dtype != torch.float32 or not t.is_contiguous():
                 setattr(cache, name, t.float().contiguous())
-        if not all(t.is_contiguous() for t in cache._conv_state):
-            cache._conv_state = tuple(t.contiguous() for t in cache._conv_state)
-        if cache.block_types is not None and not cache.block_types.is_contiguous():
-            cache.block_types = cache.block_types.contiguous()
-        if any(t.data_ptr() % 16 for t in (cache._state, cache._state_block_start, cache._k_buf, cache._v_buf, *cache._conv_state)):
+        conv, rows, types = cache._conv_state, (cache._k_buf, cache._v_buf), cache.block_types
+        if (conv is None or len(conv) != 3 or any(t is None or t.dtype != BF16 or t.device != dev for t in (*conv, *rows))
+                or [tuple(t.shape) for t in conv] != [(B, HK, 4), (B, HK, 4), (B, HV, 4)]):
             return False
-        types = cache.block_types
+        cap = rows[0].shape[1]
+        if [tuple(t.shape) for t in rows] != [(B, cap, a.HQ, HK // a.HQ), (B, cap, a.HQ, HV // a.HQ)]:
+            return False
         if types is not None:
-            if types.dtype not in (BF16, torch.float32):
+            if types.dtype not in (BF16, torch.float32) or types.device != dev or tuple(types.shape) != (B, types.shape[1], a.HN, 2):
                 return False
             a.types_f32 = int(types.dtype == torch.float32)
-        a.conv_q, a.conv_k, a.conv_v = (t.data_ptr() for t in cache._conv_state)
+            if not types.is_contiguous():
+                types = cache.block_types = types.contiguous()
+        if not all(t.is_contiguous() for t in conv):
+            conv = cache._conv_state = tuple(t.contiguous() for t in conv)
+        if any(t.data_ptr() % 16 for t in (cache._state, cache._state_block_start, *rows, *conv)):
+            return False
+        a.conv_q, a.conv_k, a.conv_v = (t.data_ptr() for t in conv)
         a.state, a.start, a.g_block = cache._state.data_ptr(), cache._state_block_start.data_ptr(), cache._g_block.data_ptr()
-        a.k_cache, a.v_cache, a.cap = cache._k_buf.data_ptr(), cache._v_buf.data_ptr(), cache._k_buf.shape[1]
+        a.k_cache, a.v_cache, a.cap = rows[0].data_ptr(), rows[1].data_ptr(), cap
         a.types = None if types is None else types.data_ptr()
-        self.cache_tensors = (cache._state, cache._state_block_start, cache._g_block, cache._pool_sum, cache._conv_state, cache._k_buf,
-                              cache._v_buf, types)
+        self.cache_tensors = (cache._state, cache._state_block_start, cache._g_block, cache._pool_sum, conv, *rows, types)
         self.pool = cache._pool_sum.data_ptr()
         return True
 
     def bound(self, cache) -> bool:
+        """Whether these are the tensors that ``bind`` has checked.  All but the types are the cache's own (``own_state``):
+        nobody else can give one of them another storage or shape."""
         t = self.cache_tensors
         return (t is not None and t[0] is cache._state and t[1] is cache._state_block_start and t[2] is cache._g_block
                 and t[3] is cache._pool_sum and t[4] is cache._conv_state and t[5] is cache._k_buf and t[6] is cache._v_buf
-                and t[7] is cache.block_types)
+                and t[7] is cache.block_types and (t[7] is None or t[7].data_ptr() == self.args.types))
 
 
 def layer_plan(layer) -> _Plan:

@@ -358,3 +358,37 @@ def test_snapshot_of_a_cache_by_reference(nat, rule, T0):
         again = [call(layer, x[:, t:t + 1], cache) for t in range(T0 + 1, T0 + 5)]
         assert all(map(torch.equal, flat(), values))
     assert all(map(torch.equal, first, again))
+
+
+@pytest.mark.parametrize("what", ["state storage", "types storage", "state shape", "tail shape", "key shape", "types shape"])
+def test_cache_tensors_of_other_storage_or_shape(nat, what):
+    """Storage exchanged behind a tensor is what the next step reads; shapes of another layer never reach the kernel."""
+    layer, x = make_layer(nat), tokens(2, 140)
+    with torch.no_grad():
+        cache, other = nat.NAtSCache(), nat.NAtSCache()
+        call(layer, x[:, :70], cache)
+        call(layer, x[:, :70].flip(0).contiguous(), other)
+        for c in (cache, other):
+            call(layer, x[:, 70:71], c)
+        c, o = cache[0], other[0]
+        if what.endswith("storage"):
+            if what == "state storage":
+                c.state.data = o.state.data.clone()
+                c.state_block_start.data = o.state_block_start.data.clone()
+            else:
+                c.block_types.data = 1 - c.block_types.data
+            import copy
+            new = nat.NAtSCache()
+            new.layers = [copy.copy(c)]
+            assert torch.equal(call(layer, x[:, 71:72], cache), call(layer, x[:, 71:72], new))
+            return
+        if what == "state shape":
+            c.state = c.state[:, :, :32]
+        elif what == "tail shape":
+            c.conv_state = tuple(t[:, :128].contiguous() for t in c.conv_state)
+        elif what == "key shape":
+            c.k_attn = c.k_attn[..., :32].contiguous()
+        else:
+            c.block_types = c.block_types[:, :, :2].contiguous()
+        from neuralattentionsearchlinear_b200.decode_step import decode_token
+        assert decode_token(layer, x[:, 71:72], cache) is None
