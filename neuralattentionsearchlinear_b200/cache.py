@@ -76,6 +76,11 @@ class NAtSLayerCache:
     def __getstate__(self):
         return dict(self.__dict__, _step=None)             # holds addresses: not for another process
 
+    def __setstate__(self, saved):
+        self.__init__(saved["nats_block_size"])
+        for name, value in saved.items():                  # also those of caches saved with plain k_attn, state, ... attributes
+            setattr(self, name, value)
+
     def own_state(self) -> None:
         """Makes the tensors that a step updates in place this cache's own: copies them if they have been handed out."""
         if self._handed_out:

@@ -152,10 +152,16 @@ class NeuralAttentionSearchLinearAttnGDN(nn.Module):
         else:
             self.o_norm = nn.ModuleList([RMSNorm(self.head_v_dim, eps=norm_eps), RMSNorm(self.head_attn_v_dim, eps=norm_eps)])
         self.o_proj = nn.Linear(self.value_dim, hidden_size, bias=False)
-        self.attn_blocks = None            # (block counts [B, HN, 2], blocks) of the last forward, behind attn_fraction
         self.attn_fraction = torch.zeros(1)
 
     # ------------------------------------------------------------------------------------------------
+    attn_blocks = None                     # (block counts [B, HN, 2], blocks) of the last forward, behind attn_fraction
+
+    def __setstate__(self, saved):
+        super().__setstate__(saved)
+        if "attn_fraction" in self.__dict__:                 # a layer saved when this was a plain attribute
+            self.attn_fraction = self.__dict__.pop("attn_fraction")
+
     @property
     def attn_fraction(self) -> torch.Tensor:
         """Share of the blocks of the last forward that took the softmax branch, per selection head."""

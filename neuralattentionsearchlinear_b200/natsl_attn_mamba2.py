@@ -129,8 +129,14 @@ class NeuralAttentionSearchLinearAttnMamba(nn.Module):
         else:
             raise NotImplementedError("use_gate=False is not built for the Mamba2 layer")
         self.o_proj = nn.Linear(self.value_dim, hidden_size, bias=False)
-        self.attn_blocks = None            # (block counts [B, HN, 2], blocks) of the last forward, behind attn_fraction
         self.attn_fraction = torch.zeros(1)
+
+    attn_blocks = None                     # (block counts [B, HN, 2], blocks) of the last forward, behind attn_fraction
+
+    def __setstate__(self, saved):
+        super().__setstate__(saved)
+        if "attn_fraction" in self.__dict__:                 # a layer saved when this was a plain attribute
+            self.attn_fraction = self.__dict__.pop("attn_fraction")
 
     @property
     def attn_fraction(self) -> torch.Tensor:
