@@ -271,10 +271,10 @@ def hybrid_fwd(rule: int, q_attn, k_attn, v_attn, q, k, v, g, beta, types, nbs: 
     _need(fp32 or q.dtype == BF16, f"unsupported dtype {q.dtype} (fp32 or bf16)", TypeError)
     _need(not (fp32 and want_start), "the block-start state needs bf16 tensors", TypeError)
     q_attn, k_attn, v_attn, q, k, v = (t_.contiguous() for t_ in (q_attn, k_attn, v_attn, q, k, v))
-    B, T, H, K = q.shape
-    V, HQ, DK, HKV, DV = v.shape[3], q_attn.shape[2], q_attn.shape[3], k_attn.shape[2], v_attn.shape[3]
+    B, T, H, K = map(int, q.shape)                           # a trace gives sizes as tensors
+    V, HQ, DK, HKV, DV = map(int, (v.shape[3], q_attn.shape[2], q_attn.shape[3], k_attn.shape[2], v_attn.shape[3]))
     dev = q.device
-    TN, HN = types.shape[1], types.shape[2]
+    TN, HN = map(int, types.shape[1:3])
     _need(tuple(k.shape) == (B, T, H, K), f"linear branch: q {tuple(q.shape)} and k {tuple(k.shape)} differ")
     _need(tuple(v.shape) == (B, T, H, V), f"linear branch: k {tuple(k.shape)} and v {tuple(v.shape)} differ in length or heads")
     _need(tuple(q_attn.shape) == (B, T, HQ, DK) and tuple(k_attn.shape) == (B, T, HKV, DK) and tuple(v_attn.shape) == (B, T, HKV, DV),
@@ -325,7 +325,7 @@ def hybrid_fwd(rule: int, q_attn, k_attn, v_attn, q, k, v, g, beta, types, nbs: 
     a.own_attn, a.decay, a.use_l2norm = int(own_attn), int(decay), int(use_l2norm)
     a.options = ((0 if PREP_TC else _lib.HYBRID_PREP_MMA) | (_lib.HYBRID_WALK_MMA if B * H <= WALK_MMA_MAX_HEADS else 0)
                  | (_lib.HYBRID_ATTN_PERSISTENT if ATTN_PERSISTENT else 0))
-    a.scale_attn, a.scale_lin = scale_attn, scale_lin
+    a.scale_attn, a.scale_lin = float(scale_attn), float(scale_lin)
     a.q_attn, a.k_attn, a.v_attn, a.q, a.k, a.v = (t_.data_ptr() for t_ in (q_attn, k_attn, v_attn, q, k, v))
     a.g, a.types, a.o_attn, a.lse, a.o_lin = g.data_ptr(), types.data_ptr(), o_attn.data_ptr(), lse.data_ptr(), o_lin.data_ptr()
     a.ht, a.hstart = _lib.ptr(ht), _lib.ptr(start)

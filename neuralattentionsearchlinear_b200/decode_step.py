@@ -13,7 +13,7 @@ import torch.nn as nn
 
 from . import _lib
 from .modules import FusedMultiInputRMSNormGated, L2Norm, RMSNorm, ShortConvolution, mean_pooling
-from .nats_util import aligned, current_stream_ptr, device_guard
+from .nats_util import aligned, current_stream_ptr, device_guard, transforms_active
 
 BF16 = torch.bfloat16
 MAX_BATCH = 64
@@ -238,7 +238,7 @@ def decode_token(layer, x: torch.Tensor, container):
         if B > MAX_BATCH:
             return None
         step = _Step(plan, B, x.device)
-    if torch.is_autocast_enabled() or torch.nn.modules.module._has_any_global_hook():
+    if torch.is_autocast_enabled() or torch.nn.modules.module._has_any_global_hook() or transforms_active():
         return None
     with torch.no_grad(), device_guard(plan.device):
         return _decode(layer, x, cache, step, pos, nbs)

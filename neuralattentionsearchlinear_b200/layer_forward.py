@@ -12,7 +12,7 @@ import torch.nn.functional as F
 from . import _lib, _ops
 from .decode_step import layer_plan
 from .modules import hard_softmax
-from .nats_util import aligned, cdiv, current_stream_ptr, device_guard
+from .nats_util import aligned, cdiv, current_stream_ptr, device_guard, transforms_active
 
 BF16 = torch.bfloat16
 
@@ -26,7 +26,7 @@ def layer_forward(layer, x: torch.Tensor, cache=None):
     """The layer's output [B, T, hidden] for a whole sequence, or None where the general path has to run.  ``cache``: an empty
     ``NAtSLayerCache`` that receives the state a decoder continues from."""
     if (x.dim() != 3 or x.dtype != BF16 or not x.is_cuda or x.shape[1] < 64 or layer.nats_sample_func is not hard_softmax
-            or torch.is_autocast_enabled()):
+            or torch.is_autocast_enabled() or transforms_active()):
         return None
     plan = layer_plan(layer)
     if not plan.ok or torch.nn.modules.module._has_any_global_hook():

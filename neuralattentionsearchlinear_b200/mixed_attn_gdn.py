@@ -12,7 +12,7 @@ import os
 import torch
 
 from . import _lib, _ops
-from .nats_util import CHUNK_SIZE, OFFSET_ATTN, OFFSET_LINEAR, build_selection_tables  # noqa: F401
+from .nats_util import CHUNK_SIZE, OFFSET_ATTN, OFFSET_LINEAR, build_selection_tables, transforms_active  # noqa: F401
 
 # which branches also compute the query's own (possibly incomplete) block — mixed_attn_gdn.py:29-42
 all_incomplete_ops = {
@@ -100,7 +100,8 @@ class NoGrad:
 
 
 def wants_grad(*tensors) -> bool:
-    return torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in tensors)
+    """Whether the call has to go through ``Function.apply``."""
+    return transforms_active() or torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in tensors)
 
 
 def hybrid_backward(ctx, rule, do_lin, do_attn, dht):

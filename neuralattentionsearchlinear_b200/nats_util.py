@@ -38,6 +38,13 @@ def device_guard(device: torch.device):
     return _SAME_DEVICE if device.index == torch.cuda.current_device() else torch.cuda.device(device)
 
 
+def transforms_active() -> bool:
+    """Whether forward-mode differentiation, a functorch transform or a jit trace is under way: what bypasses autograd functions
+    or torch ops would be left out of its result."""
+    return (torch.autograd.forward_ad._current_level >= 0 or torch._C._get_tracing_state() is not None
+            or torch._C._functorch.peek_interpreter_stack() is not None)
+
+
 def aligned(t: torch.Tensor) -> torch.Tensor:
     """A contiguous tensor as one that starts on 16 bytes: itself, or a copy where it is a view that does not."""
     return t if t.data_ptr() % 16 == 0 else t.clone()

@@ -392,3 +392,55 @@ def test_cache_tensors_of_other_storage_or_shape(nat, what):
             c.block_types = c.block_types[:, :, :2].contiguous()
         from neuralattentionsearchlinear_b200.decode_step import decode_token
         assert decode_token(layer, x[:, 71:72], cache) is None
+
+
+# ------------------------------------------------------------------------------------------------ transforms and traces
+def op_call(nat, rule):
+    op = nat.nats_mixed_attn_gdn if rule == "gdn" else nat.nats_mixed_attn_mamba
+    return lambda args, types: op(*args, types, None, nats_block_size=64, ops_for_incomplete_chunks="all")[:2]
+
+
+@pytest.mark.parametrize("rule", ["gdn", "mamba"])
+@pytest.mark.parametrize("level", ["forward_ad", "jvp", "vmap"])
+def test_op_under_a_transform_raises(nat, rule, level):
+    """The ops have no forward-mode or batching rule: they raise, with and without reverse mode on, and never drop a tangent."""
+    import torch.autograd.forward_ad as fwad
+    run = op_call(nat, rule)
+    args, types, _ = op_inputs(rule, 2, 128, 2, 64 if rule == "gdn" else 128, 64, 64)
+    with_q = lambda q: run((q, *args[1:3], q, *args[4:]), types)
+    for grad in (True, False):
+        with torch.set_grad_enabled(grad), pytest.raises((NotImplementedError, RuntimeError)):
+            if level == "forward_ad":
+                with fwad.dual_level():
+                    with_q(fwad.make_dual(args[0], torch.ones_like(args[0])))
+            elif level == "jvp":
+                torch.func.jvp(with_q, (args[0],), (torch.ones_like(args[0]),))
+            else:
+                torch.func.vmap(with_q)(args[0][None])
+    run(args, types)
+
+
+@pytest.mark.parametrize("rule", ["gdn", "mamba"])
+@pytest.mark.parametrize("what", ["prompt", "token"])
+def test_layer_under_forward_mode_raises(nat, rule, what):
+    import torch.autograd.forward_ad as fwad
+    layer, x = make_layer(nat, rule), tokens(1, 66)
+    cache = nat.NAtSCache()
+    with torch.no_grad():
+        call(layer, x[:, :65], cache)
+        with fwad.dual_level(), pytest.raises(NotImplementedError):
+            piece = x[:, :64] if what == "prompt" else x[:, 65:]
+            call(layer, fwad.make_dual(piece, torch.ones_like(piece)), None if what == "prompt" else cache)
+
+
+@pytest.mark.filterwarnings("ignore::torch.jit.TracerWarning")
+@pytest.mark.parametrize("rule", ["gdn", "mamba"])
+def test_traced_op_computes_with_new_inputs(nat, rule):
+    """A jit trace replays the op on other inputs: nothing of the traced call is frozen into it."""
+    run, K = op_call(nat, rule), 64 if rule == "gdn" else 128
+    (a, types, _), (b, _, _) = op_inputs(rule, 1, 128, 2, K, 64, 64), op_inputs(rule, 1, 128, 2, K, 64, 64, seed=1)
+    fn = lambda q, k, v: run((q, k, v, q, k, v, *a[6:]), types)
+    with torch.no_grad():
+        traced = torch.jit.trace(fn, a[:3], check_trace=False)
+        for got, want in zip(traced(*b[:3]), fn(*b[:3])):
+            close(got, want, rule)
