@@ -310,6 +310,7 @@ attn_fp32_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __re
             }
             *reinterpret_cast<float4*>(s_k + r * L::LDK + d) = x;
         }
+        bool wild = false;                               // an infinity or NaN among the values of the tile
         for (int i = tid; i < AF_K * (DV / 4); i += 128) {
             const int r = i / (DV / 4), d = (i % (DV / 4)) * 4;
             float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -318,8 +319,9 @@ attn_fp32_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __re
                 x = make_float4(ldf(p, 0), ldf(p, 1), ldf(p, 2), ldf(p, 3));
             }
             *reinterpret_cast<float4*>(s_v + r * L::LDV + d) = x;
+            wild |= !(isfinite(x.x) && isfinite(x.y) && isfinite(x.z) && isfinite(x.w));
         }
-        __syncthreads();
+        wild = __syncthreads_or(wild);
         float sc[2][4] = {};
 #pragma unroll 4
         for (int d = 0; d < DK; d += 4) {
@@ -359,7 +361,7 @@ attn_fp32_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __re
         float ps = 0.f;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            x[j] = mn == -INFINITY ? 0.f : __expf(x[j] - mn);
+            x[j] = x[j] == -INFINITY ? -0.f : __expf(x[j] - mn);      // -0: the key is not visible
             ps += x[j];
             s_p[qr * L::LDP + ql + 8 * j] = x[j];
         }
@@ -370,6 +372,15 @@ attn_fp32_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __re
         __syncwarp();                                    // the eight lanes of a query sit in one warp
 #pragma unroll
         for (int d = 0; d < DV / 8; ++d) acc[d] *= al;
+        if (wild) {                                      // 0 times such a value is not 0: only the visible keys count
+            for (int j = 0; j < AF_K; ++j) {
+                const float pj = s_p[qr * L::LDP + j];
+                if (__float_as_uint(pj) == 0x80000000u) continue;
+#pragma unroll
+                for (int d = 0; d < DV / 8; ++d) acc[d] += pj * s_v[j * L::LDV + ql * 4 + 32 * (d / 4) + d % 4];
+            }
+            continue;
+        }
         for (int j = 0; j < AF_K; j += 4) {
             const float4 pj = *reinterpret_cast<const float4*>(s_p + qr * L::LDP + j);
 #pragma unroll

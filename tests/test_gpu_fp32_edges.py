@@ -44,3 +44,24 @@ def test_fp32_attention(T, D, nbs):
                                       nats_block_size=nbs, ops_for_incomplete_chunks="all", decay_for_non_gdn_blocks=True)
     ref, _ = oattn.attn_sdpa(q.double(), k.double(), v.double(), oattn.attn_mask(types[..., 0], T, nbs, H))
     assert_close(o, ref.float(), 1e-4, "o")
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+@pytest.mark.parametrize("where", ["v", "k"])
+def test_non_finite_values_behind_the_mask(D, value, where):
+    """A token that a query does not see changes nothing for it, whatever its key and value hold; it sees its own."""
+    import neuralattentionsearchlinear_b200 as nat
+    B, H, T, bad = 1, 2, 150, 101
+    q, k, v, g, beta, _ = (x.cuda() for x in synth_gdn_inputs(B, T, H, D, D, seed=D, dtype=torch.float32))
+    types = otab.synth_types(B, 3, H, 0.5, seed=1).cuda()
+    k2, v2 = k.clone(), v.clone()
+    (v2 if where == "v" else k2)[:, bad, :, 3] = value
+    run = lambda kk, vv: nat.nats_mixed_attn_gdn(q, kk, vv, q, k, v, None, g, beta, types, None, nats_block_size=64,
+                                                 ops_for_incomplete_chunks="all", decay_for_non_gdn_blocks=True)[1]
+    clean, got = run(k, v), run(k2, v2)
+    assert torch.equal(got[:, :bad], clean[:, :bad])
+    if where == "v":
+        assert not bool(got[:, bad, :, 3].isfinite().any()) and torch.equal(got[:, bad, :, 4:], clean[:, bad, :, 4:])
+    sees = types[:, 1, :, 0] == 1                            # heads whose later queries see the token's block
+    assert torch.equal(got[:, 128:][:, :, ~sees[0]], clean[:, 128:][:, :, ~sees[0]])
