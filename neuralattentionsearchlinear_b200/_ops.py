@@ -197,14 +197,15 @@ def linear_fwd(rule: int, q, k, v, g, beta, tables: SelectionTables, scale: floa
     ht = torch.empty(B, H, K, V, dtype=torch.float32, device=dev) if output_final_state else None
     if h0 is not None:
         h0 = aligned(h0.float().contiguous())
-        _need(tuple(h0.shape) == (B, H, K, V), f"initial state must be [B,H,K,V], got {tuple(h0.shape)}")
+        _need(tuple(h0.shape) == (B, H, K, V) and h0.device == dev, f"initial state must be [B,H,K,V] on {dev}, got {tuple(h0.shape)}")
     flags = (_lib.FLAG_DECAY_SKIPPED if decay else 0) | (0 if trailing_quirk else _lib.FLAG_NO_TRAILING_QUIRK)
     start, last_code = None, _lib.DT_F32
     if want_start:
         _need(fused or mamba_fused, "the block-start state needs head dims with a fused walk", NotImplementedError)
         start = torch.empty(B, H, K, V, dtype=torch.float32, device=dev)
         if T % nbs == 0:
-            _need(last_types is not None and tuple(last_types.shape) == (B, HN, 2), "a complete last block needs its types [B,HN,2]")
+            _need(last_types is not None and tuple(last_types.shape) == (B, HN, 2) and last_types.device == dev,
+                  f"a complete last block needs its types [B,HN,2] on {dev}")
             last_types = (last_types if last_types.dtype in (BF16, torch.float32) else last_types.float()).contiguous()
             last_code = _dt_code(last_types)
         else:
@@ -301,7 +302,7 @@ def hybrid_fwd(rule: int, q_attn, k_attn, v_attn, q, k, v, g, beta, types, nbs: 
         a.beta, a.beta_dtype = beta.data_ptr(), _dt_code(beta)
     if h0 is not None:
         h0 = aligned(h0.float().contiguous())
-        _need(tuple(h0.shape) == (B, H, K, V), f"initial state must be [B,H,K,V], got {tuple(h0.shape)}")
+        _need(tuple(h0.shape) == (B, H, K, V) and h0.device == dev, f"initial state must be [B,H,K,V] on {dev}, got {tuple(h0.shape)}")
         a.h0 = h0.data_ptr()
     o_lin = torch.empty(B, T, H, V, dtype=q.dtype, device=dev)
     o_attn = torch.empty(B, T, HQ, DV, dtype=q.dtype, device=dev)
@@ -309,7 +310,8 @@ def hybrid_fwd(rule: int, q_attn, k_attn, v_attn, q, k, v, g, beta, types, nbs: 
     ht = torch.empty(B, H, K, V, dtype=torch.float32, device=dev) if want_ht else None
     start = torch.empty(B, H, K, V, dtype=torch.float32, device=dev) if want_start else None
     if want_start and T % nbs == 0:
-        _need(last_types is not None and tuple(last_types.shape) == (B, HN, 2), "a complete last block needs its types [B,HN,2]")
+        _need(last_types is not None and tuple(last_types.shape) == (B, HN, 2) and last_types.device == dev,
+              f"a complete last block needs its types [B,HN,2] on {dev}")
         last_types = (last_types if last_types.dtype in (BF16, torch.float32) else last_types.float()).contiguous()
         a.last_types, a.last_dtype, a.last_stride = last_types.data_ptr(), _dt_code(last_types), 2 * HN
     NT, NTq = cdiv(T, 64), cdiv(T, _lib.ATTN_BT)

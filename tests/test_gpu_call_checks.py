@@ -40,6 +40,22 @@ def test_chunk_inference_refuses_fp32(nat, rule, K, V, T, want):
         op(*args, types, last, None, nats_block_size=64, ops_for_incomplete_chunks="all", **{key: want})
 
 
+@pytest.mark.parametrize("rule", ["gdn", "mamba"])
+@pytest.mark.parametrize("what", ["last types", "initial state"])
+def test_host_tensors_raise(nat, rule, what):
+    """Tensors in host memory never reach a kernel by address."""
+    K, V = (64, 64) if rule == "gdn" else (128, 64)
+    args, types, last = op_inputs(rule, 2, 128, 2, K, V, 64)
+    op, key = ((nat.nats_mixed_attn_gdn_chunk_inference, "output_final_state_gated_delta") if rule == "gdn" else
+               (nat.nats_mixed_attn_mamba_chunk_inference, "output_final_state_mamba"))
+    if what == "last types":
+        last = last.cpu()
+    else:
+        args = (*args[:6], torch.zeros(2, 2, K, V), *args[7:])
+    with pytest.raises(ValueError):
+        op(*args, types, last, None, nats_block_size=64, ops_for_incomplete_chunks="all", **{key: True})
+
+
 # ------------------------------------------------------------------------------------------------ layers and their caches
 def make_layer(nat, rule="gdn", **kw):
     cls = nat.NeuralAttentionSearchLinearAttnGDN if rule == "gdn" else nat.NeuralAttentionSearchLinearAttnMamba
