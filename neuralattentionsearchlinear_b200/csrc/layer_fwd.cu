@@ -5,8 +5,6 @@
 // Why one call: a prompt of a thousand tokens is some 200 us of device work in 46 launches that took the host 900 us to
 // issue from Python (about 30 of them torch elementwise kernels over small tensors); the large-batch case read and wrote
 // every projection two or three times (convolution, norm, cast) on its way.  What each kernel is bound by stands beside it.
-#include <mutex>
-
 #include "layer_fwd.cuh"
 #include "tc_common.cuh"
 #include "../../include/natsl_b200.h"
@@ -314,43 +312,44 @@ block_rest_kernel(const float* __restrict__ g, const bf16* __restrict__ x, float
 }
 
 // ------------------------------------------------------------------------------------------------ two streams
-// The linear branch runs on a side stream of high priority (one per device; events per thread), so that its CTAs are placed
-// ahead of the softmax branch's remaining ones whenever an SM frees up: the serial walk starts earlier and the attention CTAs
-// fill in around it (0.621 - 0.633 against 0.640 - 0.644 ms for the whole op at B = 8, T = 4096, H = 16).  The caller's stream
-// forks to it and joins again before the call returns, so every buffer may belong to the caller's stream alone.
-struct ThreadEvents {
-    cudaEvent_t ev[64][3] = {};
-    ~ThreadEvents() {
-        for (auto& e : ev)
-            for (auto& x : e)
-                if (x) cudaEventDestroy(x);
+// The linear branch runs on a side stream of high priority, so that its CTAs are placed ahead of the softmax branch's
+// remaining ones whenever an SM frees up: the serial walk starts earlier and the attention CTAs fill in around it (0.621 -
+// 0.633 against 0.640 - 0.644 ms for the whole op at B = 8, T = 4096, H = 16).  The caller's stream forks to it and joins
+// again before the call returns, so every buffer may belong to the caller's stream alone.  Stream and events belong to the
+// calling thread (one stream per device, given back with the thread): calls of two threads do not queue behind each other,
+// and a thread that captures a graph takes nobody else's work into it.
+struct SideStream {
+    struct {
+        cudaStream_t stream;
+        cudaEvent_t ev[3];
+    } dev[64] = {};
+    ~SideStream() {
+        for (auto& d : dev) {
+            for (auto& e : d.ev)
+                if (e) cudaEventDestroy(e);
+            if (d.stream) cudaStreamDestroy(d.stream);
+        }
     }
 };
-thread_local ThreadEvents t_events;
+thread_local SideStream t_side;
 
 int side_stream(cudaStream_t* side, cudaEvent_t** ev) {
-    static std::mutex mu;
-    static cudaStream_t streams[64] = {};
     int dev = -1;
     cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess && dev >= 0 && dev < 64) {
-        std::lock_guard<std::mutex> lock(mu);
+    if (e == cudaSuccess && (dev < 0 || dev >= 64)) e = cudaErrorInvalidDevice;
+    if (e == cudaSuccess && !t_side.dev[dev].stream) {
         int lo = 0, hi = 0;
-        if (!streams[dev]) {
-            e = cudaDeviceGetStreamPriorityRange(&lo, &hi);
-            if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&streams[dev], cudaStreamNonBlocking, hi < 0 ? -1 : 0);
-        }
-        *side = streams[dev];
-    } else if (e == cudaSuccess) {
-        e = cudaErrorInvalidDevice;
+        e = cudaDeviceGetStreamPriorityRange(&lo, &hi);
+        if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&t_side.dev[dev].stream, cudaStreamNonBlocking, hi < 0 ? -1 : 0);
     }
     for (int i = 0; i < 3 && e == cudaSuccess; ++i)
-        if (!t_events.ev[dev][i]) e = cudaEventCreateWithFlags(&t_events.ev[dev][i], cudaEventDisableTiming);
+        if (!t_side.dev[dev].ev[i]) e = cudaEventCreateWithFlags(&t_side.dev[dev].ev[i], cudaEventDisableTiming);
     if (e != cudaSuccess) {
         set_error("cannot create the side stream: %s", cudaGetErrorString(e));
         return NATSL_ERR_CUDA;
     }
-    *ev = t_events.ev[dev];
+    *side = t_side.dev[dev].stream;
+    *ev = t_side.dev[dev].ev;
     return NATSL_OK;
 }
 

@@ -460,3 +460,77 @@ def test_traced_op_computes_with_new_inputs(nat, rule):
         traced = torch.jit.trace(fn, a[:3], check_trace=False)
         for got, want in zip(traced(*b[:3]), fn(*b[:3])):
             close(got, want, rule)
+
+
+# ------------------------------------------------------------------------------------------------ threads and streams
+def in_thread(fn):
+    """Runs fn in a thread of its own; returns its result or raises what it raised."""
+    import threading
+    box = {}
+
+    def target():
+        try:
+            box["result"] = fn()
+        except BaseException as e:
+            box["error"] = e
+
+    t = threading.Thread(target=target)
+    t.start()
+    t.join(60)
+    assert not t.is_alive()
+    if "error" in box:
+        raise box["error"]
+    return box["result"]
+
+
+@pytest.mark.parametrize("what", ["gdn op", "mamba op", "fp32 op", "layer"])
+def test_a_capture_takes_no_work_of_another_thread(nat, what):
+    """While one thread captures a call into a graph, another thread's call runs at once and stays out of it."""
+    rule, K = ("mamba", 128) if what == "mamba op" else ("gdn", 64)
+    if what == "layer":
+        layer, a, b = make_layer(nat), tokens(1, 128), tokens(1, 128, seed=1)
+        run = lambda x: call(layer, x)
+    else:
+        dtype = torch.float32 if what == "fp32 op" else torch.bfloat16
+        (a, types, _), (b, _, _) = (op_inputs(rule, 1, 128, 2, K, 64, 64, dtype=dtype, seed=s) for s in (0, 1))
+        run = lambda args: op_call(nat, rule)(args, types)[0]
+
+    def eager(x):
+        with torch.no_grad(), torch.cuda.stream(torch.cuda.Stream()):
+            y = run(x)
+            torch.cuda.current_stream().synchronize()
+        return y
+
+    want_a, want_b = eager(a), in_thread(lambda: eager(b))
+    graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.no_grad(), torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+        y = run(a)
+        got_b = in_thread(lambda: eager(b))
+        y2 = run(a)
+    assert torch.equal(got_b, want_b)
+    y.zero_(), y2.zero_()
+    torch.cuda.synchronize()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, want_a) and torch.equal(y2, want_a)
+
+
+def test_threads_on_their_own_streams(nat):
+    """Calls of four threads at once give what they give alone."""
+    import concurrent.futures as cf
+    inputs = [op_inputs("gdn", 2, 300, 2, 64, 64, 64, seed=s) for s in range(4)]
+    run = op_call(nat, "gdn")
+
+    def work(i):
+        with torch.no_grad(), torch.cuda.stream(torch.cuda.Stream()):
+            ys = [run(inputs[i][0], inputs[i][1]) for _ in range(20)]
+            torch.cuda.current_stream().synchronize()
+        return ys
+
+    torch.cuda.synchronize()
+    alone = [work(i)[0] for i in range(4)]
+    with cf.ThreadPoolExecutor(4) as pool:
+        for want, ys in zip(alone, pool.map(work, range(4))):
+            for y in ys:
+                assert all(map(torch.equal, y, want))
