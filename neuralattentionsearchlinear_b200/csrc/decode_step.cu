@@ -465,8 +465,9 @@ __device__ void core_attention(const CoreArgs& c, int idx, float* sm) {
         float mx = sc;
 #pragma unroll
         for (int o = KS / 2; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        const float mn = fmaxf(m, mx), al = exp2f(m - mn);
-        const float p = exp2f(sc - mn);
+        // scores of -inf (infinite keys) weigh nothing, also while there is nothing else
+        const float mn = fmaxf(m, mx), al = mn == -INFINITY ? 1.f : exp2f(m - mn);
+        const float p = mn == -INFINITY ? 0.f : exp2f(sc - mn);
         float ps = p;
 #pragma unroll
         for (int o = KS / 2; o > 0; o >>= 1) ps += __shfl_xor_sync(0xffffffffu, ps, o);

@@ -102,3 +102,28 @@ def test_copied_cache_continues_on_its_own():
         again = [layer(x[:, t:t + 1], past_key_values=fork)[0] for t in range(151, 160)]
     for a, b in zip(first, again):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("B,head_dim", [(1, 64), (2, 128)])
+def test_infinite_keys_weigh_nothing(B, head_dim):
+    """Keys that give every cached token a score of -inf: the new token alone counts, as in the general path."""
+    from neuralattentionsearchlinear_b200 import NAtSCache
+    from neuralattentionsearchlinear_b200.decode_step import decode_token
+    from neuralattentionsearchlinear_b200.decoding import forward_cached
+    torch.manual_seed(2)
+    layer = _gdn(hidden=256, heads=2, head_dim=head_dim, expand_v=1, attn_heads=2).cuda().bfloat16().eval()
+    x = torch.randn(B, 200, 256, device="cuda").bfloat16()
+    with torch.no_grad():
+        cache = NAtSCache()
+        layer(x[:, :199], past_key_values=cache)
+        c = cache[0]
+        q = layer.project_qkv(x[:, 199:], conv_state=c.conv_state, want_conv_state=True)["q_attn"]
+        keys = torch.zeros_like(c.k_attn)
+        keys[..., 5] = torch.where(q[..., 5] > 0, -float("inf"), float("inf")).to(keys.dtype)
+        c.k_attn = keys
+        other = NAtSCache()
+        other.layers = [copy.copy(c)]
+        y = decode_token(layer, x[:, 199:], cache)
+        want = layer.mix(x[:, 199:], *forward_cached(layer, x[:, 199:], other))
+    assert bool(want.isfinite().all())
+    assert float((y.float() - want.float()).abs().max()) <= TOL * float(want.float().abs().max())
