@@ -467,7 +467,7 @@ __device__ void core_attention(const CoreArgs& c, int idx, float* sm) {
         for (int o = KS / 2; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         // scores of -inf (infinite keys) weigh nothing, also while there is nothing else
         const float mn = fmaxf(m, mx), al = mn == -INFINITY ? 1.f : exp2f(m - mn);
-        const float p = mn == -INFINITY ? 0.f : exp2f(sc - mn);
+        const float p = sc == -INFINITY ? 0.f : exp2f(sc - mn);
         float ps = p;
 #pragma unroll
         for (int o = KS / 2; o > 0; o >>= 1) ps += __shfl_xor_sync(0xffffffffu, ps, o);
@@ -515,19 +515,18 @@ __device__ void core_attention(const CoreArgs& c, int idx, float* sm) {
     for (int w = 0; w < 4; ++w) M = fmaxf(M, s_ml[w * 2]);
     float* part = c.part + (((long)b * a.HQ + hq) * c.S + s) * (DV + 2);
     if (tid < DV) {
+        // a part without a finite score holds zeros, or the NaN of a score or value, which goes on as it is
         float L = 0.f, o = 0.f;
-        if (M != -INFINITY) {
 #pragma unroll
-            for (int w = 0; w < 4; ++w) {
-                const float f = exp2f(s_ml[w * 2] - M);
-                L += f * s_ml[w * 2 + 1];
-                o += f * s_acc[w * DV + tid];
-            }
-            if (s_new != -INFINITY) {
-                const float p = exp2f(s_new - M);
-                L += p;
-                o += p * s_vn[tid];
-            }
+        for (int w = 0; w < 4; ++w) {
+            const float f = s_ml[w * 2] == -INFINITY ? 1.f : exp2f(s_ml[w * 2] - M);
+            L += f * s_ml[w * 2 + 1];
+            o += f * s_acc[w * DV + tid];
+        }
+        if (s_new != -INFINITY) {
+            const float p = exp2f(s_new - M);
+            L += p;
+            o += p * s_vn[tid];
         }
         part[2 + tid] = o;
         if (tid == 0) { part[0] = M; part[1] = L; }
@@ -673,7 +672,7 @@ __global__ void __launch_bounds__(128) decode_merge_kernel(const MergeArgs c) {
     float M = fmaxf(m0, m1);
 #pragma unroll
     for (int k = 16; k > 0; k >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, k));
-    const float f0 = M == -INFINITY ? 0.f : exp2f(m0 - M), f1 = M == -INFINITY ? 0.f : exp2f(m1 - M);
+    const float f0 = m0 == -INFINITY ? 1.f : exp2f(m0 - M), f1 = m1 == -INFINITY ? 1.f : exp2f(m1 - M);
     const float L = warp_sum(f0 * s0 + f1 * s1);
 #pragma unroll 4
     for (int s = 0; s < c.S; ++s) {
@@ -685,7 +684,7 @@ __global__ void __launch_bounds__(128) decode_merge_kernel(const MergeArgs c) {
     float q1 = 0.f, q2 = 0.f;
 #pragma unroll
     for (int e = 0; e < E; ++e) {
-        o[e] = rb(L > 0.f ? o[e] / L : 0.f);
+        o[e] = rb(L == 0.f ? 0.f : o[e] / L);
         q1 += x1[e] * x1[e];
         q2 += o[e] * o[e];
     }

@@ -127,3 +127,28 @@ def test_infinite_keys_weigh_nothing(B, head_dim):
         want = layer.mix(x[:, 199:], *forward_cached(layer, x[:, 199:], other))
     assert bool(want.isfinite().all())
     assert float((y.float() - want.float()).abs().max()) <= TOL * float(want.float().abs().max())
+
+
+@pytest.mark.parametrize("where", ["keys", "all keys", "values", "token"])
+def test_nan_reaches_the_output(where):
+    """A NaN that a token sees is in its output, as in the general path."""
+    from neuralattentionsearchlinear_b200 import NAtSCache
+    from neuralattentionsearchlinear_b200.decode_step import decode_token
+    torch.manual_seed(2)
+    layer = _gdn(hidden=256, heads=2, head_dim=64, expand_v=1, attn_heads=2).cuda().bfloat16().eval()
+    x = torch.randn(1, 200, 256, device="cuda").bfloat16()
+    with torch.no_grad():
+        cache = NAtSCache()
+        layer(x[:, :199], past_key_values=cache)
+        c = cache[0]
+        k, v, tok = c.k_attn.clone(), c.v_attn.clone(), x[:, 199:].clone()
+        if where == "keys":
+            k[:, 194, :, 3] = float("nan")
+        elif where == "all keys":
+            k.fill_(float("nan"))
+        elif where == "values":
+            v[:, 194] = float("nan")
+        else:
+            tok[0, 0, 7] = float("nan")
+        c.k_attn, c.v_attn = k, v
+        assert bool(decode_token(layer, tok, cache).isnan().all())
