@@ -291,11 +291,12 @@ gdn_walk_mma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                 *reinterpret_cast<uint32_t*>(base_p + L::q + swz<128>(rb, nt) + qd * 4) = pack_bf16(acc[nt][2] * scale, acc[nt][3] * scale);
             }
             __syncwarp();
+            __nv_bfloat16* o_c = o_p + (long)c * 64 * H * V;
 #pragma unroll
             for (int j = 0; j < NTL / 2; ++j) {
                 const int r = r0 + (lane + 32 * j) / NTL, ch = (lane + 32 * j) % NTL;
                 if (c * 64 + r < T)
-                    *reinterpret_cast<uint4*>(o_p + (c * 64 + r) * H * V + ch * 8) =
+                    *reinterpret_cast<uint4*>(o_c + r * H * V + ch * 8) =
                         *reinterpret_cast<const uint4*>(base_p + L::q + swz<128>(r, ch));
             }
             // orders v' and these rows (written with ordinary stores) before the next tiles that TMA writes there
@@ -391,7 +392,8 @@ static int launch_walk_mma(const void* q, const void* k, const void* w, const vo
     const char* who = "natsl_gdn_walk";
     const int NT = (T + 63) / 64;
     const int smem = L::total(NT, nbs > 64);
-    NATSL_REQUIRE((long)T * H * V < (1l << 31), NATSL_ERR_TOO_LARGE, "natsl_gdn_walk: T * H * V must be below 2^31");
+    NATSL_REQUIRE((long)T * H < (1l << 31) && 64l * H * V < (1l << 31), NATSL_ERR_TOO_LARGE,
+                  "natsl_gdn_walk: T * H and 64 * H * V must be below 2^31");
     NATSL_REQUIRE(smem <= 227 * 1024, NATSL_ERR_TOO_LARGE, "natsl_gdn_walk: T=%d needs %d B of shared memory (max %d)", T, smem, 227 * 1024);
     auto kern = gdn_walk_mma_kernel<K, BV>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);

@@ -73,3 +73,22 @@ def test_mamba_walk_block_start_state(T, nbs, decay):
     assert_close(ht, fin_ref, TOL, "final state")
     assert_close(inter["start"], start_ref, TOL, "block-start state")
     assert _lib.load().natsl_device_status() == 0
+
+
+def test_walk_of_more_than_2_31_outputs():
+    """T * H * V = 2^31: offsets of the output that do not fit 32 bits, against the two-kernel form on the last tokens."""
+    import neuralattentionsearchlinear_b200 as nat
+    from neuralattentionsearchlinear_b200 import _lib, _ops
+    T, H, K, V = 65536, 128, 128, 256
+    gen = torch.Generator(device="cuda").manual_seed(0)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda", dtype=torch.bfloat16)
+    q, k, v, beta = rnd(1, T, H, K), rnd(1, T, H, K), rnd(1, T, H, V), rnd(1, T, H).sigmoid()
+    g = -torch.nn.functional.softplus(rnd(1, T, H).float())
+    types = otab.synth_types(1, T // 64, 1, 0.5, seed=0).cuda()
+    o = _ops.linear_fwd(_lib.RULE_GDN, q, k, v, g, beta, nat.build_selection_tables(types, T, 64), K ** -0.5, None, True, True, True)[0]
+    n = 4096                                                 # the decayed state forgets what lies further back
+    tail = [x[:, -n:].contiguous() for x in (q, k, v, g, beta)]
+    tb = nat.build_selection_tables(types[:, -n // 64:].contiguous(), n, 64)
+    want = _ops.linear_fwd(_lib.RULE_GDN, *tail, tb, K ** -0.5, None, True, True, True, return_intermediates=True)[0]
+    assert_close(o[:, -n // 2:], want[:, -n // 2:].float(), TOL, "o")
+    assert _lib.load().natsl_device_status() == 0
