@@ -11,13 +11,13 @@ import weakref
 import torch
 import torch.nn as nn
 
-from . import _lib
+from . import _lib, nats_util
 from .modules import FusedMultiInputRMSNormGated, L2Norm, RMSNorm, ShortConvolution, mean_pooling
 from .nats_util import aligned, current_stream_ptr, device_guard, transforms_active
 
 BF16 = torch.bfloat16
 MAX_BATCH = 64
-_kind = operator.attrgetter("dtype", "shape")
+_dtype = operator.attrgetter("dtype")
 _tls = threading.local()                     # one argument block per thread: a call in flight is never rewritten
 
 
@@ -50,27 +50,43 @@ class _Plan:
         if layer.attn_qk_norm:
             mods["q_norm"] = mods["k_norm"] = RMSNorm
         self.mods = [(layer._modules, n, layer._modules.get(n)) for n in mods]
-        attrs = [(layer.__dict__, n) for n in (*_LAYER_ATTRS, *_LAYER_HOOKS)]
-        attrs += [(m.__dict__, n) for _, _, m in self.mods if m is not None and not isinstance(m, nn.Linear)
-                  for n in ("eps", "activation", "kernel_size", "hidden_size")]
         self.hooks, self.params, self.device = [], [], None
         if all(type(m) is mods[n] for _, n, m in self.mods):
             self.hooks = [h for _, _, m in self.mods for h in (m._forward_hooks, m._forward_pre_hooks)]
-            self.ok = self._fill(layer, gdn, weighted) and not any(h in layer.__dict__ for h in _LAYER_HOOKS)
-        # what current() compares, as flat sequences for one pass in C each
-        self._mod_d, self._mod_n, self._mod_v = zip(*self.mods)
-        self._att_d, self._att_n = zip(*attrs)
+            self.ok = self._fill(layer, gdn, weighted)
+        self._hooked = any(self.hooks)
+        # what current() compares, in as few passes in C as it takes (a token's host time is some 30 us)
+        self._layer_dict, self._modules = layer.__dict__, layer._modules
+        self._replaced = list(map(layer.__dict__.__contains__, _LAYER_HOOKS))
+        self.ok = self.ok and not self._hooked and not any(self._replaced)
+        self._get_mods = operator.itemgetter(*(n for n in mods if n in layer._modules))
+        self._mods = self._get_mods(layer._modules)
+        self._get_attrs = operator.itemgetter(*(n for n in _LAYER_ATTRS if n in layer.__dict__))
+        self._attrs = self._get_attrs(layer.__dict__)
+        attrs = [(m.__dict__, n) for m in self._mods for n in ("eps", "activation", "kernel_size", "hidden_size")
+                 if m is not None and n in m.__dict__]
+        self._att_d, self._att_n = zip(*attrs) if attrs else ((), ())
         self._att_v = list(map(dict.get, self._att_d, self._att_n))
-        self._par_d, self._par_n, self._par_v = zip(*self.params) if self.params else ((), (), ())
-        self._tensors = [t for t in self._par_v if t is not None]
-        self._ptrs = [t.data_ptr() for t in self._tensors]
-        self._kinds = list(map(_kind, self._tensors))
+        there = sorted(((d, n) for d, n, p in self.params if p is not None), key=lambda e: -e[0][e[1]].dim())
+        self._n_mat = sum(d[n].dim() > 1 for d, n in there)   # matrices first
+        self._par_d, self._par_n = zip(*there) if there else ((), ())
+        absent = [(d, n) for d, n, p in self.params if p is None]
+        self._abs_d, self._abs_n = zip(*absent) if absent else ((), ())
+        self._nones = [None] * len(absent)
+        self._par_v = self._look(map(dict.get, self._par_d, self._par_n))
+
+    def _look(self, tensors):
+        """Addresses and types, of matrices also sizes and contiguity: what a kernel takes on trust of the weights."""
+        t = list(tensors)
+        mats = t[:self._n_mat]
+        return (list(map(torch.Tensor.data_ptr, t)), list(map(_dtype, t)), list(map(torch.Tensor.numel, mats)),
+                all(map(torch.Tensor.is_contiguous, mats)))
 
     def _fill(self, layer, gdn: bool, weighted: bool) -> bool:
         a = self.args = _lib.DecodeArgs()
 
         m = layer
-        self.device = m.q_proj.weight.device
+        self.device, index = m.q_proj.weight.device, m.q_proj.weight.get_device()
         linears = [mod for _, _, mod in self.mods if type(mod) is nn.Linear]
         self.params += [(mod._parameters, "bias", mod.bias) for mod in linears]          # the products add none
         H, HQ, K, V, DK, DV, D = (m.num_heads, m.num_attn_heads, m.head_k_dim, m.head_v_dim, m.head_attn_k_dim, m.head_attn_v_dim,
@@ -81,16 +97,17 @@ class _Plan:
             self.params.append((owner._parameters, name, p))
             if p is None:
                 return optional
-            if type(p) not in (nn.Parameter, torch.Tensor) or tuple(p.shape) != shape:
+            if type(p) not in (nn.Parameter, torch.Tensor) or p.shape != shape or p.get_device() != index:
                 return False
-            if any_float is not None and p.dtype == torch.float32:
+            dtype, ptr = p.dtype, p.data_ptr()
+            if any_float is not None and dtype == torch.float32:
                 setattr(a, any_float, 1)
-            elif p.dtype != BF16:
+            elif dtype != BF16:
                 return False
-            setattr(a, field, p.data_ptr())
+            setattr(a, field, ptr)
             # products read 16 bytes at a time, convolutions 8: a parameter that is a view into a flat buffer may start anywhere
             align = 16 if field.startswith("w_") else 8 if field.startswith("cw_") else 1
-            return p.is_cuda and p.is_contiguous() and p.device == self.device and p.data_ptr() % align == 0
+            return index >= 0 and p.is_contiguous() and ptr % align == 0
 
         checks = [weight("w_q", m.q_proj, H * K, D), weight("w_k", m.k_proj, H * K, D), weight("w_v", m.v_proj, H * V, D),
                   weight("w_a", m.a_proj, H, D), weight("w_g", m.g_proj, H * V, D), weight("w_o", m.o_proj, D, H * V),
@@ -123,6 +140,7 @@ class _Plan:
             and m.use_short_conv and m.use_gate and m.ops_for_incomplete_chunks != 'attn' and m.incomplete_block_start_with_ht
             and not m.usg_for_attn and m.pooling_func is mean_pooling)
         a.hidden, a.H, a.K, a.V, a.HQ, a.HN = D, H, K, V, HQ, m.num_nats_head
+        self.hidden = D
         a.nbs, a.rule = m.nats_block_size, _lib.RULE_GDN if gdn else _lib.RULE_MAMBA
         a.silu = int(m.q_conv1d.activation in ("silu", "swish"))
         a.mix_sigmoid, a.mix_eps = int(m.o_norm.activation == "sigmoid"), m.o_norm.eps
@@ -139,11 +157,14 @@ class _Plan:
         return ok
 
     def current(self) -> bool:
-        return (all(map(operator.is_, map(dict.get, self._mod_d, self._mod_n), self._mod_v))
-                and list(map(dict.get, self._att_d, self._att_n)) == self._att_v and not any(self.hooks)
-                and all(map(operator.is_, map(dict.get, self._par_d, self._par_n), self._par_v))
-                and list(map(torch.Tensor.data_ptr, self._tensors)) == self._ptrs and list(map(_kind, self._tensors)) == self._kinds
-                and all(map(torch.Tensor.is_contiguous, self._tensors)))
+        try:
+            return (self._get_mods(self._modules) == self._mods and self._get_attrs(self._layer_dict) == self._attrs
+                    and list(map(dict.get, self._att_d, self._att_n)) == self._att_v
+                    and list(map(self._layer_dict.__contains__, _LAYER_HOOKS)) == self._replaced and any(self.hooks) == self._hooked
+                    and list(map(dict.get, self._abs_d, self._abs_n)) == self._nones
+                    and self._look(map(dict.get, self._par_d, self._par_n)) == self._par_v)
+        except (KeyError, TypeError):                        # a module, attribute or weight has gone
+            return False
 
 
 class _Step:
@@ -153,7 +174,7 @@ class _Step:
         self.plan, self.cache_tensors = plan, None
         a = self.args = _lib.DecodeArgs()
         ctypes.memmove(ctypes.byref(a), ctypes.byref(plan.args), ctypes.sizeof(a))
-        a.B = B
+        a.B = self.B = B
         need = plan.ws_bytes.get(B)
         if need is None:
             need = plan.ws_bytes[B] = _lib.load().natsl_decode_workspace_bytes(ctypes.byref(a))
@@ -216,32 +237,33 @@ def layer_plan(layer) -> _Plan:
     p = plans.get(layer)
     if p is None or not p.current():
         p = plans[layer] = _Plan(layer)
-        p.ok = p.ok and not any(p.hooks)                     # a plan with hooks is never current: looked at again next time
     return p
 
 
 def decode_token(layer, x: torch.Tensor, container):
     """The layer's output [B, 1, hidden] for one new token, or None where the general path has to run (which also raises
     what there is to raise).  Updates the layer's cache."""
-    if x.dim() != 3 or x.shape[1] != 1 or x.dtype != BF16 or not x.is_cuda or layer.layer_idx is None or not hasattr(container, "layer"):
+    shape = x.shape
+    if len(shape) != 3 or shape[1] != 1 or x.dtype != BF16 or not x.is_cuda or layer.layer_idx is None or not hasattr(container, "layer"):
         return None
     plan = layer_plan(layer)
     # the kernel reads and writes batch * hidden entries of x and the output: every token's width and device count
-    if not plan.ok or x.shape[2] != plan.args.hidden or x.device != plan.device:
+    if not plan.ok or shape[2] != plan.hidden or x.get_device() != plan.device.index:
         return None
     nbs = layer.nats_block_size
     cache = container.layer(layer.layer_idx, nbs)
-    pos = cache.n_tokens
-    B = x.shape[0]
+    B = shape[0]
     step = cache._step
-    if step is None or step.plan is not plan or step.args.B != B:
+    if step is None or step.plan is not plan or step.B != B:
         if B > MAX_BATCH:
             return None
         step = _Step(plan, B, x.device)
     if torch.is_autocast_enabled() or torch.nn.modules.module._has_any_global_hook() or transforms_active():
         return None
-    with torch.no_grad(), device_guard(plan.device):
-        return _decode(layer, x, cache, step, pos, nbs)
+    if nats_util.current_device() == plan.device.index:
+        return _decode(layer, x, cache, step, cache.n_tokens, nbs)
+    with device_guard(plan.device):
+        return _decode(layer, x, cache, step, cache.n_tokens, nbs)
 
 
 def _decode(layer, x, cache, step, pos: int, nbs: int):
@@ -260,15 +282,17 @@ def _decode(layer, x, cache, step, pos: int, nbs: int):
     n_done = pos // nbs
     if n_done and (cache.block_types is None or cache.block_types.shape[1] != n_done):
         return None
-    x = aligned(x.contiguous())
+    x = aligned((x.detach() if x.requires_grad else x).contiguous())
     types_new = None
     if (pos + 1) % nbs == 0:                                 # a block's type is decided once its last token is known
-        pooled = ((cache._pool_sum + x[:, 0].float()) / nbs).to(x.dtype)[:, None, :]
-        types_new = layer.select(pooled).contiguous()
+        with torch.no_grad():
+            pooled = ((cache._pool_sum + x[:, 0].float()) / nbs).to(x.dtype)[:, None, :]
+            types_new = layer.select(pooled).contiguous()
         if types_new.dtype not in (BF16, torch.float32) or (cache.block_types is not None and cache.block_types.dtype != types_new.dtype):
             return None
     cache.reserve_kv(1)
-    cache.own_state()
+    if cache._handed_out:
+        cache.own_state()
     if not step.bound(cache) and not step.bind(cache):
         return None
     cache._step = step

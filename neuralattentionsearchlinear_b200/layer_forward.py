@@ -53,20 +53,17 @@ def _forward(layer, plan, x, cache):
     TN = cdiv(T, nbs)
     bf = dict(dtype=BF16, device=dev)
     f32 = dict(dtype=torch.float32, device=dev)
+    project = lambda name: F.linear(x, layer._modules[name]._parameters["weight"])
     pooled = torch.empty(B, TN, D, **bf)
     _lib.call("natsl_block_mean", x.data_ptr(), pooled.data_ptr(), B, T, D, nbs, st)
     logits = F.linear(pooled, sel.weight)
-    q_raw, k_raw, v_raw = (F.linear(x, m.weight) for m in (layer.q_proj, layer.k_proj, layer.v_proj))
+    q_raw, k_raw, v_raw = project("q_proj"), project("k_proj"), project("v_proj")
     a = plan.layer_args
     a.B, a.T = B, T
     a.options = ((0 if _ops.PREP_TC else _lib.HYBRID_PREP_MMA) | (_lib.HYBRID_WALK_MMA if B * H <= _ops.WALK_MMA_MAX_HEADS else 0)
                  | (_lib.HYBRID_ATTN_PERSISTENT if _ops.ATTN_PERSISTENT else 0))
-    normed = bool(d.qn_w)
     DK, DV = H * K // HQ, H * V // HQ
-    k_attn = torch.empty(B, T, HQ, DK, **bf) if (normed or a.attn_conv) else k_raw.view(B, T, HQ, DK)
-    v_attn = torch.empty(B, T, HQ, DV, **bf) if a.attn_conv else v_raw.view(B, T, HQ, DV)
-    types_raw = torch.empty(B, TN, HN, 2, **bf)
-    nt = B * TN * HN * 2
+    n, nt = B * T, B * TN * HN * 2
     tables = torch.empty(2 * nt + 3 * B * HN + B * cdiv(T, 128) * HN, dtype=torch.int32, device=dev)
     key = (B, T)
     need = plan.layer_ws.get(key)
@@ -74,10 +71,12 @@ def _forward(layer, plan, x, cache):
         if len(plan.layer_ws) > 256:
             plan.layer_ws.clear()
         need = plan.layer_ws[key] = _lib.load().natsl_layer_workspace_bytes(ctypes.byref(a))
-    # intermediates of the call, then what only the mixing behind it reads
-    n = B * T
+    own_k, own_v = bool(d.qn_w) or a.attn_conv, a.attn_conv  # keys, values that are not the projections themselves
+    # intermediates of the call, what only the mixing behind it reads, and what a cache would keep
     sizes = [_r256(need), _r256(2 * n * H * V), _r256(2 * n * H * V), _r256(4 * n * HQ), _r256(4 * n * HQ),
              _r256(2 * n * H * V) if gdn and not a.attn_conv else 0]
+    if cache is None:
+        sizes += [_r256(2 * n * H * K) if own_k else 0, _r256(2 * n * H * V) if own_v else 0, _r256(2 * nt)]
     ws = torch.empty(sum(sizes), dtype=torch.uint8, device=dev)
     p = ws.data_ptr()
     a.workspace, a.workspace_bytes = p, need
@@ -87,21 +86,29 @@ def _forward(layer, plan, x, cache):
     a.lse = a.mix + sizes[3]
     a.v_lin = a.lse + sizes[4] if sizes[5] else None
     a.x, a.logits, a.q_raw, a.k_raw, a.v_raw = x.data_ptr(), logits.data_ptr(), q_raw.data_ptr(), k_raw.data_ptr(), v_raw.data_ptr()
-    a.types_raw, a.tables, a.k_attn, a.v_attn = types_raw.data_ptr(), tables.data_ptr(), k_attn.data_ptr(), v_attn.data_ptr()
+    a.tables = tables.data_ptr()
     if cache is None:
+        kept = p + sum(sizes[:6])
+        a.k_attn = kept if own_k else a.k_raw
+        a.v_attn = kept + sizes[6] if own_v else a.v_raw
+        a.types_raw = kept + sizes[6] + sizes[7]
         a.ht = a.hstart = a.tail_q = a.tail_k = a.tail_v = a.g_block = a.pool_sum = None
     else:
+        k_attn = torch.empty(B, T, HQ, DK, **bf) if own_k else k_raw.view(B, T, HQ, DK)
+        v_attn = torch.empty(B, T, HQ, DV, **bf) if own_v else v_raw.view(B, T, HQ, DV)
+        types_raw = torch.empty(B, TN, HN, 2, **bf)
         ht, start = torch.empty(B, H, K, V, **f32), torch.empty(B, H, K, V, **f32)
         tails = tuple(torch.empty(B, c, 4, **bf) for c in (H * K, H * K, H * V))
         g_block, pool_sum = torch.empty(B, H, **f32), torch.empty(B, D, **f32)
+        a.k_attn, a.v_attn, a.types_raw = k_attn.data_ptr(), v_attn.data_ptr(), types_raw.data_ptr()
         a.ht, a.hstart, a.g_block, a.pool_sum = ht.data_ptr(), start.data_ptr(), g_block.data_ptr(), pool_sum.data_ptr()
         a.tail_q, a.tail_k, a.tail_v = (t.data_ptr() for t in tails)
     _lib.call("natsl_layer_forward", ctypes.byref(a), st)
-    gate = F.linear(x, layer.g_proj.weight)
+    gate = project("g_proj")
     y = torch.empty(B, T, H * V, **bf)
     _lib.call("natsl_norm_gate_mix", a.o_lin, a.o_attn, gate.data_ptr(), a.mix if a.w_mix else None, _lib.DT_BF16, d.w1, d.w2,
               _lib.DT_F32 if d.w12_f32 else _lib.DT_BF16, y.data_ptr(), n * HQ, DV, d.mix_eps, d.mix_sigmoid, st)
-    layer.attn_blocks = (tables[2 * nt:2 * nt + 2 * B * HN].view(B, HN, 2), TN)
+    layer.__dict__["attn_blocks"] = (tables[2 * nt:2 * nt + 2 * B * HN].view(B, HN, 2), TN)
     if cache is not None:
         r, n_done = T % nbs, T // nbs
         cache.append_kv(k_attn, v_attn)
@@ -109,4 +116,4 @@ def _forward(layer, plan, x, cache):
             cache.append_types(types_raw if n_done == TN else types_raw[:, :n_done].contiguous())
         cache.set_state(start.clone() if r == 0 else ht, start, g_block, pool_sum, tails)
         cache.n_tokens = T
-    return F.linear(y, layer.o_proj.weight)
+    return F.linear(y, layer._modules["o_proj"]._parameters["weight"])

@@ -189,7 +189,8 @@ def test_work_runs_with_the_tensors_device_current(nat, what, monkeypatch):
         def __exit__(self, *exc):
             pass
 
-    monkeypatch.setattr(torch.cuda, "current_device", lambda: 1)
+    from neuralattentionsearchlinear_b200 import nats_util
+    monkeypatch.setattr(nats_util, "current_device", lambda: 1)
     monkeypatch.setattr(torch.cuda, "device", Guard)
     with torch.no_grad():
         if what == "prompt":
