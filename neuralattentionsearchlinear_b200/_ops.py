@@ -267,8 +267,10 @@ def hybrid_fwd(rule: int, q_attn, k_attn, v_attn, q, k, v, g, beta, types, nbs: 
     for t_ in (q_attn, k_attn, v_attn, q, k, v):
         _need(t_.dim() == 4, "q, k, v must be [B, T, H, D]")
         _need(t_.is_cuda and t_.device == q.device, "q, k, v of both branches must be on one CUDA device")
-        _need(t_.dtype == q.dtype, "q, k, v of both branches must share a dtype", TypeError)
+    _need(q.dtype == k.dtype == v.dtype and q_attn.dtype == k_attn.dtype == v_attn.dtype, "q, k, v must share a dtype", TypeError)
     fp32 = q.dtype == torch.float32
+    _need(q_attn.dtype == q.dtype or (fp32 and q_attn.dtype == BF16), f"softmax branch in {q_attn.dtype} beside a linear branch "
+          f"in {q.dtype}", TypeError)
     _need(fp32 or q.dtype == BF16, f"unsupported dtype {q.dtype} (fp32 or bf16)", TypeError)
     _need(not (fp32 and want_start), "the block-start state needs bf16 tensors", TypeError)
     q_attn, k_attn, v_attn, q, k, v = (t_.contiguous() for t_ in (q_attn, k_attn, v_attn, q, k, v))
@@ -305,7 +307,7 @@ def hybrid_fwd(rule: int, q_attn, k_attn, v_attn, q, k, v, g, beta, types, nbs: 
         _need(tuple(h0.shape) == (B, H, K, V) and h0.device == dev, f"initial state must be [B,H,K,V] on {dev}, got {tuple(h0.shape)}")
         a.h0 = h0.data_ptr()
     o_lin = torch.empty(B, T, H, V, dtype=q.dtype, device=dev)
-    o_attn = torch.empty(B, T, HQ, DV, dtype=q.dtype, device=dev)
+    o_attn = torch.empty(B, T, HQ, DV, dtype=q_attn.dtype, device=dev)
     lse = torch.empty(B, T, HQ, dtype=torch.float32, device=dev)
     ht = torch.empty(B, H, K, V, dtype=torch.float32, device=dev) if want_ht else None
     start = torch.empty(B, H, K, V, dtype=torch.float32, device=dev) if want_start else None
@@ -332,7 +334,7 @@ def hybrid_fwd(rule: int, q_attn, k_attn, v_attn, q, k, v, g, beta, types, nbs: 
     a.g, a.types, a.o_attn, a.lse, a.o_lin = g.data_ptr(), types.data_ptr(), o_attn.data_ptr(), lse.data_ptr(), o_lin.data_ptr()
     a.ht, a.hstart = _lib.ptr(ht), _lib.ptr(start)
     if fp32:
-        a.options |= _lib.HYBRID_FP32
+        a.options |= _lib.HYBRID_FP32 | (_lib.HYBRID_ATTN_BF16 if q_attn.dtype == BF16 else 0)
         with device_guard(dev):
             _lib.call("natsl_hybrid_forward", ctypes.byref(a), current_stream_ptr(dev))
         return o_lin, o_attn, lse, ht, start, flat

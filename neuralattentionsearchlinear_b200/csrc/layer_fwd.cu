@@ -429,8 +429,8 @@ int hybrid_forward(const natsl_hybrid_args& a, void* types_raw, cudaStream_t st,
                                             a.T, a.H, a.HN, a.K, a.V, a.nbs, a.scale_lin, a.decay ? NATSL_FLAG_DECAY_SKIPPED : 0,
                                             a.use_l2norm, side);
         if (rc == NATSL_OK)
-            rc = natsl_attn_fwd_fp32(NATSL_DT_F32, a.q_attn, a.k_attn, a.v_attn, a.types_i, a.o_attn, a.lse, a.B, a.T, a.HQ, a.HKV, a.HN,
-                                     a.DK, a.DV, a.nbs, a.scale_attn, a.own_attn ? NATSL_FLAG_ATTN_OWN_CHUNK : 0, st);
+            rc = natsl_attn_fwd_fp32((a.options & NATSL_HYBRID_ATTN_BF16) ? NATSL_DT_BF16 : NATSL_DT_F32, a.q_attn, a.k_attn, a.v_attn,
+                                     a.types_i, a.o_attn, a.lse, a.B, a.T, a.HQ, a.HKV, a.HN, a.DK, a.DV, a.nbs, a.scale_attn, a.own_attn ? NATSL_FLAG_ATTN_OWN_CHUNK : 0, st);
         const int join = stream_after(st, side, ev[2]);
         return rc != NATSL_OK ? rc : join;
     }

@@ -65,3 +65,27 @@ def test_non_finite_values_behind_the_mask(D, value, where):
         assert not bool(got[:, bad, :, 3].isfinite().any()) and torch.equal(got[:, bad, :, 4:], clean[:, bad, :, 4:])
     sees = types[:, 1, :, 0] == 1                            # heads whose later queries see the token's block
     assert torch.equal(got[:, 128:][:, :, ~sees[0]], clean[:, 128:][:, :, ~sees[0]])
+
+
+@pytest.mark.parametrize("rule", ["gdn", "mamba"])
+def test_fp32_linear_branch_beside_a_bf16_softmax_branch(rule):
+    """Each branch takes its own dtype: outputs in it, equal to those of the branch on its own; the other mix raises."""
+    import neuralattentionsearchlinear_b200 as nat
+    from tests.helpers import synth_mamba_inputs
+    B, T, H, D = 2, 130, 2, 64
+    if rule == "gdn":
+        q, k, v, g, beta, _ = (x.cuda() for x in synth_gdn_inputs(B, T, H, D, D, seed=3, dtype=torch.float32))
+        op, rest = nat.nats_mixed_attn_gdn, (None, g, beta)
+    else:
+        q, k, v, g, _ = (x.cuda() for x in synth_mamba_inputs(B, T, H, D, D, seed=3, dtype=torch.float32))
+        op, rest = nat.nats_mixed_attn_mamba, (None, g)
+    types = otab.synth_types(B, 3, H, 0.5, seed=3)
+    low = [x.bfloat16() for x in (q, k, v)]
+    run = lambda a, l: op(*a, *l, *rest, types.cuda(), None, nats_block_size=64, ops_for_incomplete_chunks="all")[:2]
+    o_l, o_a = run(low, (q, k, v))
+    assert o_l.dtype == torch.float32 and o_a.dtype == torch.bfloat16
+    assert torch.equal(o_l, run((q, k, v), (q, k, v))[0])
+    ref, _ = oattn.attn_sdpa(*(x.double().cpu() for x in low), oattn.attn_mask(types[..., 0], T, 64, H))
+    assert_close(o_a, ref.float(), 2.0 ** -8, "o")           # one rounding of the output
+    with pytest.raises(TypeError):
+        run((q, k, v), low)
