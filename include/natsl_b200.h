@@ -256,6 +256,7 @@ int natsl_attn_fwd_fp32(int dtype, const void* q, const void* k, const void* v, 
 #define NATSL_HYBRID_WALK_MMA 2        /* mma.sync walk also where the tcgen05 one is built (few (batch, head) pairs) */
 #define NATSL_HYBRID_ATTN_PERSISTENT 4
 #define NATSL_HYBRID_FP32 8            /* fp32 tensors: natsl_linear_recurrent_fwd and natsl_attn_fwd_fp32 side by side (no workspace) */
+#define NATSL_HYBRID_WALK_VSPLIT 32    /* natsl_gdn_walk_fused_vsplit in place of the one-CTA tcgen05 walk where it is built (no hstart) */
 #define NATSL_HYBRID_ATTN_BF16 16      /* with NATSL_HYBRID_FP32: q_attn, k_attn, v_attn, o_attn are bf16 */
 typedef struct natsl_hybrid_args {
     int32_t B, T, H, HN, K, V, HQ, HKV, DK, DV, nbs, rule;

@@ -116,7 +116,7 @@ class LayerArgs(C.Structure):
         + [("workspace_bytes", C.c_int64)])
 
 
-HYBRID_PREP_MMA, HYBRID_WALK_MMA, HYBRID_ATTN_PERSISTENT, HYBRID_FP32, HYBRID_ATTN_BF16 = 1, 2, 4, 8, 16
+HYBRID_PREP_MMA, HYBRID_WALK_MMA, HYBRID_ATTN_PERSISTENT, HYBRID_FP32, HYBRID_ATTN_BF16, HYBRID_WALK_VSPLIT = 1, 2, 4, 8, 16, 32
 
 
 _lib = None

@@ -257,6 +257,12 @@ def tables_from_flat(flat, B: int, TN: int, HN: int, T: int, nbs: int) -> Select
                            T=T, nats_block_size=nbs)
 
 
+def hybrid_options(pairs: int) -> int:
+    """``options`` of the native op and layer calls for this many (batch, head) pairs of the linear branch."""
+    return ((0 if PREP_TC else _lib.HYBRID_PREP_MMA) | (_lib.HYBRID_WALK_MMA if pairs <= WALK_MMA_MAX_HEADS else 0)
+            | (_lib.HYBRID_ATTN_PERSISTENT if ATTN_PERSISTENT else 0) | (_lib.HYBRID_WALK_VSPLIT if WALK_VSPLIT else 0))
+
+
 _hybrid_ws: dict = {}
 
 
@@ -327,8 +333,7 @@ def hybrid_fwd(rule: int, q_attn, k_attn, v_attn, q, k, v, g, beta, types, nbs: 
     a.B, a.T, a.H, a.HN, a.K, a.V, a.HQ, a.HKV, a.DK, a.DV, a.nbs, a.rule = B, T, H, HN, K, V, HQ, HKV, DK, DV, nbs, rule
     a.types_dtype = _TYPE_CODES[types.dtype]
     a.own_attn, a.decay, a.use_l2norm = int(own_attn), int(decay), int(use_l2norm)
-    a.options = ((0 if PREP_TC else _lib.HYBRID_PREP_MMA) | (_lib.HYBRID_WALK_MMA if B * H <= WALK_MMA_MAX_HEADS else 0)
-                 | (_lib.HYBRID_ATTN_PERSISTENT if ATTN_PERSISTENT else 0))
+    a.options = hybrid_options(B * H)
     a.scale_attn, a.scale_lin = float(scale_attn), float(scale_lin)
     a.q_attn, a.k_attn, a.v_attn, a.q, a.k, a.v = (t_.data_ptr() for t_ in (q_attn, k_attn, v_attn, q, k, v))
     a.g, a.types, a.o_attn, a.lse, a.o_lin = g.data_ptr(), types.data_ptr(), o_attn.data_ptr(), lse.data_ptr(), o_lin.data_ptr()

@@ -430,7 +430,8 @@ int hybrid_forward(const natsl_hybrid_args& a, void* types_raw, cudaStream_t st,
                                             a.use_l2norm, side);
         if (rc == NATSL_OK)
             rc = natsl_attn_fwd_fp32((a.options & NATSL_HYBRID_ATTN_BF16) ? NATSL_DT_BF16 : NATSL_DT_F32, a.q_attn, a.k_attn, a.v_attn,
-                                     a.types_i, a.o_attn, a.lse, a.B, a.T, a.HQ, a.HKV, a.HN, a.DK, a.DV, a.nbs, a.scale_attn, a.own_attn ? NATSL_FLAG_ATTN_OWN_CHUNK : 0, st);
+                                     a.types_i, a.o_attn, a.lse, a.B, a.T, a.HQ, a.HKV, a.HN, a.DK, a.DV, a.nbs, a.scale_attn,
+                                     a.own_attn ? NATSL_FLAG_ATTN_OWN_CHUNK : 0, st);
         const int join = stream_after(st, side, ev[2]);
         return rc != NATSL_OK ? rc : join;
     }
@@ -450,9 +451,13 @@ int hybrid_forward(const natsl_hybrid_args& a, void* types_raw, cudaStream_t st,
     const int flags = (a.decay ? NATSL_FLAG_DECAY_SKIPPED : 0);
     const void* last = types_raw ? (const void*)(reinterpret_cast<bf16*>(types_raw) + (long)(TN - 1) * a.HN * 2) : a.last_types;
     const int last_dtype = types_raw ? NATSL_DT_BF16 : a.last_dtype;
-    if (rc == NATSL_OK && gdn) {
-        auto walk = (a.K == 128 && a.V == 128 && a.nbs == 64 && a.T <= 65536 && !(a.options & NATSL_HYBRID_WALK_MMA))
-                        ? natsl_gdn_walk_fused_ex : natsl_gdn_walk;
+    const bool tc_walk = gdn && a.K == 128 && a.V == 128 && a.nbs == 64 && a.T <= 65536 && !(a.options & NATSL_HYBRID_WALK_MMA);
+    if (rc == NATSL_OK && tc_walk && (a.options & NATSL_HYBRID_WALK_VSPLIT) && a.T <= 8192 && !a.hstart) {
+        rc = natsl_gdn_walk_fused_vsplit(a.q, a.k, ws + l.w, ws + l.u, ws + l.p, gcs, reinterpret_cast<float*>(ws + l.kr),
+                                         reinterpret_cast<float*>(ws + l.qr), a.types_i, a.indices, a.n_blocks, a.h0, a.o_lin, a.ht, a.B,
+                                         a.T, a.H, a.HN, a.K, a.V, a.nbs, a.scale_lin, flags, side);
+    } else if (rc == NATSL_OK && gdn) {
+        auto walk = tc_walk ? natsl_gdn_walk_fused_ex : natsl_gdn_walk;
         rc = walk(a.q, a.k, ws + l.w, ws + l.u, ws + l.p, gcs, reinterpret_cast<float*>(ws + l.kr), reinterpret_cast<float*>(ws + l.qr),
                   a.types_i, a.indices, a.n_blocks, a.h0, a.o_lin, a.ht, a.hstart, last, last_dtype, a.last_stride, a.B, a.T, a.H, a.HN,
                   a.K, a.V, a.nbs, a.scale_lin, flags, side);

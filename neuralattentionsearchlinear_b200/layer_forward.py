@@ -60,8 +60,7 @@ def _forward(layer, plan, x, cache):
     q_raw, k_raw, v_raw = project("q_proj"), project("k_proj"), project("v_proj")
     a = plan.layer_args
     a.B, a.T = B, T
-    a.options = ((0 if _ops.PREP_TC else _lib.HYBRID_PREP_MMA) | (_lib.HYBRID_WALK_MMA if B * H <= _ops.WALK_MMA_MAX_HEADS else 0)
-                 | (_lib.HYBRID_ATTN_PERSISTENT if _ops.ATTN_PERSISTENT else 0))
+    a.options = _ops.hybrid_options(B * H)
     DK, DV = H * K // HQ, H * V // HQ
     n, nt = B * T, B * TN * HN * 2
     tables = torch.empty(2 * nt + 3 * B * HN + B * cdiv(T, 128) * HN, dtype=torch.int32, device=dev)

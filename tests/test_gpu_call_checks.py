@@ -535,3 +535,33 @@ def test_threads_on_their_own_streams(nat):
         for want, ys in zip(alone, pool.map(work, range(4))):
             for y in ys:
                 assert all(map(torch.equal, y, want))
+
+
+# ------------------------------------------------------------------------------------------------ switches
+def kernels_of(fn):
+    from torch.profiler import ProfilerActivity, profile
+    fn()
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        fn()
+        torch.cuda.synchronize()
+    return [e.name for e in p.events()]
+
+
+@pytest.mark.parametrize("what", ["op", "layer"])
+def test_split_walk_switch_reaches_the_op(nat, what, monkeypatch):
+    """WALK_VSPLIT runs the walk with the value dimension split, with the results of the walk it stands in for."""
+    from neuralattentionsearchlinear_b200 import _ops
+    monkeypatch.setattr(_ops, "WALK_MMA_MAX_HEADS", 0)
+    if what == "op":
+        args, types, _ = op_inputs("gdn", 2, 300, 2, 128, 128, 64)
+        fn = lambda: op_call(nat, "gdn")(args, types)[0]
+    else:
+        layer, x = make_layer(nat, head_dim=128, num_heads=2, num_attn_heads=2), tokens(2, 300)
+        fn = lambda: call(layer, x)
+    with torch.no_grad():
+        want = fn()
+        assert not any("gdn_walk_half_kernel" in k for k in kernels_of(fn))
+        monkeypatch.setattr(_ops, "WALK_VSPLIT", True)
+        names = kernels_of(fn)
+        assert any("gdn_walk_half_kernel" in k for k in names), names
+        close(fn(), want, what)
