@@ -248,7 +248,7 @@ int natsl_attn_fwd_fp32(int dtype, const void* q, const void* k, const void* v, 
                         int flags, void* stream);
 
 /* Both branches of the op in one call, forward: selection tables, softmax branch, linear branch (preparation or cumsum, then
- * the recurrence + output walk), the linear branch on a high-priority side stream of the library's own that forks from and
+ * the recurrence + output walk), the linear branch on a high-priority side stream of the calling thread that forks from and
  * joins `stream` inside the call.  Shapes as in natsl_attn_fwd_ex / natsl_gdn_walk(_fused_ex) / natsl_mamba_walk_fused_ex;
  * gcs: chunk-local cumsum of g if the caller has it (Mamba2), else NULL; tables as in natsl_build_tables (starting_h_idx may
  * be NULL; without the compact list).  ht, hstart, h0, last_types may be NULL. */
@@ -257,6 +257,7 @@ int natsl_attn_fwd_fp32(int dtype, const void* q, const void* k, const void* v, 
 #define NATSL_HYBRID_ATTN_PERSISTENT 4
 #define NATSL_HYBRID_FP32 8            /* fp32 tensors: natsl_linear_recurrent_fwd and natsl_attn_fwd_fp32 side by side (no workspace) */
 #define NATSL_HYBRID_WALK_VSPLIT 32    /* natsl_gdn_walk_fused_vsplit in place of the one-CTA tcgen05 walk where it is built (no hstart) */
+#define NATSL_HYBRID_PLAIN_PRIORITY 64 /* linear branch on `stream`, the other one on a side stream of normal priority */
 #define NATSL_HYBRID_ATTN_BF16 16      /* with NATSL_HYBRID_FP32: q_attn, k_attn, v_attn, o_attn are bf16 */
 typedef struct natsl_hybrid_args {
     int32_t B, T, H, HN, K, V, HQ, HKV, DK, DV, nbs, rule;

@@ -116,7 +116,8 @@ class LayerArgs(C.Structure):
         + [("workspace_bytes", C.c_int64)])
 
 
-HYBRID_PREP_MMA, HYBRID_WALK_MMA, HYBRID_ATTN_PERSISTENT, HYBRID_FP32, HYBRID_ATTN_BF16, HYBRID_WALK_VSPLIT = 1, 2, 4, 8, 16, 32
+(HYBRID_PREP_MMA, HYBRID_WALK_MMA, HYBRID_ATTN_PERSISTENT, HYBRID_FP32, HYBRID_ATTN_BF16, HYBRID_WALK_VSPLIT,
+ HYBRID_PLAIN_PRIORITY) = 1, 2, 4, 8, 16, 32, 64
 
 
 _lib = None

@@ -27,6 +27,12 @@ PREP_TC = os.environ.get("NATSL_PREP_TC", "1") != "0"
 # Off by default: parity-green but measured slower (0.43 vs 0.29 ms at B=8, T=4096, H=16).
 ATTN_PERSISTENT = os.environ.get("NATSL_ATTN_PERSISTENT", "0") == "1"
 
+# The linear branch (chunk preparation -> walk) runs on a high-priority stream, so that its CTAs are placed ahead of the
+# softmax branch's remaining ones whenever an SM frees up: the serial walk then starts earlier and the attention CTAs
+# fill in around it.  Measured with the step replayed from a CUDA graph: 0.621 - 0.633 ms against 0.640 - 0.644 ms
+# (three runs each); NATSL_LINEAR_PRIORITY=0 puts the branch back on the caller's stream.
+LINEAR_BRANCH_PRIORITY = os.environ.get("NATSL_LINEAR_PRIORITY", "1") != "0"
+
 # (batch, head) pairs up to which the delta rule takes the mma.sync walk also where the tcgen05 one is built (K = V = 128,
 # block 64): its slices of the value dim fill four SMs per pair, and a chunk takes 1.6 instead of 2.8 us.  Measured at
 # T = 2048: 32 pairs 51 against 90 us, 48 and 64 pairs 78 against 91 us, 128 pairs (T = 4096) 283 against 174 us.  The line
@@ -260,7 +266,8 @@ def tables_from_flat(flat, B: int, TN: int, HN: int, T: int, nbs: int) -> Select
 def hybrid_options(pairs: int) -> int:
     """``options`` of the native op and layer calls for this many (batch, head) pairs of the linear branch."""
     return ((0 if PREP_TC else _lib.HYBRID_PREP_MMA) | (_lib.HYBRID_WALK_MMA if pairs <= WALK_MMA_MAX_HEADS else 0)
-            | (_lib.HYBRID_ATTN_PERSISTENT if ATTN_PERSISTENT else 0) | (_lib.HYBRID_WALK_VSPLIT if WALK_VSPLIT else 0))
+            | (_lib.HYBRID_ATTN_PERSISTENT if ATTN_PERSISTENT else 0) | (_lib.HYBRID_WALK_VSPLIT if WALK_VSPLIT else 0)
+            | (0 if LINEAR_BRANCH_PRIORITY else _lib.HYBRID_PLAIN_PRIORITY))
 
 
 _hybrid_ws: dict = {}

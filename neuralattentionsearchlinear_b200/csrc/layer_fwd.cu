@@ -315,32 +315,35 @@ block_rest_kernel(const float* __restrict__ g, const bf16* __restrict__ x, float
 // The linear branch runs on a side stream of high priority, so that its CTAs are placed ahead of the softmax branch's
 // remaining ones whenever an SM frees up: the serial walk starts earlier and the attention CTAs fill in around it (0.621 -
 // 0.633 against 0.640 - 0.644 ms for the whole op at B = 8, T = 4096, H = 16).  The caller's stream forks to it and joins
-// again before the call returns, so every buffer may belong to the caller's stream alone.  Stream and events belong to the
-// calling thread (one stream per device, given back with the thread): calls of two threads do not queue behind each other,
+// again before the call returns, so every buffer may belong to the caller's stream alone.  With NATSL_HYBRID_PLAIN_PRIORITY
+// the linear branch stays on the caller's stream and the other one takes a side stream of normal priority.  Streams and events
+// belong to the calling thread (one stream of a kind per device, given back with the thread): calls of two threads do not queue behind each other,
 // and a thread that captures a graph takes nobody else's work into it.
 struct SideStream {
     struct {
-        cudaStream_t stream;
+        cudaStream_t stream[2];              // of normal, of high priority
         cudaEvent_t ev[3];
     } dev[64] = {};
     ~SideStream() {
         for (auto& d : dev) {
             for (auto& e : d.ev)
                 if (e) cudaEventDestroy(e);
-            if (d.stream) cudaStreamDestroy(d.stream);
+            for (auto& s : d.stream)
+                if (s) cudaStreamDestroy(s);
         }
     }
 };
 thread_local SideStream t_side;
 
-int side_stream(cudaStream_t* side, cudaEvent_t** ev) {
+int side_stream(int high, cudaStream_t* side, cudaEvent_t** ev) {
     int dev = -1;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess && (dev < 0 || dev >= 64)) e = cudaErrorInvalidDevice;
-    if (e == cudaSuccess && !t_side.dev[dev].stream) {
+    if (e == cudaSuccess && !t_side.dev[dev].stream[high]) {
         int lo = 0, hi = 0;
         e = cudaDeviceGetStreamPriorityRange(&lo, &hi);
-        if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&t_side.dev[dev].stream, cudaStreamNonBlocking, hi < 0 ? -1 : 0);
+        if (e == cudaSuccess)
+            e = cudaStreamCreateWithPriority(&t_side.dev[dev].stream[high], cudaStreamNonBlocking, high && hi < 0 ? -1 : 0);
     }
     for (int i = 0; i < 3 && e == cudaSuccess; ++i)
         if (!t_side.dev[dev].ev[i]) e = cudaEventCreateWithFlags(&t_side.dev[dev].ev[i], cudaEventDisableTiming);
@@ -348,7 +351,7 @@ int side_stream(cudaStream_t* side, cudaEvent_t** ev) {
         set_error("cannot create the side stream: %s", cudaGetErrorString(e));
         return NATSL_ERR_CUDA;
     }
-    *side = t_side.dev[dev].stream;
+    *side = t_side.dev[dev].stream[high];
     *ev = t_side.dev[dev].ev;
     return NATSL_OK;
 }
@@ -407,13 +410,15 @@ int check_hybrid(const natsl_hybrid_args& a) {
 }
 
 // Both branches.  types_dtype TBL_LOGITS: a.types are logits, types_raw receives the sampled types.  `before_attn` is launched
-// on the caller's stream beside the linear branch.
+// beside the linear branch.
 template <typename F>
 int hybrid_forward(const natsl_hybrid_args& a, void* types_raw, cudaStream_t st, F before_attn) {
     cudaStream_t side = st;
     cudaEvent_t* ev = nullptr;
-    int rc = side_stream(&side, &ev);
+    const bool high = !(a.options & NATSL_HYBRID_PLAIN_PRIORITY);
+    int rc = side_stream(high, &side, &ev);
     if (rc != NATSL_OK) return rc;
+    const cudaStream_t lin = high ? side : st, att = high ? st : side;
     const HybridLayout l = hybrid_layout(a);
     unsigned char* ws = reinterpret_cast<unsigned char*>(a.workspace);
     float* gcs = reinterpret_cast<float*>(ws + l.gcs);
@@ -427,11 +432,11 @@ int hybrid_forward(const natsl_hybrid_args& a, void* types_raw, cudaStream_t st,
         if (rc == NATSL_OK)
             rc = natsl_linear_recurrent_fwd(a.rule, NATSL_DT_F32, a.q, a.k, a.v, a.g, a.beta, a.types_i, a.h0, a.o_lin, a.ht, a.hstart, a.B,
                                             a.T, a.H, a.HN, a.K, a.V, a.nbs, a.scale_lin, a.decay ? NATSL_FLAG_DECAY_SKIPPED : 0,
-                                            a.use_l2norm, side);
+                                            a.use_l2norm, lin);
         if (rc == NATSL_OK)
             rc = natsl_attn_fwd_fp32((a.options & NATSL_HYBRID_ATTN_BF16) ? NATSL_DT_BF16 : NATSL_DT_F32, a.q_attn, a.k_attn, a.v_attn,
                                      a.types_i, a.o_attn, a.lse, a.B, a.T, a.HQ, a.HKV, a.HN, a.DK, a.DV, a.nbs, a.scale_attn,
-                                     a.own_attn ? NATSL_FLAG_ATTN_OWN_CHUNK : 0, st);
+                                     a.own_attn ? NATSL_FLAG_ATTN_OWN_CHUNK : 0, att);
         const int join = stream_after(st, side, ev[2]);
         return rc != NATSL_OK ? rc : join;
     }
@@ -440,14 +445,14 @@ int hybrid_forward(const natsl_hybrid_args& a, void* types_raw, cudaStream_t st,
     if (rc == NATSL_OK && gdn) {
         auto prep = (a.K == 128 && a.V == 128 && !(a.options & NATSL_HYBRID_PREP_MMA)) ? natsl_gdn_chunk_prep_tc : natsl_gdn_chunk_prep_ex;
         rc = prep(a.q, a.k, a.v, a.g, a.beta, a.beta_dtype, ws + l.w, ws + l.u, gcs, reinterpret_cast<float*>(ws + l.kr),
-                  reinterpret_cast<float*>(ws + l.qr), ws + l.p, a.B, a.T, a.H, a.K, a.V, a.use_l2norm, side);
+                  reinterpret_cast<float*>(ws + l.qr), ws + l.p, a.B, a.T, a.H, a.K, a.V, a.use_l2norm, lin);
     } else if (rc == NATSL_OK && !a.gcs) {
-        rc = natsl_chunk_local_cumsum(a.g, gcs, a.B, a.T, a.H, side);
+        rc = natsl_chunk_local_cumsum(a.g, gcs, a.B, a.T, a.H, lin);
     }
     if (rc == NATSL_OK)
         rc = launch_tables(a.types, a.types_dtype, types_raw, a.B, TN, a.HN, a.T, a.nbs, a.types_i, a.indices, a.n_blocks,
-                           a.n_chunks_lin, a.starting_h_idx, a.attn_n_iters, st);
-    if (rc == NATSL_OK) rc = stream_after(side, st, ev[1]);
+                           a.n_chunks_lin, a.starting_h_idx, a.attn_n_iters, att);
+    if (rc == NATSL_OK) rc = stream_after(lin, att, ev[1]);
     const int flags = (a.decay ? NATSL_FLAG_DECAY_SKIPPED : 0);
     const void* last = types_raw ? (const void*)(reinterpret_cast<bf16*>(types_raw) + (long)(TN - 1) * a.HN * 2) : a.last_types;
     const int last_dtype = types_raw ? NATSL_DT_BF16 : a.last_dtype;
@@ -455,23 +460,23 @@ int hybrid_forward(const natsl_hybrid_args& a, void* types_raw, cudaStream_t st,
     if (rc == NATSL_OK && tc_walk && (a.options & NATSL_HYBRID_WALK_VSPLIT) && a.T <= 8192 && !a.hstart) {
         rc = natsl_gdn_walk_fused_vsplit(a.q, a.k, ws + l.w, ws + l.u, ws + l.p, gcs, reinterpret_cast<float*>(ws + l.kr),
                                          reinterpret_cast<float*>(ws + l.qr), a.types_i, a.indices, a.n_blocks, a.h0, a.o_lin, a.ht, a.B,
-                                         a.T, a.H, a.HN, a.K, a.V, a.nbs, a.scale_lin, flags, side);
+                                         a.T, a.H, a.HN, a.K, a.V, a.nbs, a.scale_lin, flags, lin);
     } else if (rc == NATSL_OK && gdn) {
         auto walk = tc_walk ? natsl_gdn_walk_fused_ex : natsl_gdn_walk;
         rc = walk(a.q, a.k, ws + l.w, ws + l.u, ws + l.p, gcs, reinterpret_cast<float*>(ws + l.kr), reinterpret_cast<float*>(ws + l.qr),
                   a.types_i, a.indices, a.n_blocks, a.h0, a.o_lin, a.ht, a.hstart, last, last_dtype, a.last_stride, a.B, a.T, a.H, a.HN,
-                  a.K, a.V, a.nbs, a.scale_lin, flags, side);
+                  a.K, a.V, a.nbs, a.scale_lin, flags, lin);
     } else if (rc == NATSL_OK) {
         rc = natsl_mamba_walk_fused_ex(a.q, a.k, a.v, a.gcs ? a.gcs : gcs, a.types_i, a.indices, a.n_blocks, a.h0, a.o_lin, a.ht,
                                        a.hstart, last, last_dtype, a.last_stride, a.B, a.T, a.H, a.HN, a.K, a.V, a.nbs, a.scale_lin,
-                                       flags, side);
+                                       flags, lin);
     }
-    if (rc == NATSL_OK) rc = before_attn(st);
+    if (rc == NATSL_OK) rc = before_attn(att);
     if (rc == NATSL_OK)
         rc = natsl_attn_fwd_ex(a.q_attn, a.k_attn, a.v_attn, a.types_i, a.indices, a.attn_n_iters, a.o_attn, a.lse, a.B, a.T, a.T, 0,
                                a.HQ, a.HKV, a.HN, a.DK, a.DV, a.nbs, a.scale_attn,
                                (a.own_attn ? NATSL_FLAG_ATTN_OWN_CHUNK : 0) |
-                                   ((a.options & NATSL_HYBRID_ATTN_PERSISTENT) ? NATSL_FLAG_ATTN_PERSISTENT : 0), st);
+                                   ((a.options & NATSL_HYBRID_ATTN_PERSISTENT) ? NATSL_FLAG_ATTN_PERSISTENT : 0), att);
     const int join = stream_after(st, side, ev[2]);          // also after an error: the side stream may hold work of this call
     return rc != NATSL_OK ? rc : join;
 }

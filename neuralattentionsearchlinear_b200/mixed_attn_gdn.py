@@ -34,11 +34,6 @@ def _get_attn_stream(device: torch.device) -> torch.cuda.Stream:
 
 
 _lin_streams: dict = {}
-# The linear branch (chunk preparation -> walk) runs on a high-priority stream, so that its CTAs are placed ahead of the
-# softmax branch's remaining ones whenever an SM frees up: the serial walk then starts earlier and the attention CTAs
-# fill in around it.  Measured with the step replayed from a CUDA graph: 0.621 - 0.633 ms against 0.640 - 0.644 ms
-# (three runs each); NATSL_LINEAR_PRIORITY=0 puts the branch back on the caller's stream.
-LINEAR_BRANCH_PRIORITY = os.environ.get("NATSL_LINEAR_PRIORITY", "1") != "0"
 
 
 def _get_linear_stream(device: torch.device) -> torch.cuda.Stream:
@@ -192,7 +187,7 @@ class NAtSMixedAttentionGDN(torch.autograd.Function):
             tables_ready = torch.cuda.Event()
             tables_ready.record(side)
             o_attn, lse = _ops.attn_fwd(q_attn, k_attn, v_attn, tables, scale_attn, own_chunk=strategy['attn'])
-        lin = _get_linear_stream(q_attn.device) if LINEAR_BRANCH_PRIORITY else cur
+        lin = _get_linear_stream(q_attn.device) if _ops.LINEAR_BRANCH_PRIORITY else cur
         if lin is not cur:
             lin.wait_stream(cur)
         with torch.cuda.stream(lin):

@@ -565,3 +565,32 @@ def test_split_walk_switch_reaches_the_op(nat, what, monkeypatch):
         names = kernels_of(fn)
         assert any("gdn_walk_half_kernel" in k for k in names), names
         close(fn(), want, what)
+
+
+@pytest.mark.parametrize("what", ["gdn op", "mamba op", "fp32 op", "layer"])
+def test_priority_switch_moves_the_linear_branch(nat, what, monkeypatch):
+    """LINEAR_BRANCH_PRIORITY: on, the linear branch leaves the caller's stream; off, the softmax branch does.  Same results."""
+    from torch.profiler import ProfilerActivity, profile
+
+    from neuralattentionsearchlinear_b200 import _ops
+    if what == "layer":
+        layer, x = make_layer(nat), tokens(2, 300)
+        fn = lambda: call(layer, x)
+    else:
+        rule, K = ("mamba", 128) if what == "mamba op" else ("gdn", 64)
+        args, types, _ = op_inputs(rule, 2, 300, 2, K, 64, 64, dtype=torch.float32 if what == "fp32 op" else torch.bfloat16)
+        fn = lambda: op_call(nat, rule)(args, types)[0]
+    mark, outs, linear = torch.zeros(256, device="cuda"), [], "linear_recurrent" if what == "fp32 op" else "walk"
+    for high in (True, False):
+        monkeypatch.setattr(_ops, "LINEAR_BRANCH_PRIORITY", high)
+        with torch.no_grad():
+            outs.append(fn())
+            with profile(activities=[ProfilerActivity.CUDA]) as p:
+                mark.add_(1)
+                fn()
+                torch.cuda.synchronize()
+        stream = {k: {e.device_resource_id for e in p.events() if k in e.name} for k in (linear, "attn", "elementwise")}
+        caller = min(stream["elementwise"], default=None)
+        assert caller is not None and stream["attn" if high else linear] == {caller}, stream
+        assert caller not in stream[linear if high else "attn"], stream
+    assert torch.equal(*outs)
