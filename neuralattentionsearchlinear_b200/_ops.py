@@ -34,10 +34,13 @@ ATTN_PERSISTENT = os.environ.get("NATSL_ATTN_PERSISTENT", "0") == "1"
 LINEAR_BRANCH_PRIORITY = os.environ.get("NATSL_LINEAR_PRIORITY", "1") != "0"
 
 # (batch, head) pairs up to which the delta rule takes the mma.sync walk also where the tcgen05 one is built (K = V = 128,
-# block 64): its slices of the value dim fill four SMs per pair, and a chunk takes 1.6 instead of 2.8 us.  Measured at
-# T = 2048: 32 pairs 51 against 90 us, 48 and 64 pairs 78 against 91 us, 128 pairs (T = 4096) 283 against 174 us.  The line
-# is drawn at 31 so that from 32 pairs on a sequence's result does not depend, bit for bit, on the batch around it.
-WALK_MMA_MAX_HEADS = 31
+# block 64): 32 value columns per CTA make four CTAs of a pair, which fit one wave of 148 SMs up to 37 pairs, and a chunk takes
+# 1.6 instead of 2.8 us.  Walk alone, mma.sync against tcgen05, T = 2048: 32 pairs 57 / 91 us; 48 - 64 pairs (64 columns per
+# CTA) 86 / 93 us; 80 pairs (two waves) 160 / 92 us.  In the whole op, where a walk on all SMs delays the softmax branch, up to
+# 36 pairs gain at every length (T = 512: 45 / 53, T = 4096: 252 / 291 us), 48 - 72 pairs gain up to 8 % at T <= 1024 and lose
+# up to 10 % at T = 4096.  Between 31 and 37 the line gives way to batches of 16-head sequences: from two of them on a
+# sequence's result does not depend, bit for bit, on the batch around it.  0 extends that to one sequence (one walk for all).
+WALK_MMA_MAX_HEADS = int(os.environ.get("NATSL_WALK_MMA_MAX_HEADS", "31"))
 
 
 def _attn_flags(own_chunk: bool) -> int:

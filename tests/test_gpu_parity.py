@@ -312,6 +312,7 @@ def test_gdn_fused_walk(nat, B, T, H, HN, decay, use_h0, vsplit, monkeypatch):
     over two CTAs)."""
     from neuralattentionsearchlinear_b200 import _lib, _ops
     monkeypatch.setattr(_ops, "WALK_VSPLIT", vsplit)
+    monkeypatch.setattr(_ops, "WALK_MMA_MAX_HEADS", 0)     # few pairs take the mma.sync walk otherwise
     K = V = 128
     q, k, v, g, beta, h0 = synth_gdn_inputs(B, T, H, K, V, seed=T + 5, normalize_qk=False)
     if not use_h0:
@@ -321,7 +322,12 @@ def test_gdn_fused_walk(nat, B, T, H, HN, decay, use_h0, vsplit, monkeypatch):
     args = (_lib.RULE_GDN, q.cuda(), k.cuda(), v.cuda(), g.cuda(), beta.cuda(), tb, K ** -0.5,
             None if h0 is None else h0.cuda(), decay, True, True)
     assert _ops.USE_FUSED_WALK
-    o, ht, inter = _ops.linear_fwd(*args)
+    ran = []
+    launch = _lib.call
+    with monkeypatch.context() as m:
+        m.setattr(_lib, "call", lambda name, *a: (ran.append(name), launch(name, *a)))
+        o, ht, inter = _ops.linear_fwd(*args)
+    assert ran[-1] == ("natsl_gdn_walk_fused_vsplit" if vsplit else "natsl_gdn_walk_fused_ex")
     assert inter is None                                   # fused path: no per-chunk states
     assert _lib.load().natsl_device_status() == 0
     o_ref, s_ref = ogdn.linear_chunk(q.float(), k.float(), v.float(), g, beta.float(), types[..., 1], nbs=64, h0=h0,
