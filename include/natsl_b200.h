@@ -186,12 +186,23 @@ int natsl_gdn_walk_fused_ex(const void* q, const void* k, const void* w, const v
                             float* hstart, const void* last_types, int last_dtype, int last_stride, int B, int T, int H, int HN, int K, int V,
                             int nbs, float scale, int flags, void* stream);
 
-/* The same recurrence + output walk on mma.sync for K in {64, 128, 192}, V a multiple of 32 (64 and up) and any
+/* The same recurrence + output walk on mma.sync for K in {64, 128}, V a multiple of 32 (64 and up) and any
  * nats_block_size; same arguments.  It cuts the value dim into slices of 32 or 64 columns per CTA. */
 int natsl_gdn_walk(const void* q, const void* k, const void* w, const void* u, const void* pmat, const float* gcs,
                    const float* k_rstd, const float* q_rstd, const int32_t* types_i, const int32_t* indices,
                    const int32_t* n_blocks, const float* h0, void* o, float* ht, float* hstart, const void* last_types,
                    int last_dtype, int last_stride, int B, int T, int H, int HN, int K, int V, int nbs, float scale, int flags, void* stream);
+
+/* Delta rule with the state and every computed operand to fp32 precision between bf16 tensors (K = 192, V a multiple of 32, any
+ * nats_block_size).  tp [B,T,H,320] bf16 = per token its rows of the chunk's (I + A)^-1 diag(beta) in three bf16 parts and of its
+ * score matrix P in two; kf, qf [B,T,H] and vf [2,B,T,H] fp32 = row factors (inverse norms times the decay from the chunk's start, for
+ * vf to its end and in two parts), egl [B,NT,H] fp32 = decay over a chunk; the other arguments as in natsl_gdn_chunk_prep_ex and natsl_gdn_walk. */
+int natsl_gdn_split_prep(const void* q, const void* k, const float* g, const void* beta, int beta_dtype, void* tp, float* kf, float* qf,
+                         float* vf, float* egl, int B, int T, int H, int K, int use_l2norm, void* stream);
+int natsl_gdn_split_walk(const void* q, const void* k, const void* v, const void* tp, const float* kf, const float* qf,
+                         const float* vf, const float* egl, const int32_t* types_i, const int32_t* indices, const int32_t* n_blocks,
+                         const float* h0, void* o, float* ht, float* hstart, const void* last_types, int last_dtype, int last_stride,
+                         int B, int T, int H, int HN, int K, int V, int nbs, float scale, int flags, void* stream);
 
 /* The same walk with the value dimension split over two CTAs per (batch, head): 256 tensor-memory columns and about
  * 107 KB of shared memory per CTA, so that two of them, or one of them and one attention CTA, share an SM (the two

@@ -44,6 +44,8 @@ PROTOTYPES = {
     "natsl_gdn_walk_fused": [_p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _f, _i, _p],
     "natsl_gdn_walk_fused_ex": [_p] * 16 + [_i] * 9 + [_f, _i, _p],
     "natsl_gdn_walk": [_p] * 16 + [_i] * 9 + [_f, _i, _p],
+    "natsl_gdn_split_prep": [_p, _p, _p, _p, _i, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _p],
+    "natsl_gdn_split_walk": [_p] * 16 + [_i] * 9 + [_f, _i, _p],
     "natsl_mamba_walk_fused_ex": [_p] * 12 + [_i] * 9 + [_f, _i, _p],
     "natsl_gdn_walk_fused_vsplit": [_p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _f, _i, _p],
     "natsl_mamba_walk_fused": [_p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _f, _i, _p],

@@ -13,7 +13,8 @@ BF16 = torch.bfloat16
 USE_MAMBA_WALK = os.environ.get("NATSL_MAMBA_WALK", "1") != "0"    # natsl_mamba_walk_fused (K = 128, V = 64)
 # recurrence + output in one walk: on tcgen05 (natsl_gdn_walk_fused, K = V = 128, block 64) or mma.sync (natsl_gdn_walk)
 USE_FUSED_WALK = True
-# (K, V) with a chunk preparation; all of them have a walk for every block size
+# (K, V) with a chunk preparation; all of them have a walk for every block size.  192 / 384 (the 760M configuration) runs the
+# form that holds state and operands to fp32 precision (natsl_gdn_split_*).
 GDN_HEAD_DIMS = {(64, 64), (64, 128), (128, 64), (128, 128), (128, 256), (192, 384)}
 # value dimension of the fused walk split over two CTAs (natsl_gdn_walk_fused_vsplit, T <= 8192): half an SM per CTA.
 # Off by default: measured alone it is no faster than the one-CTA walk (0.204 vs 0.189 ms at B=8, T=4096, H=16), and
@@ -190,13 +191,22 @@ def linear_fwd(rule: int, q, k, v, g, beta, tables: SelectionTables, scale: floa
     if rule == _lib.RULE_GDN:
         beta = beta.contiguous()
         _need(beta.dtype in (BF16, torch.float32), "beta must be bf16 or fp32", TypeError)
-        w = torch.empty(B, T, H, K, dtype=BF16, device=dev)
-        u = torch.empty(B, T, H, V, dtype=BF16, device=dev)
+        beta_code = _lib.DT_BF16 if beta.dtype == BF16 else _lib.DT_F32
         krstd = torch.empty(B, T, H, dtype=torch.float32, device=dev)
         qrstd = torch.empty(B, T, H, dtype=torch.float32, device=dev) if fused else None
+    split = rule == _lib.RULE_GDN and K == 192
+    if split:
+        tp = torch.empty(B, T, H, 320, dtype=BF16, device=dev)
+        egl = torch.empty(B, NT, H, dtype=torch.float32, device=dev)
+        factors = (gcs, krstd, torch.empty(2, B, T, H, dtype=torch.float32, device=dev), egl)
+        _lib.call("natsl_gdn_split_prep", q.data_ptr(), k.data_ptr(), g.data_ptr(), beta.data_ptr(), beta_code, tp.data_ptr(),
+                  *(t.data_ptr() for t in factors), B, T, H, K, int(use_l2norm), st)
+    elif rule == _lib.RULE_GDN:
+        w = torch.empty(B, T, H, K, dtype=BF16, device=dev)
+        u = torch.empty(B, T, H, V, dtype=BF16, device=dev)
         pmat = torch.empty(B, T, H, 64, dtype=BF16, device=dev) if fused else None
         _lib.call(prep_entry(K, V), q.data_ptr() if fused else None, k.data_ptr(), v.data_ptr(), g.data_ptr(),
-                  beta.data_ptr(), _lib.DT_BF16 if beta.dtype == BF16 else _lib.DT_F32, w.data_ptr(), u.data_ptr(),
+                  beta.data_ptr(), beta_code, w.data_ptr(), u.data_ptr(),
                   gcs.data_ptr(), krstd.data_ptr(), _lib.ptr(qrstd), _lib.ptr(pmat), B, T, H, K, V, int(use_l2norm), st)
     else:
         w, u, krstd = None, v, None
@@ -223,14 +233,16 @@ def linear_fwd(rule: int, q, k, v, g, beta, tables: SelectionTables, scale: floa
     if fused:
         # recurrence + output in one walk; the per-chunk states are never materialised
         o = torch.empty(B, T, H, V, dtype=BF16, device=dev)
-        args = (q.data_ptr(), k.data_ptr(), w.data_ptr(), u.data_ptr(), pmat.data_ptr(), gcs.data_ptr(), krstd.data_ptr(),
-                qrstd.data_ptr(), tables.types_i.data_ptr(), tables.indices.data_ptr(), tables.n_blocks.data_ptr(),
+        operands = (v, tp, *factors) if split else (w, u, pmat, gcs, krstd, qrstd)
+        args = (q.data_ptr(), k.data_ptr(), *(t.data_ptr() for t in operands),
+                tables.types_i.data_ptr(), tables.indices.data_ptr(), tables.n_blocks.data_ptr(),
                 _lib.ptr(h0), o.data_ptr(), _lib.ptr(ht))
         dims = (B, T, H, HN, K, V, nbs, float(scale), flags, st)
         if WALK_VSPLIT and tc_walk and NT <= 128 and not want_start:
             _lib.call("natsl_gdn_walk_fused_vsplit", *args, *dims)
         else:
-            _lib.call("natsl_gdn_walk_fused_ex" if tc_walk else "natsl_gdn_walk", *args, _lib.ptr(start),
+            entry = "natsl_gdn_split_walk" if split else "natsl_gdn_walk_fused_ex" if tc_walk else "natsl_gdn_walk"
+            _lib.call(entry, *args, _lib.ptr(start),
                       _lib.ptr(last_types if want_start else None), last_code, 2 * HN, *dims)
         return o, ht, inter
     if mamba_fused:

@@ -29,8 +29,8 @@ struct PrepSmem {
     static constexpr int ks = 0;
     static constexpr int vs = ks + 64 * K * 2;
     static constexpr int As = vs + 64 * V * 2;                 // fp32 [64][68]; the q tile is staged here first
-    static constexpr int as_bytes = 64 * K * 2 > 64 * A_LD * 4 ? 64 * K * 2 : 64 * A_LD * 4;
-    static constexpr int Xs = As + as_bytes;                   // fp32 [4][16][17]
+    static_assert(64 * K * 2 <= 64 * A_LD * 4, "the q tile is staged in the A buffer");
+    static constexpr int Xs = As + 64 * A_LD * 4;              // fp32 [4][16][17]
     static constexpr int Gs = Xs + 4 * 16 * X_LD * 4;          // bf16 [64][64] swizzled (128-byte rows)
     static constexpr int vec = Gs + 64 * 64 * 2;               // gcs, beta, rstd, wscale, q rstd: 5 x 64 floats
     static constexpr int total = vec + 5 * 64 * 4;
@@ -166,14 +166,12 @@ gdn_prep_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __rest
     // ---- q row norms (read only); v rows scaled by beta (in place).  k stays raw in shared memory: its row norms
     // are the diagonal of K K^T, and 1/norm enters A, P and the right-hand side of w as row / column scales.
     if (q) {
-        constexpr int CPR = K / 8;                             // 16-byte chunks of a row (at most 32)
-        constexpr int LPR = CPR <= 8 ? 8 : CPR <= 16 ? 16 : 32;    // lanes per row
-        constexpr int RPP = 32 / LPR;
-        const int sub = lane / LPR, cc = lane % LPR;
+        constexpr int CPR = K / 8;                             // 16-byte chunks and lanes of a row
+        constexpr int RPP = 32 / CPR;
+        const int sub = lane / CPR, cc = lane % CPR;
         for (int rr = 0; rr < 8; rr += RPP) {
             int r = warp * 8 + rr + sub;
-            uint4 xv = make_uint4(0, 0, 0, 0);
-            if (cc < CPR) xv = *reinterpret_cast<const uint4*>(qs_p + swz<K * 2>(r, cc));
+            const uint4 xv = *reinterpret_cast<const uint4*>(qs_p + swz<K * 2>(r, cc));
             const uint32_t* xw = reinterpret_cast<const uint32_t*>(&xv);
             float ss = 0.f;
 #pragma unroll
@@ -182,7 +180,7 @@ gdn_prep_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __rest
                 ss += t.x * t.x + t.y * t.y;
             }
 #pragma unroll
-            for (int o = LPR / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+            for (int o = CPR / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
             if (cc == 0) {
                 const float rs = use_l2norm ? rsqrtf(ss + 1e-6f) : 1.0f;
                 s_qr[r] = rs;
@@ -403,10 +401,8 @@ extern "C" int natsl_gdn_chunk_prep_ex(const void* q, const void* k, const void*
     NATSL_PREP_CASE(128, 64)
     NATSL_PREP_CASE(128, 128)
     NATSL_PREP_CASE(128, 256)
-    NATSL_PREP_CASE(192, 384)
 #undef NATSL_PREP_CASE
-    set_error("natsl_gdn_chunk_prep: unsupported head dims K=%d V=%d (64 / 64, 64 / 128, 128 / 64, 128 / 128, 128 / 256 or 192 / 384)",
-              K, V);
+    set_error("natsl_gdn_chunk_prep: unsupported head dims K=%d V=%d (64 / 64, 64 / 128, 128 / 64, 128 / 128 or 128 / 256)", K, V);
     return NATSL_ERR_UNSUPPORTED;
 }
 

@@ -1,4 +1,4 @@
-// Gated-delta-rule recurrence AND chunk output in one walk for any of the built head dims (K in {64, 128, 192}, value
+// Gated-delta-rule recurrence AND chunk output in one walk for any of the built head dims (K in {64, 128}, value
 // columns in slices of 32 or 64) and any nats_block_size: the counterpart of gdn_walk_tc.cu for shapes the tcgen05 kernel
 // has no tiles for, and for few (batch, head) pairs, where slices of the value dim are what fills the SMs.
 // One CTA per (batch, head, BV value columns) walks the 64-token chunks in order; per chunk c (S = state it reads):
@@ -11,8 +11,7 @@
 // What bounds it: the serial chain of a chunk (w S -> v' -> k^T v'' -> bf16 copy of S), so its products run as small
 // mma.sync steps of four warps (a tcgen05 round trip through TMEM costs more than these whole products), the output side
 // runs on four other warps, and TMA keeps the next chunk's tiles in flight.  Against the recurrence and
-// the output as two kernels the per-chunk states (K x V bf16 written and read) never leave the SM, and against the token
-// recurrence (the only kernel there was for K = 192) a step covers 64 tokens.
+// the output as two kernels the per-chunk states (K x V bf16 written and read) never leave the SM.
 #include "tc_common.cuh"
 #include "warp_gemm.cuh"
 #include "../../include/natsl_b200.h"
@@ -444,9 +443,8 @@ extern "C" int natsl_gdn_walk(const void* q, const void* k, const void* w, const
     if (V % 32 == 0 && V >= 64) {
         if (K == 64) { if (narrow) NATSL_GW(64, 32); else NATSL_GW(64, 64); }
         if (K == 128) { if (narrow) NATSL_GW(128, 32); else NATSL_GW(128, 64); }
-        if (K == 192) NATSL_GW(192, 32);
     }
 #undef NATSL_GW
-    set_error("natsl_gdn_walk: unsupported head dims K=%d V=%d (K in {64, 128, 192}, V a multiple of 32 from 64 on)", K, V);
+    set_error("natsl_gdn_walk: unsupported head dims K=%d V=%d (K in {64, 128}, V a multiple of 32 from 64 on)", K, V);
     return NATSL_ERR_UNSUPPORTED;
 }

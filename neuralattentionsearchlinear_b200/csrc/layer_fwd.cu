@@ -369,20 +369,23 @@ int stream_after(cudaStream_t waiter, cudaStream_t done, cudaEvent_t ev) {
 long up256(long x) { return (x + 255) / 256 * 256; }
 
 struct HybridLayout {
-    long w, u, p, gcs, kr, qr, total;
+    long w, u, p, gcs, kr, qr, egl, total;
 };
+// The delta rule with K = 192 runs natsl_gdn_split_prep and natsl_gdn_split_walk (gcs, kr, qr hold kf, qf, vf and p holds tp).
+bool split_rule(const natsl_hybrid_args& a) { return a.rule == NATSL_RULE_GDN && a.K == 192; }
 HybridLayout hybrid_layout(const natsl_hybrid_args& a) {
     HybridLayout l = {};
     const long n = (long)a.B * a.T * a.H;
-    const bool gdn = a.rule == NATSL_RULE_GDN;
+    const bool gdn = a.rule == NATSL_RULE_GDN, split = split_rule(a);
     if (a.options & NATSL_HYBRID_FP32) return l;
     l.gcs = 0;
     l.kr = up256(l.gcs + 4 * n);
     l.qr = up256(l.kr + (gdn ? 4 * n : 0));
-    l.w = up256(l.qr + (gdn ? 4 * n : 0));
-    l.u = up256(l.w + (gdn ? 2 * n * a.K : 0));
-    l.p = up256(l.u + (gdn ? 2 * n * a.V : 0));
-    l.total = up256(l.p + (gdn ? 2 * n * 64 : 0));
+    l.w = up256(l.qr + (split ? 8 * n : gdn ? 4 * n : 0));
+    l.u = up256(l.w + (gdn && !split ? 2 * n * a.K : 0));
+    l.p = up256(l.u + (gdn && !split ? 2 * n * a.V : 0));
+    l.egl = up256(l.p + (split ? 2 * n * 320 : gdn ? 2 * n * 64 : 0));
+    l.total = up256(l.egl + (split ? 4l * a.B * ((a.T + 63) / 64) * a.H : 0));
     return l;
 }
 
@@ -442,7 +445,12 @@ int hybrid_forward(const natsl_hybrid_args& a, void* types_raw, cudaStream_t st,
     }
     rc = stream_after(side, st, ev[0]);
     // the preparation reads no tables: it starts while they are built
-    if (rc == NATSL_OK && gdn) {
+    const bool split = split_rule(a);
+    if (rc == NATSL_OK && split) {
+        rc = natsl_gdn_split_prep(a.q, a.k, a.g, a.beta, a.beta_dtype, ws + l.p, gcs, reinterpret_cast<float*>(ws + l.kr),
+                                  reinterpret_cast<float*>(ws + l.qr), reinterpret_cast<float*>(ws + l.egl), a.B, a.T, a.H, a.K,
+                                  a.use_l2norm, lin);
+    } else if (rc == NATSL_OK && gdn) {
         auto prep = (a.K == 128 && a.V == 128 && !(a.options & NATSL_HYBRID_PREP_MMA)) ? natsl_gdn_chunk_prep_tc : natsl_gdn_chunk_prep_ex;
         rc = prep(a.q, a.k, a.v, a.g, a.beta, a.beta_dtype, ws + l.w, ws + l.u, gcs, reinterpret_cast<float*>(ws + l.kr),
                   reinterpret_cast<float*>(ws + l.qr), ws + l.p, a.B, a.T, a.H, a.K, a.V, a.use_l2norm, lin);
@@ -457,7 +465,11 @@ int hybrid_forward(const natsl_hybrid_args& a, void* types_raw, cudaStream_t st,
     const void* last = types_raw ? (const void*)(reinterpret_cast<bf16*>(types_raw) + (long)(TN - 1) * a.HN * 2) : a.last_types;
     const int last_dtype = types_raw ? NATSL_DT_BF16 : a.last_dtype;
     const bool tc_walk = gdn && a.K == 128 && a.V == 128 && a.nbs == 64 && a.T <= 65536 && !(a.options & NATSL_HYBRID_WALK_MMA);
-    if (rc == NATSL_OK && tc_walk && (a.options & NATSL_HYBRID_WALK_VSPLIT) && a.T <= 8192 && !a.hstart) {
+    if (rc == NATSL_OK && split) {
+        rc = natsl_gdn_split_walk(a.q, a.k, a.v, ws + l.p, gcs, reinterpret_cast<float*>(ws + l.kr), reinterpret_cast<float*>(ws + l.qr),
+                                  reinterpret_cast<float*>(ws + l.egl), a.types_i, a.indices, a.n_blocks, a.h0, a.o_lin, a.ht, a.hstart, last, last_dtype, a.last_stride, a.B,
+                                  a.T, a.H, a.HN, a.K, a.V, a.nbs, a.scale_lin, flags, lin);
+    } else if (rc == NATSL_OK && tc_walk && (a.options & NATSL_HYBRID_WALK_VSPLIT) && a.T <= 8192 && !a.hstart) {
         rc = natsl_gdn_walk_fused_vsplit(a.q, a.k, ws + l.w, ws + l.u, ws + l.p, gcs, reinterpret_cast<float*>(ws + l.kr),
                                          reinterpret_cast<float*>(ws + l.qr), a.types_i, a.indices, a.n_blocks, a.h0, a.o_lin, a.ht, a.B,
                                          a.T, a.H, a.HN, a.K, a.V, a.nbs, a.scale_lin, flags, lin);

@@ -92,3 +92,31 @@ def test_walk_of_more_than_2_31_outputs():
     want = _ops.linear_fwd(_lib.RULE_GDN, *tail, tb, K ** -0.5, None, True, True, True, return_intermediates=True)[0]
     assert_close(o[:, -n // 2:], want[:, -n // 2:].float(), TOL, "o")
     assert _lib.load().natsl_device_status() == 0
+
+
+@pytest.mark.parametrize("T,nbs,want", [(512, 64, False), (500, 64, True), (512, 256, True)])
+def test_760m_head_dims_keep_fp32(T, nbs, want):
+    """K = 192, V = 384 holds the state and its operands to fp32 precision between bf16 tensors: the output is off from float64 by
+    its one rounding to bf16 (2^-9 of an entry at most), the states by a few roundings to fp32 (2^-24 each).  Op and
+    chunk-inference op."""
+    import neuralattentionsearchlinear_b200 as nat
+    B, H, K, V = 1, 2, 192, 384
+    q, k, v, g, beta, h0 = synth_gdn_inputs(B, T, H, K, V, seed=T, normalize_qk=True)
+    raw = otab.synth_types(B, -(-T // nbs), H, 0.5, seed=nbs, force_last=False)
+    types = otab.force_last_block(raw.clone())
+    c = lambda x: x.cuda()
+    qa, ka, va = (c(x).view(B, T, 3 * H, -1) for x in (q, k, v))
+    args = (qa, ka, va, c(q), c(k), c(v), c(h0), c(g), c(beta), c(types))
+    opts = dict(nats_block_size=nbs, ops_for_incomplete_chunks="all", output_final_state_gated_delta=True, decay_for_non_gdn_blocks=True)
+    kw = dict(nbs=nbs, h0=h0.double(), decay=True, use_l2norm=True, rule="gdn", scale=K ** -0.5)
+    ref_in = (q.double(), k.double(), v.double(), g.double(), beta.double())
+    o_ref, fin_ref = ogdn.linear_recurrent(*ref_in, types[..., 1], **kw)
+    rel = lambda a, b: float((a.double().cpu() - b).norm() / b.norm())
+    if want:
+        o, _, ht, start = nat.nats_mixed_attn_gdn_chunk_inference(*args, c(raw[:, -1]) if T % nbs == 0 else None, None, **opts)
+        _, _, start_ref = ogdn.linear_recurrent(*ref_in, (raw if T % nbs == 0 else types)[..., 1], return_block_start=True, **kw)
+        assert rel(start, start_ref) <= 8 * 2.0 ** -24
+    else:
+        o, _, ht = nat.nats_mixed_attn_gdn(*args, None, **opts)
+    assert rel(o, o_ref) <= 2.0 ** -9
+    assert rel(ht, fin_ref) <= 8 * 2.0 ** -24
