@@ -107,3 +107,36 @@ def test_selection_equals_torch_hard_softmax_bit_for_bit():
         layer(x.view(B, TN * 64, 64), past_key_values=cache)
         want = hard_softmax(logits.view(B, TN, 1, 2))
     assert torch.equal(cache[0].block_types.float(), torch.round(want.float()))
+
+
+def test_silu_of_the_fused_convolution_rounds_like_the_separate_kernel():
+    """Convolutions of one tap pass the projection on, so that the layer's keys are silu(k_raw): against float64 rounded to bf16
+    they differ where the sigmoid's last fp32 bits flip a rounding, no more often than the convolution kernel's own
+    (2^-24 in front of a rounding to 2^-9: a few in 10^5)."""
+    import neuralattentionsearchlinear_b200 as nat
+    torch.manual_seed(5)
+    layer = _make("gdn", hidden=64, heads=4, head_dim=64, expand_v=1, attn_heads=4, attn_qk_norm=False).cuda().bfloat16().eval()
+    for conv in (layer.q_conv1d, layer.k_conv1d, layer.v_conv1d):
+        conv.weight.data.zero_()
+        conv.weight.data[..., 3] = 1
+    x = 40 * torch.randn(4, 4096, 64, generator=torch.Generator().manual_seed(0)).bfloat16().cuda()
+    cache = nat.NAtSCache()
+    with torch.no_grad():
+        layer(x, past_key_values=cache)
+        raw = layer.k_proj(x)
+        separate = layer.k_conv1d(raw)[0]
+        want = torch.nn.functional.silu(raw.double()).bfloat16()
+    fused = cache[0].k_attn.reshape(want.shape)
+    off = lambda t: int((t != want).sum())
+    assert off(fused) <= off(separate) + 2e-6 * want.numel(), (off(fused), off(separate), want.numel())
+    extreme = torch.tensor([0.0, -0.0, 88.0, -88.0, -200.0, 300.0, float("inf"), float("nan")])
+    x[0, :8] = 0
+    layer.k_proj.weight.data.zero_()
+    layer.k_proj.weight.data[:, 0] = 1
+    x[..., 0] = 0
+    x[0, :8, 0] = extreme.to(x)
+    with torch.no_grad():
+        cache = nat.NAtSCache()
+        layer(x, past_key_values=cache)
+        want = layer.k_conv1d(layer.k_proj(x))[0][0, :8]
+    assert torch.equal(torch.nan_to_num(cache[0].k_attn[0, :8].reshape(8, -1), 7.0), torch.nan_to_num(want, 7.0))
