@@ -1142,7 +1142,8 @@ extern "C" int natsl_linear_bwd_dh(int rule, const void* qn, const void* kn, con
 #define NATSL_ARGS qn, kn, w, d_o, dvl, gcs, carry, types_i, indices, n_blocks, dht, dS_all, dvp, dh0, B, T, H, HN, V, scale, st
     // slices of 64 value columns read q, k and w half as often; slices of 32 keep more SMs busy when there are few heads
     const bool wide = V % 64 == 0 && (long)B * H * (V / 64) >= 148;
-#define NATSL_DH(KK, GDN) return wide ? launch_dh<KK, 64, GDN>(NATSL_ARGS) : launch_dh<KK, 32, GDN>(NATSL_ARGS)
+    // beyond some 660 thousand tokens the per-chunk table leaves room for the narrow slices only
+#define NATSL_DH(KK, GDN) return wide && DhSmem<KK, 64, GDN>::total((T + 63) / 64) <= 227 * 1024 ? launch_dh<KK, 64, GDN>(NATSL_ARGS) : launch_dh<KK, 32, GDN>(NATSL_ARGS)
     if (rule == NATSL_RULE_GDN) {
         if (K == 64) NATSL_DH(64, true);
         if (K == 128) NATSL_DH(128, true);
