@@ -289,6 +289,8 @@ typedef struct natsl_hybrid_args {
 } natsl_hybrid_args;
 int64_t natsl_hybrid_workspace_bytes(const natsl_hybrid_args* args);
 int natsl_hybrid_forward(const natsl_hybrid_args* args, void* stream);
+/* Kernels that this thread's last natsl_hybrid_forward or natsl_layer_forward launched. */
+int natsl_call_kernels(void);
 
 /* A layer's forward between its projections and its output projection (no gradients): decays and betas, short convolutions
  * with both branches' norms, hard selection + tables, both branches, mixing weights, and the state a decoding cache keeps.

@@ -52,6 +52,7 @@ PROTOTYPES = {
     "natsl_linear_recurrent_fwd": [_i, _i, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _f, _i, _i, _p],
     "natsl_linear_recurrent_step": [_i, _i, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _f,
                                     _i, _i, _p],
+    "natsl_call_kernels": [],
     "natsl_hybrid_workspace_bytes": [_p],
     "natsl_hybrid_forward": [_p, _p],
     "natsl_layer_workspace_bytes": [_p],
@@ -148,11 +149,11 @@ def load() -> C.CDLL:
     return lib
 
 
-# kernels one successful call of an entry point launches (for launch accounting; entry points not listed launch one)
+# kernels one successful call of an entry point launches (for launch accounting; entry points not listed launch one).  The op's
+# and the layer's calls launch by rule, dtype and options: the library counts them.
 KERNELS_PER_CALL = {"natsl_build_tables": 2, "natsl_attn_bwd": 2, "natsl_gdn_fwd_noalloc": 3, "natsl_decode_step": 4,
-                    "natsl_hybrid_forward": 4, "natsl_layer_forward": 7,
-                    "natsl_abi_version": 0,
-                    "natsl_device_status": 0}
+                    "natsl_abi_version": 0, "natsl_device_status": 0}
+_COUNTED = {"natsl_hybrid_forward", "natsl_layer_forward"}
 _launches = 0
 
 
@@ -172,7 +173,7 @@ def call(name: str, *args) -> None:
     global _launches
     lib = load()
     status = getattr(lib, name)(*args)
-    _launches += KERNELS_PER_CALL.get(name, 1)
+    _launches += lib.natsl_call_kernels() if name in _COUNTED else KERNELS_PER_CALL.get(name, 1)
     if status != 0:
         raise NatslError(f"{name} failed with status {status}: {lib.natsl_last_error().decode()}")
     if CHECK_STATUS and name not in ("natsl_device_status", "natsl_abi_version", "natsl_bounded_wait_selftest"):

@@ -18,7 +18,12 @@ void set_error(const char* fmt, ...) {
     va_end(ap);
 }
 
+// Launches (each is followed by one check) of this thread since the start of its last counted call.
+static thread_local int g_launches = 0;
+void count_launches_from_here() { g_launches = 0; }
+
 int check_launch(const char* what) {
+    ++g_launches;
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         set_error("%s: CUDA error %d (%s)", what, (int)e, cudaGetErrorString(e));
@@ -47,5 +52,7 @@ int check_device(const void* p, const char* what) {
 }  // namespace natsl
 
 extern "C" const char* natsl_last_error(void) { return natsl::g_err; }
+
+extern "C" int natsl_call_kernels(void) { return natsl::g_launches; }
 
 extern "C" int natsl_abi_version(void) { return NATSL_B200_ABI_VERSION; }

@@ -14,6 +14,7 @@ namespace natsl {
 // ------------------------------------------------------------------ host-side errors
 void set_error(const char* fmt, ...);
 int check_launch(const char* what);
+void count_launches_from_here();                             // what natsl_call_kernels counts
 int check_device(const void* p, const char* what);      // p must be memory of the current device
 
 #define NATSL_REQUIRE(cond, code, ...)          \

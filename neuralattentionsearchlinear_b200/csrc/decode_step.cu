@@ -6,7 +6,7 @@
 // What bounds it: at batch 1 the layer reads its weights once (33 MB at hidden 1024..2048) and does almost no arithmetic,
 // so the floor is the weight read plus the dependent launches; issued step by step from Python (about 80 launches,
 // several host reads) the same token took 1.4 ms of host time.  A request of 777 + 48 tokens at hidden 2048, batch 1:
-// 69.0 -> 2.9 ms; 2048 + 32 tokens at hidden 1024, batch 32: 49.1 -> 5.5 ms (prefill included in both).
+// 70 -> 1.6 ms; 2048 + 32 tokens at hidden 1024, batch 32: 50 -> 4.2 ms (prefill included in both).
 //   * proj / out: "skinny" products y[b, n] = x[b, :] . W[n, :].  The weight rows are the M side of mma.m16n8k16, the
 //     batch the N side, so a weight element is loaded once, straight from global memory into the A fragment: with the k
 //     index permuted inside every 32-wide group a lane's fragment is one 16-byte load per row (the same permutation on

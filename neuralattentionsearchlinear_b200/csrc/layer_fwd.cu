@@ -512,6 +512,7 @@ extern "C" int natsl_hybrid_forward(const natsl_hybrid_args* args, void* stream)
     using namespace natsl;
     NATSL_REQUIRE(args, NATSL_ERR_NULL, "natsl_hybrid_forward: null argument block");
     NATSL_REQUIRE(args->types_dtype >= 0 && args->types_dtype <= NATSL_DT_I32, NATSL_ERR_UNSUPPORTED, "natsl_hybrid_forward: bad types dtype");
+    count_launches_from_here();
     int rc = check_hybrid(*args);
     if (rc == NATSL_OK) rc = check_device(args->q, "natsl_hybrid_forward");
     if (rc != NATSL_OK) return rc;
@@ -522,7 +523,7 @@ namespace natsl {
 namespace {
 
 struct LayerLayout {
-    long q, k, v, qa, ka, qc, vc, g, beta, dt, hybrid, total;
+    long q, k, v, qa, qc, g, beta, dt, hybrid, total;
 };
 // Intermediates of a layer's forward.  Tensors the caller keeps (k_attn, v_attn) are outputs and not listed here.
 LayerLayout layer_layout(const natsl_layer_args& a, const natsl_hybrid_args& h) {
@@ -535,9 +536,7 @@ LayerLayout layer_layout(const natsl_layer_args& a, const natsl_hybrid_args& h) 
     take(l.k, 2 * n * HK);
     take(l.v, mamba ? 2 * n * HV : 0);
     take(l.qa, a.qn_w || (mamba && a.attn_conv) ? 2 * n * HK : 0);
-    take(l.ka, 0);
     take(l.qc, mamba ? 2 * n * HK : 0);
-    take(l.vc, 0);
     take(l.g, 4 * n * a.H);
     take(l.beta, mamba ? 0 : 2 * n * a.H);
     take(l.dt, mamba ? 8 * n * a.H : 0);
@@ -588,7 +587,7 @@ extern "C" int natsl_layer_forward(const natsl_layer_args* args, void* stream) {
     unsigned char* ws = reinterpret_cast<unsigned char*>(a.workspace);
     auto cb = [](const void* p) { return reinterpret_cast<const bf16*>(p); };
     auto mb = [](void* p) { return reinterpret_cast<bf16*>(p); };
-    const int HK = a.H * a.K, HV = a.H * a.V, TN = (a.T + a.nbs - 1) / a.nbs, NT = (a.T + 63) / 64;
+    const int HK = a.H * a.K, HV = a.H * a.V, TN = (a.T + a.nbs - 1) / a.nbs;
 
     NarrowArgs n = {};
     n.x = cb(a.x); n.w0 = cb(a.w_a); n.w1 = mamba ? nullptr : cb(a.w_b);
@@ -598,6 +597,7 @@ extern "C" int natsl_layer_forward(const natsl_layer_args* args, void* stream) {
     n.dt = mamba ? reinterpret_cast<float*>(ws + l.dt) : nullptr;
     n.gcs = mamba ? n.dt + (long)a.B * a.T * a.H : nullptr;
     n.out = mb(ws + l.beta);
+    count_launches_from_here();
     int rc = check_device(a.x, "natsl_layer_forward");
     if (rc == NATSL_OK) rc = launch_narrow(n, a.B, st);
     if (rc != NATSL_OK) return rc;
@@ -670,7 +670,6 @@ extern "C" int natsl_layer_forward(const natsl_layer_args* args, void* stream) {
     const long nt = (long)a.B * TN * a.HN * 2;
     h.types_i = tb; h.indices = tb + nt; h.n_blocks = tb + 2 * nt; h.n_chunks_lin = h.n_blocks + 2l * a.B * a.HN;
     h.attn_n_iters = h.n_chunks_lin + (long)a.B * a.HN;
-    (void)NT;
     h.workspace = ws + l.hybrid;
     h.workspace_bytes = a.workspace_bytes - l.hybrid;
     rc = check_hybrid(h);

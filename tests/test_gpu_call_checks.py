@@ -594,3 +594,21 @@ def test_priority_switch_moves_the_linear_branch(nat, what, monkeypatch):
         assert caller is not None and stream["attn" if high else linear] == {caller}, stream
         assert caller not in stream[linear if high else "attn"], stream
     assert torch.equal(*outs)
+
+
+@pytest.mark.parametrize("what", ["gdn op", "mamba op", "fp32 op", "layer", "layer with cache", "mamba layer"])
+def test_launch_accounting(nat, what):
+    """kernel_launches() grows by the kernels of this library that a call runs."""
+    from neuralattentionsearchlinear_b200 import _lib
+    if "layer" in what:
+        layer, x = make_layer(nat, "mamba" if "mamba" in what else "gdn"), tokens(2, 300)
+        fn = lambda: call(layer, x, nat.NAtSCache() if "cache" in what else None)
+    else:
+        rule, K = ("mamba", 128) if what == "mamba op" else ("gdn", 64)
+        args, types, _ = op_inputs(rule, 2, 300, 2, K, 64, 64, dtype=torch.float32 if what == "fp32 op" else torch.bfloat16)
+        fn = lambda: op_call(nat, rule)(args, types)
+    with torch.no_grad():
+        ran = [n for n in kernels_of(fn) if "natsl::" in n]
+        before = _lib.kernel_launches()
+        fn()
+    assert _lib.kernel_launches() - before == len(ran), ran
