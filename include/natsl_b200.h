@@ -37,7 +37,7 @@ extern "C" {
 #define NATSL_FLAG_ATTN_OWN_CHUNK 2     /* softmax branch also covers the query's own block ('all', 'attn') */
 #define NATSL_FLAG_NO_TRAILING_QUIRK 4  /* carry the decay also over skipped blocks after the last selected one */
 #define NATSL_FLAG_ATTN_MMA_SYNC 8      /* natsl_attn_fwd: use the mma.sync comparison kernel instead of tcgen05 */
-#define NATSL_FLAG_ATTN_PERSISTENT 32   /* natsl_attn_fwd*: two resident CTAs per SM work through the query tiles (measured slower; off by default) */
+#define NATSL_FLAG_ATTN_PERSISTENT 32   /* natsl_attn_fwd*: accepted, without effect: the kernel is persistent */
 #define NATSL_FLAG_BWD_REFERENCE_COMPAT 16 /* natsl_attn_bwd: drop the own-block terms, as the reference's default backward does */
 
 #define NATSL_ATTN_BT 128 /* query rows per attention tile; the attn_n_iters table is built for it */
@@ -265,7 +265,7 @@ int natsl_attn_fwd_fp32(int dtype, const void* q, const void* k, const void* v, 
  * be NULL; without the compact list).  ht, hstart, h0, last_types may be NULL. */
 #define NATSL_HYBRID_PREP_MMA 1        /* mma.sync chunk preparation also where the tcgen05 one is built */
 #define NATSL_HYBRID_WALK_MMA 2        /* mma.sync walk also where the tcgen05 one is built (few (batch, head) pairs) */
-#define NATSL_HYBRID_ATTN_PERSISTENT 4
+#define NATSL_HYBRID_ATTN_PERSISTENT 4 /* accepted, without effect */
 #define NATSL_HYBRID_FP32 8            /* fp32 tensors: natsl_linear_recurrent_fwd and natsl_attn_fwd_fp32 side by side (no workspace) */
 #define NATSL_HYBRID_WALK_VSPLIT 32    /* natsl_gdn_walk_fused_vsplit in place of the one-CTA tcgen05 walk where it is built (no hstart) */
 #define NATSL_HYBRID_PLAIN_PRIORITY 64 /* linear branch on `stream`, the other one on a side stream of normal priority */

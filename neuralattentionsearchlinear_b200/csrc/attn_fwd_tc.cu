@@ -1,25 +1,39 @@
 // Chunk-masked softmax attention forward on the 5th-generation tensor cores.
 //
-// One CTA = 128 queries of one softmax head; two CTAs share an SM (2 x 256 TMEM columns,
-// 2 x ~113 KB shared memory).  Warp roles (320 threads):
-//   warp 0    TMA producer: Q once, then the K and V tiles of the key-tile walk into a 3- or 4-stage and a
-//             2-stage ring (cp.async.bulk.tensor, 128-byte swizzle, zero fill past the sequence end), in the
-//             order in which the tensor core frees the stages;
-//   warp 1    MMA issuer (one elected lane): S_j = Q K_j^T into one of two (DV = 128) or three (DV = 64) TMEM score
-//             buffers, issued that many tiles ahead, and O += P_j V_j with P read straight from TMEM;
-//             completion is signalled with tcgen05.commit on mbarriers;
-//   warps 2-9 softmax, 16 query rows per warp, four threads per row (tcgen05.ld.16x256b fragments):
-//             mask, online softmax in base 2 with a lazily updated maximum (O in TMEM is only
-//             rescaled when the running maximum grows by more than 2^8), P (bf16 pairs) written back
-//             with tcgen05.st over the score buffer it came from; at the end O / l -> bf16 -> shared
-//             memory -> coalesced global stores.
-// While the softmax warps work on tile j the tensor core runs Q K_{j+1}^T and P_{j-1} V_{j-1}.
-// The key-tile list (load coordinate, gathered bit) is computed by the producer warp, its only reader; the other
-// roles need just the tile count, and the softmax warps the selection bits of the blocks under the own span.
-// Same key-tile walk, mask and output conventions as the mma.sync kernel (attn_walk.cuh):
-// src/nats/ops/attns/attns.py:62-353 is the reference kernel this replaces.
-// Every mbarrier wait has an iteration limit; on expiry the CTA records a status, stops issuing
-// work, still frees its TMEM and returns.
+// One work item = 256 queries of one softmax head: two tiles A and B of 128 rows that share every key and value load.
+// One CTA per SM works through items until none is left: it takes over blocks of the grid that have not started yet
+// (cluster launch control), so the pipeline runs across items, an SM is never idle between two of them, and a kernel
+// of higher priority still gets its SMs (the take-over is refused then and the CTA ends).  Roles (384 threads):
+//   warps 0-3  softmax of tile A, one thread per query row (tcgen05.ld.32x32b: 128 scores of the row in registers, no
+//              shuffles): mask, online softmax in base 2 with a lazily updated maximum (O in TMEM is only rescaled when
+//              a row's maximum grows by more than 2^8), P (bf16 pairs) into TMEM; at the end of an item
+//              O / l -> bf16 -> global memory, whole 32-byte sectors per thread;
+//   warps 4-7  the same for tile B;
+//   warp 8     TMA producer: the two query tiles of an item, then pairs of 64-key tiles into a K and a V ring
+//              (cp.async.bulk.tensor, 128-byte swizzle, zero fill past the sequence end);
+//   warps 9, 11  MMA issuers of tile A and tile B: S = Q K^T (128 x 128), O += P V with P read straight from TMEM;
+//   warp 10    scheduler: takes the next item, reads its tables, works out its steps.
+// TMEM (512 columns): S of A and of B (128 columns each), O of A and of B, and, where DV = 64 leaves room, P of A and of B.
+//
+// What bounds it: at head dims 128 the tensor core and the exponentials need the same 1024 cycles per 128 x 128 tile; two
+// tiles in flight hide one behind the other.  Measured cycles per tile: 1.6 k (DK = 128, DV = 64, long lists), of which the
+// exponential unit is busy 63 %.  128-key score tiles halve the number of dependent steps of 64-key ones, and shared loads
+// halve the L2 traffic of one-tile CTAs.  What it took beyond that: no code that does not have to be there (with every wait
+// and every planning loop unrolled in place the kernel was 110 KB, missed the instruction cache and was 1.5 x slower than at
+// 50 KB), descriptors that differ by constants, and items handed out heaviest first (see Order).
+//   B = 8, T = 4096, H = 16, 128/128, 25 % selected:   260 -> 189 us (553 -> 762 TFLOP/s); 50 %: 395 -> 306 us (915 TFLOP/s)
+//   B = 1, T = 65536, H = 32, 128/64, 10 % selected:  3640 -> 2960 us (750 -> 920 TFLOP/s)
+//   B = 16, T = 4096, H = 16, 64/64, 50 % selected:    700 -> 509 us; B = 32, T = 2048: 450 -> 288 us
+// (before: one 128-query tile and 64-key steps per CTA, two CTAs per SM.)  Tried and not kept: sixteen softmax warps with half
+// a row each (207 us in the first case: the halves' maxima have to meet), the exponential unit lent to one warp at a time
+// (no change), a single issuing warp for both tiles (each waits for the other's softmax).
+//
+// Key walk, mask and output conventions as in the mma.sync kernel (attn_walk.cuh): own span first, then the selected past
+// blocks; src/nats/ops/attns/attns.py:62-353 is the reference kernel this replaces.
+// Every mbarrier wait has an iteration limit; on expiry the CTA stops issuing work, waits (again with a limit) for its own
+// copies in flight, records a status, frees its TMEM and returns.
+#include <algorithm>
+
 #include "attn_tc.cuh"
 #include "../../include/natsl_b200.h"
 
@@ -29,22 +43,150 @@ int attn_fwd_mma_sync(const void* q, const void* k, const void* v, const int32_t
                       const int32_t* attn_n_iters, void* o, float* lse, int B, int T, int HQ, int HKV, int HN, int DK,
                       int DV, int nbs, float scale, int own, cudaStream_t st);
 
-// persistent form (attn_fwd_tc_persist.cu), selected by NATSL_FLAG_ATTN_PERSISTENT
-template <int DK, int DV>
-int launch_attn_tc_persist(const void* q, const void* k_rem, const void* v_rem, const void* k, const void* v,
-                           const int* rem_base, int rem_slots, int rem_tokens, const int* types_i, const int* indices,
-                           const int* n_iters, void* o, float* lse, int B, int B_rem, int T, int Tq, int q_off, int k_split,
-                           int HQ, int HKV, int HN, int nbs, float scale, int own_chunk, cudaStream_t st);
+namespace {
+
+constexpr int AT_THREADS = 384;
+constexpr int AT_ITEM = 2 * ATT_BM;                  // queries of a work item
+constexpr int AT_SMS = 148;
+constexpr float LAZY_RESCALE_LOG2 = 8.0f;
+constexpr long AT_GROUP_BYTES = 64 << 20;            // keys and values of the heads whose items are mixed: half of L2
+constexpr uint32_t AT_O_COL = 256;
+constexpr int AT_CHUNK = 8, AT_CHUNKS = 4;           // steps are handed over in chunks (an item's last one may be shorter)
+
+// K and V ring stages of 128 keys.  Three K and two V stages are the least that the issue order needs (the tiles of an item
+// may be a pair apart); smaller head dims take what hides more of the load latency.
+template <int DK, int DV> struct AtSmem {
+    // How far the scores run ahead of the products P V.  With DV = 64 the probabilities have columns of their own, so a
+    // tile's next scores are issued as soon as its softmax holds the last ones in registers (2: the softmax never waits);
+    // with DV = 128 tensor memory is full, P lies over its scores and the next ones come behind P V (1).
+    static constexpr int LEAD = DV == 64 ? 2 : 1;
+    static constexpr int KST = DK == 64 ? 4 : 3;
+    static constexpr int VST = DV == 64 ? 4 : DK == 64 ? 3 : 2;
+    static constexpr int q = 0;                                  // tile A, tile B: DK/64 sub-tiles [128][64] each
+    static constexpr int k = q + 2 * 128 * DK * 2;               // KST stages x DK/64 sub-tiles [128][64]
+    static constexpr int v = k + KST * 128 * DK * 2;             // VST stages x DV/64 sub-tiles [128][64]
+    static constexpr int bars = v + VST * 128 * DV * 2;
+    static constexpr int items = bars + 384;                     // two slots of 8 ints
+    static constexpr int steps = items + 64;                     // AT_CHUNKS x AT_CHUNK steps of 8 ints
+    static constexpr int clc = steps + AT_CHUNKS * AT_CHUNK * 32;   // 16-byte answer of the take-over request
+    static constexpr int tmem = clc + 16;
+    static constexpr int total = tmem + 16;
+    static_assert(total <= 232448, "shared memory of one SM");
+};
+
+// Cluster launch control: ask for a block of this grid that has not started; the 16-byte answer lands in shared memory.
+__device__ __forceinline__ void request_block(uint32_t dst, uint32_t bar) {
+    asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
+                 ::"r"(dst), "r"(bar) : "memory");
+}
+__device__ __forceinline__ bool taken_block(uint32_t src, int& x) {
+    uint32_t ok, rx;
+    asm volatile(
+        "{\n .reg .pred p;\n .reg .b128 r;\n .reg .b32 y, z, w;\n ld.shared.b128 r, [%2];\n"
+        " clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n selp.u32 %0, 1, 0, p;\n mov.u32 %1, 0;\n"
+        " @p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%1, y, z, w}, r;\n}\n"
+        : "=&r"(ok), "=&r"(rx)
+        : "r"(src)
+        : "memory");
+    x = (int)rx;
+    return ok != 0;
+}
+
+// Where the gathered part of the key sequence lives (keys below k_split; see the kernel's comment).
+struct RemoteKeys {
+    int k_split;          // keys [0, k_split) are gathered keys
+    const int* base;      // first pair of (segment g, this head): base[g * stride], or nullptr for the head-major layout
+    int stride;
+    int slots;            // virtual blocks per head and gathered segment
+};
+
+// Which work item a block is.  Heads in groups whose keys and values stay in L2; in a group the items with the most keys
+// first, over all its heads, so that the last items of a group, and with them of the grid, are the lightest.  (Head by head
+// the SMs of a 16384-token call ended between 124 and 232 us.)
+struct Order {
+    uint32_t n_blocks, n_heads, group, split;            // blocks per head, heads over all batches, heads of a group, see below
+    uint32_t q_per_kv, q_per_sel, rem_segments;          // query heads of a key head, of a selection head; gathered segments
+};
+// q0: first query of the item.  With split a block is one tile of an item: only = 1 tile A, 2 tile B (0: both).  The tile goes
+// through the same keys in the same order as beside the other one, so its results do not depend on the split.
+__device__ __forceinline__ void locate(const Order& od, int block, int HQ, int q_off, int& q0, int& only, int& hq, int& b) {
+    const uint32_t grp = (uint32_t)block / (od.group * od.n_blocks), rest = block - grp * od.group * od.n_blocks;
+    const uint32_t width = min(od.group, od.n_heads - grp * od.group), level = rest / width;
+    const uint32_t head = grp * od.group + rest - level * width, i = od.n_blocks - 1 - level;
+    b = (int)(head / (uint32_t)HQ);
+    hq = (int)head - b * HQ;
+    only = od.split ? 1 + (int)(i & 1) : 0;
+    q0 = q_off + (int)(od.split ? i >> 1 : i) * AT_ITEM;
+}
+
+// One work item and the order in which its pairs of 64-key units are used.  Units 0 .. n_span-1 are the own span
+// (masked), the rest the selected past blocks; pair j = units 2j, 2j+1.  Tile A takes the pairs [0, end_a) and
+// [next_a, n_pairs): the pairs between them hold only keys behind A's rows.  Tile B takes [first_b, n_pairs): pair 0 is
+// left out if no row of B sees it.  Step i of an item = the i-th pair of A and the i-th pair of B (at most one pair apart).
+struct Item {
+    int q0, span_start, n_span, n_units, n_pairs, end_a, next_a, first_b, sel;
+    bool has_b, use_a, use_b;                            // the item has a tile B; the tiles this block works on
+};
+
+// selection block of span unit u, relative to the first one of the span (a span touches at most four)
+__device__ __forceinline__ int span_block(int u, int cpb) { return (u >= cpb) + (u >= 2 * cpb) + (u >= 3 * cpb); }
+// Whether the 32 rows of warp w of tile x see the 32-key chunk c of pair j (attn_walk.cuh: visible(); everything in it but
+// s <= t is the same for 32 aligned rows and 32 aligned keys, and rows past the end are not stored).
+__device__ __forceinline__ bool chunk_seen(const Item& t, int x, int w, int j, int c, int cpb, int nbs, int own_chunk) {
+    const int u = 2 * j + (c >> 1), row = t.q0 + x * ATT_BM + 32 * w;
+    if (u >= t.n_span) return u < t.n_units;
+    const int rb = span_block(u, cpb), blk_end = t.span_start + (rb + 1) * nbs;
+    const bool selb = (t.sel >> rb) & 1;
+    return own_chunk ? t.span_start + u * ATT_BN + 32 * (c & 1) <= row && (selb || row < blk_end) : selb && row >= blk_end;
+}
+// (the whole warp)  Bit 4w + c: chunk c of tile A's pair ja is seen by its warp w; the upper half the same for tile B and jb.
+__device__ __forceinline__ uint32_t seen_chunks(const Item& t, int ja, int jb, int lane, int cpb, int nbs, int own_chunk) {
+    const int x = lane >> 4;
+    return __ballot_sync(0xffffffffu, chunk_seen(t, x, (lane >> 2) & 3, x ? jb : ja, lane & 3, cpb, nbs, own_chunk));
+}
+__device__ __forceinline__ int span_units(int q0, int span_start, bool has_b, int T) {
+    return (min(q0 + (has_b ? AT_ITEM : ATT_BM), T) - span_start + ATT_BN - 1) / ATT_BN;
+}
+__device__ __forceinline__ Item make_item(int q0, int span_start, int n_past_blocks, int sel, int T, int q_end, int only,
+                                          int nbs, int own_chunk, int lane) {
+    Item t;
+    const int cpb = nbs / ATT_BN;
+    t.q0 = q0;
+    t.sel = sel;
+    t.has_b = q0 + ATT_BM < q_end;
+    t.use_a = only != 2;
+    t.use_b = t.has_b && only != 1;
+    t.span_start = span_start;
+    t.n_span = span_units(q0, span_start, t.has_b, T);
+    t.n_units = t.n_span + n_past_blocks * cpb;
+    t.n_pairs = (t.n_units + 1) >> 1;
+    const int a_units = min((q0 + ATT_BM - span_start) / ATT_BN, t.n_span);
+    t.end_a = (a_units + 1) >> 1;
+    t.next_a = max(t.end_a, t.n_units > t.n_span ? t.n_span >> 1 : t.n_pairs);
+    t.first_b = t.has_b && own_chunk && (seen_chunks(t, 0, 0, lane, cpb, nbs, 1) >> 16) == 0;
+    return t;
+}
+__device__ __forceinline__ bool uses_a(const Item& t, int j) { return t.use_a && (j < t.end_a || j >= t.next_a); }
+__device__ __forceinline__ bool uses_b(const Item& t, int j) { return t.use_b && j >= t.first_b; }
+
+// What one tile does in a step: flags, ring stages and phases of its pair, as one word.
+enum : uint32_t {
+    ST_VALID = 1, ST_USE0 = 2, ST_USE1 = 4,              // the tile takes part; some row sees the first / second unit
+    ST_FIRST = 8, ST_LAST = 16,                          // first / last pair of the item
+    ST_ALONE = 32, ST_TWO = 64,                          // the other tile does not use the pair; the second unit is loaded
+    ST_K = 8, ST_KPAR = 10, ST_V = 11, ST_VPAR = 13,     // shifts: K stage, its phase parity, V stage, its phase parity
+    ST_CHUNK_LAST = 1u << 14, ST_STOP = 1u << 15,        // (word of tile A)
+};
 
 template <int DK, int DV>
-__global__ void __launch_bounds__(TC_THREADS, 2)
+__global__ void __launch_bounds__(AT_THREADS, 1)
 attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                    const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_kr,
                    const __grid_constant__ CUtensorMap map_vr, int k_split, int B_rem, const int* __restrict__ rem_base,
-                   int rem_slots, const int* __restrict__ types_i,
-                   const int* __restrict__ indices, const int* __restrict__ attn_n_iters,
-                   __nv_bfloat16* __restrict__ o, float* __restrict__ lse, int T, int Tq, int q_off, int HQ, int HKV,
-                   int HN, int TN, int nbs, float scale_log2, int own_chunk, int* status) {
+                   int rem_slots, const int* __restrict__ types_i, const int* __restrict__ indices,
+                   const int* __restrict__ attn_n_iters, __nv_bfloat16* __restrict__ o, float* __restrict__ lse, int T,
+                   int Tq, int q_off, int HQ, int HKV, int HN, int TN, int nbs, float scale_log2, int own_chunk,
+                   const Order od, int* status) {
     // T = number of keys (and the length the tables were built for); the Tq queries are the tokens
     // [q_off, q_off + Tq) of that sequence (q_off = 0, Tq = T except under sequence parallelism).
     // Keys [0, k_split) live in a second pair of tensors (map_kr / map_vr, batch index b % B_rem: the
@@ -52,401 +194,576 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     // With rem_base the gathered tensors are [B_rem, tokens, 1, D]: the selected (block, head) pairs of every
     // gathered segment packed back to back; virtual block g * rem_slots + j of head hkv is pair
     // rem_base[(b % B_rem, g, hkv)] + j.
-    using L = TcSmem<DK, DV>;
+    using L = AtSmem<DK, DV>;
+    constexpr int KST = L::KST, VST = L::VST, LEAD = L::LEAD;
+    constexpr uint32_t P_COL = LEAD == 1 ? 0 : 384, P_STRIDE = LEAD == 1 ? 128 : 64;
     extern __shared__ __align__(1024) unsigned char smem[];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const uint32_t sbase = smem_u32(smem);
     if ((sbase & 1023u) != 0) {                       // swizzled tiles need 1024-byte alignment
         if (tid == 0) atomicExch(status, 2);
         return;
     }
-    const int NTq = (T + ATT_BM - 1) / ATT_BM;
-    const int it = q_off / ATT_BM + ((int)gridDim.x - 1 - (int)blockIdx.x);     // heaviest tiles first
-    const int hq = blockIdx.y, b = blockIdx.z;
-    const int hkv = hq / (HQ / HKV), hn = hq / (HQ / HN);
-    const int q0 = it * ATT_BM;
-    const int* idx = indices + ((long)b * TN * HN + hn) * 2;
-    const int* selp = types_i + ((long)b * TN * HN + hn) * 2;
-    const long tstride = (long)HN * 2;
-    const uint32_t s_q = sbase + L::q, s_k = sbase + L::k, s_v = sbase + L::v;
-    int* tile_list = reinterpret_cast<int*>(smem + L::list);
+    const uint32_t s_q = sbase + L::q, s_k = sbase + L::k, s_v = sbase + L::v, s_clc = sbase + L::clc;
+    volatile int* items = reinterpret_cast<volatile int*>(smem + L::items);
+    int4* steps = reinterpret_cast<int4*>(smem + L::steps);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::tmem);
     const uint32_t bar0 = sbase + L::bars;
     // barrier slots (8 bytes each)
-    const uint32_t bar_q = bar0, bar_k_full = bar0 + 8, bar_k_empty = bar0 + 40, bar_v_full = bar0 + 72,
-                   bar_v_empty = bar0 + 104, bar_s_full = bar0 + 136, bar_p_full = bar0 + 160, bar_pv = bar0 + 184;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::bars + 208);
-    constexpr int NSB = TcTmem<DV>::NSB, TC_KST = TcTmem<DV>::KST;
-    constexpr uint32_t TC_O_COL = TcTmem<DV>::o_col;
-
-    // requested before anything else; first used after the barrier below
-    const int n_past_blocks = __ldg(attn_n_iters + ((long)b * NTq + it) * HN + hn);
-    if (tid == 0) {
-        mbar_init(bar_q, 1);
+    const uint32_t bar_k_full = bar0, bar_k_empty = bar0 + 32, bar_v_full = bar0 + 64, bar_v_empty = bar0 + 96,
+                   bar_q_full = bar0 + 128, bar_q_empty = bar0 + 144, bar_s = bar0 + 160, bar_s_free = bar0 + 176,
+                   bar_p = bar0 + 192, bar_o = bar0 + 224, bar_item = bar0 + 240, bar_item_empty = bar0 + 256,
+                   bar_clc = bar0 + 272, bar_steps = bar0 + 280, bar_steps_empty = bar0 + 312;
+    static_assert(AT_CHUNKS == 4 && KST <= 4 && VST <= 4, "barrier slots");
+    const int cpb = nbs / ATT_BN, q_end = q_off + Tq;
+    if (tid == 256) {
         for (int i = 0; i < 4; ++i) {
             mbar_init(bar_k_full + 8 * i, 1);
-            mbar_init(bar_k_empty + 8 * i, 1);
+            mbar_init(bar_k_empty + 8 * i, 2);           // one arrival per tile (two of the only one that uses the pair)
             mbar_init(bar_v_full + 8 * i, 1);
-            mbar_init(bar_v_empty + 8 * i, 1);
+            mbar_init(bar_v_empty + 8 * i, 2);
+            mbar_init(bar_p + 8 * i, 4);                 // (tile, half): one arrival per softmax warp
+            mbar_init(bar_steps + 8 * i, 1);
+            mbar_init(bar_steps_empty + 8 * i, 10);      // eight softmax warps and two issuers are through with the chunk
         }
-        for (int i = 0; i < NSB; ++i) {
-            mbar_init(bar_s_full + 8 * i, 1);
-            mbar_init(bar_p_full + 8 * i, 8);            // one arrival per softmax warp
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(bar_item + 8 * i, 1);
+            mbar_init(bar_item_empty + 8 * i, 1);
+            mbar_init(bar_q_full + 8 * i, 1);
+            mbar_init(bar_q_empty + 8 * i, 1);
+            mbar_init(bar_s + 8 * i, 1);
+            mbar_init(bar_s_free + 8 * i, 4);
+            mbar_init(bar_o + 8 * i, 1);
         }
-        mbar_init(bar_pv, 1);
-        mbar_init(bar_pv + 8, 1);
+        mbar_init(bar_clc, 1);
         mbar_fence_init();
-        // the query tile and the first own-span key / value tiles depend on no table: their loads start at once
         prefetch_tensormap(&map_q);
-        mbar_expect_tx(bar_q, 128 * DK * 2);
-#pragma unroll
-        for (int sub = 0; sub < DK / 64; ++sub) tma_load_4d(s_q + sub * 16384, &map_q, sub * 64, hq, q0 - q_off, b, bar_q);
-        const TileWalk w0 = make_walk(q0, T, nbs, 0);
-        const int hkv0 = hq / (HQ / HKV);
-        for (int j = 0; j < min(w0.n_span, TcTmem<DV>::KST); ++j) {
-            mbar_expect_tx(bar_k_full + j * 8, 64 * DK * 2);
-#pragma unroll
-            for (int sub = 0; sub < DK / 64; ++sub)
-                tma_load_4d(s_k + j * (64 * DK * 2) + sub * 8192, &map_k, sub * 64, hkv0, w0.span_start + j * ATT_BN - k_split, b,
-                            bar_k_full + j * 8);
-        }
-        for (int j = 0; j < min(w0.n_span, TC_VST); ++j) {
-            mbar_expect_tx(bar_v_full + j * 8, 64 * DV * 2);
-#pragma unroll
-            for (int sub = 0; sub < DV / 64; ++sub)
-                tma_load_4d(s_v + j * (64 * DV * 2) + sub * 8192, &map_v, sub * 64, hkv0, w0.span_start + j * ATT_BN - k_split, b,
-                            bar_v_full + j * 8);
+        prefetch_tensormap(&map_k);
+        prefetch_tensormap(&map_v);
+        if (k_split > 0) {
+            prefetch_tensormap(&map_kr);
+            prefetch_tensormap(&map_vr);
         }
     }
-    if (warp == 1) tmem_alloc(smem_u32(tmem_slot), TC_TMEM_COLS);
-    // Nothing above waits for global memory: the barrier that publishes the mbarriers and the TMEM address comes
-    // before any table is read.  Each role then fetches what it needs by itself: every warp the tile count; the
-    // producer the tile list (it is the only reader of the index table); the softmax warps the selection bits of the
-    // one or two blocks that the own span touches.
+    if (warp == 9) tmem_alloc(smem_u32(tmem_slot), 512);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
-    const TileWalk walk = make_walk(q0, T, nbs, n_past_blocks);
-    const int n_tiles = walk.n_tiles;
-    const int b_rem = b % B_rem;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    bool ok = true;
 
-    if (warp == 0) {
-        // ------------------------------------------------------------ TMA producer
-        if (lane == 0) {
-            prefetch_tensormap(&map_k);
-            prefetch_tensormap(&map_v);
-            if (k_split > 0) {
-                prefetch_tensormap(&map_kr);
-                prefetch_tensormap(&map_vr);
-            }
-        }
-        RemoteKeys rk;
-        rk.k_split = k_split;
-        rk.slots = rem_slots;
-        rk.stride = HKV;
-        rk.base = rem_base ? rem_base + ((long)b_rem * (k_split / (rem_slots * nbs))) * HKV + hkv : nullptr;
-        for (int j = lane; j < min(n_tiles, TC_LIST_CAP); j += 32)
-            tile_list[j] = pack_tile(walk, j, idx, selp, tstride, nbs, rk);
-        __syncwarp();
-        auto tile_desc = [&](int j) -> int {
-            return j < TC_LIST_CAP ? tile_list[j] : pack_tile(walk, j, idx, selp, tstride, nbs, rk);
-        };
-        const int rem_head = rem_base ? 0 : hkv;     // packed pairs have no head axis
-        auto load_k = [&](int j) {                    // lane 0 only
-            const int td = tile_desc(j), stg = j % TC_KST;
-            const bool rem = (td >> 29) & 1;
-            const uint32_t full = bar_k_full + stg * 8;
-            mbar_expect_tx(full, 64 * DK * 2);
-#pragma unroll
-            for (int sub = 0; sub < DK / 64; ++sub)
-                tma_load_4d(s_k + stg * (64 * DK * 2) + sub * 8192, rem ? &map_kr : &map_k, sub * 64, rem ? rem_head : hkv,
-                            td & TILE_COORD_MASK, rem ? b_rem : b, full);
-        };
-        auto load_v = [&](int j) {                    // lane 0 only; also warms L2 for the tile TC_VST further on
-            const int td = tile_desc(j), stg = j % TC_VST;
-            const bool rem = (td >> 29) & 1;
-            const uint32_t full = bar_v_full + stg * 8;
-            mbar_expect_tx(full, 64 * DV * 2);
-#pragma unroll
-            for (int sub = 0; sub < DV / 64; ++sub)
-                tma_load_4d(s_v + stg * (64 * DV * 2) + sub * 8192, rem ? &map_vr : &map_v, sub * 64, rem ? rem_head : hkv,
-                            td & TILE_COORD_MASK, rem ? b_rem : b, full);
-            if (j + TC_VST < n_tiles) {
-                const int t1 = tile_desc(j + TC_VST);
-                const bool rem1 = (t1 >> 29) & 1;
-                const int c1 = t1 & TILE_COORD_MASK, b1 = rem1 ? b_rem : b, h1 = rem1 ? rem_head : hkv;
-#pragma unroll
-                for (int sub = 0; sub < DV / 64; ++sub) tma_prefetch_4d(rem1 ? &map_vr : &map_v, sub * 64, h1, c1, b1);
-#pragma unroll
-                for (int sub = 0; sub < DK / 64; ++sub) tma_prefetch_4d(rem1 ? &map_kr : &map_k, sub * 64, h1, c1, b1);
-            }
-        };
-        // The loads follow the order in which the tensor core frees the ring stages: the K stages of the first NSB
-        // tiles right after their Q K^T products, then alternately the V stage of tile i (after P_i V_i) and the
-        // K stage of tile i + NSB (Q K_{i+NSB}^T is issued right behind P_i V_i).  Every wait is for the next event
-        // of that sequence, so the producer sleeps in the barrier instead of polling two rings.
-        int jk = min(TC_KST, n_tiles), jv = min(TC_VST, n_tiles);
-        if (lane == 0) {                               // the own-span tiles among these were requested at kernel start
-            for (int j = min(walk.n_span, TC_KST); j < jk; ++j) load_k(j);
-            for (int j = min(walk.n_span, TC_VST); j < jv; ++j) load_v(j);
-        }
-        bool ok = true;
-        auto next_k = [&]() {
-            ok = __all_sync(0xffffffffu, mbar_wait(bar_k_empty + (jk % TC_KST) * 8, ((jk / TC_KST) - 1) & 1, status));
-            if (ok && lane == 0) load_k(jk);
-            ++jk;
-        };
-        for (int i = 0; ok && i < NSB && jk < n_tiles; ++i) next_k();
-        while (ok && (jk < n_tiles || jv < n_tiles)) {
-            if (jv < n_tiles) {
-                ok = __all_sync(0xffffffffu, mbar_wait(bar_v_empty + (jv % TC_VST) * 8, ((jv / TC_VST) - 1) & 1, status));
-                if (ok && lane == 0) load_v(jv);
-                ++jv;
-            }
-            if (ok && jk < n_tiles) next_k();
-            __syncwarp();
-        }
-    } else if (warp == 1) {
-        // ------------------------------------------------------------ MMA issuer
-        constexpr uint32_t idesc_qk = umma_idesc_bf16(128, 64, false);
-        constexpr uint32_t idesc_pv = umma_idesc_bf16(128, DV, true);
-        auto issue_qk = [&](int j) {                  // S_{j&1} = Q K_j^T   (the whole warp)
-            const int sb = j % NSB, stg = j % TC_KST;
-            const uint32_t kt = s_k + stg * (64 * DK * 2);
-#pragma unroll
-            for (int kk = 0; kk < DK / 16; ++kk) {
-                const uint64_t ad = umma_desc(s_q + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024);
-                const uint64_t bd = umma_desc(kt + (kk >> 2) * 8192 + (kk & 3) * 32, 16, 1024);
-                umma_ss(tmem + sb * 64, ad, bd, idesc_qk, kk > 0);
-            }
-            umma_commit(bar_s_full + sb * 8);
-            umma_commit(bar_k_empty + stg * 8);
-        };
-        bool ok = __all_sync(0xffffffffu, mbar_wait(bar_q, 0, status));
-        for (int j = 0; ok && j < min(NSB, n_tiles); ++j) {
-            ok = __all_sync(0xffffffffu, mbar_wait(bar_k_full + (j % TC_KST) * 8, (j / TC_KST) & 1, status));
-            if (ok) {
-                tc_fence_after();
-                issue_qk(j);
-            }
-            __syncwarp();
-        }
-        for (int j = 0; ok && j < n_tiles; ++j) {
-            const int sb = j % NSB, vstg = j % TC_VST;
-            ok = __all_sync(0xffffffffu, mbar_wait(bar_v_full + vstg * 8, (j / TC_VST) & 1, status));
-            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_p_full + sb * 8, (j / NSB) & 1, status));
-            if (!ok) break;
-            {
-                tc_fence_after();
-                const uint32_t vt = s_v + vstg * (64 * DV * 2);
-#pragma unroll
-                for (int kk = 0; kk < 4; ++kk) {
-                    const uint64_t bd = umma_desc(vt + kk * 2048, 8192, 1024);
-                    umma_ts(tmem + TC_O_COL, tmem + sb * 64 + kk * 8, bd, idesc_pv, (j > 0 || kk > 0) ? 1u : 0u);
+    // registers: 2 x 128 x 200 + 128 x 104 = 384 x 168, what the block is launched with
+    if (warp >= 8) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 104;");
+        if (warp == 8) {
+            // -------------------------------------------------------- TMA producer
+            int kc = 0, vc = 0;                          // pairs loaded so far
+            int nq[2] = {0, 0};                          // query tiles loaded so far
+#pragma unroll 1
+            for (int n = 0; ok; ++n) {
+                const int slot = n & 1;
+                // use: bit x = tile x; skip: one tile alone leaves out the pairs [skip, next_a) (A) or [0, skip) (B)
+                int q0, hq, b, span_start, n_span, n_units = -1, use, skip = 0;
+                auto take = [&]() {
+                    ok = warp_wait(bar_item + slot * 8, (n >> 1) & 1);
+                    q0 = items[slot * 8];
+                    hq = items[slot * 8 + 1];
+                    b = items[slot * 8 + 2];
+                    span_start = items[slot * 8 + 3];
+                    n_span = items[slot * 8 + 4];
+                    n_units = items[slot * 8 + 5];
+                    use = items[slot * 8 + 6];
+                    skip = items[slot * 8 + 7];
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar_item_empty + slot * 8);
+                };
+                if (n > 0) {
+                    take();
+                    if (!ok || q0 < 0) break;            // no items left
+                } else {                                 // tile A's first loads depend on no table
+                    int only;
+                    locate(od, blockIdx.x, HQ, q_off, q0, only, hq, b);
+                    span_start = (uint32_t)q0 / (uint32_t)nbs * nbs;
+                    n_span = span_units(q0, span_start, q0 + ATT_BM < q_end, T);
+                    use = only ? only : q0 + ATT_BM < q_end ? 3 : 1;
                 }
-                umma_commit(bar_v_empty + vstg * 8);
-                umma_commit(bar_pv + (j & 1) * 8);
+                const int hkv = (uint32_t)hq / od.q_per_kv, hn = (uint32_t)hq / od.q_per_sel, b_rem = (uint32_t)b % (uint32_t)B_rem;
+                const int* idx = indices + ((long)b * TN * HN + hn) * 2;
+                const long tstride = (long)HN * 2;
+                RemoteKeys rk;
+                rk.k_split = k_split;
+                rk.slots = rem_slots;
+                rk.stride = HKV;
+                rk.base = rem_base ? rem_base + ((long)b_rem * od.rem_segments) * HKV + hkv : nullptr;
+                const int rem_head = rem_base ? 0 : hkv;         // packed pairs have no head axis
+                // token coordinate of unit u in the tensor it is loaded from; bit 31 = gathered keys
+                auto unit = [&](int u) -> uint32_t {
+                    if (u >= (n_units < 0 ? n_span : n_units)) return 0;
+                    int s0;
+                    if (u < n_span) {
+                        s0 = span_start + u * ATT_BN;
+                    } else {
+                        const uint32_t up = u - n_span, blk = up / (uint32_t)cpb;
+                        s0 = __ldg(idx + (long)blk * tstride) * nbs + (int)(up - blk * cpb) * ATT_BN;
+                    }
+                    if (s0 >= rk.k_split) return (uint32_t)(s0 - rk.k_split);
+                    int coord = s0;
+                    if (rk.base) {
+                        const int vb = (uint32_t)s0 / (uint32_t)nbs, g = (uint32_t)vb / (uint32_t)rk.slots;
+                        coord = (rk.base[(long)g * rk.stride] + (vb - g * rk.slots)) * nbs + (s0 - vb * nbs);
+                    }
+                    return (uint32_t)coord | 0x80000000u;
+                };
+                auto load_q = [&](int x) {
+                    if (nq[x] > 0) ok = warp_wait(bar_q_empty + x * 8, (nq[x] - 1) & 1);
+                    if (ok && lane == 0) {
+                        mbar_expect_tx(bar_q_full + x * 8, 128 * DK * 2);
+#pragma unroll
+                        for (int sub = 0; sub < DK / 64; ++sub)
+                            tma_load_4d(s_q + x * (128 * DK * 2) + sub * 16384, &map_q, sub * 64, hq, q0 - q_off + x * ATT_BM, b,
+                                        bar_q_full + x * 8);
+                    }
+                    __syncwarp();
+                    if (ok) ++nq[x];
+                };
+                auto load_pair = [&](uint32_t dst, uint32_t full, const CUtensorMap* own, const CUtensorMap* rem, int subs,
+                                     uint32_t u0, uint32_t u1, bool two) {            // lane 0 only
+                    mbar_expect_tx(full, (two ? 2 : 1) * subs * 8192);
+#pragma unroll 1
+                    for (int e = 0; e < (two ? 2 : 1); ++e) {
+                        const uint32_t u = e ? u1 : u0;
+                        const bool r = (u >> 31) != 0;
+#pragma unroll 1
+                        for (int sub = 0; sub < subs; ++sub)
+                            tma_load_4d(dst + sub * 16384 + e * 8192, r ? rem : own, sub * 64, r ? rem_head : hkv,
+                                        (int)(u & 0x7fffffffu), r ? b_rem : b, full);
+                    }
+                };
+                if (use & 1) load_q(0);
+                uint32_t mine = 0;                       // lane l: unit l of the 32 that hold the pair at hand
+#pragma unroll 1
+                for (int j = 0; ok; ++j) {
+                    const bool now = n_units < 0 && (j > 0 || n_span < 2 || use == 2);
+                    if (now) take();
+                    if (!ok || (n_units >= 0 && 2 * j >= n_units)) break;
+                    if ((j & 15) == 0 || now) mine = unit(2 * (j & ~15) + lane);
+                    const uint32_t u0 = __shfl_sync(0xffffffffu, mine, (2 * j) & 31), u1 = __shfl_sync(0xffffffffu, mine, (2 * j + 1) & 31);
+                    const bool two = 2 * j + 1 < (n_units < 0 ? n_span : n_units);
+                    if (j == 0 && use == 2) load_q(1);
+                    if (!ok) break;
+                    if (skip > 0 && (use == 2 ? j < skip : j >= skip && 2 * j < n_span && !(2 * j + 1 == n_span && n_units > n_span)))
+                        continue;                        // only the other tile uses it
+                    const int ks = kc % KST;
+                    if (kc >= KST) ok = warp_wait(bar_k_empty + ks * 8, (kc / KST - 1) & 1);
+                    if (!ok) break;
+                    if (lane == 0) load_pair(s_k + ks * (128 * DK * 2), bar_k_full + ks * 8, &map_k, &map_kr, DK / 64, u0, u1, two);
+                    __syncwarp();
+                    ++kc;
+                    // behind the first keys, not before: tile A may already go on while the last scores of the previous item's
+                    // tile B, which still read the old query tile, have yet to be issued
+                    if (j == 0 && use == 3) load_q(1);
+                    if (!ok) break;
+                    const int vs = vc % VST;
+                    if (vc >= VST) ok = warp_wait(bar_v_empty + vs * 8, (vc / VST - 1) & 1);
+                    if (!ok) break;
+                    if (lane == 0) load_pair(s_v + vs * (128 * DV * 2), bar_v_full + vs * 8, &map_v, &map_vr, DV / 64, u0, u1, two);
+                    __syncwarp();
+                    ++vc;
+                }
             }
-            __syncwarp();
-            if (j + NSB < n_tiles) {
-                const int jn = j + NSB;
-                ok = __all_sync(0xffffffffu, mbar_wait(bar_k_full + (jn % TC_KST) * 8, (jn / TC_KST) & 1, status));
-                if (!ok) break;
-                {
+            if (!ok) {                                   // nothing may still be on its way into shared memory
+#pragma unroll 1
+                for (int c = max(0, kc - KST); c < kc; ++c) warp_wait(bar_k_full + (c % KST) * 8, (c / KST) & 1);
+#pragma unroll 1
+                for (int c = max(0, vc - VST); c < vc; ++c) warp_wait(bar_v_full + (c % VST) * 8, (c / VST) & 1);
+                if (nq[0] > 0) warp_wait(bar_q_full, (nq[0] - 1) & 1);
+                if (nq[1] > 0) warp_wait(bar_q_full + 8, (nq[1] - 1) & 1);
+            }
+        } else if (warp != 10) {
+            // -------------------------------------------------------- MMA issuer of one tile (the whole warp, converged)
+            // One issuing warp per tile: neither waits for the other's softmax.
+            constexpr uint32_t idesc_s1 = umma_idesc_bf16(128, 64, false), idesc_s2 = umma_idesc_bf16(128, 128, false);
+            constexpr uint32_t idesc_pv = umma_idesc_bf16(128, DV, true);
+            const int x = warp == 9 ? 0 : 1;
+            const uint32_t qlo = umma_desc_lo(s_q, 16) + x * (128 * DK * 2 >> 4), k_lo = umma_desc_lo(s_k, 16),
+                           v_lo = umma_desc_lo(s_v, 16384);
+            const uint32_t t_s = tmem + x * 128, t_p = tmem + P_COL + x * P_STRIDE, t_o = tmem + AT_O_COL + x * DV;
+            const uint32_t b_s = bar_s + x * 8, b_free = bar_s_free + x * 8, b_p = bar_p + x * 16, b_o = bar_o + x * 8;
+            bool more = true;
+            uint32_t q_par = 0, p_par = 0, f_par = 1;    // parities of the next query tile / probabilities / release of the scores
+            uint32_t acc = 0;                            // O holds a product of this item
+            int chunk = 0, pos = 0;
+            // The next step, which may be one that this tile takes no part in.  It is never looked for further ahead than LEAD
+            // steps: the items behind are only scheduled once the loads of this one, which wait for its products, are through.
+            auto next_step = [&]() -> uint32_t {
+                if (!more) return ST_STOP;
+                const int slot = chunk & (AT_CHUNKS - 1);
+                if (pos == 0) ok = warp_wait(bar_steps + slot * 8, (chunk / AT_CHUNKS) & 1);
+                const int4 e = steps[(slot * AT_CHUNK + pos) * 2];
+                // (through a shuffle: what follows from the words is the same in all lanes, which the compiler then knows)
+                const uint32_t fa = __shfl_sync(0xffffffffu, (uint32_t)e.x, 0), fx = __shfl_sync(0xffffffffu, (uint32_t)(x ? e.y : e.x), 0);
+                ++pos;
+                if (fa & ST_CHUNK_LAST) {
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar_steps_empty + slot * 8);
+                    ++chunk;
+                    pos = 0;
+                }
+                more = ok && !(fa & ST_STOP);
+                return more ? fx : ST_STOP;
+            };
+            auto issue_s = [&](uint32_t f) {             // S = Q K^T
+                if (!ok || !(f & ST_VALID)) return;
+                if (f & ST_FIRST) {
+                    ok = warp_wait(bar_q_full + x * 8, q_par);
+                    q_par ^= 1;
+                }
+                const uint32_t st = (f >> ST_K) & 3;
+                if (ok) ok = warp_wait(bar_k_full + st * 8, (f >> ST_KPAR) & 1);
+                if (LEAD == 2) {                         // the softmax holds the previous scores in registers (first time: free)
+                    if (ok) ok = warp_wait(b_free, f_par);
+                    f_par ^= 1;
+                }
+                if (!ok) return;
+                tc_fence_after();
+                const uint32_t klo = k_lo + st * (128 * DK * 2 >> 4), idesc = (f & ST_TWO) ? idesc_s2 : idesc_s1;
+#pragma unroll
+                for (int h = 0; h < DK / 64; ++h) umma_ss_x4<2, 2>(t_s, qlo + h * 1024, klo + h * 1024, idesc, h > 0);
+                umma_commit(b_s);
+                umma_commit(bar_k_empty + st * 8);
+                if (f & ST_ALONE) umma_commit(bar_k_empty + st * 8);
+                if (f & ST_LAST) umma_commit(bar_q_empty + x * 8);
+            };
+            auto issue_pv = [&](uint32_t f) {            // O += P V
+                if (!ok || !(f & ST_VALID)) return;
+                if (f & ST_FIRST) acc = 0;
+                const uint32_t st = (f >> ST_V) & 3;
+                ok = warp_wait(bar_v_full + st * 8, (f >> ST_VPAR) & 1);
+                const uint32_t vlo = v_lo + st * (128 * DV * 2 >> 4), par = p_par;
+                p_par ^= 1;
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    if (ok && (e == 0 || LEAD == 1)) ok = warp_wait(b_p + e * 8, par);
+                    if (!ok) return;
                     tc_fence_after();
-                    issue_qk(jn);
+                    if (f & (e ? ST_USE1 : ST_USE0)) {   // a unit that no row sees stays out, whatever its values are
+                        umma_ts_x4<128>(t_o, t_p + e * 32, vlo + e * 512, idesc_pv, acc);
+                        acc = 1;
+                    }
+                }
+                if (LEAD == 2 || (f & ST_LAST)) umma_commit(b_o);
+                umma_commit(bar_v_empty + st * 8);
+                if (f & ST_ALONE) umma_commit(bar_v_empty + st * 8);
+            };
+            uint32_t ring[LEAD];                         // steps whose scores are issued and whose products are not
+#pragma unroll
+            for (int e = 0; e < LEAD; ++e) ring[e] = 0;
+#pragma unroll 1
+            while (ok && !(ring[0] & ST_STOP)) {
+                const uint32_t f = next_step();
+                issue_pv(ring[0]);
+                issue_s(f);
+#pragma unroll
+                for (int e = 0; e + 1 < LEAD; ++e) ring[e] = ring[e + 1];
+                ring[LEAD - 1] = f;
+            }
+        } else {
+            // -------------------------------------------------------- scheduler: work items, and their steps, one lane per step
+            // (It runs ahead of the loads.  A single warp that works the steps out between two products costs more than the
+            // products themselves, and one that does so between two loads makes every item begin with a wait.)
+            bool stop = false;
+            int asked = -1;                              // request whose answer is outstanding
+            int chunk = 0, base = 0;                     // base: pairs of all items before
+            int block = blockIdx.x;
+            const int NTq = (T + ATT_BM - 1) / ATT_BM;
+            auto request = [&](int n) {
+                asked = n;
+                if (lane == 0) {
+                    fence_async_smem();
+                    mbar_expect_tx(bar_clc, 16);
+                    request_block(s_clc, bar_clc);
                 }
                 __syncwarp();
+            };
+#pragma unroll 1
+            for (int n = 0; ok; ++n) {
+                if (n > 0) {
+                    if (asked < 0) {                     // not before the loads of the item before have begun
+                        ok = warp_wait(bar_item_empty + ((n - 1) & 1) * 8, ((n - 1) >> 1) & 1);
+                        if (!ok) break;
+                        request(n - 1);
+                    }
+                    ok = warp_wait(bar_clc, (n - 1) & 1);
+                    if (!ok) break;
+                    asked = -1;
+                    stop = !taken_block(s_clc, block);
+                    __syncwarp();
+                }
+                const int islot = n & 1;
+                if (n >= 2) ok = warp_wait(bar_item_empty + islot * 8, ((n >> 1) - 1) & 1);
+                if (!ok) break;
+                int q0, only, hq, b;
+                locate(od, stop ? 0 : block, HQ, q_off, q0, only, hq, b);
+                const int hn = (uint32_t)hq / od.q_per_sel, blk0 = (uint32_t)q0 / (uint32_t)nbs;
+                const int* selp = types_i + ((long)b * TN * HN + hn) * 2;
+                const int n_past = __ldg(attn_n_iters + ((long)b * NTq + q0 / ATT_BM) * HN + hn);
+                // the own span touches at most four selection blocks
+                const int s_lane = (lane < 4 && blk0 + lane < TN) ? __ldg(selp + (long)(blk0 + lane) * HN * 2) : 0;
+                const int sel = (int)(__ballot_sync(0xffffffffu, s_lane != 0) & 15u);
+                const Item it = make_item(q0, blk0 * nbs, n_past, sel, T, q_end, only, nbs, own_chunk, lane);
+                if (lane == 0) {
+                    items[islot * 8 + 0] = stop ? -1 : q0;
+                    items[islot * 8 + 1] = hq;
+                    items[islot * 8 + 2] = b;
+                    items[islot * 8 + 3] = it.span_start;
+                    items[islot * 8 + 4] = it.n_span;
+                    items[islot * 8 + 5] = it.n_units;
+                    items[islot * 8 + 6] = (it.use_a ? 1 : 0) | (it.use_b ? 2 : 0);
+                    items[islot * 8 + 7] = it.use_a && it.use_b ? 0 : it.use_a ? it.end_a : it.first_b;
+                    mbar_arrive(bar_item + islot * 8);
+                }
+                __syncwarp();
+                // An item of a few pairs is over before the next one could be taken and planned: ask at once.  Behind a longer
+                // one a block is better left to an SM that is free earlier.
+                if (!stop && it.n_pairs <= 4) request(n);
+                const int n_a = it.use_a ? it.end_a + it.n_pairs - it.next_a : 0, n_b = it.use_b ? it.n_pairs - it.first_b : 0;
+                const int n_steps = stop ? 1 : max(n_a, n_b);
+#pragma unroll 1
+                for (int i0 = 0; ok && i0 < n_steps; i0 += AT_CHUNK) {
+                    const int slot = chunk & (AT_CHUNKS - 1), i = i0 + lane;
+                    if (chunk >= AT_CHUNKS) ok = warp_wait(bar_steps_empty + slot * 8, (chunk / AT_CHUNKS - 1) & 1);
+                    const bool mine = lane < AT_CHUNK && i < n_steps;
+                    const int ja = i < it.end_a ? i : i + it.next_a - it.end_a, jb = i + it.first_b;
+                    auto masked = [&](int j) { return 2 * j < it.n_span || 2 * j + 1 >= it.n_units; };
+                    uint32_t seen = 0xffffffffu;         // seen_chunks() of this lane's step
+#pragma unroll 1
+                    for (uint32_t todo = __ballot_sync(0xffffffffu, mine && (masked(ja) || masked(jb))); todo; todo &= todo - 1) {
+                        const int src = __ffs(todo) - 1;
+                        const uint32_t bits = seen_chunks(it, __shfl_sync(0xffffffffu, ja, src), __shfl_sync(0xffffffffu, jb, src),
+                                                          lane, cpb, nbs, own_chunk);
+                        if (lane == src) seen = bits;
+                    }
+                    if (ok && mine) {
+                        uint32_t f[2] = {0, 0}, mk[2] = {0, 0};
+#pragma unroll
+                        for (int x = 0; x < 2; ++x) {
+                            const int nx = x ? n_b : n_a;
+                            if (stop || i >= nx) continue;
+                            const int j = x ? jb : ja, c = base + (it.use_a && it.use_b ? j : i);
+                            const bool alone = !(uses_a(it, j) && uses_b(it, j));
+                            const uint32_t m = (seen >> (16 * x)) & 0xffffu;
+                            // the chunk whose keys are the warp's own rows is chunk w + d of the pair
+                            const int d = (it.q0 + x * ATT_BM - (it.span_start + 2 * j * ATT_BN)) / 32;
+                            const bool own = own_chunk && 2 * j < it.n_span && d > -4 && d < 4;
+                            f[x] = ST_VALID | ((m & 0x3333u) ? ST_USE0 : 0) | ((m & 0xccccu) ? ST_USE1 : 0) | (i == 0 ? ST_FIRST : 0) |
+                                   (i == nx - 1 ? ST_LAST : 0) | (alone ? ST_ALONE : 0) | (2 * j + 1 < it.n_units ? ST_TWO : 0) |
+                                   ((uint32_t)(c % KST) << ST_K) | ((uint32_t)((c / KST) & 1) << ST_KPAR) |
+                                   ((uint32_t)(c % VST) << ST_V) | ((uint32_t)((c / VST) & 1) << ST_VPAR);
+                            mk[x] = m | (own ? (uint32_t)(d + 4) << 16 : 0u);
+                        }
+                        if (lane == AT_CHUNK - 1 || i == n_steps - 1) f[0] |= ST_CHUNK_LAST;
+                        if (stop) f[0] |= ST_STOP;
+                        steps[(slot * AT_CHUNK + lane) * 2] = make_int4((int)f[0], (int)f[1], (int)mk[0], (int)mk[1]);
+                        steps[(slot * AT_CHUNK + lane) * 2 + 1] = make_int4(it.q0, hq, b, 0);
+                    }
+                    __syncwarp();
+                    if (ok && lane == 0) mbar_arrive(bar_steps + slot * 8);
+                    ++chunk;
+                }
+                if (stop) break;
+                base += it.use_a && it.use_b ? it.n_pairs : n_steps;                  // loaded pairs
             }
+            if (asked >= 0) warp_wait(bar_clc, asked & 1);       // (after a failed wait: the answer may still be on its way)
         }
     } else {
-        // ------------------------------------------------------------ softmax + epilogue (8 warps)
-        // Warp (quad, half) owns the 16 query rows quad*32 + half*16 ... of the tile (a warp reaches only its own
-        // quarter of the TMEM lanes).  In the 16x256b layout a thread holds, of rows ra and ra + 8, the columns
-        // 8k + 2(lane%4), +1 for k = 0..7: 32 scores; the four threads of a row meet through two shuffles.
-        const int quad = warp & 3, half = (warp - 2) >> 2;
-        const int row_a = quad * 32 + half * 16 + (lane >> 2), row_b = row_a + 8;
-        const int cq = (lane & 3) * 2;
-        const int t_a = q0 + row_a, t_b = q0 + row_b;
-        const uint32_t t_rows = tmem + ((uint32_t)(quad * 32 + half * 16) << 16);
-        const uint32_t t_o = t_rows + TC_O_COL;
-        float m_a = -INFINITY, m_b = -INFINITY, l_a = 0.f, l_b = 0.f;
-        // the own span lies in at most two selection blocks (nbs >= 64 and 64 | q0 - span_start)
-        const int blk0 = walk.span_start / nbs;
-        const bool sel0 = selp[(long)blk0 * tstride] != 0;
-        const bool sel1 = blk0 + 1 < TN && selp[(long)(blk0 + 1) * tstride] != 0;
-        bool ok = true;
-        for (int j = 0; j < n_tiles; ++j) {
-            const int sb = j % NSB;
-            const uint32_t t_s = t_rows + sb * 64;
-            ok = __all_sync(0xffffffffu, mbar_wait(bar_s_full + sb * 8, (j / NSB) & 1, status));
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 200;");
+        // ------------------------------------------------------------ softmax + epilogue (tile x, one row per thread)
+        const int x = warp >> 2, row = (warp & 3) * 32 + lane;
+        const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+        const uint32_t t_s = lane_base + x * 128, t_o = lane_base + AT_O_COL + x * DV, t_p = lane_base + P_COL + x * P_STRIDE;
+        const bool wide = (reinterpret_cast<uintptr_t>(o) & 31) == 0;
+        const uint32_t tri = (2u << lane) - 1;           // keys of the row's own 32-key chunk that it sees
+        int ns = 0, no = 0;                              // score tiles, phases of bar_o taken so far
+        int chunk = 0, pos = 0;
+        float m = -INFINITY;
+        uint64_t l2a = 0, l2b = 0;                       // two packed partial sums of the row
+#pragma unroll 1
+        while (ok) {
+            const int slot = chunk & (AT_CHUNKS - 1);
+            if (pos == 0) ok = warp_wait(bar_steps + slot * 8, (chunk / AT_CHUNKS) & 1);
+            if (!ok) break;
+            const int4 e0 = steps[(slot * AT_CHUNK + pos) * 2], e1 = steps[(slot * AT_CHUNK + pos) * 2 + 1];
+            const uint32_t fa = __shfl_sync(0xffffffffu, (uint32_t)e0.x, 0), f = x ? __shfl_sync(0xffffffffu, (uint32_t)e0.y, 0) : fa,
+                           mk = __shfl_sync(0xffffffffu, (uint32_t)(x ? e0.w : e0.z), 0);
+            ++pos;
+            if (fa & ST_CHUNK_LAST) {
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_steps_empty + slot * 8);
+                ++chunk;
+                pos = 0;
+            }
+            if (fa & ST_STOP) break;
+            if (!(f & ST_VALID)) continue;
+            const int t = e1.x + x * ATT_BM + row, hq = e1.y, b = e1.z;
+            if (f & ST_FIRST) {
+                m = -INFINITY;
+                l2a = l2b = 0;
+            }
+            ok = warp_wait(bar_s + x * 8, ns & 1);
+            ++ns;
             if (!ok) break;
             tc_fence_after();
-            uint32_t sr[32];
-            tmem_ld_16x256b_x8(t_s, sr);
+            uint32_t sr[4][32];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) tmem_ld32(t_s + c * 32, sr[c]);
             tmem_ld_wait();
-            if (j < walk.n_span) {
-                // own-span tile: per row the visible keys are columns [0, limit] (attn_walk.cuh: visible())
-                const int s0 = walk.span_start + j * ATT_BN;
-                const bool selb = (s0 / nbs == blk0) ? sel0 : sel1;
-                const int blk_end = (s0 / nbs + 1) * nbs;
-                int lim_a = T - 1 - s0, lim_b = lim_a;
-                if (own_chunk) {
-                    lim_a = min(lim_a, t_a - s0);
-                    lim_b = min(lim_b, t_b - s0);
-                    if (!(selb || t_a < blk_end)) lim_a = -1;
-                    if (!(selb || t_b < blk_end)) lim_b = -1;
-                } else {
-                    if (!(selb && t_a >= blk_end)) lim_a = -1;
-                    if (!(selb && t_b >= blk_end)) lim_b = -1;
-                }
+            if (LEAD == 2) {
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_s_free + x * 8);
+            }
+            // Chunks of 32 columns that no row of the warp sees cost nothing below; the one that holds the warp's own rows is
+            // masked per element, every other one is seen in full.
+            const uint32_t live = (mk >> (4 * (warp & 3))) & 15u;
+            if (mk >> 16) {
+                const int diag = (warp & 3) + (int)(mk >> 16) - 4;
 #pragma unroll
-                for (int k = 0; k < 8; ++k)
+                for (int c = 0; c < 4; ++c)
+                    if (c == diag) {
 #pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        const int c = 8 * k + cq + e;
-                        sr[4 * k + e] = (c <= lim_a) ? sr[4 * k + e] : 0xff800000u;          // -inf
-                        sr[4 * k + 2 + e] = (c <= lim_b) ? sr[4 * k + 2 + e] : 0xff800000u;
+                        for (int e = 0; e < 32; ++e) sr[c][e] = (tri & (1u << e)) ? sr[c][e] : 0xff800000u;      // -inf
                     }
             }
-            // row maxima of the raw scores (scale > 0, so max(scale * s) = scale * max(s))
-            float xa0 = -INFINITY, xa1 = -INFINITY, xb0 = -INFINITY, xb1 = -INFINITY;
+            // row maximum of the raw scores (scale > 0, so max(scale * s) = scale * max(s))
+            float mx[4];
 #pragma unroll
-            for (int k = 0; k < 8; k += 2) {
-                xa0 = fmax3(xa0, __uint_as_float(sr[4 * k]), __uint_as_float(sr[4 * k + 1]));
-                xb0 = fmax3(xb0, __uint_as_float(sr[4 * k + 2]), __uint_as_float(sr[4 * k + 3]));
-                xa1 = fmax3(xa1, __uint_as_float(sr[4 * k + 4]), __uint_as_float(sr[4 * k + 5]));
-                xb1 = fmax3(xb1, __uint_as_float(sr[4 * k + 6]), __uint_as_float(sr[4 * k + 7]));
+            for (int c = 0; c < 4; ++c) {
+                mx[c] = -INFINITY;
+                if ((live >> c) & 1) {
+#pragma unroll
+                    for (int e = 0; e < 32; e += 2) mx[c] = fmax3(mx[c], __uint_as_float(sr[c][e]), __uint_as_float(sr[c][e + 1]));
+                }
             }
-            float xa = fmaxf(xa0, xa1), xb = fmaxf(xb0, xb1);
-            xa = fmaxf(xa, __shfl_xor_sync(0xffffffffu, xa, 1));
-            xb = fmaxf(xb, __shfl_xor_sync(0xffffffffu, xb, 1));
-            xa = fmaxf(xa, __shfl_xor_sync(0xffffffffu, xa, 2));
-            xb = fmaxf(xb, __shfl_xor_sync(0xffffffffu, xb, 2));
-            const float mx_a = xa * scale_log2, mx_b = xb * scale_log2;
-            const bool need_a = mx_a > m_a + LAZY_RESCALE_LOG2, need_b = mx_b > m_b + LAZY_RESCALE_LOG2;
-            if (__any_sync(0xffffffffu, need_a || need_b)) {
-                const float new_a = need_a ? mx_a : m_a, new_b = need_b ? mx_b : m_b;
-                const float alpha_a = (new_a == -INFINITY) ? 1.f : ex2(m_a - new_a);
-                const float alpha_b = (new_b == -INFINITY) ? 1.f : ex2(m_b - new_b);
-                if (j > 0) {
-                    // O must be at rest: P_{j-1} V_{j-1} has to be complete.  Even and odd tiles signal on two
-                    // barriers.  S_j was produced behind P_{j-NSB} V_{j-NSB}, hence behind P_{j-3} V_{j-3} (the
-                    // previous phase of the barrier waited on; NSB <= 3), and P_{j+1} V_{j+1} cannot have started:
-                    // the barrier is in the phase waited for or the one after it, so a parity wait without having
-                    // watched the earlier phases is unambiguous.
-                    ok = __all_sync(0xffffffffu, mbar_wait(bar_pv + ((j - 1) & 1) * 8, ((j - 1) >> 1) & 1, status));
-                    if (!ok) break;
-                    tc_fence_after();
+            const float mnew = fmaxf(fmax3(mx[0], mx[1], mx[2]), mx[3]) * scale_log2;
+            const bool need = mnew > m + LAZY_RESCALE_LOG2;
+            if (__any_sync(0xffffffffu, need)) {
+                const float mn = need ? mnew : m;
+                const float alpha = mn == -INFINITY ? 1.f : ex2(m - mn);
+                if (!(f & ST_FIRST)) {
+                    // O must be at rest.  LEAD = 2: the product of the previous P; LEAD = 1: these scores are complete, hence
+                    // so is every product issued before them.
+                    if (LEAD == 2) {
+                        ok = warp_wait(bar_o + x * 8, no & 1);
+                        if (!ok) break;
+                        tc_fence_after();
+                    }
 #pragma unroll 1
-                    for (int c0 = 0; c0 < DV; c0 += 64) {
+                    for (int c0 = 0; c0 < DV; c0 += 32) {
                         uint32_t orr[32];
-                        tmem_ld_16x256b_x8(t_o + c0, orr);
+                        tmem_ld32(t_o + c0, orr);
                         tmem_ld_wait();
 #pragma unroll
-                        for (int k = 0; k < 8; ++k) {
-                            orr[4 * k] = __float_as_uint(__uint_as_float(orr[4 * k]) * alpha_a);
-                            orr[4 * k + 1] = __float_as_uint(__uint_as_float(orr[4 * k + 1]) * alpha_a);
-                            orr[4 * k + 2] = __float_as_uint(__uint_as_float(orr[4 * k + 2]) * alpha_b);
-                            orr[4 * k + 3] = __float_as_uint(__uint_as_float(orr[4 * k + 3]) * alpha_b);
-                        }
-                        tmem_st_16x256b_x8(t_o + c0, orr);
+                        for (int e = 0; e < 32; ++e) orr[e] = __float_as_uint(__uint_as_float(orr[e]) * alpha);
+                        tmem_st32(t_o + c0, orr);
                     }
                 }
-                l_a *= alpha_a;
-                l_b *= alpha_b;
-                m_a = new_a;
-                m_b = new_b;
+                const uint64_t al2 = pack2(alpha, alpha);
+                l2a = fma2(l2a, al2, 0);
+                l2b = fma2(l2b, al2, 0);
+                m = mn;
             }
-            const float neg_a = (m_a == -INFINITY) ? 0.f : -m_a, neg_b = (m_b == -INFINITY) ? 0.f : -m_b;
-            float la2 = 0.f, lb2 = 0.f;
-            uint32_t pr[16];
+            const float neg = m == -INFINITY ? 0.f : -m;
+            const uint64_t sc2 = pack2(scale_log2, scale_log2), ng2 = pack2(neg, neg);
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const float p0 = ex2(fmaf(__uint_as_float(sr[4 * k]), scale_log2, neg_a));
-                const float p1 = ex2(fmaf(__uint_as_float(sr[4 * k + 1]), scale_log2, neg_a));
-                const float p2 = ex2(fmaf(__uint_as_float(sr[4 * k + 2]), scale_log2, neg_b));
-                const float p3 = ex2(fmaf(__uint_as_float(sr[4 * k + 3]), scale_log2, neg_b));
-                if (k & 1) {
-                    la2 += p0 + p1;
-                    lb2 += p2 + p3;
-                } else {
-                    l_a += p0 + p1;
-                    l_b += p2 + p3;
+            for (int h = 0; h < 2; ++h) {
+                uint32_t pr[32];
+#pragma unroll
+                for (int g = 0; g < 2; ++g) {
+                    if ((live >> (2 * h + g)) & 1) {
+#pragma unroll
+                        for (int c = 0; c < 16; ++c) {
+                            const uint32_t* s2 = sr[2 * h + g] + 2 * c;
+                            float x0, x1;
+                            unpack2(fma2(pack2(__uint_as_float(s2[0]), __uint_as_float(s2[1])), sc2, ng2), x0, x1);
+                            x0 = ex2(x0);
+                            x1 = ex2(x1);
+                            if (c & 1) l2b = add2(l2b, pack2(x0, x1));
+                            else l2a = add2(l2a, pack2(x0, x1));
+                            pr[16 * g + c] = pack_bf16(x0, x1);
+                        }
+                    } else {
+#pragma unroll
+                        for (int c = 0; c < 16; ++c) pr[16 * g + c] = 0;
+                    }
                 }
-                pr[2 * k] = pack_bf16(p0, p1);                // P column 4k + lane%4 of row a
-                pr[2 * k + 1] = pack_bf16(p2, p3);            // ... of row b
+                if (LEAD == 2 && h == 0 && !(f & ST_FIRST)) {     // the previous P has been used
+                    ok = warp_wait(bar_o + x * 8, no & 1);
+                    ++no;
+                    if (!ok) break;
+                    tc_fence_after();
+                }
+                tmem_st32(t_p + h * 32, pr);
+                if (LEAD == 1 || h == 1) {               // (LEAD = 1: P V of the first 64 keys starts while the others' P is formed)
+                    tmem_st_wait();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar_p + (2 * x + (LEAD == 1 ? h : 0)) * 8);
+                }
             }
-            l_a += la2;
-            l_b += lb2;
-            tmem_st_16x128b_x8(t_s, pr);                      // P_j over the first 32 columns of S_{j&1}
-            tmem_st_wait();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_p_full + sb * 8);
-        }
-        // The last two products, in order: S of the last tile was produced behind P V of tile n-1-NSB >= n-4, the
-        // previous phase of the barrier of tile n-2; once that one is complete so is tile n-3, the previous phase
-        // of the barrier of the last tile.
-        if (ok && n_tiles >= 2)
-            ok = __all_sync(0xffffffffu, mbar_wait(bar_pv + ((n_tiles - 2) & 1) * 8, ((n_tiles - 2) >> 1) & 1, status));
-        if (ok)
-            ok = __all_sync(0xffffffffu, mbar_wait(bar_pv + ((n_tiles - 1) & 1) * 8, ((n_tiles - 1) >> 1) & 1, status));
-        unsigned char* stage = smem + L::q;
-        if (ok) {
+            if (!ok) break;
+            if (!(f & ST_LAST)) continue;
+            ok = warp_wait(bar_o + x * 8, no & 1);
+            ++no;
+            if (!ok) break;
             tc_fence_after();
-            l_a += __shfl_xor_sync(0xffffffffu, l_a, 1);
-            l_b += __shfl_xor_sync(0xffffffffu, l_b, 1);
-            l_a += __shfl_xor_sync(0xffffffffu, l_a, 2);
-            l_b += __shfl_xor_sync(0xffffffffu, l_b, 2);
-            const bool has_a = l_a > 0.f, has_b = l_b > 0.f;
-            const float inv_a = has_a ? 1.f / l_a : 0.f, inv_b = has_b ? 1.f / l_b : 0.f;
+            float l0, l1, l2, l3;
+            unpack2(l2a, l0, l1);
+            unpack2(l2b, l2, l3);
+            const float l = (l0 + l1) + (l2 + l3);
+            const bool none = l == 0.f;                  // no visible key: O may never have been written
+            const float inv = none ? 0.f : 1.f / l;
+            const int tq = t - q_off;
+            __nv_bfloat16* orow = o + (((long)b * Tq + tq) * HQ + hq) * DV;
 #pragma unroll 1
-            for (int c0 = 0; c0 < DV; c0 += 64) {
-                uint32_t orr[32];
-                tmem_ld_16x256b_x8(t_o + c0, orr);
+            for (int c0 = 0; c0 < DV; c0 += 32) {
+                uint32_t orr[32], pk[16];
+                tmem_ld32(t_o + c0, orr);
                 tmem_ld_wait();
 #pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    const int chunk = (c0 >> 3) + k;
-                    *reinterpret_cast<uint32_t*>(stage + swz<DV * 2>(row_a, chunk) + (lane & 3) * 4) =
-                        pack_bf16(__uint_as_float(orr[4 * k]) * inv_a, __uint_as_float(orr[4 * k + 1]) * inv_a);
-                    *reinterpret_cast<uint32_t*>(stage + swz<DV * 2>(row_b, chunk) + (lane & 3) * 4) =
-                        pack_bf16(__uint_as_float(orr[4 * k + 2]) * inv_b, __uint_as_float(orr[4 * k + 3]) * inv_b);
+                for (int e = 0; e < 16; ++e)
+                    pk[e] = none ? 0u : pack_bf16(__uint_as_float(orr[2 * e]) * inv, __uint_as_float(orr[2 * e + 1]) * inv);
+                if (tq < Tq) {
+                    if (wide) {                          // whole 32-byte sectors
+#pragma unroll
+                        for (int e = 0; e < 16; e += 8)
+                            asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                                         ::"l"(orow + c0 + 2 * e), "r"(pk[e]), "r"(pk[e + 1]), "r"(pk[e + 2]), "r"(pk[e + 3]),
+                                           "r"(pk[e + 4]), "r"(pk[e + 5]), "r"(pk[e + 6]), "r"(pk[e + 7])
+                                         : "memory");
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 16; e += 4)
+                            *reinterpret_cast<uint4*>(orow + c0 + 2 * e) = make_uint4(pk[e], pk[e + 1], pk[e + 2], pk[e + 3]);
+                    }
                 }
             }
-            if ((lane & 3) == 0) {
-                if (t_a - q_off < Tq) lse[((long)b * Tq + (t_a - q_off)) * HQ + hq] = has_a ? m_a + log2f(l_a) : 0.f;
-                if (t_b - q_off < Tq) lse[((long)b * Tq + (t_b - q_off)) * HQ + hq] = has_b ? m_b + log2f(l_b) : 0.f;
-            }
-        }
-        // every softmax warp reaches this barrier, also after a failed wait (no warp may be left behind)
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-        if (ok) {
-            constexpr int CPR = DV / 8;
-            __nv_bfloat16* obase = o + (((long)b * Tq + (q0 - q_off)) * HQ + hq) * DV;
-            const int st_tid = tid - 64;
-            for (int i = st_tid; i < 128 * CPR; i += 256) {
-                const int r = i / CPR, cch = i % CPR;
-                if (q0 - q_off + r < Tq) {
-                    const uint4 x = *reinterpret_cast<const uint4*>(stage + swz<DV * 2>(r, cch));
-                    *reinterpret_cast<uint4*>(obase + (long)r * HQ * DV + cch * 8) = x;
-                }
-            }
+            if (tq < Tq) lse[((long)b * Tq + tq) * HQ + hq] = l > 0.f ? m + log2f(l) : 0.f;
+            tc_fence_before();                           // O is read before the next item's first P is announced
         }
     }
     // ---------------------------------------------------------------- teardown
+    if (!ok && lane == 0) atomicExch(status, NATSL_DEV_WAIT_TIMEOUT);
     tc_fence_before();
     __syncthreads();
-    if (warp == 1) tmem_dealloc(tmem, TC_TMEM_COLS);
+    if (warp == 9) tmem_dealloc(tmem, 512);
 }
 
 template <int DK, int DV>
-static int launch_attn_tc(const void* q, const void* k_rem, const void* v_rem, const void* k, const void* v,
-                          const int* rem_base, int rem_slots, int rem_tokens, const int* types_i, const int* indices,
-                          const int* n_iters, void* o, float* lse, int B, int B_rem, int T, int Tq, int q_off, int k_split,
-                          int HQ, int HKV, int HN, int nbs, float scale, int own_chunk, cudaStream_t st) {
-    using L = TcSmem<DK, DV>;
+int launch_attn_tc(const void* q, const void* k_rem, const void* v_rem, const void* k, const void* v,
+                   const int* rem_base, int rem_slots, int rem_tokens, const int* types_i, const int* indices,
+                   const int* n_iters, void* o, float* lse, int B, int B_rem, int T, int Tq, int q_off, int k_split,
+                   int HQ, int HKV, int HN, int nbs, float scale, int own_chunk, cudaStream_t st) {
+    using L = AtSmem<DK, DV>;
     auto kern = attn_fwd_tc_kernel<DK, DV>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::total);
     if (e != cudaSuccess) {
@@ -469,16 +786,26 @@ static int launch_attn_tc(const void* q, const void* k_rem, const void* v_rem, c
     int* status = nullptr;
     if (rc == NATSL_OK) rc = status_word_ptr(&status);
     if (rc != NATSL_OK) return rc;
-    const int NTq = (Tq + ATT_BM - 1) / ATT_BM, TN = (T + nbs - 1) / nbs;
-    dim3 grid(NTq, HQ, B);
-    kern<<<grid, TC_THREADS, L::total, st>>>(mq, mk, mv, mkr, mvr, k_split, B_rem, k_split > 0 ? rem_base : nullptr,
-                                             rem_slots, types_i, indices, n_iters,
-                                             reinterpret_cast<__nv_bfloat16*>(o),
-                                             lse, T, Tq, q_off, HQ, HKV, HN, TN, nbs, scale * 1.44269504f, own_chunk,
-                                             status);
+    const int TN = (T + nbs - 1) / nbs;
+    Order od;
+    od.n_heads = HQ * B;
+    od.q_per_kv = HQ / HKV;
+    od.q_per_sel = HQ / HN;
+    od.rem_segments = k_split > 0 && rem_base ? k_split / (rem_slots * nbs) : 0;
+    // The two tiles of an item share the loads of keys and values; where all tiles together do not even fill the SMs once, each
+    // gets an SM of its own.
+    const int n_tiles = (Tq + ATT_BM - 1) / ATT_BM;
+    od.split = (long)n_tiles * od.n_heads <= AT_SMS;
+    od.n_blocks = od.split ? n_tiles : (Tq + AT_ITEM - 1) / AT_ITEM;
+    od.group = (uint32_t)std::max<long>(1, std::min<long>(od.n_heads, AT_GROUP_BYTES / ((long)T * (DK + DV) * 2)));
+    NATSL_REQUIRE((long)od.n_blocks * (long)od.n_heads <= 0x7fffffffL, NATSL_ERR_TOO_LARGE, "natsl_attn_fwd: too many query tiles");
+    kern<<<od.n_blocks * od.n_heads, AT_THREADS, L::total, st>>>(
+        mq, mk, mv, mkr, mvr, k_split, B_rem, k_split > 0 ? rem_base : nullptr, rem_slots, types_i, indices, n_iters,
+        reinterpret_cast<__nv_bfloat16*>(o), lse, T, Tq, q_off, HQ, HKV, HN, TN, nbs, scale * 1.44269504f, own_chunk, od, status);
     return check_launch("natsl_attn_fwd");
 }
 
+}  // namespace
 }  // namespace natsl
 
 extern "C" int natsl_attn_fwd_split(const void* q, const void* k_rem, const void* v_rem, const int32_t* rem_base,
@@ -516,10 +843,8 @@ extern "C" int natsl_attn_fwd_split(const void* q, const void* k_rem, const void
 #define NATSL_ATT_ARGS                                                                                                 \
     q, k_rem, v_rem, k, v, rem_base, rem_slots, rem_tokens, types_i, indices, attn_n_iters, o, lse, B, B_rem, T, Tq, q_off, \
         k_split, HQ, HKV, HN, nbs, scale, own, st
-    const bool one_item = (flags & NATSL_FLAG_ATTN_PERSISTENT) == 0;
-#define NATSL_ATT_CASE(KK, VV)                                                \
-    if (DK == KK && DV == VV)                                                 \
-        return one_item ? launch_attn_tc<KK, VV>(NATSL_ATT_ARGS) : launch_attn_tc_persist<KK, VV>(NATSL_ATT_ARGS);
+#define NATSL_ATT_CASE(KK, VV) \
+    if (DK == KK && DV == VV) return launch_attn_tc<KK, VV>(NATSL_ATT_ARGS);
     NATSL_ATT_CASE(64, 64)
     NATSL_ATT_CASE(64, 128)
     NATSL_ATT_CASE(128, 64)

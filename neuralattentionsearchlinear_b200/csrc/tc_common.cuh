@@ -69,6 +69,16 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* st
     return false;
 }
 
+// The same for kernels with many waits: a whole warp waits, and the caller records the status once, at its end.  A few
+// instructions per wait where the one above takes two dozen: code that no longer fits the instruction cache costs more than
+// the waits do.  (A try suspends the warp for some 25 us, so the limit is a few seconds.)
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity) {
+    bool done = false;
+#pragma unroll 1
+    for (int i = 0; i < (1 << 18) && !done; ++i) done = mbar_try_wait(bar, parity);
+    return __all_sync(0xffffffffu, done);
+}
+
 // ------------------------------------------------------------------ TMA
 __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, int c3,
                                             uint32_t bar) {
@@ -141,6 +151,47 @@ __device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64
         "{\n .reg .pred p, e;\n setp.ne.b32 p, %4, 0;\n elect.sync _|e, 0xffffffff;\n"
         " @e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n}\n"
         ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accum), "r"(0u)
+        : "memory");
+}
+// Four K-steps (64 elements of K) in one go, descriptors given by their low words (umma_desc_lo; the high word is that of
+// umma_desc(., ., 1024)): one election for the four, and the steps differ by constants, which the uniform datapath adds.
+// Descriptors formed anew for every product cost the issuing warp about a hundred cycles each.
+constexpr uint32_t UMMA_DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t umma_desc_lo(uint32_t saddr, uint32_t lbo_bytes) {
+    return ((saddr >> 4) & 0x3FFF) | ((lbo_bytes >> 4) << 16);
+}
+// A and B from shared memory; STEP_A / STEP_B: 16-byte units between K-steps (2 for a K-major operand, 128 for an MN-major one)
+template <int STEP_A, int STEP_B>
+__device__ __forceinline__ void umma_ss_x4(uint32_t d_tmem, uint32_t alo, uint32_t blo, uint32_t idesc, uint32_t accum) {
+    asm volatile(
+        "{\n .reg .pred p, t, e;\n .reg .b64 a, b;\n .reg .b32 x, y;\n"
+        " setp.ne.b32 p, %4, 0;\n setp.eq.u32 t, 0, 0;\n elect.sync _|e, 0xffffffff;\n"
+        " mov.b64 a, {%1, %5};\n mov.b64 b, {%2, %5};\n"
+        " @e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n"
+        " add.u32 x, %1, %6;\n add.u32 y, %2, %7;\n mov.b64 a, {x, %5};\n mov.b64 b, {y, %5};\n"
+        " @e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, t;\n"
+        " add.u32 x, x, %6;\n add.u32 y, y, %7;\n mov.b64 a, {x, %5};\n mov.b64 b, {y, %5};\n"
+        " @e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, t;\n"
+        " add.u32 x, x, %6;\n add.u32 y, y, %7;\n mov.b64 a, {x, %5};\n mov.b64 b, {y, %5};\n"
+        " @e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, t;\n}\n"
+        ::"r"(d_tmem), "r"(alo), "r"(blo), "r"(idesc), "r"(accum), "n"(UMMA_DESC_HI), "n"(STEP_A), "n"(STEP_B)
+        : "memory");
+}
+// A from tensor memory (8 columns per K-step)
+template <int STEP_B>
+__device__ __forceinline__ void umma_ts_x4(uint32_t d_tmem, uint32_t a_tmem, uint32_t blo, uint32_t idesc, uint32_t accum) {
+    asm volatile(
+        "{\n .reg .pred p, t, e;\n .reg .b64 b;\n .reg .b32 x, y;\n"
+        " setp.ne.b32 p, %4, 0;\n setp.eq.u32 t, 0, 0;\n elect.sync _|e, 0xffffffff;\n"
+        " mov.b64 b, {%2, %5};\n"
+        " @e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %3, p;\n"
+        " add.u32 x, %1, 8;\n add.u32 y, %2, %6;\n mov.b64 b, {y, %5};\n"
+        " @e tcgen05.mma.cta_group::1.kind::f16 [%0], [x], b, %3, t;\n"
+        " add.u32 x, x, 8;\n add.u32 y, y, %6;\n mov.b64 b, {y, %5};\n"
+        " @e tcgen05.mma.cta_group::1.kind::f16 [%0], [x], b, %3, t;\n"
+        " add.u32 x, x, 8;\n add.u32 y, y, %6;\n mov.b64 b, {y, %5};\n"
+        " @e tcgen05.mma.cta_group::1.kind::f16 [%0], [x], b, %3, t;\n}\n"
+        ::"r"(d_tmem), "r"(a_tmem), "r"(blo), "r"(idesc), "r"(accum), "n"(UMMA_DESC_HI), "n"(STEP_B)
         : "memory");
 }
 // mbarrier arrives once every tcgen05 operation issued so far by the elected lane has completed.
