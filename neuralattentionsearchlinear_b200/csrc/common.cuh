@@ -112,6 +112,20 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t open2(uint32_t u) {       // a pair of bf16
+    const float2 f = unpack_bf16(u);
+    return pack2(f.x, f.y);
+}
+__device__ __forceinline__ uint32_t close2(uint64_t v) {
+    float lo, hi;
+    unpack2(v, lo, hi);
+    return pack_bf16(lo, hi);
+}
 
 // ---- fragment loaders over swizzled bf16 tiles ------------------------------------
 // A fragment (16 rows x 16 k) of a row-major [rows][k] tile.

@@ -166,16 +166,29 @@ int launch_narrow(const NarrowArgs& a, int B, cudaStream_t st) {
 // Short causal convolution + SiLU of the q, k and v projections with the row norms behind it, each projection read once:
 //   lin  = conv, conv / ||conv|| (Mamba2 q, k) or conv * dt (Mamba2 v);   attn = RMS norm of conv or of the raw projection;
 //   conv = the convolution itself where the mixing weights or the softmax branch need it beside a normed copy.
-// Bandwidth: a lane owns 8 channels (16-byte accesses, 256 channels per warp) and slides over TT tokens with the next four
-// rows in flight; a norm group (a head) is 8, 16 or 32 neighbouring lanes.  The three convolutions and two norms as kernels
-// of their own took 402 us at B = 16, T = 4096, 1024 channels.  Instruction issue is close behind the bandwidth, so the
-// sigmoid's reciprocal is an approximate one with a step of Newton's iteration instead of a division (16 x 4096, 1024 channels each:
-// 510 us; 628 us with the division, 486 us without the step, whose error of 2 ulp the convolution kernel of its own has not).
-__device__ __forceinline__ float sigmoid_of(float v) {
-    const float t = __expf(-fabsf(v)), y = 1.f + t;          // y in [1, 2]: nothing overflows
-    const float r0 = __fdividef(1.f, y), r = fmaf(r0, fmaf(-y, r0, 1.f), r0);
-    return v < 0.f ? t * r : r;
+// A lane owns 4 channels (8-byte accesses, 128 channels per warp; with 8 the registers leave half the warps) and slides over
+// TT tokens with the next four rows in flight; a norm group (a head) is 16 or 32 neighbouring lanes.  The three convolutions and
+// two norms as kernels of their own took 402 us at B = 16, T = 4096, 1024 channels each.  Instruction issue is what bounds it
+// (62 % of the slots): the taps, norms and scales work on pairs of channels (two floats per instruction), the bf16 rounding of
+// the convolution is also what is stored, and tokens past the end are computed and not stored, so the four tokens of a step
+// have no branch between them.  16 x 4096 tokens, 1024 channels each: 263 us (510 us one channel at a time, 12 instead of 24
+// warps per SM).  The sigmoid's reciprocal is an approximate one with a step of Newton's iteration instead of a division:
+// without the step it is off by 2 ulp, which the convolution kernel of its own is not.
+__device__ __forceinline__ float rcp_ftz(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
 }
+__device__ __forceinline__ uint64_t silu2(uint64_t v) {
+    // (constants as immediates of scalar instructions: a pair of them would take two registers, or two moves at every use)
+    float a, b;
+    unpack2(v, a, b);
+    const float ta = __expf(-fabsf(a)), tb = __expf(-fabsf(b)), ya = 1.f + ta, yb = 1.f + tb;          // y in [1, 2]
+    const float ra = rcp_ftz(ya), rb0 = rcp_ftz(yb);
+    const uint64_t r0 = pack2(ra, rb0), r = fma2(r0, pack2(fmaf(-ya, ra, 1.f), fmaf(-yb, rb0, 1.f)), r0);
+    return mul2(v, mul2(pack2(a < 0.f ? ta : 1.f, b < 0.f ? tb : 1.f), r));
+}
+constexpr int CONV_CH = 128, CONV_CTAS = 6;                // channels of a block; blocks per SM
 struct ConvSeg {
     const bf16 *x, *w, *bias;
     bf16 *lin, *attn, *conv, *tail;
@@ -190,113 +203,142 @@ struct ConvArgs {
     float l2_eps, norm_eps;
 };
 
-__global__ void __launch_bounds__(128) conv_norm_kernel(const ConvArgs a) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, b = blockIdx.z;
-    const int si = (int)blockIdx.x >= a.seg[2].blk0 ? 2 : (int)blockIdx.x >= a.seg[1].blk0 ? 1 : 0;
-    const ConvSeg& s = a.seg[si];
-    const int D = s.D, d0 = ((int)blockIdx.x - s.blk0) * 256 + lane * 8;
-    const bool ok = d0 < D;
-    const int dd = ok ? d0 : D - 8;                        // idle lanes stay in the shuffles
-    const int t0 = ((int)blockIdx.y * 4 + warp) * a.TT, t1 = min(a.T, t0 + a.TT);
-    if (t0 >= a.T) return;
-    float w[8][4], bs[8];
+// One segment's run of tokens; ATTN and LIN are the segment's modes.
+template <int ATTN, int LIN>
+__device__ __forceinline__ void conv_run(const ConvArgs& a, const ConvSeg& s, const float* bias, int b, int d0, int t0, int t1, int lane) {
+    const int D = s.D;
+    const bool ok = d0 < D, biased = s.bias != nullptr, silu = a.silu;
+    const int dd = ok ? d0 : D - 4;                        // idle lanes stay in the shuffles
+    uint64_t w[4][2], nw[2];                               // [tap][pair of channels]
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
-        const uint2 u = *reinterpret_cast<const uint2*>(s.w + (long)(dd + c) * 4);
-        const float2 lo = unpack_bf16(u.x), hi = unpack_bf16(u.y);
-        w[c][0] = lo.x; w[c][1] = lo.y; w[c][2] = hi.x; w[c][3] = hi.y;
-        bs[c] = s.bias ? bf(s.bias, dd + c) : 0.f;
-    }
-    float nw[8];
-#pragma unroll
-    for (int c = 0; c < 8; ++c) nw[c] = s.attn_mode ? ldw(s.nw, s.nw_f32, (dd + c) & (s.attn_lanes * 8 - 1)) : 0.f;
-    const float* dt = s.lin_mode == 2 ? a.dt + (long)b * a.T * a.H + dd / s.head : nullptr;
-    const bf16* x = s.x + (long)b * a.T * D + dd;
-    const uint4 zero = make_uint4(0, 0, 0, 0);
-    auto ld = [&](int t) { return t >= 0 && t < a.T ? *reinterpret_cast<const uint4*>(x + (long)t * D) : zero; };
-    auto open = [](const uint4& v, float (&f)[8]) {
-        const uint32_t* u = reinterpret_cast<const uint32_t*>(&v);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float2 p = unpack_bf16(u[i]);
-            f[2 * i] = p.x;
-            f[2 * i + 1] = p.y;
+    for (int c = 0; c < 2; ++c) {
+        const uint2 u0 = *reinterpret_cast<const uint2*>(s.w + (long)(dd + 2 * c) * 4),
+                    u1 = *reinterpret_cast<const uint2*>(s.w + (long)(dd + 2 * c + 1) * 4);
+        const float2 a01 = unpack_bf16(u0.x), a23 = unpack_bf16(u0.y), b01 = unpack_bf16(u1.x), b23 = unpack_bf16(u1.y);
+        w[0][c] = pack2(a01.x, b01.x);
+        w[1][c] = pack2(a01.y, b01.y);
+        w[2][c] = pack2(a23.x, b23.x);
+        w[3][c] = pack2(a23.y, b23.y);
+        if (ATTN) {
+            const int i = (dd + 2 * c) & (s.attn_lanes * 4 - 1);
+            nw[c] = pack2(ldw(s.nw, s.nw_f32, i), ldw(s.nw, s.nw_f32, i + 1));
         }
+    }
+    const int lanes = ATTN ? s.attn_lanes : s.lin_lanes, lin_lanes = s.lin_lanes;
+    const float inv_n = 1.f / (lanes * 4), norm_eps = a.norm_eps, l2_eps = a.l2_eps;      // 1/n of a power of two
+    const long at = ((long)b * a.T + t0) * D + dd;
+    const bf16* x = s.x + at;                              // the token at hand
+    bf16 *lin = s.lin + at, *attn = ATTN ? s.attn + at : nullptr, *conv = s.conv ? s.conv + at : nullptr;
+    const float* dt = LIN == 2 ? a.dt + ((long)b * a.T + t0) * a.H + dd / s.head : nullptr;
+    auto ld = [&](int ahead) { return *reinterpret_cast<const uint2*>(x + (long)ahead * D); };
+    auto open = [](const uint2& v, uint64_t (&f)[2]) {
+        f[0] = open2(v.x);
+        f[1] = open2(v.y);
     };
-    float h0[8], h1[8], h2[8];                             // inputs of the three tokens before
-    open(ld(t0 - 3), h0);
-    open(ld(t0 - 2), h1);
-    open(ld(t0 - 1), h2);
-    uint4 nxt[4];
+    const uint2 zero = make_uint2(0, 0);
+    uint64_t h[3][2];                                      // inputs of the three tokens before, oldest first
 #pragma unroll
-    for (int i = 0; i < 4; ++i) nxt[i] = ld(t0 + i);
-    auto group_sum = [&](const float (&f)[8], int lanes) {
-        float ss = 0.f;
+    for (int i = 0; i < 3; ++i) open(t0 - 3 + i >= 0 ? ld(i - 3) : zero, h[i]);
+    uint2 nxt[4];
 #pragma unroll
-        for (int c = 0; c < 8; ++c) ss += f[c] * f[c];
-        for (int o = lanes >> 1; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    for (int i = 0; i < 4; ++i) nxt[i] = t0 + i < t1 ? ld(i) : zero;
+    auto group_sum = [&](const uint64_t (&f)[2], int n) {  // over n = 16 or 32 lanes
+        const uint64_t s2 = fma2(f[1], f[1], mul2(f[0], f[0]));
+        float lo, hi;
+        unpack2(s2, lo, hi);
+        float ss = lo + hi;
+        if (n > 16) ss += __shfl_xor_sync(0xffffffffu, ss, 16);
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
         return ss;
     };
-    auto st = [&](bf16* p, int t, const float (&f)[8]) {
-        if (ok) *reinterpret_cast<uint4*>(p + ((long)b * a.T + t) * D + d0) =
-            make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
-    };
+#pragma unroll 1
     for (int tb = t0; tb < t1; tb += 4) {
-        uint4 cur[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) cur[i] = nxt[i];
-        if (tb + 4 < t1)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) nxt[i] = ld(tb + 4 + i);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const int t = tb + i;
-            if (t >= t1) break;
-            float r[8], y[8];
-            open(cur[i], r);
+            const bool store = ok && tb + i < t1;
+            uint64_t r[2], y[2];
+            open(nxt[i], r);
+            nxt[i] = tb + i + 4 < t1 ? ld(4) : zero;
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                float v = bs[c];
-                v += w[c][0] * h0[c];
-                v += w[c][1] * h1[c];
-                v += w[c][2] * h2[c];
-                v += w[c][3] * r[c];
-                y[c] = rb(a.silu ? v * sigmoid_of(v) : v);
-                h0[c] = h1[c];
-                h1[c] = h2[c];
-                h2[c] = r[c];
+            for (int c = 0; c < 2; ++c) y[c] = 0;
+            if (biased) {
+#pragma unroll
+                for (int c = 0; c < 2; ++c) y[c] = *reinterpret_cast<const uint64_t*>(bias + lane * 4 + 2 * c);
             }
-            if (s.conv) st(s.conv, t, y);
-            if (s.attn_mode) {
-                float z[8];
-                const float rs = rsqrtf(group_sum(s.attn_mode == 1 ? y : r, s.attn_lanes) / (s.attn_lanes * 8) + a.norm_eps);
+            uint2 yb;
+            uint32_t* yw = reinterpret_cast<uint32_t*>(&yb);
 #pragma unroll
-                for (int c = 0; c < 8; ++c)
-                    z[c] = (s.attn_mode == 1 ? y[c] : r[c]) * rs * nw[c];
-                st(s.attn, t, z);
+            for (int c = 0; c < 2; ++c) {
+                y[c] = fma2(w[3][c], r[c], fma2(w[2][c], h[2][c], fma2(w[1][c], h[1][c], fma2(w[0][c], h[0][c], y[c]))));
+                h[0][c] = h[1][c];
+                h[1][c] = h[2][c];
+                h[2][c] = r[c];
             }
-            if (s.lin_mode == 1) {
-                const float rs = rsqrtf(group_sum(y, s.lin_lanes) + a.l2_eps);
+            if (silu) {
 #pragma unroll
-                for (int c = 0; c < 8; ++c) y[c] *= rs;
-            } else if (s.lin_mode == 2) {
-                const float d = dt[(long)t * a.H];
-#pragma unroll
-                for (int c = 0; c < 8; ++c) y[c] *= d;
+                for (int c = 0; c < 2; ++c) y[c] = silu2(y[c]);
             }
-            st(s.lin, t, y);
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                yw[c] = close2(y[c]);
+                if (ATTN == 1 || LIN) y[c] = open2(yw[c]);
+            }
+            auto put_scaled = [&](bf16* p, const uint64_t (&f)[2], float scale, bool norm) {
+                const uint64_t sc = pack2(scale, scale);
+                uint2 v;
+                uint32_t* vw = reinterpret_cast<uint32_t*>(&v);
+#pragma unroll
+                for (int c = 0; c < 2; ++c) vw[c] = close2(norm ? mul2(mul2(f[c], sc), nw[c]) : mul2(f[c], sc));
+                if (store) *reinterpret_cast<uint2*>(p) = v;
+            };
+            if (conv && store) *reinterpret_cast<uint2*>(conv) = yb;
+            if (ATTN == 1) put_scaled(attn, y, rsqrtf(group_sum(y, lanes) * inv_n + norm_eps), true);
+            if (ATTN == 2) put_scaled(attn, r, rsqrtf(group_sum(r, lanes) * inv_n + norm_eps), true);
+            if (LIN == 0 && store) *reinterpret_cast<uint2*>(lin) = yb;
+            if (LIN == 1) put_scaled(lin, y, rsqrtf(group_sum(y, lin_lanes) + l2_eps), false);
+            if (LIN == 2) put_scaled(lin, y, tb + i < t1 ? *dt : 0.f, false);
+            x += D;
+            lin += D;
+            if (ATTN) attn += D;
+            if (conv) conv += D;
+            if (LIN == 2) dt += a.H;
         }
     }
     if (s.tail && t1 == a.T && ok) {                       // the last four inputs, oldest first
+        const bf16* e = s.x + ((long)b * a.T + a.T - 4) * D + dd;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) nxt[i] = ld(a.T - 4 + i);
+        for (int i = 0; i < 4; ++i) nxt[i] = *reinterpret_cast<const uint2*>(e + (long)i * D);
         const bf16* n0 = reinterpret_cast<const bf16*>(&nxt[0]);
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-            bf16 o4[4] = {n0[c], n0[8 + c], n0[16 + c], n0[24 + c]};
+        for (int c = 0; c < 4; ++c) {
+            bf16 o4[4] = {n0[c], n0[4 + c], n0[8 + c], n0[12 + c]};
             *reinterpret_cast<uint2*>(s.tail + ((long)b * D + d0 + c) * 4) = *reinterpret_cast<const uint2*>(o4);
         }
     }
+}
+
+__global__ void __launch_bounds__(128, CONV_CTAS) conv_norm_kernel(const ConvArgs a) {
+    __shared__ __align__(16) float bias[CONV_CH];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, b = blockIdx.z;
+    const int si = (int)blockIdx.x >= a.seg[2].blk0 ? 2 : (int)blockIdx.x >= a.seg[1].blk0 ? 1 : 0;
+    const ConvSeg& s = a.seg[si];
+    const int base = ((int)blockIdx.x - s.blk0) * CONV_CH, t0 = ((int)blockIdx.y * 4 + warp) * a.TT, t1 = min(a.T, t0 + a.TT);
+    if (s.bias) {
+        bias[threadIdx.x] = base + (int)threadIdx.x < s.D ? bf(s.bias, base + threadIdx.x) : 0.f;
+        __syncthreads();
+    }
+    if (t0 >= a.T) return;
+#define NATSL_CONV(A, L) \
+    if (s.attn_mode == A && s.lin_mode == L) conv_run<A, L>(a, s, bias, b, base + lane * 4, t0, t1, lane)
+    NATSL_CONV(0, 0);
+    NATSL_CONV(1, 0);
+    NATSL_CONV(2, 0);
+    NATSL_CONV(0, 1);
+    NATSL_CONV(1, 1);
+    NATSL_CONV(2, 1);
+    NATSL_CONV(0, 2);
+#undef NATSL_CONV
 }
 
 // ------------------------------------------------------------------------------------------------ decoding state
@@ -609,8 +651,8 @@ extern "C" int natsl_layer_forward(const natsl_layer_args* args, void* stream) {
     c.dt = n.dt; c.T = a.T; c.H = a.H; c.silu = a.silu; c.l2_eps = a.l2_eps; c.norm_eps = a.norm_eps;
     bf16 *q = mb(ws + l.q), *k = mb(ws + l.k), *v = mamba ? mb(ws + l.v) : mb(a.v_attn);
     const bf16 *qa = nullptr, *q_mix = q;
-    c.seg[0] = {cb(a.q_raw), cb(a.cw_q), cb(a.cb_q), q, nullptr, nullptr, mb(a.tail_q), a.qn_w, a.qn_f32, HK, mamba ? 1 : 0, 0, a.K / 8, h.DK / 8, a.K, 0};
-    c.seg[1] = {cb(a.k_raw), cb(a.cw_k), cb(a.cb_k), k, nullptr, nullptr, mb(a.tail_k), a.kn_w, a.kn_f32, HK, mamba ? 1 : 0, 0, a.K / 8, h.DK / 8, a.K, 0};
+    c.seg[0] = {cb(a.q_raw), cb(a.cw_q), cb(a.cb_q), q, nullptr, nullptr, mb(a.tail_q), a.qn_w, a.qn_f32, HK, mamba ? 1 : 0, 0, a.K / 4, h.DK / 4, a.K, 0};
+    c.seg[1] = {cb(a.k_raw), cb(a.cw_k), cb(a.cb_k), k, nullptr, nullptr, mb(a.tail_k), a.kn_w, a.kn_f32, HK, mamba ? 1 : 0, 0, a.K / 4, h.DK / 4, a.K, 0};
     c.seg[2] = {cb(a.v_raw), cb(a.cw_v), cb(a.cb_v), v, nullptr, nullptr, mb(a.tail_v), nullptr, 0, HV, mamba ? 2 : 0, 0, 1, 1, a.V, 0};
     if (mamba) {
         c.seg[0].conv = mb(ws + l.qc);                       // the mixing weights read the query in front of its l2 norm
@@ -639,7 +681,7 @@ extern "C" int natsl_layer_forward(const natsl_layer_args* args, void* stream) {
         NATSL_REQUIRE(v, NATSL_ERR_NULL, "natsl_layer_forward: v_lin is needed beside a raw v_attn");
         c.seg[2].lin = v;
     }
-    const int kb = (HK + 255) / 256, vb = (HV + 255) / 256;
+    const int kb = (HK + CONV_CH - 1) / CONV_CH, vb = (HV + CONV_CH - 1) / CONV_CH;
     c.seg[1].blk0 = kb;
     c.seg[2].blk0 = 2 * kb;
     // tokens per warp: long runs amortise the three halo rows, short ones keep enough warps in flight (about 16 per SM)
