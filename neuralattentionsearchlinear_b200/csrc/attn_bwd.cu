@@ -100,6 +100,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         // (whose entries are masked per element)
         const int n_cand = min((q0 + ATT_BM + 63) / 64, (T + 63) / 64);
         int count = 0;
+#pragma unroll 1
         for (int base = 0; base < n_cand; base += 32) {
             const int kt = base + lane;
             const bool vis = kt < n_cand && (kt >= span0 || selp[(long)(kt / cpb) * tstride] != 0);
@@ -114,13 +115,14 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     const int n_tiles = *s_count;                             // >= 1: the own span is never empty
+    bool ok = true;
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
-        bool ok = true;
+#pragma unroll 1
         for (int j = 0; ok && j < n_tiles; ++j) {
             const int ks = j & 1, vs = j % VST, t0 = s_list[j] * 64;
-            if (j >= 2) ok = __all_sync(0xffffffffu, mbar_wait(bar_k_empty + ks * 8, ((j >> 1) - 1) & 1, status));
+            if (j >= 2) ok = warp_wait(bar_k_empty + ks * 8, ((j >> 1) - 1) & 1);
             if (!ok) break;
             if (lane == 0) {
                 mbar_expect_tx(bar_k_full + ks * 8, 64 * DK * 2);
@@ -131,7 +133,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 for (int sub = 0; sub < DV / 64; ++sub) tma_prefetch_4d(&map_v, sub * 64, hkv, t0, b);
             }
             __syncwarp();
-            if (j >= VST) ok = __all_sync(0xffffffffu, mbar_wait(bar_v_empty + vs * 8, ((j / VST) - 1) & 1, status));
+            if (j >= VST) ok = warp_wait(bar_v_empty + vs * 8, ((j / VST) - 1) & 1);
             if (!ok) break;
             if (lane == 0) {
                 mbar_expect_tx(bar_v_full + vs * 8, 64 * DV * 2);
@@ -147,51 +149,48 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         constexpr uint32_t id_dq = umma_idesc_bf16(128, DK, true);
         auto issue_s = [&](int j) {                           // S = Q K_j^T
             const uint32_t kt = s_k + (j & 1) * (64 * DK * 2);
+            const uint32_t ql = umma_desc_lo(s_q, 16), kl = umma_desc_lo(kt, 16);
 #pragma unroll
-            for (int kk = 0; kk < DK / 16; ++kk)
-                umma_ss(tmem + C_S, umma_desc(s_q + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
-                        umma_desc(kt + (kk >> 2) * 8192 + (kk & 3) * 32, 16, 1024), id_s, kk > 0);
+            for (int h = 0; h < DK / 64; ++h) umma_ss_x4<2, 2>(tmem + C_S, ql + h * 1024, kl + h * 512, id_s, h > 0);
             umma_commit(bar_s);
         };
         auto issue_dp = [&](int j) {                          // dO V_j^T
             const uint32_t vt = s_v + (j % VST) * (64 * DV * 2);
+            const uint32_t dl = umma_desc_lo(s_do, 16), vl = umma_desc_lo(vt, 16);
 #pragma unroll
-            for (int kk = 0; kk < DV / 16; ++kk)
-                umma_ss(tmem + C_DP, umma_desc(s_do + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
-                        umma_desc(vt + (kk >> 2) * 8192 + (kk & 3) * 32, 16, 1024), id_s, kk > 0);
+            for (int h = 0; h < DV / 64; ++h) umma_ss_x4<2, 2>(tmem + C_DP, dl + h * 1024, vl + h * 512, id_s, h > 0);
             umma_commit(bar_dp);
             umma_commit(bar_v_empty + (j % VST) * 8);
         };
-        bool ok = __all_sync(0xffffffffu, mbar_wait(bar_q, 0, status));
-        if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_k_full, 0, status));
+        ok = warp_wait(bar_q, 0);
+        if (ok) ok = warp_wait(bar_k_full, 0);
         if (ok) {
             tc_fence_after();
             issue_s(0);
         }
-        if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_v_full, 0, status));
+        if (ok) ok = warp_wait(bar_v_full, 0);
         if (ok) {
             tc_fence_after();
             issue_dp(0);
         }
+#pragma unroll 1
         for (int j = 0; ok && j < n_tiles; ++j) {
             const int jn = j + 1;
             if (jn < n_tiles) {                               // the next scores as soon as these have been read
-                ok = __all_sync(0xffffffffu, mbar_wait(bar_k_full + (jn & 1) * 8, (jn >> 1) & 1, status));
-                if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_s_free, j & 1, status));
+                ok = warp_wait(bar_k_full + (jn & 1) * 8, (jn >> 1) & 1);
+                if (ok) ok = warp_wait(bar_s_free, j & 1);
                 if (!ok) break;
                 tc_fence_after();
                 issue_s(jn);
             }
-            ok = __all_sync(0xffffffffu, mbar_wait(bar_ds, j & 1, status));
+            ok = warp_wait(bar_ds, j & 1);
             if (!ok) break;
             tc_fence_after();
             const uint32_t kt = s_k + (j & 1) * (64 * DK * 2);
-#pragma unroll
-            for (int kk = 0; kk < 4; ++kk)
-                umma_ts(tmem + C_DQ, tmem + C_DP + kk * 8, umma_desc(kt + kk * 2048, 8192, 1024), id_dq, (j > 0 || kk > 0) ? 1u : 0u);
+            umma_ts_x4<128>(tmem + C_DQ, tmem + C_DP, umma_desc_lo(kt, 8192), id_dq, j > 0);
             umma_commit(jn < n_tiles ? bar_k_empty + (j & 1) * 8 : bar_done);
             if (jn < n_tiles) {
-                ok = __all_sync(0xffffffffu, mbar_wait(bar_v_full + (jn % VST) * 8, (jn / VST) & 1, status));
+                ok = warp_wait(bar_v_full + (jn % VST) * 8, (jn / VST) & 1);
                 if (!ok) break;
                 tc_fence_after();
                 issue_dp(jn);                                 // behind ds k in the tensor pipe: ds may be overwritten
@@ -235,9 +234,9 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             if (t_a < T) delta_out[((long)b * T + t_a) * HQ + hq] = del_a;
             if (t_b < T) delta_out[((long)b * T + t_b) * HQ + hq] = del_b;
         }
-        bool ok = true;
+#pragma unroll 1
         for (int j = 0; j < n_tiles; ++j) {
-            ok = __all_sync(0xffffffffu, mbar_wait(bar_s, j & 1, status));
+            ok = warp_wait(bar_s, j & 1);
             if (!ok) break;
             tc_fence_after();
             uint32_t sr[32], pr[16];
@@ -271,7 +270,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
                     sr[4 * k + e] = __float_as_uint(ex2(fmaf(__uint_as_float(sr[4 * k + e]), sl2, (e >> 1) ? -lse_b : -lse_a)));
-            ok = __all_sync(0xffffffffu, mbar_wait(bar_dp, j & 1, status));
+            ok = warp_wait(bar_dp, j & 1);
             if (!ok) break;
             tc_fence_after();
             uint32_t dr[32];
@@ -290,7 +289,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_ds);
         }
-        if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_done, 0, status));
+        if (ok) ok = warp_wait(bar_done, 0);
         unsigned char* stage = smem + L::q;
         if (ok) {
             tc_fence_after();
@@ -313,6 +312,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         if (ok)
             store_tile<128, DK, 256>(stage, dq + (((long)b * T + q0) * HQ + hq) * DK, (long)HQ * DK, min(128, T - q0), tid - 64);
     }
+    if (!ok && lane == 0) atomicExch(status, NATSL_DEV_WAIT_TIMEOUT);
     tc_fence_before();
     __syncthreads();
     if (warp == 1) tmem_dealloc(tmem, TC_TMEM_COLS);
@@ -353,8 +353,10 @@ struct DkvWalk {
     }
     // moves to the first (gi, qt, u) at or after the current one; false at the end
     __device__ __forceinline__ bool settle() {
+#pragma unroll 1
         while (gi < G) {
             const int hi = max(last[gi], last[BKV_MAXG + gi]);
+#pragma unroll 1
             for (; qt <= hi; ++qt, u = 0) {
                 if (u == 0 && active(0)) return true;
                 if (u <= 1 && active(1)) {
@@ -466,6 +468,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         // tiles, the rest of the CTAs have nothing to do.
         auto selected = [&](int kt) -> bool {
             bool s = false;
+#pragma unroll 1
             for (int gi = 0; gi < G; ++gi) s |= types_i[(((long)b * TN + kt / cpb) * HN + (hkv * G + gi) / (HQ / HN)) * 2] != 0;
             return s;
         };
@@ -477,6 +480,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             kept[i] = __ballot_sync(0xffffffffu, i * 32 + lane < NT && selected(i * 32 + lane));
             n_sel += __popc(kept[i]);
         }
+#pragma unroll 1
         for (int base = KEEP * 32; base < NT; base += 32)
             n_sel += __popc(__ballot_sync(0xffffffffu, base + lane < NT && selected(base + lane)));
         const int n_pairs = (n_sel + 1) / 2;
@@ -496,12 +500,14 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
 #pragma unroll
         for (int i = 0; i < KEEP; ++i)
             if (i * 32 < NT) place(i * 32, kept[i]);
+#pragma unroll 1
         for (int base = KEEP * 32; base < NT && cnt < r0 + want; base += 32)
             place(base, __ballot_sync(0xffffffffu, base + lane < NT && selected(base + lane)));
         __syncwarp();
         if (lane == 0) *s_nsel = n_sel;
         // query tiles [first, last] of every (selected tile, head): the own block's from the keys on, the later ones if the
         // head selected the block
+#pragma unroll 1
         for (int i = lane; mine_sel && i < 2 * BKV_MAXG; i += 32) {
             const int kt = s_tile[i / BKV_MAXG], gi = i % BKV_MAXG;
             int last = -1;
@@ -532,6 +538,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
 #pragma unroll
     for (int u = 0; u < 2; ++u) w.first[u] = tile[u] < 0 ? NTq : own ? tile[u] * 64 / ATT_BM : ((tile[u] / cpb + 1) * nbs) / ATT_BM;
     auto has_items = [&](int u) -> bool {
+#pragma unroll 1
         for (int gi = 0; gi < G; ++gi)
             if (s_last[u * BKV_MAXG + gi] >= w.first[u]) return true;
         return false;
@@ -542,6 +549,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     ow.G = G;
     ow.nbs = nbs;
     ow.NTq = NTq;
+    bool ok = true;
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
@@ -562,7 +570,6 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             for (int sub = 0; sub < DV / 64; ++sub)
                 tma_load_4d(base + sub * 16384, &map_do, sub * 64, hkv * G + gi, qt * ATT_BM, b, bar_full + stg * 8);
         };
-        bool ok = true;
         int n = 0;
         if (paired) {
             if (lane == 0)
@@ -572,9 +579,10 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                         load_kv(u, tile[u], bar_kv + u * 8);
                     }
             __syncwarp();
+#pragma unroll 1
             for (bool more = w.begin(); more; more = w.next_query(), ++n) {
                 const int stg = n & 1;
-                if (n >= 2) ok = __all_sync(0xffffffffu, mbar_wait(bar_empty + stg * 8, ((n >> 1) - 1) & 1, status));
+                if (n >= 2) ok = warp_wait(bar_empty + stg * 8, ((n >> 1) - 1) & 1);
                 if (!ok) break;
                 if (lane == 0) {
                     mbar_expect_tx(bar_full + stg * 8, L::stage_bytes);
@@ -591,9 +599,10 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 __syncwarp();
             }
         } else {
+#pragma unroll 1
             for (bool more = ow.begin(); more; more = ow.next(), ++n) {
                 const int stg = n & 1;
-                if (n >= 2) ok = __all_sync(0xffffffffu, mbar_wait(bar_empty + stg * 8, ((n >> 1) - 1) & 1, status));
+                if (n >= 2) ok = warp_wait(bar_empty + stg * 8, ((n >> 1) - 1) & 1);
                 if (!ok) break;
                 if (lane == 0) {                              // every item brings its own copy of k and v
                     mbar_expect_tx(bar_full + stg * 8, L::stage_bytes + L::kv_bytes);
@@ -612,36 +621,30 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             kv = __shfl_sync(0xffffffffu, kv, 0);
             n = __shfl_sync(0xffffffffu, n, 0) & 1;
             tc_fence_after();
-            const uint32_t dos = sbase + L::stage + stg * L::stage_bytes, qs = dos + 128 * DV * 2;
-            const uint32_t kt = sbase + L::kv + kv * L::kv_bytes, vt = kt + 64 * DK * 2;
+            const uint32_t dl = umma_desc_lo(sbase + L::stage + stg * L::stage_bytes, 16), ql = dl + (128 * DV * 2 >> 4);
+            const uint32_t kl = umma_desc_lo(sbase + L::kv + kv * L::kv_bytes, 16), vl = kl + (64 * DK * 2 >> 4);
 #pragma unroll
-            for (int kk = 0; kk < DK / 16; ++kk)
-                umma_ss(tmem + C_S + n * 64, umma_desc(qs + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
-                             umma_desc(kt + (kk >> 2) * 8192 + (kk & 3) * 32, 16, 1024), id_s, kk > 0);
+            for (int h = 0; h < DK / 64; ++h) umma_ss_x4<2, 2>(tmem + C_S + n * 64, ql + h * 1024, kl + h * 512, id_s, h > 0);
 #pragma unroll
-            for (int kk = 0; kk < DV / 16; ++kk)
-                umma_ss(tmem + C_DP + n * 64, umma_desc(dos + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
-                             umma_desc(vt + (kk >> 2) * 8192 + (kk & 3) * 32, 16, 1024), id_s, kk > 0);
+            for (int h = 0; h < DV / 64; ++h) umma_ss_x4<2, 2>(tmem + C_DP + n * 64, dl + h * 1024, vl + h * 512, id_s, h > 0);
             umma_commit(bar_s + n * 8);
         };
         auto accumulate = [&](int stg, int slot, bool cont, bool release) {
             stg = __shfl_sync(0xffffffffu, stg, 0);
             slot = __shfl_sync(0xffffffffu, slot, 0);
             tc_fence_after();
-            const uint32_t dos = sbase + L::stage + stg * L::stage_bytes, qs = dos + 128 * DV * 2;
+            const uint32_t dl = umma_desc_lo(sbase + L::stage + stg * L::stage_bytes, 16384), ql = dl + (128 * DV * 2 >> 4);
+            const uint32_t pl = umma_desc_lo(sbase + L::p, 8192), dsl = umma_desc_lo(sbase + L::ds, 8192);
             const uint32_t acc = tmem + C_ACC + slot * 128;
 #pragma unroll
-            for (int kk = 0; kk < 8; ++kk)                    // dv^T += do^T p
-                umma_ss(acc, umma_desc(dos + kk * 2048, 16384, 1024), umma_desc(sbase + L::p + kk * 2048, 8192, 1024), id_acc,
-                             (cont || kk > 0) ? 1u : 0u);
+            for (int h = 0; h < 2; ++h)                       // dv^T += do^T p
+                umma_ss_x4<128, 128>(acc, dl + h * 512, pl + h * 512, id_acc, cont || h > 0);
 #pragma unroll
-            for (int kk = 0; kk < 8; ++kk)                    // dk^T += q^T ds
-                umma_ss(acc + 64, umma_desc(qs + kk * 2048, 16384, 1024), umma_desc(sbase + L::ds + kk * 2048, 8192, 1024), id_acc,
-                             (cont || kk > 0) ? 1u : 0u);
+            for (int h = 0; h < 2; ++h)                       // dk^T += q^T ds
+                umma_ss_x4<128, 128>(acc + 64, ql + h * 512, dsl + h * 512, id_acc, cont || h > 0);
             umma_commit(bar_acc);
             if (release) umma_commit(bar_empty + stg * 8);
         };
-        bool ok = true;
         if (paired) {
             DkvWalk a = w;                                    // one item ahead: scores
             bool more = w.begin(), ahead = a.begin();
@@ -650,52 +653,58 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             auto step_ahead = [&]() {
                 if (a.first_of_query()) {
                     ++nq_a;
-                    ok = __all_sync(0xffffffffu, mbar_wait(bar_full + (nq_a & 1) * 8, (nq_a >> 1) & 1, status));
+                    ok = warp_wait(bar_full + (nq_a & 1) * 8, (nq_a >> 1) & 1);
                 }
-                if (ok && !kv_seen[a.u]) ok = __all_sync(0xffffffffu, mbar_wait(bar_kv + a.u * 8, 0, status));
+                if (ok && !kv_seen[a.u]) ok = warp_wait(bar_kv + a.u * 8, 0);
                 kv_seen[a.u] = true;
                 if (ok) scores(na, nq_a & 1, a.u);
                 ++na;
                 ahead = a.next();
             };
-            if (ahead) step_ahead();
             // The scores of the next item go ahead of this item's products (their buffer was read before bar_p of item
             // i - 1) unless their tiles are still on the way: the stage that the producer fills after them is the one
-            // that these products release.
+            // that these products release.  (One place that issues scores and one that issues products: inlined at every
+            // turn of the sequence, with descriptors formed for each product, this warp had 150 KB of code.)
             auto ready = [&]() {
                 return __all_sync(0xffffffffu, !a.first_of_query() || mbar_test_wait(bar_full + ((nq_a + 1) & 1) * 8, ((nq_a + 1) >> 1) & 1));
             };
-            for (int i = 0; ok && more; ++i) {
-                const bool first = ahead && ready();
-                if (first) step_ahead();
-                if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_p, i & 1, status));
+#pragma unroll 1
+            for (int i = 0; ok && more;) {
+                if (ahead && na <= i + 1 && (na == i || ready())) {
+                    step_ahead();
+                    if (na == i + 1) continue;
+                }
+                if (ok) ok = warp_wait(bar_p, i & 1);
                 if (!ok) break;
                 if (w.first_of_query()) ++nq;
                 accumulate(nq & 1, w.u, started[w.u], w.last_of_query());
                 started[w.u] = true;
                 more = w.next();
-                if (more && !first) step_ahead();
+                ++i;
             }
         } else {
             OwnWalk a = ow;
             bool more = ow.begin(), ahead = a.begin();
             int na = 0;
             auto step_ahead = [&]() {
-                ok = __all_sync(0xffffffffu, mbar_wait(bar_full + (na & 1) * 8, (na >> 1) & 1, status));
+                ok = warp_wait(bar_full + (na & 1) * 8, (na >> 1) & 1);
                 if (ok) scores(na, na & 1, na & 1);
                 ++na;
                 ahead = a.next();
             };
-            if (ahead) step_ahead();
-            for (int i = 0; ok && more; ++i) {
-                const bool first = ahead && __all_sync(0xffffffffu, mbar_test_wait(bar_full + (na & 1) * 8, (na >> 1) & 1));
-                if (first) step_ahead();
+#pragma unroll 1
+            for (int i = 0; ok && more;) {
+                if (ahead && na <= i + 1 &&
+                    (na == i || __all_sync(0xffffffffu, mbar_test_wait(bar_full + (na & 1) * 8, (na >> 1) & 1)))) {
+                    step_ahead();
+                    if (na == i + 1) continue;
+                }
                 // the accumulators of tile u - 2 were read before the softmax warps arrived here for the item before
-                if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_p, i & 1, status));
+                if (ok) ok = warp_wait(bar_p, i & 1);
                 if (!ok) break;
                 accumulate(i & 1, ow.u & 1, !ow.first_of_tile(), true);
                 more = ow.next();
-                if (more && !first) step_ahead();
+                ++i;
             }
         }
     } else {
@@ -720,7 +729,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         // the ds of later blocks' queries to dn.  Returns once the products of the previous item have read p and ds.
         uint32_t sr[32];
         auto item_p = [&](int i, int kt, int qt, bool sel, float& dn) -> bool {
-            bool ok = __all_sync(0xffffffffu, mbar_wait(bar_s + (i & 1) * 8, (i >> 1) & 1, status));
+            bool ok = warp_wait(bar_s + (i & 1) * 8, (i >> 1) & 1);
             if (!ok) return false;
             tc_fence_after();
             uint32_t dr[32];
@@ -759,7 +768,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 sr[4 * k + 3] = pack_bf16(d2, d3);
             }
             dn += (t_a >= blk_end ? sum_a : 0.f) + (t_b >= blk_end ? sum_b : 0.f);
-            if (i > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar_acc, (i - 1) & 1, status));
+            if (i > 0) ok = warp_wait(bar_acc, (i - 1) & 1);
             return ok;
         };
         auto item_write = [&]() {
@@ -809,7 +818,6 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             store_tile<64, DK, 256>(ds_t, dk + (tok * HKV + hkv) * DK, (long)HKV * DK, n_valid, tid - 64);
             asm volatile("bar.sync 2, 256;" ::: "memory");
         };
-        bool ok = true;
         int i = 0;
         if (paired) {
             float dn[2] = {0.f, 0.f};
@@ -822,6 +830,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 }
             };
             int gi = 0;
+#pragma unroll 1
             for (bool more = w.begin(); more; more = w.next(), ++i) {
                 if (w.gi != gi) {
                     flush(gi);
@@ -841,28 +850,37 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 if (w.u) dn[1] += add; else dn[0] += add;
             }
             flush(gi);
-            if (ok && i > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar_acc, (i - 1) & 1, status));
-            finish(tile[0], 0, has_items(0), ok);
-            if (tile[1] >= 0) finish(tile[1], 1, has_items(1), ok);
+            if (ok && i > 0) ok = warp_wait(bar_acc, (i - 1) & 1);
+#pragma unroll 1
+            for (int u = 0; u < (tile[1] >= 0 ? 2 : 1); ++u) finish(s_tile[u], u, has_items(u), ok);
         } else if (!own) {
+#pragma unroll 1
             for (int u = 0; u < n_own; ++u) finish(s_tile[u], 0, false, true);
         } else {
             int done = 0;                                     // tiles written
             float unused = 0.f;
-            for (bool more = ow.begin(); more; more = ow.next(), ++i) {
-                load_rows(ow.gi, ow.qt);
-                if (ok) ok = item_p(i, s_tile[ow.u], ow.qt, false, unused);
-                if (ow.u > done) {                            // the previous item was its tile's last
+            bool more = ow.begin();
+#pragma unroll 1
+            while (true) {
+                if (more) {
+                    load_rows(ow.gi, ow.qt);
+                    if (ok) ok = item_p(i, s_tile[ow.u], ow.qt, false, unused);
+                } else if (ok) {
+                    ok = warp_wait(bar_acc, (i - 1) & 1);
+                }
+                if (!more || ow.u > done) {                   // the previous item was its tile's last
                     finish(s_tile[done], done & 1, true, ok);
                     ++done;
                 }
+                if (!more) break;
                 if (ok) item_write();
+                more = ow.next();
+                ++i;
             }
-            if (ok && i > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar_acc, (i - 1) & 1, status));
-            finish(s_tile[done], done & 1, true, ok);
         }
         asm volatile("bar.sync 1, 256;" ::: "memory");       // every softmax warp reaches it, also after a failed wait
         const int n_tiles = paired ? 2 : n_own;
+#pragma unroll 1
         for (int e = tid - 64; e < n_tiles * G; e += 256) {
             const int u = e / G, gi = e % G;
             if (s_tile[u] < 0) continue;
@@ -871,6 +889,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 paired ? ((p[0] + p[1]) + (p[2] + p[3])) + ((p[4] + p[5]) + (p[6] + p[7])) : 0.f;
         }
     }
+    if (!ok && lane == 0) atomicExch(status, NATSL_DEV_WAIT_TIMEOUT);
     tc_fence_before();
     __syncthreads();
     if (warp == 1) tmem_dealloc(tmem, 512);
