@@ -229,11 +229,9 @@ gdn_prep_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         {
             constexpr uint32_t id_1 = umma_idesc_bf16(128, 64, false);
             tc_fence_after();
+            const uint32_t l = umma_desc_lo(sbase + L::kq, 16);
 #pragma unroll
-            for (int kk = 0; kk < K / 16; ++kk) {
-                const uint64_t d = umma_desc(sbase + L::kq + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024);
-                umma_ss(tmem, d, d, id_1, kk > 0);
-            }
+            for (int h = 0; h < K / 64; ++h) umma_ss_x4<2, 2>(tmem, l + h * 1024, l + h * 1024, id_1, h > 0);
             umma_commit(bar_d1);
         }
         __syncwarp();
@@ -249,12 +247,7 @@ gdn_prep_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             }
             __syncwarp();
             tc_fence_after();
-#pragma unroll
-            for (int kk = 0; kk < 4; ++kk) {
-                const uint64_t ak = umma_desc(sbase + L::kq + kk * 2048, 16384, 1024);
-                const uint64_t bw = umma_desc(sbase + L::aiw + kk * 32, 16, 1024);
-                umma_ss(tmem + 64, ak, bw, id_2, kk > 0);
-            }
+            umma_ss_x4<128, 2>(tmem + 64, umma_desc_lo(sbase + L::kq, 16384), umma_desc_lo(sbase + L::aiw, 16), id_2, 0u);
             umma_commit(bar_d2w);
         }
         __syncwarp();
@@ -263,12 +256,7 @@ gdn_prep_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         {
             constexpr uint32_t id_2 = umma_idesc_bf16(128, 64, false) | (1u << 15);
             tc_fence_after();
-#pragma unroll
-            for (int kk = 0; kk < 4; ++kk) {
-                const uint64_t av = umma_desc(sbase + L::v + kk * 2048, 8192, 1024);
-                const uint64_t bu = umma_desc(sbase + L::aiu + kk * 32, 16, 1024);
-                umma_ss(tmem, av, bu, id_2, kk > 0);
-            }
+            umma_ss_x4<128, 2>(tmem, umma_desc_lo(sbase + L::v, 8192), umma_desc_lo(sbase + L::aiu, 16), id_2, 0u);
             umma_commit(bar_d2u);
         }
         __syncwarp();

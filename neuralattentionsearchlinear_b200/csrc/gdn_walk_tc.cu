@@ -165,12 +165,9 @@ gdn_walk_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             const uint32_t d1 = tmem + ((c & 1) ? WK_D1B : WK_D1);
             {
                 tc_fence_after();
+                const uint32_t al = umma_desc_lo(base + L::wq, 16), bl = umma_desc_lo(sbase + L::sbf, 16384);
 #pragma unroll
-                for (int kk = 0; kk < 8; ++kk) {
-                    const uint64_t ad = umma_desc(base + L::wq + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024);
-                    const uint64_t bs = umma_desc(sbase + L::sbf + kk * 2048, 16384, 1024);
-                    umma_ss(d1, ad, bs, id_1, kk > 0);
-                }
+                for (int h = 0; h < 2; ++h) umma_ss_x4<2, 128>(d1, al + h * 1024, bl + h * 512, id_1, h > 0);
                 umma_commit(bar_d1);
             }
             __syncwarp();
@@ -180,12 +177,7 @@ gdn_walk_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 // the state update first: the next chunk's products wait for it, the output does not
                 tc_fence_after();
                 if (m_sel[c]) {
-#pragma unroll
-                    for (int kk = 0; kk < 4; ++kk) {
-                        const uint64_t ak = umma_desc(base + L::k + kk * 2048, 8192, 1024);
-                        const uint64_t bv = umma_desc(sbase + L::vs + kk * 2048, 8192, 1024);
-                        umma_ss(tmem + WK_S, ak, bv, id_3, 1u);
-                    }
+                    umma_ss_x4<128, 128>(tmem + WK_S, umma_desc_lo(base + L::k, 8192), umma_desc_lo(sbase + L::vs, 8192), id_3, 1u);
                 }
                 umma_commit(bar_s3);
             }
@@ -195,12 +187,7 @@ gdn_walk_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             if (!ok) break;
             {
                 tc_fence_after();
-#pragma unroll
-                for (int kk = 0; kk < 4; ++kk) {
-                    const uint64_t ad = umma_desc(sbase + L::pp + kk * 32, 16, 1024);
-                    const uint64_t bv = umma_desc(sbase + L::vp + kk * 2048, 8192, 1024);
-                    umma_ss(tmem + WK_D2, ad, bv, id_2, kk > 0);
-                }
+                umma_ss_x4<2, 128>(tmem + WK_D2, umma_desc_lo(sbase + L::pp, 16), umma_desc_lo(sbase + L::vp, 8192), id_2, 0u);
                 umma_commit(bar_d2);
                 umma_commit(bar_pfree);
                 umma_commit(bar_empty + stg * 8);

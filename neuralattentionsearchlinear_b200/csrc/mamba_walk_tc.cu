@@ -232,12 +232,8 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 // the update of the last chunk of an unselected block would be thrown away: it is not issued
                 tc_fence_after();
                 if ((fl & MW_ACTIVE) && !(fl & MW_RESTORE)) {
-#pragma unroll
-                    for (int kk = 0; kk < 4; ++kk) {
-                        const uint64_t ak = umma_desc(base + L::a + kk * 2048, 16384, 1024);
-                        const uint64_t bv = umma_desc(sbase + L::vs + (c & 1) * 8192 + kk * 2048, 8192, 1024);
-                        umma_ss(tmem + MW_S, ak, bv, id_3, 1u);
-                    }
+                    umma_ss_x4<128, 128>(tmem + MW_S, umma_desc_lo(base + L::a, 16384),
+                                         umma_desc_lo(sbase + L::vs + (c & 1) * 8192, 8192), id_3, 1u);
                 }
                 umma_commit(bar_s3);
             }
@@ -253,11 +249,9 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             bool ok = __all_sync(0xffffffffu, mbar_wait(bar_full, 0, status));
             if (ok) {                     // q k^T of chunk 0
                 tc_fence_after();
+                const uint32_t al = umma_desc_lo(sbase + L::a, 16);          // the k operand is the first half of the same tile
 #pragma unroll
-                for (int kk = 0; kk < 8; ++kk) {
-                    const uint64_t ad = umma_desc(sbase + L::a + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024);
-                    umma_ss(tmem + MW_DP, ad, ad, id_0, kk > 0);           // the k operand is the first half of the same tile
-                }
+                for (int h = 0; h < 2; ++h) umma_ss_x4<2, 2>(tmem + MW_DP, al + h * 1024, al + h * 1024, id_0, h > 0);
                 umma_commit(bar_dp);
             }
             __syncwarp();
@@ -278,19 +272,16 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 if (ok && ahead) ok = __all_sync(0xffffffffu, mbar_wait(bar_full + nstg * 8, ((c + 1) / L::nstage) & 1, status));
                 MW_ACC(4);
                 if (ok) {
-                    // q S of this chunk and q k^T of the next one, K-step by K-step in turn
+                    // q S of this chunk and q k^T of the next one, half by half in turn
                     tc_fence_after();
                     const uint32_t d1 = tmem + ((c & 1) ? MW_D1B : MW_D1);
                     const uint32_t nbase = sbase + nstg * L::stage;
+                    const uint32_t al = umma_desc_lo(base + L::a, 16), bl = umma_desc_lo(sbase + L::sbf + cp * 16384, 16384),
+                                   nl = umma_desc_lo(nbase + L::a, 16);
 #pragma unroll
-                    for (int kk = 0; kk < 8; ++kk) {
-                        const uint64_t ad = umma_desc(base + L::a + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024);
-                        const uint64_t bs = umma_desc(sbase + L::sbf + cp * 16384 + kk * 2048, 16384, 1024);
-                        umma_ss(d1, ad, bs, id_1, kk > 0);
-                        if (ahead) {
-                            const uint64_t an = umma_desc(nbase + L::a + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024);
-                            umma_ss(tmem + (((c + 1) & 1) ? MW_DPB : MW_DP), an, an, id_0, kk > 0);
-                        }
+                    for (int h = 0; h < 2; ++h) {
+                        umma_ss_x4<2, 128>(d1, al + h * 1024, bl + h * 512, id_1, h > 0);
+                        if (ahead) umma_ss_x4<2, 2>(tmem + (((c + 1) & 1) ? MW_DPB : MW_DP), nl + h * 1024, nl + h * 1024, id_0, h > 0);
                     }
                     if (ahead) umma_commit(bar_dp + ((c + 1) & 1) * 8);
                 }
@@ -306,12 +297,7 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 if (!ok) break;
                 {
                     tc_fence_after();
-#pragma unroll
-                    for (int kk = 0; kk < 4; ++kk) {
-                        const uint64_t ad = umma_desc(sbase + L::pp + (c & 1) * 16384 + kk * 32, 16, 1024);
-                        const uint64_t bv = umma_desc(base + L::v + kk * 2048, 8192, 1024);
-                        umma_ss(tmem + MW_D2, ad, bv, id_2, kk > 0);
-                    }
+                    umma_ss_x4<2, 128>(tmem + MW_D2, umma_desc_lo(sbase + L::pp + (c & 1) * 16384, 16), umma_desc_lo(base + L::v, 8192), id_2, 0u);
                     umma_commit(bar_d2);
                 }
                 __syncwarp();

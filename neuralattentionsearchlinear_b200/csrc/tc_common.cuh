@@ -54,6 +54,7 @@ __device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
 }
 // Busy-polling variant of mbar_wait for the latency-critical hand-offs (no suspension inside the instruction).
 __device__ __forceinline__ bool mbar_spin(uint32_t bar, uint32_t parity, int* status) {
+#pragma unroll 1
     for (int i = 0; i < (1 << 26); ++i)
         if (mbar_test_wait(bar, parity)) return true;
     atomicExch(status, 1);
@@ -63,6 +64,7 @@ __device__ __forceinline__ bool mbar_spin(uint32_t bar, uint32_t parity, int* st
 // then skip their remaining work and fall through to the common teardown (never spin forever).
 constexpr int kWaitLimit = 1 << 22;
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* status) {
+#pragma unroll 1
     for (int i = 0; i < kWaitLimit; ++i)
         if (mbar_try_wait(bar, parity)) return true;
     atomicExch(status, NATSL_DEV_WAIT_TIMEOUT);
@@ -156,6 +158,8 @@ __device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64
 // Four K-steps (64 elements of K) in one go, descriptors given by their low words (umma_desc_lo; the high word is that of
 // umma_desc(., ., 1024)): one election for the four, and the steps differ by constants, which the uniform datapath adds.
 // Descriptors formed anew for every product cost the issuing warp about a hundred cycles each.
+// (With it: Mamba2 walk at T = 65536, H = 32 523 -> 434 us; at B = 8, T = 4096, H = 16, 128/128 chunk preparation 171 -> 161 us,
+// gated-delta walk 208 -> 197 us.)
 constexpr uint32_t UMMA_DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
 __device__ __forceinline__ uint32_t umma_desc_lo(uint32_t saddr, uint32_t lbo_bytes) {
     return ((saddr >> 4) & 0x3FFF) | ((lbo_bytes >> 4) << 16);
