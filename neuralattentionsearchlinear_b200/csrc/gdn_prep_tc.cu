@@ -224,7 +224,7 @@ gdn_prep_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             tma_prefetch_4d(&map_v, 64, h, t0, b);
         }
         __syncwarp();
-        mbar_wait(bar_load, 0, status);
+        mbar_wait_small(bar_load, 0, status);
         __syncwarp();
         {
             constexpr uint32_t id_1 = umma_idesc_bf16(128, 64, false);
@@ -235,7 +235,7 @@ gdn_prep_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             umma_commit(bar_d1);
         }
         __syncwarp();
-        mbar_wait(bar_ai, 0, status);
+        mbar_wait_small(bar_ai, 0, status);
         __syncwarp();
         {
             constexpr uint32_t id_2 = umma_idesc_bf16(128, 64, false) | (1u << 15);      // A MN-major (features x tokens)
@@ -251,7 +251,7 @@ gdn_prep_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             umma_commit(bar_d2w);
         }
         __syncwarp();
-        mbar_wait(bar_v, 0, status);
+        mbar_wait_small(bar_v, 0, status);
         __syncwarp();
         {
             constexpr uint32_t id_2 = umma_idesc_bf16(128, 64, false) | (1u << 15);
@@ -294,7 +294,7 @@ gdn_prep_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             if (lane < valid) gcs_out[g0] = x0;
             if (lane + 32 < valid) gcs_out[g1] = x1;
         }
-        mbar_wait(bar_load, 0, status);
+        mbar_wait_small(bar_load, 0, status);
         PT_STAMP(2);
         if (warp >= 2 && has_q) {
             // q row norms (one row per thread; the swizzle makes the 16-byte reads of eight rows conflict-free)
@@ -316,7 +316,7 @@ gdn_prep_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             s_qr[r] = rs;
             if (r < valid && qrstd_out) qrstd_out[(tok0 + r) * H + h] = rs;
         }
-        mbar_wait(bar_d1, 0, status);
+        mbar_wait_small(bar_d1, 0, status);
         tc_fence_after();
         PT_STAMP(3);
         if (warp < 2) {
@@ -447,7 +447,7 @@ gdn_prep_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             for (int x = 0; x < 8; ++x) off[x] = (uint32_t)((((cf >> 3) ^ x) << 4) + (cf & 7) * 2);
 #pragma unroll 1
             for (int arr = 0; arr < 2; ++arr) {          // 0: w, 1: u
-                mbar_wait(arr == 0 ? bar_d2w : bar_d2u, 0, status);
+                mbar_wait_small(arr == 0 ? bar_d2w : bar_d2u, 0, status);
                 tc_fence_after();
                 unsigned char* stg = smem + L::kq + sub * 16384 + (arr == 0 ? 0 : 8192);
 #pragma unroll 1

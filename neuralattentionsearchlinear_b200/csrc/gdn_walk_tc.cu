@@ -126,7 +126,7 @@ gdn_walk_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             const int stg = c & 1;
             const int t0 = c * 64;
             if (c >= 2) {
-                bool ok = mbar_wait(bar_empty + stg * 8, ((c >> 1) - 1) & 1, status);
+                bool ok = mbar_wait_small(bar_empty + stg * 8, ((c >> 1) - 1) & 1, status);
                 if (!__all_sync(0xffffffffu, ok)) break;
             }
             if (lane == 0) {
@@ -141,7 +141,7 @@ gdn_walk_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 }
             }
             if (c >= 1) {
-                bool ok = mbar_wait(bar_pfree, (c - 1) & 1, status);       // P of the previous chunk consumed
+                bool ok = mbar_wait_small(bar_pfree, (c - 1) & 1, status);       // P of the previous chunk consumed
                 if (!__all_sync(0xffffffffu, ok)) break;
             }
             if (lane == 0) {
@@ -159,8 +159,8 @@ gdn_walk_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         for (int c = 0; ok && c < NT; ++c) {
             const int stg = c & 1;
             const uint32_t base = sbase + stg * L::stage;
-            ok = __all_sync(0xffffffffu, mbar_wait(bar_full + stg * 8, (c >> 1) & 1, status));
-            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_sready, c & 1, status));
+            ok = __all_sync(0xffffffffu, mbar_wait_small(bar_full + stg * 8, (c >> 1) & 1, status));
+            if (ok) ok = __all_sync(0xffffffffu, mbar_wait_small(bar_sready, c & 1, status));
             if (!ok) break;
             const uint32_t d1 = tmem + ((c & 1) ? WK_D1B : WK_D1);
             {
@@ -171,7 +171,7 @@ gdn_walk_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 umma_commit(bar_d1);
             }
             __syncwarp();
-            ok = __all_sync(0xffffffffu, mbar_wait(bar_pv, c & 1, status));
+            ok = __all_sync(0xffffffffu, mbar_wait_small(bar_pv, c & 1, status));
             if (!ok) break;
             {
                 // the state update first: the next chunk's products wait for it, the output does not
@@ -182,8 +182,8 @@ gdn_walk_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 umma_commit(bar_s3);
             }
             __syncwarp();
-            ok = __all_sync(0xffffffffu, mbar_wait(bar_pfull, c & 1, status));
-            if (ok && c > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar_odone, (c - 1) & 1, status));   // D2 is free
+            ok = __all_sync(0xffffffffu, mbar_wait_small(bar_pfull, c & 1, status));
+            if (ok && c > 0) ok = __all_sync(0xffffffffu, mbar_wait_small(bar_odone, (c - 1) & 1, status));   // D2 is free
             if (!ok) break;
             {
                 tc_fence_after();
@@ -303,7 +303,7 @@ gdn_walk_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             // After a failed (bounded) wait the remaining work is skipped; the loop still runs to its end.
             // Every lane first sees MMA 1 of this chunk complete: it was issued behind the previous phase of the
             // "state published" barrier, so no thread can arrive on that barrier twice within one phase.
-            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_d1, c & 1, status));
+            if (ok) ok = __all_sync(0xffffffffu, mbar_wait_small(bar_d1, c & 1, status));
             if (!is_q) {
                 // ---- w lanes: v' = u - e^{carry} w S ; v'' = v' rstd_k e^{g_last - g}   (the u tile arrived with the stage)
                 if (ok) {
@@ -342,7 +342,7 @@ gdn_walk_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             // ---- every lane: publish the updated state for the next chunk (and pre-apply the next update's decay).
             // This is the serial chain of the walk; the output rows below are read after it.
             if (ok && sel) {
-                ok = __all_sync(0xffffffffu, mbar_wait(bar_s3, c & 1, status));
+                ok = __all_sync(0xffffffffu, mbar_wait_small(bar_s3, c & 1, status));
                 if (ok) {
                     tc_fence_after();
                     publish_state(next_dec(c + 1), nullptr, c < NT - 1 && starts_last(c + 1));
@@ -356,7 +356,7 @@ gdn_walk_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             if (is_q) {
                 // ---- q lanes: o = scale (rstd_q e^{g+carry} q S + P v'), off the chain (D1 is double-buffered, D2 is
                 // released by the arrival below)
-                if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_d2, c & 1, status));
+                if (ok) ok = __all_sync(0xffffffffu, mbar_wait_small(bar_d2, c & 1, status));
                 if (ok) {
                     tc_fence_after();
                     const float fq = r_cur * __expf(g_cur + carry);

@@ -190,7 +190,7 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             const int stg = c % L::nstage;
             const int t0 = c * 64;
             if (c >= L::nstage) {
-                bool ok = mbar_wait(bar_empty + stg * 8, ((c / L::nstage) - 1) & 1, status);
+                bool ok = mbar_wait_small(bar_empty + stg * 8, ((c / L::nstage) - 1) & 1, status);
                 if (!__all_sync(0xffffffffu, ok)) break;
             }
             if (lane == 0) {
@@ -222,10 +222,10 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             const uint32_t base = sbase + stg * L::stage;
             const int fl = m_fl[c];
             MW_T0();
-            ok = __all_sync(0xffffffffu, mbar_wait(bar_full + stg * 8, (c / L::nstage) & 1, status));
-            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_sready, c & 1, status));
+            ok = __all_sync(0xffffffffu, mbar_wait_small(bar_full + stg * 8, (c / L::nstage) & 1, status));
+            if (ok) ok = __all_sync(0xffffffffu, mbar_wait_small(bar_sready, c & 1, status));
             MW_ACC(0);
-            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_pv, c & 1, status));
+            if (ok) ok = __all_sync(0xffffffffu, mbar_wait_small(bar_pv, c & 1, status));
             MW_ACC(1);
             if (!ok) break;
             {
@@ -246,7 +246,7 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             constexpr uint32_t id_0 = umma_idesc_bf16(128, 64, false);                  // [0;q] k^T
             constexpr uint32_t id_1 = umma_idesc_bf16(128, 64, true);                   // [0;q] S
             constexpr uint32_t id_2 = umma_idesc_bf16(128, 64, true);                   // P v
-            bool ok = __all_sync(0xffffffffu, mbar_wait(bar_full, 0, status));
+            bool ok = __all_sync(0xffffffffu, mbar_wait_small(bar_full, 0, status));
             if (ok) {                     // q k^T of chunk 0
                 tc_fence_after();
                 const uint32_t al = umma_desc_lo(sbase + L::a, 16);          // the k operand is the first half of the same tile
@@ -263,13 +263,13 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 const int fl = m_fl[c];
                 const int cp = ncopy & 1;
                 MW_T0();
-                if (fresh) ok = __all_sync(0xffffffffu, mbar_wait(bar_cfull + cp * 8, (ncopy >> 1) & 1, status));
+                if (fresh) ok = __all_sync(0xffffffffu, mbar_wait_small(bar_cfull + cp * 8, (ncopy >> 1) & 1, status));
                 fresh = false;
                 MW_ACC(3);
                 // q k^T of the next chunk goes to the other buffer: its last reader was P of chunk c - 1, waited for
                 // before MMA 2 of that chunk
                 const bool ahead = c + 1 < NT;
-                if (ok && ahead) ok = __all_sync(0xffffffffu, mbar_wait(bar_full + nstg * 8, ((c + 1) / L::nstage) & 1, status));
+                if (ok && ahead) ok = __all_sync(0xffffffffu, mbar_wait_small(bar_full + nstg * 8, ((c + 1) / L::nstage) & 1, status));
                 MW_ACC(4);
                 if (ok) {
                     // q S of this chunk and q k^T of the next one, half by half in turn
@@ -291,8 +291,8 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                     fresh = true;
                 }
                 MW_ACC(5);
-                if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_pfull + (c & 1) * 8, (c >> 1) & 1, status));   // P of this chunk
-                if (ok && c > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar_odone, (c - 1) & 1, status));   // D2 is free
+                if (ok) ok = __all_sync(0xffffffffu, mbar_wait_small(bar_pfull + (c & 1) * 8, (c >> 1) & 1, status));   // P of this chunk
+                if (ok && c > 0) ok = __all_sync(0xffffffffu, mbar_wait_small(bar_odone, (c - 1) & 1, status));   // D2 is free
                 MW_ACC(6);
                 if (!ok) break;
                 {
@@ -332,7 +332,7 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         auto publish_state = [&](float mul, int src, const float* init_row, bool save, bool hs) {
             // copy pubs & 1: MMA 1 of the chunks that read its previous content must be complete
             if (want_o && pubs >= 2) {
-                ok = __all_sync(0xffffffffu, mbar_wait(bar_cempty + (pubs & 1) * 8, ((pubs >> 1) - 1) & 1, status));
+                ok = __all_sync(0xffffffffu, mbar_wait_small(bar_cempty + (pubs & 1) * 8, ((pubs >> 1) - 1) & 1, status));
                 if (!ok) return;
             }
             unsigned char* dst = smem + L::sbf + (pubs & 1) * 16384;
@@ -388,7 +388,7 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             MW_T0();
             // once the update of this chunk is complete, publish the state for the next chunk (and pre-apply the next
             // update's decay); after a failed (bounded) wait the remaining work is skipped
-            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_s3, c & 1, status));
+            if (ok) ok = __all_sync(0xffffffffu, mbar_wait_small(bar_s3, c & 1, status));
             if (ok) mbar_arrive(bar_empty + (c % L::nstage) * 8);       // MMA 3 is done with the k tile
             if (warp == 2) MW_ACC(8);
             if (ok && (fl & MW_ACTIVE)) {
@@ -440,7 +440,7 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         bool ok = true;
         auto stage_v = [&](int c, float gg) {             // chunk c into buffer c & 1 (the arrival follows separately)
             const int stg = c % L::nstage;
-            ok = __all_sync(0xffffffffu, mbar_wait(bar_full + stg * 8, (c / L::nstage) & 1, status));
+            ok = __all_sync(0xffffffffu, mbar_wait_small(bar_full + stg * 8, (c / L::nstage) & 1, status));
             if (!ok) return;
             const float f2 = __expf(fminf(m_gl[c] - gg, 0.f));
             const unsigned char* vt = smem + stg * L::stage + L::v;
@@ -470,7 +470,7 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             MW_T0();
             if (ok && c + 1 < NT) stage_v(c + 1, g_n1);
             if (warp == 8) MW_ACC(10);
-            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_s3, c & 1, status));
+            if (ok) ok = __all_sync(0xffffffffu, mbar_wait_small(bar_s3, c & 1, status));
             if (ok && c + 1 < NT) mbar_arrive(bar_pv);
             if (warp == 8) MW_ACC(11);
         }
@@ -489,7 +489,7 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             if (cb == 0) s_g[(c & 1) * 64 + tr] = gg;
             asm volatile("bar.sync 2, 128;" ::: "memory");
             if (warp == 6) MW_ACC(12);
-            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_dp + (c & 1) * 8, (c >> 1) & 1, status));
+            if (ok) ok = __all_sync(0xffffffffu, mbar_wait_small(bar_dp + (c & 1) * 8, (c >> 1) & 1, status));
             if (warp == 6) MW_ACC(13);
             if (!ok) return;
             tc_fence_after();
@@ -526,7 +526,7 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             if (c + 1 < NT) build_p(c + 1, g_n1);                         // runs to its barrier also after a failed wait
             MW_T0();
             // o = scale (e^{g+carry} q S + P v): MMA 2 complete means MMA 1 of the chunk is complete as well
-            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_d2, c & 1, status));
+            if (ok) ok = __all_sync(0xffffffffu, mbar_wait_small(bar_d2, c & 1, status));
             if (warp == 6) MW_ACC(15);
             if (ok) {
                 // every product that read the tile stage of this chunk, or (if an update follows) this copy of the
