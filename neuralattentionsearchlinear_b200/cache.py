@@ -24,6 +24,7 @@ from typing import List, Optional
 import torch
 
 from . import _lib
+from .nats_util import transforms_active
 
 
 _IN_PLACE = ("_state", "_state_block_start", "_g_block", "_pool_sum", "_conv_state")
@@ -47,7 +48,11 @@ def _copy(t):
 
 
 def _copy_rows(dst: torch.Tensor, src: torch.Tensor, n: int) -> None:
-    """dst[:, :n] = src[:, :n] of two [B, rows, ...] tensors, as one kernel where both are plain device memory."""
+    """dst[:, :n] = src[:, :n] of two [B, rows, ...] tensors, as one kernel where both are plain device memory and nothing
+    (a transform, a trace, a compiler) has to see the copy."""
+    if torch.compiler.is_compiling() or transforms_active():
+        dst[:, :n].copy_(src[:, :n])
+        return
     B = src.shape[0]
     row = src[0, 0].numel() * src.element_size() if src.numel() else 0
     if (n > 0 and src.is_cuda and 0 < B <= 65535 and dst.device == src.device and dst.dtype == src.dtype and src.is_contiguous()
