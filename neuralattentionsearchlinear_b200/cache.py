@@ -24,7 +24,7 @@ from typing import List, Optional
 import torch
 
 from . import _lib
-from .nats_util import transforms_active
+from .nats_util import current_stream_ptr, device_guard, transforms_active
 
 
 _IN_PLACE = ("_state", "_state_block_start", "_g_block", "_pool_sum", "_conv_state")
@@ -50,18 +50,16 @@ def _copy(t):
 def _copy_rows(dst: torch.Tensor, src: torch.Tensor, n: int) -> None:
     """dst[:, :n] = src[:, :n] of two [B, rows, ...] tensors, as one kernel where both are plain device memory and nothing
     (a transform, a trace, a compiler) has to see the copy."""
-    if torch.compiler.is_compiling() or transforms_active():
-        dst[:, :n].copy_(src[:, :n])
-        return
-    B = src.shape[0]
-    row = src[0, 0].numel() * src.element_size() if src.numel() else 0
-    if (n > 0 and src.is_cuda and 0 < B <= 65535 and dst.device == src.device and dst.dtype == src.dtype and src.is_contiguous()
-            and dst.is_contiguous() and not (torch.is_grad_enabled() and src.requires_grad) and n * row % 16 == 0
-            and dst.shape[1] * row % 16 == 0 and src.shape[1] * row % 16 == 0 and dst.data_ptr() % 16 == 0 and src.data_ptr() % 16 == 0):
-        with torch.cuda.device(src.device):
-            _lib.call("natsl_copy_batches", dst.data_ptr(), src.data_ptr(), B, n * row, dst.shape[1] * row, src.shape[1] * row,
-                      torch.cuda.current_stream(src.device).cuda_stream)
-        return
+    if (src.is_cuda and not torch.compiler.is_compiling() and not transforms_active() and n > 0 and src.numel()
+            and not (src.requires_grad and torch.is_grad_enabled()) and src.is_contiguous() and dst.is_contiguous()
+            and dst.dtype == src.dtype and dst.device == src.device):
+        B = src.shape[0]
+        from_pitch, to_pitch = src.numel() // B * src.element_size(), dst.numel() // B * dst.element_size()
+        size, to, at = from_pitch // src.shape[1] * n, dst.data_ptr(), src.data_ptr()
+        if B <= 65535 and (size | from_pitch | to_pitch | to | at) % 16 == 0:
+            with device_guard(src.device):
+                _lib.call("natsl_copy_batches", to, at, B, size, to_pitch, from_pitch, current_stream_ptr(src.device))
+            return
     dst[:, :n].copy_(src[:, :n])
 
 
