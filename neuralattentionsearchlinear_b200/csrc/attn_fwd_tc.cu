@@ -674,6 +674,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             }
             const float neg = m == -INFINITY ? 0.f : -m;
             const uint64_t sc2 = pack2(scale_log2, scale_log2), ng2 = pack2(neg, neg);
+            uint64_t ta = 0, tb = 0;                     // sums of the step: one addition to the row's sums per step, not per key
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 uint32_t pr[32];
@@ -687,8 +688,8 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                             unpack2(fma2(pack2(__uint_as_float(s2[0]), __uint_as_float(s2[1])), sc2, ng2), x0, x1);
                             x0 = ex2(x0);
                             x1 = ex2(x1);
-                            if (c & 1) l2b = add2(l2b, pack2(x0, x1));
-                            else l2a = add2(l2a, pack2(x0, x1));
+                            if (c & 1) tb = add2(tb, pack2(x0, x1));
+                            else ta = add2(ta, pack2(x0, x1));
                             pr[16 * g + c] = pack_bf16(x0, x1);
                         }
                     } else {
@@ -711,6 +712,8 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 }
             }
             if (!ok) break;
+            l2a = add2(l2a, ta);
+            l2b = add2(l2b, tb);
             if (!(f & ST_LAST)) continue;
             ok = warp_wait(bar_o + x * 8, no & 1);
             ++no;
