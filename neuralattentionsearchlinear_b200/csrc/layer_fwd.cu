@@ -684,9 +684,11 @@ extern "C" int natsl_layer_forward(const natsl_layer_args* args, void* stream) {
     const int kb = (HK + CONV_CH - 1) / CONV_CH, vb = (HV + CONV_CH - 1) / CONV_CH;
     c.seg[1].blk0 = kb;
     c.seg[2].blk0 = 2 * kb;
-    // tokens per warp: long runs amortise the three halo rows, short ones keep enough warps in flight (about 16 per SM)
-    const long rows = (long)a.B * a.T * (2 * kb + vb);
-    c.TT = rows / 64 >= 148 * 16 ? 64 : rows / 32 >= 148 * 16 ? 32 : rows / 16 >= 148 * 16 ? 16 : 8;
+    // Tokens per warp: long runs amortise the three halo rows, short ones fill the resident warps (CONV_CTAS x 4 per SM).  A run is
+    // halved below 4/3 of a full wave: 26 warps per SM are one wave and a few more, and take longer than 52 with half the tokens
+    // (layers of 4 x 1262 tokens, 2048 channels each: 363 us in whole with 64-token runs, 356 us with 32; of 4 x 1144: 334, 324 us).
+    const long rows = (long)a.B * a.T * (2 * kb + vb), full = 148l * CONV_CTAS * 4 * 4 / 3;
+    c.TT = rows / 64 >= full ? 64 : rows / 32 >= full ? 32 : rows / 16 >= full ? 16 : 8;
     conv_norm_kernel<<<dim3(2 * kb + vb, (a.T + 4 * c.TT - 1) / (4 * c.TT), a.B), 128, 0, st>>>(c);
     rc = check_launch("natsl_layer_forward (convolutions)");
     if (rc != NATSL_OK) return rc;
