@@ -681,6 +681,9 @@ extern "C" int natsl_layer_forward(const natsl_layer_args* args, void* stream) {
         NATSL_REQUIRE(v, NATSL_ERR_NULL, "natsl_layer_forward: v_lin is needed beside a raw v_attn");
         c.seg[2].lin = v;
     }
+    for (const ConvSeg& e : c.seg)                           // what conv_norm_kernel is built for
+        NATSL_REQUIRE(e.lin && e.lin_mode >= 0 && e.lin_mode <= 2 && e.attn_mode >= 0 && e.attn_mode <= (e.lin_mode == 2 ? 0 : 2),
+                      NATSL_ERR_UNSUPPORTED, "natsl_layer_forward: no convolution kernel for modes %d, %d", e.attn_mode, e.lin_mode);
     const int kb = (HK + CONV_CH - 1) / CONV_CH, vb = (HV + CONV_CH - 1) / CONV_CH;
     c.seg[1].blk0 = kb;
     c.seg[2].blk0 = 2 * kb;
