@@ -468,10 +468,11 @@ int natsl_rmsnorm_bwd(const void* s, const void* w, int w_dtype, const void* dy,
 int natsl_swiglu_fwd(const void* a, const void* b, void* y, long n, void* stream);
 int natsl_swiglu_bwd(const void* a, const void* b, const void* dy, void* da, void* db, long n, void* stream);
 
-/* Mean of x [B,T,D] over each block of nbs tokens (the last block may be shorter): y [B,cdiv(T,nbs),D].
- * Replaces: fla mean_pooling, src/nats/layers/natsl_attn_gdn.py:412-416 (src/nats/ops/utils/pooling.py:26-57). */
 /* B runs of `bytes` bytes, run b from src + b * src_pitch to dst + b * dst_pitch (all multiples of 16; no overlap). */
 int natsl_copy_batches(void* dst, const void* src, int B, int64_t bytes, int64_t dst_pitch, int64_t src_pitch, void* stream);
+
+/* Mean of x [B,T,D] over each block of nbs tokens (the last block may be shorter): y [B,cdiv(T,nbs),D].
+ * Replaces: fla mean_pooling, src/nats/layers/natsl_attn_gdn.py:412-416 (src/nats/ops/utils/pooling.py:26-57). */
 int natsl_block_mean(const void* x, void* y, int B, int T, int D, int nbs, void* stream);
 
 /* Cross entropy of bf16 logits [rows, vocab] (vocab a multiple of 8), row by row: loss_rows[r] = logsumexp(l) - l[y_r]
