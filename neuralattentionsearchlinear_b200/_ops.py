@@ -44,7 +44,7 @@ WALK_MMA_MAX_HEADS = int(os.environ.get("NATSL_WALK_MMA_MAX_HEADS", "31"))
 
 
 def _attn_flags(own_chunk: bool) -> int:
-    return (_lib.FLAG_ATTN_OWN_CHUNK if own_chunk else 0) | (_lib.FLAG_ATTN_PERSISTENT if ATTN_PERSISTENT else 0)
+    return _lib.FLAG_ATTN_OWN_CHUNK if own_chunk else 0
 
 
 def prep_entry(K: int, V: int) -> str:
@@ -280,8 +280,7 @@ def tables_from_flat(flat, B: int, TN: int, HN: int, T: int, nbs: int) -> Select
 def hybrid_options(pairs: int) -> int:
     """``options`` of the native op and layer calls for this many (batch, head) pairs of the linear branch."""
     return ((0 if PREP_TC else _lib.HYBRID_PREP_MMA) | (_lib.HYBRID_WALK_MMA if pairs <= WALK_MMA_MAX_HEADS else 0)
-            | (_lib.HYBRID_ATTN_PERSISTENT if ATTN_PERSISTENT else 0) | (_lib.HYBRID_WALK_VSPLIT if WALK_VSPLIT else 0)
-            | (0 if LINEAR_BRANCH_PRIORITY else _lib.HYBRID_PLAIN_PRIORITY))
+            | (_lib.HYBRID_WALK_VSPLIT if WALK_VSPLIT else 0) | (0 if LINEAR_BRANCH_PRIORITY else _lib.HYBRID_PLAIN_PRIORITY))
 
 
 _hybrid_ws: dict = {}

@@ -534,9 +534,7 @@ int hybrid_forward(const natsl_hybrid_args& a, void* types_raw, cudaStream_t st,
     if (rc == NATSL_OK) rc = before_attn(att);
     if (rc == NATSL_OK)
         rc = natsl_attn_fwd_ex(a.q_attn, a.k_attn, a.v_attn, a.types_i, a.indices, a.attn_n_iters, a.o_attn, a.lse, a.B, a.T, a.T, 0,
-                               a.HQ, a.HKV, a.HN, a.DK, a.DV, a.nbs, a.scale_attn,
-                               (a.own_attn ? NATSL_FLAG_ATTN_OWN_CHUNK : 0) |
-                                   ((a.options & NATSL_HYBRID_ATTN_PERSISTENT) ? NATSL_FLAG_ATTN_PERSISTENT : 0), att);
+                               a.HQ, a.HKV, a.HN, a.DK, a.DV, a.nbs, a.scale_attn, a.own_attn ? NATSL_FLAG_ATTN_OWN_CHUNK : 0, att);
     const int join = stream_after(st, side, ev[2]);          // also after an error: the side stream may hold work of this call
     return rc != NATSL_OK ? rc : join;
 }
