@@ -22,6 +22,16 @@ def _inputs(B, T, HQ, HKV, DK, DV, nbs, p, seed):
     return rnd(B, T, HQ, DK), rnd(B, T, HKV, DK), rnd(B, T, HKV, DV), types
 
 
+def _both(q, k, v, types):
+    """(o, lse, reference o, reference lse) on the CPU, blocks of 64."""
+    import neuralattentionsearchlinear_b200 as nat
+    from neuralattentionsearchlinear_b200 import _ops
+    T, scale = q.shape[1], q.shape[3] ** -0.5
+    o, lse = _ops.attn_fwd(q.cuda(), k.cuda(), v.cuda(), nat.build_selection_tables(types.cuda(), T, 64), scale, True)
+    ref = oattn.attn_sdpa(q.float(), k.float(), v.float(), oattn.attn_mask(types[..., 0], T, 64, q.shape[2], own_chunk=True), scale)
+    return o.cpu(), lse.cpu(), *ref
+
+
 def _check(q, k, v, types, nbs, own=True):
     import neuralattentionsearchlinear_b200 as nat
     from neuralattentionsearchlinear_b200 import _lib, _ops
@@ -59,6 +69,66 @@ def test_more_items_than_sms(T, DK, DV):
     tb = nat.build_selection_tables(types[5:6].cuda(), T, 64)
     one, _ = _ops.attn_fwd(q[5:6].cuda(), k[5:6].cuda(), v[5:6].cuda(), tb, DK ** -0.5, True)
     assert torch.equal(one, o[5:6])
+
+
+@pytest.mark.parametrize("nbs", [64, 128, 192, 256])
+@pytest.mark.parametrize("DK,DV", [(64, 64), (64, 128), (128, 64), (128, 128)])
+def test_one_tile_and_two_tile_items(DK, DV, nbs):
+    """Few tiles: a block of the grid is one tile; many: two tiles that share their loads.  The same bits either way."""
+    import neuralattentionsearchlinear_b200 as nat
+    from neuralattentionsearchlinear_b200 import _lib, _ops
+    q, k, v, types = (x.cuda() for x in _inputs(8, 643, 8, 4, DK, DV, nbs, 0.4, nbs))
+    o, lse = _ops.attn_fwd(q, k, v, nat.build_selection_tables(types, 643, nbs), DK ** -0.5, True)
+    for b in (0, 5):
+        few = slice(b, b + 1)
+        tb = nat.build_selection_tables(types[few].contiguous(), 643, nbs)
+        o1, lse1 = _ops.attn_fwd(q[few], k[few], v[few], tb, DK ** -0.5, True)
+        assert torch.equal(o1, o[few]) and torch.equal(lse1, lse[few])
+    assert _lib.load().natsl_device_status() == 0
+
+
+@pytest.mark.parametrize("q_off,nbs", [(128, 64), (384, 64), (384, 128), (640, 128)])
+@pytest.mark.parametrize("DK,DV", [(64, 64), (128, 128)])
+def test_window_on_an_odd_tile(q_off, nbs, DK, DV):
+    """Queries from an odd multiple of 128 on: the items do not start where those of the whole sequence do."""
+    import neuralattentionsearchlinear_b200 as nat
+    from neuralattentionsearchlinear_b200 import _ops
+    T = 900
+    q, k, v, types = _inputs(2, T, 4, 2, DK, DV, nbs, 0.5, q_off)
+    tb = nat.build_selection_tables(types.cuda(), T, nbs)
+    o, lse = _ops.attn_fwd(q[:, q_off:].contiguous().cuda(), k.cuda(), v.cuda(), tb, DK ** -0.5, True, q_off=q_off)
+    o_ref, lse_ref = oattn.attn_sdpa(q.float(), k.float(), v.float(), oattn.attn_mask(types[..., 0], T, nbs, 4, own_chunk=True), DK ** -0.5)
+    assert_close(o, o_ref[:, q_off:], 1e-2, "o_attn")
+    assert_close(lse, lse_ref[:, q_off:], 1e-2, "lse")
+
+
+@pytest.mark.parametrize("DK,DV", [(64, 64), (128, 128)])
+def test_infinite_scores(DK, DV):
+    """A key whose score is +inf for half of the rows, -inf for the others: no weight and no effect where it is -inf, NaN (as
+    softmax gives it) where it is +inf, and nothing of it where it is not visible."""
+    q, k, v, types = _inputs(1, 400, 1, 1, DK, DV, 64, 0.0, 5)
+    q[..., 0] = torch.where(torch.arange(400) % 2 == 0, 1.0, -1.0).bfloat16().view(1, 400, 1)
+    types[:, 2] = 1                                        # keys 128..191: seen by every later block
+    k[:, 130] = 0
+    k[:, 130, :, 0] = float("inf")
+    o, lse, o_ref, lse_ref = _both(q, k, v, types)
+    hit = (torch.arange(400) >= 130) & (torch.arange(400) % 2 == 0)
+    assert torch.isnan(o_ref[0, hit]).all() and torch.isnan(o[0, hit]).all()
+    assert_close(o[0, ~hit], o_ref[0, ~hit], 1e-2, "o_attn")
+    assert_close(lse[0, ~hit], lse_ref[0, ~hit], 1e-2, "lse")
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("DK,DV", [(64, 64), (128, 128)])
+def test_keys_behind_the_mask(bad, DK, DV):
+    """NaN or infinities in a key reach the rows that see it and no other: same bits as without."""
+    q, k, v, types = _inputs(1, 512, 1, 1, DK, DV, 64, 0.0, 7)
+    clean, clean_lse, _, _ = _both(q, k, v, types)
+    k[:, 70] = bad                                         # block 1, seen by the rows 70..127
+    o, lse, _, _ = _both(q, k, v, types)
+    sees = (torch.arange(512) >= 70) & (torch.arange(512) < 128)
+    assert torch.equal(o[0, ~sees], clean[0, ~sees]) and torch.equal(lse[0, ~sees], clean_lse[0, ~sees])
+    assert torch.isnan(o[0, sees]).all()
 
 
 def test_values_behind_the_mask():
