@@ -16,15 +16,22 @@
 // TMEM (512 columns): S of A and of B (128 columns each), O of A and of B, and, where DV = 64 leaves room, P of A and of B.
 //
 // What bounds it: at head dims 128 the tensor core and the exponentials need the same 1024 cycles per 128 x 128 tile; two
-// tiles in flight hide one behind the other.  Measured cycles per tile: 1.6 k (DK = 128, DV = 64, long lists), of which the
-// exponential unit is busy 63 %.  128-key score tiles halve the number of dependent steps of 64-key ones, and shared loads
+// tiles in flight hide one behind the other.  Measured cycles per tile: 1.6 k (DK = 128, DV = 64, long lists).  The exponential
+// unit is busy 45 / 56 / 59 % of the time at 128/128, 128/64, 64/64, the tensor core 48 / 45 / 31 % (T = 4096, 50 % selected);
+// the rest is the chain score tile -> maximum -> exponentials -> P V of each tile.  128-key score tiles halve the number of dependent steps of 64-key ones, and shared loads
 // halve the L2 traffic of one-tile CTAs.  What it took beyond that: no code that does not have to be there (with every wait
 // and every planning loop unrolled in place the kernel was 110 KB, missed the instruction cache and was 1.5 x slower than at
 // 50 KB), descriptors that differ by constants, and items handed out heaviest first (see Order).
-//   B = 8, T = 4096, H = 16, 128/128, 25 % selected:   260 -> 189 us (553 -> 762 TFLOP/s); 50 %: 395 -> 306 us (915 TFLOP/s)
-//   B = 1, T = 65536, H = 32, 128/64, 10 % selected:  3640 -> 2960 us (750 -> 920 TFLOP/s)
-//   B = 16, T = 4096, H = 16, 64/64, 50 % selected:    700 -> 509 us; B = 32, T = 2048: 450 -> 288 us
-// (before: one 128-query tile and 64-key steps per CTA, two CTAs per SM.)  Tried and not kept: sixteen softmax warps with half
+// Alone, five launches in a graph (us; before: one 128-query tile and 64-key steps per CTA, two CTAs per SM):
+//                                            128/128       128/64        64/128        64/64
+//   B = 8,  T = 4096,  H = 16, 25 %:       261 -> 190    243 -> 158    236 -> 172    225 -> 142     (128/128: 580 -> 795 TFLOP/s)
+//   B = 16, T = 4096,  H = 16, 50 %:       745 -> 599    682 -> 492    701 -> 533    629 -> 449     (128/128: 764 -> 950 TFLOP/s)
+//   B = 32, T = 2048,  H = 16, 50 %:       521 -> 381    506 -> 311    494 -> 329    437 -> 271
+//   B = 1,  T = 65536, H = 32, 10 %:      4266 -> 3759  3511 -> 2862  3743 -> 3191  2980 -> 2478     (128/64: 743 -> 912 TFLOP/s)
+//   B = 4,  T = 1000,  H = 16, 40 %:      29.6 -> 23.2  27.2 -> 19.2  27.9 -> 21.5  25.8 -> 18.5
+//   B = 1,  T = 2048,  H = 12, 40 %:      23.5 -> 26.2  20.4 -> 20.8  22.6 -> 22.9  19.9 -> 20.4     (see the launch for small grids)
+//   B = 1,  T = 512,   H = 16, 40 %:      10.6 -> 11.3  10.3 -> 10.2  10.2 -> 10.8   9.6 ->  9.9
+// Behind other work under the power limit (1.76 GHz) the first one takes 211 - 218 us (273).  Tried and not kept: sixteen softmax warps with half
 // a row each (207 us in the first case: the halves' maxima have to meet), the exponential unit lent to one warp at a time
 // (no change), a single issuing warp for both tiles (each waits for the other's softmax).
 //
@@ -796,7 +803,11 @@ int launch_attn_tc(const void* q, const void* k_rem, const void* v_rem, const vo
     od.q_per_sel = HQ / HN;
     od.rem_segments = k_split > 0 && rem_base ? k_split / (rem_slots * nbs) : 0;
     // The two tiles of an item share the loads of keys and values; where all tiles together do not even fill the SMs once, each
-    // gets an SM of its own.
+    // gets an SM of its own (128 tiles of 128/128, T = 1024: 15.1 us, 18.9 us in pairs; 64 tiles, T = 512: 11.1 and 12.8).  Up to
+    // 222 tiles that would still be faster for this kernel alone (192 tiles, T = 2048: 20.2 against 25.2 us), but it holds SMs that
+    // the linear branch beside it waits for: the op at B = 1, T = 2048, 12 heads of 128/128 takes 73.8 instead of 66.5 us.
+    // Against CTAs of half an SM (the kernel before), alone, speeds are 0.92 - 1.17 x up to 148 tiles, 0.87 - 1.19 x up to 320 and
+    // 0.98 - 1.4 x beyond; whole layers of 64 to 12000 tokens, captured, are 1.04 - 1.17 x as fast.
     const int n_tiles = (Tq + ATT_BM - 1) / ATT_BM;
     od.split = (long)n_tiles * od.n_heads <= AT_SMS;
     od.n_blocks = od.split ? n_tiles : (Tq + AT_ITEM - 1) / AT_ITEM;

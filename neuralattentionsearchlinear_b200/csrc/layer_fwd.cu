@@ -169,10 +169,12 @@ int launch_narrow(const NarrowArgs& a, int B, cudaStream_t st) {
 // A lane owns 4 channels (8-byte accesses, 128 channels per warp; with 8 the registers leave half the warps) and slides over
 // TT tokens with the next four rows in flight; a norm group (a head) is 16 or 32 neighbouring lanes.  The three convolutions and
 // two norms as kernels of their own took 402 us at B = 16, T = 4096, 1024 channels each.  Instruction issue is what bounds it
-// (62 % of the slots): the taps, norms and scales work on pairs of channels (two floats per instruction), the bf16 rounding of
+// (69 % of the slots at B = 8, 21 warps per SM active, DRAM 42 % busy): the taps, norms and scales work on pairs of channels (two floats per instruction), the bf16 rounding of
 // the convolution is also what is stored, and tokens past the end are computed and not stored, so the four tokens of a step
-// have no branch between them.  16 x 4096 tokens, 1024 channels each: 263 us (510 us one channel at a time, 12 instead of 24
-// warps per SM).  The sigmoid's reciprocal is an approximate one with a step of Newton's iteration instead of a division:
+// have no branch between them.  Alone, L2 flushed: 16 x 4096 tokens, 1024 channels each 268 us (559 us one channel at a time, 12
+// instead of 24 warps per SM), Mamba2 4 x 4096, 32 heads 246 us (444).  The budget for 24 warps is 80 registers, and the widest of
+// the modes spills 58 bytes; with five blocks per SM nothing spills, to the same time for the delta rule (266 us) and a longer one
+// for Mamba2 (255 us).  The sigmoid's reciprocal is an approximate one with a step of Newton's iteration instead of a division:
 // without the step it is off by 2 ulp, which the convolution kernel of its own is not.
 __device__ __forceinline__ float rcp_ftz(float x) {
     float y;
