@@ -806,8 +806,8 @@ int launch_attn_tc(const void* q, const void* k_rem, const void* v_rem, const vo
     // gets an SM of its own (128 tiles of 128/128, T = 1024: 15.1 us, 18.9 us in pairs; 64 tiles, T = 512: 11.1 and 12.8).  Up to
     // 222 tiles that would still be faster for this kernel alone (192 tiles, T = 2048: 20.2 against 25.2 us), but it holds SMs that
     // the linear branch beside it waits for: the op at B = 1, T = 2048, 12 heads of 128/128 takes 73.8 instead of 66.5 us.
-    // Against CTAs of half an SM (the kernel before), alone, speeds are 0.92 - 1.17 x up to 148 tiles, 0.87 - 1.19 x up to 320 and
-    // 0.98 - 1.4 x beyond; whole layers of 64 to 12000 tokens, captured, are 1.04 - 1.17 x as fast.
+    // Against CTAs of half an SM (the kernel before), alone, speeds are 0.92 - 1.18 x up to 148 tiles, 0.85 - 1.30 x up to 320 and
+    // 1.0 - 1.4 x beyond; whole layers of 64 to 12000 tokens, captured, are 1.04 - 1.22 x as fast.
     const int n_tiles = (Tq + ATT_BM - 1) / ATT_BM;
     od.split = (long)n_tiles * od.n_heads <= AT_SMS;
     od.n_blocks = od.split ? n_tiles : (Tq + AT_ITEM - 1) / AT_ITEM;
