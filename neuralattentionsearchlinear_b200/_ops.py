@@ -29,7 +29,7 @@ ATTN_PERSISTENT = os.environ.get("NATSL_ATTN_PERSISTENT", "0") == "1"
 
 # The linear branch (chunk preparation -> walk) runs on a high-priority stream, so that its CTAs are placed ahead of the
 # softmax branch's remaining ones whenever an SM frees up: the serial walk then starts earlier and the attention CTAs
-# fill in around it.  Measured with the step replayed from a CUDA graph: 0.621 - 0.633 ms against 0.640 - 0.644 ms
+# fill in around it.  Measured with the step replayed from a CUDA graph: 0.523 - 0.542 ms against 0.559 - 0.561 ms
 # (three runs each); NATSL_LINEAR_PRIORITY=0 puts the branch back on the caller's stream.
 LINEAR_BRANCH_PRIORITY = os.environ.get("NATSL_LINEAR_PRIORITY", "1") != "0"
 

@@ -363,8 +363,8 @@ block_rest_kernel(const float* __restrict__ g, const bf16* __restrict__ x, float
 
 // ------------------------------------------------------------------------------------------------ two streams
 // The linear branch runs on a side stream of high priority, so that its CTAs are placed ahead of the softmax branch's
-// remaining ones whenever an SM frees up: the serial walk starts earlier and the attention CTAs fill in around it (0.621 -
-// 0.633 against 0.640 - 0.644 ms for the whole op at B = 8, T = 4096, H = 16).  The caller's stream forks to it and joins
+// remaining ones whenever an SM frees up: the serial walk starts earlier and the attention CTAs fill in around it (0.523 -
+// 0.542 against 0.559 - 0.561 ms for the whole op at B = 8, T = 4096, H = 16).  The caller's stream forks to it and joins
 // again before the call returns, so every buffer may belong to the caller's stream alone.  With NATSL_HYBRID_PLAIN_PRIORITY
 // the linear branch stays on the caller's stream and the other one takes a side stream of normal priority.  Streams and events
 // belong to the calling thread (one stream of a kind per device, given back with the thread): calls of two threads do not queue behind each other,
