@@ -127,6 +127,72 @@ __device__ __forceinline__ uint32_t close2(uint64_t v) {
     return pack_bf16(lo, hi);
 }
 
+// Logistic function of a pair.  The reciprocal is an approximate one with a step of Newton's iteration (as exact as a division,
+// without its call and its branches); with exp(-|x|) its argument lies in [1, 2].
+__device__ __forceinline__ float rcp_ftz(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ uint64_t sigmoid2(uint64_t v) {
+    // (constants as immediates of scalar instructions: a pair of them would take two registers, or two moves at every use)
+    float a, b;
+    unpack2(v, a, b);
+    const float ta = __expf(-fabsf(a)), tb = __expf(-fabsf(b)), ya = 1.f + ta, yb = 1.f + tb;          // y in [1, 2]
+    const float ra = rcp_ftz(ya), rb0 = rcp_ftz(yb);
+    const uint64_t r0 = pack2(ra, rb0), r = fma2(r0, pack2(fmaf(-ya, ra, 1.f), fmaf(-yb, rb0, 1.f)), r0);
+    return mul2(pack2(a < 0.f ? ta : 1.f, b < 0.f ? tb : 1.f), r);
+}
+__device__ __forceinline__ uint64_t silu2(uint64_t v) { return mul2(v, sigmoid2(v)); }
+__device__ __forceinline__ float hsum2(uint64_t v) {
+    float lo, hi;
+    unpack2(v, lo, hi);
+    return lo + hi;
+}
+// Eight bf16 as four pairs of floats, and back.
+__device__ __forceinline__ void open8(const uint4& v, uint64_t (&f)[4]) {
+    f[0] = open2(v.x);
+    f[1] = open2(v.y);
+    f[2] = open2(v.z);
+    f[3] = open2(v.w);
+}
+__device__ __forceinline__ uint4 close8(const uint64_t (&f)[4]) { return make_uint4(close2(f[0]), close2(f[1]), close2(f[2]), close2(f[3])); }
+__device__ __forceinline__ void open8(const __nv_bfloat16* p, uint64_t (&f)[4]) { open8(*reinterpret_cast<const uint4*>(p), f); }
+// Sixteen bytes at any bf16 address; `wide` says that it is a multiple of 16 (uniform over the grid).
+__device__ __forceinline__ uint4 ld16(const __nv_bfloat16* p, bool wide) {
+    if (wide) return *reinterpret_cast<const uint4*>(p);
+    const unsigned short* h = reinterpret_cast<const unsigned short*>(p);
+    uint32_t u[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) u[i] = (uint32_t)h[2 * i] | (uint32_t)h[2 * i + 1] << 16;
+    return make_uint4(u[0], u[1], u[2], u[3]);
+}
+__device__ __forceinline__ void st16(__nv_bfloat16* p, const uint4& v, bool wide) {
+    if (wide) {
+        *reinterpret_cast<uint4*>(p) = v;
+        return;
+    }
+    unsigned short* h = reinterpret_cast<unsigned short*>(p);
+    const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        h[2 * i] = (unsigned short)u[i];
+        h[2 * i + 1] = (unsigned short)(u[i] >> 16);
+    }
+}
+// Eight neighbouring weights in fp32 or bf16 (ones where there are none).
+__device__ __forceinline__ void weights8(const void* w, bool f32, int at, uint64_t (&f)[4]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        f[i] = pack2(1.f, 1.f);
+        if (w) {
+            if (f32) f[i] = pack2(reinterpret_cast<const float*>(w)[at + 2 * i], reinterpret_cast<const float*>(w)[at + 2 * i + 1]);
+            else f[i] = pack2(__bfloat162float(reinterpret_cast<const __nv_bfloat16*>(w)[at + 2 * i]),
+                              __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(w)[at + 2 * i + 1]));
+        }
+    }
+}
+
 // ---- fragment loaders over swizzled bf16 tiles ------------------------------------
 // A fragment (16 rows x 16 k) of a row-major [rows][k] tile.
 template <int ROW_BYTES>

@@ -174,22 +174,7 @@ int launch_narrow(const NarrowArgs& a, int B, cudaStream_t st) {
 // have no branch between them.  Alone, L2 flushed: 16 x 4096 tokens, 1024 channels each 268 us (559 us one channel at a time, 12
 // instead of 24 warps per SM), Mamba2 4 x 4096, 32 heads 246 us (444).  The budget for 24 warps is 80 registers, and the widest of
 // the modes spills 58 bytes; with five blocks per SM nothing spills, to the same time for the delta rule (266 us) and a longer one
-// for Mamba2 (255 us).  The sigmoid's reciprocal is an approximate one with a step of Newton's iteration instead of a division:
-// without the step it is off by 2 ulp, which the convolution kernel of its own is not.
-__device__ __forceinline__ float rcp_ftz(float x) {
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ uint64_t silu2(uint64_t v) {
-    // (constants as immediates of scalar instructions: a pair of them would take two registers, or two moves at every use)
-    float a, b;
-    unpack2(v, a, b);
-    const float ta = __expf(-fabsf(a)), tb = __expf(-fabsf(b)), ya = 1.f + ta, yb = 1.f + tb;          // y in [1, 2]
-    const float ra = rcp_ftz(ya), rb0 = rcp_ftz(yb);
-    const uint64_t r0 = pack2(ra, rb0), r = fma2(r0, pack2(fmaf(-ya, ra, 1.f), fmaf(-yb, rb0, 1.f)), r0);
-    return mul2(v, mul2(pack2(a < 0.f ? ta : 1.f, b < 0.f ? tb : 1.f), r));
-}
+// for Mamba2 (255 us).
 constexpr int CONV_CH = 128, CONV_CTAS = 6;                // channels of a block; blocks per SM
 struct ConvSeg {
     const bf16 *x, *w, *bias;

@@ -313,73 +313,169 @@ rmsnorm_fwd_narrow_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat
 }
 
 // dx = rstd (dy w - xhat mean(dy w xhat)) (+ dadd);  dw_part [gridDim.x, D] = per-CTA sums of dy xhat.
+// A thread owns eight neighbouring features of its rows: the row, its gradient and what is added are read once, with the next
+// turn's loads in flight, and the weights and their gradients stay in registers.  Narrow rows (D <= 256): D / 8 lanes, the rows
+// of a warp side by side, no barrier.  Wide rows: D / 8 threads, 256 / (D / 8) rows of a CTA side by side, the
+// partial sums of the warps through shared memory (double-buffered: one barrier a turn); two rows deep takes 127 registers and
+// half the CTAs (127 against 121 us).  Bound by memory.  L2 flushed, against a warp per row that read it twice, one row in flight:
+// 32768 x 2048 with an added gradient 217 -> 121 us (traffic 82), 524288 x 128 137 -> 107 us (62).
+struct RmsBwd {
+    const __nv_bfloat16 *s, *dy, *dadd;
+    const void* w;
+    __nv_bfloat16* dx;
+    float* dw_part;
+    long rows;
+    float eps;
+    int w_f32, wide;                                           // wide: every tensor starts on 16 bytes
+};
+__device__ __forceinline__ void rms_sums(const uint64_t (&a)[4], const uint64_t (&g)[4], const uint64_t (&ww)[4], float& ss, float& c) {
+    uint64_t s2 = 0, c2 = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        s2 = fma2(a[i], a[i], s2);
+        c2 = fma2(mul2(g[i], ww[i]), a[i], c2);
+    }
+    ss = hsum2(s2);
+    c = hsum2(c2);
+}
+// g becomes the gradient of the row in front of the added one; ss, c are the sums over the row.
 template <int D>
-__global__ void __launch_bounds__(256)
-rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ s, const void* __restrict__ w, int w_f32,
-                   const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ dadd,
-                   __nv_bfloat16* __restrict__ dx, float* __restrict__ dw_part, long rows, float eps) {
-    constexpr int VEC = RowShape<D>::VEC, NV = RowShape<D>::NV;
-    __shared__ float s_dw[D];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float dwa[NV][VEC];
+__device__ __forceinline__ void rms_grad(const uint64_t (&a)[4], uint64_t (&g)[4], const uint64_t (&ww)[4], uint64_t (&dwa)[4], float ss, float c,
+                                         float eps, bool ok) {
+    const float rstd = rsqrtf(ss / D + eps), m = -(c * rstd / D);     // m = -mean(dy w xhat)
+    const uint64_t r2 = pack2(rstd, rstd), m2 = pack2(m, m);
 #pragma unroll
-    for (int j = 0; j < NV; ++j)
+    for (int i = 0; i < 4; ++i) {
+        const uint64_t xh = mul2(a[i], r2);
+        if (ok) dwa[i] = fma2(g[i], xh, dwa[i]);
+        g[i] = mul2(r2, fma2(xh, m2, mul2(g[i], ww[i])));
+    }
+}
+__device__ __forceinline__ void rms_store(const RmsBwd& p, long at, uint64_t (&g)[4], const uint4& add) {
+    if (p.dadd) {
+        uint64_t r[4];
+        open8(add, r);
 #pragma unroll
-        for (int e = 0; e < VEC; ++e) dwa[j][e] = 0.f;
-    for (long row = (long)blockIdx.x * 8 + warp; row < rows; row += (long)gridDim.x * 8) {
-        const __nv_bfloat16* sr = s + row * D;
-        const __nv_bfloat16* gr = dy + row * D;
-        float ss = 0.f, c = 0.f;
+        for (int i = 0; i < 4; ++i) g[i] = add2(g[i], r[i]);
+    }
+    st16(p.dx + at, close8(g), p.wide);
+}
+
+template <int D>
+__global__ void __launch_bounds__(256) rmsnorm_bwd_narrow_kernel(const RmsBwd p) {
+    constexpr int LPR = D / 8, RPW = 32 / LPR;
+    __shared__ float s_dw[8][D];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane % LPR;
+    uint64_t ww[4], dwa[4];
+    weights8(p.w, p.w_f32, sub * 8, ww);
 #pragma unroll
-        for (int j = 0; j < NV; ++j) {
-            float a[VEC], g[VEC], ww[VEC];
-            vec_load<D>(sr, lane, j, a);
-            vec_load<D>(gr, lane, j, g);
-            vec_weight<D>(w, w_f32, lane, j, ww);
+    for (int i = 0; i < 4; ++i) dwa[i] = 0;
+    const long step = (long)gridDim.x * 8 * RPW;
+    long row0 = ((long)blockIdx.x * 8 + warp) * RPW;           // the warp's first row of this turn
+    uint4 na, ng, nr = make_uint4(0, 0, 0, 0);
+    auto load = [&](long r0) {
+        const long r = r0 + lane / LPR < p.rows ? r0 + lane / LPR : p.rows - 1;      // keep every lane in the shuffles
+        const long at = r * D + sub * 8;
+        na = ld16(p.s + at, p.wide);
+        ng = ld16(p.dy + at, p.wide);
+        if (p.dadd) nr = ld16(p.dadd + at, p.wide);
+    };
+    if (row0 < p.rows) load(row0);
+    for (; row0 < p.rows; row0 += step) {
+        uint64_t a[4], g[4];
+        open8(na, a);
+        open8(ng, g);
+        const uint4 add = nr;
+        if (row0 + step < p.rows) load(row0 + step);
+        float ss, c;
+        rms_sums(a, g, ww, ss, c);
 #pragma unroll
-            for (int e = 0; e < VEC; ++e) {
-                ss += a[e] * a[e];
-                c += g[e] * ww[e] * a[e];
-            }
+        for (int o = LPR / 2; o > 0; o >>= 1) {
+            ss += __shfl_xor_sync(0xffffffffu, ss, o);
+            c += __shfl_xor_sync(0xffffffffu, c, o);
         }
+        const bool ok = row0 + lane / LPR < p.rows;
+        rms_grad<D>(a, g, ww, dwa, ss, c, p.eps, ok);
+        if (ok) rms_store(p, (row0 + lane / LPR) * D + sub * 8, g, add);
+    }
+    float o8[8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) unpack2(dwa[i], o8[2 * i], o8[2 * i + 1]);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+#pragma unroll
+        for (int o = LPR; o < 32; o <<= 1) o8[i] += __shfl_xor_sync(0xffffffffu, o8[i], o);
+        if (lane < LPR) s_dw[warp][sub * 8 + i] = o8[i];
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < D; i += 256) {
+        float s = 0.f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) s += s_dw[k][i];
+        p.dw_part[(long)blockIdx.x * D + i] = s;
+    }
+}
+
+template <int D>
+__global__ void __launch_bounds__(256, 4) rmsnorm_bwd_wide_kernel(const RmsBwd p) {
+    constexpr int TPR = D / 8, RB = 256 / TPR, W = TPR / 32;   // threads of a row; rows side by side; warps of a row
+    __shared__ float2 s_sum[2][8];
+    __shared__ float s_dw[RB > 1 ? RB * D : 1];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rb = tid / TPR, f0 = (tid % TPR) * 8;
+    uint64_t ww[4], dwa[4];
+    weights8(p.w, p.w_f32, f0, ww);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) dwa[i] = 0;
+    const long step = (long)gridDim.x * RB;
+    uint4 na, ng, nr = make_uint4(0, 0, 0, 0);
+    auto load = [&](long row0) {
+        const long at = (row0 + rb < p.rows ? row0 + rb : p.rows - 1) * D + f0;
+        na = ld16(p.s + at, p.wide);
+        ng = ld16(p.dy + at, p.wide);
+        if (p.dadd) nr = ld16(p.dadd + at, p.wide);
+    };
+    long row0 = (long)blockIdx.x * RB;
+    if (row0 < p.rows) load(row0);
+    for (int buf = 0; row0 < p.rows; row0 += step, buf ^= 1) {
+        uint64_t a[4], g[4];
+        open8(na, a);
+        open8(ng, g);
+        const uint4 add = nr;
+        float ss, c;
+        rms_sums(a, g, ww, ss, c);
         ss = warp_sum(ss);
-        const float rstd = rsqrtf(ss / D + eps);
-        c = warp_sum(c) * rstd / D;                       // mean(dy w xhat)
-#pragma unroll
-        for (int j = 0; j < NV; ++j) {
-            float a[VEC], g[VEC], ww[VEC];
-            vec_load<D>(sr, lane, j, a);
-            vec_load<D>(gr, lane, j, g);
-            vec_weight<D>(w, w_f32, lane, j, ww);
-#pragma unroll
-            for (int e = 0; e < VEC; ++e) {
-                const float xh = a[e] * rstd;
-                dwa[j][e] += g[e] * xh;
-                g[e] = rstd * (g[e] * ww[e] - xh * c);
-            }
-            if (dadd) {
-                float r[VEC];
-                vec_load<D>(dadd + row * D, lane, j, r);
-#pragma unroll
-                for (int e = 0; e < VEC; ++e) g[e] += r[e];
-            }
-            vec_store<D>(dx + row * D, lane, j, g);
-        }
-    }
-    // warps add their sums one after the other: fixed order, one row of shared memory
-    for (int wv = 0; wv < 8; ++wv) {
-        if (warp == wv) {
-#pragma unroll
-            for (int j = 0; j < NV; ++j)
-#pragma unroll
-                for (int e = 0; e < VEC; ++e) {
-                    const int col = (j * 32 + lane) * VEC + e;
-                    s_dw[col] = (wv == 0 ? 0.f : s_dw[col]) + dwa[j][e];
-                }
-        }
+        c = warp_sum(c);
+        if (lane == 0) s_sum[buf][warp] = make_float2(ss, c);
+        if (row0 + step < p.rows) load(row0 + step);
         __syncthreads();
+        ss = c = 0.f;
+#pragma unroll
+        for (int k = 0; k < W; ++k) {
+            const float2 v = s_sum[buf][rb * W + k];
+            ss += v.x;
+            c += v.y;
+        }
+        const bool ok = row0 + rb < p.rows;
+        rms_grad<D>(a, g, ww, dwa, ss, c, p.eps, ok);
+        if (ok) rms_store(p, (row0 + rb) * D + f0, g, add);
     }
-    for (int i = threadIdx.x; i < D; i += 256) dw_part[(long)blockIdx.x * D + i] = s_dw[i];
+    float o8[8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) unpack2(dwa[i], o8[2 * i], o8[2 * i + 1]);
+    if constexpr (RB == 1) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) p.dw_part[(long)blockIdx.x * D + f0 + i] = o8[i];
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) s_dw[rb * D + f0 + i] = o8[i];
+        __syncthreads();
+        for (int i = tid; i < D; i += 256) {
+            float s = 0.f;
+#pragma unroll
+            for (int k = 0; k < RB; ++k) s += s_dw[k * D + i];
+            p.dw_part[(long)blockIdx.x * D + i] = s;
+        }
+    }
 }
 
 // ------------------------------------------------------------------------------------------------ SwiGLU
@@ -414,26 +510,31 @@ swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __re
 }
 
 // ------------------------------------------------------------------------------------------------ block mean
-// y[b, c, d] = mean over the tokens of block c (the last block may be shorter); one thread = 8 channels of one block.
+// y[b, c, d] = mean over the tokens of block c (the last block may be shorter), tokens added up in their order: the selection's
+// decisions hang on the last bit.  One thread = a pair of channels of one block with MEAN_U rows in flight, so that few long blocks
+// (4 x 1030 tokens in blocks of 256: five thousand threads of eight channels) keep the memory busy too.
+constexpr int MEAN_U = 16;
 __global__ void __launch_bounds__(128)
 block_mean_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, int T, int D, int nbs, int NB) {
-    const int cg = blockIdx.x * blockDim.x + threadIdx.x;
-    if (cg * 8 >= D) return;
+    const int cp = blockIdx.x * blockDim.x + threadIdx.x;
+    if (cp * 2 >= D) return;
     const int c = blockIdx.y, b = blockIdx.z;
-    const int t0 = c * nbs, t1 = min(T, t0 + nbs);
-    float acc[8];
+    const int t0 = c * nbs, n = min(T, t0 + nbs) - t0;
+    const uint32_t* p = reinterpret_cast<const uint32_t*>(x + ((long)b * T + t0) * D) + cp;
+    const long pitch = D / 2;
+    uint64_t acc = 0;
+    int t = 0;
+    for (; t + MEAN_U <= n; t += MEAN_U) {
+        uint32_t v[MEAN_U];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) acc[e] = 0.f;
-    for (int t = t0; t < t1; ++t) {
-        float f[8];
-        ld8(x + ((long)b * T + t) * D + cg * 8, f);
+        for (int i = 0; i < MEAN_U; ++i) v[i] = p[(t + i) * pitch];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) acc[e] += f[e];
+        for (int i = 0; i < MEAN_U; ++i) acc = add2(acc, open2(v[i]));
     }
-    const float inv = 1.f / (float)(t1 - t0);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) acc[e] *= inv;
-    st8(y + ((long)b * NB + c) * D + cg * 8, acc);
+#pragma unroll 4
+    for (; t < n; ++t) acc = add2(acc, open2(p[t * pitch]));
+    const float inv = 1.f / (float)n;
+    reinterpret_cast<uint32_t*>(y + ((long)b * NB + c) * D)[cp] = close2(mul2(acc, pack2(inv, inv)));
 }
 
 static inline const __nv_bfloat16* bfc(const void* p) { return reinterpret_cast<const __nv_bfloat16*>(p); }
@@ -443,12 +544,23 @@ static inline __nv_bfloat16* bfm(void* p) { return reinterpret_cast<__nv_bfloat1
 
 using namespace natsl;
 
+// The four taps of two neighbouring channels, one pair per tap (a tap at a time they were sixteen loads of two bytes per lane,
+// which took the load unit longer than the tile).
+__device__ __forceinline__ void conv_taps(const uint4& v, uint64_t& t0, uint64_t& t1, uint64_t& t2, uint64_t& t3) {
+    const float2 a01 = unpack_bf16(v.x), a23 = unpack_bf16(v.y), b01 = unpack_bf16(v.z), b23 = unpack_bf16(v.w);
+    t0 = pack2(a01.x, b01.x);
+    t1 = pack2(a01.y, b01.y);
+    t2 = pack2(a23.x, b23.x);
+    t3 = pack2(a23.y, b23.y);
+}
+
 // Forward with the input tile staged in shared memory: one CTA = 128 channels x 64 tokens (+ 3 halo rows), every load
-// issued at once with cp.async; warp s computes the tokens 8 s .. 8 s + 7, a lane four channels.
+// issued at once with cp.async; warp s computes the tokens 8 s .. 8 s + 7, a lane four channels (two pairs).  8 x 4096 x 2048, L2
+// flushed: 104 us a channel at a time, 88 us in pairs, 78 us with the taps in two loads (traffic 41).
 constexpr int CF_TT = 64, CF_L = 32, CF_CH = 4;
 __global__ void __launch_bounds__(256)
 short_conv_fwd_tile_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
-                           const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ y, int T, int D, int silu) {
+                           const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ y, int T, int D, int silu, int wide) {
     constexpr int W = CONV_W, XR = CF_TT + W - 1, ROWB = CF_L * CF_CH * 2, CPR = ROWB / 16;
     __shared__ __align__(16) unsigned char xs[XR * ROWB];
     const int tid = threadIdx.x, lane = tid & 31, sr = tid >> 5;
@@ -463,23 +575,24 @@ short_conv_fwd_tile_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloa
         cp_async16(xs_a + r * ROWB + c * 16, ok ? (const void*)(x + ((long)b * T + t) * D + dd) : (const void*)x, ok ? 16 : 0);
     }
     cp_async_commit();
-    float wt[CF_CH][W], bs[CF_CH];
+    static_assert(CF_CH == 4, "a thread reads 8 bytes per row: two pairs of channels");
+    uint64_t wt[W][2], bs[2];                                 // [tap][pair of channels]
 #pragma unroll
-    for (int c = 0; c < CF_CH; ++c) {
-        bs[c] = (bias && ch_ok) ? __bfloat162float(bias[d0 + c]) : 0.f;
-#pragma unroll
-        for (int j = 0; j < W; ++j) wt[c][j] = ch_ok ? __bfloat162float(w[(d0 + c) * W + j]) : 0.f;
+    for (int c = 0; c < 2; ++c) {
+        const int dd = (ch_ok ? d0 : 0) + 2 * c;
+        bs[c] = bias ? pack2(__bfloat162float(bias[dd]), __bfloat162float(bias[dd + 1])) : 0;
+        conv_taps(ld16(w + dd * W, wide), wt[0][c], wt[1][c], wt[2][c], wt[3][c]);
     }
     cp_async_wait<0>();
     __syncthreads();
-    static_assert(CF_CH == 4, "a thread reads 8 bytes per row");
-    float win[W][CF_CH];
-    auto row = [&](int r, float (&f)[CF_CH]) {
+    uint64_t win[W][2];
+    auto row = [&](int r, uint64_t (&f)[2]) {
         const uint2 v = *reinterpret_cast<const uint2*>(xs + r * ROWB + lane * 8);
-        const float2 a = unpack_bf16(v.x), c = unpack_bf16(v.y);
-        f[0] = a.x; f[1] = a.y; f[2] = c.x; f[3] = c.y;
+        f[0] = open2(v.x);
+        f[1] = open2(v.y);
     };
     const int ts = sr * 8;
+    __nv_bfloat16* yp = y + ((long)b * T + t0 + ts) * D + d0;
 #pragma unroll
     for (int j = 0; j < W - 1; ++j) row(ts + j, win[j + 1]);
 #pragma unroll
@@ -487,18 +600,17 @@ short_conv_fwd_tile_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloa
 #pragma unroll
         for (int j = 0; j < W - 1; ++j)
 #pragma unroll
-            for (int c = 0; c < CF_CH; ++c) win[j][c] = win[j + 1][c];
+            for (int c = 0; c < 2; ++c) win[j][c] = win[j + 1][c];
         row(ts + i + W - 1, win[W - 1]);
-        float o[CF_CH];
+        uint64_t o[2];
 #pragma unroll
-        for (int c = 0; c < CF_CH; ++c) {
-            float a = bs[c];
+        for (int c = 0; c < 2; ++c) {
+            o[c] = bs[c];
 #pragma unroll
-            for (int j = 0; j < W; ++j) a += wt[c][j] * win[j][c];
-            o[c] = silu ? a * sigmoidf_(a) : a;
+            for (int j = 0; j < W; ++j) o[c] = fma2(wt[j][c], win[j][c], o[c]);
+            if (silu) o[c] = silu2(o[c]);
         }
-        if (ch_ok && t0 + ts + i < T)
-            *reinterpret_cast<uint2*>(y + ((long)b * T + t0 + ts + i) * D + d0) = make_uint2(pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]));
+        if (ch_ok && t0 + ts + i < T) *reinterpret_cast<uint2*>(yp + (long)i * D) = make_uint2(close2(o[0]), close2(o[1]));
     }
 }
 
@@ -509,7 +621,8 @@ extern "C" int natsl_short_conv_fwd(const void* x, const void* w, const void* bi
                   "natsl_short_conv_fwd: bad shape (D a multiple of 8)");
     NATSL_REQUIRE(W == CONV_W, NATSL_ERR_UNSUPPORTED, "natsl_short_conv_fwd: kernel size %d is not built (4)", W);
     dim3 grid((D + CF_L * CF_CH - 1) / (CF_L * CF_CH), (T + CF_TT - 1) / CF_TT, B);
-    short_conv_fwd_tile_kernel<<<grid, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(bfc(x), bfc(w), bfc(bias), bfm(y), T, D, silu);
+    short_conv_fwd_tile_kernel<<<grid, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(bfc(x), bfc(w), bfc(bias), bfm(y), T, D, silu,
+                                                                                         aligned_to(16, w));
     return check_launch("natsl_short_conv_fwd");
 }
 
@@ -519,13 +632,14 @@ extern "C" int natsl_short_conv_fwd(const void* x, const void* w, const void* bi
 // a warp (64 channels, two per lane: four would need 90 registers and leave two CTAs on an SM) slides over 16 tokens with
 // the window of x and of the pre-activation gradients in registers: each row is read and unpacked once and three of
 // nineteen gradients are computed twice.  The weight-gradient partials of the four warps of a channel group are summed in
-// shared memory in a fixed order: one partial per CTA.
+// shared memory in a fixed order: one partial per CTA.  A lane's two channels are a pair of floats.  8 x 4096 x 2048, L2 flushed:
+// 160 us a channel at a time, 141 us in pairs with the sigmoid's division taken out (traffic 61); instruction issue (72 %) bounds it.
 constexpr int CB_TT = 64, CB_CG = 32, CB_CH = 2;      // tokens per CTA, threads across channels, channels per thread
 constexpr int CB_GR = 2, CB_WT = 16;                  // channel groups per CTA, tokens per warp
 __global__ void __launch_bounds__(256, 4)
 short_conv_bwd_tile_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                            const __nv_bfloat16* __restrict__ bias, const __nv_bfloat16* __restrict__ dy,
-                           __nv_bfloat16* __restrict__ dx, float* __restrict__ dw_part, int T, int D, int silu) {
+                           __nv_bfloat16* __restrict__ dx, float* __restrict__ dw_part, int T, int D, int silu, int wide) {
     constexpr int W = CONV_W;
     constexpr int XR = CB_TT + 2 * (W - 1), YR = CB_TT + (W - 1);            // rows of the two tiles
     constexpr int ROWB = CB_GR * CB_CG * CB_CH * 2;                          // bytes per tile row
@@ -556,74 +670,59 @@ short_conv_bwd_tile_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloa
         }
         cp_async_commit();
     }
-    float wt[CB_CH][W], bs[CB_CH], dwa[CB_CH][W + 1];
+    const int dc = ch_ok ? d0 : 0;                             // a lane's two channels are one pair of floats
+    uint64_t wt[W], bs, dwa[W + 1];
+    bs = bias ? pack2(__bfloat162float(bias[dc]), __bfloat162float(bias[dc + 1])) : 0;
+    conv_taps(ld16(w + dc * W, wide), wt[0], wt[1], wt[2], wt[3]);
 #pragma unroll
-    for (int c = 0; c < CB_CH; ++c) {
-        bs[c] = (bias && ch_ok) ? __bfloat162float(bias[d0 + c]) : 0.f;
-#pragma unroll
-        for (int j = 0; j < W; ++j) wt[c][j] = ch_ok ? __bfloat162float(w[(d0 + c) * W + j]) : 0.f;
-#pragma unroll
-        for (int j = 0; j <= W; ++j) dwa[c][j] = 0.f;
-    }
+    for (int j = 0; j <= W; ++j) dwa[j] = 0;
     cp_async_wait<0>();
     __syncthreads();
-    auto row = [&](const unsigned char* tile, int r, float (&f)[CB_CH]) {
-        const float2 v = unpack_bf16(*reinterpret_cast<const uint32_t*>(tile + r * ROWB + (grp * CB_CG + lane) * 4));
-        f[0] = v.x; f[1] = v.y;
+    auto row = [&](const unsigned char* tile, int r) {
+        return open2(*reinterpret_cast<const uint32_t*>(tile + r * ROWB + (grp * CB_CG + lane) * 4));
     };
     // Step i of this warp: the pre-activation gradient of token ts + i (rows ts + i .. ts + i + 3 of the x tile are its
     // window; dy is zero outside the sequence) and, from the third step on, dx of token ts + i - 3, which needs the
     // gradients of tokens ts + i - 3 .. ts + i.  The weight gradients take the warp's own tokens only.
     const int ts = sr * CB_WT;
-    float xw[W][CB_CH], dps[W][CB_CH];
+    uint64_t xw[W], dps[W];
+    const uint64_t one = pack2(1.f, 1.f), neg = pack2(-1.f, -1.f);
 #pragma unroll
-    for (int j = 0; j < W - 1; ++j) row(xs, ts + j, xw[j]);
+    for (int j = 0; j < W - 1; ++j) xw[j] = row(xs, ts + j);
     auto step = [&](int i, bool own) {
-        row(xs, ts + i + W - 1, xw[W - 1]);
-        float g[CB_CH];
-        row(ys, ts + i, g);
+        xw[W - 1] = row(xs, ts + i + W - 1);
+        uint64_t g = row(ys, ts + i), a = bs;
 #pragma unroll
-        for (int c = 0; c < CB_CH; ++c) {
-            float a = bs[c];
-#pragma unroll
-            for (int j = 0; j < W; ++j) a += wt[c][j] * xw[j][c];
-            if (silu) {
-                const float sg = sigmoidf_(a);
-                g[c] = g[c] * sg * (1.f + a * (1.f - sg));
-            }
-            if (own) {
-#pragma unroll
-                for (int j = 0; j < W; ++j) dwa[c][j] += g[c] * xw[j][c];
-                dwa[c][W] += g[c];
-            }
-#pragma unroll
-            for (int k = 0; k < W - 1; ++k) {
-                dps[k][c] = dps[k + 1][c];
-                xw[k][c] = xw[k + 1][c];
-            }
-            dps[W - 1][c] = g[c];
+        for (int j = 0; j < W; ++j) a = fma2(wt[j], xw[j], a);
+        if (silu) {
+            const uint64_t sg = sigmoid2(a);
+            g = mul2(mul2(g, sg), fma2(a, fma2(sg, neg, one), one));
         }
+        if (own) {
+#pragma unroll
+            for (int j = 0; j < W; ++j) dwa[j] = fma2(g, xw[j], dwa[j]);
+            dwa[W] = add2(dwa[W], g);
+        }
+#pragma unroll
+        for (int k = 0; k < W - 1; ++k) {
+            dps[k] = dps[k + 1];
+            xw[k] = xw[k + 1];
+        }
+        dps[W - 1] = g;
     };
 #pragma unroll
-    for (int c = 0; c < CB_CH; ++c)
-#pragma unroll
-        for (int k = 0; k < W; ++k) dps[k][c] = 0.f;
+    for (int k = 0; k < W; ++k) dps[k] = 0;
 #pragma unroll
     for (int i = 0; i < W - 1; ++i) step(i, true);
-#pragma unroll 4
+    __nv_bfloat16* dxp = dx + ((long)b * T + t0 + ts) * D + d0;
+#pragma unroll
     for (int i = W - 1; i < CB_WT + W - 1; ++i) {
         step(i, i < CB_WT);
-        const int t = t0 + ts + i - (W - 1);
-        if (t < T && ch_ok) {
-            float o[CB_CH];
+        if (t0 + ts + i - (W - 1) < T && ch_ok) {
+            uint64_t o = mul2(wt[0], dps[W - 1]);
 #pragma unroll
-            for (int c = 0; c < CB_CH; ++c) {
-                float a = 0.f;
-#pragma unroll
-                for (int j = 0; j < W; ++j) a += wt[c][j] * dps[W - 1 - j][c];
-                o[c] = a;
-            }
-            *reinterpret_cast<uint32_t*>(dx + ((long)b * T + t) * D + d0) = pack_bf16(o[0], o[1]);
+            for (int j = 1; j < W; ++j) o = fma2(wt[j], dps[W - 1 - j], o);
+            *reinterpret_cast<uint32_t*>(dxp + (long)(i - (W - 1)) * D) = close2(o);
         }
     }
     // ---- the warps' partials -> one per CTA (fixed order)
@@ -631,18 +730,20 @@ short_conv_bwd_tile_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloa
     constexpr int NW = CB_TT / CB_WT, PER = CB_CH * (W + 1) * CB_CG;
     float* red = reinterpret_cast<float*>(smem_cb);          // [group][token warps][CB_CH * (W + 1)][32 lanes]
 #pragma unroll
-    for (int c = 0; c < CB_CH; ++c)
-#pragma unroll
-        for (int j = 0; j <= W; ++j) red[(grp * NW + sr) * PER + (c * (W + 1) + j) * CB_CG + lane] = dwa[c][j];
+    for (int j = 0; j <= W; ++j) {
+        float lo, hi;
+        unpack2(dwa[j], lo, hi);
+        red[(grp * NW + sr) * PER + j * CB_CG + lane] = lo;
+        red[(grp * NW + sr) * PER + (W + 1 + j) * CB_CG + lane] = hi;
+    }
     __syncthreads();
-    for (int e = tid; e < CB_GR * PER; e += 256) {
-        const int gr = e / PER, o = e % PER;
+    float* part = dw_part + (((long)b * gridDim.y + blockIdx.y) * D + d_cta) * (W + 1);
+    for (int e = tid; e < CB_GR * PER; e += 256) {           // in the order of the result
+        const int ch = e / (W + 1), j = e % (W + 1), gr = ch / (CB_CG * CB_CH), l = ch / CB_CH % CB_CG, c = ch % CB_CH;
         float a = 0.f;
 #pragma unroll
-        for (int k = 0; k < NW; ++k) a += red[(gr * NW + k) * PER + o];
-        const int i = o / CB_CG, cgp = o % CB_CG;
-        const int dd = d_cta + (gr * CB_CG + cgp) * CB_CH + i / (W + 1);
-        if (dd < D) dw_part[(((long)b * gridDim.y + blockIdx.y) * D + dd) * (W + 1) + i % (W + 1)] = a;
+        for (int k = 0; k < NW; ++k) a += red[(gr * NW + k) * PER + (c * (W + 1) + j) * CB_CG + l];
+        if (d_cta + ch < D) part[e] = a;
     }
 }
 
@@ -663,7 +764,7 @@ extern "C" int natsl_short_conv_bwd(const void* x, const void* w, const void* bi
         }
         dim3 grid((D + CB_GR * CB_CG * CB_CH - 1) / (CB_GR * CB_CG * CB_CH), (T + CB_TT - 1) / CB_TT, B);
         short_conv_bwd_tile_kernel<<<grid, 256, smem, reinterpret_cast<cudaStream_t>(stream)>>>(
-            bfc(x), bfc(w), bfc(bias), bfc(dy), bfm(dx), dw_part, T, D, silu);
+            bfc(x), bfc(w), bfc(bias), bfc(dy), bfm(dx), dw_part, T, D, silu, aligned_to(16, w));
         return check_launch("natsl_short_conv_bwd");
     }
     dim3 grid((groups + 127) / 128, (T + span - 1) / span, B);
@@ -674,9 +775,6 @@ extern "C" int natsl_short_conv_bwd(const void* x, const void* w, const void* bi
 
 #define NATSL_ROW_DISPATCH(CALL)                                                               \
     switch (D) {                                                                               \
-        case 64: CALL(64); break;                                                              \
-        case 128: CALL(128); break;                                                            \
-        case 256: CALL(256); break;                                                            \
         case 512: CALL(512); break;                                                            \
         case 1024: CALL(1024); break;                                                          \
         case 2048: CALL(2048); break;                                                          \
@@ -714,9 +812,18 @@ extern "C" int natsl_rmsnorm_bwd(const void* s, const void* w, int w_dtype, cons
     NATSL_REQUIRE(rows > 0 && n_part > 0, NATSL_ERR_BAD_SHAPE, "natsl_rmsnorm_bwd: empty input");
     NATSL_REQUIRE(w_dtype == NATSL_DT_BF16 || w_dtype == NATSL_DT_F32, NATSL_ERR_UNSUPPORTED, "natsl_rmsnorm_bwd: weight must be bf16 or f32");
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-#define NATSL_CALL(DD) rmsnorm_bwd_kernel<DD><<<n_part, 256, 0, st>>>(bfc(s), w, w_dtype == NATSL_DT_F32, bfc(dy), bfc(dadd), bfm(dx), dw_part, rows, eps)
-    NATSL_ROW_DISPATCH(NATSL_CALL)
-#undef NATSL_CALL
+    const RmsBwd p = {bfc(s), bfc(dy), bfc(dadd), w, bfm(dx), dw_part, rows, eps, w_dtype == NATSL_DT_F32, aligned_to(16, s, dy, dadd, dx)};
+    switch (D) {
+        case 64: rmsnorm_bwd_narrow_kernel<64><<<n_part, 256, 0, st>>>(p); break;
+        case 128: rmsnorm_bwd_narrow_kernel<128><<<n_part, 256, 0, st>>>(p); break;
+        case 256: rmsnorm_bwd_narrow_kernel<256><<<n_part, 256, 0, st>>>(p); break;
+        case 512: rmsnorm_bwd_wide_kernel<512><<<n_part, 256, 0, st>>>(p); break;
+        case 1024: rmsnorm_bwd_wide_kernel<1024><<<n_part, 256, 0, st>>>(p); break;
+        case 2048: rmsnorm_bwd_wide_kernel<2048><<<n_part, 256, 0, st>>>(p); break;
+        default:
+            set_error("unsupported row width D=%d (64, 128, 256, 512, 1024 or 2048)", D);
+            return NATSL_ERR_UNSUPPORTED;
+    }
     return check_launch("natsl_rmsnorm_bwd");
 }
 
@@ -744,7 +851,7 @@ extern "C" int natsl_block_mean(const void* x, void* y, int B, int T, int D, int
                   "natsl_block_mean: bad shape (D a multiple of 8)");
     const int NB = (T + nbs - 1) / nbs;
     NATSL_REQUIRE(NB <= 65535, NATSL_ERR_TOO_LARGE, "natsl_block_mean: too many blocks");
-    dim3 grid((D / 8 + 127) / 128, NB, B);
+    dim3 grid((D / 2 + 127) / 128, NB, B);
     block_mean_kernel<<<grid, 128, 0, reinterpret_cast<cudaStream_t>(stream)>>>(bfc(x), bfm(y), T, D, nbs, NB);
     return check_launch("natsl_block_mean");
 }

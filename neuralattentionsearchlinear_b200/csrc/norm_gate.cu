@@ -8,149 +8,167 @@
 
 namespace natsl {
 
+constexpr long NORM_GATE_GRID = 148 * 8;
+
 __device__ __forceinline__ float load_scalar(const void* p, int dtype, long i) {
     return dtype == NATSL_DT_F32 ? reinterpret_cast<const float*>(p)[i]
                                  : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p)[i]);
 }
 
-// D / 8 lanes per row with 16 bytes each (32 / (D / 8) rows per warp): one pass, the three rows in registers.
+// Rows a warp has in flight: D / 8 lanes per row with 16 bytes each, 32 / (D / 8) rows side by side.
+template <int D>
+struct MixShape {
+    static constexpr int LPR = D / 8, RPW = 32 / LPR;
+};
+template <int LPR>
+__device__ __forceinline__ float row_sum(float v) {
+#pragma unroll
+    for (int o = LPR / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// One pass with the rows in registers.  Bandwidth once the arithmetic is out of the way: pairs of features (two floats per
+// instruction), weights kept in registers over all rows of a warp, no division.  524288 x 128, L2 flushed: 129 -> 113 us (traffic 82).
 template <int D>
 __global__ void __launch_bounds__(256)
 norm_gate_mix_kernel(const __nv_bfloat16* __restrict__ x1, const __nv_bfloat16* __restrict__ x2,
                      const __nv_bfloat16* __restrict__ g, const void* __restrict__ xw, int xw_dtype,
                      const void* __restrict__ w1, const void* __restrict__ w2, int w_dtype,
                      __nv_bfloat16* __restrict__ y, long rows, float eps, int activation) {
-    constexpr int LPR = D / 8, RPW = 32 / LPR;
+    constexpr int LPR = MixShape<D>::LPR, RPW = MixShape<D>::RPW;
     const int lane = threadIdx.x & 31, sub = lane % LPR;
-    const long row_raw = ((long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * RPW + lane / LPR;
-    const bool ok = row_raw < rows;
-    const long row = ok ? row_raw : rows - 1;                 // keep every lane in the shuffles
-    const long base = row * D + sub * 8;
-    float a[8], b[8], gg[8];
-    auto load = [&](const __nv_bfloat16* p, float* out) {
-        const uint4 v = *reinterpret_cast<const uint4*>(p + base);
-        const uint32_t* u = reinterpret_cast<const uint32_t*>(&v);
+    uint64_t p1[4], p2[4];
+    weights8(w1, w_dtype == NATSL_DT_F32, sub * 8, p1);
+    weights8(w2, w_dtype == NATSL_DT_F32, sub * 8, p2);
+    for (long row0 = ((long)blockIdx.x * 8 + (threadIdx.x >> 5)) * RPW; row0 < rows; row0 += (long)gridDim.x * 8 * RPW) {
+        const bool ok = row0 + lane / LPR < rows;
+        const long row = ok ? row0 + lane / LPR : rows - 1;   // keep every lane in the shuffles
+        const long base = row * D + sub * 8;
+        const uint4 ua = *reinterpret_cast<const uint4*>(x1 + base), ub = *reinterpret_cast<const uint4*>(x2 + base),
+                    ug = *reinterpret_cast<const uint4*>(g + base);
+        float m1 = 1.f, m2 = 1.f;
+        if (xw) { m1 = load_scalar(xw, xw_dtype, row * 2); m2 = load_scalar(xw, xw_dtype, row * 2 + 1); }
+        uint64_t a[4], b[4], gg[4], q1 = 0, q2 = 0;
+        open8(ua, a);
+        open8(ub, b);
+        open8(ug, gg);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) { float2 f = unpack_bf16(u[i]); out[2 * i] = f.x; out[2 * i + 1] = f.y; }
-    };
-    load(x1, a);
-    load(x2, b);
-    load(g, gg);
-    float s1 = 0.f, s2 = 0.f;
+        for (int i = 0; i < 4; ++i) { q1 = fma2(a[i], a[i], q1); q2 = fma2(b[i], b[i], q2); }
+        const float s1 = row_sum<LPR>(hsum2(q1)), s2 = row_sum<LPR>(hsum2(q2));
+        const float r1 = rsqrtf(s1 / D + eps) * m1, r2 = rsqrtf(s2 / D + eps) * m2;
+        const uint64_t f1 = pack2(r1, r1), f2 = pack2(r2, r2);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) { s1 += a[i] * a[i]; s2 += b[i] * b[i]; }
-#pragma unroll
-    for (int o = LPR / 2; o > 0; o >>= 1) {
-        s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-        s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+        for (int i = 0; i < 4; ++i) {
+            const uint64_t v = fma2(mul2(a[i], p1[i]), f1, mul2(mul2(b[i], p2[i]), f2)), sg = sigmoid2(gg[i]);
+            a[i] = mul2(v, activation == 1 ? sg : mul2(gg[i], sg));
+        }
+        if (ok) *reinterpret_cast<uint4*>(y + base) = close8(a);
     }
-    const float r1 = rsqrtf(s1 / D + eps), r2 = rsqrtf(s2 / D + eps);
-    float m1 = 1.f, m2 = 1.f;
-    if (xw) { m1 = load_scalar(xw, xw_dtype, row * 2); m2 = load_scalar(xw, xw_dtype, row * 2 + 1); }
-    float out[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int d = sub * 8 + i;
-        const float ww1 = w1 ? load_scalar(w1, w_dtype, d) : 1.f, ww2 = w2 ? load_scalar(w2, w_dtype, d) : 1.f;
-        const float v = a[i] * r1 * ww1 * m1 + b[i] * r2 * ww2 * m2;
-        const float sg = 1.f / (1.f + __expf(-gg[i]));
-        out[i] = activation == 1 ? v * sg : v * gg[i] * sg;
-    }
-    if (ok)
-        *reinterpret_cast<uint4*>(y + base) = make_uint4(pack_bf16(out[0], out[1]), pack_bf16(out[2], out[3]),
-                                                         pack_bf16(out[4], out[5]), pack_bf16(out[6], out[7]));
 }
 
 
 // Backward of the output mixing (src/nats/modules/fused_norm_gate.py:353, :657).  With n = x * rstd and
 // v = n1 w1 a + n2 w2 b,  y = v * s(g):   dv = dy s(g),  dg = dy v s'(g),  da = <dv, n1 w1>,  db = <dv, n2 w2>,
-// dx = rstd (dn - n mean(dn n)) with dn1 = dv w1 a (dn2 likewise), and the weight gradients dw1 = sum_rows dv n1 a,
-// dw2 = sum_rows dv n2 b.  One warp per row, rows strided over a fixed grid; every CTA writes one partial sum of the
-// weight gradients (dw_part [grid, 2, D] fp32; the caller adds the CTAs up), so nothing is accumulated atomically.
+// dx = rstd (dn - n mean(dn n)) with dn1 = dv w1 a (dn2 likewise; the sum of dn1 n1 is a da), and the weight gradients
+// dw1 = sum_rows dv n1 a, dw2 = sum_rows dv n2 b.  The same rows per warp, strided over a fixed grid, the next rows' loads in
+// flight; every CTA writes one partial sum of the weight gradients (dw_part [grid, 2, D] fp32; the caller adds the CTAs up), so
+// nothing is accumulated atomically.
 template <int D>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
 norm_gate_mix_bwd_kernel(const __nv_bfloat16* __restrict__ x1, const __nv_bfloat16* __restrict__ x2,
                          const __nv_bfloat16* __restrict__ g, const void* __restrict__ xw, int xw_dtype,
                          const void* __restrict__ w1, const void* __restrict__ w2, int w_dtype,
                          const __nv_bfloat16* __restrict__ dy, __nv_bfloat16* __restrict__ dx1,
                          __nv_bfloat16* __restrict__ dx2, __nv_bfloat16* __restrict__ dg, float* __restrict__ dxw,
-                         float* __restrict__ dw_part, long rows, float eps, int activation) {
-    constexpr int EPL = D / 32;
+                         float* __restrict__ dw_part, long rows, float eps, int activation, int wide) {
+    constexpr int LPR = MixShape<D>::LPR, RPW = MixShape<D>::RPW;
     __shared__ float s_dw[8][2][D];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float ww1[EPL], ww2[EPL], dw1[EPL], dw2[EPL];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane % LPR;
+    uint64_t p1[4], p2[4], dw1[4], dw2[4];
+    weights8(w1, w_dtype == NATSL_DT_F32, sub * 8, p1);
+    weights8(w2, w_dtype == NATSL_DT_F32, sub * 8, p2);
 #pragma unroll
-    for (int i = 0; i < EPL; ++i) {
-        const int d = lane * EPL + i;
-        ww1[i] = w1 ? load_scalar(w1, w_dtype, d) : 1.f;
-        ww2[i] = w2 ? load_scalar(w2, w_dtype, d) : 1.f;
-        dw1[i] = 0.f;
-        dw2[i] = 0.f;
-    }
-    auto load = [&](const __nv_bfloat16* p, long base, float* out) {
-#pragma unroll
-        for (int i = 0; i < EPL; i += 2) {
-            const float2 f = unpack_bf16(*reinterpret_cast<const uint32_t*>(p + base + i));
-            out[i] = f.x;
-            out[i + 1] = f.y;
-        }
+    for (int i = 0; i < 4; ++i) dw1[i] = dw2[i] = 0;
+    const long step = (long)gridDim.x * 8 * RPW;
+    long row = ((long)blockIdx.x * 8 + warp) * RPW + lane / LPR;
+    uint4 na, nb, ng, nd;
+    float n1m = 1.f, n2m = 1.f;
+    auto load = [&](long r) {
+        r = r < rows ? r : rows - 1;                           // keep every lane in the shuffles
+        const long base = r * D + sub * 8;
+        na = ld16(x1 + base, wide);
+        nb = ld16(x2 + base, wide);
+        ng = ld16(g + base, wide);
+        nd = ld16(dy + base, wide);
+        if (xw) { n1m = load_scalar(xw, xw_dtype, r * 2); n2m = load_scalar(xw, xw_dtype, r * 2 + 1); }
     };
-    auto store = [&](__nv_bfloat16* p, long base, const float* v) {
+    if (row - lane / LPR < rows) load(row);
+    const uint64_t one = pack2(1.f, 1.f), neg = pack2(-1.f, -1.f);
+    for (; row - lane / LPR < rows; row += step) {
+        const bool ok = row < rows;
+        uint64_t a[4], b[4], gg[4], d[4], q1 = 0, q2 = 0;
+        open8(na, a);
+        open8(nb, b);
+        open8(ng, gg);
+        open8(nd, d);
+        const float m1 = n1m, m2 = n2m;
+        if (row - lane / LPR + step < rows) load(row + step);
 #pragma unroll
-        for (int i = 0; i < EPL; i += 2) *reinterpret_cast<uint32_t*>(p + base + i) = pack_bf16(v[i], v[i + 1]);
-    };
-    for (long row = (long)blockIdx.x * 8 + warp; row < rows; row += (long)gridDim.x * 8) {
-        const long base = row * D + lane * EPL;
-        float a[EPL], b[EPL], gg[EPL], d[EPL];
-        load(x1, base, a);
-        load(x2, base, b);
-        load(g, base, gg);
-        load(dy, base, d);
-        float s1 = 0.f, s2 = 0.f;
+        for (int i = 0; i < 4; ++i) { q1 = fma2(a[i], a[i], q1); q2 = fma2(b[i], b[i], q2); }
+        const float r1 = rsqrtf(row_sum<LPR>(hsum2(q1)) / D + eps), r2 = rsqrtf(row_sum<LPR>(hsum2(q2)) / D + eps);
+        const uint64_t e1 = pack2(r1, r1), e2 = pack2(r2, r2), k1 = pack2(m1, m1), k2 = pack2(m2, m2);
+        uint64_t da2 = 0, db2 = 0;
 #pragma unroll
-        for (int i = 0; i < EPL; ++i) { s1 += a[i] * a[i]; s2 += b[i] * b[i]; }
-        s1 = warp_sum(s1);
-        s2 = warp_sum(s2);
-        const float r1 = rsqrtf(s1 / D + eps), r2 = rsqrtf(s2 / D + eps);
-        float m1 = 1.f, m2 = 1.f;
-        if (xw) { m1 = load_scalar(xw, xw_dtype, row * 2); m2 = load_scalar(xw, xw_dtype, row * 2 + 1); }
-        float da = 0.f, db = 0.f, c1 = 0.f, c2 = 0.f;
-        float dgo[EPL], dn1[EPL], dn2[EPL];
-#pragma unroll
-        for (int i = 0; i < EPL; ++i) {
-            const float n1 = a[i] * r1, n2 = b[i] * r2;
-            const float v = n1 * ww1[i] * m1 + n2 * ww2[i] * m2;
-            const float sg = 1.f / (1.f + __expf(-gg[i]));
-            const float s = activation == 1 ? sg : gg[i] * sg;
-            const float sp = activation == 1 ? sg * (1.f - sg) : sg * (1.f + gg[i] * (1.f - sg));
-            const float dv = d[i] * s;
-            dgo[i] = d[i] * v * sp;
-            da += dv * n1 * ww1[i];
-            db += dv * n2 * ww2[i];
-            dw1[i] += dv * n1 * m1;
-            dw2[i] += dv * n2 * m2;
-            dn1[i] = dv * ww1[i] * m1;
-            dn2[i] = dv * ww2[i] * m2;
-            c1 += dn1[i] * n1;
-            c2 += dn2[i] * n2;
+        for (int i = 0; i < 4; ++i) {
+            const uint64_t n1 = mul2(a[i], e1), n2 = mul2(b[i], e2), u1 = mul2(n1, p1[i]), u2 = mul2(n2, p2[i]);
+            const uint64_t v = fma2(u1, k1, mul2(u2, k2)), sg = sigmoid2(gg[i]), om = fma2(sg, neg, one);       // 1 - sg
+            const uint64_t s = activation == 1 ? sg : mul2(gg[i], sg);
+            const uint64_t sp = mul2(sg, activation == 1 ? om : fma2(gg[i], om, one));
+            const uint64_t dv = mul2(d[i], s);
+            d[i] = mul2(mul2(d[i], v), sp);                    // dg
+            da2 = fma2(dv, u1, da2);
+            db2 = fma2(dv, u2, db2);
+            if (ok) {
+                dw1[i] = fma2(mul2(dv, n1), k1, dw1[i]);
+                dw2[i] = fma2(mul2(dv, n2), k2, dw2[i]);
+            }
+            gg[i] = dv;
             a[i] = n1;
             b[i] = n2;
         }
-        da = warp_sum(da); db = warp_sum(db); c1 = warp_sum(c1) / D; c2 = warp_sum(c2) / D;
+        const float da = row_sum<LPR>(hsum2(da2)), db = row_sum<LPR>(hsum2(db2));
+        const float c1 = -m1 * da / D, c2 = -m2 * db / D;
+        const uint64_t h1 = pack2(c1, c1), h2 = pack2(c2, c2);
 #pragma unroll
-        for (int i = 0; i < EPL; ++i) {
-            dn1[i] = r1 * (dn1[i] - a[i] * c1);
-            dn2[i] = r2 * (dn2[i] - b[i] * c2);
+        for (int i = 0; i < 4; ++i) {
+            a[i] = mul2(e1, fma2(a[i], h1, mul2(mul2(gg[i], p1[i]), k1)));
+            b[i] = mul2(e2, fma2(b[i], h2, mul2(mul2(gg[i], p2[i]), k2)));
         }
-        store(dx1, base, dn1);
-        store(dx2, base, dn2);
-        store(dg, base, dgo);
-        if (dxw && lane == 0) { dxw[row * 2] = da; dxw[row * 2 + 1] = db; }
+        if (ok) {
+            const long base = row * D + sub * 8;
+            st16(dx1 + base, close8(a), wide);
+            st16(dx2 + base, close8(b), wide);
+            st16(dg + base, close8(d), wide);
+            if (dxw && sub == 0) { dxw[row * 2] = da; dxw[row * 2 + 1] = db; }
+        }
+    }
+    float o1[8], o2[8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        unpack2(dw1[i], o1[2 * i], o1[2 * i + 1]);
+        unpack2(dw2[i], o2[2 * i], o2[2 * i + 1]);
     }
 #pragma unroll
-    for (int i = 0; i < EPL; ++i) {
-        s_dw[warp][0][lane * EPL + i] = dw1[i];
-        s_dw[warp][1][lane * EPL + i] = dw2[i];
+    for (int i = 0; i < 8; ++i) {
+#pragma unroll
+        for (int o = LPR; o < 32; o <<= 1) {                   // the rows side by side in the warp
+            o1[i] += __shfl_xor_sync(0xffffffffu, o1[i], o);
+            o2[i] += __shfl_xor_sync(0xffffffffu, o2[i], o);
+        }
+        if (lane < LPR) {
+            s_dw[warp][0][sub * 8 + i] = o1[i];
+            s_dw[warp][1][sub * 8 + i] = o2[i];
+        }
     }
     __syncthreads();
     for (int i = threadIdx.x; i < 2 * D; i += 256) {
@@ -174,8 +192,9 @@ extern "C" int natsl_norm_gate_mix(const void* x1, const void* x2, const void* g
                   NATSL_ERR_UNSUPPORTED, "natsl_norm_gate_mix: weights must be bf16 or f32");
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const int wpb = 8;
-    const long rpc = (long)wpb * (32 / (D > 0 ? (D / 8 > 0 ? D / 8 : 1) : 1));      // rows per CTA
-    const unsigned grid = (unsigned)((rows + rpc - 1) / rpc);
+    const long rpc = (long)wpb * (32 / (D > 0 ? (D / 8 > 0 ? D / 8 : 1) : 1));      // rows per CTA and turn
+    const long turns = (rows + rpc - 1) / rpc;
+    const unsigned grid = (unsigned)(turns < NORM_GATE_GRID ? turns : NORM_GATE_GRID);
 #define NATSL_NG(DD) norm_gate_mix_kernel<DD><<<grid, wpb * 32, 0, st>>>( \
         reinterpret_cast<const __nv_bfloat16*>(x1), reinterpret_cast<const __nv_bfloat16*>(x2), \
         reinterpret_cast<const __nv_bfloat16*>(g), xw, xw_dtype, w1, w2, w_dtype, reinterpret_cast<__nv_bfloat16*>(y), rows, eps, activation)
@@ -205,8 +224,9 @@ extern "C" int natsl_norm_gate_mix_bwd(const void* x1, const void* x2, const voi
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     auto bf = [](const void* p) { return reinterpret_cast<const __nv_bfloat16*>(p); };
     auto bm = [](void* p) { return reinterpret_cast<__nv_bfloat16*>(p); };
+    const int wide = aligned_to(16, x1, x2, g, dy, dx1, dx2, dg);
 #define NATSL_NGB(DD) norm_gate_mix_bwd_kernel<DD><<<n_part, 256, 0, st>>>(bf(x1), bf(x2), bf(g), xw, xw_dtype, w1, w2, w_dtype, \
-        bf(dy), bm(dx1), bm(dx2), bm(dg), dxw, dw_part, rows, eps, activation)
+        bf(dy), bm(dx1), bm(dx2), bm(dg), dxw, dw_part, rows, eps, activation, wide)
     if (D == 64) NATSL_NGB(64);
     else if (D == 128) NATSL_NGB(128);
     else if (D == 256) NATSL_NGB(256);

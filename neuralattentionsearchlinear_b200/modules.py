@@ -27,7 +27,8 @@ def _kernel_ok(x: torch.Tensor) -> bool:
 
 
 def _n_part(rows: int) -> int:
-    return int(min(-(-rows // 8), 1184))
+    """CTAs of the norms' backward kernels, each with one partial sum of the weight gradients: four per SM."""
+    return int(min(-(-rows // 8), 592))
 
 
 class _RMSNormFn(torch.autograd.Function):
@@ -267,7 +268,7 @@ class _NormGateMix(torch.autograd.Function):
         dy = dy.contiguous()
         dx1, dx2, dg = torch.empty_like(x1), torch.empty_like(x2), torch.empty_like(g)
         dxw = torch.empty(rows, 2, dtype=torch.float32, device=x1.device) if xw is not None else None
-        n_part = int(min(-(-rows // 8), 1184))
+        n_part = _n_part(rows)
         dw_part = torch.empty(n_part, 2, D, dtype=torch.float32, device=x1.device)
         _lib.call("natsl_norm_gate_mix_bwd", x1.data_ptr(), x2.data_ptr(), g.data_ptr(), _lib.ptr(xw), _dt(xw),
                   _lib.ptr(w1), _lib.ptr(w2), _dt(w1), dy.data_ptr(), dx1.data_ptr(), dx2.data_ptr(), dg.data_ptr(),
