@@ -150,6 +150,7 @@ int natsl_linear_fwd_o(int rule, const void* q, const void* k, const void* w, co
 
 /* Chunk preparation that also emits what the fused walk needs: q_rstd [B,T,H] fp32 and the intra-chunk score
  * matrix P = tril(qn kn^T e^{gcs_i - gcs_j}) [B,T,H,64] bf16 (q, q_rstd, pmat may all be NULL = natsl_gdn_chunk_prep).
+ * K = V = 64 runs on tcgen05 (as natsl_gdn_chunk_prep_tc does for 128 / 128), the other head dims on mma.sync.
  * Replaces in addition: l2norm_fwd(q) src/nats/ops/mixed_ops/mixed_attn_gdn.py:119-120 and the q k^T part of
  * chunk_fwd_kernel_o src/nats/ops/common/chunk_o.py:166,188,202-203. */
 int natsl_gdn_chunk_prep_ex(const void* q, const void* k, const void* v, const float* g, const void* beta,

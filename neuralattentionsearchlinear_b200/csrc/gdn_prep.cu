@@ -13,6 +13,7 @@
 // where Z = [v beta | kn beta e^{gcs}] and U overwrites Z in place.  Each warp owns 64 columns of Z and
 // runs its four steps on the tensor cores without block-wide synchronisation; U_j is rounded to bf16
 // between steps, the same rounding the stored u, w get.
+// (64 / 64 and, through an entry point of its own, 128 / 128 run the tcgen05 kernel of gdn_prep_tc.cu.)
 // The decay carried over skipped blocks multiplies w by one scalar per chunk (A only sees decay
 // differences), so it is applied by the consumers and w here is carry-free.
 #include "common.cuh"
@@ -359,6 +360,10 @@ gdn_prep_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __rest
     }
 }
 
+// gdn_prep_tc.cu: the tcgen05 form of K = V = 64
+int prep_tc64(const void* q, const void* k, const void* v, const float* g, const void* beta, int beta_dtype, void* w, void* u, float* gcs,
+              float* k_rstd, float* q_rstd, void* pmat, int B, int T, int H, int use_l2norm, cudaStream_t st);
+
 template <int K, int V>
 static int launch_prep(const void* q, const void* k, const void* v, const float* g, const void* beta, int beta_dtype,
                        void* w, void* u, float* gcs, float* krstd, float* qrstd, void* pmat, int B, int T, int H,
@@ -396,7 +401,7 @@ extern "C" int natsl_gdn_chunk_prep_ex(const void* q, const void* k, const void*
 #define NATSL_PREP_CASE(KK, VV) \
     if (K == KK && V == VV)     \
         return launch_prep<KK, VV>(q, k, v, g, beta, beta_dtype, w, u, gcs, k_rstd, q_rstd, pmat, B, T, H, use_l2norm, st);
-    NATSL_PREP_CASE(64, 64)
+    if (K == 64 && V == 64) return prep_tc64(q, k, v, g, beta, beta_dtype, w, u, gcs, k_rstd, q_rstd, pmat, B, T, H, use_l2norm, st);
     NATSL_PREP_CASE(64, 128)
     NATSL_PREP_CASE(128, 64)
     NATSL_PREP_CASE(128, 128)

@@ -1,27 +1,33 @@
-// Gated-delta-rule chunk preparation on the 5th-generation tensor cores (head dims K = V = 128).
+// Gated-delta-rule chunk preparation on the 5th-generation tensor cores (head dims D = K = V = 128 and 64).
 // Same inputs, outputs and conventions as gdn_prep.cu (the mma.sync kernel, kept for the other head dims):
 //   k_rstd, q_rstd, gcs, A = strictLower(beta_i (kn_i . kn_j) e^{gcs_i - gcs_j}),
 //   [u | w] = (I + A)^-1 [v beta | kn beta e^{gcs}],  P = tril(qn kn^T e^{gcs_i - gcs_j})
 // (src/nats/ops/common/chunk_scaled_dot_kkt.py:105-126, src/nats/ops/utils/solve_tril.py:350-447,
 //  src/nats/ops/gated_delta_rule/wy_fast.py:123-153, src/nats/ops/common/chunk_o.py:166,188,202-203).
 //
-// One CTA per (batch, head, 64-token chunk), 160 threads, 128 TMEM columns, ~52 KB of shared memory (four CTAs per SM):
+// One CTA per (batch, head, 64-token chunk), 160 threads; D = 128: 128 TMEM columns, 52 KB of shared memory, four CTAs per SM;
+// D = 64: 64 columns, 37 KB, six CTAs:
 //   warp 4      TMA producer (k, q tiles at the start, the v tile once A is no longer needed; 128-byte swizzle)
 //               and single-thread MMA issuer;
 //   warps 0-3   one thread per TMEM lane.
 // Steps:
-//   1. D1 = [k ; q] k^T            one stacked 128 x 64 x 128 product into TMEM (rows 0-63: K K^T, rows 64-127: Q K^T);
+//   1. D1 = [k ; q] k^T            one stacked 128 x 64 x D product into TMEM (rows 0-63: K K^T, rows 64-127: Q K^T);
 //   2. row norms of k from the diagonal of D1, A (fp32, shared memory) from rows 0-63, P (bf16, global memory,
 //      one 128-byte row per thread) from rows 64-127;
 //   3. Ai = (I + A)^-1 like the reference does it: the four 16 x 16 diagonal blocks by forward substitution in fp32,
 //      the blocks below by the block recursion Ai_ij = -X_ii sum_{j<=m<i} A_im Ai_mj, evaluated per panel of eight
 //      columns (the columns of an inverse are independent of one another) with tf32 mma.sync products, fp32
 //      accumulation; Ai diag(beta) and Ai diag(beta rstd e^{gcs}) are written as two bf16 operand tiles, so the
-//      right-hand sides never have to be scaled in shared memory;
+//      right-hand sides never have to be scaled in shared memory (D = 64 has room for the first one only: the rows of k are
+//      scaled by rstd e^{gcs} while the diagonal blocks are inverted);
 //   4. D2 = [v^T (Ai diag beta)^T | k^T (Ai diag(..))^T]: the raw v and k tiles are the (MN-major) A operands,
-//      features in the TMEM lanes, tokens in the columns: no accumulator row is wasted;
-//   5. w, then u, go from TMEM through a [token][feature] staging tile (written feature by feature, which is
-//      conflict-free) to global memory with TMA stores; P leaves the same way.
+//      features in the TMEM lanes, tokens in the columns: no accumulator row is wasted (D = 64: both in one product);
+//   5. w, then u, go from TMEM through a [token][feature] staging tile (transposed by stmatrix) to global memory with TMA
+//      stores; P leaves the same way.
+// Chains of short phases: what counts is the instructions of a chunk and how many chunks an SM has in flight.  L2 flushed:
+// 8 x 4096 tokens, 16 heads, D = 128: 180 us one element at a time and one feature per store, 152 us with the entries of A and P
+// in pairs, stmatrix and two diagonal blocks per warp (same bits; traffic 113 us); 16 x 4096 tokens, 16 heads, D = 64: 355 us on
+// mma.sync (shared memory 75 % busy), 208 us here (traffic 126 us).
 // The decay carried over skipped blocks multiplies w by one scalar per chunk and is applied by the consumers.
 // Every mbarrier wait is bounded: on expiry the status word is set and the CTA runs on to its teardown.
 #include "tc_common.cuh"
@@ -31,41 +37,31 @@ namespace natsl {
 
 constexpr int PT_THREADS = 160;
 constexpr int PT_EPI = 128;
-constexpr uint32_t PT_TMEM_COLS = 128;
 constexpr int PT_A_LD = 68;                  // fp32 row pitch of A: conflict-free 16-byte row stores and fragment loads
 
+template <int D>
 struct PtSmem {
-    // [k sub-tile 0][q sub-tile 0][k sub-tile 1][q sub-tile 1], each [64 tokens][64 features] = 8 KB: the stacked
-    // [k ; q] operand of the first product.  The q sub-tiles are reused: first sub-tile 0 for staging P, then both for
-    // the two Ai operand tiles.
+    static constexpr int SUB = D / 64;                       // sub-tiles of 64 features, [64 tokens][64 features] = 8 KB each
+    // [k sub-tile 0][q sub-tile 0][k sub-tile 1][q sub-tile 1]: the stacked [k ; q] operand of the first product.  The q sub-tiles
+    // are reused: first sub-tile 0 for staging P, then for the Ai operand tiles (one where D = 64, two where D = 128).
     static constexpr int kq = 0;
-    // fp32 A [64][68] (diagonal blocks replaced by their inverses); once Ai is formed the v tile (2 sub-tiles, 16 KB)
-    // is loaded over it -- it is needed by the last product only, and this is what lets four CTAs share an SM
-    static constexpr int As = 32768;
+    // fp32 A [64][68] (diagonal blocks replaced by their inverses); once Ai is formed the v tile is loaded over it -- it is
+    // needed by the last product only, and this is what lets four CTAs (D = 64: six) share an SM
+    static constexpr int As = SUB * 16384;
     static constexpr int v = As;
     static constexpr int scr = As + 64 * PT_A_LD * 4;        // per warp [16][8] fp32: accumulator -> B-fragment exchange
     static constexpr int vec = scr + 4 * 512;                // gcs, beta, k rstd, w scale, q rstd: 5 x 64 floats
     static constexpr int bars = vec + 5 * 64 * 4;
     static constexpr int total = bars + 64;
-    static constexpr int aiu = kq + 8192, aiw = kq + 24576;  // Ai diag(beta), Ai diag(beta rstd e^{gcs}): [64][64] bf16
+    static constexpr int aiu = kq + 8192, aiw = kq + 24576;  // Ai diag(beta), Ai diag(beta rstd e^{gcs}) (D = 128): [64][64] bf16
     static constexpr int pst = kq + 8192;                    // P staging [64][64] bf16
-    static_assert(As % 1024 == 0 && 64 * PT_A_LD * 4 >= 16384, "the v tile must fit over A, 1024-byte aligned");
-    static_assert(4 * (total + 1024) <= 232448, "four CTAs per SM");
+    static constexpr int ctas = D == 64 ? 6 : 4;             // per SM
+    static constexpr uint32_t tmem = 64 * SUB;               // columns: with D = 64 the last product lies over the first
+    static_assert(As % 1024 == 0 && 64 * PT_A_LD * 4 >= 8192 * SUB, "the v tile must fit over A, 1024-byte aligned");
+    static_assert(ctas * (total + 1024) <= 233472 && ctas * tmem <= 512, "CTAs per SM");
 };
 
 __device__ __forceinline__ void epi_barrier() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
-
-#ifdef NATSL_PREP_TIMING
-// scratch builds only: cycle stamps of thread 0 (slots 0-9) and thread 64 (slots 10-19) of every CTA
-__device__ long long* g_prep_ts = nullptr;
-#define PT_STAMP(slot)                                                                                        \
-    do {                                                                                                      \
-        if (g_prep_ts && (tid == 0 || tid == 64))                                                             \
-            g_prep_ts[(((long)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * 20 + (tid ? 10 : 0) + (slot)] = clock64(); \
-    } while (0)
-#else
-#define PT_STAMP(slot)
-#endif
 
 __device__ __forceinline__ uint32_t to_tf32(float x) {
     uint32_t r;
@@ -105,24 +101,27 @@ __device__ __forceinline__ void acc_to_b(float* scr, const float (&c)[4], int la
 }
 
 // One panel of eight columns [c0, c0+8) of Ai (c0 = 16 j + 8 half), by one warp: zero above block row j, X_jj's half,
-// then block rows j+1..3 by the recursion; every 16 x 8 block is written, scaled per column, into both operand tiles.
+// then block rows j+1..3 by the recursion; every 16 x 8 block is written, scaled per column, into the operand tile or tiles.
+template <bool TWO>
 __device__ __forceinline__ void inverse_panel(const float* As, float* scr, unsigned char* aiu, unsigned char* aiw,
                                               const float* s_beta, const float* s_wsc, int j, int half, int lane) {
     const int g = lane >> 2, q = lane & 3;
     const int c0 = 16 * j + 8 * half;
     const int chunk = c0 >> 3;
     const int ca = c0 + 2 * q;
-    const float bu0 = s_beta[ca], bu1 = s_beta[ca + 1], bw0 = s_wsc[ca], bw1 = s_wsc[ca + 1];
+    const float bu0 = s_beta[ca], bu1 = s_beta[ca + 1], bw0 = TWO ? s_wsc[ca] : 0.f, bw1 = TWO ? s_wsc[ca + 1] : 0.f;
     for (int r = lane; r < 16 * j; r += 32) {
         *reinterpret_cast<uint4*>(aiu + swz<128>(r, chunk)) = make_uint4(0, 0, 0, 0);
-        *reinterpret_cast<uint4*>(aiw + swz<128>(r, chunk)) = make_uint4(0, 0, 0, 0);
+        if (TWO) *reinterpret_cast<uint4*>(aiw + swz<128>(r, chunk)) = make_uint4(0, 0, 0, 0);
     }
     auto put = [&](int blk, const float (&y)[4]) {
         const int ra = 16 * blk + g, rb = ra + 8;
         *reinterpret_cast<uint32_t*>(aiu + swz<128>(ra, chunk) + q * 4) = pack_bf16(y[0] * bu0, y[1] * bu1);
         *reinterpret_cast<uint32_t*>(aiu + swz<128>(rb, chunk) + q * 4) = pack_bf16(y[2] * bu0, y[3] * bu1);
-        *reinterpret_cast<uint32_t*>(aiw + swz<128>(ra, chunk) + q * 4) = pack_bf16(y[0] * bw0, y[1] * bw1);
-        *reinterpret_cast<uint32_t*>(aiw + swz<128>(rb, chunk) + q * 4) = pack_bf16(y[2] * bw0, y[3] * bw1);
+        if (TWO) {
+            *reinterpret_cast<uint32_t*>(aiw + swz<128>(ra, chunk) + q * 4) = pack_bf16(y[0] * bw0, y[1] * bw1);
+            *reinterpret_cast<uint32_t*>(aiw + swz<128>(rb, chunk) + q * 4) = pack_bf16(y[2] * bw0, y[3] * bw1);
+        }
     };
     uint32_t yb[4][2][2];                        // B fragments of the panel's blocks, by block row
     {
@@ -162,15 +161,45 @@ __device__ __forceinline__ void inverse_panel(const float* As, float* scr, unsig
     }
 }
 
-__global__ void __launch_bounds__(PT_THREADS, 4)
+// Four entries x r of a row of A or P: (left * right_j) r_j e^{gi - gj}, columns from `first` on (first > 3: none) left out.
+__device__ __forceinline__ float ex2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float4 decayed4(const float* gcs, const float* right, const uint32_t* r, uint64_t gi, uint64_t left, int first) {
+    const uint64_t neg = pack2(-1.f, -1.f), l2e = pack2(1.44269504f, 1.44269504f);
+    const ulonglong2 gj = *reinterpret_cast<const ulonglong2*>(gcs), rj = *reinterpret_cast<const ulonglong2*>(right);
+    float a, b, c, d;
+    unpack2(mul2(fma2(gj.x, neg, gi), l2e), a, b);
+    unpack2(mul2(fma2(gj.y, neg, gi), l2e), c, d);
+    const uint64_t x = mul2(mul2(mul2(rj.x, left), pack2(__uint_as_float(r[0]), __uint_as_float(r[1]))), pack2(ex2(a), ex2(b)));
+    const uint64_t y = mul2(mul2(mul2(rj.y, left), pack2(__uint_as_float(r[2]), __uint_as_float(r[3]))), pack2(ex2(c), ex2(d)));
+    float4 o;
+    unpack2(x, o.x, o.y);
+    unpack2(y, o.z, o.w);
+    o.x = first > 0 ? o.x : 0.f;                               // (a select, not a factor: the exponential may have overflowed)
+    o.y = first > 1 ? o.y : 0.f;
+    o.z = first > 2 ? o.z : 0.f;
+    o.w = first > 3 ? o.w : 0.f;
+    return o;
+}
+// Four 8 x 8 bf16 matrices in the accumulator-fragment layout, stored transposed, each thread giving the address of one row.
+__device__ __forceinline__ void stsm_x4_t(uint32_t addr, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(r0), "r"(r1), "r"(r2), "r"(r3)
+                 : "memory");
+}
+
+template <int D>
+__global__ void __launch_bounds__(PT_THREADS, PtSmem<D>::ctas)
 gdn_prep_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                    const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_w,
                    const __grid_constant__ CUtensorMap map_u, const __grid_constant__ CUtensorMap map_p, int has_q,
                    const float* __restrict__ g, const void* __restrict__ beta, int beta_dtype,
                    float* __restrict__ gcs_out, float* __restrict__ krstd_out, float* __restrict__ qrstd_out, int T,
                    int H, int use_l2norm, int* status) {
-    using L = PtSmem;
-    constexpr int K = 128;
+    using L = PtSmem<D>;
+    constexpr int SUB = L::SUB;
     extern __shared__ __align__(1024) unsigned char smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t sbase = smem_u32(smem);
@@ -193,7 +222,6 @@ gdn_prep_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                    bar_v = bar_load + 32, bar_d2u = bar_load + 40;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::bars + 48);
 
-    PT_STAMP(0);
     if (tid == 0) {
         mbar_init(bar_load, 1);
         mbar_init(bar_d1, 1);
@@ -203,25 +231,24 @@ gdn_prep_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         mbar_init(bar_d2u, 1);
         mbar_fence_init();
     }
-    if (warp == 4) tmem_alloc(smem_u32(tmem_slot), PT_TMEM_COLS);
+    if (warp == 4) tmem_alloc(smem_u32(tmem_slot), L::tmem);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    PT_STAMP(1);
 
     if (warp == 4) {
         // ------------------------------------------------------------ TMA producer + MMA issuer
         if (lane == 0) {
-            mbar_expect_tx(bar_load, has_q ? 32768 : 16384);
+            mbar_expect_tx(bar_load, (has_q ? 16384 : 8192) * SUB);
 #pragma unroll
-            for (int sub = 0; sub < 2; ++sub) {
+            for (int sub = 0; sub < SUB; ++sub) {
                 tma_load_4d(sbase + L::kq + sub * 16384, &map_k, sub * 64, h, t0, b, bar_load);
                 if (has_q) tma_load_4d(sbase + L::kq + sub * 16384 + 8192, &map_q, sub * 64, h, t0, b, bar_load);
             }
             // v is only needed at the very end: warm L2 now, load it when A is dead
-            tma_prefetch_4d(&map_v, 0, h, t0, b);
-            tma_prefetch_4d(&map_v, 64, h, t0, b);
+#pragma unroll
+            for (int sub = 0; sub < SUB; ++sub) tma_prefetch_4d(&map_v, sub * 64, h, t0, b);
         }
         __syncwarp();
         mbar_wait_small(bar_load, 0, status);
@@ -231,21 +258,21 @@ gdn_prep_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             tc_fence_after();
             const uint32_t l = umma_desc_lo(sbase + L::kq, 16);
 #pragma unroll
-            for (int h = 0; h < K / 64; ++h) umma_ss_x4<2, 2>(tmem, l + h * 1024, l + h * 1024, id_1, h > 0);
+            for (int sub = 0; sub < SUB; ++sub) umma_ss_x4<2, 2>(tmem, l + sub * 1024, l + sub * 1024, id_1, sub > 0);
             umma_commit(bar_d1);
         }
         __syncwarp();
         mbar_wait_small(bar_ai, 0, status);
         __syncwarp();
-        {
-            constexpr uint32_t id_2 = umma_idesc_bf16(128, 64, false) | (1u << 15);      // A MN-major (features x tokens)
-            // every thread has finished with A (and fenced): the v tile may land on it
-            if (lane == 0) {
-                mbar_expect_tx(bar_v, 16384);
-                tma_load_4d(sbase + L::v, &map_v, 0, h, t0, b, bar_v);
-                tma_load_4d(sbase + L::v + 8192, &map_v, 64, h, t0, b, bar_v);
-            }
-            __syncwarp();
+        constexpr uint32_t id_2 = umma_idesc_bf16(128, 64, false) | (1u << 15);      // A MN-major (features x tokens)
+        // every thread has finished with A (and fenced): the v tile may land on it
+        if (lane == 0) {
+            mbar_expect_tx(bar_v, 8192 * SUB);
+#pragma unroll
+            for (int sub = 0; sub < SUB; ++sub) tma_load_4d(sbase + L::v + sub * 8192, &map_v, sub * 64, h, t0, b, bar_v);
+        }
+        __syncwarp();
+        if constexpr (D == 128) {
             tc_fence_after();
             umma_ss_x4<128, 2>(tmem + 64, umma_desc_lo(sbase + L::kq, 16384), umma_desc_lo(sbase + L::aiw, 16), id_2, 0u);
             umma_commit(bar_d2w);
@@ -253,12 +280,10 @@ gdn_prep_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         __syncwarp();
         mbar_wait_small(bar_v, 0, status);
         __syncwarp();
-        {
-            constexpr uint32_t id_2 = umma_idesc_bf16(128, 64, false) | (1u << 15);
-            tc_fence_after();
-            umma_ss_x4<128, 2>(tmem, umma_desc_lo(sbase + L::v, 8192), umma_desc_lo(sbase + L::aiu, 16), id_2, 0u);
-            umma_commit(bar_d2u);
-        }
+        tc_fence_after();
+        if constexpr (D == 128) umma_ss_x4<128, 2>(tmem, umma_desc_lo(sbase + L::v, 8192), umma_desc_lo(sbase + L::aiu, 16), id_2, 0u);
+        else umma_ss_x4<128, 2>(tmem, umma_desc_lo(sbase + L::kq, L::v - L::kq), umma_desc_lo(sbase + L::aiu, 16), id_2, 0u);
+        umma_commit(bar_d2u);
         __syncwarp();
     } else {
         // ------------------------------------------------------------ one thread per TMEM lane
@@ -295,13 +320,12 @@ gdn_prep_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             if (lane + 32 < valid) gcs_out[g1] = x1;
         }
         mbar_wait_small(bar_load, 0, status);
-        PT_STAMP(2);
         if (warp >= 2 && has_q) {
             // q row norms (one row per thread; the swizzle makes the 16-byte reads of eight rows conflict-free)
             const int r = row - 64;
             float ss = 0.f;
 #pragma unroll
-            for (int sub = 0; sub < 2; ++sub)
+            for (int sub = 0; sub < SUB; ++sub)
 #pragma unroll
                 for (int cc = 0; cc < 8; ++cc) {
                     const uint4 xv = *reinterpret_cast<const uint4*>(smem + L::kq + sub * 16384 + 8192 + swz<128>(r, cc));
@@ -318,7 +342,6 @@ gdn_prep_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         }
         mbar_wait_small(bar_d1, 0, status);
         tc_fence_after();
-        PT_STAMP(3);
         if (warp < 2) {
             // k row norms from the diagonal of K K^T: row i of warp w has its diagonal in columns [32 w, 32 w + 32)
             uint32_t r[32];
@@ -333,69 +356,57 @@ gdn_prep_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             if (row < valid) krstd_out[(tok0 + row) * H + h] = rs;
         }
         epi_barrier();                      // gcs, beta, both row norms are known; the q tile has been read for the last time
-        PT_STAMP(4);
         if (warp < 2) {
             const float gi = s_gcs[row];
             const float bi = s_beta[row] * s_rstd[row];
-            s_wsc[row] = bi * __expf(gi);
+            s_wsc[row] = (D == 64 ? s_rstd[row] : bi) * __expf(gi);
+            const uint64_t gi2 = pack2(gi, gi), bi2 = pack2(bi, bi);
 #pragma unroll 1
             for (int hh = 0; hh <= warp; ++hh) {           // columns above the row's 32-column group are never read
                 uint32_t r[32];
                 tmem_ld32(t_lane + 32 * hh, r);
                 tmem_ld_wait();
+                const int below = row - 32 * hh;           // entries left of the diagonal
 #pragma unroll
-                for (int j4 = 0; j4 < 32; j4 += 4) {
-                    const int j = 32 * hh + j4;
-                    const float4 gj = *reinterpret_cast<const float4*>(s_gcs + j);
-                    const float4 rj = *reinterpret_cast<const float4*>(s_rstd + j);
-                    // strictly below the diagonal; the exponent is clamped so that the masked entries stay finite
-                    float4 a;
-                    a.x = (row > j ? bi : 0.f) * rj.x * __uint_as_float(r[j4]) * __expf(fminf(gi - gj.x, 0.f));
-                    a.y = (row > j + 1 ? bi : 0.f) * rj.y * __uint_as_float(r[j4 + 1]) * __expf(fminf(gi - gj.y, 0.f));
-                    a.z = (row > j + 2 ? bi : 0.f) * rj.z * __uint_as_float(r[j4 + 2]) * __expf(fminf(gi - gj.z, 0.f));
-                    a.w = (row > j + 3 ? bi : 0.f) * rj.w * __uint_as_float(r[j4 + 3]) * __expf(fminf(gi - gj.w, 0.f));
-                    *reinterpret_cast<float4*>(As + row * PT_A_LD + j) = a;
-                }
+                for (int j = 0; j < 32; j += 4)
+                    *reinterpret_cast<float4*>(As + row * PT_A_LD + 32 * hh + j) =
+                        decayed4(s_gcs + 32 * hh + j, s_rstd + 32 * hh + j, r + j, gi2, bi2, below - j);
             }
         } else if (has_q) {
             // P = tril(qn kn^T e^{gcs_i - gcs_j}): one row per thread into the staging tile (the q sub-tile is free);
             // one TMA store writes the tile after the next barrier
             const int i = row - 64;
-            const float gi = s_gcs[i], qi = s_qr[i];
+            const uint64_t gi2 = pack2(s_gcs[i], s_gcs[i]), qi2 = pack2(s_qr[i], s_qr[i]);
             unsigned char* pst = smem + L::pst;
 #pragma unroll 1
             for (int hh = 0; hh < 2; ++hh) {
+                if (hh > warp - 2) {                       // above the diagonal
+#pragma unroll
+                    for (int j = 4; j < 8; ++j) *reinterpret_cast<uint4*>(pst + swz<128>(i, j)) = make_uint4(0, 0, 0, 0);
+                    break;
+                }
                 uint32_t r[32];
                 tmem_ld32(t_lane + 32 * hh, r);
                 tmem_ld_wait();
+                const int upto = i + 1 - 32 * hh;          // entries up to the diagonal
 #pragma unroll
-                for (int j8 = 0; j8 < 32; j8 += 8) {
-                    const int j = 32 * hh + j8;
-                    float pv[8];
-#pragma unroll
-                    for (int e4 = 0; e4 < 8; e4 += 4) {
-                        const float4 gj = *reinterpret_cast<const float4*>(s_gcs + j + e4);
-                        const float4 rj = *reinterpret_cast<const float4*>(s_rstd + j + e4);
-                        pv[e4] = (i >= j + e4 ? qi : 0.f) * rj.x * __uint_as_float(r[j8 + e4]) * __expf(fminf(gi - gj.x, 0.f));
-                        pv[e4 + 1] = (i >= j + e4 + 1 ? qi : 0.f) * rj.y * __uint_as_float(r[j8 + e4 + 1]) * __expf(fminf(gi - gj.y, 0.f));
-                        pv[e4 + 2] = (i >= j + e4 + 2 ? qi : 0.f) * rj.z * __uint_as_float(r[j8 + e4 + 2]) * __expf(fminf(gi - gj.z, 0.f));
-                        pv[e4 + 3] = (i >= j + e4 + 3 ? qi : 0.f) * rj.w * __uint_as_float(r[j8 + e4 + 3]) * __expf(fminf(gi - gj.w, 0.f));
-                    }
-                    *reinterpret_cast<uint4*>(pst + swz<128>(i, j >> 3)) =
-                        make_uint4(pack_bf16(pv[0], pv[1]), pack_bf16(pv[2], pv[3]), pack_bf16(pv[4], pv[5]), pack_bf16(pv[6], pv[7]));
+                for (int j = 0; j < 32; j += 8) {
+                    const float4 x = decayed4(s_gcs + 32 * hh + j, s_rstd + 32 * hh + j, r + j, gi2, qi2, upto - j);
+                    const float4 y = decayed4(s_gcs + 32 * hh + j + 4, s_rstd + 32 * hh + j + 4, r + j + 4, gi2, qi2, upto - j - 4);
+                    *reinterpret_cast<uint4*>(pst + swz<128>(i, 4 * hh + (j >> 3))) =
+                        make_uint4(pack_bf16(x.x, x.y), pack_bf16(x.z, x.w), pack_bf16(y.x, y.y), pack_bf16(y.z, y.w));
                 }
             }
             fence_async_smem();
         }
-        PT_STAMP(5);
         epi_barrier();                      // A complete, the w scale known, D1 read for the last time, P staged
         if (tid == 64 && has_q) {
             tma_store_4d(&map_p, sbase + L::pst, 0, h, t0, b);
             tma_store_commit();
         }
-        if (lane < 16) {
-            // X_dd = (I + A_dd)^-1 by forward substitution, lane = column; written over A_dd
-            const int d0 = warp * 16, cidx = lane;
+        if (warp < 2) {
+            // X_dd = (I + A_dd)^-1 by forward substitution, two blocks per warp, lane = column; written over A_dd
+            const int d0 = warp * 32 + (lane & 16), cidx = lane & 15;
             float xcol[16];
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
@@ -413,11 +424,24 @@ gdn_prep_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 }
                 xcol[i] = ((i == cidx) ? 1.f : 0.f) - ((p0 + p1) + (p2 + p3));
             }
-            __syncwarp(0x0000ffffu);
+            __syncwarp();
 #pragma unroll
             for (int i = 0; i < 16; ++i) As[(d0 + i) * PT_A_LD + d0 + cidx] = xcol[i];
+        } else if constexpr (D == 64) {
+            // meanwhile: the rows of k, the operand of w, scaled by rstd e^{gcs} (beta comes with Ai)
+#pragma unroll
+            for (int rr = 0; rr < 8; ++rr) {
+                const int r = rr * 8 + (row - 64) / 8, cc = row % 8;
+                uint4* ptr = reinterpret_cast<uint4*>(smem + L::kq + swz<128>(r, cc));
+                const float sc = s_wsc[r];
+                const uint64_t s2 = pack2(sc, sc);
+                uint64_t x[4];
+                open8(*ptr, x);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) x[e] = mul2(x[e], s2);
+                *ptr = close8(x);
+            }
         }
-        PT_STAMP(6);
         if (tid == 64 && has_q) tma_store_wait_read();      // the P tile has been read: its place becomes Ai diag(beta)
         epi_barrier();
         {
@@ -425,66 +449,97 @@ gdn_prep_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             unsigned char* aiu = smem + L::aiu;
             unsigned char* aiw = smem + L::aiw;
             if (warp < 2) {
-                inverse_panel(As, scr, aiu, aiw, s_beta, s_wsc, 0, warp, lane);
+                inverse_panel<D == 128>(As, scr, aiu, aiw, s_beta, s_wsc, 0, warp, lane);
             } else {
 #pragma unroll
-                for (int j = 1; j < 4; ++j) inverse_panel(As, scr, aiu, aiw, s_beta, s_wsc, j, warp - 2, lane);
+                for (int j = 1; j < 4; ++j) inverse_panel<D == 128>(As, scr, aiu, aiw, s_beta, s_wsc, j, warp - 2, lane);
             }
         }
-        PT_STAMP(7);
         fence_async_smem();
         tc_fence_before();
         mbar_arrive(bar_ai);
-        PT_STAMP(8);
-        // ---- w (columns 64-127, its product does not wait for the v tile) then u (columns 0-63): lane = feature,
-        // column = token.  Each thread writes its feature's 64 values as single bf16 into a [token][feature] staging
-        // tile (32 lanes = 64 contiguous bytes of one row: conflict-free), then one thread stores the tiles with TMA.
-        // Staging: w over the k sub-tiles (dead once its product is done), u over the two Ai tiles.
-        {
-            const int sub = row >> 6, cf = row & 63;
-            uint32_t off[8];                             // byte offset of this feature inside a row, by (token & 7)
-#pragma unroll
-            for (int x = 0; x < 8; ++x) off[x] = (uint32_t)((((cf >> 3) ^ x) << 4) + (cf & 7) * 2);
+        // ---- w and u: lane = feature, column = token.  A warp takes sixteen features at a time in the fragment layout, and
+        // stmatrix lays them transposed into a [token][feature] staging tile (conflict-free); one thread stores the tiles with TMA.
+        // D = 128: w (columns 64-127, its product does not wait for the v tile) then u (columns 0-63), staged over the k sub-tiles
+        // (dead once w's product is done) and over the two Ai tiles.  D = 64: lanes 0-63 are w, the others u, staged over the tiles
+        // that they were computed from.
 #pragma unroll 1
-            for (int arr = 0; arr < 2; ++arr) {          // 0: w, 1: u
-                mbar_wait_small(arr == 0 ? bar_d2w : bar_d2u, 0, status);
-                tc_fence_after();
-                unsigned char* stg = smem + L::kq + sub * 16384 + (arr == 0 ? 0 : 8192);
+        for (int arr = D == 128 ? 0 : 1; arr < 2; ++arr) {     // 0: w, 1: u (D = 64: both)
+            mbar_wait_small(arr == 0 ? bar_d2w : bar_d2u, 0, status);
+            tc_fence_after();
+            const int sub = row >> 6;
+            const uint32_t stg = sbase + (D == 64 ? (sub ? L::v : L::kq) : L::kq + sub * 16384 + (arr == 0 ? 0 : 8192));
+            // this thread's row of the four matrices: token (lane & 7) of the lower or upper eight, features of its half
+            const int tok = (lane & 7) + ((lane & 16) >> 1), half = (lane >> 3) & 1;
 #pragma unroll 1
-                for (int hh = 0; hh < 2; ++hh) {
-                    uint32_t r[32];
-                    tmem_ld32(t_lane + (arr == 0 ? 64 : 0) + 32 * hh, r);
-                    tmem_ld_wait();
+            for (int f = 0; f < 2; ++f) {                      // sixteen features
+                uint32_t r[32];
+                tmem_ld_16x256b_x8(t_lane + ((uint32_t)(16 * f) << 16) + (arr == 0 ? 64 : 0), r);
+                tmem_ld_wait();
+                const int chunk = (((row & 32) + 16 * f) >> 3) + half;
+                const uint32_t at = stg + tok * 128 + ((chunk ^ (tok & 7)) << 4);
 #pragma unroll
-                    for (int tt = 0; tt < 32; ++tt)
-                        *reinterpret_cast<__nv_bfloat16*>(stg + (32 * hh + tt) * 128 + off[tt & 7]) =
-                            __float2bfloat16(__uint_as_float(r[tt]));
+                for (int k = 0; k < 4; ++k) {                  // sixteen tokens
+                    uint32_t p[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        p[e] = pack_bf16(__uint_as_float(r[8 * k + 2 * e]), __uint_as_float(r[8 * k + 2 * e + 1]));
+                    stsm_x4_t(at + k * 16 * 128, p[0], p[1], p[2], p[3]);
                 }
-                fence_async_smem();
-                epi_barrier();
-                if (tid == 0) {
+            }
+            fence_async_smem();
+            epi_barrier();
+            if (tid == 0) {
+                if constexpr (D == 64) {
+                    tma_store_4d(&map_w, sbase + L::kq, 0, h, t0, b);
+                    tma_store_4d(&map_u, sbase + L::v, 0, h, t0, b);
+                } else {
                     const CUtensorMap* mp = arr == 0 ? &map_w : &map_u;
                     tma_store_4d(mp, sbase + L::kq + (arr == 0 ? 0 : 8192), 0, h, t0, b);
                     tma_store_4d(mp, sbase + L::kq + 16384 + (arr == 0 ? 0 : 8192), 64, h, t0, b);
-                    tma_store_commit();
                 }
+                tma_store_commit();
             }
-            if (tid == 0) tma_store_wait_read();
         }
-        PT_STAMP(9);
+        if (tid == 0) tma_store_wait_read();
         tc_fence_before();
     }
     __syncthreads();
-    if (warp == 4) tmem_dealloc(tmem, PT_TMEM_COLS);
+    if (warp == 4) tmem_dealloc(tmem, L::tmem);
+}
+
+template <int D>
+static int launch_prep_tc(const void* q, const void* k, const void* v, const float* g, const void* beta, int beta_dtype, void* w, void* u,
+                          float* gcs, float* k_rstd, float* q_rstd, void* pmat, int B, int T, int H, int use_l2norm, cudaStream_t st) {
+    using L = PtSmem<D>;
+    auto kern = gdn_prep_tc_kernel<D>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::total);
+    if (e != cudaSuccess) {
+        set_error("natsl_gdn_chunk_prep: cannot reserve %d B of shared memory (%s)", L::total, cudaGetErrorString(e));
+        return NATSL_ERR_CUDA;
+    }
+    CUtensorMap mq, mk, mv, mw, mu, mp;
+    int rc = encode_bthd_map(&mk, k, B, T, H, D, 64, "natsl_gdn_chunk_prep(k)");
+    if (rc == NATSL_OK) rc = encode_bthd_map(&mv, v, B, T, H, D, 64, "natsl_gdn_chunk_prep(v)");
+    if (rc == NATSL_OK) rc = encode_bthd_map(&mq, q ? q : k, B, T, H, D, 64, "natsl_gdn_chunk_prep(q)");
+    if (rc == NATSL_OK) rc = encode_bthd_map(&mw, w, B, T, H, D, 64, "natsl_gdn_chunk_prep(w)");
+    if (rc == NATSL_OK) rc = encode_bthd_map(&mu, u, B, T, H, D, 64, "natsl_gdn_chunk_prep(u)");
+    if (rc == NATSL_OK) rc = pmat ? encode_bthd_map(&mp, pmat, B, T, H, 64, 64, "natsl_gdn_chunk_prep(P)") : NATSL_OK;
+    if (!pmat) mp = mk;
+    int* status = nullptr;
+    if (rc == NATSL_OK) rc = status_word_ptr(&status);
+    if (rc != NATSL_OK) return rc;
+    const int NT = (T + 63) / 64;
+    kern<<<dim3(NT, H, B), PT_THREADS, L::total, st>>>(mq, mk, mv, mw, mu, mp, q ? 1 : 0, g, beta, beta_dtype, gcs, k_rstd, q_rstd, T, H,
+                                                       use_l2norm, status);
+    return check_launch("natsl_gdn_chunk_prep");
+}
+int prep_tc64(const void* q, const void* k, const void* v, const float* g, const void* beta, int beta_dtype, void* w, void* u, float* gcs,
+              float* k_rstd, float* q_rstd, void* pmat, int B, int T, int H, int use_l2norm, cudaStream_t st) {
+    return launch_prep_tc<64>(q, k, v, g, beta, beta_dtype, w, u, gcs, k_rstd, q_rstd, pmat, B, T, H, use_l2norm, st);
 }
 
 }  // namespace natsl
-
-#ifdef NATSL_PREP_TIMING
-extern "C" int natsl_prep_tc_set_timing(long long* p) {
-    return cudaMemcpyToSymbol(natsl::g_prep_ts, &p, sizeof(p)) == cudaSuccess ? 0 : 1;
-}
-#endif
 
 extern "C" int natsl_gdn_chunk_prep_tc(const void* q, const void* k, const void* v, const float* g, const void* beta,
                                        int beta_dtype, void* w, void* u, float* gcs, float* k_rstd, float* q_rstd,
@@ -499,26 +554,6 @@ extern "C" int natsl_gdn_chunk_prep_tc(const void* q, const void* k, const void*
                   "natsl_gdn_chunk_prep_tc: beta must be bf16 or f32");
     NATSL_REQUIRE(K == 128 && V == 128, NATSL_ERR_UNSUPPORTED,
                   "natsl_gdn_chunk_prep_tc: built for K = V = 128 (got K=%d V=%d); use natsl_gdn_chunk_prep_ex", K, V);
-    auto kern = gdn_prep_tc_kernel;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PtSmem::total);
-    if (e != cudaSuccess) {
-        set_error("natsl_gdn_chunk_prep_tc: cannot reserve %d B of shared memory (%s)", PtSmem::total, cudaGetErrorString(e));
-        return NATSL_ERR_CUDA;
-    }
-    CUtensorMap mq, mk, mv, mw, mu, mp;
-    int rc = encode_bthd_map(&mk, k, B, T, H, K, 64, "natsl_gdn_chunk_prep_tc(k)");
-    if (rc == NATSL_OK) rc = encode_bthd_map(&mv, v, B, T, H, V, 64, "natsl_gdn_chunk_prep_tc(v)");
-    if (rc == NATSL_OK) rc = encode_bthd_map(&mq, q ? q : k, B, T, H, K, 64, "natsl_gdn_chunk_prep_tc(q)");
-    if (rc == NATSL_OK) rc = encode_bthd_map(&mw, w, B, T, H, K, 64, "natsl_gdn_chunk_prep_tc(w)");
-    if (rc == NATSL_OK) rc = encode_bthd_map(&mu, u, B, T, H, V, 64, "natsl_gdn_chunk_prep_tc(u)");
-    if (rc == NATSL_OK) rc = pmat ? encode_bthd_map(&mp, pmat, B, T, H, 64, 64, "natsl_gdn_chunk_prep_tc(P)") : NATSL_OK;
-    if (!pmat) mp = mk;
-    int* status = nullptr;
-    if (rc == NATSL_OK) rc = status_word_ptr(&status);
-    if (rc != NATSL_OK) return rc;
-    const int NT = (T + 63) / 64;
-    dim3 grid(NT, H, B);
-    kern<<<grid, PT_THREADS, PtSmem::total, reinterpret_cast<cudaStream_t>(stream)>>>(
-        mq, mk, mv, mw, mu, mp, q ? 1 : 0, g, beta, beta_dtype, gcs, k_rstd, q_rstd, T, H, use_l2norm, status);
-    return check_launch("natsl_gdn_chunk_prep_tc");
+    return launch_prep_tc<128>(q, k, v, g, beta, beta_dtype, w, u, gcs, k_rstd, q_rstd, pmat, B, T, H, use_l2norm,
+                               reinterpret_cast<cudaStream_t>(stream));
 }
