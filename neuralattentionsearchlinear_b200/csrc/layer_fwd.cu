@@ -16,150 +16,8 @@ namespace {
 using bf16 = __nv_bfloat16;
 
 __device__ __forceinline__ float bf(const bf16* p, long i) { return __bfloat162float(p[i]); }
-__device__ __forceinline__ float rb(float x) { return __bfloat162float(__float2bfloat16(x)); }
 __device__ __forceinline__ float ldw(const void* p, int f32, long i) {
     return f32 ? reinterpret_cast<const float*>(p)[i] : __bfloat162float(reinterpret_cast<const bf16*>(p)[i]);
-}
-
-// ------------------------------------------------------------------------------------------------ narrow projections
-// y[t, n] = x[t, :] . W[n, :] for a few rows n (2 H decays and betas, or 2 HQ mixing logits) with the pointwise steps
-// behind it.  Bound by reading x once; the torch form read it once per GEMM and took seven more kernels over the results.
-// One CTA = one 64-token chunk: eight warps = 2 groups of 32 tokens x 4 slices of the contraction, fragments loaded
-// straight from global memory (a lane's 16 bytes are the fragment pairs of a 32-wide k group under a permuted k order).
-struct NarrowArgs {
-    const bf16 *x, *w0, *w1;                  // x [B,T,Kdim]; w0 [n0,Kdim], w1 [n1,Kdim] or NULL
-    int n0, n1, T, Kdim, mode;                // mode 0: decays (w0) and betas (w1); mode 1: softmax over pairs of rows
-    const void *A_log, *dt_bias;
-    int alog_f32, dt_f32, neg_eigval;
-    float *g, *gcs, *dt;                      // [B,T,n0]; gcs, dt or NULL
-    bf16* out;                                // mode 0: beta [B,T,n1]; mode 1: weights [B,T,n0]
-};
-
-template <int NB>
-__global__ void __launch_bounds__(256) narrow_kernel(const NarrowArgs a) {
-    constexpr int N = NB * 8, LD = N + 1;
-    extern __shared__ float red[];            // [4][64][LD]
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-    const int mg = warp & 1, wk = warp >> 1;
-    const int c = blockIdx.x, b = blockIdx.y, valid = min(64, a.T - c * 64);
-    const int n_all = a.n0 + a.n1, n_base = blockIdx.z * N;
-    const bf16* x = a.x + ((long)b * a.T + (long)c * 64) * a.Kdim;
-    const int nc = a.Kdim / 32, c0 = nc * wk / 4, c1 = nc * (wk + 1) / 4;
-    const bf16* xr[4];
-    const bf16* wr[NB];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) xr[i] = x + (long)min(mg * 32 + i * 8 + g, valid - 1) * a.Kdim + t * 8;
-#pragma unroll
-    for (int n = 0; n < NB; ++n) {
-        const int row = min(n_base + n * 8 + g, n_all - 1);
-        wr[n] = (row < a.n0 ? a.w0 + (long)row * a.Kdim : a.w1 + (long)(row - a.n0) * a.Kdim) + t * 8;
-    }
-    float acc[2][NB][4];
-#pragma unroll
-    for (int m = 0; m < 2; ++m)
-#pragma unroll
-        for (int n = 0; n < NB; ++n)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc[m][n][e] = 0.f;
-    constexpr int UN = NB >= 8 ? 1 : 2;
-    for (int k = c0; k < c1; k += UN) {
-        uint4 xv[UN][4], wv[UN][NB];
-#pragma unroll
-        for (int u = 0; u < UN; ++u) {
-            const int kk = min(k + u, c1 - 1) * 32;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) xv[u][i] = *reinterpret_cast<const uint4*>(xr[i] + kk);
-#pragma unroll
-            for (int n = 0; n < NB; ++n) wv[u][n] = __ldg(reinterpret_cast<const uint4*>(wr[n] + kk));
-        }
-#pragma unroll
-        for (int u = 0; u < UN; ++u) {
-            if (k + u >= c1) break;
-#pragma unroll
-            for (int m = 0; m < 2; ++m) {
-                const uint4 p = xv[u][2 * m], q = xv[u][2 * m + 1];
-                const uint32_t f0[4] = {p.x, q.x, p.y, q.y}, f1[4] = {p.z, q.z, p.w, q.w};
-#pragma unroll
-                for (int n = 0; n < NB; ++n) {
-                    mma_bf16(acc[m][n], f0, wv[u][n].x, wv[u][n].y);
-                    mma_bf16(acc[m][n], f1, wv[u][n].z, wv[u][n].w);
-                }
-            }
-        }
-    }
-#pragma unroll
-    for (int m = 0; m < 2; ++m)
-#pragma unroll
-        for (int n = 0; n < NB; ++n)
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-                red[(wk * 64 + mg * 32 + m * 16 + g + 8 * (e >> 1)) * LD + n * 8 + 2 * t + (e & 1)] = acc[m][n][e];
-    __syncthreads();
-    const long tok0 = (long)b * a.T + (long)c * 64;
-    auto total = [&](int r, int n) {
-        return rb(((red[r * LD + n] + red[(64 + r) * LD + n]) + red[(128 + r) * LD + n]) + red[(192 + r) * LD + n]);
-    };
-    if (a.mode == 1) {
-        for (int i = tid; i < 64 * (N / 2); i += 256) {
-            const int r = i / (N / 2), n = (i % (N / 2)) * 2;
-            if (r < valid && n_base + n < a.n0) {
-                const float l0 = total(r, n), l1 = total(r, n + 1), mx = fmaxf(l0, l1);
-                const float e0 = expf(l0 - mx), e1 = expf(l1 - mx), s = e0 + e1;
-                *reinterpret_cast<__nv_bfloat162*>(a.out + (tok0 + r) * a.n0 + n_base + n) = __floats2bfloat162_rn(e0 / s, e1 / s);
-            }
-        }
-        return;
-    }
-    for (int i = tid; i < 64 * N; i += 256) {
-        const int r = i / N, nn = i % N, n = n_base + nn;
-        float gt = 0.f;
-        if (r < valid && n < n_all) {
-            const float y = total(r, nn);
-            if (n < a.n0) {
-                const float z = y + ldw(a.dt_bias, a.dt_f32, n);
-                const float sp = z > 20.f ? z : log1pf(expf(z));
-                gt = -expf(ldw(a.A_log, a.alog_f32, n)) * sp;
-                a.g[(tok0 + r) * a.n0 + n] = gt;
-                if (a.dt) a.dt[(tok0 + r) * a.n0 + n] = sp;
-            } else {
-                float be = rb(1.f / (1.f + expf(-y)));
-                if (a.neg_eigval) be *= 2.f;
-                a.out[(tok0 + r) * a.n1 + n - a.n0] = __float2bfloat16(be);
-            }
-        }
-        if (a.gcs) red[r * LD + nn] = gt;                  // this thread's own entry: nobody else reads it before the barrier
-    }
-    if (a.gcs) {                                           // chunk-local cumsum, one warp per head
-        __syncthreads();
-        for (int nn = warp; nn < N && n_base + nn < a.n0; nn += 8) {
-            float lo = red[lane * LD + nn], hi = red[(lane + 32) * LD + nn];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const float u = __shfl_up_sync(0xffffffffu, lo, o), v = __shfl_up_sync(0xffffffffu, hi, o);
-                if (lane >= o) { lo += u; hi += v; }
-            }
-            hi += __shfl_sync(0xffffffffu, lo, 31);
-            if (lane < valid) a.gcs[(tok0 + lane) * a.n0 + n_base + nn] = lo;
-            if (lane + 32 < valid) a.gcs[(tok0 + lane + 32) * a.n0 + n_base + nn] = hi;
-        }
-    }
-}
-
-int launch_narrow(const NarrowArgs& a, int B, cudaStream_t st) {
-    const int n = a.n0 + a.n1;
-    const int NB = n <= 16 ? 2 : n <= 32 ? 4 : 8;
-    const size_t smem = (size_t)4 * 64 * (NB * 8 + 1) * 4;
-    dim3 grid((a.T + 63) / 64, B, (n + NB * 8 - 1) / (NB * 8));
-    cudaError_t e = cudaSuccess;
-    if (NB == 8) e = cudaFuncSetAttribute(narrow_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) {
-        set_error("natsl_layer_forward: cannot reserve %d B of shared memory (%s)", (int)smem, cudaGetErrorString(e));
-        return NATSL_ERR_CUDA;
-    }
-    if (NB == 2) narrow_kernel<2><<<grid, 256, smem, st>>>(a);
-    else if (NB == 4) narrow_kernel<4><<<grid, 256, smem, st>>>(a);
-    else narrow_kernel<8><<<grid, 256, smem, st>>>(a);
-    return check_launch("natsl_layer_forward (narrow projection)");
 }
 
 // ------------------------------------------------------------------------------------------------ convolutions + norms

@@ -52,15 +52,11 @@ static EncodeTiledFn encode_fn() {
     return fn;
 }
 
-int encode_bthd_map(CUtensorMap* out, const void* base, int B, int T, int H, int D, int box_rows, const char* who, int box_cols) {
+static int encode_map(CUtensorMap* out, const void* base, int B, int T, int H, int D, int box_rows, const char* who, int box_cols) {
     EncodeTiledFn enc = encode_fn();
     if (!enc) {
         set_error("%s: the driver does not provide cuTensorMapEncodeTiled", who);
         return NATSL_ERR_CUDA;
-    }
-    if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || D % box_cols != 0) {
-        set_error("%s: TMA needs a 16-byte aligned base and a head dim multiple of %d (D=%d)", who, box_cols, D);
-        return NATSL_ERR_UNSUPPORTED;
     }
     cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)H, (cuuint64_t)T, (cuuint64_t)B};
     cuuint64_t strides[3] = {(cuuint64_t)D * 2, (cuuint64_t)H * D * 2, (cuuint64_t)T * H * D * 2};
@@ -75,6 +71,22 @@ int encode_bthd_map(CUtensorMap* out, const void* base, int B, int T, int H, int
         return NATSL_ERR_CUDA;
     }
     return NATSL_OK;
+}
+
+int encode_bthd_map(CUtensorMap* out, const void* base, int B, int T, int H, int D, int box_rows, const char* who, int box_cols) {
+    if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || D % box_cols != 0) {
+        set_error("%s: TMA needs a 16-byte aligned base and a head dim multiple of %d (D=%d)", who, box_cols, D);
+        return NATSL_ERR_UNSUPPORTED;
+    }
+    return encode_map(out, base, B, T, H, D, box_rows, who, box_cols);
+}
+
+int encode_rows_map(CUtensorMap* out, const void* base, int B, int T, int D, int box_rows, const char* who) {
+    if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || D % 8 != 0) {
+        set_error("%s: TMA needs a 16-byte aligned base and rows of a multiple of 8 elements (%d)", who, D);
+        return NATSL_ERR_UNSUPPORTED;
+    }
+    return encode_map(out, base, B, T, 1, D, box_rows, who, 64);
 }
 
 // Self-test of the bounded-wait path: one warp waits on an mbarrier that nobody arrives at, with the same wait loop

@@ -256,5 +256,8 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
 // layout of swz<128> / swz<64>), zero fill out of range.
 int encode_bthd_map(CUtensorMap* out, const void* base, int B, int T, int H, int D, int box_rows, const char* who,
                     int box_cols = 64);
+// bf16 rows [B][T][D] (contiguous, D any multiple of 8) in boxes of 64 elements x `box_rows` rows, 128-byte swizzle, zero fill out
+// of range.
+int encode_rows_map(CUtensorMap* out, const void* base, int B, int T, int D, int box_rows, const char* who);
 
 }  // namespace natsl
