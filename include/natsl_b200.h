@@ -353,6 +353,7 @@ int natsl_decode_step(const natsl_decode_args* args, void* stream);
  * natsl_sp_prefix_states: for N consecutive segments (a [N,B,H], S [N,B,H,K,V] fp32) and the state h0 [B,H,K,V]
  *   (or NULL = zero) the first one starts from: P[0] = h0, P[i+1] = a[i] P[i] + S[i]; writes prefix [N,B,H,K,V] = P[0..N)
  *   (or NULL), total_S [B,H,K,V] = P[N] (or NULL) and total_a [B,H] = prod a (or NULL).
+ * natsl_sp_prefix_states_scaled: the same with S[i] trail[i] in the place of S[i] (trail [N,B,H] or NULL).
  * natsl_pack_selected_blocks: packed [B, cap_blocks*nbs, H, D] <- the selected blocks (column `op`) of
  *   x [B,T,H,D] bf16 in index-table order, per head; slots past the number of selected blocks are left untouched.
  * natsl_pack_selected_pairs: packed [B, cap_pairs*nbs, D] <- the same blocks with no padding: the selected
@@ -365,6 +366,8 @@ int natsl_sp_state_combine(const float* a, const float* S, float* h_in, int rank
                            void* stream);
 int natsl_sp_prefix_states(const float* a, const float* S, const float* h0, float* prefix, float* total_S,
                            float* total_a, int N, int B, int H, int K, int V, void* stream);
+int natsl_sp_prefix_states_scaled(const float* a, const float* S, const float* trail, const float* h0, float* prefix,
+                                  float* total_S, float* total_a, int N, int B, int H, int K, int V, void* stream);
 int natsl_pack_selected_blocks(const void* x, const int32_t* indices, const int32_t* n_blocks, void* packed, int B,
                                int T, int H, int HN, int D, int nbs, int op, int cap_blocks, void* stream);
 int natsl_pack_selected_pairs(const void* x, const int32_t* indices, const int32_t* n_blocks, void* packed, int B,

@@ -30,6 +30,7 @@ PROTOTYPES = {
                              _i, _f, _i, _p],
     "natsl_pack_selected_pairs": [_p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _i, _i, _p],
     "natsl_sp_prefix_states": [_p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _p],
+    "natsl_sp_prefix_states_scaled": [_p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _p],
     "natsl_sp_segment_decay": [_p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _p],
     "natsl_sp_state_combine": [_p, _p, _p, _i, _i, _i, _i, _i, _i, _p],
     "natsl_pack_selected_blocks": [_p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _i, _p],
