@@ -227,18 +227,31 @@ __device__ __forceinline__ void load_b_kn(uint32_t tile, int k0, int n0, int lan
 }
 
 // Copy a [ROWS][COLS] bf16 tile from global (row stride `gstride` elements) into a swizzled
-// shared tile with cp.async; rows >= valid_rows are zero-filled.  NT = threads taking part.
+// shared tile with cp.async; rows >= valid_rows are zero-filled.  NT = threads taking part.  A thread's 16-byte chunks lie
+// NT / CPR rows apart: where that is a multiple of eight the swizzle is the same for all of them, and a chunk costs two additions.
 template <int ROWS, int COLS, int NT>
 __device__ __forceinline__ void load_tile_async(uint32_t tile, const __nv_bfloat16* g, long gstride, int valid_rows,
                                                 int tid) {
     constexpr int CPR = COLS / 8;  // 16-byte chunks per row
-    constexpr int TOTAL = ROWS * CPR;
+    constexpr int TOTAL = ROWS * CPR, RS = NT / CPR;
+    if constexpr (NT % CPR == 0 && RS % 8 == 0 && ROWS % RS == 0) {
+        const int r0 = tid / CPR, c = tid % CPR;
+        const uint32_t dst = tile + swz<COLS * 2>(r0, c);
+        const __nv_bfloat16* src = g + (long)r0 * gstride + c * 8;
 #pragma unroll
-    for (int i = tid; i < TOTAL; i += NT) {
-        int r = i / CPR, c = i % CPR;
-        bool ok = r < valid_rows;
-        const __nv_bfloat16* src = g + (ok ? (long)r * gstride + c * 8 : 0);
-        cp_async16(tile + swz<COLS * 2>(r, c), src, ok ? 16 : 0);
+        for (int j = 0; j < ROWS / RS; ++j) {
+            const bool ok = r0 + j * RS < valid_rows;
+            cp_async16(dst + j * RS * COLS * 2, ok ? src : g, ok ? 16 : 0);
+            src += RS * gstride;
+        }
+    } else {
+#pragma unroll
+        for (int i = tid; i < TOTAL; i += NT) {
+            int r = i / CPR, c = i % CPR;
+            bool ok = r < valid_rows;
+            const __nv_bfloat16* src = g + (ok ? (long)r * gstride + c * 8 : 0);
+            cp_async16(tile + swz<COLS * 2>(r, c), src, ok ? 16 : 0);
+        }
     }
 }
 
@@ -247,13 +260,25 @@ template <int ROWS, int COLS, int NT>
 __device__ __forceinline__ void store_tile(const unsigned char* tile, __nv_bfloat16* g, long gstride, int valid_rows,
                                            int tid) {
     constexpr int CPR = COLS / 8;
-    constexpr int TOTAL = ROWS * CPR;
+    constexpr int TOTAL = ROWS * CPR, RS = NT / CPR;
+    if constexpr (NT % CPR == 0 && RS % 8 == 0 && ROWS % RS == 0) {
+        const int r0 = tid / CPR, c = tid % CPR;
+        const unsigned char* src = tile + swz<COLS * 2>(r0, c);
+        __nv_bfloat16* dst = g + (long)r0 * gstride + c * 8;
 #pragma unroll
-    for (int i = tid; i < TOTAL; i += NT) {
-        int r = i / CPR, c = i % CPR;
-        if (r < valid_rows) {
-            uint4 v = *reinterpret_cast<const uint4*>(tile + swz<COLS * 2>(r, c));
-            *reinterpret_cast<uint4*>(g + (long)r * gstride + c * 8) = v;
+        for (int j = 0; j < ROWS / RS; ++j) {
+            if (r0 + j * RS < valid_rows)
+                *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(src + j * RS * COLS * 2);
+            dst += RS * gstride;
+        }
+    } else {
+#pragma unroll
+        for (int i = tid; i < TOTAL; i += NT) {
+            int r = i / CPR, c = i % CPR;
+            if (r < valid_rows) {
+                uint4 v = *reinterpret_cast<const uint4*>(tile + swz<COLS * 2>(r, c));
+                *reinterpret_cast<uint4*>(g + (long)r * gstride + c * 8) = v;
+            }
         }
     }
 }

@@ -31,7 +31,7 @@ namespace natsl {
 
 constexpr int LB_THREADS = 256;
 constexpr int LB_A_LD = 68;
-constexpr int LB_X_LD = 17;
+constexpr int LB_X_LD = 20;
 
 __device__ __forceinline__ float kdecay(float gl, float g, bool gdn) {
     const float d = gl - g;
@@ -96,7 +96,7 @@ linear_bwd_pre_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* 
                       __nv_bfloat16* __restrict__ kn, float* __restrict__ q_rstd, float* __restrict__ k_rstd,
                       __nv_bfloat16* __restrict__ dvl, int T, int H, float scale, int use_l2norm) {
     using L = PreSmem<K, V>;
-    extern __shared__ __align__(128) unsigned char smem[];
+    extern __shared__ __align__(256) unsigned char smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int gq = lane >> 2, qd = lane & 3;
     const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
@@ -138,7 +138,7 @@ linear_bwd_pre_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* 
     {
         float acc[4][4];
         zero_acc(acc);
-        warp_gemm<K * 2, A_ROW, K * 2, B_NK, 4>(acc, qs, r0, ks, 32 * half, 0, K, lane);
+        warp_gemm<K * 2, A_ROW, K * 2, B_NK, K, 4>(acc, qs, r0, ks, 32 * half, lane);
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
@@ -155,7 +155,7 @@ linear_bwd_pre_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* 
         constexpr int NT8 = V / 16;
         float acc[NT8][4];
         zero_acc(acc);
-        warp_gemm<128, A_TRANS, V * 2, B_KN, NT8>(acc, ps, r0, dos, half * (V / 2), 0, 64, lane);
+        warp_gemm<128, A_TRANS, V * 2, B_KN, 64, NT8>(acc, ps, r0, dos, half * (V / 2), lane);
 #pragma unroll
         for (int nt = 0; nt < NT8; ++nt)
 #pragma unroll
@@ -198,7 +198,7 @@ linear_bwd_dh_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat16* 
     constexpr int DH_THREADS = BV * 4;                      // a warp: 16 tokens (K / 4 rows of dS) x 32 value columns
     constexpr int MT = K / 64;
     constexpr int NTL = 4;
-    extern __shared__ __align__(128) unsigned char smem[];
+    extern __shared__ __align__(256) unsigned char smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int rw = warp & 3, n0 = (warp >> 2) * 32;         // row group, first column
     const int gq = lane >> 2, qd = lane & 3;
@@ -290,7 +290,7 @@ linear_bwd_dh_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat16* 
         // ---- dv' = act (kn dS) kd + dv'_loc
         float acc[NTL][4];
         zero_acc(acc);
-        if (act) warp_gemm<K * 2, A_ROW, BV * 2, B_KN, NTL>(acc, ks, r0, dsb, n0, 0, K, lane);
+        if (act) warp_gemm<K * 2, A_ROW, BV * 2, B_KN, K, NTL>(acc, ks, r0, dsb, n0, lane);
         const float kda = kdecay(gl, s_g[ia], GDN), kdb = kdecay(gl, s_g[ib], GDN);
         const float ec = __expf(car);
         const float ea = scale * __expf(s_g[ia] + car), eb = scale * __expf(s_g[ib] + car);
@@ -330,8 +330,8 @@ linear_bwd_dh_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat16* 
         }
 #pragma unroll
         for (int mt = 0; mt < MT; ++mt) {
-            warp_gemm<K * 2, A_TRANS, BV * 2, B_KN, NTL>(dS[mt], qs, krow0 + mt * 16, smem_u32(dob_p), n0, 0, 64, lane);
-            if (GDN) warp_gemm<K * 2, A_TRANS, BV * 2, B_KN, NTL>(dS[mt], ws, krow0 + mt * 16, smem_u32(dvl_p), n0, 0, 64, lane);
+            warp_gemm<K * 2, A_TRANS, BV * 2, B_KN, 64, NTL>(dS[mt], qs, krow0 + mt * 16, smem_u32(dob_p), n0, lane);
+            if (GDN) warp_gemm<K * 2, A_TRANS, BV * 2, B_KN, 64, NTL>(dS[mt], ws, krow0 + mt * 16, smem_u32(dvl_p), n0, lane);
         }
     }
     if (dht && last_sel < 0) add_dht();                     // no chunk updated the state: the final state is h0
@@ -350,23 +350,27 @@ linear_bwd_dh_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat16* 
 }
 
 // ================================================================================================ state
+// Two phases, so that two CTAs share an SM (128 / 128: 113 KB each; with everything resident one CTA waited for 160 KB per chunk,
+// 507 us at B = 8, T = 4096, 16 heads, now 365 us, 5.1 TB/s): what contracts with S first, then dS and k over the operands that S has used.  The
+// results of the first phase leave from registers meanwhile.
 template <int K, int V, bool GDN>
 struct StSmem {
+    static constexpr int cmax(int x, int y) { return x > y ? x : y; }
+    static constexpr int KB = 64 * K * 2, VB = 64 * V * 2, SB = K * V * 2;
     static constexpr int Ss = 0;                              // S [K][V]
-    static constexpr int dSs = Ss + K * V * 2;                // dS [K][V]
-    static constexpr int ks = dSs + K * V * 2;
-    static constexpr int ws = ks + 64 * K * 2;
-    static constexpr int us = ws + 64 * K * 2;                // u, then v'
-    static constexpr int dvs = us + 64 * V * 2;               // dv'
-    static constexpr int dos = dvs + 64 * V * 2;
-    static constexpr int vs = dos + 64 * V * 2;               // raw v (chunks that do not update the state, GDN)
-    static constexpr int vec = vs + (GDN ? 64 * V * 2 : 0);   // g[64], r[64], red[8 warps][2] + red2[2]
+    static constexpr int us = Ss + SB;                        // u, then v'
+    static constexpr int vs = us + VB;                        // raw v (chunks that do not update the state, GDN)
+    static constexpr int ws = vs + (GDN ? VB : 0);            // w | dv', then dS [K][V]
+    static constexpr int dvs = ws + (GDN ? KB : 0);
+    static constexpr int dos = ws + cmax((GDN ? KB + VB : 0), SB);       // do, then k
+    static constexpr int vec = dos + cmax(VB, KB);            // g[64], r[64], red[8 warps][2] + red2[2]
     static constexpr int total = vec + (64 + 64 + 32) * 4;
-    static_assert(K * V * 2 >= 64 * K * 2, "the dS tile doubles as an output staging buffer");
+    static constexpr int ctas = 3 * (total + 1024) <= 233472 ? 3 : 2;    // per SM, for the register budget
+    static_assert(2 * (total + 1024) <= 233472, "two CTAs per SM");
 };
 
 template <int K, int V, bool GDN>
-__global__ void __launch_bounds__(LB_THREADS)
+__global__ void __launch_bounds__(LB_THREADS, StSmem<K, V, GDN>::ctas)
 linear_bwd_state_kernel(const __nv_bfloat16* __restrict__ kn, const __nv_bfloat16* __restrict__ v,
                         const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ u,
                         const __nv_bfloat16* __restrict__ d_o, const __nv_bfloat16* __restrict__ dvp,
@@ -378,7 +382,7 @@ linear_bwd_state_kernel(const __nv_bfloat16* __restrict__ kn, const __nv_bfloat1
                         __nv_bfloat16* __restrict__ dk1_out, float* __restrict__ dkd_out, float* __restrict__ scal,
                         float* __restrict__ dnats_lin, int T, int H, int HN, float scale, int invalid_dnats) {
     using L = StSmem<K, V, GDN>;
-    extern __shared__ __align__(128) unsigned char smem[];
+    extern __shared__ __align__(256) unsigned char smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int gq = lane >> 2, qd = lane & 3;
     const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
@@ -397,15 +401,11 @@ linear_bwd_state_kernel(const __nv_bfloat16* __restrict__ kn, const __nv_bfloat1
             if (j < nsel) slot = indices[(((long)b * TN + j) * HN + hn) * 2 + 1];
         }
     }
-    unsigned char* Ss_p = smem + L::Ss;
-    unsigned char* dSs_p = smem + L::dSs;
-    unsigned char* ks_p = smem + L::ks;
-    unsigned char* ws_p = smem + L::ws;
+    const unsigned char* Ss_p = smem + L::Ss;
     unsigned char* us_p = smem + L::us;
-    const unsigned char* dvs_p = smem + L::dvs;
-    const unsigned char* vs_p = smem + L::vs;
-    const uint32_t Ss = smem_u32(Ss_p), dSs = smem_u32(dSs_p), ks = smem_u32(ks_p), ws = smem_u32(ws_p), us = smem_u32(us_p),
-                   dvs = smem_u32(smem + L::dvs), dos = smem_u32(smem + L::dos), vs = smem_u32(smem + L::vs);
+    const unsigned char *dSs_p = smem + L::ws, *dvs_p = smem + L::dvs, *vs_p = smem + L::vs;
+    const uint32_t Ss = smem_u32(Ss_p), ws = smem_u32(smem + L::ws), dSs = ws, us = smem_u32(us_p), dvs = smem_u32(dvs_p),
+                   dos = smem_u32(smem + L::dos), ks = dos;
     float* s_g = reinterpret_cast<float*>(smem + L::vec);
     float* s_r = s_g + 64;
     float* s_red = s_r + 64;
@@ -414,13 +414,15 @@ linear_bwd_state_kernel(const __nv_bfloat16* __restrict__ kn, const __nv_bfloat1
     load_tile_async<K, V, LB_THREADS>(Ss, hS + st_off, V, K, tid);
     if (GDN) load_tile_async<64, K, LB_THREADS>(ws, w + (tok0 * H + h) * K, (long)H * K, valid, tid);
     load_tile_async<64, V, LB_THREADS>(us, u + (tok0 * H + h) * V, (long)H * V, valid, tid);
-    load_tile_async<64, V, LB_THREADS>(dvs, dvp + (tok0 * H + h) * V, (long)H * V, valid, tid);
+    if (GDN) load_tile_async<64, V, LB_THREADS>(dvs, dvp + (tok0 * H + h) * V, (long)H * V, valid, tid);
     load_tile_async<64, V, LB_THREADS>(dos, d_o + (tok0 * H + h) * V, (long)H * V, valid, tid);
-    if (slot >= 0) {
-        load_tile_async<K, V, LB_THREADS>(dSs, dS_all + (((long)b * NT + slot) * H + h) * (long)K * V, V, K, tid);
-        load_tile_async<64, K, LB_THREADS>(ks, kn + (tok0 * H + h) * K, (long)H * K, valid, tid);
-        if (GDN && !act) load_tile_async<64, V, LB_THREADS>(vs, v + (tok0 * H + h) * V, (long)H * V, valid, tid);
-    }
+    cp_async_commit();
+    // what the second phase reads; without w and dv' (Mamba2) dS has its place to itself and comes at once
+    auto load_ds = [&]() {
+        if (slot >= 0) load_tile_async<K, V, LB_THREADS>(dSs, dS_all + (((long)b * NT + slot) * H + h) * (long)K * V, V, K, tid);
+    };
+    if (GDN && slot >= 0 && !act) load_tile_async<64, V, LB_THREADS>(smem_u32(vs_p), v + (tok0 * H + h) * V, (long)H * V, valid, tid);
+    if (!GDN) load_ds();
     cp_async_commit();
     if (tid < 64) {
         s_g[tid] = gcs[(tok0 + min(tid, valid - 1)) * H + h];
@@ -429,7 +431,7 @@ linear_bwd_state_kernel(const __nv_bfloat16* __restrict__ kn, const __nv_bfloat1
     if (tid < 32) s_red[tid] = 0.f;
     const float car = carry_in[((long)b * NT + c) * H + h];
     const float ec = __expf(car);
-    cp_async_wait<0>();
+    cp_async_wait<1>();
     __syncthreads();
     const float gl = s_g[valid - 1];
 
@@ -444,7 +446,7 @@ linear_bwd_state_kernel(const __nv_bfloat16* __restrict__ kn, const __nv_bfloat1
     if (GDN) {
         float acc[NV][4];
         zero_acc(acc);
-        warp_gemm<K * 2, A_ROW, V * 2, B_KN, NV>(acc, ws, r0, Ss, nv0, 0, K, lane);
+        warp_gemm<K * 2, A_ROW, V * 2, B_KN, K, NV>(acc, ws, r0, Ss, nv0, lane);
 #pragma unroll
         for (int nt = 0; nt < NV; ++nt) {
             const int col = nv0 + nt * 8 + qd * 2;
@@ -457,13 +459,42 @@ linear_bwd_state_kernel(const __nv_bfloat16* __restrict__ kn, const __nv_bfloat1
             *pb = pack_bf16(ub.x - ec * acc[nt][2], ub.y - ec * acc[nt][3]);
         }
     }
-    __syncthreads();                                         // v' complete (rows are shared by two warps)
+    // ---- products with S over the value dim: dqn1 = s e^{g+car} do S^T, dw = -e^{car} dv' S^T
+    {
+        float acc_q[NK][4], acc_w[GDN ? NK : 2][4];
+        zero_acc(acc_q);
+        warp_gemm<V * 2, A_ROW, V * 2, B_NK, V, NK>(acc_q, dos, r0, Ss, nk0, lane);
+        if constexpr (GDN) {
+            zero_acc(acc_w);
+            warp_gemm<V * 2, A_ROW, V * 2, B_NK, V, NK>(acc_w, dvs, r0, Ss, nk0, lane);
+        }
+        __syncthreads();                                     // w, dv' and do are done with; v' complete (rows are shared by two warps)
+        if (GDN) load_ds();
+        if (slot >= 0) load_tile_async<64, K, LB_THREADS>(ks, kn + (tok0 * H + h) * K, (long)H * K, valid, tid);
+        cp_async_commit();
+        const float ea = scale * __expf(s_g[ia] + car), eb = scale * __expf(s_g[ib] + car);
+#pragma unroll
+        for (int nt = 0; nt < NK; ++nt) {
+            acc_q[nt][0] *= ea; acc_q[nt][1] *= ea; acc_q[nt][2] *= eb; acc_q[nt][3] *= eb;
+            if constexpr (GDN) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc_w[nt][e] *= -ec;
+            }
+        }
+        store_acc_global<NK>(dq1_out + (tok0 * H + h) * K, (long)H * K, acc_q, r0, nk0, valid, lane);
+        if constexpr (GDN) {
+            store_acc_global<NK>(dw_out + (tok0 * H + h) * K, (long)H * K, acc_w, r0, nk0, valid, lane);
+            store_tile<64, V, LB_THREADS>(us_p, vp_out + (tok0 * H + h) * V, (long)H * V, valid, tid);
+        }
+    }
+    cp_async_wait<0>();
+    __syncthreads();                                         // dS and k in place
 
     // ---- r_i = sum_v (kn dS)_iv x_iv,  x = v' (updating chunk) or the raw values (other chunks, for dnats)
     if (slot >= 0) {
         float acc[NV][4];
         zero_acc(acc);
-        warp_gemm<K * 2, A_ROW, V * 2, B_KN, NV>(acc, ks, r0, dSs, nv0, 0, K, lane);
+        warp_gemm<K * 2, A_ROW, V * 2, B_KN, K, NV>(acc, ks, r0, dSs, nv0, lane);
         const unsigned char* x_p = (GDN && !act) ? vs_p : us_p;
         float ra = 0.f, rb = 0.f;
 #pragma unroll
@@ -480,32 +511,16 @@ linear_bwd_state_kernel(const __nv_bfloat16* __restrict__ kn, const __nv_bfloat1
             atomicAdd(&s_r[ib], rb);
         }
     }
-    // ---- products with S and dS over the value dim: dkn1 = kd (v' dS^T), dqn1 = s e^{g+car} do S^T, dw = -e^{car} dv' S^T
-    float acc_k[NK][4], acc_q[NK][4], acc_w[GDN ? NK : 2][4];
-    zero_acc(acc_k);
-    zero_acc(acc_q);
-    if (act) warp_gemm<V * 2, A_ROW, V * 2, B_NK, NK>(acc_k, us, r0, dSs, nk0, 0, V, lane);
-    warp_gemm<V * 2, A_ROW, V * 2, B_NK, NK>(acc_q, dos, r0, Ss, nk0, 0, V, lane);
-    if constexpr (GDN) {
-        zero_acc(acc_w);
-        warp_gemm<V * 2, A_ROW, V * 2, B_NK, NK>(acc_w, dvs, r0, Ss, nk0, 0, V, lane);
-    }
-    {
-        const float kda = kdecay(gl, s_g[ia], GDN), kdb = kdecay(gl, s_g[ib], GDN);
-        const float ea = scale * __expf(s_g[ia] + car), eb = scale * __expf(s_g[ib] + car);
-#pragma unroll
-        for (int nt = 0; nt < NK; ++nt) {
-            acc_k[nt][0] *= kda; acc_k[nt][1] *= kda; acc_k[nt][2] *= kdb; acc_k[nt][3] *= kdb;
-            acc_q[nt][0] *= ea; acc_q[nt][1] *= ea; acc_q[nt][2] *= eb; acc_q[nt][3] *= eb;
-            if constexpr (GDN) {
-#pragma unroll
-                for (int e = 0; e < 4; ++e) acc_w[nt][e] *= -ec;
-            }
-        }
-    }
-    // ---- ddec = e^{g_L+car} <dS, S>
+    // ---- dkn1 = kd (v' dS^T),  ddec = e^{g_L+car} <dS, S>
     float dd = 0.f;
     if (act) {
+        float acc_k[NK][4];
+        zero_acc(acc_k);
+        warp_gemm<V * 2, A_ROW, V * 2, B_NK, V, NK>(acc_k, us, r0, dSs, nk0, lane);
+        const float kda = kdecay(gl, s_g[ia], GDN), kdb = kdecay(gl, s_g[ib], GDN);
+#pragma unroll
+        for (int nt = 0; nt < NK; ++nt) { acc_k[nt][0] *= kda; acc_k[nt][1] *= kda; acc_k[nt][2] *= kdb; acc_k[nt][3] *= kdb; }
+        store_acc_global<NK>(dk1_out + (tok0 * H + h) * K, (long)H * K, acc_k, r0, nk0, valid, lane);
         constexpr int CPR = V / 8;
         for (int i = tid; i < K * CPR; i += LB_THREADS) {
             const int r = i / CPR, cc = i % CPR;
@@ -526,7 +541,7 @@ linear_bwd_state_kernel(const __nv_bfloat16* __restrict__ kn, const __nv_bfloat1
         s_red[2 * warp] = dd;
         s_red[2 * warp + 1] = t1;
     }
-    __syncthreads();                                         // all products done: k, w, dS tiles become staging buffers
+    __syncthreads();
     // ---- per-token decay gradient of the state write, dnats
     if (tid < 64) {
         const float kd = kdecay(gl, s_g[tid], GDN);
@@ -537,16 +552,7 @@ linear_bwd_state_kernel(const __nv_bfloat16* __restrict__ kn, const __nv_bfloat1
         dn = warp_sum(dn);
         if (lane == 0) s_red[16 + warp] = dn;
     }
-    store_acc_bf16<K * 2, NK>(ks_p, acc_k, r0, nk0, lane);
-    store_acc_bf16<K * 2, NK>(ws_p, acc_q, r0, nk0, lane);
-    if constexpr (GDN) store_acc_bf16<K * 2, NK>(dSs_p, acc_w, r0, nk0, lane);
     __syncthreads();
-    if (act) store_tile<64, K, LB_THREADS>(ks_p, dk1_out + (tok0 * H + h) * K, (long)H * K, valid, tid);
-    store_tile<64, K, LB_THREADS>(ws_p, dq1_out + (tok0 * H + h) * K, (long)H * K, valid, tid);
-    if (GDN) {
-        store_tile<64, K, LB_THREADS>(dSs_p, dw_out + (tok0 * H + h) * K, (long)H * K, valid, tid);
-        store_tile<64, V, LB_THREADS>(us_p, vp_out + (tok0 * H + h) * V, (long)H * V, valid, tid);
-    }
     if (tid == 0) {
         float* sc = scal + (((long)b * NT + c) * H + h) * 4;
         const float dn = s_red[16] + s_red[17];
@@ -566,8 +572,9 @@ linear_bwd_state_kernel(const __nv_bfloat16* __restrict__ kn, const __nv_bfloat1
 // Six tile buffers hold what each phase needs, loaded behind the products of the phase before, so that two CTAs share an
 // SM: alone, a CTA is a chain of short phases that leaves the SM waiting at its barriers and loads.
 //     c: do, then dv' -> dzu -> dv      d: v', then dw -> dzw
-//     e: H, then u, then dq1 (later dq staging)      f: A, then w, then dk1 (later dk staging)
-//     m: dqk, then the diagonal blocks X, then dkk
+//     e: dq1, then H, then u      f: A, then w, then dk1      m: dqk, then the diagonal blocks X, then dkk
+// dq is finished and stored before the solves, so that its accumulators do not live through them (they were spilled: 709 us at
+// B = 8, T = 4096, 16 heads of 128 / 128, now 637 us); dq and dk leave from registers.
 template <int K, int V, bool GDN>
 struct InSmem {
     static constexpr int cmax(int x, int y) { return x > y ? x : y; }
@@ -581,10 +588,10 @@ struct InSmem {
     static constexpr int m = f + (GDN ? cmax(KB, 64 * LB_A_LD * 4) : KB);     // A: fp32 [64][68]
     static constexpr int vec = m + 64 * 64 * 2;
     // g, beta, zk, dE, dotq, dotk (6 x 64); decay-gradient row sums [2 phases][2 halves][64] and column sums
-    // [2 phases][4 row blocks][64]; dbeta parts [2 halves + value part][64]; + 16
-    static constexpr int total = vec + ((6 + 4 + 8 + 3) * 64 + 16) * 4;
+    // [2 phases][4 row blocks][64]; dbeta parts [2 halves + value part][64]; q rstd, k rstd, dkd (3 x 64); + 16
+    static constexpr int total = vec + ((6 + 4 + 8 + 3 + 3) * 64 + 16) * 4;
     static_assert(4 * 16 * LB_X_LD * 4 <= 64 * 64 * 2, "the X blocks fit over dqk");
-    static_assert(total <= 115712, "two CTAs per SM");
+    static_assert(total <= 115712, "two CTAs per SM");        // (a third one at 64 / 64: 80 registers, 425 -> 443 us)
 };
 
 // In-place solve of (I + A)^T X = R for 32 columns [col0, col0+32) of a [64][COLS] bf16 tile by one warp:
@@ -592,18 +599,20 @@ struct InSmem {
 // Y_j = R_i for j = i and the already solved X_j for j > i.
 template <int COLS>
 __device__ __forceinline__ void solve_t_group(uint32_t htile, uint32_t ztile, unsigned char* zptr, int col0, int lane) {
+    const uint32_t bt = b_addr<COLS * 2, B_KN>(ztile, col0, lane);
 #pragma unroll
     for (int i = 3; i >= 0; --i) {
         float acc[4][4];
         zero_acc(acc);
+        const uint32_t at = a_addr<128, A_TRANS>(htile, 16 * i, lane);
 #pragma unroll
         for (int j = i; j < 4; ++j) {
             uint32_t af[4];
-            load_a_t<128>(htile, 16 * i, 16 * j, lane, af);
+            ld_a<128, A_TRANS>(at, 16 * j, af);
 #pragma unroll
             for (int p = 0; p < 2; ++p) {
                 uint32_t bf[4];
-                load_b_kn<COLS * 2>(ztile, 16 * j, col0 + 16 * p, lane, bf);
+                ld_b<COLS * 2, B_KN>(bt, p, 16 * j, bf);
                 mma_bf16(acc[2 * p], af, bf[0], bf[1]);
                 mma_bf16(acc[2 * p + 1], af, bf[2], bf[3]);
             }
@@ -628,7 +637,7 @@ linear_bwd_intra_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat1
                         float* __restrict__ dg_tok, float* __restrict__ scal, int T, int H, int HN, float scale,
                         int use_l2norm) {
     using L = InSmem<K, V, GDN>;
-    extern __shared__ __align__(128) unsigned char smem[];
+    extern __shared__ __align__(256) unsigned char smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int gq = lane >> 2, qd = lane & 3;
     const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
@@ -658,17 +667,20 @@ linear_bwd_intra_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat1
     float* s_dgr = s_dotk + 64;                              // [phase][half][64]: one writer per slot, fixed summation order
     float* s_dgc = s_dgr + 4 * 64;                           // [phase][row block][64]
     float* s_dbp = s_dgc + 8 * 64;                           // [half 0 | half 1 | value part][64]
-    float* s_red = s_dbp + 3 * 64;
+    float* s_qr = s_dbp + 3 * 64;
+    float* s_kr = s_qr + 64;
+    float* s_dkd = s_kr + 64;
+    float* s_red = s_dkd + 64;
 
     load_tile_async<64, K, LB_THREADS>(qns, qn + (tok0 * H + h) * K, (long)H * K, valid, tid);
     load_tile_async<64, K, LB_THREADS>(kns, kn + (tok0 * H + h) * K, (long)H * K, valid, tid);
     load_tile_async<64, V, LB_THREADS>(dt, vp + (tok0 * H + h) * V, (long)H * V, valid, tid);
     load_tile_async<64, V, LB_THREADS>(ct, d_o + (tok0 * H + h) * V, (long)H * V, valid, tid);
-    auto load_state_parts = [&]() {                          // dk1 exists for updating chunks only
-        load_tile_async<64, K, LB_THREADS>(et, dq1 + (tok0 * H + h) * K, (long)H * K, valid, tid);
+    load_tile_async<64, K, LB_THREADS>(et, dq1 + (tok0 * H + h) * K, (long)H * K, valid, tid);
+    auto load_dk1 = [&]() {                                  // dk1 exists for updating chunks only
         if (act) load_tile_async<64, K, LB_THREADS>(ft, dk1 + (tok0 * H + h) * K, (long)H * K, valid, tid);
     };
-    if (!GDN) load_state_parts();
+    if (!GDN) load_dk1();
     cp_async_commit();
     if (tid < 64) {
         const long gi = (tok0 + min(tid, valid - 1)) * H + h;
@@ -678,6 +690,9 @@ linear_bwd_intra_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat1
             bv = beta_dtype == NATSL_DT_F32 ? reinterpret_cast<const float*>(beta)[gi]
                                             : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(beta)[gi]);
         s_b[tid] = bv;
+        s_qr[tid] = use_l2norm ? q_rstd[gi] : 1.f;
+        s_kr[tid] = use_l2norm ? k_rstd[gi] : 1.f;
+        s_dkd[tid] = dkd[gi];
         s_zk[tid] = 0.f; s_dE[tid] = 0.f; s_dotq[tid] = 0.f; s_dotk[tid] = 0.f;
         for (int i = 0; i < 15; ++i) s_dgr[i * 64 + tid] = 0.f;
     }
@@ -697,9 +712,9 @@ linear_bwd_intra_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat1
         float qk[4][4], dpr[4][4];
         zero_acc(qk);
         zero_acc(dpr);
-        warp_gemm<K * 2, A_ROW, K * 2, B_NK, 4>(qk, qns, r0, kns, c0, 0, K, lane);
-        if (GDN) warp_gemm<K * 2, A_ROW, K * 2, B_NK, 4>(kk, kns, r0, kns, c0, 0, K, lane);
-        warp_gemm<V * 2, A_ROW, V * 2, B_NK, 4>(dpr, ct, r0, dt, c0, 0, V, lane);
+        warp_gemm<K * 2, A_ROW, K * 2, B_NK, K, 4>(qk, qns, r0, kns, c0, lane);
+        if (GDN) warp_gemm<K * 2, A_ROW, K * 2, B_NK, K, 4>(kk, kns, r0, kns, c0, lane);
+        warp_gemm<V * 2, A_ROW, V * 2, B_NK, V, 4>(dpr, ct, r0, dt, c0, lane);
         float rs_a = 0.f, rs_b = 0.f;
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) {
@@ -739,48 +754,89 @@ linear_bwd_intra_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat1
         cp_async_commit();
     }
 
-    // ---- phase 2: dqn = dqk kn, dkn = dqk^T qn
+    // ---- phase 2: dqn = dqk kn + dq1, dkn = dqk^T qn; dq
     constexpr int NK = K / 16;
     const int nk0 = half * (K / 2);
-    float acc_q[NK][4], acc_k[NK][4];
-    zero_acc(acc_q);
-    zero_acc(acc_k);
-    warp_gemm<128, A_ROW, K * 2, B_KN, NK>(acc_q, mt, r0, kns, nk0, 0, 64, lane);
-    warp_gemm<128, A_TRANS, K * 2, B_KN, NK>(acc_k, mt, r0, qns, nk0, 0, 64, lane);
+    float acc_k[NK][4];
+    {
+        float acc_q[NK][4];
+        zero_acc(acc_q);
+        warp_gemm<128, A_ROW, K * 2, B_KN, 64, NK>(acc_q, mt, r0, kns, nk0, lane);
+        float dE_a = 0.f, dE_b = 0.f, dq_a = 0.f, dq_b = 0.f;
+#pragma unroll
+        for (int nt = 0; nt < NK; ++nt) {
+            const int col = nk0 + nt * 8 + qd * 2;
+            const float2 qna = load_pair_bf16<K * 2>(qns_p, ia, col), qnb = load_pair_bf16<K * 2>(qns_p, ib, col);
+            const float2 xa = load_pair_bf16<K * 2>(e_p, ia, col), xb = load_pair_bf16<K * 2>(e_p, ib, col);
+            acc_q[nt][0] += xa.x; acc_q[nt][1] += xa.y; acc_q[nt][2] += xb.x; acc_q[nt][3] += xb.y;
+            dE_a += xa.x * qna.x + xa.y * qna.y;
+            dE_b += xb.x * qnb.x + xb.y * qnb.y;
+            dq_a += acc_q[nt][0] * qna.x + acc_q[nt][1] * qna.y;
+            dq_b += acc_q[nt][2] * qnb.x + acc_q[nt][3] * qnb.y;
+        }
+        dE_a = quad_sum(dE_a); dE_b = quad_sum(dE_b);
+        dq_a = quad_sum(dq_a); dq_b = quad_sum(dq_b);
+        if (qd == 0) {
+            atomicAdd(&s_dE[ia], dE_a); atomicAdd(&s_dE[ib], dE_b);
+            atomicAdd(&s_dotq[ia], dq_a); atomicAdd(&s_dotq[ib], dq_b);
+        }
+        zero_acc(acc_k);
+        warp_gemm<128, A_TRANS, K * 2, B_KN, 64, NK>(acc_k, mt, r0, qns, nk0, lane);
+        __syncthreads();                                     // dqk and dq1 have been read, the row sums are complete
+        const float qra = s_qr[ia], qrb = s_qr[ib];
+        const float pq_a = use_l2norm ? s_dotq[ia] : 0.f, pq_b = use_l2norm ? s_dotq[ib] : 0.f;
+#pragma unroll
+        for (int nt = 0; nt < NK; ++nt) {
+            const int col = nk0 + nt * 8 + qd * 2;
+            const float2 qna = load_pair_bf16<K * 2>(qns_p, ia, col), qnb = load_pair_bf16<K * 2>(qns_p, ib, col);
+            acc_q[nt][0] = qra * (acc_q[nt][0] - qna.x * pq_a); acc_q[nt][1] = qra * (acc_q[nt][1] - qna.y * pq_a);
+            acc_q[nt][2] = qrb * (acc_q[nt][2] - qnb.x * pq_b); acc_q[nt][3] = qrb * (acc_q[nt][3] - qnb.y * pq_b);
+        }
+        store_acc_global<NK>(dq + (tok0 * H + h) * K, (long)H * K, acc_q, r0, nk0, valid, lane);
+    }
 
     if (GDN) {
         // ---- phase 3: X_dd = (I + A_dd)^-1 (forward substitution, one warp per diagonal block), then H
-        __syncthreads();                                     // dqk has been read: X goes over it
-        if (warp < 4 && lane < 16) {
-            const int d0 = warp * 16, cidx = lane;
+        if (warp < 2) {                                      // two diagonal blocks per warp, lane = column
+            const int d0 = warp * 32 + (lane & 16), cidx = lane & 15;
             float xcol[16];
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
-                float s = 0.f;
+                float arow[16];
 #pragma unroll
-                for (int j = 0; j < i; ++j) s += As[(d0 + i) * LB_A_LD + d0 + j] * xcol[j];
-                xcol[i] = ((i == cidx) ? 1.f : 0.f) - s;
+                for (int j4 = 0; j4 < 16; j4 += 4)
+                    if (j4 < i) *reinterpret_cast<float4*>(&arow[j4]) = *reinterpret_cast<const float4*>(&As[(d0 + i) * LB_A_LD + d0 + j4]);
+                float p0 = 0.f, p1 = 0.f, p2 = 0.f, p3 = 0.f;
+#pragma unroll
+                for (int j = 0; j < i; ++j) {
+                    const float t = arow[j] * xcol[j];
+                    if ((j & 3) == 0) p0 += t; else if ((j & 3) == 1) p1 += t; else if ((j & 3) == 2) p2 += t; else p3 += t;
+                }
+                xcol[i] = ((i == cidx) ? 1.f : 0.f) - ((p0 + p1) + (p2 + p3));
             }
 #pragma unroll
-            for (int i = 0; i < 16; ++i) Xs[(warp * 16 + i) * LB_X_LD + cidx] = xcol[i];
+            for (int i = 0; i < 16; ++i) Xs[(d0 + i) * LB_X_LD + cidx] = xcol[i];
         }
         __syncthreads();
-        for (int e = tid; e < 4 * 16 * 16; e += LB_THREADS) {          // diagonal blocks: H_dd = X_dd
-            const int d = e >> 8, r = (e >> 4) & 15, cc = e & 15;
-            const int row = d * 16 + r, col = d * 16 + cc;
-            reinterpret_cast<__nv_bfloat16*>(e_p + swz<128>(row, col >> 3))[col & 7] =
-                __float2bfloat16(Xs[(d * 16 + r) * LB_X_LD + cc]);
+        {                                                    // diagonal blocks: H_dd = X_dd, four columns per thread
+            const int row = tid >> 2, c4 = (tid & 3) * 4, col = (row & 48) + c4;
+            const float4 x = *reinterpret_cast<const float4*>(&Xs[row * LB_X_LD + c4]);
+            *reinterpret_cast<uint2*>(e_p + swz<128>(row, col >> 3) + (col & 7) * 2) = make_uint2(pack_bf16(x.x, x.y), pack_bf16(x.z, x.w));
         }
-        for (int e = tid; e < 6 * 16 * 16; e += LB_THREADS) {          // below the diagonal: H_ji = -A_ji X_ii
-            const int blk = e >> 8, r = (e >> 4) & 15, cc = e & 15;
+        for (int e = tid; e < 6 * 16 * 4; e += LB_THREADS) {           // below the diagonal: H_ji = -A_ji X_ii
+            const int blk = e >> 6, r = (e >> 2) & 15, c4 = (e & 3) * 4;
             // block pairs (j, i): (1,0) (2,0) (2,1) (3,0) (3,1) (3,2)
             const int bj = blk < 1 ? 1 : (blk < 3 ? 2 : 3);
             const int bi = blk - (bj == 1 ? 0 : (bj == 2 ? 1 : 3));
-            float a = 0.f;
+            float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-            for (int m = 0; m < 16; ++m) a -= As[(bj * 16 + r) * LB_A_LD + bi * 16 + m] * Xs[(bi * 16 + m) * LB_X_LD + cc];
-            const int row = bj * 16 + r, col = bi * 16 + cc;
-            reinterpret_cast<__nv_bfloat16*>(e_p + swz<128>(row, col >> 3))[col & 7] = __float2bfloat16(a);
+            for (int m = 0; m < 16; ++m) {
+                const float am = As[(bj * 16 + r) * LB_A_LD + bi * 16 + m];
+                const float4 x = *reinterpret_cast<const float4*>(&Xs[(bi * 16 + m) * LB_X_LD + c4]);
+                a.x -= am * x.x; a.y -= am * x.y; a.z -= am * x.z; a.w -= am * x.w;
+            }
+            const int row = bj * 16 + r, col = bi * 16 + c4;
+            *reinterpret_cast<uint2*>(e_p + swz<128>(row, col >> 3) + (col & 7) * 2) = make_uint2(pack_bf16(a.x, a.y), pack_bf16(a.z, a.w));
         }
         cp_async_wait<0>();
         __syncthreads();                                     // H, dv', dw in place; A is done with
@@ -800,10 +856,10 @@ linear_bwd_intra_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat1
         {
             float dar[4][4];
             zero_acc(dar);
-            warp_gemm<K * 2, A_ROW, K * 2, B_NK, 4>(dar, dt, r0, ft, c0, 0, K, lane);
+            warp_gemm<K * 2, A_ROW, K * 2, B_NK, K, 4>(dar, dt, r0, ft, c0, lane);
             cp_async_wait<0>();
             __syncthreads();
-            warp_gemm<V * 2, A_ROW, V * 2, B_NK, 4>(dar, ct, r0, et, c0, 0, V, lane);
+            warp_gemm<V * 2, A_ROW, V * 2, B_NK, V, 4>(dar, ct, r0, et, c0, lane);
             float rs_a = 0.f, rs_b = 0.f, db_a = 0.f, db_b = 0.f;
 #pragma unroll
             for (int nt = 0; nt < 4; ++nt) {
@@ -839,52 +895,54 @@ linear_bwd_intra_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat1
             store_acc_bf16<128, 4>(m_p, dar, r0, c0, lane);
         }
         __syncthreads();                                     // u and w are done with
-        load_state_parts();
+        load_dk1();
         cp_async_commit();
+        // the raw values that dbeta needs, requested ahead of the products
+        constexpr int CPR = V / 8, RPP = 32 / CPR;
+        static_assert(CPR <= 32, "value rows wider than 256 are not handled");
+        const int sub = lane / CPR, cc = lane % CPR;
+        uint4 raw[8 / RPP];
+#pragma unroll
+        for (int i = 0; i < 8 / RPP; ++i) {
+            const int r = warp * 8 + i * RPP + sub;
+            raw[i] = r < valid ? *reinterpret_cast<const uint4*>(v + ((tok0 + r) * H + h) * V + cc * 8) : make_uint4(0, 0, 0, 0);
+        }
         // ---- phase 6: dkn += dkk kn + dkk^T kn
-        warp_gemm<128, A_ROW, K * 2, B_KN, NK>(acc_k, mt, r0, kns, nk0, 0, 64, lane);
-        warp_gemm<128, A_TRANS, K * 2, B_KN, NK>(acc_k, mt, r0, kns, nk0, 0, 64, lane);
+        warp_gemm<128, A_ROW, K * 2, B_KN, 64, NK>(acc_k, mt, r0, kns, nk0, lane);
+        warp_gemm<128, A_TRANS, K * 2, B_KN, 64, NK>(acc_k, mt, r0, kns, nk0, lane);
         // ---- dv = dzu beta (in place), dbeta += <dzu, v>
-        {
-            constexpr int CPR = V / 8;
-            constexpr int RPP = 32 / CPR > 0 ? 32 / CPR : 1;
-            static_assert(CPR <= 32, "value rows wider than 256 are not handled");
-            const int sub = lane / CPR, cc = lane % CPR;
-            for (int rr = 0; rr < 8; rr += RPP) {
-                const int r = warp * 8 + rr + sub;
-                uint4* pz = reinterpret_cast<uint4*>(c_p + swz<V * 2>(r, cc));
-                uint4 z = *pz;
-                uint4 vv = make_uint4(0, 0, 0, 0);
-                if (r < valid) vv = *reinterpret_cast<const uint4*>(v + ((tok0 + r) * H + h) * V + cc * 8);
-                uint32_t* zw = reinterpret_cast<uint32_t*>(&z);
-                const uint32_t* vw = reinterpret_cast<const uint32_t*>(&vv);
-                const float bt = s_b[r];
-                float s = 0.f;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const float2 a = unpack_bf16(zw[j]), x = unpack_bf16(vw[j]);
-                    s += a.x * x.x + a.y * x.y;
-                    zw[j] = pack_bf16(a.x * bt, a.y * bt);
-                }
-                *pz = z;
+        for (int i = 0; i < 8 / RPP; ++i) {
+            const int r = warp * 8 + i * RPP + sub;
+            uint4* pz = reinterpret_cast<uint4*>(c_p + swz<V * 2>(r, cc));
+            uint4 z = *pz;
+            uint32_t* zw = reinterpret_cast<uint32_t*>(&z);
+            const uint32_t* vw = reinterpret_cast<const uint32_t*>(&raw[i]);
+            const float bt = s_b[r];
+            float s = 0.f;
 #pragma unroll
-                for (int o = CPR / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-                if (cc == 0) s_dbp[2 * 64 + r] = s;
+            for (int j = 0; j < 4; ++j) {
+                const float2 a = unpack_bf16(zw[j]), x = unpack_bf16(vw[j]);
+                s += a.x * x.x + a.y * x.y;
+                zw[j] = pack_bf16(a.x * bt, a.y * bt);
             }
+            *pz = z;
+#pragma unroll
+            for (int o = CPR / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (cc == 0) s_dbp[2 * 64 + r] = s;
         }
         cp_async_wait<0>();
         __syncthreads();
     }
-    // ---- phase 7: per-element epilogue in the accumulator layout of dqn / dkn
+    // ---- phase 7: per-element epilogue in the accumulator layout of dkn
     {
         const float ega = __expf(s_g[ia]), egb = __expf(s_g[ib]);
         const float fa = s_b[ia] * ega, fb = s_b[ib] * egb;
-        float zk_a = 0.f, zk_b = 0.f, dE_a = 0.f, dE_b = 0.f;
+        float zk_a = 0.f, zk_b = 0.f, dk_a = 0.f, dk_b = 0.f;
 #pragma unroll
         for (int nt = 0; nt < NK; ++nt) {
             const int col = nk0 + nt * 8 + qd * 2;
             const float2 kna = load_pair_bf16<K * 2>(kns_p, ia, col), knb = load_pair_bf16<K * 2>(kns_p, ib, col);
-            const float2 qna = load_pair_bf16<K * 2>(qns_p, ia, col), qnb = load_pair_bf16<K * 2>(qns_p, ib, col);
             if (GDN) {
                 const float2 za = load_pair_bf16<K * 2>(d_p, ia, col), zb = load_pair_bf16<K * 2>(d_p, ib, col);
                 zk_a += za.x * kna.x + za.y * kna.y;
@@ -892,62 +950,35 @@ linear_bwd_intra_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat1
                 acc_k[nt][0] += za.x * fa; acc_k[nt][1] += za.y * fa;
                 acc_k[nt][2] += zb.x * fb; acc_k[nt][3] += zb.y * fb;
             }
-            const float2 xa = load_pair_bf16<K * 2>(e_p, ia, col), xb = load_pair_bf16<K * 2>(e_p, ib, col);
-            acc_q[nt][0] += xa.x; acc_q[nt][1] += xa.y; acc_q[nt][2] += xb.x; acc_q[nt][3] += xb.y;
-            dE_a += xa.x * qna.x + xa.y * qna.y;
-            dE_b += xb.x * qnb.x + xb.y * qnb.y;
             if (act) {
                 const float2 ya = load_pair_bf16<K * 2>(f_p, ia, col), yb = load_pair_bf16<K * 2>(f_p, ib, col);
                 acc_k[nt][0] += ya.x; acc_k[nt][1] += ya.y; acc_k[nt][2] += yb.x; acc_k[nt][3] += yb.y;
             }
-        }
-        // dot products of the l2-norm backward, over the finished dqn / dkn
-        float dq_a = 0.f, dq_b = 0.f, dk_a = 0.f, dk_b = 0.f;
-#pragma unroll
-        for (int nt = 0; nt < NK; ++nt) {
-            const int col = nk0 + nt * 8 + qd * 2;
-            const float2 kna = load_pair_bf16<K * 2>(kns_p, ia, col), knb = load_pair_bf16<K * 2>(kns_p, ib, col);
-            const float2 qna = load_pair_bf16<K * 2>(qns_p, ia, col), qnb = load_pair_bf16<K * 2>(qns_p, ib, col);
-            dq_a += acc_q[nt][0] * qna.x + acc_q[nt][1] * qna.y;
-            dq_b += acc_q[nt][2] * qnb.x + acc_q[nt][3] * qnb.y;
+            // dot product of the l2-norm backward, over the finished dkn
             dk_a += acc_k[nt][0] * kna.x + acc_k[nt][1] * kna.y;
             dk_b += acc_k[nt][2] * knb.x + acc_k[nt][3] * knb.y;
         }
         zk_a = quad_sum(zk_a); zk_b = quad_sum(zk_b);
-        dE_a = quad_sum(dE_a); dE_b = quad_sum(dE_b);
-        dq_a = quad_sum(dq_a); dq_b = quad_sum(dq_b);
         dk_a = quad_sum(dk_a); dk_b = quad_sum(dk_b);
         if (qd == 0) {
             atomicAdd(&s_zk[ia], zk_a); atomicAdd(&s_zk[ib], zk_b);
-            atomicAdd(&s_dE[ia], dE_a); atomicAdd(&s_dE[ib], dE_b);
-            atomicAdd(&s_dotq[ia], dq_a); atomicAdd(&s_dotq[ib], dq_b);
             atomicAdd(&s_dotk[ia], dk_a); atomicAdd(&s_dotk[ib], dk_b);
         }
     }
-    __syncthreads();                                         // row sums complete; dq1 and dk1 have been read
-    // ---- phase 8: l2-norm backward, staging, stores
+    __syncthreads();                                         // row sums complete, dv in place
+    // ---- phase 8: l2-norm backward, stores
     {
-        float qra = 1.f, qrb = 1.f, kra = 1.f, krb = 1.f;
-        if (use_l2norm) {
-            qra = ia < valid ? q_rstd[(tok0 + ia) * H + h] : 0.f;
-            qrb = ib < valid ? q_rstd[(tok0 + ib) * H + h] : 0.f;
-            kra = ia < valid ? k_rstd[(tok0 + ia) * H + h] : 0.f;
-            krb = ib < valid ? k_rstd[(tok0 + ib) * H + h] : 0.f;
-        }
-        const float pq_a = use_l2norm ? s_dotq[ia] : 0.f, pq_b = use_l2norm ? s_dotq[ib] : 0.f;
+        const float kra = s_kr[ia], krb = s_kr[ib];
         const float pk_a = use_l2norm ? s_dotk[ia] : 0.f, pk_b = use_l2norm ? s_dotk[ib] : 0.f;
 #pragma unroll
         for (int nt = 0; nt < NK; ++nt) {
             const int col = nk0 + nt * 8 + qd * 2;
             const float2 kna = load_pair_bf16<K * 2>(kns_p, ia, col), knb = load_pair_bf16<K * 2>(kns_p, ib, col);
-            const float2 qna = load_pair_bf16<K * 2>(qns_p, ia, col), qnb = load_pair_bf16<K * 2>(qns_p, ib, col);
-            acc_q[nt][0] = qra * (acc_q[nt][0] - qna.x * pq_a); acc_q[nt][1] = qra * (acc_q[nt][1] - qna.y * pq_a);
-            acc_q[nt][2] = qrb * (acc_q[nt][2] - qnb.x * pq_b); acc_q[nt][3] = qrb * (acc_q[nt][3] - qnb.y * pq_b);
             acc_k[nt][0] = kra * (acc_k[nt][0] - kna.x * pk_a); acc_k[nt][1] = kra * (acc_k[nt][1] - kna.y * pk_a);
             acc_k[nt][2] = krb * (acc_k[nt][2] - knb.x * pk_b); acc_k[nt][3] = krb * (acc_k[nt][3] - knb.y * pk_b);
         }
-        store_acc_bf16<K * 2, NK>(e_p, acc_q, r0, nk0, lane);
-        store_acc_bf16<K * 2, NK>(f_p, acc_k, r0, nk0, lane);
+        store_acc_global<NK>(dk + (tok0 * H + h) * K, (long)H * K, acc_k, r0, nk0, valid, lane);
+        if (GDN) store_tile<64, V, LB_THREADS>(c_p, dv + (tok0 * H + h) * V, (long)H * V, valid, tid);
     }
     if (tid < 64) {
         const float eg = __expf(s_g[tid]);
@@ -955,7 +986,7 @@ linear_bwd_intra_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat1
         if (tid < valid) {
             const long gi = (tok0 + tid) * H + h;
             float dgt = (s_dgr[tid] + s_dgr[64 + tid]) +
-                        ((s_dgc[tid] + s_dgc[64 + tid]) + (s_dgc[128 + tid] + s_dgc[192 + tid])) + dE - dkd[gi];
+                        ((s_dgc[tid] + s_dgc[64 + tid]) + (s_dgc[128 + tid] + s_dgc[192 + tid])) + dE - s_dkd[tid];
             if (GDN) {
                 dgt += (s_dgr[128 + tid] + s_dgr[192 + tid]) +
                        ((s_dgc[256 + tid] + s_dgc[320 + tid]) + (s_dgc[384 + tid] + s_dgc[448 + tid]));
@@ -969,9 +1000,6 @@ linear_bwd_intra_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat1
         if (lane == 0) atomicAdd(&s_red[0], se);
     }
     __syncthreads();
-    store_tile<64, K, LB_THREADS>(e_p, dq + (tok0 * H + h) * K, (long)H * K, valid, tid);
-    store_tile<64, K, LB_THREADS>(f_p, dk + (tok0 * H + h) * K, (long)H * K, valid, tid);
-    if (GDN) store_tile<64, V, LB_THREADS>(c_p, dv + (tok0 * H + h) * V, (long)H * V, valid, tid);
     if (tid == 0) scal[(((long)b * NT + c) * H + h) * 4 + 3] = s_red[0];
 }
 

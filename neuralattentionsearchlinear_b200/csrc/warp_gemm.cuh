@@ -22,54 +22,49 @@ __device__ __forceinline__ void zero_acc(float (&acc)[NT8][4]) {
         for (int e = 0; e < 4; ++e) acc[i][e] = 0.f;
 }
 
-// acc += A[m0.., k_begin..k_end) * B[k_begin..k_end), n0..)   (k range a multiple of 16)
-template <int A_RB, int A_MODE, int B_RB, int B_MODE, int NT8>
-__device__ __forceinline__ void warp_gemm(float (&acc)[NT8][4], uint32_t atile, int m0, uint32_t btile, int n0, int k_begin,
-                                          int k_end, int lane) {
-    static_assert(NT8 % 2 == 0, "n-tiles come in pairs");
-#pragma unroll 2
-    for (int k0 = k_begin; k0 < k_end; k0 += 16) {
+// Addresses of a lane's ldmatrix rows.  Tiles start on a multiple of their row length (256 bytes at most), m0 is a multiple of 16
+// and n0 of 8 * NT8, so a step along a row is an exclusive or with a constant and a step over rows an addition that goes into the
+// instruction: one integer operation per fragment at most.  (Against addresses formed anew for every fragment, with the tile copies
+// treated the same way; B = 8, T = 4096, 16 heads of 128 / 128: reverse walk 291 -> 260 us, state part 539 -> 507, 64 x 64 part
+// 736 -> 709.)
+template <int RB, int MODE>
+__device__ __forceinline__ uint32_t a_addr(uint32_t tile, int m0, int lane) {
+    if (MODE == A_ROW) return tile + swz<RB>(m0 + (lane & 15), lane >> 4);
+    const int i = lane >> 3;
+    return tile + swz<RB>((lane & 7) + ((i >> 1) << 3), (m0 >> 3) + (i & 1));
+}
+template <int RB, int MODE>
+__device__ __forceinline__ void ld_a(uint32_t at, int k0, uint32_t (&a)[4]) {           // k0: a constant after unrolling
+    if (MODE == A_ROW) ldsm_x4(at ^ (k0 * 2), a[0], a[1], a[2], a[3]);
+    else ldsm_x4_t(at + k0 * RB, a[0], a[1], a[2], a[3]);
+}
+template <int RB, int MODE>
+__device__ __forceinline__ uint32_t b_addr(uint32_t tile, int n0, int lane) {
+    if (MODE == B_NK) return tile + swz<RB>(n0 + (lane & 7) + ((lane >> 4) << 3), (lane >> 3) & 1);
+    return tile + swz<RB>((lane & 7) + (((lane >> 3) & 1) << 3), (n0 >> 3) + (lane >> 4));
+}
+template <int RB, int MODE>
+__device__ __forceinline__ void ld_b(uint32_t at, int p, int k0, uint32_t (&b)[4]) {    // n-tiles 2 p and 2 p + 1
+    if (MODE == B_NK) ldsm_x4((at ^ (k0 * 2)) + p * 16 * RB, b[0], b[1], b[2], b[3]);
+    else ldsm_x4_t((at ^ (p * 32)) + k0 * RB, b[0], b[1], b[2], b[3]);
+}
+
+// acc += A[m0.., 0..KLEN) * B[0..KLEN), n0..)
+template <int A_RB, int A_MODE, int B_RB, int B_MODE, int KLEN, int NT8>
+__device__ __forceinline__ void warp_gemm(float (&acc)[NT8][4], uint32_t atile, int m0, uint32_t btile, int n0, int lane) {
+    static_assert(NT8 % 2 == 0 && (NT8 & (NT8 - 1)) == 0 && KLEN % 16 == 0, "n-tiles come in pairs");
+    const uint32_t at = a_addr<A_RB, A_MODE>(atile, m0, lane), bt = b_addr<B_RB, B_MODE>(btile, n0, lane);
+#pragma unroll
+    for (int k0 = 0; k0 < KLEN; k0 += 16) {
         uint32_t a[4];
-        if (A_MODE == A_ROW) load_a<A_RB>(atile, m0, k0, lane, a);
-        else load_a_t<A_RB>(atile, m0, k0, lane, a);
+        ld_a<A_RB, A_MODE>(at, k0, a);
 #pragma unroll
         for (int p = 0; p < NT8 / 2; ++p) {
             uint32_t b[4];
-            if (B_MODE == B_NK) load_b_nk<B_RB>(btile, n0 + 16 * p, k0, lane, b);
-            else load_b_kn<B_RB>(btile, k0, n0 + 16 * p, lane, b);
+            ld_b<B_RB, B_MODE>(bt, p, k0, b);
             mma_bf16(acc[2 * p], a, b[0], b[1]);
             mma_bf16(acc[2 * p + 1], a, b[2], b[3]);
         }
-    }
-}
-
-// Same with A taken from registers: afrag[j] is the A fragment of contraction step j (16 values of k each),
-// typically made from an accumulator strip with acc_to_afrag().  B rows start at kb0.
-template <int KSTEPS, int B_RB, int B_MODE, int NT8>
-__device__ __forceinline__ void warp_gemm_ra(float (&acc)[NT8][4], const uint32_t (&afrag)[KSTEPS][4], uint32_t btile, int n0,
-                                             int kb0, int lane) {
-#pragma unroll
-    for (int j = 0; j < KSTEPS; ++j) {
-#pragma unroll
-        for (int p = 0; p < NT8 / 2; ++p) {
-            uint32_t b[4];
-            if (B_MODE == B_NK) load_b_nk<B_RB>(btile, n0 + 16 * p, kb0 + 16 * j, lane, b);
-            else load_b_kn<B_RB>(btile, kb0 + 16 * j, n0 + 16 * p, lane, b);
-            mma_bf16(acc[2 * p], afrag[j], b[0], b[1]);
-            mma_bf16(acc[2 * p + 1], afrag[j], b[2], b[3]);
-        }
-    }
-}
-
-// A 16 x (8*NT8) accumulator strip, rounded to bf16, is the A operand of a product that contracts over its columns.
-template <int NT8>
-__device__ __forceinline__ void acc_to_afrag(const float (&acc)[NT8][4], uint32_t (&afrag)[NT8 / 2][4]) {
-#pragma unroll
-    for (int j = 0; j < NT8 / 2; ++j) {
-        afrag[j][0] = pack_bf16(acc[2 * j][0], acc[2 * j][1]);
-        afrag[j][1] = pack_bf16(acc[2 * j][2], acc[2 * j][3]);
-        afrag[j][2] = pack_bf16(acc[2 * j + 1][0], acc[2 * j + 1][1]);
-        afrag[j][3] = pack_bf16(acc[2 * j + 1][2], acc[2 * j + 1][3]);
     }
 }
 
@@ -82,6 +77,27 @@ __device__ __forceinline__ void store_acc_bf16(unsigned char* tile, const float 
         const int ch = (n0 >> 3) + nt;
         *reinterpret_cast<uint32_t*>(tile + swz<RB>(m0 + gq, ch) + qd * 4) = pack_bf16(acc[nt][0], acc[nt][1]);
         *reinterpret_cast<uint32_t*>(tile + swz<RB>(m0 + gq + 8, ch) + qd * 4) = pack_bf16(acc[nt][2], acc[nt][3]);
+    }
+}
+
+// Write a strip straight to global memory (row r at g + r * gstride, columns n0..), rows from `valid` on left out: neighbouring lanes
+// swap halves of neighbouring n-tiles, so that a store covers whole 32-byte sectors and no staging tile or barrier is needed.
+template <int NT8>
+__device__ __forceinline__ void store_acc_global(__nv_bfloat16* g, long gstride, const float (&acc)[NT8][4], int m0, int n0, int valid, int lane) {
+    const int gq = lane >> 2, qd = lane & 3;
+    const bool odd = qd & 1;
+    __nv_bfloat16* pa = g + (long)(m0 + gq) * gstride + n0 + (odd ? 8 : 0) + (qd >> 1) * 4;
+    __nv_bfloat16* pb = pa + 8 * gstride;
+    const bool oka = m0 + gq < valid, okb = m0 + gq + 8 < valid;
+#pragma unroll
+    for (int p = 0; p < NT8 / 2; ++p) {
+#pragma unroll
+        for (int e = 0; e < 4; e += 2) {
+            const uint32_t x = pack_bf16(acc[2 * p][e], acc[2 * p][e + 1]), y = pack_bf16(acc[2 * p + 1][e], acc[2 * p + 1][e + 1]);
+            const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? x : y, 1);
+            const uint2 v = odd ? make_uint2(got, y) : make_uint2(x, got);
+            if (e ? okb : oka) *reinterpret_cast<uint2*>((e ? pb : pa) + 16 * p) = v;
+        }
     }
 }
 
