@@ -467,6 +467,35 @@ int natsl_rmsnorm_fwd(const void* x, const void* res, const void* w, int w_dtype
 int natsl_rmsnorm_bwd(const void* s, const void* w, int w_dtype, const void* dy, const void* dadd, void* dx, float* dw_part,
                       int n_part, long rows, int D, float eps, void* stream);
 
+/* l2 norm over rows of D = 64, 128 or 256 bf16 elements, y = x * rsqrt(sum(x^2) + eps), and its backward
+ * (src/nats/layers/natsl_attn_mamba2.py:193-194). */
+int natsl_l2norm_fwd(const void* x, void* y, int64_t rows, int D, float eps, void* stream);
+int natsl_l2norm_bwd(const void* x, const void* dy, void* dx, int64_t rows, int D, float eps, void* stream);
+
+/* Gates of a layer's training path: dt = softplus(a + dt_bias), g [rows,H] fp32 = -exp(A_log) dt, beta = sigmoid(b) (times two with
+ * neg_eigval; b and beta may be NULL), v_out = v dt (v, v_out [rows,H,V] or NULL); a, b, beta [rows,H], v bf16, A_log and dt_bias [H]
+ * bf16 or fp32, H <= 256.  Backward: from dg, dbeta, dv_out (each may be NULL) da, db, dv and n_part partial sums part [n_part,2,H]
+ * of the gradients of A_log and dt_bias (V = 32, 64, 128 or 256).
+ * Replaces src/nats/layers/natsl_attn_gdn.py:461-480, src/nats/layers/natsl_attn_mamba2.py:402-440. */
+int natsl_gates_fwd(const void* a, const void* b, const void* v, const void* A_log, int alog_dtype, const void* dt_bias, int dtb_dtype,
+                    int neg_eigval, float* g, void* beta, void* v_out, int64_t rows, int H, int V, void* stream);
+int natsl_gates_bwd(const void* a, const void* b, const void* v, const void* A_log, int alog_dtype, const void* dt_bias, int dtb_dtype,
+                    int neg_eigval, const float* dg, const void* dbeta, int dbeta_dtype, const void* dv_out, void* da, void* db, void* dv,
+                    float* part, int n_part, int64_t rows, int H, int V, void* stream);
+
+/* Gradient of natsl_block_mean: dx [B,T,D] = dy [B,cdiv(T,nbs),D] of the token's block / tokens of the block. */
+int natsl_block_mean_bwd(const void* dy, void* dx, int B, int T, int D, int nbs, void* stream);
+
+/* Sums of partial weight gradients: over p of part [P,N] fp32, rounded to out*_dtype.  mode 0: out0 [N]; 1: the two halves of N to out0 and
+ * out1; w > 1: N = groups of w + 1, the first w of a group to out0 [N / (w + 1), w], the last to out1 (or dropped where it is NULL). */
+int natsl_column_sums(const float* part, int P, int N, int mode, void* out0, int out0_dtype, void* out1, int out1_dtype, void* stream);
+
+/* Gradient of the block types [B,TN,HN,2] (bf16 or fp32) at block size 64 from the two branches' sums per tile: attn_tiles [B,TN,HQ]
+ * (counted where types_i selects the block), linear_tiles [B,TN,H] (src/nats/ops/attns/attns.py:975-978,
+ * src/nats/ops/common/chunk_o.py:459-492). */
+int natsl_types_grad(const float* attn_tiles, const float* linear_tiles, const int32_t* types_i, void* out, int out_dtype, int B, int TN,
+                     int HN, int HQ, int H, void* stream);
+
 /* SwiGLU: y = silu(a) * b over n elements (a multiple of 8); backward da, db.
  * Replaces: the activation of fla GatedMLP, src/nats/models/natsl_attn_gdn/modeling_natsl_attn_gdn.py:111-117. */
 int natsl_swiglu_fwd(const void* a, const void* b, void* y, long n, void* stream);

@@ -74,6 +74,13 @@ PROTOTYPES = {
     "natsl_short_conv_bwd": [_p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _p],
     "natsl_rmsnorm_fwd": [_p, _p, _p, _i, _p, _p, C.c_long, _i, _f, _p],
     "natsl_rmsnorm_bwd": [_p, _p, _i, _p, _p, _p, _p, _i, C.c_long, _i, _f, _p],
+    "natsl_l2norm_fwd": [_p, _p, C.c_int64, _i, _f, _p],
+    "natsl_l2norm_bwd": [_p, _p, _p, C.c_int64, _i, _f, _p],
+    "natsl_gates_fwd": [_p, _p, _p, _p, _i, _p, _i, _i, _p, _p, _p, C.c_int64, _i, _i, _p],
+    "natsl_gates_bwd": [_p, _p, _p, _p, _i, _p, _i, _i, _p, _p, _i, _p, _p, _p, _p, _p, _i, C.c_int64, _i, _i, _p],
+    "natsl_block_mean_bwd": [_p, _p, _i, _i, _i, _i, _p],
+    "natsl_column_sums": [_p, _i, _i, _i, _p, _i, _p, _i, _p],
+    "natsl_types_grad": [_p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _p],
     "natsl_swiglu_fwd": [_p, _p, _p, C.c_long, _p],
     "natsl_swiglu_bwd": [_p, _p, _p, _p, _p, C.c_long, _p],
     "natsl_copy_batches": [_p, _p, _i, C.c_int64, C.c_int64, C.c_int64, _p],

@@ -473,11 +473,12 @@ def _call(timer, stage, name, *args):
 
 
 def attn_bwd(q, k, v, o, lse, do, tables: SelectionTables, scale: float, own_chunk: bool, reference_compat: bool = False,
-             timer: StageTimer | None = None):
+             timer: StageTimer | None = None, per_tile: bool = False):
     """Backward of the softmax branch.  -> (dq, dk, dv bf16, dnats_attn [B,TN,HN] fp32): ``dnats_attn`` is the sum of the
     score gradients of the keys of a softmax-selected block over the queries of later blocks, summed over the heads
     of a selection group and zero for the other blocks (src/nats/ops/attns/attns.py:922, 975-978, 1625-1629, 1749-1755).
-    ``reference_compat``: leave out every own-block term like the reference's default backward."""
+    ``reference_compat``: leave out every own-block term like the reference's default backward.  ``per_tile``: the sums of the
+    key tiles [B,NT,HQ], whatever their blocks' types, in the place of ``dnats_attn``."""
     for t_ in (q, k, v, o, do):
         _need(t_.dtype == BF16, "softmax-branch backward needs bf16 tensors", TypeError)
     _check_qkv(q, k, v, tables, "softmax branch (backward)", same_heads=False)
@@ -497,6 +498,8 @@ def attn_bwd(q, k, v, o, lse, do, tables: SelectionTables, scale: float, own_chu
     _call(timer, "attn_bwd", "natsl_attn_bwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(), lse.data_ptr(),
               tables.types_i.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), delta.data_ptr(), part.data_ptr(),
               B, T, HQ, HKV, HN, DK, DV, nbs, float(scale), flags, current_stream_ptr(dev))
+    if per_tile:
+        return dq, dk, dv, part
     cpb = nbs // 64
     if NT != TN * cpb:                                        # ragged last block: pad the tile axis
         part = torch.nn.functional.pad(part, (0, 0, 0, TN * cpb - NT))
@@ -507,10 +510,11 @@ def attn_bwd(q, k, v, o, lse, do, tables: SelectionTables, scale: float, own_chu
 
 def linear_bwd(rule: int, q, k, v, g, beta, tables: SelectionTables, scale: float, h0, decay: bool, use_l2norm: bool,
                do, dht=None, invalid_dnats: bool = True, trailing_quirk: bool = True, return_intermediates: bool = False,
-               timer: StageTimer | None = None):
+               timer: StageTimer | None = None, per_tile: bool = False):
     """Backward of the linear branch (block size 64).  Recomputes the forward's preparation and recurrence, then runs the
     five backward stages.  -> dict(dq, dk, dv bf16; dg fp32; dbeta fp32 or None; dh0 fp32 or None; dnats [B,NT,HN] fp32
-    = the reference's dnats column for the linear branch, src/nats/ops/common/chunk_o.py:440-443, 459-492, 1568-1575)."""
+    = the reference's dnats column for the linear branch, src/nats/ops/common/chunk_o.py:440-443, 459-492, 1568-1575; with
+    ``per_tile`` [B,NT,H], per head)."""
     gdn = rule == _lib.RULE_GDN
     for t_ in (q, k, v, do):
         _need(t_.dtype == BF16, "linear-branch backward needs bf16 tensors", TypeError)
@@ -596,7 +600,7 @@ def linear_bwd(rule: int, q, k, v, g, beta, tables: SelectionTables, scale: floa
     dg = torch.empty(B, T, H, **f32)
     _call(timer, "bwd_dg", "natsl_linear_bwd_dg", dg_tok.data_ptr(), scal.data_ptr(), tables.types_i.data_ptr(), tables.indices.data_ptr(),
               tables.n_blocks.data_ptr(), dg.data_ptr(), B, T, H, HN, flags, st)
-    dnats = dn_lin.view(B, NT, HN, H // HN).sum(-1)
+    dnats = dn_lin if per_tile else dn_lin.view(B, NT, HN, H // HN).sum(-1)
     out = dict(dq=dq, dk=dk, dv=dv, dg=dg, dbeta=dbeta, dh0=dh0, dnats=dnats)
     if return_intermediates:
         out.update(dS=dS_all, dvp=dvp, dw=dw, vp=vp, h=h, carry=carry, gcs=gcs, w=w, u=u)

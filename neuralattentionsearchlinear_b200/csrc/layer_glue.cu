@@ -281,7 +281,7 @@ template <int D>
 __global__ void __launch_bounds__(256)
 rmsnorm_fwd_narrow_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
                           const void* __restrict__ w, int w_f32, __nv_bfloat16* __restrict__ y,
-                          __nv_bfloat16* __restrict__ sum_out, long rows, float eps) {
+                          __nv_bfloat16* __restrict__ sum_out, long rows, float inv_n, float eps) {
     constexpr int LPR = D / 8, RPW = 32 / LPR;
     const int lane = threadIdx.x & 31, sub = lane % LPR;
     const long row_raw = ((long)blockIdx.x * 8 + (threadIdx.x >> 5)) * RPW + lane / LPR;
@@ -306,7 +306,7 @@ rmsnorm_fwd_narrow_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat
     for (int e = 0; e < 8; ++e) ss += a[e] * a[e];
 #pragma unroll
     for (int o = LPR / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    const float rstd = rsqrtf(ss / D + eps);
+    const float rstd = rsqrtf(ss * inv_n + eps);              // 1 / D, or 1 for the l2 norm
 #pragma unroll
     for (int e = 0; e < 8; ++e) a[e] = a[e] * rstd * ww[e];
     if (ok) st8(y + row * D + sub * 8, a);
@@ -323,9 +323,9 @@ struct RmsBwd {
     const __nv_bfloat16 *s, *dy, *dadd;
     const void* w;
     __nv_bfloat16* dx;
-    float* dw_part;
+    float* dw_part;                                            // NULL: no weight
     long rows;
-    float eps;
+    float inv_n, eps;                                          // 1 / D, or 1 for the l2 norm
     int w_f32, wide;                                           // wide: every tensor starts on 16 bytes
 };
 __device__ __forceinline__ void rms_sums(const uint64_t (&a)[4], const uint64_t (&g)[4], const uint64_t (&ww)[4], float& ss, float& c) {
@@ -339,10 +339,9 @@ __device__ __forceinline__ void rms_sums(const uint64_t (&a)[4], const uint64_t 
     c = hsum2(c2);
 }
 // g becomes the gradient of the row in front of the added one; ss, c are the sums over the row.
-template <int D>
 __device__ __forceinline__ void rms_grad(const uint64_t (&a)[4], uint64_t (&g)[4], const uint64_t (&ww)[4], uint64_t (&dwa)[4], float ss, float c,
-                                         float eps, bool ok) {
-    const float rstd = rsqrtf(ss / D + eps), m = -(c * rstd / D);     // m = -mean(dy w xhat)
+                                         float inv_n, float eps, bool ok) {
+    const float rstd = rsqrtf(ss * inv_n + eps), m = -(c * rstd * inv_n);     // m = -mean(dy w xhat)
     const uint64_t r2 = pack2(rstd, rstd), m2 = pack2(m, m);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -395,9 +394,10 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_narrow_kernel(const RmsBwd p)
             c += __shfl_xor_sync(0xffffffffu, c, o);
         }
         const bool ok = row0 + lane / LPR < p.rows;
-        rms_grad<D>(a, g, ww, dwa, ss, c, p.eps, ok);
+        rms_grad(a, g, ww, dwa, ss, c, p.inv_n, p.eps, ok);
         if (ok) rms_store(p, (row0 + lane / LPR) * D + sub * 8, g, add);
     }
+    if (!p.dw_part) return;
     float o8[8];
 #pragma unroll
     for (int i = 0; i < 4; ++i) unpack2(dwa[i], o8[2 * i], o8[2 * i + 1]);
@@ -456,9 +456,10 @@ __global__ void __launch_bounds__(256, 4) rmsnorm_bwd_wide_kernel(const RmsBwd p
             c += v.y;
         }
         const bool ok = row0 + rb < p.rows;
-        rms_grad<D>(a, g, ww, dwa, ss, c, p.eps, ok);
+        rms_grad(a, g, ww, dwa, ss, c, p.inv_n, p.eps, ok);
         if (ok) rms_store(p, (row0 + rb) * D + f0, g, add);
     }
+    if (!p.dw_part) return;
     float o8[8];
 #pragma unroll
     for (int i = 0; i < 4; ++i) unpack2(dwa[i], o8[2 * i], o8[2 * i + 1]);
@@ -792,7 +793,7 @@ extern "C" int natsl_rmsnorm_fwd(const void* x, const void* res, const void* w, 
     if (D == 64 || D == 128 || D == 256) {
         const int rpc = 8 * (32 / (D / 8));                  // rows per CTA
         const unsigned gridn = (unsigned)((rows + rpc - 1) / rpc);
-#define NATSL_NARROW(DD) rmsnorm_fwd_narrow_kernel<DD><<<gridn, 256, 0, st>>>(bfc(x), bfc(res), w, w_dtype == NATSL_DT_F32, bfm(y), bfm(sum_out), rows, eps)
+#define NATSL_NARROW(DD) rmsnorm_fwd_narrow_kernel<DD><<<gridn, 256, 0, st>>>(bfc(x), bfc(res), w, w_dtype == NATSL_DT_F32, bfm(y), bfm(sum_out), rows, 1.f / DD, eps)
         if (D == 64) NATSL_NARROW(64);
         else if (D == 128) NATSL_NARROW(128);
         else NATSL_NARROW(256);
@@ -812,7 +813,8 @@ extern "C" int natsl_rmsnorm_bwd(const void* s, const void* w, int w_dtype, cons
     NATSL_REQUIRE(rows > 0 && n_part > 0, NATSL_ERR_BAD_SHAPE, "natsl_rmsnorm_bwd: empty input");
     NATSL_REQUIRE(w_dtype == NATSL_DT_BF16 || w_dtype == NATSL_DT_F32, NATSL_ERR_UNSUPPORTED, "natsl_rmsnorm_bwd: weight must be bf16 or f32");
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    const RmsBwd p = {bfc(s), bfc(dy), bfc(dadd), w, bfm(dx), dw_part, rows, eps, w_dtype == NATSL_DT_F32, aligned_to(16, s, dy, dadd, dx)};
+    const RmsBwd p = {bfc(s), bfc(dy), bfc(dadd), w, bfm(dx), dw_part, rows, D > 0 ? 1.f / D : 0.f, eps, w_dtype == NATSL_DT_F32,
+                      aligned_to(16, s, dy, dadd, dx)};
     switch (D) {
         case 64: rmsnorm_bwd_narrow_kernel<64><<<n_part, 256, 0, st>>>(p); break;
         case 128: rmsnorm_bwd_narrow_kernel<128><<<n_part, 256, 0, st>>>(p); break;
@@ -825,6 +827,34 @@ extern "C" int natsl_rmsnorm_bwd(const void* s, const void* w, int w_dtype, cons
             return NATSL_ERR_UNSUPPORTED;
     }
     return check_launch("natsl_rmsnorm_bwd");
+}
+
+// y = x * rsqrt(sum(x^2) + eps) and its backward: the narrow rows' kernels with the sum of squares in the place of its mean.
+extern "C" int natsl_l2norm_fwd(const void* x, void* y, int64_t rows, int D, float eps, void* stream) {
+    NATSL_REQUIRE(x && y, NATSL_ERR_NULL, "natsl_l2norm_fwd: null pointer");
+    NATSL_REQUIRE(rows > 0, NATSL_ERR_BAD_SHAPE, "natsl_l2norm_fwd: empty input");
+    NATSL_REQUIRE(D == 64 || D == 128 || D == 256, NATSL_ERR_UNSUPPORTED, "natsl_l2norm_fwd: row width D=%d (64, 128 or 256)", D);
+    NATSL_REQUIRE(aligned_to(16, x, y), NATSL_ERR_UNSUPPORTED, "natsl_l2norm_fwd: x and y must start on 16 bytes");
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    const unsigned grid = (unsigned)((rows + 8 * (256 / D) - 1) / (8 * (256 / D)));
+    if (D == 64) rmsnorm_fwd_narrow_kernel<64><<<grid, 256, 0, st>>>(bfc(x), nullptr, nullptr, 0, bfm(y), nullptr, rows, 1.f, eps);
+    else if (D == 128) rmsnorm_fwd_narrow_kernel<128><<<grid, 256, 0, st>>>(bfc(x), nullptr, nullptr, 0, bfm(y), nullptr, rows, 1.f, eps);
+    else rmsnorm_fwd_narrow_kernel<256><<<grid, 256, 0, st>>>(bfc(x), nullptr, nullptr, 0, bfm(y), nullptr, rows, 1.f, eps);
+    return check_launch("natsl_l2norm_fwd");
+}
+
+extern "C" int natsl_l2norm_bwd(const void* x, const void* dy, void* dx, int64_t rows, int D, float eps, void* stream) {
+    NATSL_REQUIRE(x && dy && dx, NATSL_ERR_NULL, "natsl_l2norm_bwd: null pointer");
+    NATSL_REQUIRE(rows > 0, NATSL_ERR_BAD_SHAPE, "natsl_l2norm_bwd: empty input");
+    NATSL_REQUIRE(D == 64 || D == 128 || D == 256, NATSL_ERR_UNSUPPORTED, "natsl_l2norm_bwd: row width D=%d (64, 128 or 256)", D);
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    const RmsBwd p = {bfc(x), bfc(dy), nullptr, nullptr, bfm(dx), nullptr, rows, 1.f, eps, 0, aligned_to(16, x, dy, dx)};
+    const long turns = (rows + 8 * (256 / D) - 1) / (8 * (256 / D));
+    const unsigned grid = (unsigned)(turns < 592 ? turns : 592);
+    if (D == 64) rmsnorm_bwd_narrow_kernel<64><<<grid, 256, 0, st>>>(p);
+    else if (D == 128) rmsnorm_bwd_narrow_kernel<128><<<grid, 256, 0, st>>>(p);
+    else rmsnorm_bwd_narrow_kernel<256><<<grid, 256, 0, st>>>(p);
+    return check_launch("natsl_l2norm_bwd");
 }
 
 extern "C" int natsl_swiglu_fwd(const void* a, const void* b, void* y, long n, void* stream) {

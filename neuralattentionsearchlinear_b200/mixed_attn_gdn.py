@@ -12,7 +12,7 @@ import os
 import torch
 
 from . import _lib, _ops
-from .nats_util import CHUNK_SIZE, OFFSET_ATTN, OFFSET_LINEAR, build_selection_tables, transforms_active  # noqa: F401
+from .nats_util import CHUNK_SIZE, OFFSET_ATTN, OFFSET_LINEAR, build_selection_tables, current_stream_ptr, transforms_active  # noqa: F401
 
 # which branches also compute the query's own (possibly incomplete) block — mixed_attn_gdn.py:29-42
 all_incomplete_ops = {
@@ -110,11 +110,19 @@ def hybrid_backward(ctx, rule, do_lin, do_attn, dht):
         do_attn = torch.zeros_like(o_attn)
     if do_lin is None:
         do_lin = torch.zeros(q.shape[:3] + (v.shape[3],), dtype=q.dtype, device=q.device)
+    one = ctx.types_dtype in (torch.bfloat16, torch.float32)          # the gradient of the types in one kernel
     dqa, dka, dva, dn_attn = _ops.attn_bwd(q_attn, k_attn, v_attn, o_attn, lse, do_attn.to(o_attn.dtype), tables,
-                                           ctx.scale_attn, ctx.own_attn, reference_compat=ctx.compat)
+                                           ctx.scale_attn, ctx.own_attn, reference_compat=ctx.compat, per_tile=one)
     r = _ops.linear_bwd(rule, q, k, v, g, beta, tables, ctx.scale_lattn, h0, ctx.decay, ctx.use_l2norm,
-                        do_lin.to(q.dtype), dht=dht, invalid_dnats=ctx.invalid_dnats_linear)
-    dnats = torch.stack([dn_attn, r['dnats']], -1).to(ctx.types_dtype)
+                        do_lin.to(q.dtype), dht=dht, invalid_dnats=ctx.invalid_dnats_linear, per_tile=one)
+    if one:
+        B, TN, HN, _ = tables.types_i.shape
+        dnats = torch.empty(B, TN, HN, 2, dtype=ctx.types_dtype, device=q.device)
+        _lib.call("natsl_types_grad", dn_attn.data_ptr(), r['dnats'].data_ptr(), tables.types_i.data_ptr(), dnats.data_ptr(),
+                  _lib.DT_BF16 if ctx.types_dtype == torch.bfloat16 else _lib.DT_F32, B, TN, HN, q_attn.shape[2], q.shape[2],
+                  current_stream_ptr(q.device))
+    else:
+        dnats = torch.stack([dn_attn, r['dnats']], -1).to(ctx.types_dtype)
     dg = r['dg'].to(g.dtype)
     dbeta = None if r['dbeta'] is None else r['dbeta'].to(beta.dtype)
     dh0 = None if (h0 is None or r['dh0'] is None) else r['dh0'].to(h0.dtype)

@@ -12,7 +12,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from . import _lib
-from .nats_util import current_stream_ptr
+from .nats_util import aligned, current_stream_ptr, transforms_active
 
 
 _ROW_WIDTHS = (64, 128, 256, 512, 1024, 2048)
@@ -29,6 +29,16 @@ def _kernel_ok(x: torch.Tensor) -> bool:
 def _n_part(rows: int) -> int:
     """CTAs of the norms' backward kernels, each with one partial sum of the weight gradients: four per SM."""
     return int(min(-(-rows // 8), 592))
+
+
+_SUM_DTYPES = (torch.bfloat16, torch.float32)
+
+
+def _column_sums(part: torch.Tensor, mode: int, out0: torch.Tensor, out1: Optional[torch.Tensor] = None) -> None:
+    """Partial sums [P, ...] of the CTAs -> their totals in the parameters' dtypes (``natsl_column_sums``)."""
+    P = part.shape[0]
+    _lib.call("natsl_column_sums", part.data_ptr(), P, part.numel() // P, mode, out0.data_ptr(), _dt(out0), _lib.ptr(out1), _dt(out1),
+              current_stream_ptr(part.device))
 
 
 class _RMSNormFn(torch.autograd.Function):
@@ -56,7 +66,10 @@ class _RMSNormFn(torch.autograd.Function):
         dw_part = torch.empty(n_part, D, dtype=torch.float32, device=s.device)
         _lib.call("natsl_rmsnorm_bwd", s.data_ptr(), _lib.ptr(weight), _dt(weight), dy.data_ptr(), _lib.ptr(dadd), dx.data_ptr(),
                   dw_part.data_ptr(), n_part, rows, D, ctx.eps, current_stream_ptr(s.device))
-        dw = None if weight is None else dw_part.sum(0).to(weight.dtype)
+        dw = None
+        if weight is not None:
+            dw = torch.empty(D, dtype=weight.dtype, device=s.device)
+            _column_sums(dw_part, 0, dw)
         return dx, (dx if ctx.has_res else None), dw, None
 
 
@@ -86,16 +99,97 @@ class RMSNorm(nn.Module):
         return (y, x) if prenorm else y
 
 
+def _l2norm(x: torch.Tensor, eps: float) -> torch.Tensor:
+    xf = x.float()
+    return (xf * torch.rsqrt(xf.pow(2).sum(-1, keepdim=True) + eps)).to(x.dtype)
+
+
+class _L2NormFn(torch.autograd.Function):
+    """``natsl_l2norm_fwd`` / ``natsl_l2norm_bwd`` on [rows, D] bf16."""
+
+    @staticmethod
+    def forward(ctx, x, eps):
+        y = torch.empty_like(x)
+        _lib.call("natsl_l2norm_fwd", x.data_ptr(), y.data_ptr(), x.shape[0], x.shape[1], eps, current_stream_ptr(x.device))
+        ctx.save_for_backward(x)
+        ctx.eps = eps
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        x, = ctx.saved_tensors
+        if torch.is_grad_enabled():                          # a graph of the gradient is asked for: the same in torch operations
+            return torch.autograd.grad(_l2norm(x, ctx.eps), x, dy, create_graph=True)[0], None
+        dy = dy.contiguous()
+        dx = torch.empty_like(x)
+        _lib.call("natsl_l2norm_bwd", x.data_ptr(), dy.data_ptr(), dx.data_ptr(), x.shape[0], x.shape[1], ctx.eps, current_stream_ptr(x.device))
+        return dx, None
+
+
 class L2Norm(nn.Module):
-    """y = x * rsqrt(sum(x^2) + eps) (src/nats/layers/natsl_attn_mamba2.py:193-194)."""
+    """y = x * rsqrt(sum(x^2) + eps) (src/nats/layers/natsl_attn_mamba2.py:193-194).  CUDA bf16 inputs of 64, 128 or 256 features run
+    ``natsl_l2norm_fwd`` / ``natsl_l2norm_bwd``: 7 launches forward and 12 backward as torch operations."""
 
     def __init__(self, eps: float = 1e-6):
         super().__init__()
         self.eps = eps
 
     def forward(self, x):
-        xf = x.float()
-        return (xf * torch.rsqrt(xf.pow(2).sum(-1, keepdim=True) + self.eps)).to(x.dtype)
+        D = x.shape[-1]
+        if _kernel_ok(x) and D in (64, 128, 256) and x.numel() and not transforms_active():
+            return _L2NormFn.apply(aligned(x.contiguous()).view(-1, D), float(self.eps)).view(x.shape)
+        return _l2norm(x, self.eps)
+
+
+class _GatesFn(torch.autograd.Function):
+    """``natsl_gates_fwd`` / ``natsl_gates_bwd``: (g, beta or None, v * dt or None)."""
+
+    @staticmethod
+    def forward(ctx, a, b, v, A_log, dt_bias, neg_eigval):
+        H = a.shape[-1]
+        rows, V = a.numel() // H, (0 if v is None else v.shape[-1])
+        g = torch.empty(a.shape, dtype=torch.float32, device=a.device)
+        beta, vo = (None if x is None else torch.empty_like(x) for x in (b, v))
+        _lib.call("natsl_gates_fwd", a.data_ptr(), _lib.ptr(b), _lib.ptr(v), A_log.data_ptr(), _dt(A_log), dt_bias.data_ptr(), _dt(dt_bias),
+                  int(neg_eigval), g.data_ptr(), _lib.ptr(beta), _lib.ptr(vo), rows, H, V, current_stream_ptr(a.device))
+        ctx.save_for_backward(a, b, v, A_log, dt_bias)
+        ctx.neg = int(neg_eigval)
+        ctx.set_materialize_grads(False)
+        return g, beta, vo
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, dg, dbeta, dvo):
+        a, b, v, A_log, dt_bias = ctx.saved_tensors
+        H = a.shape[-1]
+        rows = a.numel() // H
+        dg, dbeta, dvo = (None if x is None else x.contiguous() for x in (dg, dbeta, dvo))
+        da, db = torch.empty_like(a), (None if b is None else torch.empty_like(b))
+        dv = None if dvo is None else torch.empty_like(v)
+        part = torch.empty(min(-(-rows // (256 // H)), 592), 2, H, dtype=torch.float32, device=a.device)
+        _lib.call("natsl_gates_bwd", a.data_ptr(), _lib.ptr(b), _lib.ptr(v), A_log.data_ptr(), _dt(A_log), dt_bias.data_ptr(), _dt(dt_bias),
+                  ctx.neg, _lib.ptr(dg), _lib.ptr(dbeta), _lib.DT_BF16 if dbeta is None else _dt(dbeta), _lib.ptr(dvo), da.data_ptr(),
+                  _lib.ptr(db), _lib.ptr(dv), part.data_ptr(), part.shape[0], rows, H, 0 if v is None else v.shape[-1],
+                  current_stream_ptr(a.device))
+        dA, dt_ = torch.empty_like(A_log), torch.empty_like(dt_bias)
+        _column_sums(part, 1, dA, dt_)
+        return da, db, dv, dA, dt_, None
+
+
+def layer_gates(a, A_log, dt_bias, b=None, v=None, neg_eigval: bool = False):
+    """dt = softplus(a + dt_bias), g = -exp(A_log) dt, beta = sigmoid(b) (times two with ``neg_eigval``), v * dt, in one kernel:
+    (g, beta, v * dt), or None where the torch operations have to run (a [B,T,H], b [B,T,H] or None, v [B,T,H,V] or None)."""
+    H = a.shape[-1]
+    if not (_kernel_ok(a) and 0 < H <= 256 and a.numel() and A_log.numel() == H == dt_bias.numel() and A_log.dtype in _SUM_DTYPES
+            and dt_bias.dtype in _SUM_DTYPES and A_log.is_contiguous() and dt_bias.is_contiguous() and A_log.device == a.device == dt_bias.device
+            and not transforms_active()):
+        return None
+    if b is not None and not (_kernel_ok(b) and b.shape == a.shape and b.device == a.device):
+        return None
+    if v is not None and not (_kernel_ok(v) and v.shape[:-1] == a.shape and v.shape[-1] in (32, 64, 128, 256) and v.device == a.device):
+        return None
+    return _GatesFn.apply(a.contiguous(), None if b is None else b.contiguous(), None if v is None else v.contiguous(), A_log, dt_bias,
+                          bool(neg_eigval))
 
 
 class _ShortConvFn(torch.autograd.Function):
@@ -128,6 +222,11 @@ class _ShortConvFn(torch.autograd.Function):
         dw_part = torch.empty(B * (-(-T // span)), D, W + 1, dtype=torch.float32, device=x.device)
         _lib.call("natsl_short_conv_bwd", x.data_ptr(), w2.data_ptr(), _lib.ptr(b2), dy.data_ptr(), dx.data_ptr(),
                   dw_part.data_ptr(), B, T, D, W, ctx.silu, span, current_stream_ptr(x.device))
+        if weight.dtype in _SUM_DTYPES and (bias is None or bias.dtype in _SUM_DTYPES):
+            dweight = torch.empty(weight.shape, dtype=weight.dtype, device=x.device)
+            dbias = None if bias is None else torch.empty(bias.shape, dtype=bias.dtype, device=x.device)
+            _column_sums(dw_part, W, dweight, dbias)
+            return dx, dweight, dbias, None
         dw = dw_part.sum(0)
         dweight = dw[:, :W].reshape(weight.shape).to(weight.dtype)
         dbias = None if bias is None else dw[:, W].to(bias.dtype)
@@ -189,6 +288,12 @@ class _BlockMeanFn(torch.autograd.Function):
     def backward(ctx, dy):
         T, nbs = ctx.T, ctx.nbs
         NB = dy.shape[1]
+        if _kernel_ok(dy) and not torch.is_grad_enabled():
+            B, _, D = dy.shape
+            dy = dy.contiguous()
+            dx = torch.empty(B, T, D, dtype=dy.dtype, device=dy.device)
+            _lib.call("natsl_block_mean_bwd", dy.data_ptr(), dx.data_ptr(), B, T, D, nbs, current_stream_ptr(dy.device))
+            return dx, None
         cnt = torch.full((NB,), float(nbs), device=dy.device)
         cnt[-1] = T - (NB - 1) * nbs
         dx = (dy.float() / cnt.view(1, NB, 1)).to(dy.dtype).repeat_interleave(nbs, dim=1)[:, :T]
@@ -275,8 +380,8 @@ class _NormGateMix(torch.autograd.Function):
                   _lib.ptr(dxw), dw_part.data_ptr(), n_part, rows, D, ctx.eps, ctx.activation, current_stream_ptr(x1.device))
         dw1 = dw2 = None
         if w1 is not None:
-            dw = dw_part.sum(0)
-            dw1, dw2 = dw[0].to(w1.dtype), dw[1].to(w2.dtype)
+            dw1, dw2 = (torch.empty(D, dtype=w.dtype, device=x1.device) for w in (w1, w2))
+            _column_sums(dw_part, 1, dw1, dw2)
         return dx1, dx2, dg, (None if xw is None else dxw.to(xw.dtype)), dw1, dw2, None, None
 
 

@@ -20,7 +20,7 @@ from .mixed_attn_gdn import nats_mixed_attn_gdn, nats_mixed_attn_gdn_chunk_infer
 from .decode_step import decode_token
 from .decoding import forward_cached
 from .layer_forward import layer_forward
-from .modules import FusedMultiInputRMSNormGated, RMSNorm, ShortConvolution, hard_softmax, mean_pooling
+from .modules import FusedMultiInputRMSNormGated, RMSNorm, ShortConvolution, hard_softmax, layer_gates, mean_pooling
 
 
 class NeuralAttentionSearchLinearAttnGDN(nn.Module):
@@ -214,10 +214,15 @@ class NeuralAttentionSearchLinearAttnGDN(nn.Module):
         v_attn = v_attn.unflatten(-1, (-1, self.head_attn_v_dim))
         if self.attn_qk_norm:
             q_attn, k_attn = self.q_norm(q_attn), self.k_norm(k_attn)
-        beta = self.b_proj(hidden_states).sigmoid()
-        if self.allow_neg_eigval:
-            beta = beta * 2.
-        g = -self.A_log.float().exp() * F.softplus(self.a_proj(hidden_states).float() + self.dt_bias)
+        a, b = self.a_proj(hidden_states), self.b_proj(hidden_states)
+        gates = layer_gates(a, self.A_log, self.dt_bias, b=b, neg_eigval=self.allow_neg_eigval)
+        if gates is not None:
+            g, beta, _ = gates
+        else:
+            beta = b.sigmoid()
+            if self.allow_neg_eigval:
+                beta = beta * 2.
+            g = -self.A_log.float().exp() * F.softplus(a.float() + self.dt_bias)
         return dict(q=q, k=k, v=v, q_attn=q_attn, k_attn=k_attn, v_attn=v_attn, beta=beta, g=g, o_weights=o_weights,
                     conv_state=new_state)
 
@@ -232,7 +237,7 @@ class NeuralAttentionSearchLinearAttnGDN(nn.Module):
         op_type_last = types[:, -1].clone()
         types[:, -1] = 1                                   # natsl_attn_gdn.py:553
         n_blocks = types.int().sum(1)
-        self.attn_fraction = (n_blocks.float()[..., 0] / types.shape[1]).mean(0).detach()
+        self.attn_blocks = (n_blocks, types.shape[1])
         p.update(types=types, types_raw=types_raw, n_blocks=n_blocks, op_type_last=op_type_last)
         return p
 

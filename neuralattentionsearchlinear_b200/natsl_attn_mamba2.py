@@ -20,7 +20,7 @@ from .decoding import forward_cached
 from .layer_forward import layer_forward
 from .mixed_attn_mamba import (nats_mixed_attn_mamba, nats_mixed_attn_mamba_chunk_inference,
                                nats_mixed_attn_mamba_recurrent)
-from .modules import FusedMultiInputRMSNormGated, L2Norm, RMSNorm, ShortConvolution, hard_softmax, mean_pooling
+from .modules import FusedMultiInputRMSNormGated, L2Norm, RMSNorm, ShortConvolution, hard_softmax, layer_gates, mean_pooling
 
 
 class NeuralAttentionSearchLinearAttnMamba(nn.Module):
@@ -191,9 +191,14 @@ class NeuralAttentionSearchLinearAttnMamba(nn.Module):
         if self.attn_qk_norm:
             q_attn, k_attn = self.q_norm(q_attn), self.k_norm(k_attn)
         q, k = self.q_norm2(q), self.k_norm2(k)
-        dt = F.softplus(self.a_proj(hidden_states).float() + self.dt_bias)
-        v = (v * dt.unsqueeze(-1)).to(v.dtype)
-        g = -self.A_log.float().exp() * dt
+        a = self.a_proj(hidden_states)
+        gates = layer_gates(a, self.A_log, self.dt_bias, v=v)
+        if gates is not None:
+            g, _, v = gates
+        else:
+            dt = F.softplus(a.float() + self.dt_bias)
+            v = (v * dt.unsqueeze(-1)).to(v.dtype)
+            g = -self.A_log.float().exp() * dt
         return dict(q=q, k=k, v=v, q_attn=q_attn, k_attn=k_attn, v_attn=v_attn, g=g, o_weights=o_weights,
                     conv_state=new_state)
 
@@ -207,7 +212,7 @@ class NeuralAttentionSearchLinearAttnMamba(nn.Module):
         op_type_last = types[:, -1].clone()
         types[:, -1] = 1
         n_blocks = types.int().sum(1)
-        self.attn_fraction = (n_blocks.float()[..., 0] / types.shape[1]).mean(0).detach()
+        self.attn_blocks = (n_blocks, types.shape[1])
         p.update(types=types, types_raw=types_raw, n_blocks=n_blocks, op_type_last=op_type_last)
         return p
 
