@@ -410,6 +410,8 @@ int natsl_attn_bwd(const void* q, const void* k, const void* v, const void* o, c
  *                            (invalid_dnats: also for chunks that do not update the state, from the raw values and the
  *                            state gradient of the next updating chunk).
  *  4 natsl_linear_bwd_intra  dq, dk [B,T,H,K], dv [B,T,H,V] bf16, dbeta, dg_tok [B,T,H] fp32, scal slot 3.
+ *    natsl_linear_bwd_intra_onto: the same, with dq (onto & 1), dk (& 2) and dv (& 4, delta rule) added to what the buffer
+ *                            holds, each sum of the two bf16 values rounded (buffers of 16-byte alignment).
  *  5 natsl_linear_bwd_dg     dg [B,T,H] fp32 from dg_tok and scal; flags as natsl_linear_fwd_h.
  * Replaces: chunk_gated_delta_rule_nats_bwd src/nats/ops/gated_delta_rule/chunk.py:170-332 (kernels
  * src/nats/ops/common/chunk_o.py:234-571, 927-1173, src/nats/ops/common/chunk_delta_h.py:346-635,
@@ -434,6 +436,12 @@ int natsl_linear_bwd_intra(int rule, const void* qn, const void* kn, const void*
                            const float* k_rstd, const float* dkd, const int32_t* types_i, void* dq, void* dk, void* dv,
                            float* dbeta, float* dg_tok, float* scal, int B, int T, int H, int HN, int K, int V, float scale,
                            int use_l2norm, void* stream);
+int natsl_linear_bwd_intra_onto(int rule, const void* qn, const void* kn, const void* v, const void* w, const void* u,
+                           const void* vp, const void* dvp, const void* dw, const void* d_o, const void* dq1,
+                           const void* dk1, const float* gcs, const void* beta, int beta_dtype, const float* q_rstd,
+                           const float* k_rstd, const float* dkd, const int32_t* types_i, void* dq, void* dk, void* dv,
+                           float* dbeta, float* dg_tok, float* scal, int B, int T, int H, int HN, int K, int V, float scale,
+                           int use_l2norm, int onto, void* stream);
 int natsl_linear_bwd_dg(const float* dg_tok, const float* scal, const int32_t* types_i, const int32_t* indices,
                         const int32_t* n_blocks, float* dg, int B, int T, int H, int HN, int flags, void* stream);
 

@@ -68,6 +68,8 @@ PROTOTYPES = {
                                _i, _i, _i, _i, _i, _i, _f, _i, _p],
     "natsl_linear_bwd_intra": [_i, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i, _p, _p, _p, _p, _p, _p, _p, _p,
                                _p, _p, _i, _i, _i, _i, _i, _i, _f, _i, _p],
+    "natsl_linear_bwd_intra_onto": [_i, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i, _p, _p, _p, _p, _p, _p, _p, _p,
+                                    _p, _p, _i, _i, _i, _i, _i, _i, _f, _i, _i, _p],
     "natsl_linear_bwd_dg": [_p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _p],
     "natsl_norm_gate_mix_bwd": [_p, _p, _p, _p, _i, _p, _p, _i, _p, _p, _p, _p, _p, _p, _i, C.c_long, _i, _f, _i, _p],
     "natsl_short_conv_fwd": [_p, _p, _p, _p, _i, _i, _i, _i, _i, _p],

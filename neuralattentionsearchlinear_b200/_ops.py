@@ -510,11 +510,12 @@ def attn_bwd(q, k, v, o, lse, do, tables: SelectionTables, scale: float, own_chu
 
 def linear_bwd(rule: int, q, k, v, g, beta, tables: SelectionTables, scale: float, h0, decay: bool, use_l2norm: bool,
                do, dht=None, invalid_dnats: bool = True, trailing_quirk: bool = True, return_intermediates: bool = False,
-               timer: StageTimer | None = None, per_tile: bool = False):
+               timer: StageTimer | None = None, per_tile: bool = False, onto=None):
     """Backward of the linear branch (block size 64).  Recomputes the forward's preparation and recurrence, then runs the
     five backward stages.  -> dict(dq, dk, dv bf16; dg fp32; dbeta fp32 or None; dh0 fp32 or None; dnats [B,NT,HN] fp32
     = the reference's dnats column for the linear branch, src/nats/ops/common/chunk_o.py:440-443, 459-492, 1568-1575; with
-    ``per_tile`` [B,NT,H], per head)."""
+    ``per_tile`` [B,NT,H], per head).  ``onto``: gradients of q, k and (delta rule) v (or None) to add to, in place; a separate sum of two
+    [8,4096,16,128] tensors is a pass of 59 us."""
     gdn = rule == _lib.RULE_GDN
     for t_ in (q, k, v, do):
         _need(t_.dtype == BF16, "linear-branch backward needs bf16 tensors", TypeError)
@@ -586,16 +587,25 @@ def linear_bwd(rule: int, q, k, v, g, beta, tables: SelectionTables, scale: floa
               tables.starting_h_idx.data_ptr(), _lib.ptr(vp if gdn else None), _lib.ptr(dw), dq1.data_ptr(), dk1.data_ptr(),
               dkd.data_ptr(), scal.data_ptr(), dn_lin.data_ptr(), B, T, H, HN, K, V, float(scale), int(invalid_dnats), st)
     # ---- 4: the 64 x 64 part, the WY transform and the l2 norm
-    dq, dk = torch.empty_like(q), torch.empty_like(k)
-    dv = torch.empty_like(v) if gdn else dvp
+    bits = 0
+    if onto is None:
+        dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v) if gdn else dvp
+    else:
+        _need(gdn or onto[2] is None, "Mamba2's dv is not added to another gradient", NotImplementedError)
+        for i, (d, x) in enumerate(zip(onto, (q, k, v))):
+            _need(d is None or (d.shape == x.shape and d.dtype == BF16 and d.is_contiguous()), "a gradient to add to has another form")
+            bits |= 0 if d is None else 1 << i
+        dq, dk, dv = (torch.empty_like(x) if d is None else d for d, x in zip(onto, (q, k, v)))
+        if not gdn:
+            dv = dvp
     dbeta = torch.empty(B, T, H, **f32) if gdn else None
     dg_tok = torch.empty(B, T, H, **f32)
-    _call(timer, "bwd_intra", "natsl_linear_bwd_intra", rule, qn.data_ptr(), kn.data_ptr(), _lib.ptr(v if gdn else None), _lib.ptr(w),
+    _call(timer, "bwd_intra", "natsl_linear_bwd_intra_onto", rule, qn.data_ptr(), kn.data_ptr(), _lib.ptr(v if gdn else None), _lib.ptr(w),
               _lib.ptr(u if gdn else None), vp.data_ptr(), _lib.ptr(dvp if gdn else None), _lib.ptr(dw), do.data_ptr(),
               dq1.data_ptr(), dk1.data_ptr(), gcs.data_ptr(), _lib.ptr(beta if gdn else None),
               _lib.DT_BF16 if (gdn and beta.dtype == BF16) else _lib.DT_F32, _lib.ptr(qrs), _lib.ptr(krs), dkd.data_ptr(),
               tables.types_i.data_ptr(), dq.data_ptr(), dk.data_ptr(), _lib.ptr(dv if gdn else None), _lib.ptr(dbeta),
-              dg_tok.data_ptr(), scal.data_ptr(), B, T, H, HN, K, V, float(scale), int(l2), st)
+              dg_tok.data_ptr(), scal.data_ptr(), B, T, H, HN, K, V, float(scale), int(l2), bits, st)
     # ---- 5: decay gradients
     dg = torch.empty(B, T, H, **f32)
     _call(timer, "bwd_dg", "natsl_linear_bwd_dg", dg_tok.data_ptr(), scal.data_ptr(), tables.types_i.data_ptr(), tables.indices.data_ptr(),

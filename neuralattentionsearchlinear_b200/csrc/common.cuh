@@ -255,6 +255,27 @@ __device__ __forceinline__ void load_tile_async(uint32_t tile, const __nv_bfloat
     }
 }
 
+// Add four or eight bf16 values to those in global memory, each sum rounded to nearest.  With one writer per address the result is that
+// of a load, an add and a store; the addition is done at the L2 cache and nothing waits for it.
+__device__ __forceinline__ void red_bf16x4(__nv_bfloat16* p, uint2 v) {
+    asm volatile("red.relaxed.gpu.global.add.noftz.v2.bf16x2 [%0], {%1, %2};" ::"l"(p), "r"(v.x), "r"(v.y) : "memory");
+}
+__device__ __forceinline__ void red_bf16x8(__nv_bfloat16* p, uint4 v) {
+    asm volatile("red.relaxed.gpu.global.add.noftz.v4.bf16x2 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
+                 : "memory");
+}
+
+// Add a swizzled [ROWS][COLS] bf16 shared tile to global memory, 16 bytes per lane.
+template <int ROWS, int COLS, int NT>
+__device__ __forceinline__ void add_tile(const unsigned char* tile, __nv_bfloat16* g, long gstride, int valid_rows, int tid) {
+    constexpr int CPR = COLS / 8;
+#pragma unroll
+    for (int i = tid; i < ROWS * CPR; i += NT) {
+        const int r = i / CPR, c = i % CPR;
+        if (r < valid_rows) red_bf16x8(g + (long)r * gstride + c * 8, *reinterpret_cast<const uint4*>(tile + swz<COLS * 2>(r, c)));
+    }
+}
+
 // Store a swizzled [ROWS][COLS] bf16 shared tile to global with 16-byte coalesced stores.
 template <int ROWS, int COLS, int NT>
 __device__ __forceinline__ void store_tile(const unsigned char* tile, __nv_bfloat16* g, long gstride, int valid_rows,

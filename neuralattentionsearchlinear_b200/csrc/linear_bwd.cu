@@ -575,6 +575,9 @@ linear_bwd_state_kernel(const __nv_bfloat16* __restrict__ kn, const __nv_bfloat1
 //     e: dq1, then H, then u      f: A, then w, then dk1      m: dqk, then the diagonal blocks X, then dkk
 // dq is finished and stored before the solves, so that its accumulators do not live through them (they were spilled: 709 us at
 // B = 8, T = 4096, 16 heads of 128 / 128, now 637 us); dq and dk leave from registers.
+// Where both branches read one tensor, its gradient is added onto the softmax branch's (ONTO, bits of q, k, v) with reductions at the
+// L2 cache: 645 us at that size for all three, 641 us without, and no sums of 178 us behind it.  An instance of its own: tested at
+// run time in one kernel for both, calls that add nothing took longer (Mamba2 at B = 4, T = 1000, 16 heads: 40.5 against 37.6 us).
 template <int K, int V, bool GDN>
 struct InSmem {
     static constexpr int cmax(int x, int y) { return x > y ? x : y; }
@@ -623,7 +626,7 @@ __device__ __forceinline__ void solve_t_group(uint32_t htile, uint32_t ztile, un
     }
 }
 
-template <int K, int V, bool GDN>
+template <int K, int V, bool GDN, bool ONTO>
 __global__ void __launch_bounds__(LB_THREADS, 2)
 linear_bwd_intra_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat16* __restrict__ kn,
                         const __nv_bfloat16* __restrict__ v, const __nv_bfloat16* __restrict__ w,
@@ -635,7 +638,7 @@ linear_bwd_intra_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat1
                         const float* __restrict__ dkd, const int* __restrict__ types_i, __nv_bfloat16* __restrict__ dq,
                         __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv, float* __restrict__ dbeta,
                         float* __restrict__ dg_tok, float* __restrict__ scal, int T, int H, int HN, float scale,
-                        int use_l2norm) {
+                        int use_l2norm, int onto) {
     using L = InSmem<K, V, GDN>;
     extern __shared__ __align__(256) unsigned char smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -792,7 +795,7 @@ linear_bwd_intra_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat1
             acc_q[nt][0] = qra * (acc_q[nt][0] - qna.x * pq_a); acc_q[nt][1] = qra * (acc_q[nt][1] - qna.y * pq_a);
             acc_q[nt][2] = qrb * (acc_q[nt][2] - qnb.x * pq_b); acc_q[nt][3] = qrb * (acc_q[nt][3] - qnb.y * pq_b);
         }
-        store_acc_global<NK>(dq + (tok0 * H + h) * K, (long)H * K, acc_q, r0, nk0, valid, lane);
+        store_acc_global<NK>(dq + (tok0 * H + h) * K, (long)H * K, acc_q, r0, nk0, valid, lane, ONTO && (onto & 1));
     }
 
     if (GDN) {
@@ -977,8 +980,11 @@ linear_bwd_intra_kernel(const __nv_bfloat16* __restrict__ qn, const __nv_bfloat1
             acc_k[nt][0] = kra * (acc_k[nt][0] - kna.x * pk_a); acc_k[nt][1] = kra * (acc_k[nt][1] - kna.y * pk_a);
             acc_k[nt][2] = krb * (acc_k[nt][2] - knb.x * pk_b); acc_k[nt][3] = krb * (acc_k[nt][3] - knb.y * pk_b);
         }
-        store_acc_global<NK>(dk + (tok0 * H + h) * K, (long)H * K, acc_k, r0, nk0, valid, lane);
-        if (GDN) store_tile<64, V, LB_THREADS>(c_p, dv + (tok0 * H + h) * V, (long)H * V, valid, tid);
+        store_acc_global<NK>(dk + (tok0 * H + h) * K, (long)H * K, acc_k, r0, nk0, valid, lane, ONTO && (onto & 2));
+        if (GDN) {
+            if (ONTO && (onto & 4)) add_tile<64, V, LB_THREADS>(c_p, dv + (tok0 * H + h) * V, (long)H * V, valid, tid);
+            else store_tile<64, V, LB_THREADS>(c_p, dv + (tok0 * H + h) * V, (long)H * V, valid, tid);
+        }
     }
     if (tid < 64) {
         const float eg = __expf(s_g[tid]);
@@ -1124,13 +1130,13 @@ static int launch_intra(const void* qn, const void* kn, const void* v, const voi
                         const void* dvp, const void* dw, const void* d_o, const void* dq1, const void* dk1, const float* gcs,
                         const void* beta, int beta_dtype, const float* q_rstd, const float* k_rstd, const float* dkd,
                         const int* types_i, void* dq, void* dk, void* dv, float* dbeta, float* dg_tok, float* scal, int B,
-                        int T, int H, int HN, float scale, int use_l2norm, cudaStream_t st) {
-    auto kern = linear_bwd_intra_kernel<K, V, GDN>;
+                        int T, int H, int HN, float scale, int use_l2norm, int onto, cudaStream_t st) {
+    auto kern = onto ? linear_bwd_intra_kernel<K, V, GDN, true> : linear_bwd_intra_kernel<K, V, GDN, false>;
     int rc = reserve_smem(kern, InSmem<K, V, GDN>::total, "natsl_linear_bwd_intra");
     if (rc != NATSL_OK) return rc;
     kern<<<dim3((T + 63) / 64, H, B), LB_THREADS, InSmem<K, V, GDN>::total, st>>>(
         bfc(qn), bfc(kn), bfc(v), bfc(w), bfc(u), bfc(vp), bfc(dvp), bfc(dw), bfc(d_o), bfc(dq1), bfc(dk1), gcs, beta,
-        beta_dtype, q_rstd, k_rstd, dkd, types_i, bfm(dq), bfm(dk), bfm(dv), dbeta, dg_tok, scal, T, H, HN, scale, use_l2norm);
+        beta_dtype, q_rstd, k_rstd, dkd, types_i, bfm(dq), bfm(dk), bfm(dv), dbeta, dg_tok, scal, T, H, HN, scale, use_l2norm, onto);
     return check_launch("natsl_linear_bwd_intra");
 }
 
@@ -1212,12 +1218,12 @@ extern "C" int natsl_linear_bwd_state(int rule, const void* kn, const void* v, c
     return NATSL_ERR_UNSUPPORTED;
 }
 
-extern "C" int natsl_linear_bwd_intra(int rule, const void* qn, const void* kn, const void* v, const void* w, const void* u,
-                                      const void* vp, const void* dvp, const void* dw, const void* d_o, const void* dq1,
-                                      const void* dk1, const float* gcs, const void* beta, int beta_dtype, const float* q_rstd,
-                                      const float* k_rstd, const float* dkd, const int32_t* types_i, void* dq, void* dk,
-                                      void* dv, float* dbeta, float* dg_tok, float* scal, int B, int T, int H, int HN, int K,
-                                      int V, float scale, int use_l2norm, void* stream) {
+extern "C" int natsl_linear_bwd_intra_onto(int rule, const void* qn, const void* kn, const void* v, const void* w, const void* u,
+                                           const void* vp, const void* dvp, const void* dw, const void* d_o, const void* dq1,
+                                           const void* dk1, const float* gcs, const void* beta, int beta_dtype, const float* q_rstd,
+                                           const float* k_rstd, const float* dkd, const int32_t* types_i, void* dq, void* dk,
+                                           void* dv, float* dbeta, float* dg_tok, float* scal, int B, int T, int H, int HN, int K,
+                                           int V, float scale, int use_l2norm, int onto, void* stream) {
     using namespace natsl;
     NATSL_REQUIRE(qn && kn && vp && d_o && dq1 && dk1 && gcs && dkd && types_i && dq && dk && dg_tok && scal, NATSL_ERR_NULL,
                   "natsl_linear_bwd_intra: null pointer");
@@ -1227,8 +1233,12 @@ extern "C" int natsl_linear_bwd_intra(int rule, const void* qn, const void* kn, 
     NATSL_REQUIRE(!use_l2norm || (q_rstd && k_rstd), NATSL_ERR_NULL, "natsl_linear_bwd_intra: 1/norm factors are required");
     NATSL_REQUIRE(B > 0 && T > 0 && H > 0 && HN > 0 && H % HN == 0 && B <= 65535 && H <= 65535, NATSL_ERR_BAD_SHAPE,
                   "natsl_linear_bwd_intra: bad shape");
+    NATSL_REQUIRE(onto >= 0 && onto < 8 && (rule == NATSL_RULE_GDN || !(onto & 4)), NATSL_ERR_UNSUPPORTED,
+                  "natsl_linear_bwd_intra: onto=%d (bits of dq, dk and, with the delta rule, dv)", onto);
+    NATSL_REQUIRE(!onto || aligned_to(16, dq, dk, dv), NATSL_ERR_UNSUPPORTED,
+                  "natsl_linear_bwd_intra: a gradient to be added to does not start on 16 bytes");
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-#define NATSL_ARGS qn, kn, v, w, u, vp, dvp, dw, d_o, dq1, dk1, gcs, beta, beta_dtype, q_rstd, k_rstd, dkd, types_i, dq, dk, dv, dbeta, dg_tok, scal, B, T, H, HN, scale, use_l2norm, st
+#define NATSL_ARGS qn, kn, v, w, u, vp, dvp, dw, d_o, dq1, dk1, gcs, beta, beta_dtype, q_rstd, k_rstd, dkd, types_i, dq, dk, dv, dbeta, dg_tok, scal, B, T, H, HN, scale, use_l2norm, onto, st
 #define NATSL_CASE(KK, VV)                                                             \
     if (K == KK && V == VV)                                                            \
         return rule == NATSL_RULE_GDN ? launch_intra<KK, VV, true>(NATSL_ARGS) : launch_intra<KK, VV, false>(NATSL_ARGS);
@@ -1237,6 +1247,17 @@ extern "C" int natsl_linear_bwd_intra(int rule, const void* qn, const void* kn, 
 #undef NATSL_ARGS
     set_error("natsl_linear_bwd_intra: unsupported head dims K=%d V=%d (64 or 128 each)", K, V);
     return NATSL_ERR_UNSUPPORTED;
+}
+
+extern "C" int natsl_linear_bwd_intra(int rule, const void* qn, const void* kn, const void* v, const void* w, const void* u,
+                                      const void* vp, const void* dvp, const void* dw, const void* d_o, const void* dq1,
+                                      const void* dk1, const float* gcs, const void* beta, int beta_dtype, const float* q_rstd,
+                                      const float* k_rstd, const float* dkd, const int32_t* types_i, void* dq, void* dk,
+                                      void* dv, float* dbeta, float* dg_tok, float* scal, int B, int T, int H, int HN, int K,
+                                      int V, float scale, int use_l2norm, void* stream) {
+    return natsl_linear_bwd_intra_onto(rule, qn, kn, v, w, u, vp, dvp, dw, d_o, dq1, dk1, gcs, beta, beta_dtype, q_rstd,
+                                       k_rstd, dkd, types_i, dq, dk, dv, dbeta, dg_tok, scal, B, T, H, HN, K, V, scale,
+                                       use_l2norm, 0, stream);
 }
 
 extern "C" int natsl_linear_bwd_dg(const float* dg_tok, const float* scal, const int32_t* types_i, const int32_t* indices,

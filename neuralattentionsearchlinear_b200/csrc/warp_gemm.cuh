@@ -82,8 +82,10 @@ __device__ __forceinline__ void store_acc_bf16(unsigned char* tile, const float 
 
 // Write a strip straight to global memory (row r at g + r * gstride, columns n0..), rows from `valid` on left out: neighbouring lanes
 // swap halves of neighbouring n-tiles, so that a store covers whole 32-byte sectors and no staging tile or barrier is needed.
+// onto: the strip is added to what is there.
 template <int NT8>
-__device__ __forceinline__ void store_acc_global(__nv_bfloat16* g, long gstride, const float (&acc)[NT8][4], int m0, int n0, int valid, int lane) {
+__device__ __forceinline__ void store_acc_global(__nv_bfloat16* g, long gstride, const float (&acc)[NT8][4], int m0, int n0, int valid, int lane,
+                                                 bool onto = false) {
     const int gq = lane >> 2, qd = lane & 3;
     const bool odd = qd & 1;
     __nv_bfloat16* pa = g + (long)(m0 + gq) * gstride + n0 + (odd ? 8 : 0) + (qd >> 1) * 4;
@@ -96,7 +98,11 @@ __device__ __forceinline__ void store_acc_global(__nv_bfloat16* g, long gstride,
             const uint32_t x = pack_bf16(acc[2 * p][e], acc[2 * p][e + 1]), y = pack_bf16(acc[2 * p + 1][e], acc[2 * p + 1][e + 1]);
             const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? x : y, 1);
             const uint2 v = odd ? make_uint2(got, y) : make_uint2(x, got);
-            if (e ? okb : oka) *reinterpret_cast<uint2*>((e ? pb : pa) + 16 * p) = v;
+            __nv_bfloat16* to = (e ? pb : pa) + 16 * p;
+            if (e ? okb : oka) {
+                if (onto) red_bf16x4(to, v);
+                else *reinterpret_cast<uint2*>(to) = v;
+            }
         }
     }
 }

@@ -114,7 +114,10 @@ def hybrid_backward(ctx, rule, do_lin, do_attn, dht):
     dqa, dka, dva, dn_attn = _ops.attn_bwd(q_attn, k_attn, v_attn, o_attn, lse, do_attn.to(o_attn.dtype), tables,
                                            ctx.scale_attn, ctx.own_attn, reference_compat=ctx.compat, per_tile=one)
     r = _ops.linear_bwd(rule, q, k, v, g, beta, tables, ctx.scale_lattn, h0, ctx.decay, ctx.use_l2norm,
-                        do_lin.to(q.dtype), dht=dht, invalid_dnats=ctx.invalid_dnats_linear, per_tile=one)
+                        do_lin.to(q.dtype), dht=dht, invalid_dnats=ctx.invalid_dnats_linear, per_tile=one,
+                        onto=None if ctx.shared is None else [d if s else None for d, s in zip((dqa, dka, dva), ctx.shared)])
+    if ctx.shared is not None:
+        dqa, dka, dva = (None if s else d for d, s in zip((dqa, dka, dva), ctx.shared))
     if one:
         B, TN, HN, _ = tables.types_i.shape
         dnats = torch.empty(B, TN, HN, 2, dtype=ctx.types_dtype, device=q.device)
@@ -129,7 +132,7 @@ def hybrid_backward(ctx, rule, do_lin, do_attn, dht):
     return dqa, dka, dva, r['dq'], r['dk'], r['dv'], dh0, dg, dbeta, dnats
 
 
-def save_hybrid(ctx, tensors, flat, types, T, nbs, scale_attn, scale_lattn, own_attn, decay, use_l2norm, invalid_dnats):
+def save_hybrid(ctx, rule, tensors, flat, types, T, nbs, scale_attn, scale_lattn, own_attn, decay, use_l2norm, invalid_dnats):
     """What ``hybrid_backward`` needs from a forward of ``_ops.hybrid_fwd``."""
     K, V = tensors[5].shape[-1], tensors[7].shape[-1]
     if nbs != CHUNK_SIZE:
@@ -137,11 +140,19 @@ def save_hybrid(ctx, tensors, flat, types, T, nbs, scale_attn, scale_lattn, own_
     elif K not in (64, 128) or V not in (64, 128):
         ctx.bwd_ok, ctx.bwd_why = False, "the backward pass is built for linear-branch head dims 64 and 128"
     ctx.save_for_backward(*tensors)
+    ctx.shared = shared_inputs(rule, tensors[:3], tensors[5:8])
     ctx.tables, ctx.flat_tables = None, (flat, types.shape[0], types.shape[1], types.shape[2], T, nbs)
     ctx.scale_attn, ctx.scale_lattn, ctx.own_attn = float(scale_attn), float(scale_lattn), own_attn
     ctx.decay, ctx.use_l2norm, ctx.invalid_dnats_linear = bool(decay), bool(use_l2norm), bool(invalid_dnats)
     ctx.compat = REFERENCE_COMPAT_BWD
     ctx.types_dtype = types.dtype
+
+
+def shared_inputs(rule, attn, lin):
+    """Which of q, k and v are one tensor for both branches (None: none of them): its gradients are added up by the linear branch's
+    backward (v's with the delta rule only) instead of by autograd."""
+    same = attn[0] is lin[0], attn[1] is lin[1], attn[2] is lin[2] and rule == _lib.RULE_GDN
+    return same if True in same else None
 
 
 class NAtSMixedAttentionGDN(torch.autograd.Function):
@@ -178,7 +189,7 @@ class NAtSMixedAttentionGDN(torch.autograd.Function):
                 _lib.RULE_GDN, q_attn, k_attn, v_attn, q_lattn, k_lattn, v_lattn, g, beta, nats_block_types, nats_block_size,
                 scale_attn, scale_lattn, initial_state_gated_delta, strategy['attn'], decay_for_non_gdn_blocks,
                 lattn_use_qk_l2norm_in_kernel, output_final_state_gated_delta)
-            save_hybrid(ctx, (q_attn, k_attn, v_attn, o_attn, lse, q_lattn, k_lattn, v_lattn, g, beta, initial_state_gated_delta),
+            save_hybrid(ctx, _lib.RULE_GDN, (q_attn, k_attn, v_attn, o_attn, lse, q_lattn, k_lattn, v_lattn, g, beta, initial_state_gated_delta),
                         flat, nats_block_types, T, nats_block_size, scale_attn, scale_lattn, strategy['attn'],
                         decay_for_non_gdn_blocks, lattn_use_qk_l2norm_in_kernel, compute_dnats_for_invalid_blocks_linear_att)
             return o_gdn, o_attn, ht
@@ -227,6 +238,7 @@ class NAtSMixedAttentionGDN(torch.autograd.Function):
             ctx.bwd_ok, ctx.bwd_why = False, "the backward pass is built for linear-branch head dims 64 and 128"
         ctx.save_for_backward(q_attn, k_attn, v_attn, o_attn, lse, q_lattn, k_lattn, v_lattn, g, beta,
                               initial_state_gated_delta)
+        ctx.shared = shared_inputs(_lib.RULE_GDN, (q_attn, k_attn, v_attn), (q_lattn, k_lattn, v_lattn))
         ctx.tables = tables
         ctx.scale_attn, ctx.scale_lattn, ctx.own_attn = float(scale_attn), float(scale_lattn), strategy['attn']
         ctx.decay, ctx.use_l2norm = bool(decay_for_non_gdn_blocks), bool(lattn_use_qk_l2norm_in_kernel)

@@ -43,7 +43,7 @@ class NAtSMixedAttentionMamba(torch.autograd.Function):
                 _lib.RULE_MAMBA, q_attn, k_attn, v_attn, q_lattn, k_lattn, v_lattn, g, None, nats_block_types, nats_block_size,
                 scale_attn, scale_lattn, initial_state_mamba, strategy['attn'], decay_for_non_mamba_blocks, False,
                 output_final_state_mamba)
-            gdn_ops.save_hybrid(ctx, (q_attn, k_attn, v_attn, o_attn, lse, q_lattn, k_lattn, v_lattn, g, None, initial_state_mamba),
+            gdn_ops.save_hybrid(ctx, _lib.RULE_MAMBA, (q_attn, k_attn, v_attn, o_attn, lse, q_lattn, k_lattn, v_lattn, g, None, initial_state_mamba),
                                 flat, nats_block_types, T, nats_block_size, scale_attn, scale_lattn, strategy['attn'],
                                 decay_for_non_mamba_blocks, False, compute_dnats_for_invalid_blocks_linear_att)
             return o_m, o_attn, ht
@@ -68,6 +68,7 @@ class NAtSMixedAttentionMamba(torch.autograd.Function):
         elif nats_block_size != 64:
             ctx.bwd_ok, ctx.bwd_why = False, "the backward pass is built for nats_block_size = 64"
         ctx.save_for_backward(q_attn, k_attn, v_attn, o_attn, lse, q_lattn, k_lattn, v_lattn, g, None, initial_state_mamba)
+        ctx.shared = gdn_ops.shared_inputs(_lib.RULE_MAMBA, (q_attn, k_attn, v_attn), (q_lattn, k_lattn, v_lattn))
         ctx.tables = tables
         ctx.scale_attn, ctx.scale_lattn, ctx.own_attn = float(scale_attn), float(scale_lattn), strategy['attn']
         ctx.decay, ctx.use_l2norm = bool(decay_for_non_mamba_blocks), False

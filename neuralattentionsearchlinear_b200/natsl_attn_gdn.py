@@ -208,10 +208,11 @@ class NeuralAttentionSearchLinearAttnGDN(nn.Module):
             o_weights = self.nats_out_weights_layer(q).unflatten(-1, (self.num_attn_heads, self.n_ops)).softmax(-1)
         q = q.unflatten(-1, (-1, self.head_k_dim))
         k = k.unflatten(-1, (-1, self.head_k_dim))
+        one_v = v_attn is v and self.head_attn_v_dim == self.head_v_dim
         v = v.unflatten(-1, (-1, self.head_v_dim))
         q_attn = q_attn.unflatten(-1, (-1, self.head_attn_k_dim))
         k_attn = k_attn.unflatten(-1, (-1, self.head_attn_k_dim))
-        v_attn = v_attn.unflatten(-1, (-1, self.head_attn_v_dim))
+        v_attn = v if one_v else v_attn.unflatten(-1, (-1, self.head_attn_v_dim))
         if self.attn_qk_norm:
             q_attn, k_attn = self.q_norm(q_attn), self.k_norm(k_attn)
         a, b = self.a_proj(hidden_states), self.b_proj(hidden_states)
