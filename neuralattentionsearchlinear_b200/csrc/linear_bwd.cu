@@ -38,16 +38,20 @@ __device__ __forceinline__ float kdecay(float gl, float g, bool gdn) {
     return __expf(gdn ? fminf(d, 80.f) : fminf(d, 0.f));
 }
 
-// Row sums of squares of a [64][COLS] bf16 tile -> rstd[64] (1 when !use), 8 warps.
+// The rows of a [64][COLS] bf16 tile over their l2 norms, in place and to global memory, with the 1/norm factors; 8 warps, COLS / 8
+// lanes per row, which keep the row between its sum and its scaling.
 template <int COLS>
-__device__ __forceinline__ void row_rstd(const unsigned char* tile, float* rstd, int use, int warp, int lane) {
-    constexpr int CPR = COLS / 8;
-    constexpr int RPP = 32 / CPR;
-    const int sub = lane / CPR, cc = lane % CPR;
-    for (int rr = 0; rr < 8; rr += RPP) {
-        const int r = warp * 8 + rr + sub;
-        const uint4 xv = *reinterpret_cast<const uint4*>(tile + swz<COLS * 2>(r, cc));
-        const uint32_t* xw = reinterpret_cast<const uint32_t*>(&xv);
+__device__ __forceinline__ void l2norm_rows(unsigned char* tile, __nv_bfloat16* g, long gstride, float* rstd, int rstride, int valid,
+                                            int warp, int lane) {
+    constexpr int CPR = COLS / 8, RPP = 32 / CPR, N = 8 / RPP;
+    const int cc = lane % CPR, row0 = warp * 8 + lane / CPR;
+    uint4 x[N];
+#pragma unroll
+    for (int n = 0; n < N; ++n) x[n] = *reinterpret_cast<const uint4*>(tile + swz<COLS * 2>(row0 + n * RPP, cc));
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+        const int r = row0 + n * RPP;
+        uint32_t* xw = reinterpret_cast<uint32_t*>(&x[n]);
         float ss = 0.f;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -56,41 +60,37 @@ __device__ __forceinline__ void row_rstd(const unsigned char* tile, float* rstd,
         }
 #pragma unroll
         for (int o = CPR / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        if (cc == 0) rstd[r] = use ? rsqrtf(ss + 1e-6f) : 1.0f;
-    }
-}
-
-template <int COLS>
-__device__ __forceinline__ void scale_rows(unsigned char* tile, const float* rowscale, int tid) {
-    constexpr int CPR = COLS / 8;
-    for (int i = tid; i < 64 * CPR; i += LB_THREADS) {
-        const int r = i / CPR, c = i % CPR;
-        uint4* p = reinterpret_cast<uint4*>(tile + swz<COLS * 2>(r, c));
-        uint4 x = *p;
-        const float s = rowscale[r];
-        uint32_t* xw = reinterpret_cast<uint32_t*>(&x);
+        const float f = rsqrtf(ss + 1e-6f);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const float2 f = unpack_bf16(xw[j]);
-            xw[j] = pack_bf16(f.x * s, f.y * s);
+            const float2 t = unpack_bf16(xw[j]);
+            xw[j] = pack_bf16(t.x * f, t.y * f);
         }
-        *p = x;
+        *reinterpret_cast<uint4*>(tile + swz<COLS * 2>(r, cc)) = x[n];
+        if (r < valid) {
+            *reinterpret_cast<uint4*>(g + (long)r * gstride + cc * 8) = x[n];
+            if (cc == 0) rstd[(long)r * rstride] = f;
+        }
     }
 }
 
 // ================================================================================================ pre
+// Bound by memory (q, k, do in, qn, kn, dv'_loc out: 805 MB at B = 8, T = 4096, 16 heads of 128 / 128, 123 us at the copy rate; it
+// takes 144 us).  P takes the place of q, so that 49 KB and 64 registers leave room for four blocks per SM; a row is summed, scaled
+// and stored by the lanes that hold it, do is waited for before the second product, dv'_loc leaves from registers, and tiles above
+// the diagonal are left out.  With a pass each for sums, scaling and stores, and three blocks per SM, it took 195 us.
 template <int K, int V>
 struct PreSmem {
-    static constexpr int qs = 0;
+    static constexpr int qs = 0;                          // q, then P
     static constexpr int ks = qs + 64 * K * 2;
     static constexpr int dos = ks + 64 * K * 2;
-    static constexpr int ps = dos + 64 * V * 2;
-    static constexpr int vec = ps + 64 * 64 * 2;          // g, q rstd, k rstd
-    static constexpr int total = vec + 3 * 64 * 4;
+    static constexpr int vec = dos + 64 * V * 2;          // g
+    static constexpr int total = vec + 64 * 4;
+    static_assert(64 * 64 * 2 <= ks, "P takes q's place");
 };
 
 template <int K, int V>
-__global__ void __launch_bounds__(LB_THREADS)
+__global__ void __launch_bounds__(LB_THREADS, 4)
 linear_bwd_pre_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
                       const __nv_bfloat16* __restrict__ d_o, const float* __restrict__ gcs, __nv_bfloat16* __restrict__ qn,
                       __nv_bfloat16* __restrict__ kn, float* __restrict__ q_rstd, float* __restrict__ k_rstd,
@@ -104,33 +104,21 @@ linear_bwd_pre_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* 
     const long tok0 = (long)b * T + (long)c * 64;
     unsigned char* qs_p = smem + L::qs;
     unsigned char* ks_p = smem + L::ks;
-    unsigned char* dos_p = smem + L::dos;
-    unsigned char* ps_p = smem + L::ps;
-    const uint32_t qs = smem_u32(qs_p), ks = smem_u32(ks_p), dos = smem_u32(dos_p), ps = smem_u32(ps_p);
+    const uint32_t qs = smem_u32(qs_p), ks = smem_u32(ks_p), dos = smem_u32(smem + L::dos);
     float* s_g = reinterpret_cast<float*>(smem + L::vec);
-    float* s_qr = s_g + 64;
-    float* s_kr = s_qr + 64;
 
     load_tile_async<64, K, LB_THREADS>(qs, q + (tok0 * H + h) * K, (long)H * K, valid, tid);
     load_tile_async<64, K, LB_THREADS>(ks, k + (tok0 * H + h) * K, (long)H * K, valid, tid);
+    cp_async_commit();
     load_tile_async<64, V, LB_THREADS>(dos, d_o + (tok0 * H + h) * V, (long)H * V, valid, tid);
     cp_async_commit();
     if (tid < 64) s_g[tid] = gcs[(tok0 + min(tid, valid - 1)) * H + h];
-    cp_async_wait<0>();
-    __syncthreads();
-    row_rstd<K>(qs_p, s_qr, use_l2norm, warp, lane);
-    row_rstd<K>(ks_p, s_kr, use_l2norm, warp, lane);
+    cp_async_wait<1>();
     __syncthreads();
     if (use_l2norm) {
-        scale_rows<K>(qs_p, s_qr, tid);
-        scale_rows<K>(ks_p, s_kr, tid);
-        if (tid < valid) {
-            q_rstd[(tok0 + tid) * H + h] = s_qr[tid];
-            k_rstd[(tok0 + tid) * H + h] = s_kr[tid];
-        }
+        l2norm_rows<K>(qs_p, qn + (tok0 * H + h) * K, (long)H * K, q_rstd + tok0 * H + h, H, valid, warp, lane);
+        l2norm_rows<K>(ks_p, kn + (tok0 * H + h) * K, (long)H * K, k_rstd + tok0 * H + h, H, valid, warp, lane);
         __syncthreads();
-        store_tile<64, K, LB_THREADS>(qs_p, qn + (tok0 * H + h) * K, (long)H * K, valid, tid);
-        store_tile<64, K, LB_THREADS>(ks_p, kn + (tok0 * H + h) * K, (long)H * K, valid, tid);
     }
     // ---- P = tril(qn kn^T Gam)
     const int rw = warp & 3, half = warp >> 2;
@@ -138,7 +126,8 @@ linear_bwd_pre_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* 
     {
         float acc[4][4];
         zero_acc(acc);
-        warp_gemm<K * 2, A_ROW, K * 2, B_NK, K, 4>(acc, qs, r0, ks, 32 * half, lane);
+        if (r0 + 15 >= 32 * half)                            // else above the diagonal
+            warp_gemm<K * 2, A_ROW, K * 2, B_NK, K, 4>(acc, qs, r0, ks, 32 * half, lane);
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
@@ -147,7 +136,9 @@ linear_bwd_pre_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* 
                 const int j = 32 * half + nt * 8 + qd * 2 + (e & 1);
                 acc[nt][e] = (j <= i && i < valid) ? acc[nt][e] * __expf(s_g[i] - s_g[j]) : 0.f;
             }
-        store_acc_bf16<128, 4>(ps_p, acc, r0, 32 * half, lane);
+        __syncthreads();                                     // every warp has read q
+        store_acc_bf16<128, 4>(qs_p, acc, r0, 32 * half, lane);
+        cp_async_wait<0>();
     }
     __syncthreads();
     // ---- dv'_loc = s P^T do
@@ -155,16 +146,13 @@ linear_bwd_pre_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* 
         constexpr int NT8 = V / 16;
         float acc[NT8][4];
         zero_acc(acc);
-        warp_gemm<128, A_TRANS, V * 2, B_KN, 64, NT8>(acc, ps, r0, dos, half * (V / 2), lane);
+        warp_gemm<128, A_TRANS, V * 2, B_KN, 64, NT8>(acc, qs, r0, dos, half * (V / 2), lane);
 #pragma unroll
         for (int nt = 0; nt < NT8; ++nt)
 #pragma unroll
             for (int e = 0; e < 4; ++e) acc[nt][e] *= scale;
-        __syncthreads();                                   // every warp has read do
-        store_acc_bf16<V * 2, NT8>(dos_p, acc, r0, half * (V / 2), lane);
+        store_acc_global<NT8>(dvl + (tok0 * H + h) * V, (long)H * V, acc, r0, half * (V / 2), valid, lane);
     }
-    __syncthreads();
-    store_tile<64, V, LB_THREADS>(dos_p, dvl + (tok0 * H + h) * V, (long)H * V, valid, tid);
 }
 
 // ================================================================================================ dh (reverse walk)
