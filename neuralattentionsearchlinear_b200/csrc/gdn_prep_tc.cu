@@ -19,15 +19,19 @@
 //      columns (the columns of an inverse are independent of one another) with tf32 mma.sync products, fp32
 //      accumulation; Ai diag(beta) and Ai diag(beta rstd e^{gcs}) are written as two bf16 operand tiles, so the
 //      right-hand sides never have to be scaled in shared memory (D = 64 has room for the first one only: the rows of k are
-//      scaled by rstd e^{gcs} while the diagonal blocks are inverted);
+//      scaled by rstd e^{gcs} while the diagonal blocks are inverted, and the tile leaves the unit diagonal out);
 //   4. D2 = [v^T (Ai diag beta)^T | k^T (Ai diag(..))^T]: the raw v and k tiles are the (MN-major) A operands,
-//      features in the TMEM lanes, tokens in the columns: no accumulator row is wasted (D = 64: both in one product);
+//      features in the TMEM lanes, tokens in the columns: no accumulator row is wasted (D = 64: both in one product, and the
+//      diagonal's share, beta v and beta rstd e^{gcs} k of the raw tiles, is added in fp32: it makes up most of u and w, and as part
+//      of the product it would be rounded with both operands before the result is, w's error 1.66e-3 -> 2.3e-3 with a bf16 beta and
+//      2.8e-3 with an fp32 one; on mma.sync it was 1.9e-3);
 //   5. w, then u, go from TMEM through a [token][feature] staging tile (transposed by stmatrix) to global memory with TMA
 //      stores; P leaves the same way.
 // Chains of short phases: what counts is the instructions of a chunk and how many chunks an SM has in flight.  L2 flushed:
 // 8 x 4096 tokens, 16 heads, D = 128: 180 us one element at a time and one feature per store, 152 us with the entries of A and P
 // in pairs, stmatrix and two diagonal blocks per warp (same bits; traffic 113 us); 16 x 4096 tokens, 16 heads, D = 64: 355 us on
-// mma.sync (shared memory 75 % busy), 208 us here (traffic 126 us).
+// mma.sync (shared memory 75 % busy), 226 us here (traffic 126 us; 208 us with the diagonal in the product; with k's scaled rows in
+// a tile of their own instead of a second load of k, five CTAs per SM, 240 us).
 // The decay carried over skipped blocks multiplies w by one scalar per chunk and is applied by the consumers.
 // Every mbarrier wait is bounded: on expiry the status word is set and the CTA runs on to its teardown.
 #include "tc_common.cuh"
@@ -49,6 +53,7 @@ struct PtSmem {
     // needed by the last product only, and this is what lets four CTAs (D = 64: six) share an SM
     static constexpr int As = SUB * 16384;
     static constexpr int v = As;
+    static constexpr int kraw = As + 8192;                   // D = 64: k as it came, beside v
     static constexpr int scr = As + 64 * PT_A_LD * 4;        // per warp [16][8] fp32: accumulator -> B-fragment exchange
     static constexpr int vec = scr + 4 * 512;                // gcs, beta, k rstd, w scale, q rstd: 5 x 64 floats
     static constexpr int bars = vec + 5 * 64 * 4;
@@ -57,7 +62,7 @@ struct PtSmem {
     static constexpr int pst = kq + 8192;                    // P staging [64][64] bf16
     static constexpr int ctas = D == 64 ? 6 : 4;             // per SM
     static constexpr uint32_t tmem = 64 * SUB;               // columns: with D = 64 the last product lies over the first
-    static_assert(As % 1024 == 0 && 64 * PT_A_LD * 4 >= 8192 * SUB, "the v tile must fit over A, 1024-byte aligned");
+    static_assert(As % 1024 == 0 && 64 * PT_A_LD * 4 >= 16384, "v (D = 64: v and k) must fit over A, 1024-byte aligned");
     static_assert(ctas * (total + 1024) <= 233472 && ctas * tmem <= 512, "CTAs per SM");
 };
 
@@ -101,7 +106,8 @@ __device__ __forceinline__ void acc_to_b(float* scr, const float (&c)[4], int la
 }
 
 // One panel of eight columns [c0, c0+8) of Ai (c0 = 16 j + 8 half), by one warp: zero above block row j, X_jj's half,
-// then block rows j+1..3 by the recursion; every 16 x 8 block is written, scaled per column, into the operand tile or tiles.
+// then block rows j+1..3 by the recursion; every 16 x 8 block is written, scaled per column, into the operand tiles, or (one tile)
+// without the unit diagonal, whose products are added up in fp32 at the end.
 template <bool TWO>
 __device__ __forceinline__ void inverse_panel(const float* As, float* scr, unsigned char* aiu, unsigned char* aiw,
                                               const float* s_beta, const float* s_wsc, int j, int half, int lane) {
@@ -116,8 +122,11 @@ __device__ __forceinline__ void inverse_panel(const float* As, float* scr, unsig
     }
     auto put = [&](int blk, const float (&y)[4]) {
         const int ra = 16 * blk + g, rb = ra + 8;
-        *reinterpret_cast<uint32_t*>(aiu + swz<128>(ra, chunk) + q * 4) = pack_bf16(y[0] * bu0, y[1] * bu1);
-        *reinterpret_cast<uint32_t*>(aiu + swz<128>(rb, chunk) + q * 4) = pack_bf16(y[2] * bu0, y[3] * bu1);
+        const bool unit = !TWO;
+        *reinterpret_cast<uint32_t*>(aiu + swz<128>(ra, chunk) + q * 4) =
+            pack_bf16(unit && ra == ca ? 0.f : y[0] * bu0, unit && ra == ca + 1 ? 0.f : y[1] * bu1);
+        *reinterpret_cast<uint32_t*>(aiu + swz<128>(rb, chunk) + q * 4) =
+            pack_bf16(unit && rb == ca ? 0.f : y[2] * bu0, unit && rb == ca + 1 ? 0.f : y[3] * bu1);
         if (TWO) {
             *reinterpret_cast<uint32_t*>(aiw + swz<128>(ra, chunk) + q * 4) = pack_bf16(y[0] * bw0, y[1] * bw1);
             *reinterpret_cast<uint32_t*>(aiw + swz<128>(rb, chunk) + q * 4) = pack_bf16(y[2] * bw0, y[3] * bw1);
@@ -267,9 +276,10 @@ gdn_prep_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         constexpr uint32_t id_2 = umma_idesc_bf16(128, 64, false) | (1u << 15);      // A MN-major (features x tokens)
         // every thread has finished with A (and fenced): the v tile may land on it
         if (lane == 0) {
-            mbar_expect_tx(bar_v, 8192 * SUB);
+            mbar_expect_tx(bar_v, 16384);
 #pragma unroll
             for (int sub = 0; sub < SUB; ++sub) tma_load_4d(sbase + L::v + sub * 8192, &map_v, sub * 64, h, t0, b, bar_v);
+            if (D == 64) tma_load_4d(sbase + L::kraw, &map_k, 0, h, t0, b, bar_v);      // (from L2: its tile here has been scaled)
         }
         __syncwarp();
         if constexpr (D == 128) {
@@ -428,7 +438,8 @@ gdn_prep_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
 #pragma unroll
             for (int i = 0; i < 16; ++i) As[(d0 + i) * PT_A_LD + d0 + cidx] = xcol[i];
         } else if constexpr (D == 64) {
-            // meanwhile: the rows of k, the operand of w, scaled by rstd e^{gcs} (beta comes with Ai)
+            // meanwhile: the rows of k, the operand of w, scaled by rstd e^{gcs} (beta comes with Ai); q's factors are done with
+            s_qr[row - 64] = s_beta[row - 64] * s_wsc[row - 64];
 #pragma unroll
             for (int rr = 0; rr < 8; ++rr) {
                 const int r = rr * 8 + (row - 64) / 8, cc = row % 8;
@@ -466,11 +477,14 @@ gdn_prep_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
 #pragma unroll 1
         for (int arr = D == 128 ? 0 : 1; arr < 2; ++arr) {     // 0: w, 1: u (D = 64: both)
             mbar_wait_small(arr == 0 ? bar_d2w : bar_d2u, 0, status);
+            if (D == 64) mbar_wait_small(bar_v, 0, status);
             tc_fence_after();
             const int sub = row >> 6;
             const uint32_t stg = sbase + (D == 64 ? (sub ? L::v : L::kq) : L::kq + sub * 16384 + (arr == 0 ? 0 : 8192));
             // this thread's row of the four matrices: token (lane & 7) of the lower or upper eight, features of its half
             const int tok = (lane & 7) + ((lane & 16) >> 1), half = (lane >> 3) & 1;
+            const float* s_unit = (sub ? s_beta : s_qr) + 2 * (lane & 3);
+            const uint32_t unit = sbase + (sub ? L::v : L::kraw) - stg;      // D = 64: from an output's place to its raw input's
 #pragma unroll 1
             for (int f = 0; f < 2; ++f) {                      // sixteen features
                 uint32_t r[32];
@@ -481,9 +495,18 @@ gdn_prep_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {                  // sixteen tokens
                     uint32_t p[4];
+                    if constexpr (D == 64) {                   // the inverse's diagonal: beta v, or beta rstd e^{gcs} k, in fp32
+                        ldsm_x4_t(at + unit + k * 16 * 128, p[0], p[1], p[2], p[3]);
 #pragma unroll
-                    for (int e = 0; e < 4; ++e)
-                        p[e] = pack_bf16(__uint_as_float(r[8 * k + 2 * e]), __uint_as_float(r[8 * k + 2 * e + 1]));
+                        for (int e = 0; e < 4; ++e) {
+                            const uint64_t s = *reinterpret_cast<const uint64_t*>(s_unit + 16 * k + 8 * (e >> 1));
+                            p[e] = close2(fma2(open2(p[e]), s, pack2(__uint_as_float(r[8 * k + 2 * e]), __uint_as_float(r[8 * k + 2 * e + 1]))));
+                        }
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+                            p[e] = pack_bf16(__uint_as_float(r[8 * k + 2 * e]), __uint_as_float(r[8 * k + 2 * e + 1]));
+                    }
                     stsm_x4_t(at + k * 16 * 128, p[0], p[1], p[2], p[3]);
                 }
             }

@@ -32,6 +32,31 @@ def test_prep64_against_the_formulas(B, T, H, with_q, beta_f32, l2):
         assert err < 2 ** -8, (NAMES[i], float(err))
 
 
+@pytest.mark.parametrize("beta_f32", [False, True])
+@pytest.mark.parametrize("T,decay", [(512, 4.0), (512, 1.0), (1000, 0.05), (512, 0.01)])
+def test_prep64_rounds_the_diagonal_once(T, decay, beta_f32):
+    """The inverse's diagonal is exactly one: its share of u and w, beta v and beta rstd e^gcs k, reaches the output with the
+    output's rounding alone, in bf16 as in fp32 beta.  What is off the diagonal takes two more (the inverse's entry, and k or v)."""
+    q, k, v, g, beta, _ = synth_gdn_inputs(1, T, 4, 64, 64, seed=T)
+    g = g * decay
+    if beta_f32:
+        beta = torch.rand(beta.shape, generator=torch.Generator().manual_seed(1))
+    ref = _reference(q, k, v, g, beta)
+    got = _run(PREP, q, k, v, g, beta, True)
+    n = -(-T // 64)
+    pad = lambda x: torch.nn.functional.pad(x.double(), (0, 0) * (x.dim() - 2) + (0, n * 64 - T))
+    ch = lambda x: pad(x).reshape(1, n, 64, 4, -1).transpose(2, 3)             # [B, chunk, head, token, feature]
+    kn, b, gc = ch(k) * ch(ref[1][..., None]), ch(beta[..., None]), ch(g[..., None]).cumsum(-2)
+    A = torch.tril(b * (kn @ kn.mT) * (gc - gc.mT).clamp(max=0).exp(), -1)
+    off = torch.linalg.inv(torch.eye(64, dtype=torch.float64) + A) - torch.eye(64, dtype=torch.float64)
+    for i, rhs in ((3, kn * b * gc.exp()), (4, ch(v) * b)):
+        one = (ref[i].bfloat16().double() - ref[i]).norm()                     # what storing the exact result loses
+        terms = (off.square() @ rhs.square()).sum() / ref[i].square().sum()    # errors of the products, of independent signs
+        err = (got[i].double().cpu() - ref[i]).norm()
+        # a tenth for the tf32 products of the inverse (2^-11 of an entry) and the spread of the estimate
+        assert err < 1.1 * one * (1 + 2 * terms) ** 0.5, (NAMES[i], float(err / one), float(terms))
+
+
 def test_prep64_strong_decay_and_large_beta():
     q, k, v, g, beta, _ = synth_gdn_inputs(1, 256, 2, 64, 64, seed=11)
     g, beta = g * 6.0, (beta.float() * 2.0).bfloat16()
