@@ -141,10 +141,10 @@ class NeuralAttentionSearchLinearAttnMamba(nn.Module):
     @property
     def attn_fraction(self) -> torch.Tensor:
         """Share of the blocks of the last forward that took the softmax branch, per selection head."""
-        if self.attn_blocks is not None:
-            counts, n = self.attn_blocks
-            self.attn_fraction = (counts[..., 0].float() / n).mean(0)
-        return self._attn_fraction
+        if self.attn_blocks is None:
+            return self._attn_fraction
+        counts, n = self.attn_blocks                         # (formed at every read: a graph's replay writes new counts)
+        return (counts[..., 0].float() / n).mean(0)
 
     @attn_fraction.setter
     def attn_fraction(self, value: torch.Tensor) -> None:
@@ -213,6 +213,8 @@ class NeuralAttentionSearchLinearAttnMamba(nn.Module):
         types[:, -1] = 1
         n_blocks = types.int().sum(1)
         self.attn_blocks = (n_blocks, types.shape[1])
+        if types.is_cuda and torch.cuda.is_current_stream_capturing():
+            self.attn_fraction = self.attn_fraction          # part of the graph, so that a tensor read once follows its replays
         p.update(types=types, types_raw=types_raw, n_blocks=n_blocks, op_type_last=op_type_last)
         return p
 

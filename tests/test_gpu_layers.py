@@ -154,3 +154,38 @@ def test_ops_replay_from_a_cuda_graph(rule):
         assert torch.equal(a, b)
     from neuralattentionsearchlinear_b200 import _lib
     assert _lib.load().natsl_device_status() == 0
+
+
+@pytest.mark.parametrize("train", [True, False])
+@pytest.mark.parametrize("rule", ["gdn", "mamba"])
+def test_attn_fraction_follows_the_replays_of_a_graph(rule, train):
+    """A forward captured in a graph runs no Python when it is replayed: every read after a replay is that replay's share, and in
+    training mode a tensor read once holds it too."""
+    import neuralattentionsearchlinear_b200 as nat
+    torch.manual_seed(2)
+    make, kw = ((nat.NeuralAttentionSearchLinearAttnGDN, dict(head_dim=64, expand_v=1)) if rule == "gdn" else
+                (nat.NeuralAttentionSearchLinearAttnMamba, dict(head_dim=128, expand_v=0.5)))
+    layer = make(hidden_size=128, num_heads=2, num_attn_heads=2, nats_block_size=64, layer_idx=0, **kw).cuda().bfloat16().train(train)
+    xs = [torch.randn(2, 256, 128, device="cuda").bfloat16() * s for s in (1.0, 30.0, -30.0)]
+    want = []
+    with torch.set_grad_enabled(train):
+        for x in xs:
+            layer(x)
+            want.append(layer.attn_fraction.clone())
+            assert torch.equal(layer.attn_fraction, want[-1])
+        x, side = xs[0].clone(), torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            for _ in range(2):
+                layer(x)
+        torch.cuda.current_stream().wait_stream(side)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            layer(x)
+    held = layer.attn_fraction
+    for n in (0, 1, 2, 1):
+        x.copy_(xs[n])
+        graph.replay()
+        assert torch.equal(layer.attn_fraction, want[n]) and torch.equal(layer.attn_fraction, want[n])
+        assert not train or torch.equal(held, want[n])
+    assert not torch.equal(want[1], want[2])

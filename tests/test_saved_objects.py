@@ -34,3 +34,5 @@ def test_layer_saved_with_plain_attributes(cls):
     layer.attn_blocks = (torch.tensor([[[1, 2]]]), 4)
     assert float(copy.deepcopy(layer).attn_fraction) == 0.25
     assert float(layer.attn_fraction) == 0.25
+    layer.attn_blocks[0].mul_(2)                             # what a graph's replay does to the counts
+    assert float(layer.attn_fraction) == 0.5
