@@ -42,14 +42,19 @@ last_kv_capacity = None          # (blocks per head, pairs) the last call withou
 class CudaSegmentOps:
     """Compute steps of one rank, on the CUDA kernels of this package."""
 
-    def side_stream(self, device):
+    def side_stream(self, device, high: bool = False):
+        """The stream of the linear branch; ``high``: of high priority, unless NATSL_LINEAR_PRIORITY=0.
+
+        The branch is the chain: of high priority it gets its SMs while the softmax branch, which keeps every SM busy for most of
+        the call, works through its blocks.  One GPU, blocks of 256, a tenth of them selected, normal -> high (medians of twelve
+        rounds in turn): 16384 tokens, 32 heads 555 -> 532 us; 32768, 16 heads 728 -> 704; 32768, 32 heads 1334 -> 1312; 65536,
+        32 heads 4.06 -> 4.00 ms (within the spread of its rounds); up to 16384 tokens of 16 heads no difference, no length slower.
+        Over several ranks nothing is measured: normal there."""
+        high = high and _ops.LINEAR_BRANCH_PRIORITY
         idx = device.index if device.index is not None else torch.cuda.current_device()
-        if idx not in _side_streams:
-            # the linear branch is the chain: of high priority it gets its SMs while the softmax branch, which keeps every SM
-            # busy for most of the call, works through its blocks.  On one GPU, normal -> high priority: 16384 tokens, 32 heads
-            # 527 -> 473 us; 8192, 16 heads 349 -> 330; 32768, 16 heads 638 -> 611; 65536, 32 heads 3.51 -> 3.58 ms (power limit)
-            _side_streams[idx] = torch.cuda.Stream(device=idx, priority=-1)
-        return _side_streams[idx]
+        if (idx, high) not in _side_streams:
+            _side_streams[idx, high] = torch.cuda.Stream(device=idx, priority=-1 if high else 0)
+        return _side_streams[idx, high]
 
     def tables(self, types, T, nbs):
         return build_selection_tables(types, T, nbs)
@@ -245,7 +250,9 @@ def nats_mixed_attn_mamba_sp(q_attn, k_attn, v_attn, q_lattn, k_lattn, v_lattn, 
         y = x_all.reshape(world * n_seg, B, *x_all.shape[2:])
         return y if layout == 'contiguous' else y[order].contiguous()
 
-    side = be.side_stream(dev) if hasattr(be, 'side_stream') else None
+    side = None
+    if hasattr(be, 'side_stream'):
+        side = be.side_stream(dev, high=True) if world == 1 and type(be) is CudaSegmentOps else be.side_stream(dev)
     cur = torch.cuda.current_stream(dev) if side is not None else None
     on_side = (lambda: torch.cuda.stream(side)) if side is not None else contextlib.nullcontext
     made_on_side = []

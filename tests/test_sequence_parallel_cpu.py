@@ -129,6 +129,17 @@ def test_pick_linear_splits():
     assert pick_linear_splits(2048, 64, target_tokens=512) == 4
 
 
+def test_priority_of_the_linear_branch(monkeypatch):
+    """High on one rank only, and not where NATSL_LINEAR_PRIORITY=0 has been set."""
+    from neuralattentionsearchlinear_b200 import _ops, sequence_parallel as sp
+    monkeypatch.setattr(torch.cuda, "Stream", lambda device, priority: (device, priority))
+    monkeypatch.setattr(sp, "_side_streams", {})
+    ops, dev = sp.CudaSegmentOps(), torch.device("cuda", 3)
+    assert ops.side_stream(dev) == (3, 0) and ops.side_stream(dev, high=True) == (3, -1)
+    monkeypatch.setattr(_ops, "LINEAR_BRANCH_PRIORITY", False)
+    assert ops.side_stream(dev) == (3, 0) and ops.side_stream(dev, high=True) == (3, 0)
+
+
 def test_single_rank_sub_segment_split_matches_oracle():
     """One process, no process group: only the sub-segment split of the linear branch is exercised."""
     from neuralattentionsearchlinear_b200.sequence_parallel import nats_mixed_attn_mamba_sp
