@@ -158,8 +158,27 @@ class _GatesFn(torch.autograd.Function):
         return g, beta, vo
 
     @staticmethod
-    @torch.autograd.function.once_differentiable
+    def in_torch(ctx, dg, dbeta, dvo):
+        """The gradients as torch operations, which have derivatives of their own."""
+        a, b, v, A_log, dt_bias = ctx.saved_tensors
+        z, A = a.float() + dt_bias, A_log.float().exp()
+        dt = F.softplus(z)
+        heads = lambda x: x.sum(tuple(range(x.dim() - 1)))
+        ddt, dA, db, dv = torch.zeros_like(z), torch.zeros_like(A_log), None, None
+        if dg is not None:
+            ddt, dA = ddt - A * dg, heads(-A * dt * dg).to(A_log.dtype)
+        if dvo is not None:
+            ddt, dv = ddt + (dvo.float() * v.float()).sum(-1), (dvo.float() * dt.unsqueeze(-1)).to(v.dtype)
+        if b is not None:
+            y = b.sigmoid().float()
+            db = torch.zeros_like(b) if dbeta is None else (dbeta.float() * ((2. if ctx.neg else 1.) * (1. - y) * y)).to(b.dtype)
+        dz = ddt * torch.where(z > 20., torch.ones_like(z), z.sigmoid())
+        return dz.to(a.dtype), db, dv, dA, heads(dz).to(dt_bias.dtype), None
+
+    @staticmethod
     def backward(ctx, dg, dbeta, dvo):
+        if torch.is_grad_enabled():                          # a graph of the gradient is asked for
+            return _GatesFn.in_torch(ctx, dg, dbeta, dvo)
         a, b, v, A_log, dt_bias = ctx.saved_tensors
         H = a.shape[-1]
         rows = a.numel() // H

@@ -71,6 +71,31 @@ def test_gates_with_a_gradient_missing_and_where_torch_runs():
     assert layer_gates(a, A, bias, v=v[..., :24]) is None and layer_gates(a, torch.zeros(3, device="cuda"), bias) is None
 
 
+@pytest.mark.parametrize("with_b,neg,V", [(True, True, None), (True, False, 64), (False, False, 64)])
+def test_gates_second_derivatives(with_b, neg, V):
+    """Differentiable gradients (``create_graph``): first and second derivatives of a scalar of the three outputs, against float64."""
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    rnd = lambda *s, dt=BF: torch.randn(*s, generator=gen, device="cuda").to(dt).requires_grad_(True)
+    a, b, v = rnd(2, 70, 4), rnd(2, 70, 4) if with_b else None, None if V is None else rnd(2, 70, 4, V)
+    with torch.no_grad():
+        a.view(-1)[0] = 30.0
+    ins = (a, b, v, rnd(4, dt=torch.float32), rnd(4, dt=torch.float32))
+    refs = tuple(None if t is None else t.detach().double().requires_grad_(True) for t in ins)
+
+    def derivatives(run, ins):
+        some = [t for t in ins if t is not None]
+        out = [x for x in run(*ins) if x is not None]
+        first = torch.autograd.grad(sum(x.to(torch.float64).square().sum() for x in out), some, create_graph=True)
+        return first, torch.autograd.grad(sum(x.to(torch.float64).square().sum() for x in first), some)
+
+    got = derivatives(lambda a, b, v, A, bias: layer_gates(a, A, bias, b=b, v=v, neg_eigval=neg), ins)
+    want = derivatives(lambda a, b, v, A, bias: _reference(a, b, v, A, bias, neg), refs)
+    for order, g, w in ((1, got[0], want[0]), (2, got[1], want[1])):
+        for x, y in zip(g, w):
+            # every bf16 tensor on the way (outputs, gradients, their gradients: five at most) is rounded once, 2^-9 each
+            assert (x.double() - y).norm() <= 5 * 2 ** -9 * order * y.norm(), (order, x.shape)
+
+
 @pytest.mark.parametrize("shape", [(1, 64), (7, 5, 128), (3, 41, 2, 256)])
 def test_l2norm(shape):
     x = torch.randn(*shape, device="cuda").to(BF).requires_grad_(True)
