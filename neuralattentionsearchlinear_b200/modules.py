@@ -41,6 +41,13 @@ def _column_sums(part: torch.Tensor, mode: int, out0: torch.Tensor, out1: Option
               current_stream_ptr(part.device))
 
 
+def _plain(*grads) -> bool:
+    """Whether a backward pass may run its kernel: no graph of the gradient is asked for, and the gradients are tensors with memory of
+    their own (``is_grads_batched`` and ``jacobian(vectorize=True)`` hand in batched ones, which no query of the transforms names)."""
+    return (not torch.is_grad_enabled() and not transforms_active()
+            and all(g is None or torch._C._has_storage(g) for g in grads))
+
+
 class _RMSNormFn(torch.autograd.Function):
     """``natsl_rmsnorm_fwd`` / ``natsl_rmsnorm_bwd`` on [rows, D] bf16: (y, s) with s = x (+ residual)."""
 
@@ -118,8 +125,10 @@ class _L2NormFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x, = ctx.saved_tensors
-        if torch.is_grad_enabled():                          # a graph of the gradient is asked for: the same in torch operations
-            return torch.autograd.grad(_l2norm(x, ctx.eps), x, dy, create_graph=True)[0], None
+        if not _plain(dy):                                   # the same in torch operations
+            xf, d = x.float(), dy.float()
+            r = torch.rsqrt(xf.pow(2).sum(-1, keepdim=True) + ctx.eps)
+            return (r * d - xf * (r.pow(3) * (d * xf).sum(-1, keepdim=True))).to(x.dtype), None
         dy = dy.contiguous()
         dx = torch.empty_like(x)
         _lib.call("natsl_l2norm_bwd", x.data_ptr(), dy.data_ptr(), dx.data_ptr(), x.shape[0], x.shape[1], ctx.eps, current_stream_ptr(x.device))
@@ -177,7 +186,7 @@ class _GatesFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dg, dbeta, dvo):
-        if torch.is_grad_enabled():                          # a graph of the gradient is asked for
+        if not _plain(dg, dbeta, dvo):
             return _GatesFn.in_torch(ctx, dg, dbeta, dvo)
         a, b, v, A_log, dt_bias = ctx.saved_tensors
         H = a.shape[-1]
@@ -307,7 +316,7 @@ class _BlockMeanFn(torch.autograd.Function):
     def backward(ctx, dy):
         T, nbs = ctx.T, ctx.nbs
         NB = dy.shape[1]
-        if _kernel_ok(dy) and not torch.is_grad_enabled():
+        if _kernel_ok(dy) and _plain(dy):
             B, _, D = dy.shape
             dy = dy.contiguous()
             dx = torch.empty(B, T, D, dtype=dy.dtype, device=dy.device)

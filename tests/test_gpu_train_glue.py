@@ -96,6 +96,20 @@ def test_gates_second_derivatives(with_b, neg, V):
             assert (x.double() - y).norm() <= 5 * 2 ** -9 * order * y.norm(), (order, x.shape)
 
 
+@pytest.mark.parametrize("what", ["l2norm", "block mean", "gates"])
+def test_batched_gradients(what):
+    """``is_grads_batched`` and ``vmap`` over a backward pass: the rows of one gradient at a time."""
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.randn(2, 70, 4 if what == "gates" else 64, generator=gen, device="cuda").to(BF).requires_grad_(True)
+    A = torch.randn(4, generator=gen, device="cuda")
+    y = L2Norm()(x) if what == "l2norm" else _BlockMeanFn.apply(x, 64) if what == "block mean" else layer_gates(x, A, A)[0]
+    dys = torch.randn(3, *y.shape, generator=gen, device="cuda").to(y.dtype)
+    one = lambda dy: torch.autograd.grad(y, x, dy, retain_graph=True)[0]
+    want = torch.stack([one(dy) for dy in dys])
+    for got in (torch.autograd.grad(y, x, dys, retain_graph=True, is_grads_batched=True)[0], torch.vmap(one)(dys)):
+        _close(got, want, 64)
+
+
 @pytest.mark.parametrize("shape", [(1, 64), (7, 5, 128), (3, 41, 2, 256)])
 def test_l2norm(shape):
     x = torch.randn(*shape, device="cuda").to(BF).requires_grad_(True)
