@@ -26,6 +26,12 @@ def _kernel_ok(x: torch.Tensor) -> bool:
     return x.is_cuda and x.dtype == torch.bfloat16
 
 
+def _eager(*tensors) -> bool:
+    """Whether nothing (a transform, a trace, a compiler, a subclass of tensors without memory) has to see torch operations."""
+    return (not transforms_active() and not torch.compiler.is_compiling()
+            and all(t is None or type(t) in (torch.Tensor, nn.Parameter) for t in tensors))
+
+
 def _n_part(rows: int) -> int:
     """CTAs of the norms' backward kernels, each with one partial sum of the weight gradients: four per SM."""
     return int(min(-(-rows // 8), 592))
@@ -145,7 +151,7 @@ class L2Norm(nn.Module):
 
     def forward(self, x):
         D = x.shape[-1]
-        if _kernel_ok(x) and D in (64, 128, 256) and x.numel() and not transforms_active():
+        if _kernel_ok(x) and D in (64, 128, 256) and x.numel() and _eager(x):
             return _L2NormFn.apply(aligned(x.contiguous()).view(-1, D), float(self.eps)).view(x.shape)
         return _l2norm(x, self.eps)
 
@@ -210,7 +216,7 @@ def layer_gates(a, A_log, dt_bias, b=None, v=None, neg_eigval: bool = False):
     H = a.shape[-1]
     if not (_kernel_ok(a) and 0 < H <= 256 and a.numel() and A_log.numel() == H == dt_bias.numel() and A_log.dtype in _SUM_DTYPES
             and dt_bias.dtype in _SUM_DTYPES and A_log.is_contiguous() and dt_bias.is_contiguous() and A_log.device == a.device == dt_bias.device
-            and not transforms_active()):
+            and _eager(a, b, v, A_log, dt_bias)):
         return None
     if b is not None and not (_kernel_ok(b) and b.shape == a.shape and b.device == a.device):
         return None

@@ -129,6 +129,17 @@ def test_l2norm(shape):
     assert torch.isfinite(tangent).all()
 
 
+def test_l2norm_and_gates_in_one_compiled_graph():
+    x, A = torch.randn(2, 70, 64, device="cuda").to(BF), torch.randn(64, device="cuda")
+
+    def run(x):
+        gates = layer_gates(x, A, A)
+        return L2Norm()(x), gates[0] if gates is not None else _reference(x.float(), None, None, A, A, False)[0]
+
+    for got, want in zip(torch.compile(run, backend="eager", fullgraph=True)(x), run(x)):
+        _close(got, want, 4)
+
+
 @pytest.mark.parametrize("P,N,mode", [(1, 2, 1), (592, 2048, 0), (131, 33 * 5, 4), (40, 10, 4), (97, 256, 1)])
 @pytest.mark.parametrize("dtypes", [(BF, torch.float32), (torch.float32, BF)])
 def test_column_sums(P, N, mode, dtypes):
