@@ -353,7 +353,11 @@ struct StSmem {
     static constexpr int dos = ws + cmax((GDN ? KB + VB : 0), SB);       // do, then k
     static constexpr int vec = dos + cmax(VB, KB);            // g[64], r[64], red[8 warps][2] + red2[2]
     static constexpr int total = vec + (64 + 64 + 32) * 4;
-    static constexpr int ctas = 3 * (total + 1024) <= 233472 ? 3 : 2;    // per SM, for the register budget
+    // CTAs per SM, for the register budget: three where the shared memory has room, but not with two strips of K / 2 features in
+    // registers (128 / 64 with the delta rule spilled 96 bytes).  Two against three, us at B x T x heads 8 x 4096 x 16, 4 x 1000 x 16,
+    // 1 x 500 x 4: delta rule 64 / 64 186, 26.3, 5.1 -> 155, 23.3, 5.2; Mamba2 128 / 64 190, 27.9, 5.3 -> 163, 26.7, 5.3; delta rule
+    // 128 / 64 257, 39.4, 6.7 -> 256, 40.9, 7.5.
+    static constexpr int ctas = 3 * (total + 1024) <= 233472 && !(GDN && K == 128) ? 3 : 2;
     static_assert(2 * (total + 1024) <= 233472, "two CTAs per SM");
 };
 
