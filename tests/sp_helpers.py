@@ -126,3 +126,11 @@ class OracleSegmentOps:
 
     def n_attn_blocks(self, tables):
         return tables.n_blocks[..., 0].to(torch.int32).contiguous()
+
+
+class FoldingSegmentOps(OracleSegmentOps):
+    """The same with a fold that takes the factors of the states' last blocks along, as the CUDA backend's does."""
+    folds_trail = True
+
+    def prefix_states(self, a, S, h0, want_prefix, trail):
+        return super().prefix_states(a, S * trail[..., None, None], h0, want_prefix)

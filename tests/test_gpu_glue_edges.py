@@ -116,3 +116,41 @@ def test_block_mean_adds_tokens_in_their_order(B, T, D, nbs):
             acc = acc + rows[:, t]
         inv = (torch.ones((), device="cuda") / rows.shape[1])
         assert torch.equal(y[:, c], (acc * inv).to(BF))
+
+
+@pytest.mark.parametrize("act", [0, 1])
+def test_sigmoid_of_pairs_in_fp32(act):
+    """The mixing weights' gradient is a sum over a row in fp32: with one feature that is not zero it is the gate's function itself, for
+    every bf16 gate up to 80.  ``__expf`` is off by 2 + 1.173 |x| units of 2^-23 at most, the reciprocal with its step of Newton's
+    iteration by one, the sum in front of it and the products by half a one each."""
+    bits = torch.arange(65536, dtype=torch.int32, device="cuda").to(torch.uint16).view(BF)
+    gate = bits[(bits.float().abs() <= 80) & ((bits.float().abs() >= 2 ** -60) | (bits == 0))]
+    rows, D, j = gate.numel(), 64, 21
+    one = torch.zeros(rows, D, dtype=BF, device="cuda")
+    one[:, j] = 1
+    gt = one * gate[:, None]
+    xw = torch.ones(rows, 2, device="cuda")
+    n_part = min(-(-rows // 8), 592)
+    outs = [torch.empty(rows, D, dtype=BF, device="cuda") for _ in range(3)]
+    dxw, part = torch.empty(rows, 2, device="cuda"), torch.empty(n_part, 2, D, device="cuda")
+    _lib.call("natsl_norm_gate_mix_bwd", one.data_ptr(), one.data_ptr(), gt.data_ptr(), xw.data_ptr(), _lib.DT_F32, None, None, 0, one.data_ptr(),
+              *(o.data_ptr() for o in outs), dxw.data_ptr(), part.data_ptr(), n_part, rows, D, 0.0, act, _st())
+    x = gate.double()
+    want = 8.0 * x.sigmoid() * (1.0 if act else x)            # x / sqrt(mean(x^2)) = 8, up to the two units of rsqrtf
+    for got in dxw.double().unbind(1):
+        assert bool(((got - want).abs() <= 2 ** -23 * (7 + 1.173 * x.abs()) * want.abs()).all())
+
+
+@pytest.mark.parametrize("B,T,D,span", [(2, 131, 72, 32), (1, 300, 136, 100), (2, 64, 8, 7)])
+def test_short_conv_bwd_over_other_spans(B, T, D, span):
+    """Spans of other than 64 tokens per partial sum (a kernel of their own) give the same gradients."""
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x, dy, w, bias = _rand(g, B, T, D), _rand(g, B, T, D), _rand(g, D, 4), _rand(g, D)
+    got = []
+    for s in (64, span):
+        dx, part = torch.empty_like(x), torch.full((B * -(-T // s), D, 5), float("nan"), device="cuda")
+        _lib.call("natsl_short_conv_bwd", x.data_ptr(), w.data_ptr(), bias.data_ptr(), dy.data_ptr(), dx.data_ptr(), part.data_ptr(), B, T, D, 4,
+                  1, s, _st())
+        got.append((dx, part.sum(0)))
+    _close(got[1][0], got[0][0])
+    _close(got[1][1], got[0][1], fp32=True)

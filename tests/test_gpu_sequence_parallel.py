@@ -199,3 +199,30 @@ def test_pack_pairs_capacity_overflow_sets_status():
     be.pack_pairs(x, tb, 16, 4)                                      # more blocks per head than announced
     assert _lib.load().natsl_device_status() == 3
     assert _lib.load().natsl_device_status() == 0                    # reading clears it
+
+
+@pytest.mark.parametrize("N,with_h0", [(1, False), (5, True)])
+def test_prefix_states_with_and_without_factors(N, with_h0):
+    """The fold with a factor per state against float64; with factors of one it is the fold without them, bit for bit."""
+    from neuralattentionsearchlinear_b200 import _lib
+    B, H, K, V = 2, 3, 16, 24
+    gen = torch.Generator(device="cuda").manual_seed(N)
+    rnd = lambda *s: torch.rand(*s, generator=gen, device="cuda")
+    a, S, trail, h0 = rnd(N, B, H), rnd(N, B, H, K, V) - 0.5, rnd(N, B, H), rnd(B, H, K, V) if with_h0 else None
+
+    def fold(name, *trail):
+        out = torch.empty_like(S), torch.empty(B, H, K, V, device="cuda"), torch.empty(B, H, device="cuda")
+        _lib.call(name, a.data_ptr(), S.data_ptr(), *(_lib.ptr(t) for t in trail), _lib.ptr(h0), *(o.data_ptr() for o in out), N, B, H, K, V,
+                  torch.cuda.current_stream().cuda_stream)
+        return out
+
+    plain = fold("natsl_sp_prefix_states")
+    for other in (fold("natsl_sp_prefix_states_scaled", None), fold("natsl_sp_prefix_states_scaled", torch.ones_like(trail))):
+        assert all(torch.equal(x, y) for x, y in zip(plain, other))
+    got, p, f = fold("natsl_sp_prefix_states_scaled", trail), torch.zeros(B, H, K, V, dtype=torch.float64, device="cuda"), 1.0
+    p = p if h0 is None else h0.double()
+    wide = lambda x: x.double()[..., None, None]
+    for n in range(N):
+        assert (got[0][n].double() - p).abs().max() < 2 ** -22 * (n + 1)       # three roundings of values below one and a half each turn
+        p, f = wide(a[n]) * p + wide(trail[n]) * S[n].double(), f * a[n].double()
+    assert (got[1].double() - p).abs().max() < 2 ** -22 * (N + 1) and torch.allclose(got[2].double(), f, rtol=2 ** -22 * N)

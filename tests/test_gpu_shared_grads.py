@@ -35,3 +35,32 @@ def test_shared_inputs_get_the_sum_of_both_gradients(rule, B, T, H, K, V, which)
             assert one_l is one_a and torch.equal(one_l, l + a), n
         else:
             assert torch.equal(one_l, l) and torch.equal(one_a, a), n
+
+
+@pytest.mark.parametrize("rule,K,V", [("gdn", 64, 64), ("mamba", 128, 64)])
+def test_entry_point_that_adds_nothing(rule, K, V, monkeypatch):
+    """``natsl_linear_bwd_intra`` is ``natsl_linear_bwd_intra_onto`` with nothing to add to."""
+    import neuralattentionsearchlinear_b200 as nat
+    from neuralattentionsearchlinear_b200 import _lib
+    gen, call, names = torch.Generator().manual_seed(5), _lib.call, []
+    rnd = lambda *s: torch.randn(*s, generator=gen).cuda()
+    base, attn = ([rnd(1, 200, 2, d).bfloat16() for d in (K, K, V)] for _ in range(2))
+    g, beta = -torch.nn.functional.softplus(rnd(1, 200, 2)), rnd(1, 200, 2).sigmoid().bfloat16()
+    types, do = (rnd(1, 4, 2, 2) > 0).float(), rnd(1, 200, 2, V).bfloat16()
+
+    def other(name, *args):
+        if name == "natsl_linear_bwd_intra_onto":
+            assert args[-2] == 0
+            names.append(name)
+            return call("natsl_linear_bwd_intra", *args[:-2], args[-1])
+        return call(name, *args)
+
+    got = []
+    for route in (call, other):
+        monkeypatch.setattr(_lib, "call", route)
+        lin = [t.clone().requires_grad_() for t in base]
+        op = nat.nats_mixed_attn_gdn if rule == "gdn" else nat.nats_mixed_attn_mamba
+        out = op(*attn, *lin, None, g, *((beta,) if rule == "gdn" else ()), types, None, nats_block_size=64, ops_for_incomplete_chunks="all")
+        out[0].backward(do)
+        got.append([t.grad for t in lin])
+    assert names and all(torch.equal(a, b) for a, b in zip(*got))

@@ -31,12 +31,12 @@ def _inputs(B, T, H, K, V, nbs, seed):
     return q, k, v, g, types
 
 
-def _worker(rank, world, port, B, T, H, K, V, nbs, decay, seed, ret, layout="contiguous", splits=None):
+def _worker(rank, world, port, B, T, H, K, V, nbs, decay, seed, ret, layout="contiguous", splits=None, folds=False):
     os.environ["MASTER_ADDR"], os.environ["MASTER_PORT"] = "127.0.0.1", str(port)
     dist.init_process_group("gloo", rank=rank, world_size=world)
     try:
         from neuralattentionsearchlinear_b200.sequence_parallel import nats_mixed_attn_mamba_sp
-        from tests.sp_helpers import OracleSegmentOps
+        from tests.sp_helpers import FoldingSegmentOps, OracleSegmentOps
         q, k, v, g, types = _inputs(B, T, H, K, V, nbs, seed)
         TN = types.shape[1]
         if layout == "contiguous":
@@ -53,20 +53,21 @@ def _worker(rank, world, port, B, T, H, K, V, nbs, decay, seed, ret, layout="con
         c = lambda x: x[:, tsel].contiguous()
         o_l, o_a, ht = nats_mixed_attn_mamba_sp(c(q), c(k), c(v), c(q), c(k), c(v), c(g), types[:, bsel].contiguous(),
                                                 nats_block_size=nbs, decay_for_non_mamba_blocks=decay, layout=layout,
-                                                linear_splits=splits, backend=OracleSegmentOps())
+                                                linear_splits=splits,
+                                                backend=FoldingSegmentOps() if folds else OracleSegmentOps())
         ret[rank] = (o_l, o_a, ht, tsel)
     finally:
         dist.destroy_process_group()
 
 
-@pytest.mark.parametrize("world,T,nbs,decay,splits", [(2, 1024, 128, True, None), (3, 1100, 128, True, None),
-                                                      (2, 768, 256, False, None), (2, 1024, 128, True, 2),
-                                                      (2, 1024, 256, False, 2)])
-def test_sp_matches_single_process_oracle(world, T, nbs, decay, splits):
+@pytest.mark.parametrize("world,T,nbs,decay,splits,folds", [
+    (2, 1024, 128, True, None, False), (3, 1100, 128, True, None, False), (2, 768, 256, False, None, False), (2, 1024, 128, True, 2, False),
+    (2, 1024, 256, False, 2, False), (2, 1024, 128, True, 2, True), (2, 1024, 256, False, 2, True), (2, 768, 256, True, None, True)])
+def test_sp_matches_single_process_oracle(world, T, nbs, decay, splits, folds):
     B, H, K, V, seed = 1, 2, 16, 8, 3
     mgr = mp.Manager()
     ret = mgr.dict()
-    mp.spawn(_worker, args=(world, _free_port(), B, T, H, K, V, nbs, decay, seed, ret, "contiguous", splits), nprocs=world,
+    mp.spawn(_worker, args=(world, _free_port(), B, T, H, K, V, nbs, decay, seed, ret, "contiguous", splits, folds), nprocs=world,
              join=True)
     q, k, v, g, types = _inputs(B, T, H, K, V, nbs, seed)
     o_ref, s_ref = ogdn.linear_recurrent(q, k, v, g, None, types[..., 1], nbs=nbs, scale=1.0, decay=decay,
@@ -86,12 +87,13 @@ def _check(ret, world, o_ref, oa_ref, s_ref, holder):
     assert (ret[holder][2] - s_ref).abs().max() < 1e-9
 
 
-@pytest.mark.parametrize("world,T,nbs,splits", [(2, 1024, 128, None), (3, 1536, 128, 2), (2, 2048, 128, 4)])
-def test_sp_zigzag_matches_single_process_oracle(world, T, nbs, splits):
+@pytest.mark.parametrize("world,T,nbs,splits,folds", [(2, 1024, 128, None, False), (3, 1536, 128, 2, False), (2, 2048, 128, 4, False),
+                                                      (3, 1536, 128, 2, True)])
+def test_sp_zigzag_matches_single_process_oracle(world, T, nbs, splits, folds):
     B, H, K, V, seed = 2, 2, 16, 8, 5
     mgr = mp.Manager()
     ret = mgr.dict()
-    mp.spawn(_worker, args=(world, _free_port(), B, T, H, K, V, nbs, True, seed, ret, "zigzag", splits), nprocs=world,
+    mp.spawn(_worker, args=(world, _free_port(), B, T, H, K, V, nbs, True, seed, ret, "zigzag", splits, folds), nprocs=world,
              join=True)
     q, k, v, g, types = _inputs(B, T, H, K, V, nbs, seed)
     o_ref, s_ref = ogdn.linear_recurrent(q, k, v, g, None, types[..., 1], nbs=nbs, scale=1.0, decay=True,
@@ -143,14 +145,13 @@ def test_priority_of_the_linear_branch(monkeypatch):
 def test_single_rank_sub_segment_split_matches_oracle():
     """One process, no process group: only the sub-segment split of the linear branch is exercised."""
     from neuralattentionsearchlinear_b200.sequence_parallel import nats_mixed_attn_mamba_sp
-    from tests.sp_helpers import OracleSegmentOps
+    from tests.sp_helpers import FoldingSegmentOps, OracleSegmentOps
     B, T, H, K, V, nbs, seed = 2, 1024, 2, 16, 8, 128, 11
     q, k, v, g, types = _inputs(B, T, H, K, V, nbs, seed)
     types[:, -1] = 1
-    for decay in (True, False):
+    for decay, backend in ((True, OracleSegmentOps()), (False, OracleSegmentOps()), (True, FoldingSegmentOps()), (False, FoldingSegmentOps())):
         o_l, o_a, ht = nats_mixed_attn_mamba_sp(q, k, v, q, k, v, g, types, nats_block_size=nbs,
-                                                decay_for_non_mamba_blocks=decay, linear_splits=4,
-                                                backend=OracleSegmentOps())
+                                                decay_for_non_mamba_blocks=decay, linear_splits=4, backend=backend)
         o_ref, s_ref = ogdn.linear_recurrent(q, k, v, g, None, types[..., 1], nbs=nbs, scale=1.0, decay=decay,
                                              use_l2norm=False, rule="mamba")
         oa_ref, _ = oattn.attn_sdpa(q, k, v, oattn.attn_mask(types[..., 0], T, nbs, H))
