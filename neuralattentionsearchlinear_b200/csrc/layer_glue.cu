@@ -29,52 +29,8 @@ __device__ __forceinline__ float sigmoidf_(float x) { return 1.f / (1.f + __expf
 
 // ------------------------------------------------------------------------------------------------ short conv + SiLU
 constexpr int CONV_W = 4;
-constexpr int CONV_TT = 32;          // tokens per thread (forward)
 
-// y[b,t,d] = act(bias[d] + sum_j w[d,j] x[b, t-(W-1)+j, d]); one thread = 8 channels x CONV_TT tokens.
-__global__ void __launch_bounds__(128)
-short_conv_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
-                      const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ y, int T, int D, int silu) {
-    const int cg = blockIdx.x * blockDim.x + threadIdx.x;          // group of 8 channels
-    if (cg * 8 >= D) return;
-    const int d0 = cg * 8;
-    const int t0 = blockIdx.y * CONV_TT, b = blockIdx.z;
-    float wt[8][CONV_W], bs[8];
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-        bs[c] = bias ? __bfloat162float(bias[d0 + c]) : 0.f;
-#pragma unroll
-        for (int j = 0; j < CONV_W; ++j) wt[c][j] = __bfloat162float(w[(d0 + c) * CONV_W + j]);
-    }
-    float win[CONV_W][8];                                           // sliding window: win[j] = x[t-(W-1)+j]
-#pragma unroll
-    for (int j = 0; j < CONV_W - 1; ++j) {
-        const int t = t0 - (CONV_W - 1) + j;
-        if (t >= 0) ld8(x + ((long)b * T + t) * D + d0, win[j + 1]);
-        else {
-#pragma unroll
-            for (int c = 0; c < 8; ++c) win[j + 1][c] = 0.f;
-        }
-    }
-    const int t_end = min(T, t0 + CONV_TT);
-    for (int t = t0; t < t_end; ++t) {
-#pragma unroll
-        for (int j = 0; j < CONV_W - 1; ++j)
-#pragma unroll
-            for (int c = 0; c < 8; ++c) win[j][c] = win[j + 1][c];
-        ld8(x + ((long)b * T + t) * D + d0, win[CONV_W - 1]);
-        float out[8];
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-            float a = bs[c];
-#pragma unroll
-            for (int j = 0; j < CONV_W; ++j) a += wt[c][j] * win[j][c];
-            out[c] = silu ? a * sigmoidf_(a) : a;
-        }
-        st8(y + ((long)b * T + t) * D + d0, out);
-    }
-}
-
+// y[b,t,d] = act(bias[d] + sum_j w[d,j] x[b, t-(W-1)+j, d]).
 // Backward: dpre = dy * act'(pre) with pre recomputed; dx[t] = sum_j w[j] dpre[t+(W-1)-j];
 // dw[d,j] = sum_{b,t} dpre[t] x[t-(W-1)+j], dbias[d] = sum dpre: per-(batch, token range) partial sums
 // dw_part [B * gridDim.y, D, W + 1] (column W = bias).  One thread = 8 channels x `span` tokens.
