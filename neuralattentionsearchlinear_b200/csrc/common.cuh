@@ -127,12 +127,18 @@ __device__ __forceinline__ uint32_t close2(uint64_t v) {
     return pack_bf16(lo, hi);
 }
 
-// Logistic function of a pair.  The reciprocal is an approximate one with a step of Newton's iteration (as exact as a division,
-// without its call and its branches); with exp(-|x|) its argument lies in [1, 2].
+// Logistic function of a pair.  The reciprocal is an approximate one (off by e <= 2^-23) with a step of Newton's iteration, which
+// leaves e^2 and two roundings, less than one unit of 2^-23, without a division's call and branches; with exp(-|x|) its argument lies
+// in [1, 2].  In all 2 + 1.173 |x| units from __expf, one from the reciprocal, half a one each from 1 + t and, for x < 0, from the
+// product with t.
 __device__ __forceinline__ float rcp_ftz(float x) {
     float y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
+}
+__device__ __forceinline__ float rcp_newton(float y) {        // 1 / y, y in [1, 2]
+    const float r = rcp_ftz(y);
+    return fmaf(r, fmaf(-y, r, 1.f), r);
 }
 __device__ __forceinline__ uint64_t sigmoid2(uint64_t v) {
     // (constants as immediates of scalar instructions: a pair of them would take two registers, or two moves at every use)

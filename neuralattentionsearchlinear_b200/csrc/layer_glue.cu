@@ -272,9 +272,12 @@ rmsnorm_fwd_narrow_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat
 // A thread owns eight neighbouring features of its rows: the row, its gradient and what is added are read once, with the next
 // turn's loads in flight, and the weights and their gradients stay in registers.  Narrow rows (D <= 256): D / 8 lanes, the rows
 // of a warp side by side, no barrier.  Wide rows: D / 8 threads, 256 / (D / 8) rows of a CTA side by side, the
-// partial sums of the warps through shared memory (double-buffered: one barrier a turn); two rows deep takes 127 registers and
-// half the CTAs (127 against 121 us).  Bound by memory.  L2 flushed, against a warp per row that read it twice, one row in flight:
-// 32768 x 2048 with an added gradient 217 -> 121 us (traffic 82), 524288 x 128 137 -> 107 us (62).
+// partial sums of the warps through shared memory (double-buffered: one barrier a turn), 64 registers for four CTAs per SM with 86 to
+// 112 bytes spilled; two rows deep takes 127 registers and half the CTAs (127 against 121 us).  Bound by memory.  L2 flushed, against a warp per row that read it twice, one row in flight:
+// 32768 x 2048 with an added gradient 217 -> 121 us (traffic 82), 524288 x 128 137 -> 107 us (62).  Few rows are bound by the turns of
+// a CTA (min(rows / 8, RMS_BWD_CTAS) CTAs, so eight turns of one row at 2048 features), in a graph, warm: 300 x 2048 15.5 -> 11.0 us,
+// 1000 x 2048 14.9 -> 10.9, 4000 x 2048 52 -> 19, 1000 x 64 2.3 -> 2.4, 16000 x 64 4.9 -> 4.1.
+constexpr int RMS_BWD_CTAS = 592;                              // four per SM, one partial sum of the weight gradient each
 struct RmsBwd {
     const __nv_bfloat16 *s, *dy, *dadd;
     const void* w;
@@ -806,7 +809,7 @@ extern "C" int natsl_l2norm_bwd(const void* x, const void* dy, void* dx, int64_t
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const RmsBwd p = {bfc(x), bfc(dy), nullptr, nullptr, bfm(dx), nullptr, rows, 1.f, eps, 0, aligned_to(16, x, dy, dx)};
     const long turns = (rows + 8 * (256 / D) - 1) / (8 * (256 / D));
-    const unsigned grid = (unsigned)(turns < 592 ? turns : 592);
+    const unsigned grid = (unsigned)(turns < RMS_BWD_CTAS ? turns : RMS_BWD_CTAS);
     if (D == 64) rmsnorm_bwd_narrow_kernel<64><<<grid, 256, 0, st>>>(p);
     else if (D == 128) rmsnorm_bwd_narrow_kernel<128><<<grid, 256, 0, st>>>(p);
     else rmsnorm_bwd_narrow_kernel<256><<<grid, 256, 0, st>>>(p);

@@ -22,8 +22,9 @@
 //                            then the l2-norm backward (mixed_attn_gdn.py:273-275).
 //   linear_bwd_dg_kernel     per (batch, head): the scalar chain of the carried decay over skipped chunks and the
 //                            reverse chunk-local cumsum (chunk.py:318-331, src/nats/ops/utils/cumsum.py REVERSED).
-// All products run on mma.sync with bf16 operands and fp32 accumulation.  No atomics on global memory; shared-memory
-// sums either have one writer per slot or exactly two terms, so results are reproducible bit for bit.
+// All products run on mma.sync with bf16 operands and fp32 accumulation.  Reductions on global memory (gradients added onto the
+// softmax branch's) have one writer per element; shared-memory sums either have one writer per slot or exactly two terms, so results
+// are reproducible bit for bit.
 #include "warp_gemm.cuh"
 #include "../../include/natsl_b200.h"
 

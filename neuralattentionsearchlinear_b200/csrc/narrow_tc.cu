@@ -1,8 +1,8 @@
 // Narrow projections of a layer: y[t, n] = x[t, :] . W[n, :] for a few rows n (2 H decays and betas, or 2 HQ mixing logits) with
 // the pointwise steps behind them (src/nats/layers/natsl_attn_gdn.py:461-480, 590-600, src/nats/layers/natsl_attn_mamba2.py:402-440).
 // Bound by reading x once.  One CTA = 128 tokens of a sequence x up to 64 rows of W: TMA brings x and W in steps of 64 features
-// through a ring of stages, tcgen05 adds the products up in tensor memory, one thread per token then works on its row of
-// results.  (On mma.sync, fragments straight from global memory, the registers left one CTA on an SM: 16 x 4096 tokens of 1024
+// through a ring of stages, tcgen05 adds the products up in tensor memory, two threads per token then work on a half of its row of
+// results each.  (On mma.sync, fragments straight from global memory, the registers left one CTA on an SM: 16 x 4096 tokens of 1024
 // features, 32 rows took 72 us, here 33 us; the traffic needs 21 us.  What a small call is bound by is the issue of a step: a
 // commit as long as its products, and every further TMA box, so W comes in one box per matrix and stages are given back in pairs:
 // 4 x 1030 tokens of 2048 features 32 -> 21 us.)
@@ -17,12 +17,13 @@ namespace natsl {
 namespace {
 
 using bf16 = __nv_bfloat16;
+constexpr int NW_BACK = 2;                                   // stages given back together: a commit costs as much as a step's products
 constexpr int NW_MAX_STAGES = 8, NW_EPI = 256, NW_THREADS = NW_EPI + 64, NW_TOK = 128;
 
 struct NarrowPlan {
     int n0p;                                                 // columns of w0, padded to groups of eight
     int rows;                                                // rows of a box of W
-    int steps, stages, back;                                  // stages given back together (1, 2 or 4: a commit costs as much as a step's products)
+    int steps, stages;
 };
 template <int NT>
 struct NwSmem {                                              // the ring of stages lies behind the rest
@@ -54,10 +55,6 @@ __device__ __forceinline__ void tmem_row(uint32_t taddr, uint32_t (&r)[N]) {
                      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                      : "r"(taddr));
     tmem_ld_wait();
-}
-__device__ __forceinline__ float rcp_step(float y) {         // 1 / y, y in [1, 2]
-    const float r = rcp_ftz(y);
-    return fmaf(r, fmaf(-y, r, 1.f), r);
 }
 
 template <int NT>
@@ -103,7 +100,7 @@ narrow_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
 #pragma unroll 1
             for (int k = 0, s = 0, turn = 0; k < p.steps; ++k) {
                 const uint32_t st = sbase + L::ring + s * L::stage, full = bar_full + 8 * s;
-                if (turn && (s & (p.back - 1)) == 0) mbar_wait_small(bar_empty + 8 * s, (turn - 1) & 1, status);
+                if (turn && (s & (NW_BACK - 1)) == 0) mbar_wait_small(bar_empty + 8 * s, (turn - 1) & 1, status);
                 mbar_expect_tx(full, (NW_TOK + boxes * p.rows) * 128);
                 tma_load_4d(st, &map_x, k * 64, 0, t0, b, full);
 #pragma unroll 1
@@ -124,7 +121,7 @@ narrow_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             __syncwarp();
             tc_fence_after();
             umma_ss_x4<2, 2>(tmem, umma_desc_lo(st, 16), umma_desc_lo(st + NW_TOK * 128, 16), id, k > 0);
-            if ((s & (p.back - 1)) == p.back - 1) umma_commit(bar_empty + 8 * (s - p.back + 1));
+            if ((s & (NW_BACK - 1)) == NW_BACK - 1) umma_commit(bar_empty + 8 * (s - NW_BACK + 1));
             if (++s == p.stages) { s = 0; ++turn; }
         }
         umma_commit(bar_done);
@@ -150,7 +147,7 @@ narrow_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {                  // softmax over a pair
                     const float d = rb(__uint_as_float(r[i + 2 * e])) - rb(__uint_as_float(r[i + 2 * e + 1]));
-                    const float ex = expf(-fabsf(d)), hi = rcp_step(1.f + ex), lo = ex * hi;
+                    const float ex = expf(-fabsf(d)), hi = rcp_newton(1.f + ex), lo = ex * hi;
                     o[e] = d < 0.f ? pack_bf16(lo, hi) : pack_bf16(hi, lo);
                 }
                 if (!ok) continue;
@@ -194,7 +191,7 @@ narrow_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                     float v[4];
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
-                        const float y = rb(__uint_as_float(r[i + e])), ex = expf(-fabsf(y)), hi = rcp_step(1.f + ex);
+                        const float y = rb(__uint_as_float(r[i + e])), ex = expf(-fabsf(y)), hi = rcp_newton(1.f + ex);
                         v[e] = rb(y < 0.f ? ex * hi : hi);
                         if (a.neg_eigval) v[e] *= 2.f;
                     }
@@ -257,8 +254,8 @@ int launch(const NarrowArgs& a, int n0p, int B, cudaStream_t st) {
     // have the GPU to themselves (the decays; the mixing weights run beside the walk, and a CTA that takes more of an SM is in its
     // way: layer of 2 x 2048 tokens, 16 x 128 heads 329 us, 358 to 370 us with eight stages) the ring is twice as deep: 4 x 1030
     // tokens of 2048 features, 32 rows 21 us against 24 us.
-    p.stages = a.mode == 0 && ctas <= 148 ? 8 : 4;
-    p.back = 2;
+    p.stages = a.mode == 0 && ctas <= 148 ? NW_MAX_STAGES : 4;
+    while (p.stages > NW_BACK && p.stages - NW_BACK >= p.steps) p.stages -= NW_BACK;          // no more than the contraction fills
     p.rows = NT;                                             // a box of W lies in one matrix
     while (a.n1 && n0p % p.rows) p.rows /= 2;
     CUtensorMap mx, m0, m1;

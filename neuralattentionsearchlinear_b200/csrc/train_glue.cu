@@ -150,7 +150,8 @@ block_mean_bwd_kernel(const bf16* __restrict__ dy, bf16* __restrict__ dx, int T,
 }
 
 // ------------------------------------------------------------------------------------------------ sums of partial gradients
-// out[n] = sum_p part[p, n], p in order over eight groups of rows and then over the groups.  A CTA: 32 columns x 8 x 4 threads.
+// out[n] = sum_p part[p, n].  A CTA: 32 columns x 32 threads; a thread adds up every 32nd row in four sums (rows 128 apart each, what is
+// left over in the first), then the four in pairs, and a warp the 32 threads of a column as a tree: the same order on every run.
 struct ColArgs {
     const float* part;
     void *o0, *o1;

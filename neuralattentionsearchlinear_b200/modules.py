@@ -32,9 +32,12 @@ def _eager(*tensors) -> bool:
             and all(t is None or type(t) in (torch.Tensor, nn.Parameter) for t in tensors))
 
 
+_PARTS = 592                         # CTAs with a partial sum of the weight gradients each, at most: four per SM
+
+
 def _n_part(rows: int) -> int:
-    """CTAs of the norms' backward kernels, each with one partial sum of the weight gradients: four per SM."""
-    return int(min(-(-rows // 8), 592))
+    """CTAs of the norms' backward kernels."""
+    return int(min(-(-rows // 8), _PARTS))
 
 
 _SUM_DTYPES = (torch.bfloat16, torch.float32)
@@ -200,7 +203,7 @@ class _GatesFn(torch.autograd.Function):
         dg, dbeta, dvo = (None if x is None else x.contiguous() for x in (dg, dbeta, dvo))
         da, db = torch.empty_like(a), (None if b is None else torch.empty_like(b))
         dv = None if dvo is None else torch.empty_like(v)
-        part = torch.empty(min(-(-rows // (256 // H)), 592), 2, H, dtype=torch.float32, device=a.device)
+        part = torch.empty(min(-(-rows // (256 // H)), _PARTS), 2, H, dtype=torch.float32, device=a.device)
         _lib.call("natsl_gates_bwd", a.data_ptr(), _lib.ptr(b), _lib.ptr(v), A_log.data_ptr(), _dt(A_log), dt_bias.data_ptr(), _dt(dt_bias),
                   ctx.neg, _lib.ptr(dg), _lib.ptr(dbeta), _lib.DT_BF16 if dbeta is None else _dt(dbeta), _lib.ptr(dvo), da.data_ptr(),
                   _lib.ptr(db), _lib.ptr(dv), part.data_ptr(), part.shape[0], rows, H, 0 if v is None else v.shape[-1],
