@@ -580,6 +580,8 @@ extern "C" int natsl_short_conv_fwd(const void* x, const void* w, const void* bi
     NATSL_REQUIRE(B > 0 && T > 0 && D > 0 && D % 8 == 0 && B <= 65535, NATSL_ERR_BAD_SHAPE,
                   "natsl_short_conv_fwd: bad shape (D a multiple of 8)");
     NATSL_REQUIRE(W == CONV_W, NATSL_ERR_UNSUPPORTED, "natsl_short_conv_fwd: kernel size %d is not built (4)", W);
+    NATSL_REQUIRE(natsl::aligned_to(16, x) && natsl::aligned_to(8, y), NATSL_ERR_UNSUPPORTED,
+                  "natsl_short_conv_fwd: a tensor does not start on 16 bytes (y: 8)");
     dim3 grid((D + CF_L * CF_CH - 1) / (CF_L * CF_CH), (T + CF_TT - 1) / CF_TT, B);
     short_conv_fwd_tile_kernel<<<grid, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(bfc(x), bfc(w), bfc(bias), bfm(y), T, D, silu,
                                                                                          aligned_to(16, w));
@@ -713,6 +715,8 @@ extern "C" int natsl_short_conv_bwd(const void* x, const void* w, const void* bi
     NATSL_REQUIRE(B > 0 && T > 0 && D > 0 && D % 8 == 0 && B <= 65535 && span > 0, NATSL_ERR_BAD_SHAPE,
                   "natsl_short_conv_bwd: bad shape (D a multiple of 8)");
     NATSL_REQUIRE(W == CONV_W, NATSL_ERR_UNSUPPORTED, "natsl_short_conv_bwd: kernel size %d is not built (4)", W);
+    NATSL_REQUIRE(natsl::aligned_to(16, x, dy) && natsl::aligned_to(span == CB_TT ? 4 : 16, dx), NATSL_ERR_UNSUPPORTED,
+                  "natsl_short_conv_bwd: a tensor does not start on 16 bytes (dx: 4 with spans of 64 tokens)");
     const int groups = D / 8;
     if (span == CB_TT) {
         constexpr int smem = ((CB_TT + 2 * (CONV_W - 1)) + (CB_TT + CONV_W - 1)) * CB_GR * CB_CG * CB_CH * 2;
@@ -748,6 +752,7 @@ extern "C" int natsl_rmsnorm_fwd(const void* x, const void* res, const void* w, 
     NATSL_REQUIRE(x && y, NATSL_ERR_NULL, "natsl_rmsnorm_fwd: null pointer");
     NATSL_REQUIRE(rows > 0, NATSL_ERR_BAD_SHAPE, "natsl_rmsnorm_fwd: empty input");
     NATSL_REQUIRE(w_dtype == NATSL_DT_BF16 || w_dtype == NATSL_DT_F32, NATSL_ERR_UNSUPPORTED, "natsl_rmsnorm_fwd: weight must be bf16 or f32");
+    NATSL_REQUIRE(natsl::aligned_to(16, x, res, y, sum_out), NATSL_ERR_UNSUPPORTED, "natsl_rmsnorm_fwd: a tensor does not start on 16 bytes");
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     if (D == 64 || D == 128 || D == 256) {
         const int rpc = 8 * (32 / (D / 8));                  // rows per CTA
@@ -819,6 +824,7 @@ extern "C" int natsl_l2norm_bwd(const void* x, const void* dy, void* dx, int64_t
 extern "C" int natsl_swiglu_fwd(const void* a, const void* b, void* y, long n, void* stream) {
     NATSL_REQUIRE(a && b && y, NATSL_ERR_NULL, "natsl_swiglu_fwd: null pointer");
     NATSL_REQUIRE(n > 0 && n % 8 == 0, NATSL_ERR_BAD_SHAPE, "natsl_swiglu_fwd: element count must be a positive multiple of 8");
+    NATSL_REQUIRE(natsl::aligned_to(16, a, b, y), NATSL_ERR_UNSUPPORTED, "natsl_swiglu_fwd: a tensor does not start on 16 bytes");
     const long n8 = n / 8;
     const unsigned grid = (unsigned)((n8 + 255) / 256 < 148 * 16 ? (n8 + 255) / 256 : 148 * 16);
     swiglu_fwd_kernel<<<grid, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(bfc(a), bfc(b), bfm(y), n8);
@@ -828,6 +834,7 @@ extern "C" int natsl_swiglu_fwd(const void* a, const void* b, void* y, long n, v
 extern "C" int natsl_swiglu_bwd(const void* a, const void* b, const void* dy, void* da, void* db, long n, void* stream) {
     NATSL_REQUIRE(a && b && dy && da && db, NATSL_ERR_NULL, "natsl_swiglu_bwd: null pointer");
     NATSL_REQUIRE(n > 0 && n % 8 == 0, NATSL_ERR_BAD_SHAPE, "natsl_swiglu_bwd: element count must be a positive multiple of 8");
+    NATSL_REQUIRE(natsl::aligned_to(16, a, b, dy, da, db), NATSL_ERR_UNSUPPORTED, "natsl_swiglu_bwd: a tensor does not start on 16 bytes");
     const long n8 = n / 8;
     const unsigned grid = (unsigned)((n8 + 255) / 256 < 148 * 16 ? (n8 + 255) / 256 : 148 * 16);
     swiglu_bwd_kernel<<<grid, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(bfc(a), bfc(b), bfc(dy), bfm(da), bfm(db), n8);
@@ -840,6 +847,7 @@ extern "C" int natsl_block_mean(const void* x, void* y, int B, int T, int D, int
                   "natsl_block_mean: bad shape (D a multiple of 8)");
     const int NB = (T + nbs - 1) / nbs;
     NATSL_REQUIRE(NB <= 65535, NATSL_ERR_TOO_LARGE, "natsl_block_mean: too many blocks");
+    NATSL_REQUIRE(natsl::aligned_to(4, x, y), NATSL_ERR_UNSUPPORTED, "natsl_block_mean: a tensor does not start on 4 bytes");
     dim3 grid((D / 2 + 127) / 128, NB, B);
     block_mean_kernel<<<grid, 128, 0, reinterpret_cast<cudaStream_t>(stream)>>>(bfc(x), bfm(y), T, D, nbs, NB);
     return check_launch("natsl_block_mean");

@@ -190,6 +190,7 @@ extern "C" int natsl_norm_gate_mix(const void* x1, const void* x2, const void* g
     NATSL_REQUIRE(activation == 0 || activation == 1, NATSL_ERR_UNSUPPORTED, "natsl_norm_gate_mix: activation 0 (swish) or 1 (sigmoid)");
     NATSL_REQUIRE((xw_dtype == NATSL_DT_BF16 || xw_dtype == NATSL_DT_F32) && (w_dtype == NATSL_DT_BF16 || w_dtype == NATSL_DT_F32),
                   NATSL_ERR_UNSUPPORTED, "natsl_norm_gate_mix: weights must be bf16 or f32");
+    NATSL_REQUIRE(natsl::aligned_to(16, x1, x2, g, y), NATSL_ERR_UNSUPPORTED, "natsl_norm_gate_mix: a tensor does not start on 16 bytes");
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const int wpb = 8;
     const long rpc = (long)wpb * (32 / (D > 0 ? (D / 8 > 0 ? D / 8 : 1) : 1));      // rows per CTA and turn

@@ -154,3 +154,18 @@ def test_short_conv_bwd_over_other_spans(B, T, D, span):
         got.append((dx, part.sum(0)))
     _close(got[1][0], got[0][0])
     _close(got[1][1], got[0][1], fp32=True)
+
+
+def test_forward_kernels_refuse_tensors_between_their_loads():
+    """What reads or writes whole vectors is refused on the host where a tensor starts between two of them."""
+    t = torch.zeros(4096, dtype=BF, device="cuda")
+    on, off = t.data_ptr(), t.data_ptr() + 2
+    calls = {"natsl_rmsnorm_fwd": ([on, None, None, 0, on, None], (1, 64, EPS)), "natsl_norm_gate_mix": ([on, on, on, None, 0, None, None, 0, on], (1, 64, EPS, 0)),
+             "natsl_short_conv_fwd": ([on, on, None, on], (1, 4, 8, 4, 1)), "natsl_short_conv_bwd": ([on, on, None, on, on, on], (1, 4, 8, 4, 1, 64)),
+             "natsl_swiglu_fwd": ([on, on, on], (8,)), "natsl_swiglu_bwd": ([on] * 5, (8,)), "natsl_block_mean": ([on, on], (1, 4, 8, 64))}
+    weights = {("natsl_short_conv_fwd", 1), ("natsl_short_conv_bwd", 1), ("natsl_short_conv_bwd", 5)}      # (and partial sums, fp32)
+    for name, (tensors, sizes) in calls.items():
+        for i, p in enumerate(tensors):
+            if p == on and (name, i) not in weights:
+                with pytest.raises(_lib.NatslError, match="does not start"):
+                    _lib.call(name, *tensors[:i], off, *tensors[i + 1:], *sizes, _st())
