@@ -145,9 +145,10 @@ narrow_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 if (n >= a.n0) break;
                 uint32_t o[4];
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {                  // softmax over a pair
-                    const float d = rb(__uint_as_float(r[i + 2 * e])) - rb(__uint_as_float(r[i + 2 * e + 1]));
-                    const float ex = expf(-fabsf(d)), hi = rcp_newton(1.f + ex), lo = ex * hi;
+                for (int e = 0; e < 4; ++e) {                  // softmax over a pair (a larger logit of +inf: NaN, by m - m)
+                    const float l0 = rb(__uint_as_float(r[i + 2 * e])), l1 = rb(__uint_as_float(r[i + 2 * e + 1]));
+                    const float d = l0 - l1, m = fmaxf(l0, l1);
+                    const float ex = expf(-fabsf(d)) + (m - m), hi = rcp_newton(1.f + ex), lo = ex * hi;
                     o[e] = d < 0.f ? pack_bf16(lo, hi) : pack_bf16(hi, lo);
                 }
                 if (!ok) continue;

@@ -118,3 +118,18 @@ def test_outputs_against_float64(rule, args, B, T, monkeypatch):
     want, exact = _bf16(w, 2 ** -19 * w)
     both = sure.unflatten(-1, (-1, 2)).all(-1, keepdim=True) & exact
     assert float(both.double().mean()) > 0.7 and bool((got["mix"].double() == want)[both].all())
+
+
+def test_infinite_mixing_logits(monkeypatch):
+    """As torch's softmax: a logit of +inf gives NaN, one of -inf beside a finite one a weight of zero."""
+    torch.manual_seed(1)
+    layer = _make("gdn", hidden=96, heads=2, head_dim=64, expand_v=1, attn_heads=2).cuda().bfloat16().eval()
+    w = layer.nats_out_weights_layer.weight
+    with torch.no_grad():
+        w[::2] = 0
+        w[0, 5], w[2, 70] = 3e38, -3e38                      # the heads' first logits: one product each, of activations above -0.3
+    got = _own_outputs(layer, torch.randn(1, 300, 96).bfloat16().cuda() * 20, monkeypatch)
+    z = torch.nn.functional.linear(got["q"].double(), w.detach().double()).to(torch.bfloat16).unflatten(-1, (-1, 2))
+    inf, want = z[..., 0].isinf(), z.softmax(-1)
+    assert inf[..., 0].any() and (z[..., 0, 0][inf[..., 0]] > 0).all() and inf[..., 1].any() and (z[..., 1, 0][inf[..., 1]] < 0).all()
+    assert want[..., 0, :][inf[..., 0]].isnan().all() and torch.equal(got["mix"][inf].nan_to_num(2.0), want[inf].nan_to_num(2.0))
