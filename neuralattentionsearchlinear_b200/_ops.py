@@ -35,11 +35,11 @@ LINEAR_BRANCH_PRIORITY = os.environ.get("NATSL_LINEAR_PRIORITY", "1") != "0"
 
 # (batch, head) pairs up to which the delta rule takes the mma.sync walk also where the tcgen05 one is built (K = V = 128,
 # block 64): 32 value columns per CTA make four CTAs of a pair, which fit one wave of 148 SMs up to 37 pairs, and a chunk takes
-# 1.6 instead of 2.8 us.  Walk alone, mma.sync against tcgen05, T = 2048: 32 pairs 57 / 91 us; 48 - 64 pairs (64 columns per
-# CTA) 86 / 93 us; 80 pairs (two waves) 160 / 92 us.  In the whole op, where a walk on all SMs delays the softmax branch, up to
-# 36 pairs gain at every length (T = 512: 45 / 53, T = 4096: 252 / 291 us), 48 - 72 pairs gain up to 8 % at T <= 1024 and lose
-# up to 10 % at T = 4096.  Between 31 and 37 the line gives way to batches of 16-head sequences: from two of them on a
-# sequence's result does not depend, bit for bit, on the batch around it.  0 extends that to one sequence (one walk for all).
+# 1.6 instead of 1.8 us.  Whole ops captured in a graph, mma.sync against tcgen05: 4 to 28 pairs 18 / 22 us at T = 256, 62 - 89 /
+# 70 - 96 us at T = 2048, 111 - 172 / 124 - 179 us at T = 4096; 32 pairs 93 / 101 us at T = 2048, 201 / 190 us at T = 4096; 48
+# pairs (two waves) 28 / 24, 135 / 117 and 261 / 216 us.  Between 31 and 37 the line gives way to batches of 16-head sequences:
+# from two of them on a sequence's result does not depend, bit for bit, on the batch around it.  0 extends that to one sequence
+# (one walk for all).
 WALK_MMA_MAX_HEADS = int(os.environ.get("NATSL_WALK_MMA_MAX_HEADS", "31"))
 
 

@@ -10,18 +10,27 @@
 // src/nats/ops/common/chunk_o.py:124-215 (output) and the carry of src/nats/ops/utils/cumsum.py:85-133.
 // The decay of the state is applied when the state is copied to shared memory for the next chunk
 // (one TMEM pass per update: bf16 copy out, multiply by the next update's decay, write back), so the
-// accumulating MMA 3 needs no separate rescale.  P is padded to 128 rows (rows 0-63 zero) so that
-// P v' lands in the TMEM lanes of the q rows.
-// Warp roles: warp 0 TMA producer (w, q, k, u tiles in two stages, P single-buffered), warp 1 MMA issuer,
-// warps 2-9 two threads per TMEM lane (64 columns each).  All mbarrier waits are bounded (status word +
-// clean teardown on expiry).
+// accumulating MMA 3 needs no separate rescale.  The product P v' has 128 rows: P in the rows of q, whatever lies in front of the
+// tile in the others, whose results nobody reads.
+//
+// What bounds it: the chain w S -> v' -> k^T v'' -> copy of the state, chunk after chunk, one CTA per SM.  Hence sixteen warps
+// with 32 columns of a TMEM lane each (loads, products and stores of a step in one go, not in a loop), one arrival per warp on a
+// barrier, everything that does not depend on the step's product read or computed in front of the wait for it, the multiplied
+// state written back behind the announcement of its copy, and outputs that leave through shared memory by TMA: rows of 16 bytes
+// per lane kept the load/store unit busy for half of a chunk, and the next chunk's v' waited behind them.
+// Alone (us; before: eight warps of 64 columns each, outputs stored row by row): B = 8, T = 4096, H = 16, 75 % of the chunks
+// selected 173 -> 130 (738 MB: 5.7 TB/s), 50 % 168 -> 127; 32 CTAs, T = 8192 333 -> 234, 1.8 us a chunk.  Of 4.6 k cycles per chunk the
+// old form spent 2.1 k on v' and 1.7 k of the output warps on their stores.
+// Warp roles: warp 0 loads w, q and k, u (two stages, each half of a stage given back on its own), warp 1 issues the products,
+// warps 2-17 the rows, warp 18 loads P (one buffer) and stores the outputs.  All mbarrier waits are bounded (status word + clean
+// teardown on expiry).
 #include "tc_common.cuh"
 #include "../../include/natsl_b200.h"
 
 namespace natsl {
 
-constexpr int WK_THREADS = 320;
-constexpr int WK_EPI = 256;
+constexpr int WK_THREADS = 608;
+constexpr int WK_ROW_WARPS = 16;
 constexpr uint32_t WK_TMEM_COLS = 512;
 constexpr uint32_t WK_S = 0, WK_D1 = 128, WK_D2 = 256, WK_D1B = 384;     // TMEM column offsets (D1 double-buffered)
 constexpr int WK_MAX_NT = 1024;
@@ -32,25 +41,27 @@ struct WkSmem {
     static constexpr int sbf = 2 * stage;                 // S bf16: 2 sub-tiles [128 k-rows][64 v-cols]   32 KB
     static constexpr int vp = sbf + 32768;                // v'  : 2 sub-tiles [64 tok][64]                16 KB
     static constexpr int vs = vp + 16384;                 // v'' : same layout                              16 KB
-    static constexpr int pp = vs + 16384;                 // P padded to 128 rows: [128][64 tok]            16 KB
-    static constexpr int meta = pp + 16384;               // per chunk: carry, dec, g_last (float), sel (int)
-    static constexpr int bars = meta + 4 * 4 * WK_MAX_NT;
+    static constexpr int pp = vs + 16384;                 // P : [64][64 tok]; the operand begins 8 KB in front of it
+    static constexpr int out = pp + 8192;                 // outputs on their way: 2 sub-tiles [64 tok][64] 16 KB
+    static constexpr int carry = out + 16384;             // per chunk: decay of the skipped blocks in front of it;
+    static constexpr int mul = carry + 4 * WK_MAX_NT;     // the next update's decay, sign bit set where the chunk updates the state
+    static constexpr int bars = mul + 4 * WK_MAX_NT;
     static constexpr int total = bars + 256;
+    static_assert(total <= 232448, "shared memory of one SM");
 };
 
-template <bool kDummy>
 __global__ void __launch_bounds__(WK_THREADS, 1)
 gdn_walk_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_q,
                    const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_u,
-                   const __grid_constant__ CUtensorMap map_p, const float* __restrict__ gcs,
-                   const float* __restrict__ krstd, const float* __restrict__ qrstd, const int* __restrict__ types_i,
-                   const int* __restrict__ indices, const int* __restrict__ n_blocks, const float* __restrict__ h0,
-                   __nv_bfloat16* __restrict__ o, float* __restrict__ ht, float* hstart, const void* __restrict__ last_types,
+                   const __grid_constant__ CUtensorMap map_p, const __grid_constant__ CUtensorMap map_o,
+                   const float* __restrict__ gcs, const float* __restrict__ krstd, const float* __restrict__ qrstd,
+                   const int* __restrict__ types_i, const int* __restrict__ indices, const int* __restrict__ n_blocks,
+                   const float* __restrict__ h0, float* __restrict__ ht, float* hstart, const void* __restrict__ last_types,
                    int last_f32, int last_stride, int T, int H, int HN, int TN, float scale, int decay, int trailing_quirk, int* status) {
     using L = WkSmem;
     constexpr int K = 128, V = 128;
     extern __shared__ __align__(1024) unsigned char smem[];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const uint32_t sbase = smem_u32(smem);
     if ((sbase & 1023u) != 0) {
         if (tid == 0) atomicExch(status, 2);
@@ -59,334 +70,360 @@ gdn_walk_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     const int h = blockIdx.x, b = blockIdx.y;
     const int hn = h / (H / HN);
     const int NT = (T + 63) / 64;
-    float* m_carry = reinterpret_cast<float*>(smem + L::meta);
-    float* m_dec = m_carry + WK_MAX_NT;
-    float* m_gl = m_dec + WK_MAX_NT;
-    int* m_sel = reinterpret_cast<int*>(m_gl + WK_MAX_NT);
+    float* m_carry = reinterpret_cast<float*>(smem + L::carry);
+    uint32_t* m_mul = reinterpret_cast<uint32_t*>(smem + L::mul);
     const uint32_t bar0 = sbase + L::bars;
-    // barriers: full[2] / empty[2] tile stages; pfull / pfree the P tile; d1 (MMA 1 done); pv (v', v'' written by the
-    // w lanes); d2 (MMA 2 done); s3 (MMA 3 done); sready (state copy published); odone (output rows read from TMEM)
-    const uint32_t bar_full = bar0, bar_empty = bar0 + 16, bar_pfull = bar0 + 32, bar_pfree = bar0 + 40, bar_d1 = bar0 + 48,
-                   bar_pv = bar0 + 56, bar_d2 = bar0 + 64, bar_s3 = bar0 + 72, bar_sready = bar0 + 80, bar_odone = bar0 + 88;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::bars + 128);
+    // barriers: full / empty of the two stages of [w;q] and of k, u; pfull (P has landed); d1, s3, d2 (MMA 1, 3, 2 done);
+    // pv (v', v'' written and the state written back); sready (state copy published); odone (output rows read from TMEM);
+    // ofull / ofree (output rows written to shared memory / stored)
+    const uint32_t bar_wq = bar0, bar_wq_free = bar0 + 16, bar_ku = bar0 + 32, bar_ku_free = bar0 + 48, bar_p = bar0 + 64,
+                   bar_d1 = bar0 + 72, bar_pv = bar0 + 80, bar_d2 = bar0 + 88, bar_s3 = bar0 + 96, bar_sready = bar0 + 104,
+                   bar_odone = bar0 + 112, bar_ofull = bar0 + 120, bar_ofree = bar0 + 128;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::bars + 192);
+    int* hs_slot = reinterpret_cast<int*>(smem + L::bars + 196);
 
     if (tid == 0) {
         for (int i = 0; i < 2; ++i) {
-            mbar_init(bar_full + 8 * i, 1);
-            mbar_init(bar_empty + 8 * i, 1);
+            mbar_init(bar_wq + 8 * i, 1);
+            mbar_init(bar_wq_free + 8 * i, 1);
+            mbar_init(bar_ku + 8 * i, 1);
+            mbar_init(bar_ku_free + 8 * i, WK_ROW_WARPS / 2);
         }
-        mbar_init(bar_pfull, 1);
-        mbar_init(bar_pfree, 1);
+        mbar_init(bar_p, 1);
         mbar_init(bar_d1, 1);
-        mbar_init(bar_pv, WK_EPI / 2);
+        mbar_init(bar_pv, WK_ROW_WARPS);
         mbar_init(bar_d2, 1);
         mbar_init(bar_s3, 1);
-        mbar_init(bar_sready, WK_EPI);
-        mbar_init(bar_odone, WK_EPI / 2);
+        mbar_init(bar_sready, WK_ROW_WARPS);
+        mbar_init(bar_odone, WK_ROW_WARPS / 2);
+        mbar_init(bar_ofull, WK_ROW_WARPS / 2);
+        mbar_init(bar_ofree, 1);
         mbar_fence_init();
+        *hs_slot = -1;
     }
     if (warp == 1) tmem_alloc(smem_u32(tmem_slot), WK_TMEM_COLS);
-    // ---- per-chunk metadata: selection, carry before the chunk, decay factor of the chunk's update
-    for (int c = tid; c < NT; c += WK_THREADS) {
-        m_sel[c] = types_i[(((long)b * TN + c) * HN + hn) * 2 + 1] != 0;
-        m_gl[c] = gcs[((long)b * T + min(c * 64 + 63, T - 1)) * H + h];
-    }
-    // the P operand is padded to 128 rows; rows 0-63 stay zero
-    for (int i = tid; i < 8192 / 16; i += WK_THREADS) reinterpret_cast<uint4*>(smem + L::pp)[i] = make_uint4(0, 0, 0, 0);
-    __syncthreads();
-    if (tid == 0) {
+    // ---- per-chunk scalars.  Every chunk adds up its own run of skipped chunks, first to last, as one thread would do for all.
+    {
+        float* gl = reinterpret_cast<float*>(smem + L::sbf);          // (overwritten by the initial state)
+        int* sel = reinterpret_cast<int*>(smem + L::sbf) + WK_MAX_NT;
+        for (int c = tid; c < NT; c += WK_THREADS) {
+            sel[c] = types_i[(((long)b * TN + c) * HN + hn) * 2 + 1] != 0;
+            gl[c] = gcs[((long)b * T + min(c * 64 + 63, T - 1)) * H + h];
+        }
         const int nsel = n_blocks[((long)b * HN + hn) * 2 + 1];
         const int last_sel = nsel > 0 ? indices[(((long)b * TN + (nsel - 1)) * HN + hn) * 2 + 1] : -1;
-        float carry = 0.f;
-        for (int c = 0; c < NT; ++c) {
-            const float gl = m_gl[c];
-            m_carry[c] = carry;
-            if (m_sel[c]) {
-                m_dec[c] = __expf(gl + carry);
-                carry = 0.f;
-            } else {
-                m_dec[c] = 1.f;
-                if (decay && (!trailing_quirk || c < last_sel)) carry += gl;
+        __syncthreads();
+        for (int c = tid; c < NT; c += WK_THREADS) {
+            float carry = 0.f;
+            if (decay) {
+                int j = c;
+                while (j > 0 && !sel[j - 1]) --j;
+                for (; j < c; ++j)
+                    if (!trailing_quirk || j < last_sel) carry += gl[j];
             }
+            m_carry[c] = carry;
+        }
+        __syncthreads();
+        for (int c = tid; c < NT; c += WK_THREADS) {
+            int j = c + 1;
+            while (j < NT && !sel[j]) ++j;
+            const float mul = j < NT ? __expf(gl[j] + m_carry[j]) : 1.f;
+            m_mul[c] = (__float_as_uint(mul) & 0x7fffffffu) | (sel[c] ? 0x80000000u : 0u);
+            if (sel[c] && c < NT - 1 && j >= NT - 1) *hs_slot = c;     // the last update in front of the last chunk
         }
     }
-    fence_async_smem();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    bool ok = true;
 
     if (warp == 0) {
-        // ------------------------------------------------------------ TMA producer
+        // ------------------------------------------------------------ loads of w, q and of k, u
         if (lane == 0) {
             prefetch_tensormap(&map_w); prefetch_tensormap(&map_q); prefetch_tensormap(&map_k);
-            prefetch_tensormap(&map_u); prefetch_tensormap(&map_p);
+            prefetch_tensormap(&map_u);
         }
+        int n_wq = 0, n_ku = 0;                           // chunks asked for
+#pragma unroll 1
         for (int c = 0; c < NT; ++c) {
-            const int stg = c & 1;
-            const int t0 = c * 64;
-            if (c >= 2) {
-                bool ok = mbar_wait_small(bar_empty + stg * 8, ((c >> 1) - 1) & 1, status);
-                if (!__all_sync(0xffffffffu, ok)) break;
-            }
+            const int stg = c & 1, t0 = c * 64;
+            const uint32_t par = ((c >> 1) - 1) & 1, base = sbase + stg * L::stage;
+            if (c >= 2) ok = warp_wait(bar_wq_free + stg * 8, par);
+            if (!ok) break;
             if (lane == 0) {
-                const uint32_t full = bar_full + stg * 8, base = sbase + stg * L::stage;
-                mbar_expect_tx(full, 65536);
+                const uint32_t full = bar_wq + stg * 8;
+                mbar_expect_tx(full, 32768);
 #pragma unroll
                 for (int sub = 0; sub < 2; ++sub) {
                     tma_load_4d(base + L::wq + sub * 16384, &map_w, sub * 64, h, t0, b, full);          // rows 0-63
                     tma_load_4d(base + L::wq + sub * 16384 + 8192, &map_q, sub * 64, h, t0, b, full);   // rows 64-127
-                    tma_load_4d(base + L::k + sub * 8192, &map_k, sub * 64, h, t0, b, full);
-                    tma_load_4d(base + L::u + sub * 8192, &map_u, sub * 64, h, t0, b, full);
                 }
             }
-            if (c >= 1) {
-                bool ok = mbar_wait_small(bar_pfree, (c - 1) & 1, status);       // P of the previous chunk consumed
-                if (!__all_sync(0xffffffffu, ok)) break;
-            }
+            __syncwarp();
+            ++n_wq;
+            if (c >= 2) ok = warp_wait(bar_ku_free + stg * 8, par);
+            if (!ok) break;
             if (lane == 0) {
-                mbar_expect_tx(bar_pfull, 8192);
-                tma_load_4d(sbase + L::pp + 8192, &map_p, 0, h, t0, b, bar_pfull);                      // rows 64-127
+                const uint32_t full = bar_ku + stg * 8;
+                mbar_expect_tx(full, 32768);
+#pragma unroll
+                for (int sub = 0; sub < 2; ++sub) {
+                    tma_load_4d(base + L::u + sub * 8192, &map_u, sub * 64, h, t0, b, full);
+                    tma_load_4d(base + L::k + sub * 8192, &map_k, sub * 64, h, t0, b, full);
+                }
             }
             __syncwarp();
+            ++n_ku;
+        }
+        if (!ok) {                                        // nothing may still be on its way into shared memory
+            for (int c = max(0, n_wq - 2); c < n_wq; ++c) warp_wait(bar_wq + (c & 1) * 8, (c >> 1) & 1);
+            for (int c = max(0, n_ku - 2); c < n_ku; ++c) warp_wait(bar_ku + (c & 1) * 8, (c >> 1) & 1);
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        constexpr uint32_t id_1 = umma_idesc_bf16(128, 128, true);                       // [w;q] S
-        constexpr uint32_t id_2 = umma_idesc_bf16(128, 128, true);                       // P v'
-        constexpr uint32_t id_3 = umma_idesc_bf16(128, 128, true) | (1u << 15);          // k^T v'' (A MN-major)
-        bool ok = true;
-        for (int c = 0; ok && c < NT; ++c) {
+        constexpr uint32_t id = umma_idesc_bf16(128, 128, true);                         // [w;q] S, P v'
+        constexpr uint32_t id_3 = id | (1u << 15);                                       // k^T v'' (A MN-major)
+#pragma unroll 1
+        for (int c = 0; c < NT; ++c) {
             const int stg = c & 1;
-            const uint32_t base = sbase + stg * L::stage;
-            ok = __all_sync(0xffffffffu, mbar_wait_small(bar_full + stg * 8, (c >> 1) & 1, status));
-            if (ok) ok = __all_sync(0xffffffffu, mbar_wait_small(bar_sready, c & 1, status));
+            const uint32_t base = sbase + stg * L::stage, par = (c >> 1) & 1;
+            const bool sel = (m_mul[c] >> 31) != 0;
+            ok = warp_wait(bar_wq + stg * 8, par);
+            if (ok) ok = warp_wait(bar_sready, c & 1);
             if (!ok) break;
-            const uint32_t d1 = tmem + ((c & 1) ? WK_D1B : WK_D1);
+            tc_fence_after();
             {
-                tc_fence_after();
+                const uint32_t d1 = tmem + ((c & 1) ? WK_D1B : WK_D1);
                 const uint32_t al = umma_desc_lo(base + L::wq, 16), bl = umma_desc_lo(sbase + L::sbf, 16384);
 #pragma unroll
-                for (int h = 0; h < 2; ++h) umma_ss_x4<2, 128>(d1, al + h * 1024, bl + h * 512, id_1, h > 0);
+                for (int e = 0; e < 2; ++e) umma_ss_x4<2, 128>(d1, al + e * 1024, bl + e * 512, id, e > 0);
                 umma_commit(bar_d1);
             }
-            __syncwarp();
-            ok = __all_sync(0xffffffffu, mbar_wait_small(bar_pv, c & 1, status));
+            // (k: the phase of its barrier stands still only while the chunk's update, which gives the stage back, is to come)
+            if (sel) ok = warp_wait(bar_ku + stg * 8, par);
+            if (ok) ok = warp_wait(bar_pv, c & 1);
             if (!ok) break;
-            {
-                // the state update first: the next chunk's products wait for it, the output does not
-                tc_fence_after();
-                if (m_sel[c]) {
-                    umma_ss_x4<128, 128>(tmem + WK_S, umma_desc_lo(base + L::k, 8192), umma_desc_lo(sbase + L::vs, 8192), id_3, 1u);
-                }
+            tc_fence_after();
+            // the state update first: the next chunk's products wait for it, the output does not
+            if (sel) {
+                umma_ss_x4<128, 128>(tmem + WK_S, umma_desc_lo(base + L::k, 8192), umma_desc_lo(sbase + L::vs, 8192), id_3, 1u);
                 umma_commit(bar_s3);
             }
-            __syncwarp();
-            ok = __all_sync(0xffffffffu, mbar_wait_small(bar_pfull, c & 1, status));
-            if (ok && c > 0) ok = __all_sync(0xffffffffu, mbar_wait_small(bar_odone, (c - 1) & 1, status));   // D2 is free
+            ok = warp_wait(bar_p, c & 1);
+            if (ok && c > 0) ok = warp_wait(bar_odone, (c - 1) & 1);                     // D2 is free
             if (!ok) break;
-            {
-                tc_fence_after();
-                umma_ss_x4<2, 128>(tmem + WK_D2, umma_desc_lo(sbase + L::pp, 16), umma_desc_lo(sbase + L::vp, 8192), id_2, 0u);
-                umma_commit(bar_d2);
-                umma_commit(bar_pfree);
-                umma_commit(bar_empty + stg * 8);
+            tc_fence_after();
+            umma_ss_x4<2, 128>(tmem + WK_D2, umma_desc_lo(sbase + L::pp - 8192, 16), umma_desc_lo(sbase + L::vp, 8192), id, 0u);
+            umma_commit(bar_d2);
+        }
+    } else if (warp == WK_ROW_WARPS + 2) {
+        // ------------------------------------------------------------ loads of P, stores of the outputs
+        int n_p = 0;                                      // tiles asked for
+#pragma unroll 1
+        for (int c = 0; c < NT; ++c) {
+            if (c > 0) ok = warp_wait(bar_d2, (c - 1) & 1);              // P of the chunk before is used up
+            if (!ok) break;
+            if (lane == 0) {
+                mbar_expect_tx(bar_p, 8192);
+                tma_load_4d(sbase + L::pp, &map_p, 0, h, c * 64, b, bar_p);
+            }
+            __syncwarp();
+            ++n_p;
+            if (c > 0) ok = warp_wait(bar_ofull, (c - 1) & 1);
+            if (!ok) break;
+            if (c > 0 && lane == 0) {
+                tma_store_4d(&map_o, sbase + L::out, 0, h, (c - 1) * 64, b);
+                tma_store_4d(&map_o, sbase + L::out + 8192, 64, h, (c - 1) * 64, b);
+                tma_store_commit();
+                tma_store_wait_read();
+                mbar_arrive(bar_ofree);
             }
             __syncwarp();
         }
+        if (!ok && n_p > 0) warp_wait(bar_p, (n_p - 1) & 1);
+        if (ok) ok = warp_wait(bar_ofull, (NT - 1) & 1);
+        if (ok && lane == 0) {
+            tma_store_4d(&map_o, sbase + L::out, 0, h, (NT - 1) * 64, b);
+            tma_store_4d(&map_o, sbase + L::out + 8192, 64, h, (NT - 1) * 64, b);
+            tma_store_commit();
+            tma_store_wait_read();
+        }
+        __syncwarp();
     } else {
-        // ------------------------------------------------------------ two threads per TMEM lane (64 columns each)
+        // ------------------------------------------------------------ four threads per TMEM lane (32 columns each)
         const int quad = warp & 3;
-        const int half = (warp - 2) >> 2;
         const int row = quad * 32 + lane;                 // TMEM lane: S row (k index); w row (0-63) or q row (64-127)
-        const int cb = half * 64;                         // this thread's first column
-        const uint32_t t_lane = tmem + ((uint32_t)(quad * 32) << 16);
-        const bool is_q = row >= 64;
+        const int cb = ((warp - 2) >> 2) * 32;            // this thread's first column
+        const uint32_t t_lane = tmem + ((uint32_t)(quad * 32) << 16) + cb;
+        const bool is_q = quad >= 2;
         const int tr = row & 63;                          // token row inside the chunk
-        bool ok = true;
-
-        // the state in front of the last chunk (with its carried decay), for a decoder that continues the sequence: it is
-        // the one published when no chunk from `c` up to the last one updates the state
-        float* hs_row = hstart ? hstart + (((long)b * H + h) * K + row) * V : nullptr;
-        auto starts_last = [&](int c) -> bool {
-            if (!hs_row) return false;
-            for (int j = c; j < NT - 1; ++j)
-                if (m_sel[j]) return false;
-            return true;
+        const int hs_at = *hs_slot;
+        // 16-byte pieces of this thread's columns: row `tr` of a [64][64] tile, row `row` of the state's copy
+        const uint32_t tile_row = (cb >> 6) * 8192 + tr * 128, copy_row = (cb >> 6) * 16384 + row * 128;
+        auto piece = [&](int i) -> uint32_t { return (uint32_t)((((cb & 63) >> 3) + i) ^ (lane & 7)) << 4; };
+        auto arrive = [&](uint32_t bar) {                 // behind the writes and TMEM accesses of the whole warp
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar);
         };
-        auto store_row = [&](float* dst, int c0, const uint32_t (&r)[32], float f) {
+
+        // the state in front of the last chunk (with its carried decay), for a decoder that continues the sequence
+        float* hs_row = hstart ? hstart + (((long)b * H + h) * K + row) * V + cb : nullptr;
+        auto store_row = [&](float* dst, const uint32_t (&r)[32], float f) {
 #pragma unroll
             for (int i = 0; i < 32; i += 4)
-                *reinterpret_cast<float4*>(dst + c0 + i) = make_float4(__uint_as_float(r[i]) * f, __uint_as_float(r[i + 1]) * f,
-                                                                      __uint_as_float(r[i + 2]) * f, __uint_as_float(r[i + 3]) * f);
+                *reinterpret_cast<float4*>(dst + i) = make_float4(__uint_as_float(r[i]) * f, __uint_as_float(r[i + 1]) * f,
+                                                                 __uint_as_float(r[i + 2]) * f, __uint_as_float(r[i + 3]) * f);
         };
-        // copies columns [cb, cb+64) of this lane's S row as bf16 into the shared copy and leaves S * mul in TMEM
-        auto publish_state = [&](float mul, const float* init_row, bool hs) {
-#pragma unroll 1
-            for (int c0 = cb; c0 < cb + 64; c0 += 32) {
-                uint32_t r[32];
-                if (init_row) {
+        // the state's row as bf16 into the shared copy (announced), then S * mul into TMEM
+        auto publish_state = [&](uint32_t (&r)[32], float mul, bool always, bool hs, float hs_decay) {
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(init_row[c0 + i]);
-                } else {
-                    tmem_ld32(t_lane + WK_S + c0, r);
-                    tmem_ld_wait();
-                }
+            for (int i = 0; i < 4; ++i) {
+                uint32_t w4[4];
 #pragma unroll
-                for (int cc = 0; cc < 4; ++cc) {
-                    uint32_t w4[4];
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        w4[i] = pack_bf16(__uint_as_float(r[cc * 8 + 2 * i]), __uint_as_float(r[cc * 8 + 2 * i + 1]));
-                    const int col = c0 + cc * 8;          // v column of this 16-byte chunk
-                    *reinterpret_cast<uint4*>(smem + L::sbf + (col >> 6) * 16384 + swz<128>(row, (col & 63) >> 3)) =
-                        make_uint4(w4[0], w4[1], w4[2], w4[3]);
-                }
-                if (hs) store_row(hs_row, c0, r, __expf(m_carry[NT - 1]));
-                if (mul != 1.f || init_row) {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * mul);
-                    tmem_st32(t_lane + WK_S + c0, r);
-                }
-            }
-            tmem_st_wait();
-        };
-        // decay factor of the next update at or after chunk c
-        auto next_dec = [&](int c) -> float {
-            for (int j = c; j < NT; ++j)
-                if (m_sel[j]) return m_dec[j];
-            return 1.f;
-        };
-        {   // initial state
-            const float* init = h0 ? h0 + (((long)b * H + h) * K + row) * V : nullptr;
-            if (init) {
-                publish_state(next_dec(0), init, starts_last(0));
-            } else {
-                const bool hs = starts_last(0);
-#pragma unroll 1
-                for (int c0 = cb; c0 < cb + 64; c0 += 32) {
-                    uint32_t r[32];
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) r[i] = 0u;
-                    tmem_st32(t_lane + WK_S + c0, r);
-                    if (hs) store_row(hs_row, c0, r, 1.f);
-                }
-                tmem_st_wait();
-                for (int i = 0; i < 8; ++i)
-                    *reinterpret_cast<uint4*>(smem + L::sbf + half * 16384 + swz<128>(row, i)) = make_uint4(0, 0, 0, 0);
+                for (int e = 0; e < 4; ++e) w4[e] = pack_bf16(__uint_as_float(r[i * 8 + 2 * e]), __uint_as_float(r[i * 8 + 2 * e + 1]));
+                *reinterpret_cast<uint4*>(smem + L::sbf + copy_row + piece(i)) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
             }
             fence_async_smem();
             tc_fence_before();
-            mbar_arrive(bar_sready);
+            arrive(bar_sready);
+            if (hs_row && hs) store_row(hs_row, r, hs_decay);
+            if (mul != 1.f || always) {
+#pragma unroll
+                for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * mul);
+                tmem_st32(t_lane + WK_S, r);
+                tmem_st_wait();
+            }
+            tc_fence_before();
+        };
+        {   // initial state; the rows of q have nothing else to add to the first chunk's update
+            uint32_t r[32];
+            const float* init = h0 ? h0 + (((long)b * H + h) * K + row) * V + cb : nullptr;
+#pragma unroll
+            for (int i = 0; i < 32; ++i) r[i] = init ? __float_as_uint(init[i]) : 0u;
+            float mul = 1.f;
+            if (init) {
+                int j = 0;
+                while (j < NT && !(m_mul[j] >> 31)) ++j;
+                if (j < NT) mul = __expf(gcs[((long)b * T + min(j * 64 + 63, T - 1)) * H + h] + m_carry[j]);
+            }
+            publish_state(r, mul, true, hs_at < 0, init ? __expf(m_carry[NT - 1]) : 1.f);
+            if (is_q) arrive(bar_pv);
         }
-        // per-row scalars of the chunk: cumsum g and the l2 norm factor (k rows for w lanes, q rows for q lanes)
-        auto load_scalars = [&](int c, float& gg, float& rr) {
+        // per-row scalars of the chunk: cumsum g (of the row and of the chunk's last token) and the l2 norm factor (k rows for w
+        // lanes, q rows for q lanes)
+        auto load_scalars = [&](int c, float& gg, float& rr, float& gl) {
             const int valid = min(64, T - c * 64);
             const long tok0 = (long)b * T + (long)c * 64;
             gg = gcs[(tok0 + min(tr, valid - 1)) * H + h];
+            gl = gcs[(tok0 + valid - 1) * H + h];
             const float* rs = is_q ? qrstd : krstd;
             rr = (tr < valid) ? rs[(tok0 + tr) * H + h] : 0.f;
         };
-        float g_cur, r_cur, g_nxt = 0.f, r_nxt = 0.f;
-        load_scalars(0, g_cur, r_cur);
+        int n_upd = 0;                                    // updates so far: phases of bar_s3
+        float g_cur, r_cur, gl_cur, g_nxt = 0.f, r_nxt = 0.f, gl_nxt = 0.f;
+        load_scalars(0, g_cur, r_cur, gl_cur);
 
-        for (int c = 0; c < NT; ++c) {
+#pragma unroll 1
+        for (int c = 0; ok && c < NT; ++c) {
             const int stg = c & 1;
-            const int valid = min(64, T - c * 64);
-            const long tok0 = (long)b * T + (long)c * 64;
-            unsigned char* stage = smem + stg * L::stage;
-            if (c + 1 < NT) load_scalars(c + 1, g_nxt, r_nxt);          // prefetch; consumed next iteration
+            const unsigned char* stage = smem + stg * L::stage;
+            if (c + 1 < NT) load_scalars(c + 1, g_nxt, r_nxt, gl_nxt);  // prefetch; consumed next iteration
             const float carry = m_carry[c];
-            const float gl = m_gl[c];
-            const bool sel = m_sel[c] != 0;
+            const uint32_t mulw = m_mul[c];
+            const bool sel = (mulw >> 31) != 0;
             const uint32_t t_d1 = t_lane + ((c & 1) ? WK_D1B : WK_D1);
-            // After a failed (bounded) wait the remaining work is skipped; the loop still runs to its end.
-            // Every lane first sees MMA 1 of this chunk complete: it was issued behind the previous phase of the
-            // "state published" barrier, so no thread can arrive on that barrier twice within one phase.
-            if (ok) ok = __all_sync(0xffffffffu, mbar_wait_small(bar_d1, c & 1, status));
+            uint32_t r[32];
             if (!is_q) {
-                // ---- w lanes: v' = u - e^{carry} w S ; v'' = v' rstd_k e^{g_last - g}   (the u tile arrived with the stage)
-                if (ok) {
-                    tc_fence_after();
-                    const float ec = __expf(carry);
-                    const float f2 = r_cur * __expf(fminf(gl - g_cur, 80.f));
-#pragma unroll 1
-                    for (int c0 = cb; c0 < cb + 64; c0 += 32) {
-                        uint32_t r[32];
-                        tmem_ld32(t_d1 + c0, r);
-                        tmem_ld_wait();
+                // ---- w lanes: v' = u - e^{carry} w S ; v'' = v' rstd_k e^{g_last - g}
+                const float ec = __expf(carry);
+                const float f2 = r_cur * __expf(fminf(gl_cur - g_cur, 80.f));
+                ok = warp_wait(bar_ku + stg * 8, (c >> 1) & 1);
+                if (!ok) break;
+                uint4 ux[4];
 #pragma unroll
-                        for (int cc = 0; cc < 4; ++cc) {
-                            const int col = c0 + cc * 8;
-                            const uint32_t off = (col >> 6) * 8192 + swz<128>(tr, (col & 63) >> 3);
-                            const uint4 ux = *reinterpret_cast<const uint4*>(stage + L::u + off);
-                            const uint32_t* uw = reinterpret_cast<const uint32_t*>(&ux);
-                            uint32_t a4[4], b4[4];
+                for (int i = 0; i < 4; ++i) ux[i] = *reinterpret_cast<const uint4*>(stage + L::u + tile_row + piece(i));
+                ok = warp_wait(bar_d1, c & 1);
+                if (!ok) break;
+                tc_fence_after();
+                tmem_ld32(t_d1, r);
+                tmem_ld_wait();
+                if (warp == 4 && lane == 0) mbar_arrive(bar_wq_free + stg * 8);          // MMA 1 has read the stage
 #pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                const float2 uf = unpack_bf16(uw[i]);
-                                const float v0 = uf.x - ec * __uint_as_float(r[cc * 8 + 2 * i]);
-                                const float v1 = uf.y - ec * __uint_as_float(r[cc * 8 + 2 * i + 1]);
-                                a4[i] = pack_bf16(v0, v1);
-                                b4[i] = pack_bf16(v0 * f2, v1 * f2);
-                            }
-                            *reinterpret_cast<uint4*>(smem + L::vp + off) = make_uint4(a4[0], a4[1], a4[2], a4[3]);
-                            *reinterpret_cast<uint4*>(smem + L::vs + off) = make_uint4(b4[0], b4[1], b4[2], b4[3]);
-                        }
+                for (int i = 0; i < 4; ++i) {
+                    const uint32_t* uw = reinterpret_cast<const uint32_t*>(&ux[i]);
+                    uint32_t a4[4], b4[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const float2 uf = unpack_bf16(uw[e]);
+                        const float v0 = uf.x - ec * __uint_as_float(r[i * 8 + 2 * e]);
+                        const float v1 = uf.y - ec * __uint_as_float(r[i * 8 + 2 * e + 1]);
+                        a4[e] = pack_bf16(v0, v1);
+                        b4[e] = pack_bf16(v0 * f2, v1 * f2);
                     }
-                    fence_async_smem();
-                    tc_fence_before();
-                    mbar_arrive(bar_pv);
+                    *reinterpret_cast<uint4*>(smem + L::vs + tile_row + piece(i)) = make_uint4(b4[0], b4[1], b4[2], b4[3]);
+                    *reinterpret_cast<uint4*>(smem + L::vp + tile_row + piece(i)) = make_uint4(a4[0], a4[1], a4[2], a4[3]);
                 }
-            }
-            // ---- every lane: publish the updated state for the next chunk (and pre-apply the next update's decay).
-            // This is the serial chain of the walk; the output rows below are read after it.
-            if (ok && sel) {
-                ok = __all_sync(0xffffffffu, mbar_wait_small(bar_s3, c & 1, status));
-                if (ok) {
-                    tc_fence_after();
-                    publish_state(next_dec(c + 1), nullptr, c < NT - 1 && starts_last(c + 1));
-                    fence_async_smem();
-                }
-            }
-            if (ok) {
+                fence_async_smem();
                 tc_fence_before();
-                mbar_arrive(bar_sready);
+                arrive(bar_pv);
+            } else {
+                ok = warp_wait(bar_d1, c & 1);
+                if (!ok) break;
             }
-            if (is_q) {
-                // ---- q lanes: o = scale (rstd_q e^{g+carry} q S + P v'), off the chain (D1 is double-buffered, D2 is
-                // released by the arrival below)
-                if (ok) ok = __all_sync(0xffffffffu, mbar_wait_small(bar_d2, c & 1, status));
-                if (ok) {
-                    tc_fence_after();
-                    const float fq = r_cur * __expf(g_cur + carry);
-                    __nv_bfloat16* orow = o + ((tok0 + tr) * H + h) * V;
-#pragma unroll 1
-                    for (int c0 = cb; c0 < cb + 64; c0 += 32) {
-                        uint32_t r1[32], r2[32];
-                        tmem_ld32(t_d1 + c0, r1);
-                        tmem_ld32(t_lane + WK_D2 + c0, r2);
-                        tmem_ld_wait();
-                        if (tr < valid) {
+            // ---- every lane: publish the updated state for the next chunk (and pre-apply the next update's decay).  This is the
+            // serial chain of the walk; the output rows are read after it.  (Every lane has seen MMA 1 of this chunk complete: it
+            // was issued behind the previous phase of the "state published" barrier, so no warp arrives on that barrier twice
+            // within one phase.)
+            if (sel) {
+                ok = warp_wait(bar_s3, n_upd & 1);
+                ++n_upd;
+                if (!ok) break;
+                tc_fence_after();
+                tmem_ld32(t_lane + WK_S, r);
+                tmem_ld_wait();
+                publish_state(r, __uint_as_float(mulw & 0x7fffffffu), false, c == hs_at, c == hs_at ? __expf(m_carry[NT - 1]) : 0.f);
+            } else {
+                tc_fence_before();
+                arrive(bar_sready);
+            }
+            if (!is_q) {
+                if (lane == 0) mbar_arrive(bar_ku_free + stg * 8);       // (u is in registers, MMA 3 has read k)
+            } else {
+                // ---- q lanes: o = scale (rstd_q e^{g+carry} q S + P v'), off the chain (D1 is double-buffered).  MMA 3 of the next
+                // chunk may add to the state once it is written back: with an update that has just happened; without one the
+                // arrival has to wait until the barrier's phase of this chunk is over, which MMA 2 tells.
+                if (sel && c + 1 < NT) arrive(bar_pv);
+                const float fq = r_cur * __expf(g_cur + carry);
+                ok = warp_wait(bar_d2, c & 1);
+                if (!ok) break;
+                if (!sel && c + 1 < NT) arrive(bar_pv);
+                tc_fence_after();
+                uint32_t r2[32];
+                tmem_ld32(t_d1, r);
+                tmem_ld32(t_lane + WK_D2, r2);
+                tmem_ld_wait();
+                tc_fence_before();
+                arrive(bar_odone);
+                if (c > 0) ok = warp_wait(bar_ofree, (c - 1) & 1);
+                if (!ok) break;
 #pragma unroll
-                            for (int cc = 0; cc < 4; ++cc) {
-                                uint32_t w4[4];
+                for (int i = 0; i < 4; ++i) {
+                    uint32_t w4[4];
 #pragma unroll
-                                for (int i = 0; i < 4; ++i) {
-                                    const int e = cc * 8 + 2 * i;
-                                    w4[i] = pack_bf16(scale * (fq * __uint_as_float(r1[e]) + __uint_as_float(r2[e])),
-                                                      scale * (fq * __uint_as_float(r1[e + 1]) + __uint_as_float(r2[e + 1])));
-                                }
-                                *reinterpret_cast<uint4*>(orow + c0 + cc * 8) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
-                            }
-                        }
+                    for (int e = 0; e < 4; ++e) {
+                        const int x = i * 8 + 2 * e;
+                        w4[e] = pack_bf16(scale * (fq * __uint_as_float(r[x]) + __uint_as_float(r2[x])),
+                                          scale * (fq * __uint_as_float(r[x + 1]) + __uint_as_float(r2[x + 1])));
                     }
-                    tc_fence_before();
-                    mbar_arrive(bar_odone);
+                    *reinterpret_cast<uint4*>(smem + L::out + tile_row + piece(i)) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
                 }
+                fence_async_smem();
+                arrive(bar_ofull);
             }
             g_cur = g_nxt;
             r_cur = r_nxt;
+            gl_cur = gl_nxt;
         }
         // every update's decay was pre-applied except after the last one: TMEM holds the final state.  A complete last
         // block: the decoder continues from it if that block's own type is linear, else from the state in front of the
@@ -400,24 +437,21 @@ gdn_walk_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         }
         if (ok && (ht || last_lin || last_roll)) {
             tc_fence_after();
-            float* hrow = ht ? ht + (((long)b * H + h) * K + row) * V : nullptr;
-            const float f = last_roll ? __expf(m_gl[NT - 1]) : 1.f;
-#pragma unroll 1
-            for (int c0 = cb; c0 < cb + 64; c0 += 32) {
-                uint32_t r[32];
-                tmem_ld32(t_lane + WK_S + c0, r);
-                tmem_ld_wait();
-                if (hrow) store_row(hrow, c0, r, 1.f);
-                if (last_lin) store_row(hs_row, c0, r, 1.f);
-                if (last_roll) {
+            float* hrow = ht ? ht + (((long)b * H + h) * K + row) * V + cb : nullptr;
+            uint32_t r[32];
+            tmem_ld32(t_lane + WK_S, r);
+            tmem_ld_wait();
+            if (hrow) store_row(hrow, r, 1.f);
+            if (last_lin) store_row(hs_row, r, 1.f);
+            if (last_roll) {
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(hs_row[c0 + i]);
-                    store_row(hs_row, c0, r, f);
-                }
+                for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(hs_row[i]);
+                store_row(hs_row, r, __expf(gcs[((long)b * T + T - 1) * H + h]));
             }
         }
     }
     // ---------------------------------------------------------------- teardown
+    if (!ok && lane == 0) atomicExch(status, NATSL_DEV_WAIT_TIMEOUT);
     tc_fence_before();
     __syncthreads();
     if (warp == 1) tmem_dealloc(tmem, WK_TMEM_COLS);
@@ -441,26 +475,28 @@ extern "C" int natsl_gdn_walk_fused_ex(const void* q, const void* k, const void*
     NATSL_REQUIRE(H <= 65535 && B <= 65535, NATSL_ERR_TOO_LARGE, "natsl_gdn_walk_fused: B, H <= 65535");
     NATSL_REQUIRE(!hstart || T % nbs != 0 || (last_types && (last_dtype == NATSL_DT_F32 || last_dtype == NATSL_DT_BF16)),
                   NATSL_ERR_NULL, "natsl_gdn_walk_fused: the block-start state of a complete last block needs that block's types");
-    auto kern = gdn_walk_tc_kernel<true>;
+    auto kern = gdn_walk_tc_kernel;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, WkSmem::total);
     if (e != cudaSuccess) {
         set_error("natsl_gdn_walk_fused: cannot reserve %d B of shared memory (%s)", WkSmem::total, cudaGetErrorString(e));
         return NATSL_ERR_CUDA;
     }
-    CUtensorMap mw, mq, mk, mu, mp;
+    CUtensorMap mw, mq, mk, mu, mp, mo;
     int rc = encode_bthd_map(&mw, w, B, T, H, K, 64, "natsl_gdn_walk_fused(w)");
     if (rc == NATSL_OK) rc = encode_bthd_map(&mq, q, B, T, H, K, 64, "natsl_gdn_walk_fused(q)");
     if (rc == NATSL_OK) rc = encode_bthd_map(&mk, k, B, T, H, K, 64, "natsl_gdn_walk_fused(k)");
     if (rc == NATSL_OK) rc = encode_bthd_map(&mu, u, B, T, H, V, 64, "natsl_gdn_walk_fused(u)");
     if (rc == NATSL_OK) rc = encode_bthd_map(&mp, pmat, B, T, H, 64, 64, "natsl_gdn_walk_fused(P)");
+    if (rc == NATSL_OK) rc = encode_bthd_map(&mo, o, B, T, H, V, 64, "natsl_gdn_walk_fused(o)");
     int* status = nullptr;
     if (rc == NATSL_OK) rc = status_word_ptr(&status);
     if (rc != NATSL_OK) return rc;
     const int TN = (T + nbs - 1) / nbs;
     dim3 grid(H, B);
     kern<<<grid, WK_THREADS, WkSmem::total, reinterpret_cast<cudaStream_t>(stream)>>>(
-        mw, mq, mk, mu, mp, gcs, k_rstd, q_rstd, types_i, indices, n_blocks, h0, reinterpret_cast<__nv_bfloat16*>(o), ht, hstart,
-        last_types, last_dtype == NATSL_DT_F32, last_stride, T, H, HN, TN, scale, (flags & NATSL_FLAG_DECAY_SKIPPED) ? 1 : 0, (flags & NATSL_FLAG_NO_TRAILING_QUIRK) ? 0 : 1, status);
+        mw, mq, mk, mu, mp, mo, gcs, k_rstd, q_rstd, types_i, indices, n_blocks, h0, ht, hstart, last_types,
+        last_dtype == NATSL_DT_F32, last_stride, T, H, HN, TN, scale, (flags & NATSL_FLAG_DECAY_SKIPPED) ? 1 : 0,
+        (flags & NATSL_FLAG_NO_TRAILING_QUIRK) ? 0 : 1, status);
     return check_launch("natsl_gdn_walk_fused");
 }
 

@@ -52,6 +52,12 @@ def test_walk_outputs_and_states(K, V, T, nbs, H, HN, decay, use_h0, tc, wide, m
     assert _lib.load().natsl_device_status() == 0
 
 
+@pytest.mark.parametrize("T,decay", [(1, True), (63, True), (65, True), (127, False), (128, True), (1100, True)])
+def test_tc_walk_at_chunk_edges(T, decay, monkeypatch):
+    """The tcgen05 walk stores whole chunks by TMA, which clips the last one, and every chunk adds up its own run of skipped ones."""
+    test_walk_outputs_and_states(128, 128, T, 64, 3, 3, decay, True, True, False, monkeypatch)
+
+
 @pytest.mark.parametrize("T,nbs,decay", [(64, 64, True), (300, 64, True), (512, 128, False), (640, 256, True)])
 def test_mamba_walk_block_start_state(T, nbs, decay):
     import neuralattentionsearchlinear_b200 as nat
