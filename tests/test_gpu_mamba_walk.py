@@ -75,6 +75,21 @@ def test_walk_state_only_and_reproducible(nat):
     assert_close(ht_s, ht_s2, 2 * TOL, "state-only: fused walk vs scan")
 
 
+@pytest.mark.parametrize("T,nbs,decay", [(1, 64, True), (63, 128, True), (65, 64, False), (129, 64, True), (193, 128, True)])
+def test_walk_at_chunk_edges(nat, T, nbs, decay):
+    """One chunk (the warps of the odd ones idle), odd and even numbers of them, a last token alone; without an output too."""
+    B, H, K, V = 2, 3, 128, 64
+    q, k, v, g, h0 = synth_mamba_inputs(B, T, H, K, V, seed=T)
+    types = otab.synth_types(B, -(-T // nbs), H, 0.5, seed=T)
+    (o, ht), _ = _both(nat, q, k, v, g, h0, types, T, nbs, decay)
+    o_ref, s_ref = ogdn.linear_chunk(q.float(), k.float(), v.float(), g, None, types[..., 1], nbs=nbs, scale=1.0, h0=h0,
+                                     decay=decay, use_l2norm=False, rule="mamba")
+    assert_close(o, o_ref, TOL, "o")
+    assert_close(ht, s_ref, 2 * TOL, "final state")
+    (_, ht_s), _ = _both(nat, q, k, v, g, h0, types, T, nbs, decay, skip_out=True)
+    assert torch.equal(ht_s, ht)
+
+
 def test_walk_without_the_trailing_quirk(nat):
     B, T, H, K, V, nbs = 1, 768, 2, 128, 64, 64
     q, k, v, g, h0 = synth_mamba_inputs(B, T, H, K, V, seed=9)
