@@ -122,6 +122,18 @@ def test_virtual_types_layout():
     assert t2[1, :, 1, 0].tolist() == [0, 0, 0, 0, 0, 0, 1, 0, 0, 0, 0]
 
 
+def test_one_rank_splits():
+    """Whole blocks and 128-token tiles, sequences the walk takes, no cut where the heads alone fill the SMs."""
+    from neuralattentionsearchlinear_b200.sequence_parallel import one_rank_splits
+    for L in (128, 1024, 3072, 4096, 49152, 65536, 131072, 1100):
+        for nbs in (64, 128, 256):
+            for units in (1, 4, 16, 32, 100, 148, 256):
+                s = one_rank_splits(L, nbs, units)
+                assert s == 1 if L % max(nbs, 128) else L % (s * max(nbs, 128)) == 0 and L // s <= 65536
+    assert one_rank_splits(65536, 256, 32) * 32 == 128 and one_rank_splits(8192, 64, 16) * 16 == 128
+    assert one_rank_splits(65536, 64, 148) == 1 and one_rank_splits(1024, 64, 32) == 1
+
+
 def test_pick_linear_splits():
     from neuralattentionsearchlinear_b200.sequence_parallel import pick_linear_splits
     assert pick_linear_splits(65536, 256) == 64
