@@ -5,16 +5,15 @@
 // the gradients are dq = scale * ds k, dk = scale * ds^T q, dv = p^T do.
 //
 // Two kernels on the 5th-generation tensor cores, both deterministic (no atomics; every reduction has a fixed order).
-// Warp roles as in the forward (320 threads): warp 0 TMA producer, warp 1 MMA issuer, warps 2-9 softmax with 16 query
-// rows each, four threads per row.  All score tiles are 128 queries x 64 keys with the queries in the TMEM lanes.
-//   attn_bwd_dq_kernel    one CTA per (128 queries, query head), two per SM: walks the visible 64-key tiles, dq stays in
-//                         TMEM; also writes delta (the preprocess kernel of the reference folded in).  ds goes back to
-//                         TMEM (over do.v) as the A operand of ds k.
-//   attn_bwd_dkdv_kernel  one CTA per two selected 64-key tiles of a key/value head (walks the 128-query tiles that see
-//                         either) or per eight unselected ones (own blocks only); accumulates dk^T and dv^T (head dim in
-//                         the lanes, keys in the columns) of two key tiles in TMEM; p and ds go to shared memory as the B
-//                         operands of do^T p and q^T ds.  It also sums ds over the later blocks' queries: the reference's
-//                         `dnats` column for the softmax branch (attns.py:922, 975-978), per (64-key tile, query head).
+//   attn_bwd_dq_kernel    one CTA per (128 queries, query head), two per SM, warp roles as in the forward (320 threads: TMA
+//                         producer, MMA issuer, eight softmax warps with 16 query rows each, four threads per row): walks the
+//                         visible 64-key tiles, queries in the TMEM lanes, dq stays in TMEM; also writes delta (the preprocess
+//                         kernel of the reference folded in).  ds goes back to TMEM (over do.v) as the A operand of ds k.
+//   attn_bwd_dkdv_kernel  pairs of 64-key tiles (two of selected blocks, or what is unselected of two neighbours) against the
+//                         128-query tiles that see either, keys in the TMEM lanes: k q^T and v do^T (128 x 128), p and ds back
+//                         into TMEM as the A operands of dv += p do and dk += ds q.  It also sums ds over the later blocks'
+//                         queries: the reference's `dnats` column for the softmax branch (attns.py:922, 975-978), per (64-key
+//                         tile, query head).
 // `compat` reproduces the reference's default backward, which drops every own-block entry of ds and p
 // (attns.py:590-591, 631-633, 842, 884 with the flag passed at mixed_attn_gdn.py:237) while lse and delta still
 // come from the full forward.
@@ -319,576 +318,652 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
 }
 
 // ------------------------------------------------------------------------------------------------- dk, dv
+// With the keys in the lanes all four products are 128 x 128 (x head dim): their operands are read half as often as by 128 x 64 ones
+// with p and ds in shared memory, p and ds need no shared memory at all, and a query tile is loaded once for two key tiles.
+// Results of a tile that the queries at hand do not see are kept out by the products' lane mask, whatever the queries hold.
+// One persistent CTA per SM takes blocks of the grid over (cluster launch control); a planning warp works out their steps, and
+// lse and delta of the queries, while the others are at the steps before.  Roles: warp 0 loads, warp 1 issues the products, warps 2-9
+// p and ds (a key and 64 queries per thread), warp 10 plans.
+// What bounds it: the chain scores -> p -> dv product and do.v -> ds -> dk product of a step, 3.5 k cycles against 2 k of the tensor
+// core (tensor memory holds one step: 128 columns each of scores, do.v, dk and dv), and 64 KB of q and do from L2 a step.
+// Alone (us; before: 128 x 64 score tiles, p and ds through shared memory, one CTA per pair of tiles), block 64:
+//   128/128, B = 8, T = 4096, H = 16: 25 % selected 678 -> 389, 50 % 1069 -> 607, 2 % 338 -> 194;  64/64, 30 %: 630 -> 369
+//   128/64, B = 4, T = 1000, H = 16, 50 %: 72 -> 44;  128/128, B = 1, T = 2048, H = 16, 30 %: 65 -> 43
+//   64/128, B = 2, T = 2048, 12 heads over 6, block 128, 40 %: 113 -> 67;  the smallest, B = 2, T = 64, H = 4: 8.5 -> 9.6
+constexpr int BKV_THREADS = 352;                              // TMA, MMA, 8 softmax warps, planner
 constexpr int BKV_MAXG = 16;
+constexpr int BKV_DESCS = 4;
 template <int DK, int DV>
 struct DkvSmem {
-    // A stage is [do | q], both as [128][64] sub-tiles.  With a head dim of 64 the M = 128 products read the 64 columns
-    // behind the tile as well (the next sub-tile, always inside the buffers) and those result rows are never used.
-    static constexpr int stage_bytes = 128 * (DK + DV) * 2;
-    static constexpr int stage = 0;                           // 2 stages
-    static constexpr int kv = stage + 2 * stage_bytes;        // per key tile: DK/64 + DV/64 sub-tiles [64][64]
-    static constexpr int kv_bytes = 64 * (DK + DV) * 2;
-    static constexpr int p = kv + 2 * kv_bytes;               // p [128 queries][64 keys]
-    static constexpr int ds = p + 16384;                      // ds, same layout
-    static constexpr int dn = ds + 16384;                     // dnats parts [2 tiles][16 heads][8 warps]
-    static constexpr int last = dn + 2 * BKV_MAXG * 8 * 4;    // last query tile [2 tiles][16 heads]
-    static constexpr int tiles = last + 2 * BKV_MAXG * 4;     // key tiles of this CTA [8]
-    static constexpr int bars = tiles + 32;
-    static constexpr int total = bars + 96;
+    static constexpr int kv = 0;                              // k: DK/64 sub-tiles [128 keys][64], then v the same way
+    static constexpr int q = kv + 128 * (DK + DV) * 2;        // 2 stages x DK/64 sub-tiles [128 queries][64]
+    static constexpr int dos = q + 2 * 128 * DK * 2;          // 2 stages x DV/64 sub-tiles
+    static constexpr int out = dos + 2 * 128 * DV * 2;        // per softmax warp: 32 rows x 64 columns on their way out
+    static constexpr int stat = out + 8 * 4096;               // 2 x (-lse, -delta) of 128 queries
+    static constexpr int dn = stat + 2 * 1024;                // dnats parts [2 tiles][16 heads][4 warps]
+    static constexpr int desc = dn + 2 * BKV_MAXG * 4 * 4;    // steps, 32 bytes each
+    static constexpr int last = desc + BKV_DESCS * 32;        // last query tile [2 tiles][16 heads] of a selected pair
+    static constexpr int clc = last + 2 * BKV_MAXG * 2;       // answer of the take-over request
+    static constexpr int bars = clc + 16;
+    static constexpr int total = bars + 240;
     static_assert(total <= 227 * 1024, "one CTA per SM");
 };
 
-// What a CTA walks: for every query head of the group the query tiles that see either key tile, and inside a query
-// tile the key tiles that it sees.  All roles step through the same sequence.
-struct DkvWalk {
-    const int* last;                                          // shared memory [2][16]; -1: no query tile
-    int first[2];
-    int G;
-    int gi, qt, u;
-    __device__ __forceinline__ bool active(int uu) const { return qt >= first[uu] && qt <= last[uu * BKV_MAXG + gi]; }
-    __device__ __forceinline__ void enter() {                 // first query tile of head gi
-        const int l0 = last[gi], l1 = last[BKV_MAXG + gi];
-        qt = min(l0 >= first[0] ? first[0] : 0x7fffffff, l1 >= first[1] ? first[1] : 0x7fffffff);
-        u = 0;
-    }
-    // moves to the first (gi, qt, u) at or after the current one; false at the end
-    __device__ __forceinline__ bool settle() {
-#pragma unroll 1
-        while (gi < G) {
-            const int hi = max(last[gi], last[BKV_MAXG + gi]);
-#pragma unroll 1
-            for (; qt <= hi; ++qt, u = 0) {
-                if (u == 0 && active(0)) return true;
-                if (u <= 1 && active(1)) {
-                    u = 1;
-                    return true;
-                }
-            }
-            if (++gi < G) enter();
-        }
-        return false;
-    }
-    __device__ __forceinline__ bool begin() {
-        gi = 0;
-        enter();
-        return settle();
-    }
-    __device__ __forceinline__ bool next() {
-        ++u;
-        return settle();
-    }
-    __device__ __forceinline__ bool next_query() {
-        u = 2;
-        return settle();
-    }
-    __device__ __forceinline__ bool first_of_query() const { return u == 0 || !active(0); }
-    __device__ __forceinline__ bool last_of_query() const { return u == 1 || !active(1); }
-};
-
-// The key tiles of unselected blocks, one after the other: only queries of their own block see them.
-constexpr int BKV_OWN = 8;                                    // tiles per CTA
-struct OwnWalk {
-    const volatile int* tiles;
-    int n, G, nbs, NTq;
-    int u, gi, qt, last;
-    __device__ __forceinline__ void enter() {
-        const int k0 = tiles[u] * 64;
-        qt = k0 / ATT_BM;
-        last = min(((k0 / nbs + 1) * nbs - 1) / ATT_BM, NTq - 1);
-    }
-    __device__ __forceinline__ bool begin() {
-        u = gi = 0;
-        if (n > 0) enter();
-        return n > 0;
-    }
-    __device__ __forceinline__ bool next() {
-        if (++qt > last) {
-            if (++gi == G) {
-                gi = 0;
-                if (++u == n) return false;
-            }
-            enter();
-        }
-        return true;
-    }
-    __device__ __forceinline__ bool first_of_tile() const { return gi == 0 && qt == tiles[u] * 64 / ATT_BM; }
+// What a CTA does in a step, worked out by the planner: first query, flags, query head of the group, head whose sums of ds are
+// complete (BKV_FLUSH); the two key tiles (-1: none), key head, batch.
+enum : int {
+    BKV_ACT0 = 1, BKV_ACT1 = 2,                               // the queries see the first / second key tile of the pair
+    BKV_SEL0 = 4, BKV_SEL1 = 8,                               // the head selected the tile's block
+    BKV_FIRST = 16, BKV_LAST = 32,                            // first / last step of the pair
+    BKV_EMPTY = 64, BKV_STOP = 128,                           // no query sees either tile; no pair is left
+    BKV_FLUSH = 256, BKV_ANY0 = 512, BKV_ANY1 = 1024,         // some query sees the first / second tile
+    BKV_SUMS = 2048                                           // a pair of selected tiles: sums of ds for it
 };
 
 // Heads whose CTAs are interleaved, heaviest first: the last CTAs to start are then light ones, and q and do of that many
 // heads (2 MB each at 4096 x 128) stay in L2 for the CTAs of a head that run at the same time.
 constexpr int BKV_HEADS = 32;
 
+// Four K-steps, A from tensor memory, results added in the lanes whose bit is not set: m01 for lanes 0-63, m23 for lanes 64-127.
+template <int STEP_B>
+__device__ __forceinline__ void umma_ts_x4_lanes(uint32_t d_tmem, uint32_t a_tmem, uint32_t blo, uint32_t idesc, uint32_t m01, uint32_t m23) {
+    asm volatile(
+        "{\n .reg .pred t, e;\n .reg .b64 b;\n .reg .b32 x, y;\n"
+        " setp.eq.u32 t, 0, 0;\n elect.sync _|e, 0xffffffff;\n"
+        " mov.b64 b, {%2, %4};\n"
+        " @e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %3, {%6, %6, %7, %7}, t;\n"
+        " add.u32 x, %1, 8;\n add.u32 y, %2, %5;\n mov.b64 b, {y, %4};\n"
+        " @e tcgen05.mma.cta_group::1.kind::f16 [%0], [x], b, %3, {%6, %6, %7, %7}, t;\n"
+        " add.u32 x, x, 8;\n add.u32 y, y, %5;\n mov.b64 b, {y, %4};\n"
+        " @e tcgen05.mma.cta_group::1.kind::f16 [%0], [x], b, %3, {%6, %6, %7, %7}, t;\n"
+        " add.u32 x, x, 8;\n add.u32 y, y, %5;\n mov.b64 b, {y, %4};\n"
+        " @e tcgen05.mma.cta_group::1.kind::f16 [%0], [x], b, %3, {%6, %6, %7, %7}, t;\n}\n"
+        ::"r"(d_tmem), "r"(a_tmem), "r"(blo), "r"(idesc), "n"(UMMA_DESC_HI), "n"(STEP_B), "r"(m01), "r"(m23)
+        : "memory");
+}
+
 template <int DK, int DV>
-__global__ void __launch_bounds__(TC_THREADS, 1)
+__global__ void __launch_bounds__(BKV_THREADS, 1)
 attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                      const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
+                     const __grid_constant__ CUtensorMap map_dk, const __grid_constant__ CUtensorMap map_dv,
                      const float* __restrict__ lse, const float* __restrict__ delta, const int* __restrict__ types_i,
-                     __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv, float* __restrict__ dnats_part, int T, int HQ,
-                     int HKV, int HN, int TN, int nbs, float scale, int own, int heads, int ctas_per_head, int* status) {
+                     float* __restrict__ dnats_part, int T, int HQ, int HKV, int HN, int TN, int nbs, float scale, int own, int heads,
+                     int ctas_per_head, int* status) {
     using L = DkvSmem<DK, DV>;
-    // TMEM: scores 2 x 64 columns, do.v 2 x 64, then two accumulator pairs dv^T (64), dk^T (64)
-    constexpr uint32_t C_S = 0, C_DP = 128, C_ACC = 256;
+    // TMEM: scores [128 keys][128 queries], then p over each half's first columns; do.v, then ds; dv; dk
+    constexpr uint32_t C_S = 0, C_DP = 128, C_DV = 256, C_DK = 384;
+    constexpr int NB = (DK + DV) / 64;                        // 64-column blocks of results: dv, then dk
     extern __shared__ __align__(1024) unsigned char smem[];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const uint32_t sbase = smem_u32(smem);
     if ((sbase & 1023u) != 0) {
         if (tid == 0) atomicExch(status, 2);
         return;
     }
-    const int hbase = (int)blockIdx.x / (BKV_HEADS * ctas_per_head) * BKV_HEADS, hcount = min(BKV_HEADS, heads - hbase);
-    const int within = (int)blockIdx.x - hbase * ctas_per_head;
-    const int item = within / hcount, head = hbase + within % hcount;
-    const int hkv = head % HKV, b = head / HKV;
     const int G = HQ / HKV, cpb = nbs / 64;
     const int NT = (T + 63) / 64, NTq = (T + ATT_BM - 1) / ATT_BM;
     float* s_dn = reinterpret_cast<float*>(smem + L::dn);
-    int* s_last = reinterpret_cast<int*>(smem + L::last);
-    volatile int* s_tile = reinterpret_cast<volatile int*>(smem + L::tiles);
+    int4* s_desc = reinterpret_cast<int4*>(smem + L::desc);
+    volatile int16_t* s_last = reinterpret_cast<volatile int16_t*>(smem + L::last);
     const uint32_t bar0 = sbase + L::bars;
-    const uint32_t bar_full = bar0, bar_empty = bar0 + 16, bar_kv = bar0 + 32, bar_s = bar0 + 48, bar_p = bar0 + 64, bar_acc = bar0 + 72;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::bars + 80);
-    volatile int* s_nsel = reinterpret_cast<volatile int*>(smem + L::bars + 84);
+    // barriers: desc_full / desc_empty (steps); st_full / st_empty (lse and delta); q_full / q_empty, do_full / do_empty (stages);
+    // kv_full / kv_empty; s, dp (scores, do.v complete); p, ds (written by the softmax warps); acc (dk, dv of the pair complete);
+    // acc_free (read and set to zero)
+    const uint32_t desc_full = bar0, desc_empty = bar0 + 32, st_full = bar0 + 64, st_empty = bar0 + 80, q_full = bar0 + 96,
+                   q_empty = bar0 + 112, do_full = bar0 + 128, do_empty = bar0 + 144, kv_full = bar0 + 160, kv_empty = bar0 + 168,
+                   bar_s = bar0 + 176, bar_dp = bar0 + 184, bar_p = bar0 + 192, bar_ds = bar0 + 200, bar_acc = bar0 + 208,
+                   bar_acc_free = bar0 + 216, bar_clc = bar0 + 224;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::bars + 232);
+    auto arrive = [&](uint32_t bar) {                         // behind what the whole warp has done so far
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar);
+    };
 
     if (tid == 0) {
-        for (int i = 0; i < 2; ++i) {
-            mbar_init(bar_full + 8 * i, 1);
-            mbar_init(bar_empty + 8 * i, 1);
-            mbar_init(bar_kv + 8 * i, 1);
-            mbar_init(bar_s + 8 * i, 1);
+        for (int i = 0; i < BKV_DESCS; ++i) {
+            mbar_init(desc_full + 8 * i, 1);
+            mbar_init(desc_empty + 8 * i, 10);                // eight softmax warps, TMA, MMA
         }
-        mbar_init(bar_p, 8);                                  // one arrival per softmax warp
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(st_full + 8 * i, 1);
+            mbar_init(st_empty + 8 * i, 8);
+            mbar_init(q_full + 8 * i, 1);
+            mbar_init(q_empty + 8 * i, 1);
+            mbar_init(do_full + 8 * i, 1);
+            mbar_init(do_empty + 8 * i, 1);
+        }
+        mbar_init(kv_full, 1);
+        mbar_init(kv_empty, 1);
+        mbar_init(bar_s, 1);
+        mbar_init(bar_dp, 1);
+        mbar_init(bar_p, 8);
+        mbar_init(bar_ds, 8);
         mbar_init(bar_acc, 1);
+        mbar_init(bar_acc_free, 8);
+        mbar_init(bar_clc, 1);
         mbar_fence_init();
     }
-    for (int i = tid; i < 2 * BKV_MAXG * 8; i += TC_THREADS) s_dn[i] = 0.f;
-    if (warp == 2) {
-        // Key tiles in the order: those of selected blocks (of any head of the group), then the others.  The first
-        // ceil(n / 2) CTAs of a head take two selected tiles each: neighbours see nearly the same queries, so the pair
-        // shares the loads of q and do (64 KB per 128 x 64 scores of one tile).  The next ones take eight unselected
-        // tiles, the rest of the CTAs have nothing to do.
-        auto selected = [&](int kt) -> bool {
-            bool s = false;
-#pragma unroll 1
-            for (int gi = 0; gi < G; ++gi) s |= types_i[(((long)b * TN + kt / cpb) * HN + (hkv * G + gi) / (HQ / HN)) * 2] != 0;
-            return s;
-        };
-        constexpr int KEEP = 4;                               // ballots kept from the counting pass (8192 tokens)
-        unsigned kept[KEEP];
-        int n_sel = 0;
-#pragma unroll
-        for (int i = 0; i < KEEP; ++i) {
-            kept[i] = __ballot_sync(0xffffffffu, i * 32 + lane < NT && selected(i * 32 + lane));
-            n_sel += __popc(kept[i]);
-        }
-#pragma unroll 1
-        for (int base = KEEP * 32; base < NT; base += 32)
-            n_sel += __popc(__ballot_sync(0xffffffffu, base + lane < NT && selected(base + lane)));
-        const int n_pairs = (n_sel + 1) / 2;
-        const bool mine_sel = item < n_pairs;
-        const int r0 = mine_sel ? 2 * item : (item - n_pairs) * BKV_OWN;
-        const int want = mine_sel ? 2 : BKV_OWN;              // ranks [r0, r0 + want) among the tiles of that kind
-        if (lane < BKV_OWN) s_tile[lane] = -1;
-        __syncwarp();
-        int cnt = 0;
-        auto place = [&](int base, unsigned ms) {
-            const unsigned in = base + 32 <= NT ? 0xffffffffu : (1u << (NT - base)) - 1;
-            const unsigned m = mine_sel ? ms : in & ~ms;
-            const int r = cnt + __popc(m & ((1u << lane) - 1)) - r0;
-            if (((m >> lane) & 1) && r >= 0 && r < want) s_tile[r] = base + lane;
-            cnt += __popc(m);
-        };
-#pragma unroll
-        for (int i = 0; i < KEEP; ++i)
-            if (i * 32 < NT) place(i * 32, kept[i]);
-#pragma unroll 1
-        for (int base = KEEP * 32; base < NT && cnt < r0 + want; base += 32)
-            place(base, __ballot_sync(0xffffffffu, base + lane < NT && selected(base + lane)));
-        __syncwarp();
-        if (lane == 0) *s_nsel = n_sel;
-        // query tiles [first, last] of every (selected tile, head): the own block's from the keys on, the later ones if the
-        // head selected the block
-#pragma unroll 1
-        for (int i = lane; mine_sel && i < 2 * BKV_MAXG; i += 32) {
-            const int kt = s_tile[i / BKV_MAXG], gi = i % BKV_MAXG;
-            int last = -1;
-            if (kt >= 0 && gi < G) {
-                const int blk = kt / cpb, blk_end = (blk + 1) * nbs;
-                const bool s = G == 1 || types_i[(((long)b * TN + blk) * HN + (hkv * G + gi) / (HQ / HN)) * 2] != 0;
-                if (s && blk_end < T) last = NTq - 1;
-                else if (own) last = min((blk_end - 1) / ATT_BM, NTq - 1);
-            }
-            s_last[i] = last;
-        }
-    }
-    __syncthreads();
-    const int n_pairs = (*s_nsel + 1) / 2;
-    const bool paired = item < n_pairs;
-    if (s_tile[0] < 0) return;                                // no tile of either kind is left for this CTA
+    for (int i = tid; i < 2 * BKV_MAXG * 4; i += BKV_THREADS) s_dn[i] = 0.f;
     if (warp == 1) tmem_alloc(smem_u32(tmem_slot), 512);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
-    const int tile[2] = {s_tile[0], s_tile[1]};
-    int n_own = 0;
-    while (n_own < BKV_OWN && s_tile[n_own] >= 0) ++n_own;
-    DkvWalk w;
-    w.last = s_last;
-    w.G = G;
-#pragma unroll
-    for (int u = 0; u < 2; ++u) w.first[u] = tile[u] < 0 ? NTq : own ? tile[u] * 64 / ATT_BM : ((tile[u] / cpb + 1) * nbs) / ATT_BM;
-    auto has_items = [&](int u) -> bool {
-#pragma unroll 1
-        for (int gi = 0; gi < G; ++gi)
-            if (s_last[u * BKV_MAXG + gi] >= w.first[u]) return true;
-        return false;
-    };
-    OwnWalk ow;
-    ow.tiles = s_tile;
-    ow.n = own ? n_own : 0;
-    ow.G = G;
-    ow.nbs = nbs;
-    ow.NTq = NTq;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     bool ok = true;
+    int n_step = 0;                                           // steps taken over
+    int4 d, loc;                                              // the step's words
+    auto next_step = [&]() -> int {                           // its flags
+        const int slot = n_step & (BKV_DESCS - 1);
+        ok = warp_wait(desc_full + slot * 8, (n_step / BKV_DESCS) & 1);
+        d = s_desc[2 * slot];
+        loc = s_desc[2 * slot + 1];
+        d.y = ok ? __shfl_sync(0xffffffffu, d.y, 0) : BKV_STOP;
+        arrive(desc_empty + slot * 8);
+        ++n_step;
+        return d.y;
+    };
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
-        auto load_kv = [&](int slot, int kt, uint32_t bar) {
-            const uint32_t dst = sbase + L::kv + slot * L::kv_bytes;
-#pragma unroll
-            for (int sub = 0; sub < DK / 64; ++sub) tma_load_4d(dst + sub * 8192, &map_k, sub * 64, hkv, kt * 64, b, bar);
-#pragma unroll
-            for (int sub = 0; sub < DV / 64; ++sub)
-                tma_load_4d(dst + 64 * DK * 2 + sub * 8192, &map_v, sub * 64, hkv, kt * 64, b, bar);
-        };
-        auto load_q = [&](int stg, int gi, int qt) {
-            const uint32_t base = sbase + L::stage + stg * L::stage_bytes;
-#pragma unroll
-            for (int sub = 0; sub < DK / 64; ++sub)
-                tma_load_4d(base + 128 * DV * 2 + sub * 16384, &map_q, sub * 64, hkv * G + gi, qt * ATT_BM, b, bar_full + stg * 8);
-#pragma unroll
-            for (int sub = 0; sub < DV / 64; ++sub)
-                tma_load_4d(base + sub * 16384, &map_do, sub * 64, hkv * G + gi, qt * ATT_BM, b, bar_full + stg * 8);
-        };
-        int n = 0;
-        if (paired) {
-            if (lane == 0)
-                for (int u = 0; u < 2; ++u)
-                    if (has_items(u)) {
-                        mbar_expect_tx(bar_kv + u * 8, L::kv_bytes);
-                        load_kv(u, tile[u], bar_kv + u * 8);
-                    }
-            __syncwarp();
+        int ni = 0, pairs = 0;                                // steps with queries, pairs that have some
 #pragma unroll 1
-            for (bool more = w.begin(); more; more = w.next_query(), ++n) {
-                const int stg = n & 1;
-                if (n >= 2) ok = warp_wait(bar_empty + stg * 8, ((n >> 1) - 1) & 1);
+        while (ok) {
+            next_step();
+            if (d.y & BKV_STOP) break;
+            if (d.y & BKV_EMPTY) continue;
+            const int hkv = loc.z, b = loc.w;
+            if (d.y & BKV_FIRST) {
+                if (pairs > 0) ok = warp_wait(kv_empty, (pairs - 1) & 1);
                 if (!ok) break;
                 if (lane == 0) {
-                    mbar_expect_tx(bar_full + stg * 8, L::stage_bytes);
-                    load_q(stg, w.gi, w.qt);
-                    if (w.qt + 2 < NTq) {                     // warm L2 for the tile this stage most likely receives next
+                    const int t[2] = {loc.x, loc.y};
+                    mbar_expect_tx(kv_full, ((t[0] >= 0) + (t[1] >= 0)) * 64 * (DK + DV) * 2);
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        if (t[u] < 0) continue;
 #pragma unroll
                         for (int sub = 0; sub < DK / 64; ++sub)
-                            tma_prefetch_4d(&map_q, sub * 64, hkv * G + w.gi, (w.qt + 2) * ATT_BM, b);
+                            tma_load_4d(sbase + L::kv + sub * 16384 + u * 8192, &map_k, sub * 64, hkv, t[u] * 64, b, kv_full);
 #pragma unroll
                         for (int sub = 0; sub < DV / 64; ++sub)
-                            tma_prefetch_4d(&map_do, sub * 64, hkv * G + w.gi, (w.qt + 2) * ATT_BM, b);
+                            tma_load_4d(sbase + L::kv + 128 * DK * 2 + sub * 16384 + u * 8192, &map_v, sub * 64, hkv, t[u] * 64, b, kv_full);
                     }
                 }
                 __syncwarp();
+                ++pairs;
             }
-        } else {
-#pragma unroll 1
-            for (bool more = ow.begin(); more; more = ow.next(), ++n) {
-                const int stg = n & 1;
-                if (n >= 2) ok = warp_wait(bar_empty + stg * 8, ((n >> 1) - 1) & 1);
-                if (!ok) break;
-                if (lane == 0) {                              // every item brings its own copy of k and v
-                    mbar_expect_tx(bar_full + stg * 8, L::stage_bytes + L::kv_bytes);
-                    load_kv(stg, s_tile[ow.u], bar_full + stg * 8);
-                    load_q(stg, ow.gi, ow.qt);
-                }
-                __syncwarp();
+            const int st = ni & 1, par = ((ni >> 1) - 1) & 1, hq = hkv * G + d.z;
+            if (lane == 0 && ni >= 2) {                       // into L2 while the stages are still read
+#pragma unroll
+                for (int sub = 0; sub < DK / 64; ++sub) tma_prefetch_4d(&map_q, sub * 64, hq, d.x, b);
+#pragma unroll
+                for (int sub = 0; sub < DV / 64; ++sub) tma_prefetch_4d(&map_do, sub * 64, hq, d.x, b);
+            }
+            __syncwarp();
+            if (ni >= 2) ok = warp_wait(q_empty + st * 8, par);
+            if (!ok) break;
+            if (lane == 0) {
+                mbar_expect_tx(q_full + st * 8, 128 * DK * 2);
+#pragma unroll
+                for (int sub = 0; sub < DK / 64; ++sub)
+                    tma_load_4d(sbase + L::q + st * (128 * DK * 2) + sub * 16384, &map_q, sub * 64, hq, d.x, b, q_full + st * 8);
+            }
+            __syncwarp();
+            if (ni >= 2) ok = warp_wait(do_empty + st * 8, par);
+            if (!ok) {
+                warp_wait(q_full + st * 8, (ni >> 1) & 1);    // nothing may still be on its way into shared memory
+                break;
+            }
+            if (lane == 0) {
+                mbar_expect_tx(do_full + st * 8, 128 * DV * 2);
+#pragma unroll
+                for (int sub = 0; sub < DV / 64; ++sub)
+                    tma_load_4d(sbase + L::dos + st * (128 * DV * 2) + sub * 16384, &map_do, sub * 64, hq, d.x, b, do_full + st * 8);
+            }
+            __syncwarp();
+            ++ni;
+        }
+        if (!ok) {
+            if (pairs > 0) warp_wait(kv_full, (pairs - 1) & 1);
+            for (int i = max(0, ni - 2); i < ni; ++i) {
+                warp_wait(q_full + (i & 1) * 8, (i >> 1) & 1);
+                warp_wait(do_full + (i & 1) * 8, (i >> 1) & 1);
             }
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        constexpr uint32_t id_s = umma_idesc_bf16(128, 64, false);
-        constexpr uint32_t id_acc = umma_idesc_bf16(128, 64, true) | (1u << 15);         // A MN-major too
-        auto scores = [&](int n, int stg, int kv) {           // S and dO V^T of item n into buffer n & 1
-            stg = __shfl_sync(0xffffffffu, stg, 0);
-            kv = __shfl_sync(0xffffffffu, kv, 0);
-            n = __shfl_sync(0xffffffffu, n, 0) & 1;
+        constexpr uint32_t id_s = umma_idesc_bf16(128, 128, false);
+        constexpr uint32_t id_dv = umma_idesc_bf16(128, DV, true), id_dk = umma_idesc_bf16(128, DK, true);
+        const uint32_t kl = umma_desc_lo(sbase + L::kv, 16), vl = umma_desc_lo(sbase + L::kv + 128 * DK * 2, 16);
+        auto scores = [&](int st) {                           // K Q^T
             tc_fence_after();
-            const uint32_t dl = umma_desc_lo(sbase + L::stage + stg * L::stage_bytes, 16), ql = dl + (128 * DV * 2 >> 4);
-            const uint32_t kl = umma_desc_lo(sbase + L::kv + kv * L::kv_bytes, 16), vl = kl + (64 * DK * 2 >> 4);
+            const uint32_t ql = umma_desc_lo(sbase + L::q + st * (128 * DK * 2), 16);
 #pragma unroll
-            for (int h = 0; h < DK / 64; ++h) umma_ss_x4<2, 2>(tmem + C_S + n * 64, ql + h * 1024, kl + h * 512, id_s, h > 0);
-#pragma unroll
-            for (int h = 0; h < DV / 64; ++h) umma_ss_x4<2, 2>(tmem + C_DP + n * 64, dl + h * 1024, vl + h * 512, id_s, h > 0);
-            umma_commit(bar_s + n * 8);
+            for (int h = 0; h < DK / 64; ++h) umma_ss_x4<2, 2>(tmem + C_S, kl + h * 1024, ql + h * 1024, id_s, h > 0);
+            umma_commit(bar_s);
         };
-        auto accumulate = [&](int stg, int slot, bool cont, bool release) {
-            stg = __shfl_sync(0xffffffffu, stg, 0);
-            slot = __shfl_sync(0xffffffffu, slot, 0);
+        auto products = [&](int st, bool last) {              // V dO^T
             tc_fence_after();
-            const uint32_t dl = umma_desc_lo(sbase + L::stage + stg * L::stage_bytes, 16384), ql = dl + (128 * DV * 2 >> 4);
-            const uint32_t pl = umma_desc_lo(sbase + L::p, 8192), dsl = umma_desc_lo(sbase + L::ds, 8192);
-            const uint32_t acc = tmem + C_ACC + slot * 128;
+            const uint32_t dl = umma_desc_lo(sbase + L::dos + st * (128 * DV * 2), 16);
 #pragma unroll
-            for (int h = 0; h < 2; ++h)                       // dv^T += do^T p
-                umma_ss_x4<128, 128>(acc, dl + h * 512, pl + h * 512, id_acc, cont || h > 0);
-#pragma unroll
-            for (int h = 0; h < 2; ++h)                       // dk^T += q^T ds
-                umma_ss_x4<128, 128>(acc + 64, ql + h * 512, dsl + h * 512, id_acc, cont || h > 0);
-            umma_commit(bar_acc);
-            if (release) umma_commit(bar_empty + stg * 8);
+            for (int h = 0; h < DV / 64; ++h) umma_ss_x4<2, 2>(tmem + C_DP, vl + h * 1024, dl + h * 1024, id_s, h > 0);
+            umma_commit(bar_dp);
+            if (last) umma_commit(kv_empty);
         };
-        if (paired) {
-            DkvWalk a = w;                                    // one item ahead: scores
-            bool more = w.begin(), ahead = a.begin();
-            int na = 0, nq_a = -1, nq = -1;                   // items issued; query tiles entered by a / w
-            bool kv_seen[2] = {false, false}, started[2] = {false, false};
-            auto step_ahead = [&]() {
-                if (a.first_of_query()) {
-                    ++nq_a;
-                    ok = warp_wait(bar_full + (nq_a & 1) * 8, (nq_a >> 1) & 1);
-                }
-                if (ok && !kv_seen[a.u]) ok = warp_wait(bar_kv + a.u * 8, 0);
-                kv_seen[a.u] = true;
-                if (ok) scores(na, nq_a & 1, a.u);
-                ++na;
-                ahead = a.next();
-            };
-            // The scores of the next item go ahead of this item's products (their buffer was read before bar_p of item
-            // i - 1) unless their tiles are still on the way: the stage that the producer fills after them is the one
-            // that these products release.  (One place that issues scores and one that issues products: inlined at every
-            // turn of the sequence, with descriptors formed for each product, this warp had 150 KB of code.)
-            auto ready = [&]() {
-                return __all_sync(0xffffffffu, !a.first_of_query() || mbar_test_wait(bar_full + ((nq_a + 1) & 1) * 8, ((nq_a + 1) >> 1) & 1));
-            };
+        int ni = 0, pairs = 0;
+        int f = next_step();
 #pragma unroll 1
-            for (int i = 0; ok && more;) {
-                if (ahead && na <= i + 1 && (na == i || ready())) {
-                    step_ahead();
-                    if (na == i + 1) continue;
-                }
-                if (ok) ok = warp_wait(bar_p, i & 1);
-                if (!ok) break;
-                if (w.first_of_query()) ++nq;
-                accumulate(nq & 1, w.u, started[w.u], w.last_of_query());
-                started[w.u] = true;
-                more = w.next();
-                ++i;
+        while (ok && !(f & BKV_STOP)) {
+            if (f & BKV_EMPTY) {
+                f = next_step();
+                continue;
             }
-        } else {
-            OwnWalk a = ow;
-            bool more = ow.begin(), ahead = a.begin();
-            int na = 0;
-            auto step_ahead = [&]() {
-                ok = warp_wait(bar_full + (na & 1) * 8, (na >> 1) & 1);
-                if (ok) scores(na, na & 1, na & 1);
-                ++na;
-                ahead = a.next();
-            };
-#pragma unroll 1
-            for (int i = 0; ok && more;) {
-                if (ahead && na <= i + 1 &&
-                    (na == i || __all_sync(0xffffffffu, mbar_test_wait(bar_full + (na & 1) * 8, (na >> 1) & 1)))) {
-                    step_ahead();
-                    if (na == i + 1) continue;
-                }
-                // the accumulators of tile u - 2 were read before the softmax warps arrived here for the item before
-                if (ok) ok = warp_wait(bar_p, i & 1);
+            if (f & BKV_FIRST) {
+                ok = warp_wait(kv_full, pairs & 1);
+                if (ok) ok = warp_wait(q_full + (ni & 1) * 8, (ni >> 1) & 1);
                 if (!ok) break;
-                accumulate(i & 1, ow.u & 1, !ow.first_of_tile(), true);
-                more = ow.next();
-                ++i;
+                scores(ni & 1);
+                ok = warp_wait(do_full + (ni & 1) * 8, (ni >> 1) & 1);
+                if (!ok) break;
+                products(ni & 1, (f & BKV_LAST) != 0);
+                ok = warp_wait(bar_acc_free, pairs & 1);
+                ++pairs;
             }
+            const int st = ni & 1, nst = st ^ 1, npar = ((ni + 1) >> 1) & 1;
+            const uint32_t m01 = f & BKV_ACT0 ? 0u : 0xffffffffu, m23 = f & BKV_ACT1 ? 0u : 0xffffffffu;
+            const bool last = (f & BKV_LAST) != 0;
+            if (ok) ok = warp_wait(bar_p, ni & 1);
+            if (!ok) break;
+            tc_fence_after();
+            {                                                 // dv += p dO
+                const uint32_t dl = umma_desc_lo(sbase + L::dos + st * (128 * DV * 2), 16384);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) umma_ts_x4_lanes<128>(tmem + C_DV, tmem + C_S + h * 64, dl + h * 512, id_dv, m01, m23);
+                umma_commit(do_empty + st * 8);
+            }
+            int fn = BKV_STOP;
+            if (!last) {                                      // the next scores as soon as p has been used
+                fn = next_step();
+                if (ok) ok = warp_wait(q_full + nst * 8, npar);
+                if (!ok) break;
+                scores(nst);
+            }
+            ok = warp_wait(bar_ds, ni & 1);
+            if (!ok) break;
+            tc_fence_after();
+            {                                                 // dk += ds Q
+                const uint32_t ql = umma_desc_lo(sbase + L::q + st * (128 * DK * 2), 16384);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) umma_ts_x4_lanes<128>(tmem + C_DK, tmem + C_DP + h * 64, ql + h * 512, id_dk, m01, m23);
+                umma_commit(q_empty + st * 8);
+            }
+            if (last) {
+                umma_commit(bar_acc);
+                f = next_step();
+            } else {
+                ok = warp_wait(do_full + nst * 8, npar);
+                if (!ok) break;
+                products(nst, (fn & BKV_LAST) != 0);
+                f = fn;
+            }
+            ++ni;
         }
-    } else {
-        // ------------------------------------------------------------ softmax (8 warps)
-        const int quad = warp & 3, half = (warp - 2) >> 2, sw = warp - 2;
-        const int row_a = quad * 32 + half * 16 + (lane >> 2), row_b = row_a + 8;
-        const int cq = (lane & 3) * 2;
-        const uint32_t t_rows = tmem + ((uint32_t)(quad * 32 + half * 16) << 16);
-        const float sl2 = scale * kLog2e;
-        unsigned char* p_t = smem + L::p;
-        unsigned char* ds_t = smem + L::ds;
-        float lse_a = 0.f, lse_b = 0.f, del_a = 0.f, del_b = 0.f;
-        auto load_rows = [&](int gi, int qt) {
-            const int t_a = qt * ATT_BM + row_a, t_b = t_a + 8;
-            const long r = ((long)b * T + t_a) * HQ + hkv * G + gi;
-            lse_a = t_a < T ? lse[r] : 0.f;
-            del_a = t_a < T ? delta[r] : 0.f;
-            lse_b = t_b < T ? lse[r + 8L * HQ] : 0.f;
-            del_b = t_b < T ? delta[r + 8L * HQ] : 0.f;
+    } else if (warp == 10) {
+        // ------------------------------------------------------------ planner: blocks, their steps, lse and delta of the queries
+        int n = 0, ni = 0, asked = 0, answers = 0;            // steps, steps with queries, take-over requests
+        int block = blockIdx.x;
+        auto put = [&](int4 x, int4 y) {
+            const int slot = n & (BKV_DESCS - 1);
+            if (n >= BKV_DESCS) ok = warp_wait(desc_empty + slot * 8, (n / BKV_DESCS - 1) & 1);
+            if (!ok) return;
+            if (lane == 0) {
+                s_desc[2 * slot] = x;
+                s_desc[2 * slot + 1] = y;
+            }
+            arrive(desc_full + slot * 8);
+            ++n;
         };
-        // p and ds of item i (key tile kt, query tile qt; `sel`: later blocks see the keys) into registers, bf16 pairs; adds
-        // the ds of later blocks' queries to dn.  Returns once the products of the previous item have read p and ds.
-        uint32_t sr[32];
-        auto item_p = [&](int i, int kt, int qt, bool sel, float& dn) -> bool {
-            bool ok = warp_wait(bar_s + (i & 1) * 8, (i >> 1) & 1);
-            if (!ok) return false;
-            tc_fence_after();
-            uint32_t dr[32];
-            tmem_ld_16x256b_x8(t_rows + C_S + (i & 1) * 64, sr);
-            tmem_ld_16x256b_x8(t_rows + C_DP + (i & 1) * 64, dr);
-            tmem_ld_wait();
-            const int t_a = qt * ATT_BM + row_a, t_b = t_a + 8;
-            const int s0 = kt * 64, blk_end = (kt / cpb + 1) * nbs;
-            if (qt * ATT_BM < blk_end) {
-                // rows of the own block see columns [0, t - s0], rows behind it all or none
-                const int lim_a = t_a >= blk_end ? (sel ? 63 : -1) : (own ? t_a - s0 : -1);
-                const int lim_b = t_b >= blk_end ? (sel ? 63 : -1) : (own ? t_b - s0 : -1);
-#pragma unroll
-                for (int k = 0; k < 8; ++k)
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        const int c = 8 * k + cq + e;
-                        if (c > lim_a) sr[4 * k + e] = 0xff800000u;
-                        if (c > lim_b) sr[4 * k + 2 + e] = 0xff800000u;
-                    }
+        auto request = [&]() {
+            if (lane == 0) {
+                fence_async_smem();
+                mbar_expect_tx(bar_clc, 16);
+                request_block(sbase + L::clc, bar_clc);
             }
-            float sum_a = 0.f, sum_b = 0.f;
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const float p0 = ex2(fmaf(__uint_as_float(sr[4 * k]), sl2, -lse_a));
-                const float p1 = ex2(fmaf(__uint_as_float(sr[4 * k + 1]), sl2, -lse_a));
-                const float p2 = ex2(fmaf(__uint_as_float(sr[4 * k + 2]), sl2, -lse_b));
-                const float p3 = ex2(fmaf(__uint_as_float(sr[4 * k + 3]), sl2, -lse_b));
-                const float d0 = p0 * (__uint_as_float(dr[4 * k]) - del_a), d1 = p1 * (__uint_as_float(dr[4 * k + 1]) - del_a);
-                const float d2 = p2 * (__uint_as_float(dr[4 * k + 2]) - del_b), d3 = p3 * (__uint_as_float(dr[4 * k + 3]) - del_b);
-                sum_a += d0 + d1;
-                sum_b += d2 + d3;
-                sr[4 * k] = pack_bf16(p0, p1);
-                sr[4 * k + 1] = pack_bf16(p2, p3);
-                sr[4 * k + 2] = pack_bf16(d0, d1);
-                sr[4 * k + 3] = pack_bf16(d2, d3);
-            }
-            dn += (t_a >= blk_end ? sum_a : 0.f) + (t_b >= blk_end ? sum_b : 0.f);
-            if (i > 0) ok = warp_wait(bar_acc, (i - 1) & 1);
-            return ok;
-        };
-        auto item_write = [&]() {
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const uint32_t oa = swz<128>(row_a, k) + (lane & 3) * 4, ob = swz<128>(row_b, k) + (lane & 3) * 4;
-                *reinterpret_cast<uint32_t*>(p_t + oa) = sr[4 * k];
-                *reinterpret_cast<uint32_t*>(p_t + ob) = sr[4 * k + 1];
-                *reinterpret_cast<uint32_t*>(ds_t + oa) = sr[4 * k + 2];
-                *reinterpret_cast<uint32_t*>(ds_t + ob) = sr[4 * k + 3];
-            }
-            fence_async_smem();
-            tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar_p);
+            ++asked;
         };
-        // dk, dv of key tile kt from accumulator pair `slot` (zeros without `any`): lane = head-dim index, columns = keys.
-        // Transposed through the p and ds tiles, which no product reads at that time, so that the rows leave in 16-byte
-        // pieces (two-byte stores straight from the registers took 8000 clocks a tile, most of an unselected tile's time).
-        // Every softmax warp calls it, also after a failed wait (`good` false: nothing is read or stored).
-        auto finish = [&](int kt, int slot, bool any, bool good) {
-            const int d = quad * 32 + lane;
-            const uint32_t acc = tmem + ((uint32_t)(quad * 32) << 16) + C_ACC + slot * 128 + half * 32;
-            tc_fence_after();
-            uint32_t r[32];
-            if (good && quad * 32 < DV) {
-                tmem_ld32(acc, r);
-                tmem_ld_wait();
+#pragma unroll 1
+        while (ok) {
+            // Block `item` of a head: the item-th pair of the tiles whose block some head of the group selected, in their order
+            // (neighbours see nearly the same queries), then what is unselected of tiles 2 item and 2 item + 1, which only
+            // their own blocks' queries see.
+            const int hbase = block / (BKV_HEADS * ctas_per_head) * BKV_HEADS, hcount = min(BKV_HEADS, heads - hbase);
+            const int within = block - hbase * ctas_per_head;
+            const int item = within / hcount, head = hbase + within % hcount;
+            const int hkv = head % HKV, b = head / HKV;
+            auto selected = [&](int kt) -> bool {
+                bool s = false;
+#pragma unroll 1
+                for (int gi = 0; gi < G; ++gi) s |= types_i[(((long)b * TN + kt / cpb) * HN + (hkv * G + gi) / (HQ / HN)) * 2] != 0;
+                return s;
+            };
+            int chosen[2] = {-1, -1}, rest[2] = {-1, -1};
+            unsigned mine = 0;                                // bit i: tile 2 item + i is selected
+            int cnt = 0;
+#pragma unroll 1
+            for (int base = 0; base < NT; base += 32) {
+                const unsigned m = __ballot_sync(0xffffffffu, base + lane < NT && selected(base + lane));
+                const int k = __popc(m);
+                if (2 * item >= base && 2 * item < base + 32) mine = m >> (2 * item - base);
 #pragma unroll
-                for (int c = 0; c < 32; ++c)
-                    *reinterpret_cast<__nv_bfloat16*>(p_t + swz<DV * 2>(half * 32 + c, d >> 3) + (d & 7) * 2) =
-                        __float2bfloat16(any ? __uint_as_float(r[c]) : 0.f);
+                for (int i = 0; i < 2; ++i) {
+                    const int r = 2 * item + i - cnt;
+                    if (r >= 0 && r < k) chosen[i] = base + __fns(m, 0, r + 1);
+                }
+                cnt += k;
+                if (cnt >= 2 * item + 2 && base + 32 > 2 * item + 1) break;
             }
-            if (good && quad * 32 < DK) {
-                tmem_ld32(acc + 64, r);
-                tmem_ld_wait();
 #pragma unroll
-                for (int c = 0; c < 32; ++c)
-                    *reinterpret_cast<__nv_bfloat16*>(ds_t + swz<DK * 2>(half * 32 + c, d >> 3) + (d & 7) * 2) =
-                        __float2bfloat16(any ? __uint_as_float(r[c]) * scale : 0.f);
+            for (int i = 0; i < 2; ++i)
+                if (!((mine >> i) & 1) && 2 * item + i < NT) rest[i] = 2 * item + i;
+            bool requested = chosen[0] < 0;                   // a step or none: ask for the next block at once
+            if (requested) {
+                request();
+            } else {
+                // last query tile of every (tile, head): the sequence's if the head selected the block, else the own block's
+                __syncwarp();
+#pragma unroll 1
+                for (int i = lane; i < 2 * BKV_MAXG; i += 32) {
+                    const int kt = i / BKV_MAXG ? chosen[1] : chosen[0], gi = i % BKV_MAXG;
+                    int last = -1;
+                    if (kt >= 0 && gi < G) {
+                        const int blk = kt / cpb, blk_end = (blk + 1) * nbs;
+                        const bool s = G == 1 || types_i[(((long)b * TN + blk) * HN + (hkv * G + gi) / (HQ / HN)) * 2] != 0;
+                        if (s && blk_end < T) last = NTq - 1;
+                        else if (own) last = min((blk_end - 1) / ATT_BM, NTq - 1);
+                    }
+                    s_last[i] = (int16_t)last;
+                }
+                __syncwarp();
             }
-            tc_fence_before();
-            asm volatile("bar.sync 2, 256;" ::: "memory");
-            const long tok = (long)b * T + kt * 64;
-            const int n_valid = good ? min(64, T - kt * 64) : 0;
-            store_tile<64, DV, 256>(p_t, dv + (tok * HKV + hkv) * DV, (long)HKV * DV, n_valid, tid - 64);
-            store_tile<64, DK, 256>(ds_t, dk + (tok * HKV + hkv) * DK, (long)HKV * DK, n_valid, tid - 64);
-            asm volatile("bar.sync 2, 256;" ::: "memory");
-        };
-        int i = 0;
-        if (paired) {
-            float dn[2] = {0.f, 0.f};
-            auto flush = [&](int gi) {                        // one slot per (key tile, head, warp): a fixed order of summation
+#pragma unroll 1
+            for (int pass = chosen[0] < 0; ok && pass < 2; ++pass) {
+                const bool sums = pass == 0;
+                const int t[2] = {sums ? chosen[0] : rest[0], sums ? chosen[1] : rest[1]};
+                if (t[0] < 0 && t[1] < 0) continue;
+                const int4 where = make_int4(t[0], t[1], hkv, b);
+                int first[2], end[2], own_last[2];            // tile u: query tiles [first, last(head)]
+                bool any[2] = {false, false};
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
-                    dn[u] = warp_sum(dn[u]);
-                    if (lane == 0) s_dn[(u * BKV_MAXG + gi) * 8 + sw] = dn[u];
-                    dn[u] = 0.f;
+                    end[u] = (t[u] / cpb + 1) * nbs;
+                    first[u] = t[u] < 0 ? NTq : own ? t[u] * 64 / ATT_BM : end[u] / ATT_BM;
+                    own_last[u] = t[u] >= 0 && own ? min((end[u] - 1) / ATT_BM, NTq - 1) : -1;
                 }
-            };
-            int gi = 0;
+                auto last_of = [&](int u, int gi) -> int { return sums ? (int)s_last[u * BKV_MAXG + gi] : own_last[u]; };
+                for (int gi = 0; gi < G; ++gi) {
+                    any[0] |= last_of(0, gi) >= first[0];
+                    any[1] |= last_of(1, gi) >= first[1];
+                }
+                const int base = (sums ? BKV_SUMS : 0) | (any[0] ? BKV_ANY0 : 0) | (any[1] ? BKV_ANY1 : 0);
+                if (!any[0] && !any[1]) {
+                    put(make_int4(0, base | BKV_EMPTY, 0, 0), where);
+                    continue;
+                }
+                int held = -1, h_qt = 0, h_gi = 0, h_prev = 0;    // the step that is announced once it is known whether another follows
+                float nl[4], nd[4];
+                auto announce = [&](int more) {
+                    const int st = ni & 1;
+                    if (ni >= 2) ok = warp_wait(st_empty + st * 8, ((ni >> 1) - 1) & 1);
+                    if (!ok) return;
+                    float* x = reinterpret_cast<float*>(smem + L::stat + st * 1024);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        x[lane + 32 * i] = nl[i];
+                        x[128 + lane + 32 * i] = nd[i];
+                    }
+                    arrive(st_full + st * 8);
+                    ++ni;
+                    put(make_int4(h_qt * ATT_BM, held | more, h_gi, h_prev), where);
+                };
+                int prev = -1;
 #pragma unroll 1
-            for (bool more = w.begin(); more; more = w.next(), ++i) {
-                if (w.gi != gi) {
-                    flush(gi);
-                    gi = w.gi;
+                for (int gi = 0; ok && gi < G; ++gi) {
+                    const int l0 = last_of(0, gi), l1 = last_of(1, gi), hi = max(l0, l1);
+                    int sel = sums ? BKV_SEL0 | BKV_SEL1 : 0;
+                    if (sums && G > 1) {
+                        sel = 0;
+#pragma unroll
+                        for (int u = 0; u < 2; ++u)
+                            if (t[u] >= 0 && types_i[(((long)b * TN + t[u] / cpb) * HN + (hkv * G + gi) / (HQ / HN)) * 2] != 0)
+                                sel |= u ? BKV_SEL1 : BKV_SEL0;
+                    }
+#pragma unroll 1
+                    for (int qt = min(l0 >= first[0] ? first[0] : NTq, l1 >= first[1] ? first[1] : NTq); ok && qt <= hi; ++qt) {
+                        const int act = (qt >= first[0] && qt <= l0 ? BKV_ACT0 : 0) | (qt >= first[1] && qt <= l1 ? BKV_ACT1 : 0);
+                        if (!act) continue;
+                        if (held >= 0) announce(0);
+                        held = base | act | sel | (prev < 0 ? BKV_FIRST : 0) | (prev >= 0 && prev != gi ? BKV_FLUSH : 0);
+                        h_qt = qt;
+                        h_gi = gi;
+                        h_prev = prev;
+                        prev = gi;
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {         // a query behind the end has probability 0
+                            const int q = qt * ATT_BM + lane + 32 * i;
+                            const long r = ((long)b * T + q) * HQ + hkv * G + gi;
+                            nl[i] = q < T ? -lse[r] : -INFINITY;
+                            nd[i] = q < T ? -delta[r] : 0.f;
+                        }
+                    }
                 }
-                if (w.first_of_query()) load_rows(gi, w.qt);
-                const int kt = w.u ? tile[1] : tile[0];
-                // rows behind the own block are in the walk only where the head selected the block; in a tile that holds
-                // both, the flag decides
-                bool sel = true;
-                if (G > 1 && w.qt * ATT_BM < (kt / cpb + 1) * nbs)
-                    sel = types_i[(((long)b * TN + kt / cpb) * HN + (hkv * G + gi) / (HQ / HN)) * 2] != 0;
-                float add = 0.f;
-                ok = item_p(i, kt, w.qt, sel, add);
+                if (ok) announce(BKV_LAST);
+                // the pair's last steps are under way: early enough to work out the next block, late enough to leave it to an SM
+                // that is free earlier
+                if (ok && sums) {
+                    request();
+                    requested = true;
+                }
+            }
+            if (ok && !requested) request();                  // (the chosen pair had no step)
+            if (asked > answers) {                            // (also after a failed wait: the answer is on its way)
+                const bool came = warp_wait(bar_clc, answers & 1);
+                ++answers;
+                ok = ok && came;
+            }
+            if (!ok || !taken_block(sbase + L::clc, block)) break;
+            __syncwarp();
+        }
+        if (ok) put(make_int4(0, BKV_STOP, 0, 0), make_int4(0, 0, 0, 0));
+    } else {
+        // ------------------------------------------------------------ softmax: one key per thread and half, 64 queries each
+        const int quad = warp & 3, half = (warp - 2) >> 2, u = quad >> 1, part = (quad & 1) * 2 + half;
+        const uint32_t t_lane = tmem + ((uint32_t)(quad * 32) << 16);
+        const uint32_t t_s = t_lane + C_S + half * 64, t_dp = t_lane + C_DP + half * 64;
+        const float sl2 = scale * kLog2e;
+        unsigned char* const out = smem + L::out + (warp - 2) * 4096;
+        float dn = 0.f;
+        auto flush = [&](int gi, int f) {                     // one slot per (key tile, head, warp): a fixed order of summation
+            dn = warp_sum(dn);
+            if (lane == 0 && (f & BKV_SUMS)) s_dn[(u * BKV_MAXG + gi) * 4 + part] = dn;
+            dn = 0.f;
+        };
+        auto zero = [&](uint32_t col) {
+            uint32_t z[32];
+#pragma unroll
+            for (int e = 0; e < 32; ++e) z[e] = 0;
+            tmem_st32(t_lane + col, z);
+            tmem_st32(t_lane + col + 32, z);
+        };
+        auto block_col = [&](int blk) -> uint32_t { return blk < DV / 64 ? C_DV + blk * 64 : C_DK + (blk - DV / 64) * 64; };
+        // this warp's rows of dv and dk: 64 columns at a time through its own 4 KB, then zeros for the next pair
+        auto finish = [&](bool any, bool acc) {
+            const int kt = u ? loc.y : loc.x, row0 = kt * 64 + (quad & 1) * 32;
+#pragma unroll 1
+            for (int blk = half; blk < NB; blk += 2) {
+                uint32_t w[32];
+#pragma unroll
+                for (int e = 0; e < 32; ++e) w[e] = 0;
+                if (acc) {
+                    if (any) {
+                        uint32_t r0[32], r1[32];
+                        tmem_ld32(t_lane + block_col(blk), r0);
+                        tmem_ld32(t_lane + block_col(blk) + 32, r1);
+                        tmem_ld_wait();
+                        const float f = blk < DV / 64 ? 1.f : scale;
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) {
+                            w[e] = pack_bf16(__uint_as_float(r0[2 * e]) * f, __uint_as_float(r0[2 * e + 1]) * f);
+                            w[16 + e] = pack_bf16(__uint_as_float(r1[2 * e]) * f, __uint_as_float(r1[2 * e + 1]) * f);
+                        }
+                    }
+                    zero(block_col(blk));
+                }
+                if (lane == 0) tma_store_wait_read();         // the block before has left
+                __syncwarp();
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    *reinterpret_cast<uint4*>(out + lane * 128 + ((i ^ (lane & 7)) << 4)) =
+                        make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+                fence_async_smem();
+                __syncwarp();
+                if (lane == 0 && kt >= 0 && row0 < T) {
+                    if (blk < DV / 64) tma_store_4d(&map_dv, smem_u32(out), blk * 64, loc.z, row0, loc.w);
+                    else tma_store_4d(&map_dk, smem_u32(out), (blk - DV / 64) * 64, loc.z, row0, loc.w);
+                    tma_store_commit();
+                }
+            }
+        };
+        // (one warp)  the pair's sums of ds for every head, which are then zero again
+        auto write_sums = [&](bool some) {
+#pragma unroll 1
+            for (int i = lane; i < 2 * G; i += 32) {
+                const int v = i / G, gi = i - v * G, kt = v ? loc.y : loc.x;
+                float* x = s_dn + (v * BKV_MAXG + gi) * 4;
+                const float sum = some ? (x[0] + x[1]) + (x[2] + x[3]) : 0.f;
+                x[0] = x[1] = x[2] = x[3] = 0.f;
+                if (kt >= 0) dnats_part[((long)loc.w * NT + kt) * HQ + loc.z * G + gi] = sum;
+            }
+            __syncwarp();
+        };
+        auto release_acc = [&]() {
+            tmem_st_wait();
+            tc_fence_before();
+            arrive(bar_acc_free);
+        };
+#pragma unroll 1
+        for (int blk = half; blk < NB; blk += 2) zero(block_col(blk));
+        release_acc();
+        int ni = 0, pairs = 0;
+#pragma unroll 1
+        while (true) {
+            const int f = next_step();
+            if (!ok || (f & BKV_STOP)) break;
+            if (f & BKV_EMPTY) {
+                finish(false, false);
+                if (warp == 2) write_sums(false);
+                continue;
+            }
+            const bool act = (f & (BKV_ACT0 << u)) != 0;
+            const int kt = u ? loc.y : loc.x, blk_end = (kt / cpb + 1) * nbs - d.x;      // relative to the first query
+            const float* st = reinterpret_cast<const float*>(smem + L::stat + (ni & 1) * 1024) + half * 64;
+            ok = warp_wait(st_full + (ni & 1) * 8, (ni >> 1) & 1);
+            if (ok) ok = warp_wait(bar_s, ni & 1);
+            if (!ok) break;
+            tc_fence_after();
+            if (f & BKV_FLUSH) flush(d.w, f);                 // (every warp has left the pair before: its sums have been written)
+            uint32_t r[64];
+            if (act) {
+                uint32_t(&r0)[32] = *reinterpret_cast<uint32_t(*)[32]>(r);
+                uint32_t(&r1)[32] = *reinterpret_cast<uint32_t(*)[32]>(r + 32);
+                tmem_ld32(t_s, r0);
+                tmem_ld32(t_s + 32, r1);
+                tmem_ld_wait();
+                if (blk_end > half * 64 || !(f & (BKV_SEL0 << u))) {          // not all of them behind the own block and seeing it
+                    const int lo = (own ? kt * 64 + (quad & 1) * 32 + lane - d.x : blk_end) - half * 64;
+                    const int hi = (f & (BKV_SEL0 << u)) ? 64 : blk_end - half * 64;
+#pragma unroll
+                    for (int e = 0; e < 64; ++e)
+                        if (e < lo || e >= hi) r[e] = 0xff800000u;
+                }
+                uint32_t pk[32];
+                const uint64_t sc2 = pack2(sl2, sl2);
+#pragma unroll
+                for (int e = 0; e < 32; e += 2) {
+                    const float4 l4 = *reinterpret_cast<const float4*>(st + 2 * e);
+                    float x0, x1, x2, x3;
+                    unpack2(fma2(pack2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1])), sc2, pack2(l4.x, l4.y)), x0, x1);
+                    unpack2(fma2(pack2(__uint_as_float(r[2 * e + 2]), __uint_as_float(r[2 * e + 3])), sc2, pack2(l4.z, l4.w)), x2, x3);
+                    x0 = ex2(x0), x1 = ex2(x1), x2 = ex2(x2), x3 = ex2(x3);
+                    r[2 * e] = __float_as_uint(x0), r[2 * e + 1] = __float_as_uint(x1);
+                    r[2 * e + 2] = __float_as_uint(x2), r[2 * e + 3] = __float_as_uint(x3);
+                    pk[e] = pack_bf16(x0, x1);
+                    pk[e + 1] = pack_bf16(x2, x3);
+                }
+                tmem_st32(t_s, pk);
+                tmem_st_wait();
+            }
+            tc_fence_before();
+            arrive(bar_p);
+            ok = warp_wait(bar_dp, ni & 1);
+            if (!ok) break;
+            tc_fence_after();
+            if (act) {
+                uint32_t pk[32];
+                uint64_t sum = 0;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t x[32];
+                    tmem_ld32(t_dp + h * 32, x);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int e = 0; e < 16; e += 2) {
+                        const float4 d4 = *reinterpret_cast<const float4*>(st + 128 + h * 32 + 2 * e);
+                        const uint32_t* p = r + h * 32 + 2 * e;
+                        const uint64_t a = mul2(pack2(__uint_as_float(p[0]), __uint_as_float(p[1])),
+                                                add2(pack2(__uint_as_float(x[2 * e]), __uint_as_float(x[2 * e + 1])), pack2(d4.x, d4.y)));
+                        const uint64_t c = mul2(pack2(__uint_as_float(p[2]), __uint_as_float(p[3])),
+                                                add2(pack2(__uint_as_float(x[2 * e + 2]), __uint_as_float(x[2 * e + 3])), pack2(d4.z, d4.w)));
+                        pk[h * 16 + e] = close2(a);
+                        pk[h * 16 + e + 1] = close2(c);
+                        if (blk_end <= half * 64) {           // all of them behind the own block
+                            sum = add2(sum, add2(a, c));
+                        } else {
+                            float a0, a1, c0, c1;
+                            unpack2(a, a0, a1);
+                            unpack2(c, c0, c1);
+                            const int at = half * 64 + h * 32 + 2 * e;
+                            dn += ((at >= blk_end ? a0 : 0.f) + (at + 1 >= blk_end ? a1 : 0.f)) + ((at + 2 >= blk_end ? c0 : 0.f) + (at + 3 >= blk_end ? c1 : 0.f));
+                        }
+                    }
+                }
+                dn += hsum2(sum);
+                tmem_st32(t_dp, pk);
+                tmem_st_wait();
+            }
+            tc_fence_before();
+            arrive(bar_ds);
+            if (lane == 0) mbar_arrive(st_empty + (ni & 1) * 8);
+            ++ni;
+            if (!(f & BKV_LAST)) continue;
+            ok = warp_wait(bar_acc, pairs & 1);
+            if (!ok) break;
+            ++pairs;
+            tc_fence_after();
+            flush(d.z, f);
+            finish((f & (BKV_ANY0 << u)) != 0, true);
+            release_acc();
+            if (warp == 2) {                                  // in front of its part in the next step, behind which others flush again
+                if (f & BKV_SUMS) ok = warp_wait(bar_acc_free, pairs & 1);
                 if (!ok) break;
-                item_write();
-                if (w.u) dn[1] += add; else dn[0] += add;
-            }
-            flush(gi);
-            if (ok && i > 0) ok = warp_wait(bar_acc, (i - 1) & 1);
-#pragma unroll 1
-            for (int u = 0; u < (tile[1] >= 0 ? 2 : 1); ++u) finish(s_tile[u], u, has_items(u), ok);
-        } else if (!own) {
-#pragma unroll 1
-            for (int u = 0; u < n_own; ++u) finish(s_tile[u], 0, false, true);
-        } else {
-            int done = 0;                                     // tiles written
-            float unused = 0.f;
-            bool more = ow.begin();
-#pragma unroll 1
-            while (true) {
-                if (more) {
-                    load_rows(ow.gi, ow.qt);
-                    if (ok) ok = item_p(i, s_tile[ow.u], ow.qt, false, unused);
-                } else if (ok) {
-                    ok = warp_wait(bar_acc, (i - 1) & 1);
-                }
-                if (!more || ow.u > done) {                   // the previous item was its tile's last
-                    finish(s_tile[done], done & 1, true, ok);
-                    ++done;
-                }
-                if (!more) break;
-                if (ok) item_write();
-                more = ow.next();
-                ++i;
+                write_sums((f & BKV_SUMS) != 0);
             }
         }
-        asm volatile("bar.sync 1, 256;" ::: "memory");       // every softmax warp reaches it, also after a failed wait
-        const int n_tiles = paired ? 2 : n_own;
-#pragma unroll 1
-        for (int e = tid - 64; e < n_tiles * G; e += 256) {
-            const int u = e / G, gi = e % G;
-            if (s_tile[u] < 0) continue;
-            const float* p = s_dn + (u * BKV_MAXG + gi) * 8;
-            dnats_part[((long)b * NT + s_tile[u]) * HQ + hkv * G + gi] =
-                paired ? ((p[0] + p[1]) + (p[2] + p[3])) + ((p[4] + p[5]) + (p[6] + p[7])) : 0.f;
-        }
+        if (lane == 0) tma_store_wait_read();
+        __syncwarp();
     }
+    // ---------------------------------------------------------------- teardown
     if (!ok && lane == 0) atomicExch(status, NATSL_DEV_WAIT_TIMEOUT);
     tc_fence_before();
     __syncthreads();
@@ -914,12 +989,14 @@ static int launch_attn_bwd(const void* q, const void* k, const void* v, const vo
         set_error("natsl_attn_bwd: cannot reserve %d B of shared memory (%s)", smem, cudaGetErrorString(e));
         return NATSL_ERR_CUDA;
     }
-    CUtensorMap mq, mk, mv, mdo;
+    CUtensorMap mq, mk, mv, mdo, mdk, mdv;
     int* status = nullptr;
     int rc = encode_bthd_map(&mq, q, B, T, HQ, DK, 128, "natsl_attn_bwd(q)");
     if (rc == NATSL_OK) rc = encode_bthd_map(&mk, k, B, T, HKV, DK, 64, "natsl_attn_bwd(k)");
     if (rc == NATSL_OK) rc = encode_bthd_map(&mv, v, B, T, HKV, DV, 64, "natsl_attn_bwd(v)");
     if (rc == NATSL_OK) rc = encode_bthd_map(&mdo, d_o, B, T, HQ, DV, 128, "natsl_attn_bwd(do)");
+    if (rc == NATSL_OK) rc = encode_bthd_map(&mdk, dk, B, T, HKV, DK, 32, "natsl_attn_bwd(dk)");
+    if (rc == NATSL_OK) rc = encode_bthd_map(&mdv, dv, B, T, HKV, DV, 32, "natsl_attn_bwd(dv)");
     if (rc == NATSL_OK) rc = status_word_ptr(&status);
     if (rc != NATSL_OK) return rc;
     auto bf = [](const void* p) { return reinterpret_cast<const __nv_bfloat16*>(p); };
@@ -928,11 +1005,9 @@ static int launch_attn_bwd(const void* q, const void* k, const void* v, const vo
                                                   delta, T, HQ, HKV, HN, TN, nbs, scale, own, status);
     rc = check_launch("natsl_attn_bwd (dq)");
     if (rc != NATSL_OK) return rc;
-    // ceil(n / 2) + ceil((NT - n) / 8) CTAs per head for n selected tiles, known on the device only
-    const int per_head = NT / 2 + 1, heads = HKV * B;
-    k2<<<per_head * heads, TC_THREADS, DkvSmem<DK, DV>::total, st>>>(
-        mq, mk, mv, mdo, lse, delta, types_i, reinterpret_cast<__nv_bfloat16*>(dk), reinterpret_cast<__nv_bfloat16*>(dv), dnats_part, T,
-        HQ, HKV, HN, TN, nbs, scale, own, heads, per_head, status);
+    const int per_head = (NT + 1) / 2, heads = HKV * B;      // pairs of key tiles
+    k2<<<per_head * heads, BKV_THREADS, DkvSmem<DK, DV>::total, st>>>(mq, mk, mv, mdo, mdk, mdv, lse, delta, types_i, dnats_part, T, HQ,
+                                                                      HKV, HN, TN, nbs, scale, own, heads, per_head, status);
     return check_launch("natsl_attn_bwd (dk, dv)");
 }
 
