@@ -14,9 +14,12 @@
 //     the programmatic-launch wait.
 //   * core: three kinds of CTA in one grid.  Every CTA recomputes the short convolution of the channels it needs (four
 //     taps), which costs less than a launch in between, and loads everything but the projections (states, tails, weights,
-//     the first keys) before it waits for them.  The recurrence reads the state once: S^T k and S^T q are formed
+//     the first keys and values) before it waits for them.  The recurrence reads the state once: S^T k and S^T q are formed
 //     together (o = e^g S^T q + (q.k) v').  Attention splits the 64-key units of the finished blocks over CTAs; a warp
-//     takes 16 keys of a unit, K and V loads of all of them in flight.
+//     takes 16 keys of a unit, several units on their way through shared memory.
+//     On the device, from the first projection to the output (us, by time stamps; before: one step of 8 or 16 keys ahead in
+//     registers, ranges of units per split, all mixing rows in one CTA, attention first): 1 row, 777 tokens, 16 heads of 128 22.0 ->
+//     20.4; 32 rows, 2048 tokens, 16 heads of 64 50.6 -> 47.2; 4 rows, 1030 tokens, 32 heads of 128 / 64 37.9 -> 34.1.
 //   * merge: combines the splits, both RMS norms, mixing weights and gate; extra CTAs shift the convolution tails.
 // All state (recurrent state, tails, decay sums, pooled input, key/value rows) is updated in place.
 #include "common.cuh"
@@ -29,7 +32,7 @@ namespace {
 using bf16 = __nv_bfloat16;
 constexpr int DS_THREADS = 128;               // core CTAs
 constexpr int DS_MAXK = 256;
-constexpr int DS_MIX = 512;                   // channels per CTA of the mixing logits
+constexpr int DS_MIX = 512, DS_MIX_ROWS = 16; // channels and rows per CTA of the mixing logits
 constexpr float kLog2e = 1.4426950408889634f;
 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -153,7 +156,7 @@ struct CoreArgs {
     float* wlog;                              // [B, n_slices, 2*HQ] partial mixing logits
     float* part;                              // [B, HQ, S, DV + 2]
     float* gnew;                              // [B, H]
-    int NR, S, n_attn, n_rec, vs, n_slices;
+    int NR, S, n_mix, n_attn, n_rec, attn0, rec0, vs, n_slices;
 };
 
 // What a convolution needs besides the new input: the tail (the last four inputs), weights, bias.  None of it is written by
@@ -188,6 +191,25 @@ __device__ __forceinline__ float block_sum(float v, float* s_red, int tid) {
 #pragma unroll
     for (int i = 0; i < NTHR / 32; ++i) r += s_red[i];
     return r;
+}
+
+// Two sums over the block with one pair of barriers; s_red: 2 x NTHR / 32 floats.
+template <int NTHR>
+__device__ __forceinline__ void block_sum2(float& u, float& v, float* s_red, int tid) {
+    u = warp_sum(u);
+    v = warp_sum(v);
+    __syncthreads();
+    if ((tid & 31) == 0) {
+        s_red[tid >> 5] = u;
+        s_red[NTHR / 32 + (tid >> 5)] = v;
+    }
+    __syncthreads();
+    u = v = 0.f;
+#pragma unroll
+    for (int i = 0; i < NTHR / 32; ++i) {
+        u += s_red[i];
+        v += s_red[NTHR / 32 + i];
+    }
 }
 
 // VS value columns (32 or 64) per CTA: rows of the state rg + RP i, four columns per thread.
@@ -252,8 +274,7 @@ __device__ void core_recurrence(const CoreArgs& c, int idx, float* sm) {
         if (!gdn) vv = rb(vv * sp);
         s_v[tid] = vv;
     }
-    sq = block_sum<DS_THREADS>(sq, s_red, tid);
-    sk = block_sum<DS_THREADS>(sk, s_red + 4, tid);
+    block_sum2<DS_THREADS>(sq, sk, s_red, tid);
     const float eps = gdn ? 1e-6f : a.l2_eps;
     const float rq = rsqrtf(sq + eps), rk = rsqrtf(sk + eps);
     float qk = 0.f;
@@ -325,6 +346,17 @@ __device__ void core_recurrence(const CoreArgs& c, int idx, float* sm) {
     if (vs == 0 && tid == 0) c.gnew[(long)b * H + h] = gt;
 }
 
+__device__ __forceinline__ float warp_max_redux(float x) {
+    float y;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// Ring of a warp of the attention: steps of 16 keys; three of them where four CTAs then still share an SM, else two.
+template <int DK, int DV> struct Ring {
+    static constexpr int step = 16 * (DK + DV) * 2, D = DK + DV == 128 ? 3 : 2, bytes = 4 * D * step;
+};
+
 template <int DK, int DV>
 __device__ void core_attention(const CoreArgs& c, int idx, float* sm) {
     const Args& a = c.a;
@@ -335,70 +367,96 @@ __device__ void core_attention(const CoreArgs& c, int idx, float* sm) {
     float* s_q = sm;                                   // [DK] query, scaled
     float* s_kn = s_q + DK;                            // [DK] new key
     float* s_vn = s_kn + DK;                           // [DV] new value
-    float* s_p = s_vn + DV;                            // [4][16]
-    float* s_ml = s_p + 64;                            // [4][2]
+    float* s_ml = s_vn + DV;                           // [4][2]
     float* s_red = s_ml + 8;                           // [8]
     float* s_acc = s_red + 8;                          // [4][DV]
     const bool last = s == c.S - 1;
-    float m = -INFINITY, l = 0.f, acc[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) acc[e] = 0.f;
+    float m = -INFINITY, l = 0.f;
+    uint64_t acc2[4] = {0, 0, 0, 0};
     const bf16* kb = a.k_cache + ((long)b * a.cap * a.HQ + hq) * DK + (lane % LK) * 8;
     const bf16* vb = a.v_cache + ((long)b * a.cap * a.HQ + hq) * DV + (lane % LV) * 8;
-    float* my_p = s_p + warp * 16;
-    // A step of a warp = KS keys, four 16-byte K loads and as many V loads as their width takes, with the next step's loads
-    // in flight while this one is computed.  Steps: the warp's quarter of every selected 64-key unit of this split (32 units'
-    // selection bits per load, by ballot), then of the current block.
-    constexpr int KM = KG < VG ? KG : VG, KS = 4 * KM < 16 ? 4 * KM : 16, NK = KS / KG, NV = KS / VG;
-    static_assert(NK >= 1 && NV >= 1, "lanes per row");
+    // A step of a warp = 16 keys, its quarter of a selected 64-key unit of this split (32 units' selection bits per load, by ballot),
+    // then of the current block.  Keys and values come through the warp's own ring in shared memory, D steps deep: the first D are
+    // on their way before the wait for the projections, and a split of few units is no chain of loads (one step ahead in
+    // registers, 8 keys at head dims 128, it was: 4 rows of 32 heads, 1030 tokens: attention 14.5 us behind the wait).
+    using R = Ring<DK, DV>;
+    constexpr int D = R::D, KS = 16, NK = KS / KG, NV = KS / VG;
+    static_assert(LK >= NK && NV >= 1, "lanes per row");
+    extern __shared__ __align__(16) unsigned char ring_all[];
+    unsigned char* const ring = ring_all + warp * (D * R::step);
+    const uint32_t ring_s = smem_u32(ring);
     const int hn = hq / (a.HQ / a.HN), upb = a.nbs / 64;
     const int n_units = a.n_done * upb;
-    const int u0 = (int)((long)n_units * s / c.S), u1 = (int)((long)n_units * (s + 1) / c.S);
-    const int own0 = (last && a.own_chunk) ? a.pos / a.nbs * a.nbs : a.pos;     // keys of the current block before the new token
+    const int own0 = a.own_chunk ? a.pos / a.nbs * a.nbs : a.pos;               // keys of the current block before the new token
     const long tstride = (long)a.HN * 2;
     const long tbase = ((long)b * a.n_done * a.HN + hn) * 2;
-    unsigned mask = 0;
-    int base = u0 - 32, sub = 0, unit = -1, own = own0 + warp * 16;
-    auto next = [&](int& key0, int& n) -> bool {
-        if (unit >= 0 && sub + KS < 16) {                                       // rest of the warp's 16 keys of this unit
-            sub += KS;
-            key0 = unit * 64 + warp * 16 + sub;
-            n = KS;
-            return true;
+    auto chosen = [&](int u, int end) -> bool { return u < end && ldw(a.types, a.types_f32, tbase + (long)(u / upb) * tstride) > 0.5f; };
+    // Which units are this split's.  Up to 128 (8192 tokens) every split reads all selection bits and takes every S-th selected unit,
+    // then every S-th unit of the current block: equal shares, where a range of its own holds none of them or all (4 rows of 32
+    // heads, 16 units over 5 splits: the last CTA had twice the mean).  Beyond, a range of its own, 32 units at a time.
+    constexpr int FEW = 4;
+    const bool few = n_units <= FEW * 32;
+    unsigned mask = 0, more[FEW - 1] = {0, 0, 0};       // units base .. base + 31 that are left, and the words behind
+    int base = 0, end = 0, own_unit = last ? 0 : 1 << 20, own_step = 1;
+    if (few) {
+        bool sel[FEW];
+#pragma unroll
+        for (int i = 0; i < FEW; ++i) sel[i] = chosen(i * 32 + lane, n_units);
+        int rank = 0;                                   // selected units so far, modulo S
+#pragma unroll
+        for (int i = 0; i < FEW; ++i) {
+            const unsigned all = __ballot_sync(0xffffffffu, sel[i]);
+            const unsigned m = __ballot_sync(0xffffffffu, sel[i] && (rank + __popc(all & ((1u << lane) - 1))) % c.S == s);
+            rank = (rank + __popc(all)) % c.S;
+            if (i == 0) mask = m;
+            else more[i - 1] = m;
         }
-        while (mask == 0 && base + 32 < u1) {
+        own_unit = s - rank + (s < rank ? c.S : 0);
+        own_step = c.S;
+        end = n_units;
+    } else {
+        end = (int)((long)n_units * (s + 1) / c.S);
+        base = (int)((long)n_units * s / c.S) - 32;
+    }
+    auto next = [&](int& key0) -> int {                 // keys of the warp's next step, 0 at the end
+        while (mask == 0 && base + 32 < end) {
             base += 32;
-            const int u = base + lane;
-            mask = __ballot_sync(0xffffffffu, u < u1 && ldw(a.types, a.types_f32, tbase + (long)(u / upb) * tstride) > 0.5f);
+            if (few) {
+                mask = more[0];
+#pragma unroll
+                for (int i = 0; i + 2 < FEW; ++i) more[i] = more[i + 1];
+                more[FEW - 2] = 0;
+            } else {
+                mask = __ballot_sync(0xffffffffu, chosen(base + lane, end));
+            }
         }
         if (mask) {
-            unit = base + __ffs(mask) - 1;
+            key0 = (base + __ffs(mask) - 1) * 64 + warp * 16;
             mask &= mask - 1;
-            sub = 0;
-            key0 = unit * 64 + warp * 16;
-            n = KS;
-            return true;
+            return KS;
         }
-        unit = -1;
-        if (own >= a.pos) return false;
-        key0 = own;
-        n = min(KS, a.pos - own);
-        const int in = (own - own0) & 15;
-        own += in + KS < 16 ? KS : 64 - in;
-        return true;
+        key0 = own0 + own_unit * 64 + warp * 16;
+        if (own_unit >= 1 << 20 || key0 >= a.pos) return 0;
+        own_unit += own_step;
+        return min(KS, a.pos - key0);
     };
-    auto fetch = [&](int key0, int n, uint4 (&kr)[NK], uint4 (&vr)[NV]) {
+    auto fetch = [&](int slot) -> int {                 // the next step into `slot`; always one group of copies
+        int key0 = 0;
+        const int n = next(key0);
+        if (n > 0) {
+            const uint32_t dst = ring_s + slot * R::step + lane * 16;
 #pragma unroll
-        for (int i = 0; i < NK; ++i)
-            kr[i] = *reinterpret_cast<const uint4*>(kb + (long)(key0 + min(i * KG + lane / LK, n - 1)) * a.HQ * DK);
+            for (int i = 0; i < NK; ++i) cp_async16(dst + i * 512, kb + (long)(key0 + min(i * KG + lane / LK, n - 1)) * a.HQ * DK, 16);
 #pragma unroll
-        for (int i = 0; i < NV; ++i)
-            vr[i] = *reinterpret_cast<const uint4*>(vb + (long)(key0 + min(i * VG + lane / LV, n - 1)) * a.HQ * DV);
+            for (int i = 0; i < NV; ++i)
+                cp_async16(dst + KS * DK * 2 + i * 512, vb + (long)(key0 + min(i * VG + lane / LV, n - 1)) * a.HQ * DV, 16);
+        }
+        cp_async_commit();
+        return n;
     };
-    uint4 k0[NK], v0[NV], k1[NK], v1[NV];
-    int key0 = 0, n0 = 0, n1 = 0;
-    bool more0 = next(key0, n0), more1 = false;
-    if (more0) fetch(key0, n0, k0, v0);
+    int count[D];                                       // keys of the steps on their way
+#pragma unroll
+    for (int i = 0; i < D; ++i) count[i] = fetch(i);
 
     // ---- query of this head, and (last split) the new token's key and value: they wait for the projections
     {
@@ -423,8 +481,8 @@ __device__ void core_attention(const CoreArgs& c, int idx, float* sm) {
             vv = cv(vv, a.silu);
         }
         if (a.qn_w) {
-            const float sq = block_sum<DS_THREADS>(tid < DK ? qv * qv : 0.f, s_red, tid);
-            const float sk = block_sum<DS_THREADS>(tid < DK ? kv * kv : 0.f, s_red + 4, tid);
+            float sq = tid < DK ? qv * qv : 0.f, sk = tid < DK ? kv * kv : 0.f;
+            block_sum2<DS_THREADS>(sq, sk, s_red, tid);
             qv = rb(qv * rsqrtf(sq / DK + a.norm_eps) * wq);
             kv = rb(kv * rsqrtf(sk / DK + a.norm_eps) * wk);
         }
@@ -439,66 +497,87 @@ __device__ void core_attention(const CoreArgs& c, int idx, float* sm) {
         }
     }
     __syncthreads();
-    float q8[8];
+    uint64_t q2[4];
     {
         const int d0 = (lane % LK) * 8;
 #pragma unroll
-        for (int e = 0; e < 8; ++e) q8[e] = s_q[d0 + e];
+        for (int e = 0; e < 4; ++e) q2[e] = pack2(s_q[d0 + 2 * e], s_q[d0 + 2 * e + 1]);
     }
-    auto step = [&](const uint4 (&kr)[NK], const uint4 (&vr)[NV], int n_keys) {
+    // Scores: a row's LK lanes each hold a part of its dot product.  The lanes hand half of their rows' parts to each other until one
+    // row is left per lane (eight shuffles for eight rows of sixteen lanes, where summing row by row takes 32), so that a lane
+    // has the score of one key, my_key, shared with LK / NK - 1 others, and the probabilities need no shared memory.
+    int my_key = lane / LK, src[NV];                    // src: lane that has the probability of this lane's i-th value row
+#pragma unroll
+    for (int n = NK, o = LK / 2; n > 1; n >>= 1, o >>= 1) my_key += (lane & o) ? n / 2 * KG : 0;
+    const bool counts = (lane & (LK / NK - 1)) == 0;    // one of the lanes that share a key
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const int key = i * VG + lane / LV;
+        src[i] = key % KG * LK;
+#pragma unroll
+        for (int n = NK, o = LK / 2; n > 1; n >>= 1, o >>= 1) src[i] += (key / KG) & (n / 2) ? o : 0;
+    }
+    auto step = [&](const unsigned char* at, int n_keys) {
+        float d[NK];
 #pragma unroll
         for (int i = 0; i < NK; ++i) {
-            const uint32_t* w = reinterpret_cast<const uint32_t*>(&kr[i]);
-            float d = 0.f;
+            const uint4 kr = *reinterpret_cast<const uint4*>(at + i * 512 + lane * 16);
+            const uint32_t* w = reinterpret_cast<const uint32_t*>(&kr);
+            uint64_t x = mul2(open2(w[0]), q2[0]);
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float2 f = unpack_bf16(w[e]);
-                d += f.x * q8[2 * e];
-                d += f.y * q8[2 * e + 1];
-            }
-#pragma unroll
-            for (int o = LK / 2; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-            if (lane % LK == 0) my_p[i * KG + lane / LK] = d;
+            for (int e = 1; e < 4; ++e) x = fma2(open2(w[e]), q2[e], x);
+            d[i] = hsum2(x);
         }
-        __syncwarp();
-        const float sc = (lane & (KS - 1)) < n_keys ? my_p[lane & (KS - 1)] : -INFINITY;
-        float mx = sc;
+        int o = LK / 2;
 #pragma unroll
-        for (int o = KS / 2; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        for (int n = NK; n > 1; n >>= 1, o >>= 1) {
+            const bool hi = (lane & o) != 0;
+#pragma unroll
+            for (int i = 0; i < n / 2; ++i) {
+                const float keep = hi ? d[i + n / 2] : d[i], give = hi ? d[i] : d[i + n / 2];
+                d[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+            }
+        }
+#pragma unroll
+        for (int r = LK / NK / 2; r > 0; r >>= 1) d[0] += __shfl_xor_sync(0xffffffffu, d[0], r);
+        const float sc = my_key < n_keys ? d[0] : -INFINITY;
         // scores of -inf (infinite keys) weigh nothing, also while there is nothing else
-        const float mn = fmaxf(m, mx), al = mn == -INFINITY ? 1.f : exp2f(m - mn);
-        const float p = sc == -INFINITY ? 0.f : exp2f(sc - mn);
-        float ps = p;
+        const float mn = fmaxf(m, warp_max_redux(sc));
+        if (mn != m) {                                  // (the same in all lanes)
+            const float al = mn == -INFINITY ? 1.f : exp2f(m - mn);
+            l *= al;
 #pragma unroll
-        for (int o = KS / 2; o > 0; o >>= 1) ps += __shfl_xor_sync(0xffffffffu, ps, o);
-        l = l * al + ps;
-        m = mn;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) acc[e] *= al;
+            for (int e = 0; e < 4; ++e) acc2[e] = mul2(acc2[e], pack2(al, al));
+            m = mn;
+        }
+        const float p = sc == -INFINITY ? 0.f : exp2f(sc - m);
+        l += counts ? p : 0.f;
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
-            const float pj = __shfl_sync(0xffffffffu, p, i * VG + lane / LV);
-            const uint32_t* w = reinterpret_cast<const uint32_t*>(&vr[i]);
+            const float pj = __shfl_sync(0xffffffffu, p, src[i]);
+            const uint4 vr = *reinterpret_cast<const uint4*>(at + KS * DK * 2 + i * 512 + lane * 16);
+            const uint32_t* w = reinterpret_cast<const uint32_t*>(&vr);
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float2 f = unpack_bf16(w[e]);
-                acc[2 * e] += pj * f.x;
-                acc[2 * e + 1] += pj * f.y;
-            }
+            for (int e = 0; e < 4; ++e) acc2[e] = fma2(pack2(pj, pj), open2(w[e]), acc2[e]);
         }
-        __syncwarp();
     };
-    // two register buffers in turn (a copy from one to the other would wait for its loads before the next ones are issued)
-    while (more0) {
-        more1 = next(key0, n1);
-        if (more1) fetch(key0, n1, k1, v1);
-        step(k0, v0, n0);
-        if (!more1) break;
-        more0 = next(key0, n0);
-        if (more0) fetch(key0, n0, k0, v0);
-        step(k1, v1, n1);
+    int slot = 0;
+    while (count[0] > 0) {
+        cp_async_wait<D - 1>();
+        __syncwarp();
+        step(ring + slot * R::step, count[0]);
+        __syncwarp();                                   // every lane has read the slot
+#pragma unroll
+        for (int i = 0; i + 1 < D; ++i) count[i] = count[i + 1];
+        count[D - 1] = fetch(slot);
+        slot = slot + 1 == D ? 0 : slot + 1;
     }
+    cp_async_wait<0>();
     // sum the key groups of a warp, then the warps
+    l = warp_sum(l);
+    float acc[8];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) unpack2(acc2[e], acc[2 * e], acc[2 * e + 1]);
 #pragma unroll
     for (int o = LV; o < 32; o <<= 1)
 #pragma unroll
@@ -533,20 +612,30 @@ __device__ void core_attention(const CoreArgs& c, int idx, float* sm) {
     }
 }
 
-// Partial logits of the mixing weights: all rows of w_mix [2 HQ, H K] times one slice of DS_MIX channels of the convolved
-// query of one batch row (the merge adds the slices up; whole rows per CTA took 16 us at H K = 4096, a chain of 32
-// convolutions per thread).
+// Partial logits of the mixing weights: DS_MIX_ROWS rows of w_mix [2 HQ, H K] times one slice of DS_MIX channels of the convolved
+// query of one batch row (the merge adds the slices up).  A CTA's weights, four rows a warp, are on their way before the wait for the
+// projections; all rows in one CTA took 11 us from there, four rounds of loads one after the other.
 __device__ void core_mix_logits(const CoreArgs& c, int idx, float* sm) {
     const Args& a = c.a;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int HK = a.H * a.K, rows = 2 * a.HQ, slice = idx % c.n_slices, b = idx / c.n_slices, d0 = slice * DS_MIX;
-    constexpr int PER = DS_MIX / DS_THREADS;
+    const int HK = a.H * a.K, rows = 2 * a.HQ, groups = (rows + DS_MIX_ROWS - 1) / DS_MIX_ROWS;
+    const int r0 = idx % groups * DS_MIX_ROWS + warp * (DS_MIX_ROWS / 4), slice = idx / groups % c.n_slices, b = idx / (groups * c.n_slices);
+    const int d0 = slice * DS_MIX;
+    constexpr int PER = DS_MIX / DS_THREADS, RW = DS_MIX_ROWS / 4;
     Conv cq[PER];
 #pragma unroll
     for (int j = 0; j < PER; ++j) {
         const int d = min(d0 + tid + j * DS_THREADS, HK - 1);
         cq[j].load(a.conv_q, a.cw_q, a.cb_q, (long)b * HK + d, d);
     }
+    uint4 wr[RW][DS_MIX / 256];                             // channels (lane + 32 i) * 8 .. + 7
+#pragma unroll
+    for (int r = 0; r < RW; ++r)
+#pragma unroll
+        for (int i = 0; i < DS_MIX / 256; ++i) {
+            const int d = d0 + (lane + 32 * i) * 8;
+            wr[r][i] = d < HK && r0 + r < rows ? *reinterpret_cast<const uint4*>(a.w_mix + (long)(r0 + r) * HK + d) : make_uint4(0, 0, 0, 0);
+        }
     pdl_wait();
     float x[PER];
 #pragma unroll
@@ -554,47 +643,44 @@ __device__ void core_mix_logits(const CoreArgs& c, int idx, float* sm) {
 #pragma unroll
     for (int j = 0; j < PER; ++j) sm[tid + j * DS_THREADS] = d0 + tid + j * DS_THREADS < HK ? cq[j](x[j], a.silu) : 0.f;
     __syncthreads();
-    float q[DS_MIX / 32];                                   // channels (lane + 32 i) * 8 .. + 7
+    float acc[RW];
 #pragma unroll
-    for (int i = 0; i < DS_MIX / 256; ++i)
+    for (int r = 0; r < RW; ++r) acc[r] = 0.f;
 #pragma unroll
-        for (int e = 0; e < 8; ++e) q[i * 8 + e] = sm[(lane + 32 * i) * 8 + e];
-#pragma unroll 4
-    for (int r = warp; r < rows; r += DS_THREADS / 32) {
-        float acc = 0.f;
+    for (int i = 0; i < DS_MIX / 256; ++i) {
+        if (d0 + (lane + 32 * i) * 8 >= HK) continue;
+        float q[8];
 #pragma unroll
-        for (int i = 0; i < DS_MIX / 256; ++i) {
-            const int d = d0 + (lane + 32 * i) * 8;
-            if (d < HK) {
-                const uint4 v = *reinterpret_cast<const uint4*>(a.w_mix + (long)r * HK + d);
-                const uint32_t* w = reinterpret_cast<const uint32_t*>(&v);
+        for (int e = 0; e < 8; ++e) q[e] = sm[(lane + 32 * i) * 8 + e];
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float2 f = unpack_bf16(w[e]);
-                    acc += f.x * q[i * 8 + 2 * e];
-                    acc += f.y * q[i * 8 + 2 * e + 1];
-                }
+        for (int r = 0; r < RW; ++r) {
+            const uint32_t* w = reinterpret_cast<const uint32_t*>(&wr[r][i]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float2 f = unpack_bf16(w[e]);
+                acc[r] += f.x * q[2 * e];
+                acc[r] += f.y * q[2 * e + 1];
             }
         }
-        acc = warp_sum(acc);
-        if (lane == 0) c.wlog[((long)b * c.n_slices + slice) * rows + r] = acc;
+    }
+#pragma unroll
+    for (int r = 0; r < RW; ++r) {
+        const float v = warp_sum(acc[r]);
+        if (lane == 0 && r0 + r < rows) c.wlog[((long)b * c.n_slices + slice) * rows + r0 + r] = v;
     }
 }
 
 template <int DK, int DV>
 __global__ void __launch_bounds__(DS_THREADS, 4) decode_core_kernel(const CoreArgs c) {
     __shared__ __align__(16) float sm[2 * DS_MAXK + 64 + 8 + 2 * DS_THREADS * 4];
-    static_assert(2 * DK + DV + 64 + 16 + 4 * DV <= 2 * DS_MAXK + 64 + 8 + 2 * DS_THREADS * 4, "attention scratch");
+    static_assert(2 * DK + DV + 16 + 4 * DV <= 2 * DS_MAXK + 64 + 8 + 2 * DS_THREADS * 4, "attention scratch");
     pdl_trigger();
-    int idx = blockIdx.x;
-    if (idx < c.n_attn) {
-        core_attention<DK, DV>(c, idx, sm);
-    } else if (idx < c.n_attn + c.n_rec) {
-        if (c.vs == 64) core_recurrence<64>(c, idx - c.n_attn, sm);
-        else core_recurrence<32>(c, idx - c.n_attn, sm);
-    } else {
-        core_mix_logits(c, idx - c.n_attn - c.n_rec, sm);
-    }
+    // The mixing logits first, then the longer of recurrence and attention (rec0, attn0: their first CTAs).
+    const int idx = blockIdx.x;
+    if (idx < c.n_mix) core_mix_logits(c, idx, sm);
+    else if (idx >= c.attn0 && idx < c.attn0 + c.n_attn) core_attention<DK, DV>(c, idx - c.attn0, sm);
+    else if (c.vs == 64) core_recurrence<64>(c, idx - c.rec0, sm);
+    else core_recurrence<32>(c, idx - c.rec0, sm);
 }
 
 // ------------------------------------------------------------------------------------------------ merge
@@ -655,27 +741,47 @@ __global__ void __launch_bounds__(128) decode_merge_kernel(const MergeArgs c) {
         gg[e] = bf(c.raw, (long)b * c.NR + 2 * HK + HV + d0 + e);
         o[e] = 0.f;
     }
+    // splits s = lane, lane + 32 (at most 64); the values of the first four are on their way before their weights are known
+    constexpr int AHEAD = 4;
+    float m0 = -INFINITY, m1 = -INFINITY, s0 = 0.f, s1 = 0.f, pv[AHEAD][E];
+    if (lane < c.S) { m0 = part[(long)lane * (DV + 2)]; s0 = part[(long)lane * (DV + 2) + 1]; }
+    if (lane + 32 < c.S) { m1 = part[(long)(lane + 32) * (DV + 2)]; s1 = part[(long)(lane + 32) * (DV + 2) + 1]; }
+#pragma unroll
+    for (int s = 0; s < AHEAD; ++s)
+#pragma unroll
+        for (int e = 0; e < E; ++e) pv[s][e] = s < c.S ? part[(long)s * (DV + 2) + 2 + lane * E + e] : 0.f;
     float l1 = 0.f, l2 = 0.f;
-    if (a.w_mix) {
+    if (a.w_mix) {                                       // slices by lane, summed in their order
+        float2 wl = make_float2(0.f, 0.f);
+        if (lane < c.n_slices) wl = *reinterpret_cast<const float2*>(c.wlog + (((long)b * c.n_slices + lane) * a.HQ + hq) * 2);
         for (int k = 0; k < c.n_slices; ++k) {
-            const float2 w = *reinterpret_cast<const float2*>(c.wlog + (((long)b * c.n_slices + k) * a.HQ + hq) * 2);
+            float2 w;
+            if (k < 32) {
+                w.x = __shfl_sync(0xffffffffu, wl.x, k);
+                w.y = __shfl_sync(0xffffffffu, wl.y, k);
+            } else {
+                w = *reinterpret_cast<const float2*>(c.wlog + (((long)b * c.n_slices + k) * a.HQ + hq) * 2);
+            }
             l1 += w.x;
             l2 += w.y;
         }
         l1 = rb(l1);
         l2 = rb(l2);
     }
-    // splits s = lane, lane + 32 (at most 64)
-    float m0 = -INFINITY, m1 = -INFINITY, s0 = 0.f, s1 = 0.f;
-    if (lane < c.S) { m0 = part[(long)lane * (DV + 2)]; s0 = part[(long)lane * (DV + 2) + 1]; }
-    if (lane + 32 < c.S) { m1 = part[(long)(lane + 32) * (DV + 2)]; s1 = part[(long)(lane + 32) * (DV + 2) + 1]; }
     float M = fmaxf(m0, m1);
 #pragma unroll
     for (int k = 16; k > 0; k >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, k));
     const float f0 = m0 == -INFINITY ? 1.f : exp2f(m0 - M), f1 = m1 == -INFINITY ? 1.f : exp2f(m1 - M);
     const float L = warp_sum(f0 * s0 + f1 * s1);
+#pragma unroll
+    for (int s = 0; s < AHEAD; ++s) {
+        if (s >= c.S) break;
+        const float f = __shfl_sync(0xffffffffu, f0, s);
+#pragma unroll
+        for (int e = 0; e < E; ++e) o[e] += f * pv[s][e];
+    }
 #pragma unroll 4
-    for (int s = 0; s < c.S; ++s) {
+    for (int s = AHEAD; s < c.S; ++s) {
         const float f = __shfl_sync(0xffffffffu, s < 32 ? f0 : f1, s & 31);
         const float* p = part + (long)s * (DV + 2) + 2 + lane * E;
 #pragma unroll
@@ -705,10 +811,12 @@ __global__ void __launch_bounds__(128) decode_merge_kernel(const MergeArgs c) {
 
 // ------------------------------------------------------------------------------------------------ host
 template <typename Arg>
-cudaError_t launch_pdl(void (*kern)(const Arg), unsigned grid, unsigned block, cudaStream_t st, const Arg& arg, bool overlap = true) {
+cudaError_t launch_pdl(void (*kern)(const Arg), unsigned grid, unsigned block, cudaStream_t st, const Arg& arg, bool overlap = true,
+                       unsigned smem = 0) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -716,6 +824,14 @@ cudaError_t launch_pdl(void (*kern)(const Arg), unsigned grid, unsigned block, c
     cfg.attrs = at;
     cfg.numAttrs = overlap ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kern, arg);
+}
+
+template <int DK, int DV>
+cudaError_t launch_core(const CoreArgs& c, cudaStream_t st) {
+    auto kern = decode_core_kernel<DK, DV>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Ring<DK, DV>::bytes);
+    if (e != cudaSuccess) return e;
+    return launch_pdl(kern, c.n_mix + c.n_rec + c.n_attn, DS_THREADS, st, c, true, Ring<DK, DV>::bytes);
 }
 
 // Row tiles of every segment, then the launch.  Up to 32 batch rows all eight warps share the contraction of 16 weight rows
@@ -848,10 +964,16 @@ extern "C" int natsl_decode_step(const natsl_decode_args* args, void* stream) {
     c.vs = a.K <= 64 && a.V % 64 == 0 && (long)a.B * a.H * (a.V / 32) > 148 * 4 ? 64 : 32;
     c.n_rec = a.B * a.H * (a.V / c.vs);
     c.n_slices = l.slices;
-    const int n_mix = a.w_mix ? a.B * l.slices : 0;
-    auto core = DK == 64 ? (DV == 64 ? decode_core_kernel<64, 64> : decode_core_kernel<64, 128>)
-                         : (DV == 64 ? decode_core_kernel<128, 64> : decode_core_kernel<128, 128>);
-    if (e == cudaSuccess) e = launch_pdl(core, c.n_attn + c.n_rec + n_mix, DS_THREADS, st, c);
+    c.n_mix = a.w_mix ? a.B * l.slices * ((2 * a.HQ + DS_MIX_ROWS - 1) / DS_MIX_ROWS) : 0;
+    // A recurrence CTA takes as long as an attention CTA of some eight 64-key units, half of them selected: below that it goes first
+    // (4 rows of 32 heads, 1030 tokens, 3 units a split, 1024 CTAs over 592 places: a token takes 37.9 us the other way and 34.6 us
+    // this way; 32 rows of 16 heads, 2048 tokens, 16 units: 48.1 us and 53.1 us).
+    const bool rec_first = a.n_done * (a.nbs / 64) <= 8 * l.S;
+    c.rec0 = c.n_mix + (rec_first ? 0 : c.n_attn);
+    c.attn0 = c.n_mix + (rec_first ? c.n_rec : 0);
+    if (e == cudaSuccess)
+        e = DK == 64 ? (DV == 64 ? launch_core<64, 64>(c, st) : launch_core<64, 128>(c, st))
+                     : (DV == 64 ? launch_core<128, 64>(c, st) : launch_core<128, 128>(c, st));
 
     MergeArgs g = {};
     g.a = a;

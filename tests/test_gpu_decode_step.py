@@ -86,6 +86,16 @@ def test_token_kernel_matches_the_general_path(make, args, B, T0):
         assert cache[0].n_tokens == ref_cache[0].n_tokens == T0 + n_new
 
 
+@pytest.mark.parametrize("make,args,B,T0", [
+    (_gdn, dict(hidden=256, heads=4, head_dim=64, expand_v=1, attn_heads=4), 1, 8200),
+    (_mamba, dict(hidden=256, heads=4, head_dim=128, expand_v=0.5, attn_heads=4, nats_block_size=256), 2, 1270),
+])
+def test_token_kernel_over_many_units(make, args, B, T0):
+    """Splits that take every S-th selected unit and unit of the current block (up to 128 units), and ranges of units (beyond);
+    the tokens cross the line, and the end of a block of several units."""
+    test_token_kernel_matches_the_general_path(make, args, B, T0)
+
+
 def test_copied_cache_continues_on_its_own():
     from neuralattentionsearchlinear_b200 import NAtSCache
     torch.manual_seed(1)
