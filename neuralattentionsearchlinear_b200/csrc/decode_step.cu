@@ -18,8 +18,9 @@
 //     together (o = e^g S^T q + (q.k) v').  Attention splits the 64-key units of the finished blocks over CTAs; a warp
 //     takes 16 keys of a unit, several units on their way through shared memory.
 //     On the device, from the first projection to the output (us, by time stamps; before: one step of 8 or 16 keys ahead in
-//     registers, ranges of units per split, all mixing rows in one CTA, attention first): 1 row, 777 tokens, 16 heads of 128 22.0 ->
-//     20.4; 32 rows, 2048 tokens, 16 heads of 64 50.6 -> 47.2; 4 rows, 1030 tokens, 32 heads of 128 / 64 37.9 -> 34.1.
+//     registers, ranges of units per split, all mixing rows in one CTA): 32 rows, 2048 tokens, 16 heads of 64 50.0 -> 42.6; 4 rows,
+//     1030 tokens, 32 heads of 128 / 64 37.9 -> 29.3; 16 rows, 2048 tokens, 16 heads of 128 59.6 -> 51.7; 1 row, 300 tokens, 6 heads of
+//     128 / 256 17.5 -> 16.7.
 //   * merge: combines the splits, both RMS norms, mixing weights and gate; extra CTAs shift the convolution tails.
 // All state (recurrent state, tails, decay sums, pooled input, key/value rows) is updated in place.
 #include "common.cuh"
@@ -156,7 +157,7 @@ struct CoreArgs {
     float* wlog;                              // [B, n_slices, 2*HQ] partial mixing logits
     float* part;                              // [B, HQ, S, DV + 2]
     float* gnew;                              // [B, H]
-    int NR, S, n_mix, n_attn, n_rec, attn0, rec0, vs, n_slices;
+    int NR, S, n_mix, n_attn, n_rec, vs, n_slices;
 };
 
 // What a convolution needs besides the new input: the tail (the last four inputs), weights, bias.  None of it is written by
@@ -352,6 +353,17 @@ __device__ __forceinline__ float warp_max_redux(float x) {
     return y;
 }
 
+// Keys and values leave L2 first: a token reads each of them once, and what stays is weights and states (a token of 32 rows, 2048
+// tokens, 16 heads of 64: 47.1 -> 42.6 us; 16 rows, 16 heads of 128: 58.4 -> 51.7 us).
+__device__ __forceinline__ uint64_t evict_first() {
+    uint64_t p;
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+__device__ __forceinline__ void copy_first(uint32_t dst, const void* src, uint64_t policy) {
+    asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "l"(policy) : "memory");
+}
+
 // Ring of a warp of the attention: steps of 16 keys; three of them where four CTAs then still share an SM, else two.
 template <int DK, int DV> struct Ring {
     static constexpr int step = 16 * (DK + DV) * 2, D = DK + DV == 128 ? 3 : 2, bytes = 4 * D * step;
@@ -385,6 +397,7 @@ __device__ void core_attention(const CoreArgs& c, int idx, float* sm) {
     extern __shared__ __align__(16) unsigned char ring_all[];
     unsigned char* const ring = ring_all + warp * (D * R::step);
     const uint32_t ring_s = smem_u32(ring);
+    const uint64_t hint = evict_first();
     const int hn = hq / (a.HQ / a.HN), upb = a.nbs / 64;
     const int n_units = a.n_done * upb;
     const int own0 = a.own_chunk ? a.pos / a.nbs * a.nbs : a.pos;               // keys of the current block before the new token
@@ -446,10 +459,10 @@ __device__ void core_attention(const CoreArgs& c, int idx, float* sm) {
         if (n > 0) {
             const uint32_t dst = ring_s + slot * R::step + lane * 16;
 #pragma unroll
-            for (int i = 0; i < NK; ++i) cp_async16(dst + i * 512, kb + (long)(key0 + min(i * KG + lane / LK, n - 1)) * a.HQ * DK, 16);
+            for (int i = 0; i < NK; ++i) copy_first(dst + i * 512, kb + (long)(key0 + min(i * KG + lane / LK, n - 1)) * a.HQ * DK, hint);
 #pragma unroll
             for (int i = 0; i < NV; ++i)
-                cp_async16(dst + KS * DK * 2 + i * 512, vb + (long)(key0 + min(i * VG + lane / LV, n - 1)) * a.HQ * DV, 16);
+                copy_first(dst + KS * DK * 2 + i * 512, vb + (long)(key0 + min(i * VG + lane / LV, n - 1)) * a.HQ * DV, hint);
         }
         cp_async_commit();
         return n;
@@ -675,12 +688,13 @@ __global__ void __launch_bounds__(DS_THREADS, 4) decode_core_kernel(const CoreAr
     __shared__ __align__(16) float sm[2 * DS_MAXK + 64 + 8 + 2 * DS_THREADS * 4];
     static_assert(2 * DK + DV + 16 + 4 * DV <= 2 * DS_MAXK + 64 + 8 + 2 * DS_THREADS * 4, "attention scratch");
     pdl_trigger();
-    // The mixing logits first, then the longer of recurrence and attention (rec0, attn0: their first CTAs).
+    // The mixing logits, then attention, then the recurrence, whose CTAs are the shorter ones.  (In turn, so that both end together:
+    // tokens of 32 rows, 2048 tokens, 47.1 -> 49.8 us, 16 rows of 128 / 128 61 -> 65 us; the recurrence first: 50.8 and 65 us.)
     const int idx = blockIdx.x;
     if (idx < c.n_mix) core_mix_logits(c, idx, sm);
-    else if (idx >= c.attn0 && idx < c.attn0 + c.n_attn) core_attention<DK, DV>(c, idx - c.attn0, sm);
-    else if (c.vs == 64) core_recurrence<64>(c, idx - c.rec0, sm);
-    else core_recurrence<32>(c, idx - c.rec0, sm);
+    else if (idx < c.n_mix + c.n_attn) core_attention<DK, DV>(c, idx - c.n_mix, sm);
+    else if (c.vs == 64) core_recurrence<64>(c, idx - c.n_mix - c.n_attn, sm);
+    else core_recurrence<32>(c, idx - c.n_mix - c.n_attn, sm);
 }
 
 // ------------------------------------------------------------------------------------------------ merge
@@ -965,12 +979,6 @@ extern "C" int natsl_decode_step(const natsl_decode_args* args, void* stream) {
     c.n_rec = a.B * a.H * (a.V / c.vs);
     c.n_slices = l.slices;
     c.n_mix = a.w_mix ? a.B * l.slices * ((2 * a.HQ + DS_MIX_ROWS - 1) / DS_MIX_ROWS) : 0;
-    // A recurrence CTA takes as long as an attention CTA of some eight 64-key units, half of them selected: below that it goes first
-    // (4 rows of 32 heads, 1030 tokens, 3 units a split, 1024 CTAs over 592 places: a token takes 37.9 us the other way and 34.6 us
-    // this way; 32 rows of 16 heads, 2048 tokens, 16 units: 48.1 us and 53.1 us).
-    const bool rec_first = a.n_done * (a.nbs / 64) <= 8 * l.S;
-    c.rec0 = c.n_mix + (rec_first ? 0 : c.n_attn);
-    c.attn0 = c.n_mix + (rec_first ? c.n_rec : 0);
     if (e == cudaSuccess)
         e = DK == 64 ? (DV == 64 ? launch_core<64, 64>(c, st) : launch_core<64, 128>(c, st))
                      : (DV == 64 ? launch_core<128, 64>(c, st) : launch_core<128, 128>(c, st));
