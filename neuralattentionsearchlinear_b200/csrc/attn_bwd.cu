@@ -19,6 +19,8 @@
 // come from the full forward.
 // Every mbarrier wait has an iteration limit; on expiry the CTA records a status, stops issuing work, still frees its
 // TMEM and returns.
+#include <type_traits>
+
 #include "attn_tc.cuh"
 #include "../../include/natsl_b200.h"
 
@@ -322,25 +324,29 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
 // with p and ds in shared memory, p and ds need no shared memory at all, and a query tile is loaded once for two key tiles.
 // Results of a tile that the queries at hand do not see are kept out by the products' lane mask, whatever the queries hold.
 // One persistent CTA per SM takes blocks of the grid over (cluster launch control); a planning warp works out their steps, and
-// lse and delta of the queries, while the others are at the steps before.  Roles: warp 0 loads, warp 1 issues the products, warps 2-9
-// p and ds (a key and 64 queries per thread), warp 10 plans.
-// What bounds it: the chain scores -> p -> dv product and do.v -> ds -> dk product of a step, 3.5 k cycles against 2 k of the tensor
+// lse and delta of the queries, while the others are at the steps before.  Roles: warp 0 loads, warp 1 issues the products, warp 2
+// plans, warps 4-11 p and ds (a key and 64 queries per thread).
+// Registers: 384 threads get 168 each, of which the first four warps give back what the others need for p, ds and do.v of 64 queries.
+// Nothing may spill: the shared memory leaves so little of the first-level cache that a spilled word comes back from L2, some 400
+// cycles in a chain in which nothing else hides them (168 for all, 56 bytes of spills: 389 us where the figures below have 355).
+// What bounds it: the chain scores -> p -> dv product and do.v -> ds -> dk product of a step, 3 k cycles against 2 k of the tensor
 // core (tensor memory holds one step: 128 columns each of scores, do.v, dk and dv), and 64 KB of q and do from L2 a step.
 // Alone (us; before: 128 x 64 score tiles, p and ds through shared memory, one CTA per pair of tiles), block 64:
-//   128/128, B = 8, T = 4096, H = 16: 25 % selected 678 -> 389, 50 % 1069 -> 607, 2 % 338 -> 194;  64/64, 30 %: 630 -> 369
-//   128/64, B = 4, T = 1000, H = 16, 50 %: 72 -> 44;  128/128, B = 1, T = 2048, H = 16, 30 %: 65 -> 43
-//   64/128, B = 2, T = 2048, 12 heads over 6, block 128, 40 %: 113 -> 67;  the smallest, B = 2, T = 64, H = 4: 8.5 -> 9.6
-constexpr int BKV_THREADS = 352;                              // TMA, MMA, 8 softmax warps, planner
+//   128/128, B = 8, T = 4096, H = 16: 25 % selected 678 -> 355, 50 % 1069 -> 545, 2 % 338 -> 182;  64/64, 30 %: 630 -> 336
+//   128/64, B = 4, T = 1000, H = 16, 50 %: 72 -> 41;  128/128, B = 1, T = 2048, H = 16, 30 %: 65 -> 36
+//   64/128, B = 2, T = 2048, 12 heads over 6, block 128, 40 %: 113 -> 56;  the smallest, B = 2, T = 64, H = 4: 8.5 -> 8.7
+constexpr int BKV_THREADS = 384;                              // TMA, MMA, planner, (no work), 8 softmax warps
 constexpr int BKV_MAXG = 16;
-constexpr int BKV_DESCS = 4;
+constexpr int BKV_DESCS = 2;                                  // steps that the planner is ahead
+constexpr int BKV_REGS_LOW = 88, BKV_REGS_HIGH = 208;         // a thread: 128 x 88 + 256 x 208 = 384 x 168
 template <int DK, int DV>
 struct DkvSmem {
     static constexpr int kv = 0;                              // k: DK/64 sub-tiles [128 keys][64], then v the same way
     static constexpr int q = kv + 128 * (DK + DV) * 2;        // 2 stages x DK/64 sub-tiles [128 queries][64]
     static constexpr int dos = q + 2 * 128 * DK * 2;          // 2 stages x DV/64 sub-tiles
     static constexpr int out = dos + 2 * 128 * DV * 2;        // per softmax warp: 32 rows x 64 columns on their way out
-    static constexpr int stat = out + 8 * 4096;               // 2 x (-lse, -delta) of 128 queries
-    static constexpr int dn = stat + 2 * 1024;                // dnats parts [2 tiles][16 heads][4 warps]
+    static constexpr int stat = out + 8 * 4096;               // per step (-lse, -delta) of 128 queries
+    static constexpr int dn = stat + BKV_DESCS * 1024;        // dnats parts [2 tiles][16 heads][4 warps]
     static constexpr int desc = dn + 2 * BKV_MAXG * 4 * 4;    // steps, 32 bytes each
     static constexpr int last = desc + BKV_DESCS * 32;        // last query tile [2 tiles][16 heads] of a selected pair
     static constexpr int clc = last + 2 * BKV_MAXG * 2;       // answer of the take-over request
@@ -407,10 +413,10 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     int4* s_desc = reinterpret_cast<int4*>(smem + L::desc);
     volatile int16_t* s_last = reinterpret_cast<volatile int16_t*>(smem + L::last);
     const uint32_t bar0 = sbase + L::bars;
-    // barriers: desc_full / desc_empty (steps); st_full / st_empty (lse and delta); q_full / q_empty, do_full / do_empty (stages);
+    // barriers: desc_full / desc_empty (steps, with lse and delta); q_full / q_empty, do_full / do_empty (stages);
     // kv_full / kv_empty; s, dp (scores, do.v complete); p, ds (written by the softmax warps); acc (dk, dv of the pair complete);
-    // acc_free (read and set to zero)
-    const uint32_t desc_full = bar0, desc_empty = bar0 + 32, st_full = bar0 + 64, st_empty = bar0 + 80, q_full = bar0 + 96,
+    // dv (of the pair complete: its rows leave during dk's last product); acc_free (read and set to zero)
+    const uint32_t desc_full = bar0, desc_empty = bar0 + 32, bar_dv = bar0 + 64, q_full = bar0 + 96,
                    q_empty = bar0 + 112, do_full = bar0 + 128, do_empty = bar0 + 144, kv_full = bar0 + 160, kv_empty = bar0 + 168,
                    bar_s = bar0 + 176, bar_dp = bar0 + 184, bar_p = bar0 + 192, bar_ds = bar0 + 200, bar_acc = bar0 + 208,
                    bar_acc_free = bar0 + 216, bar_clc = bar0 + 224;
@@ -426,8 +432,6 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             mbar_init(desc_empty + 8 * i, 10);                // eight softmax warps, TMA, MMA
         }
         for (int i = 0; i < 2; ++i) {
-            mbar_init(st_full + 8 * i, 1);
-            mbar_init(st_empty + 8 * i, 8);
             mbar_init(q_full + 8 * i, 1);
             mbar_init(q_empty + 8 * i, 1);
             mbar_init(do_full + 8 * i, 1);
@@ -442,6 +446,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         mbar_init(bar_acc, 1);
         mbar_init(bar_acc_free, 8);
         mbar_init(bar_clc, 1);
+        mbar_init(bar_dv, 1);
         mbar_fence_init();
     }
     for (int i = tid; i < 2 * BKV_MAXG * 4; i += BKV_THREADS) s_dn[i] = 0.f;
@@ -459,330 +464,338 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         d = s_desc[2 * slot];
         loc = s_desc[2 * slot + 1];
         d.y = ok ? __shfl_sync(0xffffffffu, d.y, 0) : BKV_STOP;
-        arrive(desc_empty + slot * 8);
-        ++n_step;
         return d.y;
     };
+    auto release_step = [&]() { arrive(desc_empty + (n_step++ & (BKV_DESCS - 1)) * 8); };
 
-    if (warp == 0) {
-        // ------------------------------------------------------------ TMA producer
-        int ni = 0, pairs = 0;                                // steps with queries, pairs that have some
+    if (warp < 4) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(BKV_REGS_LOW));
+        if (warp == 0) {
+            // ------------------------------------------------------------ TMA producer
+            int ni = 0, pairs = 0;                                // steps with queries, pairs that have some
 #pragma unroll 1
-        while (ok) {
-            next_step();
-            if (d.y & BKV_STOP) break;
-            if (d.y & BKV_EMPTY) continue;
-            const int hkv = loc.z, b = loc.w;
-            if (d.y & BKV_FIRST) {
-                if (pairs > 0) ok = warp_wait(kv_empty, (pairs - 1) & 1);
-                if (!ok) break;
-                if (lane == 0) {
-                    const int t[2] = {loc.x, loc.y};
-                    mbar_expect_tx(kv_full, ((t[0] >= 0) + (t[1] >= 0)) * 64 * (DK + DV) * 2);
+            while (ok) {
+                next_step();
+                release_step();
+                if (d.y & BKV_STOP) break;
+                if (d.y & BKV_EMPTY) continue;
+                const int hkv = loc.z, b = loc.w;
+                if (d.y & BKV_FIRST) {
+                    if (pairs > 0) ok = warp_wait(kv_empty, (pairs - 1) & 1);
+                    if (!ok) break;
+                    if (lane == 0) {
+                        const int t[2] = {loc.x, loc.y};
+                        mbar_expect_tx(kv_full, ((t[0] >= 0) + (t[1] >= 0)) * 64 * (DK + DV) * 2);
 #pragma unroll
-                    for (int u = 0; u < 2; ++u) {
-                        if (t[u] < 0) continue;
+                        for (int u = 0; u < 2; ++u) {
+                            if (t[u] < 0) continue;
 #pragma unroll
-                        for (int sub = 0; sub < DK / 64; ++sub)
-                            tma_load_4d(sbase + L::kv + sub * 16384 + u * 8192, &map_k, sub * 64, hkv, t[u] * 64, b, kv_full);
+                            for (int sub = 0; sub < DK / 64; ++sub)
+                                tma_load_4d(sbase + L::kv + sub * 16384 + u * 8192, &map_k, sub * 64, hkv, t[u] * 64, b, kv_full);
 #pragma unroll
-                        for (int sub = 0; sub < DV / 64; ++sub)
-                            tma_load_4d(sbase + L::kv + 128 * DK * 2 + sub * 16384 + u * 8192, &map_v, sub * 64, hkv, t[u] * 64, b, kv_full);
-                    }
-                }
-                __syncwarp();
-                ++pairs;
-            }
-            const int st = ni & 1, par = ((ni >> 1) - 1) & 1, hq = hkv * G + d.z;
-            if (lane == 0 && ni >= 2) {                       // into L2 while the stages are still read
-#pragma unroll
-                for (int sub = 0; sub < DK / 64; ++sub) tma_prefetch_4d(&map_q, sub * 64, hq, d.x, b);
-#pragma unroll
-                for (int sub = 0; sub < DV / 64; ++sub) tma_prefetch_4d(&map_do, sub * 64, hq, d.x, b);
-            }
-            __syncwarp();
-            if (ni >= 2) ok = warp_wait(q_empty + st * 8, par);
-            if (!ok) break;
-            if (lane == 0) {
-                mbar_expect_tx(q_full + st * 8, 128 * DK * 2);
-#pragma unroll
-                for (int sub = 0; sub < DK / 64; ++sub)
-                    tma_load_4d(sbase + L::q + st * (128 * DK * 2) + sub * 16384, &map_q, sub * 64, hq, d.x, b, q_full + st * 8);
-            }
-            __syncwarp();
-            if (ni >= 2) ok = warp_wait(do_empty + st * 8, par);
-            if (!ok) {
-                warp_wait(q_full + st * 8, (ni >> 1) & 1);    // nothing may still be on its way into shared memory
-                break;
-            }
-            if (lane == 0) {
-                mbar_expect_tx(do_full + st * 8, 128 * DV * 2);
-#pragma unroll
-                for (int sub = 0; sub < DV / 64; ++sub)
-                    tma_load_4d(sbase + L::dos + st * (128 * DV * 2) + sub * 16384, &map_do, sub * 64, hq, d.x, b, do_full + st * 8);
-            }
-            __syncwarp();
-            ++ni;
-        }
-        if (!ok) {
-            if (pairs > 0) warp_wait(kv_full, (pairs - 1) & 1);
-            for (int i = max(0, ni - 2); i < ni; ++i) {
-                warp_wait(q_full + (i & 1) * 8, (i >> 1) & 1);
-                warp_wait(do_full + (i & 1) * 8, (i >> 1) & 1);
-            }
-        }
-    } else if (warp == 1) {
-        // ------------------------------------------------------------ MMA issuer
-        constexpr uint32_t id_s = umma_idesc_bf16(128, 128, false);
-        constexpr uint32_t id_dv = umma_idesc_bf16(128, DV, true), id_dk = umma_idesc_bf16(128, DK, true);
-        const uint32_t kl = umma_desc_lo(sbase + L::kv, 16), vl = umma_desc_lo(sbase + L::kv + 128 * DK * 2, 16);
-        auto scores = [&](int st) {                           // K Q^T
-            tc_fence_after();
-            const uint32_t ql = umma_desc_lo(sbase + L::q + st * (128 * DK * 2), 16);
-#pragma unroll
-            for (int h = 0; h < DK / 64; ++h) umma_ss_x4<2, 2>(tmem + C_S, kl + h * 1024, ql + h * 1024, id_s, h > 0);
-            umma_commit(bar_s);
-        };
-        auto products = [&](int st, bool last) {              // V dO^T
-            tc_fence_after();
-            const uint32_t dl = umma_desc_lo(sbase + L::dos + st * (128 * DV * 2), 16);
-#pragma unroll
-            for (int h = 0; h < DV / 64; ++h) umma_ss_x4<2, 2>(tmem + C_DP, vl + h * 1024, dl + h * 1024, id_s, h > 0);
-            umma_commit(bar_dp);
-            if (last) umma_commit(kv_empty);
-        };
-        int ni = 0, pairs = 0;
-        int f = next_step();
-#pragma unroll 1
-        while (ok && !(f & BKV_STOP)) {
-            if (f & BKV_EMPTY) {
-                f = next_step();
-                continue;
-            }
-            if (f & BKV_FIRST) {
-                ok = warp_wait(kv_full, pairs & 1);
-                if (ok) ok = warp_wait(q_full + (ni & 1) * 8, (ni >> 1) & 1);
-                if (!ok) break;
-                scores(ni & 1);
-                ok = warp_wait(do_full + (ni & 1) * 8, (ni >> 1) & 1);
-                if (!ok) break;
-                products(ni & 1, (f & BKV_LAST) != 0);
-                ok = warp_wait(bar_acc_free, pairs & 1);
-                ++pairs;
-            }
-            const int st = ni & 1, nst = st ^ 1, npar = ((ni + 1) >> 1) & 1;
-            const uint32_t m01 = f & BKV_ACT0 ? 0u : 0xffffffffu, m23 = f & BKV_ACT1 ? 0u : 0xffffffffu;
-            const bool last = (f & BKV_LAST) != 0;
-            if (ok) ok = warp_wait(bar_p, ni & 1);
-            if (!ok) break;
-            tc_fence_after();
-            {                                                 // dv += p dO
-                const uint32_t dl = umma_desc_lo(sbase + L::dos + st * (128 * DV * 2), 16384);
-#pragma unroll
-                for (int h = 0; h < 2; ++h) umma_ts_x4_lanes<128>(tmem + C_DV, tmem + C_S + h * 64, dl + h * 512, id_dv, m01, m23);
-                umma_commit(do_empty + st * 8);
-            }
-            int fn = BKV_STOP;
-            if (!last) {                                      // the next scores as soon as p has been used
-                fn = next_step();
-                if (ok) ok = warp_wait(q_full + nst * 8, npar);
-                if (!ok) break;
-                scores(nst);
-            }
-            ok = warp_wait(bar_ds, ni & 1);
-            if (!ok) break;
-            tc_fence_after();
-            {                                                 // dk += ds Q
-                const uint32_t ql = umma_desc_lo(sbase + L::q + st * (128 * DK * 2), 16384);
-#pragma unroll
-                for (int h = 0; h < 2; ++h) umma_ts_x4_lanes<128>(tmem + C_DK, tmem + C_DP + h * 64, ql + h * 512, id_dk, m01, m23);
-                umma_commit(q_empty + st * 8);
-            }
-            if (last) {
-                umma_commit(bar_acc);
-                f = next_step();
-            } else {
-                ok = warp_wait(do_full + nst * 8, npar);
-                if (!ok) break;
-                products(nst, (fn & BKV_LAST) != 0);
-                f = fn;
-            }
-            ++ni;
-        }
-    } else if (warp == 10) {
-        // ------------------------------------------------------------ planner: blocks, their steps, lse and delta of the queries
-        int n = 0, ni = 0, asked = 0, answers = 0;            // steps, steps with queries, take-over requests
-        int block = blockIdx.x;
-        auto put = [&](int4 x, int4 y) {
-            const int slot = n & (BKV_DESCS - 1);
-            if (n >= BKV_DESCS) ok = warp_wait(desc_empty + slot * 8, (n / BKV_DESCS - 1) & 1);
-            if (!ok) return;
-            if (lane == 0) {
-                s_desc[2 * slot] = x;
-                s_desc[2 * slot + 1] = y;
-            }
-            arrive(desc_full + slot * 8);
-            ++n;
-        };
-        auto request = [&]() {
-            if (lane == 0) {
-                fence_async_smem();
-                mbar_expect_tx(bar_clc, 16);
-                request_block(sbase + L::clc, bar_clc);
-            }
-            __syncwarp();
-            ++asked;
-        };
-#pragma unroll 1
-        while (ok) {
-            // Block `item` of a head: the item-th pair of the tiles whose block some head of the group selected, in their order
-            // (neighbours see nearly the same queries), then what is unselected of tiles 2 item and 2 item + 1, which only
-            // their own blocks' queries see.
-            const int hbase = block / (BKV_HEADS * ctas_per_head) * BKV_HEADS, hcount = min(BKV_HEADS, heads - hbase);
-            const int within = block - hbase * ctas_per_head;
-            const int item = within / hcount, head = hbase + within % hcount;
-            const int hkv = head % HKV, b = head / HKV;
-            auto selected = [&](int kt) -> bool {
-                bool s = false;
-#pragma unroll 1
-                for (int gi = 0; gi < G; ++gi) s |= types_i[(((long)b * TN + kt / cpb) * HN + (hkv * G + gi) / (HQ / HN)) * 2] != 0;
-                return s;
-            };
-            int chosen[2] = {-1, -1}, rest[2] = {-1, -1};
-            unsigned mine = 0;                                // bit i: tile 2 item + i is selected
-            int cnt = 0;
-#pragma unroll 1
-            for (int base = 0; base < NT; base += 32) {
-                const unsigned m = __ballot_sync(0xffffffffu, base + lane < NT && selected(base + lane));
-                const int k = __popc(m);
-                if (2 * item >= base && 2 * item < base + 32) mine = m >> (2 * item - base);
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    const int r = 2 * item + i - cnt;
-                    if (r >= 0 && r < k) chosen[i] = base + __fns(m, 0, r + 1);
-                }
-                cnt += k;
-                if (cnt >= 2 * item + 2 && base + 32 > 2 * item + 1) break;
-            }
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-                if (!((mine >> i) & 1) && 2 * item + i < NT) rest[i] = 2 * item + i;
-            bool requested = chosen[0] < 0;                   // a step or none: ask for the next block at once
-            if (requested) {
-                request();
-            } else {
-                // last query tile of every (tile, head): the sequence's if the head selected the block, else the own block's
-                __syncwarp();
-#pragma unroll 1
-                for (int i = lane; i < 2 * BKV_MAXG; i += 32) {
-                    const int kt = i / BKV_MAXG ? chosen[1] : chosen[0], gi = i % BKV_MAXG;
-                    int last = -1;
-                    if (kt >= 0 && gi < G) {
-                        const int blk = kt / cpb, blk_end = (blk + 1) * nbs;
-                        const bool s = G == 1 || types_i[(((long)b * TN + blk) * HN + (hkv * G + gi) / (HQ / HN)) * 2] != 0;
-                        if (s && blk_end < T) last = NTq - 1;
-                        else if (own) last = min((blk_end - 1) / ATT_BM, NTq - 1);
-                    }
-                    s_last[i] = (int16_t)last;
-                }
-                __syncwarp();
-            }
-#pragma unroll 1
-            for (int pass = chosen[0] < 0; ok && pass < 2; ++pass) {
-                const bool sums = pass == 0;
-                const int t[2] = {sums ? chosen[0] : rest[0], sums ? chosen[1] : rest[1]};
-                if (t[0] < 0 && t[1] < 0) continue;
-                const int4 where = make_int4(t[0], t[1], hkv, b);
-                int first[2], end[2], own_last[2];            // tile u: query tiles [first, last(head)]
-                bool any[2] = {false, false};
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    end[u] = (t[u] / cpb + 1) * nbs;
-                    first[u] = t[u] < 0 ? NTq : own ? t[u] * 64 / ATT_BM : end[u] / ATT_BM;
-                    own_last[u] = t[u] >= 0 && own ? min((end[u] - 1) / ATT_BM, NTq - 1) : -1;
-                }
-                auto last_of = [&](int u, int gi) -> int { return sums ? (int)s_last[u * BKV_MAXG + gi] : own_last[u]; };
-                for (int gi = 0; gi < G; ++gi) {
-                    any[0] |= last_of(0, gi) >= first[0];
-                    any[1] |= last_of(1, gi) >= first[1];
-                }
-                const int base = (sums ? BKV_SUMS : 0) | (any[0] ? BKV_ANY0 : 0) | (any[1] ? BKV_ANY1 : 0);
-                if (!any[0] && !any[1]) {
-                    put(make_int4(0, base | BKV_EMPTY, 0, 0), where);
-                    continue;
-                }
-                int held = -1, h_qt = 0, h_gi = 0, h_prev = 0;    // the step that is announced once it is known whether another follows
-                float nl[4], nd[4];
-                auto announce = [&](int more) {
-                    const int st = ni & 1;
-                    if (ni >= 2) ok = warp_wait(st_empty + st * 8, ((ni >> 1) - 1) & 1);
-                    if (!ok) return;
-                    float* x = reinterpret_cast<float*>(smem + L::stat + st * 1024);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        x[lane + 32 * i] = nl[i];
-                        x[128 + lane + 32 * i] = nd[i];
-                    }
-                    arrive(st_full + st * 8);
-                    ++ni;
-                    put(make_int4(h_qt * ATT_BM, held | more, h_gi, h_prev), where);
-                };
-                int prev = -1;
-#pragma unroll 1
-                for (int gi = 0; ok && gi < G; ++gi) {
-                    const int l0 = last_of(0, gi), l1 = last_of(1, gi), hi = max(l0, l1);
-                    int sel = sums ? BKV_SEL0 | BKV_SEL1 : 0;
-                    if (sums && G > 1) {
-                        sel = 0;
-#pragma unroll
-                        for (int u = 0; u < 2; ++u)
-                            if (t[u] >= 0 && types_i[(((long)b * TN + t[u] / cpb) * HN + (hkv * G + gi) / (HQ / HN)) * 2] != 0)
-                                sel |= u ? BKV_SEL1 : BKV_SEL0;
-                    }
-#pragma unroll 1
-                    for (int qt = min(l0 >= first[0] ? first[0] : NTq, l1 >= first[1] ? first[1] : NTq); ok && qt <= hi; ++qt) {
-                        const int act = (qt >= first[0] && qt <= l0 ? BKV_ACT0 : 0) | (qt >= first[1] && qt <= l1 ? BKV_ACT1 : 0);
-                        if (!act) continue;
-                        if (held >= 0) announce(0);
-                        held = base | act | sel | (prev < 0 ? BKV_FIRST : 0) | (prev >= 0 && prev != gi ? BKV_FLUSH : 0);
-                        h_qt = qt;
-                        h_gi = gi;
-                        h_prev = prev;
-                        prev = gi;
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {         // a query behind the end has probability 0
-                            const int q = qt * ATT_BM + lane + 32 * i;
-                            const long r = ((long)b * T + q) * HQ + hkv * G + gi;
-                            nl[i] = q < T ? -lse[r] : -INFINITY;
-                            nd[i] = q < T ? -delta[r] : 0.f;
+                            for (int sub = 0; sub < DV / 64; ++sub)
+                                tma_load_4d(sbase + L::kv + 128 * DK * 2 + sub * 16384 + u * 8192, &map_v, sub * 64, hkv, t[u] * 64, b, kv_full);
                         }
                     }
+                    __syncwarp();
+                    ++pairs;
                 }
-                if (ok) announce(BKV_LAST);
-                // the pair's last steps are under way: early enough to work out the next block, late enough to leave it to an SM
-                // that is free earlier
-                if (ok && sums) {
+                const int st = ni & 1, par = ((ni >> 1) - 1) & 1, hq = hkv * G + d.z;
+                if (lane == 0 && ni >= 2) {                       // into L2 while the stages are still read
+#pragma unroll
+                    for (int sub = 0; sub < DK / 64; ++sub) tma_prefetch_4d(&map_q, sub * 64, hq, d.x, b);
+#pragma unroll
+                    for (int sub = 0; sub < DV / 64; ++sub) tma_prefetch_4d(&map_do, sub * 64, hq, d.x, b);
+                }
+                __syncwarp();
+                if (ni >= 2) ok = warp_wait(q_empty + st * 8, par);
+                if (!ok) break;
+                if (lane == 0) {
+                    mbar_expect_tx(q_full + st * 8, 128 * DK * 2);
+#pragma unroll
+                    for (int sub = 0; sub < DK / 64; ++sub)
+                        tma_load_4d(sbase + L::q + st * (128 * DK * 2) + sub * 16384, &map_q, sub * 64, hq, d.x, b, q_full + st * 8);
+                }
+                __syncwarp();
+                if (ni >= 2) ok = warp_wait(do_empty + st * 8, par);
+                if (!ok) {
+                    warp_wait(q_full + st * 8, (ni >> 1) & 1);    // nothing may still be on its way into shared memory
+                    break;
+                }
+                if (lane == 0) {
+                    mbar_expect_tx(do_full + st * 8, 128 * DV * 2);
+#pragma unroll
+                    for (int sub = 0; sub < DV / 64; ++sub)
+                        tma_load_4d(sbase + L::dos + st * (128 * DV * 2) + sub * 16384, &map_do, sub * 64, hq, d.x, b, do_full + st * 8);
+                }
+                __syncwarp();
+                ++ni;
+            }
+            if (!ok) {
+                if (pairs > 0) warp_wait(kv_full, (pairs - 1) & 1);
+                for (int i = max(0, ni - 2); i < ni; ++i) {
+                    warp_wait(q_full + (i & 1) * 8, (i >> 1) & 1);
+                    warp_wait(do_full + (i & 1) * 8, (i >> 1) & 1);
+                }
+            }
+        } else if (warp == 1) {
+            // ------------------------------------------------------------ MMA issuer
+            constexpr uint32_t id_s = umma_idesc_bf16(128, 128, false);
+            constexpr uint32_t id_dv = umma_idesc_bf16(128, DV, true), id_dk = umma_idesc_bf16(128, DK, true);
+            const uint32_t kl = umma_desc_lo(sbase + L::kv, 16), vl = umma_desc_lo(sbase + L::kv + 128 * DK * 2, 16);
+            auto scores = [&](int st) {                           // K Q^T
+                tc_fence_after();
+                const uint32_t ql = umma_desc_lo(sbase + L::q + st * (128 * DK * 2), 16);
+#pragma unroll
+                for (int h = 0; h < DK / 64; ++h) umma_ss_x4<2, 2>(tmem + C_S, kl + h * 1024, ql + h * 1024, id_s, h > 0);
+                umma_commit(bar_s);
+            };
+            auto products = [&](int st, bool last) {              // V dO^T
+                tc_fence_after();
+                const uint32_t dl = umma_desc_lo(sbase + L::dos + st * (128 * DV * 2), 16);
+#pragma unroll
+                for (int h = 0; h < DV / 64; ++h) umma_ss_x4<2, 2>(tmem + C_DP, vl + h * 1024, dl + h * 1024, id_s, h > 0);
+                umma_commit(bar_dp);
+                if (last) umma_commit(kv_empty);
+            };
+            int ni = 0, pairs = 0;
+            int f = next_step();
+            release_step();
+#pragma unroll 1
+            while (ok && !(f & BKV_STOP)) {
+                if (f & BKV_EMPTY) {
+                    f = next_step();
+                    release_step();
+                    continue;
+                }
+                if (f & BKV_FIRST) {
+                    ok = warp_wait(kv_full, pairs & 1);
+                    if (ok) ok = warp_wait(q_full + (ni & 1) * 8, (ni >> 1) & 1);
+                    if (!ok) break;
+                    scores(ni & 1);
+                    ok = warp_wait(do_full + (ni & 1) * 8, (ni >> 1) & 1);
+                    if (!ok) break;
+                    products(ni & 1, (f & BKV_LAST) != 0);
+                    ok = warp_wait(bar_acc_free, pairs & 1);
+                    ++pairs;
+                }
+                const int st = ni & 1, nst = st ^ 1, npar = ((ni + 1) >> 1) & 1;
+                const uint32_t m01 = f & BKV_ACT0 ? 0u : 0xffffffffu, m23 = f & BKV_ACT1 ? 0u : 0xffffffffu;
+                const bool last = (f & BKV_LAST) != 0;
+                if (ok) ok = warp_wait(bar_p, ni & 1);
+                if (!ok) break;
+                tc_fence_after();
+                {                                                 // dv += p dO
+                    const uint32_t dl = umma_desc_lo(sbase + L::dos + st * (128 * DV * 2), 16384);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) umma_ts_x4_lanes<128>(tmem + C_DV, tmem + C_S + h * 64, dl + h * 512, id_dv, m01, m23);
+                    umma_commit(do_empty + st * 8);
+                    if (last) umma_commit(bar_dv);
+                }
+                int fn = BKV_STOP;
+                if (!last) {                                      // the next scores as soon as p has been used
+                    fn = next_step();
+                    release_step();
+                    if (ok) ok = warp_wait(q_full + nst * 8, npar);
+                    if (!ok) break;
+                    scores(nst);
+                }
+                ok = warp_wait(bar_ds, ni & 1);
+                if (!ok) break;
+                tc_fence_after();
+                {                                                 // dk += ds Q
+                    const uint32_t ql = umma_desc_lo(sbase + L::q + st * (128 * DK * 2), 16384);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) umma_ts_x4_lanes<128>(tmem + C_DK, tmem + C_DP + h * 64, ql + h * 512, id_dk, m01, m23);
+                    umma_commit(q_empty + st * 8);
+                }
+                if (last) {
+                    umma_commit(bar_acc);
+                    f = next_step();
+                    release_step();
+                } else {
+                    ok = warp_wait(do_full + nst * 8, npar);
+                    if (!ok) break;
+                    products(nst, (fn & BKV_LAST) != 0);
+                    f = fn;
+                }
+                ++ni;
+            }
+        } else if (warp == 2) {
+            // ------------------------------------------------------------ planner: blocks, their steps, lse and delta of the queries
+            int n = 0, asked = 0, answers = 0;                    // steps, take-over requests
+            int block = blockIdx.x;
+            auto open = [&]() {
+                if (n >= BKV_DESCS) ok = warp_wait(desc_empty + (n & (BKV_DESCS - 1)) * 8, (n / BKV_DESCS - 1) & 1);
+                return ok;
+            };
+            auto put = [&](int4 x, int4 y) {
+                const int slot = n & (BKV_DESCS - 1);
+                if (lane == 0) {
+                    s_desc[2 * slot] = x;
+                    s_desc[2 * slot + 1] = y;
+                }
+                arrive(desc_full + slot * 8);
+                ++n;
+            };
+            auto request = [&]() {
+                if (lane == 0) {
+                    fence_async_smem();
+                    mbar_expect_tx(bar_clc, 16);
+                    request_block(sbase + L::clc, bar_clc);
+                }
+                __syncwarp();
+                ++asked;
+            };
+#pragma unroll 1
+            while (ok) {
+                // Block `item` of a head: the item-th pair of the tiles whose block some head of the group selected, in their order
+                // (neighbours see nearly the same queries), then what is unselected of tiles 2 item and 2 item + 1, which only
+                // their own blocks' queries see.
+                const int hbase = block / (BKV_HEADS * ctas_per_head) * BKV_HEADS, hcount = min(BKV_HEADS, heads - hbase);
+                const int within = block - hbase * ctas_per_head;
+                const int item = within / hcount, head = hbase + within % hcount;
+                const int hkv = head % HKV, b = head / HKV;
+                auto selected = [&](int kt) -> bool {
+                    bool s = false;
+#pragma unroll 1
+                    for (int gi = 0; gi < G; ++gi) s |= types_i[(((long)b * TN + kt / cpb) * HN + (hkv * G + gi) / (HQ / HN)) * 2] != 0;
+                    return s;
+                };
+                int chosen[2] = {-1, -1}, rest[2] = {-1, -1};
+                unsigned mine = 0;                                // bit i: tile 2 item + i is selected
+                int cnt = 0;
+#pragma unroll 1
+                for (int base = 0; base < NT; base += 32) {
+                    const unsigned m = __ballot_sync(0xffffffffu, base + lane < NT && selected(base + lane));
+                    const int k = __popc(m);
+                    if (2 * item >= base && 2 * item < base + 32) mine = m >> (2 * item - base);
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        const int r = 2 * item + i - cnt;
+                        if (r >= 0 && r < k) chosen[i] = base + __fns(m, 0, r + 1);
+                    }
+                    cnt += k;
+                    if (cnt >= 2 * item + 2 && base + 32 > 2 * item + 1) break;
+                }
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+                    if (!((mine >> i) & 1) && 2 * item + i < NT) rest[i] = 2 * item + i;
+                bool requested = chosen[0] < 0;                   // a step or none: ask for the next block at once
+                if (requested) {
                     request();
-                    requested = true;
+                } else {
+                    // last query tile of every (tile, head): the sequence's if the head selected the block, else the own block's
+                    __syncwarp();
+#pragma unroll 1
+                    for (int i = lane; i < 2 * BKV_MAXG; i += 32) {
+                        const int kt = i / BKV_MAXG ? chosen[1] : chosen[0], gi = i % BKV_MAXG;
+                        int last = -1;
+                        if (kt >= 0 && gi < G) {
+                            const int blk = kt / cpb, blk_end = (blk + 1) * nbs;
+                            const bool s = G == 1 || types_i[(((long)b * TN + blk) * HN + (hkv * G + gi) / (HQ / HN)) * 2] != 0;
+                            if (s && blk_end < T) last = NTq - 1;
+                            else if (own) last = min((blk_end - 1) / ATT_BM, NTq - 1);
+                        }
+                        s_last[i] = (int16_t)last;
+                    }
+                    __syncwarp();
                 }
+#pragma unroll 1
+                for (int pass = chosen[0] < 0; ok && pass < 2; ++pass) {
+                    const bool sums = pass == 0;
+                    const int t[2] = {sums ? chosen[0] : rest[0], sums ? chosen[1] : rest[1]};
+                    if (t[0] < 0 && t[1] < 0) continue;
+                    const int4 where = make_int4(t[0], t[1], hkv, b);
+                    int first[2], end[2], own_last[2];            // tile u: query tiles [first, last(head)]
+                    bool any[2] = {false, false};
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        end[u] = (t[u] / cpb + 1) * nbs;
+                        first[u] = t[u] < 0 ? NTq : own ? t[u] * 64 / ATT_BM : end[u] / ATT_BM;
+                        own_last[u] = t[u] >= 0 && own ? min((end[u] - 1) / ATT_BM, NTq - 1) : -1;
+                    }
+                    auto last_of = [&](int u, int gi) -> int { return sums ? (int)s_last[u * BKV_MAXG + gi] : own_last[u]; };
+                    for (int gi = 0; gi < G; ++gi) {
+                        any[0] |= last_of(0, gi) >= first[0];
+                        any[1] |= last_of(1, gi) >= first[1];
+                    }
+                    const int base = (sums ? BKV_SUMS : 0) | (any[0] ? BKV_ANY0 : 0) | (any[1] ? BKV_ANY1 : 0);
+                    if (!any[0] && !any[1]) {
+                        if (open()) put(make_int4(0, base | BKV_EMPTY, 0, 0), where);
+                        continue;
+                    }
+                    int held = -1, h_qt = 0, h_gi = 0, h_prev = 0;    // the step that is announced once it is known whether another follows
+                    float nl[4], nd[4];
+                    auto announce = [&](int more) {
+                        if (!open()) return;
+                        float* x = reinterpret_cast<float*>(smem + L::stat + (n & (BKV_DESCS - 1)) * 1024);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            x[lane + 32 * i] = nl[i];
+                            x[128 + lane + 32 * i] = nd[i];
+                        }
+                        put(make_int4(h_qt * ATT_BM, held | more, h_gi, h_prev), where);
+                    };
+                    int prev = -1;
+#pragma unroll 1
+                    for (int gi = 0; ok && gi < G; ++gi) {
+                        const int l0 = last_of(0, gi), l1 = last_of(1, gi), hi = max(l0, l1);
+                        int sel = sums ? BKV_SEL0 | BKV_SEL1 : 0;
+                        if (sums && G > 1) {
+                            sel = 0;
+#pragma unroll
+                            for (int u = 0; u < 2; ++u)
+                                if (t[u] >= 0 && types_i[(((long)b * TN + t[u] / cpb) * HN + (hkv * G + gi) / (HQ / HN)) * 2] != 0)
+                                    sel |= u ? BKV_SEL1 : BKV_SEL0;
+                        }
+#pragma unroll 1
+                        for (int qt = min(l0 >= first[0] ? first[0] : NTq, l1 >= first[1] ? first[1] : NTq); ok && qt <= hi; ++qt) {
+                            const int act = (qt >= first[0] && qt <= l0 ? BKV_ACT0 : 0) | (qt >= first[1] && qt <= l1 ? BKV_ACT1 : 0);
+                            if (!act) continue;
+                            if (held >= 0) announce(0);
+                            held = base | act | sel | (prev < 0 ? BKV_FIRST : 0) | (prev >= 0 && prev != gi ? BKV_FLUSH : 0);
+                            h_qt = qt;
+                            h_gi = gi;
+                            h_prev = prev;
+                            prev = gi;
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {         // a query behind the end has probability 0
+                                const int q = qt * ATT_BM + lane + 32 * i;
+                                const long r = ((long)b * T + q) * HQ + hkv * G + gi;
+                                nl[i] = q < T ? -lse[r] : -INFINITY;
+                                nd[i] = q < T ? -delta[r] : 0.f;
+                            }
+                        }
+                    }
+                    if (ok) announce(BKV_LAST);
+                    // the pair's last steps are under way: early enough to work out the next block, late enough to leave it to an SM
+                    // that is free earlier
+                    if (ok && sums) {
+                        request();
+                        requested = true;
+                    }
+                }
+                if (ok && !requested) request();                  // (the chosen pair had no step)
+                if (asked > answers) {                            // (also after a failed wait: the answer is on its way)
+                    const bool came = warp_wait(bar_clc, answers & 1);
+                    ++answers;
+                    ok = ok && came;
+                }
+                if (!ok || !taken_block(sbase + L::clc, block)) break;
+                __syncwarp();
             }
-            if (ok && !requested) request();                  // (the chosen pair had no step)
-            if (asked > answers) {                            // (also after a failed wait: the answer is on its way)
-                const bool came = warp_wait(bar_clc, answers & 1);
-                ++answers;
-                ok = ok && came;
-            }
-            if (!ok || !taken_block(sbase + L::clc, block)) break;
-            __syncwarp();
+            if (ok && open()) put(make_int4(0, BKV_STOP, 0, 0), make_int4(0, 0, 0, 0));
         }
-        if (ok) put(make_int4(0, BKV_STOP, 0, 0), make_int4(0, 0, 0, 0));
     } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(BKV_REGS_HIGH));
         // ------------------------------------------------------------ softmax: one key per thread and half, 64 queries each
-        const int quad = warp & 3, half = (warp - 2) >> 2, u = quad >> 1, part = (quad & 1) * 2 + half;
+        const int quad = warp & 3, half = (warp - 4) >> 2, u = quad >> 1, part = (quad & 1) * 2 + half;
         const uint32_t t_lane = tmem + ((uint32_t)(quad * 32) << 16);
         const uint32_t t_s = t_lane + C_S + half * 64, t_dp = t_lane + C_DP + half * 64;
         const float sl2 = scale * kLog2e;
-        unsigned char* const out = smem + L::out + (warp - 2) * 4096;
+        unsigned char* const out = smem + L::out + (warp - 4) * 4096;
+        int ni = 0, pairs = 0;                                // steps with queries, pairs that have some
         float dn = 0.f;
         auto flush = [&](int gi, int f) {                     // one slot per (key tile, head, warp): a fixed order of summation
             dn = warp_sum(dn);
@@ -802,6 +815,11 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             const int kt = u ? loc.y : loc.x, row0 = kt * 64 + (quad & 1) * 32;
 #pragma unroll 1
             for (int blk = half; blk < NB; blk += 2) {
+                if (acc) {                                    // dv is complete while dk's last product is still under way
+                    ok = warp_wait(blk < DV / 64 ? bar_dv : bar_acc, pairs & 1);
+                    if (!ok) return;
+                    tc_fence_after();
+                }
                 uint32_t w[32];
 #pragma unroll
                 for (int e = 0; e < 32; ++e) w[e] = 0;
@@ -855,21 +873,23 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
 #pragma unroll 1
         for (int blk = half; blk < NB; blk += 2) zero(block_col(blk));
         release_acc();
-        int ni = 0, pairs = 0;
+        int end_own = 0;                                      // end of the own block
 #pragma unroll 1
         while (true) {
             const int f = next_step();
             if (!ok || (f & BKV_STOP)) break;
             if (f & BKV_EMPTY) {
+                release_step();
                 finish(false, false);
-                if (warp == 2) write_sums(false);
+                if (warp == 4) write_sums(false);
                 continue;
             }
             const bool act = (f & (BKV_ACT0 << u)) != 0;
-            const int kt = u ? loc.y : loc.x, blk_end = (kt / cpb + 1) * nbs - d.x;      // relative to the first query
-            const float* st = reinterpret_cast<const float*>(smem + L::stat + (ni & 1) * 1024) + half * 64;
-            ok = warp_wait(st_full + (ni & 1) * 8, (ni >> 1) & 1);
-            if (ok) ok = warp_wait(bar_s, ni & 1);
+            const int kt = u ? loc.y : loc.x;
+            if (f & BKV_FIRST) end_own = (kt / cpb + 1) * nbs;
+            const int blk_end = end_own - d.x;                // relative to the first query
+            const float* st = reinterpret_cast<const float*>(smem + L::stat + (n_step & (BKV_DESCS - 1)) * 1024) + half * 64;
+            ok = warp_wait(bar_s, ni & 1);
             if (!ok) break;
             tc_fence_after();
             if (f & BKV_FLUSH) flush(d.w, f);                 // (every warp has left the pair before: its sums have been written)
@@ -887,21 +907,25 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                     for (int e = 0; e < 64; ++e)
                         if (e < lo || e >= hi) r[e] = 0xff800000u;
                 }
-                uint32_t pk[32];
                 const uint64_t sc2 = pack2(sl2, sl2);
 #pragma unroll
-                for (int e = 0; e < 32; e += 2) {
-                    const float4 l4 = *reinterpret_cast<const float4*>(st + 2 * e);
-                    float x0, x1, x2, x3;
-                    unpack2(fma2(pack2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1])), sc2, pack2(l4.x, l4.y)), x0, x1);
-                    unpack2(fma2(pack2(__uint_as_float(r[2 * e + 2]), __uint_as_float(r[2 * e + 3])), sc2, pack2(l4.z, l4.w)), x2, x3);
-                    x0 = ex2(x0), x1 = ex2(x1), x2 = ex2(x2), x3 = ex2(x3);
-                    r[2 * e] = __float_as_uint(x0), r[2 * e + 1] = __float_as_uint(x1);
-                    r[2 * e + 2] = __float_as_uint(x2), r[2 * e + 3] = __float_as_uint(x3);
-                    pk[e] = pack_bf16(x0, x1);
-                    pk[e + 1] = pack_bf16(x2, x3);
+                for (int h = 0; h < 2; ++h) {                 // (in halves: what is held in registers has to fit)
+                    uint32_t pk[16];
+#pragma unroll
+                    for (int i = 0; i < 16; i += 2) {
+                        const int e = h * 16 + i;
+                        const float4 l4 = *reinterpret_cast<const float4*>(st + 2 * e);
+                        float x0, x1, x2, x3;
+                        unpack2(fma2(pack2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1])), sc2, pack2(l4.x, l4.y)), x0, x1);
+                        unpack2(fma2(pack2(__uint_as_float(r[2 * e + 2]), __uint_as_float(r[2 * e + 3])), sc2, pack2(l4.z, l4.w)), x2, x3);
+                        x0 = ex2(x0), x1 = ex2(x1), x2 = ex2(x2), x3 = ex2(x3);
+                        r[2 * e] = __float_as_uint(x0), r[2 * e + 1] = __float_as_uint(x1);
+                        r[2 * e + 2] = __float_as_uint(x2), r[2 * e + 3] = __float_as_uint(x3);
+                        pk[i] = pack_bf16(x0, x1);
+                        pk[i + 1] = pack_bf16(x2, x3);
+                    }
+                    tmem_st16(t_s + h * 16, pk);
                 }
-                tmem_st32(t_s, pk);
                 tmem_st_wait();
             }
             tc_fence_before();
@@ -910,51 +934,58 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             if (!ok) break;
             tc_fence_after();
             if (act) {
-                uint32_t pk[32];
                 uint64_t sum = 0;
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    uint32_t x[32];
-                    tmem_ld32(t_dp + h * 32, x);
+                auto gradients = [&](auto behind) {
+                    constexpr bool later = decltype(behind)::value;
+                    uint32_t x0[32], x1[32];
+                    tmem_ld32(t_dp, x0);
+                    tmem_ld32(t_dp + 32, x1);
                     tmem_ld_wait();
 #pragma unroll
-                    for (int e = 0; e < 16; e += 2) {
-                        const float4 d4 = *reinterpret_cast<const float4*>(st + 128 + h * 32 + 2 * e);
-                        const uint32_t* p = r + h * 32 + 2 * e;
-                        const uint64_t a = mul2(pack2(__uint_as_float(p[0]), __uint_as_float(p[1])),
-                                                add2(pack2(__uint_as_float(x[2 * e]), __uint_as_float(x[2 * e + 1])), pack2(d4.x, d4.y)));
-                        const uint64_t c = mul2(pack2(__uint_as_float(p[2]), __uint_as_float(p[3])),
-                                                add2(pack2(__uint_as_float(x[2 * e + 2]), __uint_as_float(x[2 * e + 3])), pack2(d4.z, d4.w)));
-                        pk[h * 16 + e] = close2(a);
-                        pk[h * 16 + e + 1] = close2(c);
-                        if (blk_end <= half * 64) {           // all of them behind the own block
-                            sum = add2(sum, add2(a, c));
-                        } else {
-                            float a0, a1, c0, c1;
-                            unpack2(a, a0, a1);
-                            unpack2(c, c0, c1);
-                            const int at = half * 64 + h * 32 + 2 * e;
-                            dn += ((at >= blk_end ? a0 : 0.f) + (at + 1 >= blk_end ? a1 : 0.f)) + ((at + 2 >= blk_end ? c0 : 0.f) + (at + 3 >= blk_end ? c1 : 0.f));
+                    for (int h = 0; h < 2; ++h) {
+                        uint32_t pk[16];
+                        uint32_t(&x)[32] = h ? x1 : x0;
+#pragma unroll
+                        for (int e = 0; e < 16; e += 2) {
+                            const float4 d4 = *reinterpret_cast<const float4*>(st + 128 + h * 32 + 2 * e);
+                            const uint32_t* p = r + h * 32 + 2 * e;
+                            const uint64_t a = mul2(pack2(__uint_as_float(p[0]), __uint_as_float(p[1])),
+                                                    add2(pack2(__uint_as_float(x[2 * e]), __uint_as_float(x[2 * e + 1])), pack2(d4.x, d4.y)));
+                            const uint64_t c = mul2(pack2(__uint_as_float(p[2]), __uint_as_float(p[3])),
+                                                    add2(pack2(__uint_as_float(x[2 * e + 2]), __uint_as_float(x[2 * e + 3])), pack2(d4.z, d4.w)));
+                            pk[e] = close2(a);
+                            pk[e + 1] = close2(c);
+                            if (later) {
+                                sum = add2(sum, add2(a, c));
+                            } else {                              // queries of the own block do not count
+                                float a0, a1, c0, c1;
+                                unpack2(a, a0, a1);
+                                unpack2(c, c0, c1);
+                                const int at = half * 64 + h * 32 + 2 * e;
+                                sum = add2(sum, add2(pack2(at >= blk_end ? a0 : 0.f, at + 1 >= blk_end ? a1 : 0.f),
+                                                     pack2(at + 2 >= blk_end ? c0 : 0.f, at + 3 >= blk_end ? c1 : 0.f)));
+                            }
                         }
+                        tmem_st16(t_dp + h * 16, pk);
                     }
-                }
+                };
+                if (blk_end <= half * 64) gradients(std::true_type());       // all of them behind the own block
+                else gradients(std::false_type());
                 dn += hsum2(sum);
-                tmem_st32(t_dp, pk);
                 tmem_st_wait();
             }
             tc_fence_before();
             arrive(bar_ds);
-            if (lane == 0) mbar_arrive(st_empty + (ni & 1) * 8);
+            release_step();
             ++ni;
             if (!(f & BKV_LAST)) continue;
-            ok = warp_wait(bar_acc, pairs & 1);
-            if (!ok) break;
-            ++pairs;
-            tc_fence_after();
             flush(d.z, f);
             finish((f & (BKV_ANY0 << u)) != 0, true);
+            if (ok) ok = warp_wait(bar_acc, pairs & 1);       // (a phase passes by every warp: some have blocks of dv only)
+            if (!ok) break;
+            ++pairs;
             release_acc();
-            if (warp == 2) {                                  // in front of its part in the next step, behind which others flush again
+            if (warp == 4) {                                  // in front of its part in the next step, behind which others flush again
                 if (f & BKV_SUMS) ok = warp_wait(bar_acc_free, pairs & 1);
                 if (!ok) break;
                 write_sums((f & BKV_SUMS) != 0);
