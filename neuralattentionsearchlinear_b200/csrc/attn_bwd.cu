@@ -5,10 +5,9 @@
 // the gradients are dq = scale * ds k, dk = scale * ds^T q, dv = p^T do.
 //
 // Two kernels on the 5th-generation tensor cores, both deterministic (no atomics; every reduction has a fixed order).
-//   attn_bwd_dq_kernel    one CTA per (128 queries, query head), two per SM, warp roles as in the forward (320 threads: TMA
-//                         producer, MMA issuer, eight softmax warps with 16 query rows each, four threads per row): walks the
-//                         visible 64-key tiles, queries in the TMEM lanes, dq stays in TMEM; also writes delta (the preprocess
-//                         kernel of the reference folded in).  ds goes back to TMEM (over do.v) as the A operand of ds k.
+//   attn_bwd_dq_kernel    128 queries of a head against pairs of the 64-key tiles that they see, queries in the TMEM lanes: q k^T
+//                         and do v^T (128 x 128), ds back into TMEM (over do.v) as the A operand of dq += ds k, dq stays in TMEM.
+//                         It also writes delta (the preprocess kernel of the reference folded in).
 //   attn_bwd_dkdv_kernel  pairs of 64-key tiles (two of selected blocks, or what is unselected of two neighbours) against the
 //                         128-query tiles that see either, keys in the TMEM lanes: k q^T and v do^T (128 x 128), p and ds back
 //                         into TMEM as the A operands of dv += p do and dk += ds q.  It also sums ds over the later blocks'
@@ -29,294 +28,524 @@ namespace natsl {
 constexpr float kLog2e = 1.4426950408889634f;
 
 // ------------------------------------------------------------------------------------------------- dq
-template <int DK, int DV>
-struct DqSmem {
-    // 128 / 128: one V stage (its tile is free as soon as do.v is done) keeps the CTA at half an SM's shared memory
-    static constexpr int VST = DK + DV == 256 ? 1 : 2;
-    static constexpr int q = 0;                               // DK/64 sub-tiles [128][64]; at the end the dq staging
-    static constexpr int dos = q + 128 * DK * 2;              // DV/64 sub-tiles [128][64]
-    static constexpr int k = dos + 128 * DV * 2;              // 2 stages x DK/64 sub-tiles [64][64]
-    static constexpr int v = k + 2 * 64 * DK * 2;             // VST stages x DV/64 sub-tiles [64][64]
-    static constexpr int bars = v + VST * 64 * DV * 2;
-    static constexpr int list = bars + 160;                   // visible key tiles (16 bits each), NT entries
-    static int total(int NT) { return list + ((NT * 2 + 15) & ~15); }
-};
+// 128 queries against pairs of visible key tiles: all three products are 128 x 128 (x head dim), whose operands are read half as often
+// as by 128 x 64 ones, and p never leaves the registers.  One persistent CTA per SM takes blocks of the grid over (cluster launch
+// control).  Roles: warp 0 loads, warp 1 issues the products, warp 2 plans the steps, warps 4-11 p and ds (a query and 64 keys per
+// thread; half the warps per key tile).  o and do of the next block's rows, whose product is delta, are on their way to registers while
+// dq of the block before leaves.
+// Registers: 384 threads get 168 each, of which the first four warps give back what the others need to hold 64 scores and 64 values of
+// do.v, or a block's o and do.  Nothing may spill: the shared memory leaves so little of the first-level cache that a spilled word
+// comes back from L2, some 400 cycles in a chain in which nothing else hides them.
+// What bounds it: the chain scores -> p -> ds -> dq product of a step, 2.7 k cycles (1.45 k of them p, whose exponentials alone take the
+// special function units 1.0 k) against 1.5 k of the tensor core, and 4.4 k cycles between two blocks (delta, dq on its way out).
+// Alone (us; before: 128 x 64 score tiles, two CTAs per SM, one block each), block 64:
+//   128/128, B = 8, T = 4096, H = 16: 25 % selected 323 -> 265, 50 % 508 -> 410, 2 % 175 -> 141;  64/64, 30 %: 286 -> 239
+//   128/64, B = 4, T = 1000, H = 16, 50 %: 38 -> 30;  128/128, B = 1, T = 2048, H = 16, 30 %: 25.6 -> 23.5
+//   64/128, B = 2, T = 2048, 12 heads over 6, block 128, 40 %: 36 -> 30;  the smallest, B = 2, T = 64, H = 4: 6.3 -> 6.6
+// Of that the rows asked into L2 ahead are 8 us at 25 % and 9 us at 2 %.  Eight threads per row for delta, in whole lines: 275 us.
+constexpr int BDQ_THREADS = 384;                              // TMA, MMA, planner, (no work), 8 softmax warps
+constexpr int BDQ_STEPS = 2;                                  // steps that the planner is ahead
+constexpr int BWD_REGS_LOW = 88, BWD_REGS_HIGH = 208;         // a thread: 128 x 88 + 256 x 208 = 384 x 168
+// Heads whose blocks are interleaved, heaviest first: the last blocks to start are then light ones, and k and v of that many heads
+// (2 MB each at 4096 x 128) stay in L2.
+constexpr int BDQ_HEADS = 32;
 
 template <int DK, int DV>
-__global__ void __launch_bounds__(TC_THREADS, 2)
+struct DqSmem {
+    static constexpr int q = 0;                               // DK/64 sub-tiles [128][64]
+    static constexpr int dos = q + 128 * DK * 2;              // DV/64 sub-tiles
+    static constexpr int k = dos + 128 * DV * 2;              // 2 stages x DK/64 sub-tiles [128 keys][64]
+    static constexpr int v = k + 2 * 128 * DK * 2;            // 2 stages x DV/64 sub-tiles
+    static constexpr int out = v + 2 * 128 * DV * 2;          // per softmax warp: 32 rows x 64 columns on their way out
+    static constexpr int delta = out + 8 * 4096;              // delta of the rows, of an even / odd block
+    static constexpr int desc = delta + 2 * 512;              // steps, 32 bytes each
+    static constexpr int clc = desc + BDQ_STEPS * 32;         // answer of the take-over request
+    static constexpr int bars = clc + 16;
+    static constexpr int total = bars + 240;
+    static_assert(total <= 227 * 1024, "one CTA per SM");
+};
+
+// What a CTA does in a step: first key tile, flags, second key tile (-1: none); first query, query head, batch.
+enum : int {
+    BDQ_FIRST = 1, BDQ_LAST = 2,                              // first / last step of the block
+    BDQ_STOP = 4,                                             // no block is left
+    BDQ_OWN0 = 8, BDQ_OWN1 = 16,                              // the key tile is of the own span: masked per element
+    BDQ_SEL0 = 32, BDQ_SEL1 = 64                              // its block is selected
+};
+
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
+template <int DK, int DV>
+__global__ void __launch_bounds__(BDQ_THREADS, 1)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                    const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
-                   const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o, const float* __restrict__ lse,
-                   const int* __restrict__ types_i, __nv_bfloat16* __restrict__ dq, float* __restrict__ delta_out, int T, int HQ,
-                   int HKV, int HN, int TN, int nbs, float scale, int own, int* status) {
+                   const __grid_constant__ CUtensorMap map_dq, const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ o,
+                   const __nv_bfloat16* __restrict__ d_o, const float* __restrict__ lse, const int* __restrict__ types_i,
+                   float* __restrict__ delta_out, int T, int HQ, int HKV, int HN, int TN, int nbs, float scale, int own, int heads, int* status) {
     using L = DqSmem<DK, DV>;
-    constexpr int VST = L::VST;
-    constexpr uint32_t C_S = 0, C_DP = 64, C_DQ = 128;        // TMEM columns: scores; do.v, then ds; dq
+    constexpr uint32_t C_S = 0, C_DP = 128, C_DQ = 256;       // TMEM: scores; do.v, then ds over each half's first columns; dq
     extern __shared__ __align__(1024) unsigned char smem[];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const uint32_t sbase = smem_u32(smem);
     if ((sbase & 1023u) != 0) {
         if (tid == 0) atomicExch(status, 2);
         return;
     }
-    const int it = (int)gridDim.x - 1 - (int)blockIdx.x;      // heavy (late) query tiles first
-    const int hq = blockIdx.y, b = blockIdx.z;
-    const int hkv = hq / (HQ / HKV), hn = hq / (HQ / HN);
-    const int q0 = it * ATT_BM;
-    const int* selp = types_i + ((long)b * TN * HN + hn) * 2;  // column 0
-    const long tstride = (long)HN * 2;
-    const uint32_t s_q = sbase + L::q, s_do = sbase + L::dos, s_k = sbase + L::k, s_v = sbase + L::v;
+    const int NT = (T + 63) / 64, NTq = (T + ATT_BM - 1) / ATT_BM, cpb = nbs / 64;
+    float* s_delta = reinterpret_cast<float*>(smem + L::delta);
+    int4* s_desc = reinterpret_cast<int4*>(smem + L::desc);
     const uint32_t bar0 = sbase + L::bars;
-    const uint32_t bar_q = bar0, bar_k_full = bar0 + 8, bar_k_empty = bar0 + 24, bar_v_full = bar0 + 40, bar_v_empty = bar0 + 56,
-                   bar_s = bar0 + 72, bar_dp = bar0 + 80, bar_s_free = bar0 + 88, bar_ds = bar0 + 96, bar_done = bar0 + 104;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::bars + 112);
-    int* s_count = reinterpret_cast<int*>(smem + L::bars + 116);
-    uint16_t* s_list = reinterpret_cast<uint16_t*>(smem + L::list);
-    const int span0 = (q0 / nbs) * nbs / 64;                  // first key tile of the own span
-    const int cpb = nbs / 64;
-
+    // barriers: desc_full / desc_empty (steps); q_full / q_empty, do_full / do_empty (the block's); k_full / k_empty, v_full / v_empty
+    // (stages); s, dp (scores, do.v complete); s_free (scores read); ds (written); acc (dq complete); acc_free (read); delta (of all rows)
+    const uint32_t desc_full = bar0, desc_empty = bar0 + 16, k_full = bar0 + 32, k_empty = bar0 + 48, v_full = bar0 + 64,
+                   v_empty = bar0 + 80, q_full = bar0 + 96, q_empty = bar0 + 104, do_full = bar0 + 112, do_empty = bar0 + 120,
+                   bar_s = bar0 + 128, bar_s_free = bar0 + 136, bar_dp = bar0 + 144, bar_ds = bar0 + 152, bar_acc = bar0 + 160,
+                   bar_acc_free = bar0 + 168, bar_delta = bar0 + 176, bar_clc = bar0 + 184;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::bars + 192);
+    auto arrive = [&](uint32_t bar) {                         // behind what the whole warp has done so far
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar);
+    };
     if (tid == 0) {
-        mbar_init(bar_q, 1);
         for (int i = 0; i < 2; ++i) {
-            mbar_init(bar_k_full + 8 * i, 1);
-            mbar_init(bar_k_empty + 8 * i, 1);
-            mbar_init(bar_v_full + 8 * i, 1);
-            mbar_init(bar_v_empty + 8 * i, 1);
+            mbar_init(desc_full + 8 * i, 1);
+            mbar_init(desc_empty + 8 * i, 10);                // eight softmax warps, TMA, MMA
+            mbar_init(k_full + 8 * i, 1);
+            mbar_init(k_empty + 8 * i, 1);
+            mbar_init(v_full + 8 * i, 1);
+            mbar_init(v_empty + 8 * i, 1);
         }
+        mbar_init(q_full, 1);
+        mbar_init(q_empty, 1);
+        mbar_init(do_full, 1);
+        mbar_init(do_empty, 1);
         mbar_init(bar_s, 1);
+        mbar_init(bar_s_free, 8);
         mbar_init(bar_dp, 1);
-        mbar_init(bar_s_free, 8);                             // one arrival per softmax warp
         mbar_init(bar_ds, 8);
-        mbar_init(bar_done, 1);
+        mbar_init(bar_acc, 1);
+        mbar_init(bar_acc_free, 8);
+        mbar_init(bar_delta, 8);
+        mbar_init(bar_clc, 1);
         mbar_fence_init();
-        mbar_expect_tx(bar_q, 128 * (DK + DV) * 2);
-#pragma unroll
-        for (int sub = 0; sub < DK / 64; ++sub) tma_load_4d(s_q + sub * 16384, &map_q, sub * 64, hq, q0, b, bar_q);
-#pragma unroll
-        for (int sub = 0; sub < DV / 64; ++sub) tma_load_4d(s_do + sub * 16384, &map_do, sub * 64, hq, q0, b, bar_q);
     }
-    if (warp == 1) tmem_alloc(smem_u32(tmem_slot), TC_TMEM_COLS);
-    if (warp == 2) {
-        // visible key tiles in ascending order: sub-tiles of selected blocks before the own span, then the own span
-        // (whose entries are masked per element)
-        const int n_cand = min((q0 + ATT_BM + 63) / 64, (T + 63) / 64);
-        int count = 0;
-#pragma unroll 1
-        for (int base = 0; base < n_cand; base += 32) {
-            const int kt = base + lane;
-            const bool vis = kt < n_cand && (kt >= span0 || selp[(long)(kt / cpb) * tstride] != 0);
-            const unsigned m = __ballot_sync(0xffffffffu, vis);
-            if (vis) s_list[count + __popc(m & ((1u << lane) - 1))] = (uint16_t)kt;
-            count += __popc(m);
-        }
-        if (lane == 0) *s_count = count;
-    }
+    if (warp == 1) tmem_alloc(smem_u32(tmem_slot), 512);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
-    const int n_tiles = *s_count;                             // >= 1: the own span is never empty
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     bool ok = true;
+    int n_step = 0;
+    int4 d, loc;                                              // the step's words
+    auto next_step = [&]() -> int {                           // its flags
+        const int slot = n_step & (BDQ_STEPS - 1);
+        ok = warp_wait(desc_full + slot * 8, (n_step / BDQ_STEPS) & 1);
+        d = s_desc[2 * slot];
+        loc = s_desc[2 * slot + 1];
+        d.y = ok ? __shfl_sync(0xffffffffu, d.y, 0) : BDQ_STOP;
+        return d.y;
+    };
+    auto release_step = [&]() { arrive(desc_empty + (n_step++ & (BDQ_STEPS - 1)) * 8); };
 
-    if (warp == 0) {
-        // ------------------------------------------------------------ TMA producer
+    if (warp < 4) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(BWD_REGS_LOW));
+        if (warp == 0) {
+            // -------------------------------------------------------- TMA producer
+            int n = 0, nq = 0, ndo = 0, nk = 0, nv = 0;       // steps; loads under way or done
 #pragma unroll 1
-        for (int j = 0; ok && j < n_tiles; ++j) {
-            const int ks = j & 1, vs = j % VST, t0 = s_list[j] * 64;
-            if (j >= 2) ok = warp_wait(bar_k_empty + ks * 8, ((j >> 1) - 1) & 1);
-            if (!ok) break;
-            if (lane == 0) {
-                mbar_expect_tx(bar_k_full + ks * 8, 64 * DK * 2);
+            while (true) {
+                next_step();
+                release_step();
+                if (d.y & BDQ_STOP) break;
+                const int q0 = loc.x, hq = loc.y, b = loc.z, hkv = hq / (HQ / HKV);
+                const int st = n & 1, par = ((n >> 1) - 1) & 1, tiles = d.z < 0 ? 1 : 2;
+                auto rows = [&](int u) -> int { return (u ? d.z : d.x) * 64; };
+                if (lane == 0 && n >= 2) {                    // into L2 while the stages are still read
+                    for (int u = 0; u < tiles; ++u) {
 #pragma unroll
-                for (int sub = 0; sub < DK / 64; ++sub)
-                    tma_load_4d(s_k + ks * (64 * DK * 2) + sub * 8192, &map_k, sub * 64, hkv, t0, b, bar_k_full + ks * 8);
+                        for (int sub = 0; sub < DK / 64; ++sub) tma_prefetch_4d(&map_k, sub * 64, hkv, rows(u), b);
 #pragma unroll
-                for (int sub = 0; sub < DV / 64; ++sub) tma_prefetch_4d(&map_v, sub * 64, hkv, t0, b);
+                        for (int sub = 0; sub < DV / 64; ++sub) tma_prefetch_4d(&map_v, sub * 64, hkv, rows(u), b);
+                    }
+                }
+                __syncwarp();
+                if (d.y & BDQ_FIRST) {
+                    if (nq > 0) ok = warp_wait(q_empty, (nq - 1) & 1);
+                    if (!ok) break;
+                    if (lane == 0) {
+                        mbar_expect_tx(q_full, 128 * DK * 2);
+#pragma unroll
+                        for (int sub = 0; sub < DK / 64; ++sub) tma_load_4d(sbase + L::q + sub * 16384, &map_q, sub * 64, hq, q0, b, q_full);
+                    }
+                    __syncwarp();
+                    ++nq;
+                }
+                if (n >= 2) ok = warp_wait(k_empty + st * 8, par);
+                if (!ok) break;
+                if (lane == 0) {
+                    mbar_expect_tx(k_full + st * 8, tiles * 64 * DK * 2);
+                    for (int u = 0; u < tiles; ++u)
+#pragma unroll
+                        for (int sub = 0; sub < DK / 64; ++sub)
+                            tma_load_4d(sbase + L::k + st * (128 * DK * 2) + sub * 16384 + u * 8192, &map_k, sub * 64, hkv, rows(u), b,
+                                        k_full + st * 8);
+                }
+                __syncwarp();
+                ++nk;
+                if (d.y & BDQ_FIRST) {
+                    if (ndo > 0) ok = warp_wait(do_empty, (ndo - 1) & 1);
+                    if (!ok) break;
+                    if (lane == 0) {
+                        mbar_expect_tx(do_full, 128 * DV * 2);
+#pragma unroll
+                        for (int sub = 0; sub < DV / 64; ++sub) tma_load_4d(sbase + L::dos + sub * 16384, &map_do, sub * 64, hq, q0, b, do_full);
+                    }
+                    __syncwarp();
+                    ++ndo;
+                }
+                if (n >= 2) ok = warp_wait(v_empty + st * 8, par);
+                if (!ok) break;
+                if (lane == 0) {
+                    mbar_expect_tx(v_full + st * 8, tiles * 64 * DV * 2);
+                    for (int u = 0; u < tiles; ++u)
+#pragma unroll
+                        for (int sub = 0; sub < DV / 64; ++sub)
+                            tma_load_4d(sbase + L::v + st * (128 * DV * 2) + sub * 16384 + u * 8192, &map_v, sub * 64, hkv, rows(u), b,
+                                        v_full + st * 8);
+                }
+                __syncwarp();
+                ++nv;
+                ++n;
             }
-            __syncwarp();
-            if (j >= VST) ok = warp_wait(bar_v_empty + vs * 8, ((j / VST) - 1) & 1);
-            if (!ok) break;
-            if (lane == 0) {
-                mbar_expect_tx(bar_v_full + vs * 8, 64 * DV * 2);
-#pragma unroll
-                for (int sub = 0; sub < DV / 64; ++sub)
-                    tma_load_4d(s_v + vs * (64 * DV * 2) + sub * 8192, &map_v, sub * 64, hkv, t0, b, bar_v_full + vs * 8);
+            if (!ok) {                                        // nothing may still be on its way into shared memory
+                if (nq > 0) warp_wait(q_full, (nq - 1) & 1);
+                if (ndo > 0) warp_wait(do_full, (ndo - 1) & 1);
+                for (int i = max(0, nk - 2); i < nk; ++i) warp_wait(k_full + (i & 1) * 8, (i >> 1) & 1);
+                for (int i = max(0, nv - 2); i < nv; ++i) warp_wait(v_full + (i & 1) * 8, (i >> 1) & 1);
             }
-            __syncwarp();
-        }
-    } else if (warp == 1) {
-        // ------------------------------------------------------------ MMA issuer
-        constexpr uint32_t id_s = umma_idesc_bf16(128, 64, false);
-        constexpr uint32_t id_dq = umma_idesc_bf16(128, DK, true);
-        auto issue_s = [&](int j) {                           // S = Q K_j^T
-            const uint32_t kt = s_k + (j & 1) * (64 * DK * 2);
-            const uint32_t ql = umma_desc_lo(s_q, 16), kl = umma_desc_lo(kt, 16);
+        } else if (warp == 1) {
+            // -------------------------------------------------------- MMA issuer
+            constexpr uint32_t id_s = umma_idesc_bf16(128, 128, false), id_dq = umma_idesc_bf16(128, DK, true);
+            const uint32_t ql = umma_desc_lo(sbase + L::q, 16), dl = umma_desc_lo(sbase + L::dos, 16);
+            int n = 0, nq = 0, ndo = 0, done = 0;             // steps; blocks begun (scores, do.v) and complete
+            auto scores = [&](int i, int f) {                 // Q K^T of step i
+                ok = warp_wait(k_full + (i & 1) * 8, (i >> 1) & 1);
+                if (ok && (f & BDQ_FIRST)) ok = warp_wait(q_full, nq++ & 1);
+                if (!ok) return;
+                tc_fence_after();
+                const uint32_t kl = umma_desc_lo(sbase + L::k + (i & 1) * (128 * DK * 2), 16);
 #pragma unroll
-            for (int h = 0; h < DK / 64; ++h) umma_ss_x4<2, 2>(tmem + C_S, ql + h * 1024, kl + h * 512, id_s, h > 0);
-            umma_commit(bar_s);
-        };
-        auto issue_dp = [&](int j) {                          // dO V_j^T
-            const uint32_t vt = s_v + (j % VST) * (64 * DV * 2);
-            const uint32_t dl = umma_desc_lo(s_do, 16), vl = umma_desc_lo(vt, 16);
+                for (int h = 0; h < DK / 64; ++h) umma_ss_x4<2, 2>(tmem + C_S, ql + h * 1024, kl + h * 1024, id_s, h > 0);
+                umma_commit(bar_s);
+                if (f & BDQ_LAST) umma_commit(q_empty);
+            };
+            auto products = [&](int i, int f) {               // dO V^T
+                ok = warp_wait(v_full + (i & 1) * 8, (i >> 1) & 1);
+                if (ok && (f & BDQ_FIRST)) ok = warp_wait(do_full, ndo++ & 1);
+                if (!ok) return;
+                tc_fence_after();
+                const uint32_t vl = umma_desc_lo(sbase + L::v + (i & 1) * (128 * DV * 2), 16);
 #pragma unroll
-            for (int h = 0; h < DV / 64; ++h) umma_ss_x4<2, 2>(tmem + C_DP, dl + h * 1024, vl + h * 512, id_s, h > 0);
-            umma_commit(bar_dp);
-            umma_commit(bar_v_empty + (j % VST) * 8);
-        };
-        ok = warp_wait(bar_q, 0);
-        if (ok) ok = warp_wait(bar_k_full, 0);
-        if (ok) {
-            tc_fence_after();
-            issue_s(0);
-        }
-        if (ok) ok = warp_wait(bar_v_full, 0);
-        if (ok) {
-            tc_fence_after();
-            issue_dp(0);
-        }
+                for (int h = 0; h < DV / 64; ++h) umma_ss_x4<2, 2>(tmem + C_DP, dl + h * 1024, vl + h * 1024, id_s, h > 0);
+                umma_commit(bar_dp);
+                umma_commit(v_empty + (i & 1) * 8);
+                if (f & BDQ_LAST) umma_commit(do_empty);
+            };
+            int f = next_step();
+            bool two = d.z >= 0;
+            release_step();
+            if (!(f & BDQ_STOP)) {
+                scores(0, f);
+                if (ok) products(0, f);
+            }
 #pragma unroll 1
-        for (int j = 0; ok && j < n_tiles; ++j) {
-            const int jn = j + 1;
-            if (jn < n_tiles) {                               // the next scores as soon as these have been read
-                ok = warp_wait(bar_k_full + (jn & 1) * 8, (jn >> 1) & 1);
-                if (ok) ok = warp_wait(bar_s_free, j & 1);
+            while (ok && !(f & BDQ_STOP)) {
+                const int fn = next_step();                   // the next scores as soon as these have been read
+                const bool two_n = d.z >= 0;
+                release_step();
+                const bool more = !(fn & BDQ_STOP);
+                if (ok && more) {
+                    ok = warp_wait(bar_s_free, n & 1);
+                    if (ok) {
+                        tc_fence_after();
+                        scores(n + 1, fn);
+                    }
+                }
+                if (ok) ok = warp_wait(bar_ds, n & 1);
+                if (ok && (f & BDQ_FIRST) && done > 0) ok = warp_wait(bar_acc_free, (done - 1) & 1);
                 if (!ok) break;
                 tc_fence_after();
-                issue_s(jn);
+                const uint32_t kl = umma_desc_lo(sbase + L::k + (n & 1) * (128 * DK * 2), 16384);
+                umma_ts_x4<128>(tmem + C_DQ, tmem + C_DP, kl, id_dq, !(f & BDQ_FIRST));
+                if (two) umma_ts_x4<128>(tmem + C_DQ, tmem + C_DP + 64, kl + 512, id_dq, 1u);
+                umma_commit(k_empty + (n & 1) * 8);
+                if (f & BDQ_LAST) {
+                    umma_commit(bar_acc);
+                    ++done;
+                }
+                if (more) products(n + 1, fn);                // behind ds k in the tensor pipe: ds may be overwritten
+                f = fn;
+                two = two_n;
+                ++n;
             }
-            ok = warp_wait(bar_ds, j & 1);
-            if (!ok) break;
-            tc_fence_after();
-            const uint32_t kt = s_k + (j & 1) * (64 * DK * 2);
-            umma_ts_x4<128>(tmem + C_DQ, tmem + C_DP, umma_desc_lo(kt, 8192), id_dq, j > 0);
-            umma_commit(jn < n_tiles ? bar_k_empty + (j & 1) * 8 : bar_done);
-            if (jn < n_tiles) {
-                ok = warp_wait(bar_v_full + (jn % VST) * 8, (jn / VST) & 1);
-                if (!ok) break;
-                tc_fence_after();
-                issue_dp(jn);                                 // behind ds k in the tensor pipe: ds may be overwritten
+        } else if (warp == 2) {
+            // -------------------------------------------------------- planner: blocks and their steps
+            int n = 0, asked = 0, answers = 0;                // steps, take-over requests
+            int block = blockIdx.x;
+            auto put = [&](int4 x, int4 y) {
+                const int slot = n & (BDQ_STEPS - 1);
+                if (n >= BDQ_STEPS) ok = warp_wait(desc_empty + slot * 8, (n / BDQ_STEPS - 1) & 1);
+                if (!ok) return;
+                if (lane == 0) {
+                    s_desc[2 * slot] = x;
+                    s_desc[2 * slot + 1] = y;
+                }
+                arrive(desc_full + slot * 8);
+                ++n;
+            };
+#pragma unroll 1
+            while (ok) {
+                if (lane == 0) {                              // ask for the next block: heavy ones come first, so one ahead does no harm
+                    fence_async_smem();
+                    mbar_expect_tx(bar_clc, 16);
+                    request_block(sbase + L::clc, bar_clc);
+                }
+                __syncwarp();
+                ++asked;
+                const int hbase = block / (BDQ_HEADS * NTq) * BDQ_HEADS, hcount = min(BDQ_HEADS, heads - hbase);
+                const int within = block - hbase * NTq, item = within / hcount, head = hbase + within % hcount;
+                const int hq = head % HQ, b = head / HQ, q0 = (NTq - 1 - item) * ATT_BM;
+                const int* selp = types_i + ((long)b * TN * HN + hq / (HQ / HN)) * 2;              // column 0
+                const long tstride = (long)HN * 2;
+                const int span0 = (q0 / nbs) * cpb;           // first key tile of the own span
+                const int n_cand = min((q0 + ATT_BM + 63) / 64, NT);
+                const int4 where = make_int4(q0, hq, b, 0);
+                for (int i = n > 0 ? lane : 128; i < 128; i += 32) {       // its rows into L2 while the block before is worked on
+                    const long t = ((long)b * T + min(q0 + i, T - 1)) * HQ + hq;
+#pragma unroll
+                    for (int c = 0; c < DK; c += 64) prefetch_l2(q + t * DK + c);
+#pragma unroll
+                    for (int c = 0; c < DV; c += 64) {
+                        prefetch_l2(o + t * DV + c);
+                        prefetch_l2(d_o + t * DV + c);
+                    }
+                }
+                // visible key tiles in ascending order, two to a step: those of selected blocks in front of the own span, then the
+                // own span.  A step is announced once it is known whether another follows.
+                int held0 = -1, held1 = -1, flags = BDQ_FIRST;
+                auto selected = [&](int kt) -> bool { return kt < n_cand && selp[(long)(kt / cpb) * tstride] != 0; };
+                bool sel_n = selected(lane);
+#pragma unroll 1
+                for (int base = 0; ok && base < n_cand; base += 32) {
+                    const bool sel = sel_n;
+                    if (base + 32 < n_cand) sel_n = selected(base + 32 + lane);
+                    const unsigned ms = __ballot_sync(0xffffffffu, sel);
+                    unsigned m = __ballot_sync(0xffffffffu, base + lane < n_cand && (base + lane >= span0 || sel));
+                    while (ok && m) {
+                        const int i = __ffs(m) - 1, kt = base + i;
+                        m &= m - 1;
+                        const int mine = (kt >= span0 ? BDQ_OWN0 : 0) | ((ms >> i) & 1 ? BDQ_SEL0 : 0);
+                        if (held0 >= 0 && held1 < 0) {
+                            held1 = kt;
+                            flags |= mine << 1;
+                            continue;
+                        }
+                        if (held0 >= 0) {
+                            put(make_int4(held0, flags, held1, 0), where);
+                            flags = 0;
+                        }
+                        held0 = kt;
+                        held1 = -1;
+                        flags |= mine;
+                    }
+                }
+                if (ok) put(make_int4(held0, flags | BDQ_LAST, held1, 0), where);    // (the own span is never empty)
+                const bool came = warp_wait(bar_clc, answers & 1);                   // (also after a failed wait: the answer is on its way)
+                ++answers;
+                ok = ok && came;
+                if (!ok || !taken_block(sbase + L::clc, block)) break;
+                __syncwarp();
             }
+            if (ok) put(make_int4(0, BDQ_STOP, -1, 0), make_int4(0, 0, 0, 0));
         }
     } else {
-        // ------------------------------------------------------------ softmax (8 warps)
-        const int quad = warp & 3, half = (warp - 2) >> 2;
-        const int row_a = quad * 32 + half * 16 + (lane >> 2), row_b = row_a + 8;
-        const int cq = (lane & 3) * 2;
-        const int t_a = q0 + row_a, t_b = q0 + row_b;
-        const uint32_t t_rows = tmem + ((uint32_t)(quad * 32 + half * 16) << 16);
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(BWD_REGS_HIGH));
+        // ------------------------------------------------------------ softmax: one query per thread and half, 64 keys each
+        const int quad = warp & 3, half = (warp - 4) >> 2, row = quad * 32 + lane;
+        const uint32_t t_lane = tmem + ((uint32_t)(quad * 32) << 16);
+        const uint32_t t_s = t_lane + C_S + half * 64, t_dp = t_lane + C_DP + half * 64;
         const float sl2 = scale * kLog2e;
-        // delta = rowsum(o * do): four threads per row
-        auto row_delta = [&](int t) -> float {
-            float s = 0.f;
-            if (t < T) {
+        unsigned char* const out = smem + L::out + (warp - 4) * 4096;
+        // delta = rowsum(o * do): this warp's 16 rows, four threads per row and eight rows at a time
+        constexpr int NC = DV / 32;
+        const int drow = (warp - 4) * 16 + (lane >> 2);
+        uint4 xo[2][NC], xd[2][NC];
+        float nlse = 0.f;
+        auto load_rows = [&]() {                              // of the block in `loc`
+            const int q0 = loc.x, hq = loc.y, b = loc.z;
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int t = q0 + drow + 8 * i;
                 const long off = (((long)b * T + t) * HQ + hq) * DV + (lane & 3) * 8;
 #pragma unroll
-                for (int c = 0; c < DV / 32; ++c) {
-                    const uint4 x = *reinterpret_cast<const uint4*>(o + off + c * 32);
-                    const uint4 y = *reinterpret_cast<const uint4*>(d_o + off + c * 32);
-                    const uint32_t* xw = reinterpret_cast<const uint32_t*>(&x);
-                    const uint32_t* yw = reinterpret_cast<const uint32_t*>(&y);
+                for (int c = 0; c < NC; ++c) {
+                    xo[i][c] = t < T ? *reinterpret_cast<const uint4*>(o + off + c * 32) : make_uint4(0, 0, 0, 0);
+                    xd[i][c] = t < T ? *reinterpret_cast<const uint4*>(d_o + off + c * 32) : make_uint4(0, 0, 0, 0);
+                }
+            }
+            nlse = q0 + row < T ? -lse[((long)b * T + q0 + row) * HQ + hq] : 0.f;
+        };
+        auto make_delta = [&](int block) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                uint64_t s2 = 0;
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    const uint32_t* xw = reinterpret_cast<const uint32_t*>(&xo[i][c]);
+                    const uint32_t* yw = reinterpret_cast<const uint32_t*>(&xd[i][c]);
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
                         const float2 u = unpack_bf16(xw[e]), w = unpack_bf16(yw[e]);
-                        s += u.x * w.x + u.y * w.y;
+                        s2 = fma2(pack2(u.x, u.y), pack2(w.x, w.y), s2);
+                    }
+                }
+                float s = hsum2(s2);
+                s += __shfl_xor_sync(0xffffffffu, s, 1);
+                s += __shfl_xor_sync(0xffffffffu, s, 2);
+                const int r = drow + 8 * i, t = loc.x + r;
+                if ((lane & 3) == 0) {
+                    s_delta[(block & 1) * 128 + r] = s;
+                    if (t < T) delta_out[((long)loc.z * T + t) * HQ + loc.y] = s;
+                }
+            }
+            arrive(bar_delta);
+        };
+        // this warp's rows of dq: 64 columns at a time through its own 4 KB
+        auto finish = [&](int q0, int hq, int b, int block) {
+            if (!ok) return;
+            ok = warp_wait(bar_acc, block & 1);
+            if (!ok) return;
+            tc_fence_after();
+            if (half < DK / 64) {
+                if (lane == 0) tma_store_wait_read();         // the block before has left
+                __syncwarp();
+#pragma unroll
+                for (int c = 0; c < 64; c += 32) {            // (in halves: o and do of the next block are held as well)
+                    uint32_t x[32];
+                    tmem_ld32(t_lane + C_DQ + half * 64 + c, x);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        uint32_t w[4];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+                            w[e] = pack_bf16(__uint_as_float(x[8 * i + 2 * e]) * scale, __uint_as_float(x[8 * i + 2 * e + 1]) * scale);
+                        *reinterpret_cast<uint4*>(out + lane * 128 + (((c / 8 + i) ^ (lane & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
                     }
                 }
             }
-            s += __shfl_xor_sync(0xffffffffu, s, 1);
-            s += __shfl_xor_sync(0xffffffffu, s, 2);
-            return s;
+            tc_fence_before();
+            arrive(bar_acc_free);
+            if (half >= DK / 64) return;
+            fence_async_smem();
+            __syncwarp();
+            if (lane == 0 && q0 + quad * 32 < T) {
+                tma_store_4d(&map_dq, smem_u32(out), half * 64, hq, q0 + quad * 32, b);
+                tma_store_commit();
+            }
         };
-        const float del_a = row_delta(t_a), del_b = row_delta(t_b);
-        float lse_a = 0.f, lse_b = 0.f;
-        if (t_a < T) lse_a = lse[((long)b * T + t_a) * HQ + hq];
-        if (t_b < T) lse_b = lse[((long)b * T + t_b) * HQ + hq];
-        if ((lane & 3) == 0) {
-            if (t_a < T) delta_out[((long)b * T + t_a) * HQ + hq] = del_a;
-            if (t_b < T) delta_out[((long)b * T + t_b) * HQ + hq] = del_b;
-        }
+        int n = 0, blocks = 0;                                // steps, blocks begun
+        float ndel = 0.f;
+        int f = next_step();
+        if (!(f & BDQ_STOP)) load_rows();
 #pragma unroll 1
-        for (int j = 0; j < n_tiles; ++j) {
-            ok = warp_wait(bar_s, j & 1);
+        while (ok && !(f & BDQ_STOP)) {
+            if (f & BDQ_FIRST) make_delta(blocks++);
+            const int kt = half ? d.z : d.x;
+            const bool act = kt >= 0;
+            ok = warp_wait(bar_s, n & 1);
             if (!ok) break;
             tc_fence_after();
-            uint32_t sr[32], pr[16];
-            tmem_ld_16x256b_x8(t_rows + C_S, sr);
-            tmem_ld_wait();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_s_free);
-            const int kt = s_list[j];
-            if (kt >= span0) {
-                // own-span tile: per row the visible keys are columns [0, limit] (attn_walk.cuh: visible()); an invisible
-                // score becomes -inf, its p zero
-                const int s0 = kt * 64, blk = s0 / nbs, blk_end = (blk + 1) * nbs;
-                const bool selb = selp[(long)blk * tstride] != 0;
-                int lim_a = T - 1 - s0, lim_b = lim_a;
-                if (t_a < blk_end) lim_a = own ? min(lim_a, t_a - s0) : -1;
-                else if (!selb) lim_a = -1;
-                if (t_b < blk_end) lim_b = own ? min(lim_b, t_b - s0) : -1;
-                else if (!selb) lim_b = -1;
-#pragma unroll
-                for (int k = 0; k < 8; ++k)
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        const int c = 8 * k + cq + e;
-                        if (c > lim_a) sr[4 * k + e] = 0xff800000u;
-                        if (c > lim_b) sr[4 * k + 2 + e] = 0xff800000u;
-                    }
+            uint32_t r[64];
+            if (act) {
+                uint32_t(&r0)[32] = *reinterpret_cast<uint32_t(*)[32]>(r);
+                uint32_t(&r1)[32] = *reinterpret_cast<uint32_t(*)[32]>(r + 32);
+                tmem_ld32(t_s, r0);
+                tmem_ld32(t_s + 32, r1);
+                tmem_ld_wait();
             }
+            tc_fence_before();
+            arrive(bar_s_free);
+            if (act) {
+                if (f & (BDQ_OWN0 << half)) {
+                    // own-span tile: the row's visible keys are columns [0, lim] (attn_walk.cuh: visible()); an invisible score
+                    // becomes -inf, its p zero
+                    const int s0 = kt * 64, blk_end = (kt / cpb + 1) * nbs, t = loc.x + row;
+                    int lim = T - 1 - s0;
+                    if (t < blk_end) lim = own ? min(lim, t - s0) : -1;
+                    else if (!(f & (BDQ_SEL0 << half))) lim = -1;
 #pragma unroll
-            for (int k = 0; k < 8; ++k)
+                    for (int e = 0; e < 64; ++e)
+                        if (e > lim) r[e] = 0xff800000u;
+                }
+                const uint64_t sc2 = pack2(sl2, sl2), l2 = pack2(nlse, nlse);
 #pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    sr[4 * k + e] = __float_as_uint(ex2(fmaf(__uint_as_float(sr[4 * k + e]), sl2, (e >> 1) ? -lse_b : -lse_a)));
-            ok = warp_wait(bar_dp, j & 1);
+                for (int e = 0; e < 64; e += 2) {
+                    float x0, x1;
+                    unpack2(fma2(pack2(__uint_as_float(r[e]), __uint_as_float(r[e + 1])), sc2, l2), x0, x1);
+                    r[e] = __float_as_uint(ex2(x0));
+                    r[e + 1] = __float_as_uint(ex2(x1));
+                }
+            }
+            if (f & BDQ_FIRST) {
+                ok = warp_wait(bar_delta, (blocks - 1) & 1);
+                if (!ok) break;
+                ndel = -s_delta[((blocks - 1) & 1) * 128 + row];
+            }
+            ok = warp_wait(bar_dp, n & 1);
             if (!ok) break;
             tc_fence_after();
-            uint32_t dr[32];
-            tmem_ld_16x256b_x8(t_rows + C_DP, dr);
-            tmem_ld_wait();
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                pr[2 * k] = pack_bf16(__uint_as_float(sr[4 * k]) * (__uint_as_float(dr[4 * k]) - del_a),
-                                      __uint_as_float(sr[4 * k + 1]) * (__uint_as_float(dr[4 * k + 1]) - del_a));
-                pr[2 * k + 1] = pack_bf16(__uint_as_float(sr[4 * k + 2]) * (__uint_as_float(dr[4 * k + 2]) - del_b),
-                                          __uint_as_float(sr[4 * k + 3]) * (__uint_as_float(dr[4 * k + 3]) - del_b));
-            }
-            tmem_st_16x128b_x8(t_rows + C_DP, pr);            // ds over the first 32 columns of do.v
-            tmem_st_wait();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_ds);
-        }
-        if (ok) ok = warp_wait(bar_done, 0);
-        unsigned char* stage = smem + L::q;
-        if (ok) {
-            tc_fence_after();
-#pragma unroll 1
-            for (int c0 = 0; c0 < DK; c0 += 64) {
-                uint32_t r[32];
-                tmem_ld_16x256b_x8(t_rows + C_DQ + c0, r);
+            if (act) {
+                const uint64_t d2 = pack2(ndel, ndel);
+                uint32_t x0[32], x1[32];
+                tmem_ld32(t_dp, x0);
+                tmem_ld32(t_dp + 32, x1);
                 tmem_ld_wait();
 #pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    const int chunk = (c0 >> 3) + k;
-                    *reinterpret_cast<uint32_t*>(stage + swz<DK * 2>(row_a, chunk) + (lane & 3) * 4) =
-                        pack_bf16(__uint_as_float(r[4 * k]) * scale, __uint_as_float(r[4 * k + 1]) * scale);
-                    *reinterpret_cast<uint32_t*>(stage + swz<DK * 2>(row_b, chunk) + (lane & 3) * 4) =
-                        pack_bf16(__uint_as_float(r[4 * k + 2]) * scale, __uint_as_float(r[4 * k + 3]) * scale);
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t pk[16];
+                    uint32_t(&x)[32] = h ? x1 : x0;
+#pragma unroll
+                    for (int e = 0; e < 16; ++e)
+                        pk[e] = close2(mul2(pack2(__uint_as_float(r[h * 32 + 2 * e]), __uint_as_float(r[h * 32 + 2 * e + 1])),
+                                            add2(pack2(__uint_as_float(x[2 * e]), __uint_as_float(x[2 * e + 1])), d2)));
+                    tmem_st16(t_dp + h * 16, pk);
                 }
+                tmem_st_wait();
             }
+            tc_fence_before();
+            arrive(bar_ds);
+            ++n;
+            const int4 was = loc;
+            release_step();
+            const int fn = next_step();
+            if (f & BDQ_LAST) {
+                const bool had = ok;                          // (the block is complete also if no next one is known)
+                if (!(fn & BDQ_STOP)) load_rows();
+                ok = true;
+                finish(was.x, was.y, was.z, blocks - 1);
+                ok = ok && had;
+            }
+            f = fn;
         }
-        asm volatile("bar.sync 1, 256;" ::: "memory");       // every softmax warp reaches it, also after a failed wait
-        if (ok)
-            store_tile<128, DK, 256>(stage, dq + (((long)b * T + q0) * HQ + hq) * DK, (long)HQ * DK, min(128, T - q0), tid - 64);
+        if (lane == 0) tma_store_wait_read();
+        __syncwarp();
     }
+    // ---------------------------------------------------------------- teardown
     if (!ok && lane == 0) atomicExch(status, NATSL_DEV_WAIT_TIMEOUT);
     tc_fence_before();
     __syncthreads();
-    if (warp == 1) tmem_dealloc(tmem, TC_TMEM_COLS);
+    if (warp == 1) tmem_dealloc(tmem, 512);
 }
 
 // ------------------------------------------------------------------------------------------------- dk, dv
@@ -326,9 +555,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
 // One persistent CTA per SM takes blocks of the grid over (cluster launch control); a planning warp works out their steps, and
 // lse and delta of the queries, while the others are at the steps before.  Roles: warp 0 loads, warp 1 issues the products, warp 2
 // plans, warps 4-11 p and ds (a key and 64 queries per thread).
-// Registers: 384 threads get 168 each, of which the first four warps give back what the others need for p, ds and do.v of 64 queries.
-// Nothing may spill: the shared memory leaves so little of the first-level cache that a spilled word comes back from L2, some 400
-// cycles in a chain in which nothing else hides them (168 for all, 56 bytes of spills: 389 us where the figures below have 355).
+// Registers as above: 168 for all threads and 56 bytes of spills took 389 us where the figures below have 355.
 // What bounds it: the chain scores -> p -> dv product and do.v -> ds -> dk product of a step, 3 k cycles against 2 k of the tensor
 // core (tensor memory holds one step: 128 columns each of scores, do.v, dk and dv), and 64 KB of q and do from L2 a step.
 // Alone (us; before: 128 x 64 score tiles, p and ds through shared memory, one CTA per pair of tiles), block 64:
@@ -338,7 +565,6 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
 constexpr int BKV_THREADS = 384;                              // TMA, MMA, planner, (no work), 8 softmax warps
 constexpr int BKV_MAXG = 16;
 constexpr int BKV_DESCS = 2;                                  // steps that the planner is ahead
-constexpr int BKV_REGS_LOW = 88, BKV_REGS_HIGH = 208;         // a thread: 128 x 88 + 256 x 208 = 384 x 168
 template <int DK, int DV>
 struct DkvSmem {
     static constexpr int kv = 0;                              // k: DK/64 sub-tiles [128 keys][64], then v the same way
@@ -469,7 +695,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     auto release_step = [&]() { arrive(desc_empty + (n_step++ & (BKV_DESCS - 1)) * 8); };
 
     if (warp < 4) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(BKV_REGS_LOW));
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(BWD_REGS_LOW));
         if (warp == 0) {
             // ------------------------------------------------------------ TMA producer
             int ni = 0, pairs = 0;                                // steps with queries, pairs that have some
@@ -788,7 +1014,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             if (ok && open()) put(make_int4(0, BKV_STOP, 0, 0), make_int4(0, 0, 0, 0));
         }
     } else {
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(BKV_REGS_HIGH));
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(BWD_REGS_HIGH));
         // ------------------------------------------------------------ softmax: one key per thread and half, 64 queries each
         const int quad = warp & 3, half = (warp - 4) >> 2, u = quad >> 1, part = (quad & 1) * 2 + half;
         const uint32_t t_lane = tmem + ((uint32_t)(quad * 32) << 16);
@@ -1007,33 +1233,33 @@ static int launch_attn_bwd(const void* q, const void* k, const void* v, const vo
                            int HQ, int HKV, int HN, int nbs, float scale, int own_chunk, int compat, cudaStream_t st) {
     const int NT = (T + 63) / 64, NTq = (T + ATT_BM - 1) / ATT_BM;
     const int TN = (T + nbs - 1) / nbs;
-    const int smem = DqSmem<DK, DV>::total(NT);
-    if (smem > 227 * 1024) {
-        set_error("natsl_attn_bwd: T=%d needs %d B of shared memory (max %d)", T, smem, 227 * 1024);
+    if (NTq > 32767) {                                       // the dk, dv kernel keeps numbers of query tiles in 16 bits
+        set_error("natsl_attn_bwd: T=%d is too long (max %d)", T, 32767 * ATT_BM);
         return NATSL_ERR_TOO_LARGE;
     }
     auto k1 = attn_bwd_dq_kernel<DK, DV>;
     auto k2 = attn_bwd_dkdv_kernel<DK, DV>;
-    cudaError_t e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, DqSmem<DK, DV>::total);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, DkvSmem<DK, DV>::total);
     if (e != cudaSuccess) {
-        set_error("natsl_attn_bwd: cannot reserve %d B of shared memory (%s)", smem, cudaGetErrorString(e));
+        set_error("natsl_attn_bwd: cannot reserve %d B of shared memory (%s)", DkvSmem<DK, DV>::total, cudaGetErrorString(e));
         return NATSL_ERR_CUDA;
     }
-    CUtensorMap mq, mk, mv, mdo, mdk, mdv;
+    CUtensorMap mq, mk, mv, mdo, mdq, mdk, mdv;
     int* status = nullptr;
     int rc = encode_bthd_map(&mq, q, B, T, HQ, DK, 128, "natsl_attn_bwd(q)");
     if (rc == NATSL_OK) rc = encode_bthd_map(&mk, k, B, T, HKV, DK, 64, "natsl_attn_bwd(k)");
     if (rc == NATSL_OK) rc = encode_bthd_map(&mv, v, B, T, HKV, DV, 64, "natsl_attn_bwd(v)");
     if (rc == NATSL_OK) rc = encode_bthd_map(&mdo, d_o, B, T, HQ, DV, 128, "natsl_attn_bwd(do)");
+    if (rc == NATSL_OK) rc = encode_bthd_map(&mdq, dq, B, T, HQ, DK, 32, "natsl_attn_bwd(dq)");
     if (rc == NATSL_OK) rc = encode_bthd_map(&mdk, dk, B, T, HKV, DK, 32, "natsl_attn_bwd(dk)");
     if (rc == NATSL_OK) rc = encode_bthd_map(&mdv, dv, B, T, HKV, DV, 32, "natsl_attn_bwd(dv)");
     if (rc == NATSL_OK) rc = status_word_ptr(&status);
     if (rc != NATSL_OK) return rc;
     auto bf = [](const void* p) { return reinterpret_cast<const __nv_bfloat16*>(p); };
     const int own = own_chunk && !compat;
-    k1<<<dim3(NTq, HQ, B), TC_THREADS, smem, st>>>(mq, mk, mv, mdo, bf(o), bf(d_o), lse, types_i, reinterpret_cast<__nv_bfloat16*>(dq),
-                                                  delta, T, HQ, HKV, HN, TN, nbs, scale, own, status);
+    k1<<<NTq * HQ * B, BDQ_THREADS, DqSmem<DK, DV>::total, st>>>(mq, mk, mv, mdo, mdq, bf(q), bf(o), bf(d_o), lse, types_i, delta, T, HQ, HKV,
+                                                                 HN, TN, nbs, scale, own, HQ * B, status);
     rc = check_launch("natsl_attn_bwd (dq)");
     if (rc != NATSL_OK) return rc;
     const int per_head = (NT + 1) / 2, heads = HKV * B;      // pairs of key tiles

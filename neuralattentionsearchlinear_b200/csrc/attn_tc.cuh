@@ -5,9 +5,6 @@
 
 namespace natsl {
 
-constexpr int TC_THREADS = 320;             // dq: TMA producer, MMA issuer, 8 softmax warps
-constexpr uint32_t TC_TMEM_COLS = 256;      // dq: tensor-memory columns of a CTA (two CTAs per SM)
-
 __device__ __forceinline__ float ex2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

@@ -44,3 +44,23 @@ def test_softmax_backward_tiles(T, HQ, HKV, HN, DK, DV, nbs, p, own, compat):
     assert _lib.load().natsl_device_status() == 0
     again = _ops.attn_bwd(*c, o, lse, do.cuda(), tb, scale, own, reference_compat=compat)
     assert all(torch.equal(x, y) for x, y in zip(got, again))
+
+
+@pytest.mark.parametrize("B,T,HQ,HKV,DK,DV", [(3, 700, 12, 6, 128, 128), (5, 300, 14, 7, 64, 64)])
+def test_query_blocks_over_several_groups_of_heads(B, T, HQ, HKV, DK, DV):
+    """More blocks of 128 queries than SMs, more heads than the 32 whose blocks are interleaved: what a CTA takes over from the
+    grid, and the last group of heads, which is a smaller one."""
+    import neuralattentionsearchlinear_b200 as nat
+    from neuralattentionsearchlinear_b200 import _lib, _ops
+    gen = torch.Generator().manual_seed(T)
+    rnd = lambda *s: torch.randn(*s, generator=gen).bfloat16()
+    q, k, v, do = rnd(B, T, HQ, DK), rnd(B, T, HKV, DK), rnd(B, T, HKV, DV), rnd(B, T, HQ, DV)
+    types = otab.synth_types(B, -(-T // 64), HQ, 0.4, seed=T)
+    tb = nat.build_selection_tables(types.cuda(), T, 64)
+    c = [x.cuda() for x in (q, k, v)]
+    o, lse = _ops.attn_fwd(*c, tb, DK ** -0.5, True)
+    got = _ops.attn_bwd(*c, o, lse, do.cuda(), tb, DK ** -0.5, True)
+    ref = ograd.attn_grads(q.double(), k.double(), v.double(), types[..., 0], do.double(), nbs=64, scale=DK ** -0.5, own_chunk=True)
+    for x, name in zip(got, ("dq", "dk", "dv", "dnats")):     # (the bounds above)
+        close_scaled(x, ref[name], name, tol=2e-2 if name == "dq" else 1e-2, scale="max" if name == "dnats" else "auto")
+    assert _lib.load().natsl_device_status() == 0
