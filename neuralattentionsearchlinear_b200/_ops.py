@@ -17,7 +17,7 @@ USE_FUSED_WALK = True
 # form that holds state and operands to fp32 precision (natsl_gdn_split_*).
 GDN_HEAD_DIMS = {(64, 64), (64, 128), (128, 64), (128, 128), (128, 256), (192, 384)}
 # value dimension of the fused walk split over two CTAs (natsl_gdn_walk_fused_vsplit, T <= 8192): half an SM per CTA.
-# Off by default: measured alone it is no faster than the one-CTA walk (0.204 vs 0.189 ms at B=8, T=4096, H=16), and
+# Off by default: measured alone it is no faster than the one-CTA walk (0.204 vs 0.130 ms at B=8, T=4096, H=16), and
 # the kernels of the two branches do not overlap in practice (the block scheduler drains one grid before the next).
 WALK_VSPLIT = os.environ.get("NATSL_WALK_VSPLIT", "0") == "1"
 # chunk preparation on tcgen05 for K = V = 128 (natsl_gdn_chunk_prep_tc); "0" takes the mma.sync kernel there
