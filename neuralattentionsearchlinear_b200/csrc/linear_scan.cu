@@ -22,6 +22,11 @@
 namespace natsl {
 
 constexpr int SCAN_THREADS = 128;
+// (batch, head) pairs and tokens from which the gated delta rule's states at 128/128, block 64, come from gdn_states_tc.cu: one CTA per
+// pair there, four here, whose steps take longer only when they share SMs.  This kernel / that one (us): 32 pairs 37 / 40 at T = 2048, 49 / 55
+// and 109 / 109 at T = 4096 (25 and 90 % selected); 48 pairs 19 / 22 at T = 1000, 60 / 60 and 117 / 101 at T = 4096 (25 and 75 %); 64 pairs
+// 27 / 24 at T = 1000, 51 / 44 at T = 2048, 135 / 110 at T = 4096; 192 pairs of 256 tokens 21 / 18, 256 of 64 tokens 9.7 / 10.4.
+constexpr int STATES_TC_PAIRS = 64, STATES_TC_TOKENS = 256;
 
 template <int K, int BV, bool GDN>
 struct ScanSmem {
@@ -298,6 +303,10 @@ linear_scan_kernel(const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __r
     }
 }
 
+int gdn_states_tc(const void* k, const void* w, const void* u, const float* gcs, const float* k_rstd, const int32_t* types_i,
+                  const int32_t* indices, const int32_t* n_blocks, const float* h0, void* h, float* carry, int B, int T, int H, int HN,
+                  int decay, int trailing_quirk, cudaStream_t st);                // gdn_states_tc.cu
+
 template <int K, int BV, bool GDN>
 static int launch_scan(const void* k, const void* w, const void* u, const float* gcs, const float* krstd,
                        const int* types_i, const int* indices, const int* n_blocks, const float* h0, void* hout,
@@ -350,6 +359,9 @@ extern "C" int natsl_linear_fwd_h(int rule, const void* k, const void* w, const 
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
 #define NATSL_SCAN_ARGS k, w, u, gcs, k_rstd, types_i, indices, n_blocks, h0, h, carry, ht, B, T, H, HN, V, nbs, decay, quirk, st
     if (rule == NATSL_RULE_GDN) {
+        if (K == 128 && V == 128 && nbs == 64 && h && !ht && k_rstd && T >= STATES_TC_TOKENS && T <= 65536 && B * H >= STATES_TC_PAIRS &&
+            (long)B * ((T + 63) / 64) * H <= INT32_MAX && aligned_to(16, k, w, u, h))
+            return gdn_states_tc(k, w, u, gcs, k_rstd, types_i, indices, n_blocks, h0, h, carry, B, T, H, HN, decay, quirk, st);
         if (K == 64) return launch_scan<64, 32, true>(NATSL_SCAN_ARGS);
         if (K == 128) return launch_scan<128, 32, true>(NATSL_SCAN_ARGS);
     } else {
