@@ -1205,12 +1205,12 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             release_step();
             ++ni;
             if (!(f & BKV_LAST)) continue;
-            flush(d.z, f);
             finish((f & (BKV_ANY0 << u)) != 0, true);
             if (ok) ok = warp_wait(bar_acc, pairs & 1);       // (a phase passes by every warp: some have blocks of dv only)
             if (!ok) break;
             ++pairs;
-            release_acc();
+            flush(d.z, f);                                    // behind the products of the pair, which warp 4 has joined in: it has
+            release_acc();                                    // written the sums of the pair before, also if this one is a single step
             if (warp == 4) {                                  // in front of its part in the next step, behind which others flush again
                 if (f & BKV_SUMS) ok = warp_wait(bar_acc_free, pairs & 1);
                 if (!ok) break;

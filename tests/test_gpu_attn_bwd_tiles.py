@@ -64,3 +64,24 @@ def test_query_blocks_over_several_groups_of_heads(B, T, HQ, HKV, DK, DV):
     for x, name in zip(got, ("dq", "dk", "dv", "dnats")):     # (the bounds above)
         close_scaled(x, ref[name], name, tol=2e-2 if name == "dq" else 1e-2, scale="max" if name == "dnats" else "auto")
     assert _lib.load().natsl_device_status() == 0
+
+
+@pytest.mark.parametrize("B,T,H,DK,DV,p", [(8, 128, 32, 64, 64, 1.0), (16, 256, 16, 128, 64, 0.5), (4, 1000, 16, 128, 64, 0.5)])
+def test_sums_of_short_pairs_repeat(B, T, H, DK, DV, p):
+    """Many pairs of key tiles with one or two steps each, one behind the other on an SM: the sums of a pair are not touched by the
+    next one.  Bit for bit the same in every run, and the oracle's."""
+    import neuralattentionsearchlinear_b200 as nat
+    from neuralattentionsearchlinear_b200 import _lib, _ops
+    gen = torch.Generator().manual_seed(T + H)
+    rnd = lambda *s: torch.randn(*s, generator=gen).bfloat16()
+    q, k, v, do = rnd(B, T, H, DK), rnd(B, T, H, DK), rnd(B, T, H, DV), rnd(B, T, H, DV)
+    types = otab.synth_types(B, -(-T // 64), H, p, seed=T)
+    tb = nat.build_selection_tables(types.cuda(), T, 64)
+    c = [x.cuda() for x in (q, k, v)]
+    o, lse = _ops.attn_fwd(*c, tb, DK ** -0.5, True)
+    runs = [_ops.attn_bwd(*c, o, lse, do.cuda(), tb, DK ** -0.5, True) for _ in range(30)]
+    assert all(torch.equal(x, y) for r in runs[1:] for x, y in zip(runs[0], r))
+    ref = ograd.attn_grads(q[:1].double(), k[:1].double(), v[:1].double(), types[:1, ..., 0], do[:1].double(), nbs=64, scale=DK ** -0.5,
+                           own_chunk=True)
+    close_scaled(runs[0][3][:1], ref["dnats"], "dnats", tol=1e-2, scale="max")                # (the bound above)
+    assert _lib.load().natsl_device_status() == 0
