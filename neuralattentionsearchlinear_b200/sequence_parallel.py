@@ -228,7 +228,7 @@ def nats_mixed_attn_mamba_sp(q_attn, k_attn, v_attn, q_lattn, k_lattn, v_lattn, 
     with a single rank, where only the sub-segment split of the linear branch remains).
     All tensors hold this rank's segment(s) along the time axis ([B, T_local, ...]; block types
     [B, TN_local, HN, 2]); with ``layout='zigzag'`` T_local covers the rank's two equally long segments one after
-    the other (see ``segment_ids``).  ``linear_splits``: sub-segments per segment in the linear branch (default:
+    the other (see ``segment_ids``; a single rank holds the whole sequence).  ``linear_splits``: sub-segments per segment in the linear branch (default:
     about 1024 tokens each, on one rank what ``one_rank_splits`` says).  ``kv_capacity`` = (softmax-selected blocks per head, selected (block, head) pairs) a
     segment may have at most: sizes the key/value gather without reading the counts back to the host (no host
     synchronisation, so the call can be captured in a CUDA graph); if a segment exceeds it the device status
@@ -256,8 +256,11 @@ def nats_mixed_attn_mamba_sp(q_attn, k_attn, v_attn, q_lattn, k_lattn, v_lattn, 
     if n_seg > 1 or not last_holder:
         if T_loc % (n_seg * max(nbs, 128)):
             raise ValueError("every segment but the last of the sequence must be a multiple of the block size (and of 128)")
+    if world == 1 and n_seg > 1:        # all segments of the sequence, in order: nothing lies between them, so they are one
+        linear_splits = int(linear_splits) * n_seg if linear_splits else linear_splits
+        layout, seg, n_seg, n_glob = 'contiguous', [0], 1, 1
     L = T_loc // n_seg
-    s_lin = int(linear_splits) if linear_splits else one_rank_splits(L, nbs, n_seg * B * H) if world == 1 else pick_linear_splits(L, nbs)
+    s_lin = int(linear_splits) if linear_splits else one_rank_splits(L, nbs, B * H) if world == 1 else pick_linear_splits(L, nbs)
     if s_lin > 1 and L % (s_lin * max(nbs, 128)):
         raise ValueError(f"linear_splits={s_lin} does not cut a {L}-token segment into multiples of the block size")
     n_sub = n_seg * s_lin

@@ -172,6 +172,27 @@ def test_single_rank_sub_segment_split_matches_oracle():
         assert (ht - s_ref).abs().max() < 1e-9
 
 
+@pytest.mark.parametrize("splits", [None, 1, 2])
+@pytest.mark.parametrize("T", [1024, 2048])
+def test_zigzag_on_a_single_rank_is_the_whole_sequence(T, splits):
+    """One rank holds both segments of the zigzag layout, one behind the other: the later one sees the earlier one."""
+    from neuralattentionsearchlinear_b200.sequence_parallel import nats_mixed_attn_mamba_sp
+    from tests.sp_helpers import OracleSegmentOps
+    B, H, K, V, nbs, seed = 2, 2, 16, 8, 128, 13
+    q, k, v, g, types = _inputs(B, T, H, K, V, nbs, seed)
+    types[:, -1] = 1
+    call = lambda n, layout: nats_mixed_attn_mamba_sp(*(x[:, :n] for x in (q, k, v, q, k, v, g)), types, nats_block_size=nbs,
+                                                      layout=layout, linear_splits=splits, backend=OracleSegmentOps())
+    o_l, o_a, ht = call(T, "zigzag")
+    o_ref, s_ref = ogdn.linear_recurrent(q, k, v, g, None, types[..., 1], nbs=nbs, scale=1.0, decay=True, use_l2norm=False, rule="mamba")
+    oa_ref, _ = oattn.attn_sdpa(q, k, v, oattn.attn_mask(types[..., 0], T, nbs, H))
+    assert (o_l - o_ref).abs().max() < 1e-9
+    assert (o_a - oa_ref).abs().max() < 1e-9
+    assert (ht - s_ref).abs().max() < 1e-9
+    with pytest.raises(ValueError):                      # two segments of whole blocks, as on several ranks
+        call(T - 100, "zigzag")
+
+
 # ------------------------------------------------------------------------------- failure on one rank (host side)
 class _FailingOps:
     """Wraps the per-rank compute; on ``bad_rank`` the linear branch raises (or stalls for ``delay`` seconds) right before
