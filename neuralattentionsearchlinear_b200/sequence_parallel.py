@@ -188,15 +188,18 @@ def pick_linear_splits(L: int, nbs: int, target_tokens: int = 1024) -> int:
     return best
 
 
-@functools.lru_cache(maxsize=None)
+@functools.lru_cache(maxsize=1024)
 def one_rank_splits(L: int, nbs: int, units: int) -> int:
-    """The same for one rank, which walks ``units`` = batch x heads sequences and has no exchange to hide: the number of
-    sub-segments with the least time for both passes, from what the walk takes on the device: 1.3 us a chunk and 8 us a CTA, waves
-    of 148 CTAs, a first pass of 0.6 of the second, 35 us of folding around them; an uncut sequence needs one pass.  Mostly that is
-    one wave of CTAs.  Op captured in a graph (us), sub-segments of 1024 tokens against it: T = 4096 H = 16 86 / 76, T = 8192
-    H = 32 185 / 174, T = 16384 H = 16 207 / 192, H = 32 377 / 324, T = 32768 H = 32 965 / 871, T = 65536 H = 32 3069 / 3006 (2 % of
-    the blocks softmax instead of 8 %: 1411 / 1170).  An uncut sequence beside a long attention would save the first pass (T = 65536
-    H = 32, 10 %: 3401 / 3518) but is what the op waits for where few blocks are selected (2 %: 1597 / 1170)."""
+    """The same for one rank, which walks ``units`` = batch x heads sequences and has no exchange to hide, at the fused walk's head
+    dims (K = 128, V = 64): the number of sub-segments with the least time for both passes, from what that walk takes on the device:
+    1.3 us a chunk and 8 us a CTA, waves of 148 CTAs, a first pass of 0.6 of the second, 35 us of folding around them; an uncut
+    sequence needs one pass.  Mostly that is one wave of CTAs.  Op captured in a graph (us), sub-segments of 1024 tokens against it:
+    T = 4096 H = 16 86 / 76, T = 8192 H = 32 185 / 174, T = 16384 H = 16 207 / 192, H = 32 377 / 324, T = 32768 H = 32 965 / 871,
+    T = 65536 H = 32 3069 / 3006 (2 % of the blocks softmax instead of 8 %: 1411 / 1170).  An uncut sequence beside a long attention
+    would save the first pass (T = 65536 H = 32, 10 %: 3401 / 3518) but is what the op waits for where few blocks are selected (2 %:
+    1597 / 1170).  At other head dims the recurrence is a scan of 32 value columns per CTA, several to an SM, which wants more and
+    shorter sub-segments (2 % softmax, 1024 tokens against this rule: 64/64, T = 16384 H = 32 341 / 418, T = 2048 H = 32 83 / 101;
+    128/128, T = 16384 H = 16 417 / 454): they keep ``pick_linear_splits``."""
     unit = max(nbs, 128)
     if L % unit:
         return 1
@@ -229,7 +232,7 @@ def nats_mixed_attn_mamba_sp(q_attn, k_attn, v_attn, q_lattn, k_lattn, v_lattn, 
     All tensors hold this rank's segment(s) along the time axis ([B, T_local, ...]; block types
     [B, TN_local, HN, 2]); with ``layout='zigzag'`` T_local covers the rank's two equally long segments one after
     the other (see ``segment_ids``; a single rank holds the whole sequence).  ``linear_splits``: sub-segments per segment in the linear branch (default:
-    about 1024 tokens each, on one rank what ``one_rank_splits`` says).  ``kv_capacity`` = (softmax-selected blocks per head, selected (block, head) pairs) a
+    about 1024 tokens each, on one rank at the fused walk's head dims what ``one_rank_splits`` says).  ``kv_capacity`` = (softmax-selected blocks per head, selected (block, head) pairs) a
     segment may have at most: sizes the key/value gather without reading the counts back to the host (no host
     synchronisation, so the call can be captured in a CUDA graph); if a segment exceeds it the device status
     (``natsl_device_status``) reads 3 and the outputs are invalid.  Without it the exact maxima are read back (one
@@ -260,7 +263,12 @@ def nats_mixed_attn_mamba_sp(q_attn, k_attn, v_attn, q_lattn, k_lattn, v_lattn, 
         linear_splits = int(linear_splits) * n_seg if linear_splits else linear_splits
         layout, seg, n_seg, n_glob = 'contiguous', [0], 1, 1
     L = T_loc // n_seg
-    s_lin = int(linear_splits) if linear_splits else one_rank_splits(L, nbs, B * H) if world == 1 else pick_linear_splits(L, nbs)
+    if linear_splits:
+        s_lin = int(linear_splits)
+    elif world == 1 and K == 128 and v_lattn.shape[3] == 64 and _ops.USE_MAMBA_WALK:       # head dims of the fused walk
+        s_lin = one_rank_splits(L, nbs, B * H)
+    else:
+        s_lin = pick_linear_splits(L, nbs)
     if s_lin > 1 and L % (s_lin * max(nbs, 128)):
         raise ValueError(f"linear_splits={s_lin} does not cut a {L}-token segment into multiples of the block size")
     n_sub = n_seg * s_lin

@@ -134,6 +134,28 @@ def test_one_rank_splits():
     assert one_rank_splits(65536, 64, 148) == 1 and one_rank_splits(1024, 64, 32) == 1
 
 
+@pytest.mark.parametrize("K,V,rule", [(128, 64, "one_rank_splits"), (64, 64, "pick_linear_splits"), (128, 128, "pick_linear_splits"),
+                                      (64, 128, "pick_linear_splits")])
+def test_cut_on_one_rank_follows_the_kernel_that_walks(K, V, rule):
+    """The cost model of one rank is the fused walk's: head dims that take the scan are cut as on several ranks."""
+    from neuralattentionsearchlinear_b200 import sequence_parallel as sp
+    from tests.sp_helpers import OracleSegmentOps
+    B, T, H, nbs = 1, 2048, 32, 64
+    assert sp.one_rank_splits(T, nbs, B * H) != sp.pick_linear_splits(T, nbs)
+
+    class Cut(Exception):
+        pass
+
+    class Ops(OracleSegmentOps):
+        def linear(self, q, *args):
+            raise Cut(q.shape[0] // B)
+
+    q, v, g = torch.zeros(B, T, H, K), torch.zeros(B, T, H, V), torch.zeros(B, T, H)
+    with pytest.raises(Cut) as e:
+        sp.nats_mixed_attn_mamba_sp(q, q, v, q, q, v, g, torch.ones(B, T // nbs, H, 2), nats_block_size=nbs, backend=Ops())
+    assert e.value.args[0] == (sp.one_rank_splits(T, nbs, B * H) if rule == "one_rank_splits" else sp.pick_linear_splits(T, nbs))
+
+
 def test_pick_linear_splits():
     from neuralattentionsearchlinear_b200.sequence_parallel import pick_linear_splits
     assert pick_linear_splits(65536, 256) == 64
