@@ -205,7 +205,7 @@ def one_rank_splits(L: int, nbs: int, units: int) -> int:
         return 1
     cost = lambda s: (1.6 if s > 1 else 1.0) * -(-s * units // 148) * (L // s / 64 * 1.3 + 8) + (30 + 0.6 * s if s > 1 else 0)
     cuts = [s for s in range(1, L // unit + 1) if L % (s * unit) == 0 and L // s <= 65536]      # the walk's longest sequence
-    return min(cuts, key=cost)
+    return min(cuts, key=cost) if cuts else pick_linear_splits(L, nbs)        # (longer blocks are the scan's)
 
 
 def _split(x, B, n):                    # [B, n*m, ...] -> [n*B, m, ...]   (segment-major batch)

@@ -134,6 +134,11 @@ def test_one_rank_splits():
     assert one_rank_splits(65536, 64, 148) == 1 and one_rank_splits(1024, 64, 32) == 1
 
 
+def test_one_rank_splits_of_blocks_longer_than_the_walk():
+    from neuralattentionsearchlinear_b200.sequence_parallel import one_rank_splits
+    assert one_rank_splits(131072, 131072, 4) == 1 and one_rank_splits(262144, 131072, 4) == 2
+
+
 @pytest.mark.parametrize("K,V,rule", [(128, 64, "one_rank_splits"), (64, 64, "pick_linear_splits"), (128, 128, "pick_linear_splits"),
                                       (64, 128, "pick_linear_splits")])
 def test_cut_on_one_rank_follows_the_kernel_that_walks(K, V, rule):
