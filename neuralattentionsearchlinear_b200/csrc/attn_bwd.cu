@@ -129,6 +129,21 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         mbar_init(bar_clc, 1);
         mbar_fence_init();
     }
+    // the planner's block: first query, query head, batch; its first 32 flags, under way while the rest is set up
+    int4 where = make_int4(0, 0, 0, 0);
+    bool sel_n = false;
+    auto place = [&](int block) {
+        const int hbase = block / (BDQ_HEADS * NTq) * BDQ_HEADS, hcount = min(BDQ_HEADS, heads - hbase);
+        const int within = block - hbase * NTq, item = within / hcount, head = hbase + (within - item * hcount);
+        where = make_int4((NTq - 1 - item) * ATT_BM, head % HQ, head / HQ, 0);
+    };
+    auto selected = [&](int kt) -> bool {                     // key tile kt's block, for the queries there (column 0)
+        return kt < min((where.x + ATT_BM + 63) / 64, NT) && types_i[(((long)where.z * TN + kt / cpb) * HN + where.y / (HQ / HN)) * 2] != 0;
+    };
+    if (warp == 2) {
+        place(blockIdx.x);
+        sel_n = selected(lane);
+    }
     if (warp == 1) tmem_alloc(smem_u32(tmem_slot), 512);
     tc_fence_before();
     __syncthreads();
@@ -290,8 +305,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             }
         } else if (warp == 2) {
             // -------------------------------------------------------- planner: blocks and their steps
-            int n = 0, asked = 0, answers = 0;                // steps, take-over requests
-            int block = blockIdx.x;
+            int n = 0, answers = 0, block;                    // steps, take-over requests
             auto put = [&](int4 x, int4 y) {
                 const int slot = n & (BDQ_STEPS - 1);
                 if (n >= BDQ_STEPS) ok = warp_wait(desc_empty + slot * 8, (n / BDQ_STEPS - 1) & 1);
@@ -311,15 +325,9 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                     request_block(sbase + L::clc, bar_clc);
                 }
                 __syncwarp();
-                ++asked;
-                const int hbase = block / (BDQ_HEADS * NTq) * BDQ_HEADS, hcount = min(BDQ_HEADS, heads - hbase);
-                const int within = block - hbase * NTq, item = within / hcount, head = hbase + within % hcount;
-                const int hq = head % HQ, b = head / HQ, q0 = (NTq - 1 - item) * ATT_BM;
-                const int* selp = types_i + ((long)b * TN * HN + hq / (HQ / HN)) * 2;              // column 0
-                const long tstride = (long)HN * 2;
+                const int q0 = where.x, hq = where.y, b = where.z;
                 const int span0 = (q0 / nbs) * cpb;           // first key tile of the own span
                 const int n_cand = min((q0 + ATT_BM + 63) / 64, NT);
-                const int4 where = make_int4(q0, hq, b, 0);
                 for (int i = n > 0 ? lane : 128; i < 128; i += 32) {       // its rows into L2 while the block before is worked on
                     const long t = ((long)b * T + min(q0 + i, T - 1)) * HQ + hq;
 #pragma unroll
@@ -333,8 +341,6 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 // visible key tiles in ascending order, two to a step: those of selected blocks in front of the own span, then the
                 // own span.  A step is announced once it is known whether another follows.
                 int held0 = -1, held1 = -1, flags = BDQ_FIRST;
-                auto selected = [&](int kt) -> bool { return kt < n_cand && selp[(long)(kt / cpb) * tstride] != 0; };
-                bool sel_n = selected(lane);
 #pragma unroll 1
                 for (int base = 0; ok && base < n_cand; base += 32) {
                     const bool sel = sel_n;
@@ -365,6 +371,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 ok = ok && came;
                 if (!ok || !taken_block(sbase + L::clc, block)) break;
                 __syncwarp();
+                place(block);
+                sel_n = selected(lane);
             }
             if (ok) put(make_int4(0, BDQ_STOP, -1, 0), make_int4(0, 0, 0, 0));
         }
