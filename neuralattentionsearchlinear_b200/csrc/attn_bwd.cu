@@ -603,6 +603,14 @@ enum : int {
 // Heads whose CTAs are interleaved, heaviest first: the last CTAs to start are then light ones, and q and do of that many
 // heads (2 MB each at 4096 x 128) stay in L2 for the CTAs of a head that run at the same time.
 constexpr int BKV_HEADS = 32;
+// A grid of no more blocks than the 148 SMs takes the form SMALL, whose blocks are half as long: a block's pair of selected tiles and
+// what is unselected of its neighbours are blocks of their own, which in one block would be one behind the other while SMs are idle
+// (us, one block for both / halves: 16 query heads over one, T = 100 64/64 75 / 43, T = 256 76 / 43; 12 over 6, B = 2, T = 100
+// 128/128 17.5 / 12.4; 4 heads, B = 2, T = 256 12.6 / 9.5).  Where the halves fit the SMs at once nothing is taken over; otherwise they are
+// taken over like the others (B = 4, T = 256, H = 16 13.1 / 12.7; a CTA for each of the 256 halves 16.1).  Blocks of larger grids stay
+// whole (16 heads, B = 16, T = 100 64/64 18.9, halves 21.8), in a form of their own: its code is what it was, and these kernels
+// lose 5 % to the way that code lies in the instruction cache.  A sequence of one key tile has nothing to halve.
+constexpr int BKV_SMALL = 148;
 
 // Four K-steps, A from tensor memory, results added in the lanes whose bit is not set: m01 for lanes 0-63, m23 for lanes 64-127.
 template <int STEP_B>
@@ -622,14 +630,14 @@ __device__ __forceinline__ void umma_ts_x4_lanes(uint32_t d_tmem, uint32_t a_tme
         : "memory");
 }
 
-template <int DK, int DV>
+template <int DK, int DV, bool SMALL>
 __global__ void __launch_bounds__(BKV_THREADS, 1)
 attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                      const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
                      const __grid_constant__ CUtensorMap map_dk, const __grid_constant__ CUtensorMap map_dv,
                      const float* __restrict__ lse, const float* __restrict__ delta, const int* __restrict__ types_i,
                      float* __restrict__ dnats_part, int T, int HQ, int HKV, int HN, int TN, int nbs, float scale, int own, int heads,
-                     int ctas_per_head, int* status) {
+                     int ctas_per_head, int halves, int* status) {
     using L = DkvSmem<DK, DV>;
     // TMEM: scores [128 keys][128 queries], then p over each half's first columns; do.v, then ds; dv; dk
     constexpr uint32_t C_S = 0, C_DP = 128, C_DV = 256, C_DK = 384;
@@ -859,6 +867,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             // ------------------------------------------------------------ planner: blocks, their steps, lse and delta of the queries
             int n = 0, asked = 0, answers = 0;                    // steps, take-over requests
             int block = blockIdx.x;
+            const bool persist = !SMALL || gridDim.x > BKV_SMALL;
             auto open = [&]() {
                 if (n >= BKV_DESCS) ok = warp_wait(desc_empty + (n & (BKV_DESCS - 1)) * 8, (n / BKV_DESCS - 1) & 1);
                 return ok;
@@ -885,7 +894,9 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             while (ok) {
                 // Block `item` of a head: the item-th pair of the tiles whose block some head of the group selected, in their order
                 // (neighbours see nearly the same queries), then what is unselected of tiles 2 item and 2 item + 1, which only
-                // their own blocks' queries see.
+                // their own blocks' queries see; in halves, the first `halves` blocks are the pairs alone, the others the rest.
+                const bool rest_only = SMALL && halves && block >= halves;
+                if (rest_only) block -= halves;
                 const int hbase = block / (BKV_HEADS * ctas_per_head) * BKV_HEADS, hcount = min(BKV_HEADS, heads - hbase);
                 const int within = block - hbase * ctas_per_head;
                 const int item = within / hcount, head = hbase + within % hcount;
@@ -915,10 +926,10 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
 #pragma unroll
                 for (int i = 0; i < 2; ++i)
                     if (!((mine >> i) & 1) && 2 * item + i < NT) rest[i] = 2 * item + i;
-                bool requested = chosen[0] < 0;                   // a step or none: ask for the next block at once
-                if (requested) {
-                    request();
-                } else {
+                if (rest_only) chosen[0] = -1;
+                bool requested = !persist || chosen[0] < 0;       // a step or none: ask for the next block at once
+                if (persist && requested) request();
+                if (chosen[0] >= 0) {
                     // last query tile of every (tile, head): the sequence's if the head selected the block, else the own block's
                     __syncwarp();
 #pragma unroll 1
@@ -936,7 +947,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                     __syncwarp();
                 }
 #pragma unroll 1
-                for (int pass = chosen[0] < 0; ok && pass < 2; ++pass) {
+                for (int pass = chosen[0] < 0; ok && pass < (SMALL && halves && !rest_only ? 1 : 2); ++pass) {
                     const bool sums = pass == 0;
                     const int t[2] = {sums ? chosen[0] : rest[0], sums ? chosen[1] : rest[1]};
                     if (t[0] < 0 && t[1] < 0) continue;
@@ -1005,11 +1016,12 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                     if (ok) announce(BKV_LAST);
                     // the pair's last steps are under way: early enough to work out the next block, late enough to leave it to an SM
                     // that is free earlier
-                    if (ok && sums) {
+                    if (persist && ok && sums) {
                         request();
                         requested = true;
                     }
                 }
+                if (!persist) break;
                 if (ok && !requested) request();                  // (the chosen pair had no step)
                 if (asked > answers) {                            // (also after a failed wait: the answer is on its way)
                     const bool came = warp_wait(bar_clc, answers & 1);
@@ -1246,7 +1258,10 @@ static int launch_attn_bwd(const void* q, const void* k, const void* v, const vo
         return NATSL_ERR_TOO_LARGE;
     }
     auto k1 = attn_bwd_dq_kernel<DK, DV>;
-    auto k2 = attn_bwd_dkdv_kernel<DK, DV>;
+    const int per_head = (NT + 1) / 2, heads = HKV * B, blocks = per_head * heads;      // pairs of key tiles
+    const bool few = blocks <= BKV_SMALL;
+    const int halves = few && NT > 1 ? blocks : 0;
+    auto k2 = few ? attn_bwd_dkdv_kernel<DK, DV, true> : attn_bwd_dkdv_kernel<DK, DV, false>;
     cudaError_t e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, DqSmem<DK, DV>::total);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, DkvSmem<DK, DV>::total);
     if (e != cudaSuccess) {
@@ -1270,9 +1285,8 @@ static int launch_attn_bwd(const void* q, const void* k, const void* v, const vo
                                                                  HN, TN, nbs, scale, own, HQ * B, status);
     rc = check_launch("natsl_attn_bwd (dq)");
     if (rc != NATSL_OK) return rc;
-    const int per_head = (NT + 1) / 2, heads = HKV * B;      // pairs of key tiles
-    k2<<<per_head * heads, BKV_THREADS, DkvSmem<DK, DV>::total, st>>>(mq, mk, mv, mdo, mdk, mdv, lse, delta, types_i, dnats_part, T, HQ,
-                                                                      HKV, HN, TN, nbs, scale, own, heads, per_head, status);
+    k2<<<blocks + halves, BKV_THREADS, DkvSmem<DK, DV>::total, st>>>(mq, mk, mv, mdo, mdk, mdv, lse, delta, types_i, dnats_part, T, HQ,
+                                                                     HKV, HN, TN, nbs, scale, own, heads, per_head, halves, status);
     return check_launch("natsl_attn_bwd (dk, dv)");
 }
 
