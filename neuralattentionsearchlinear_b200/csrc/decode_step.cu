@@ -404,44 +404,36 @@ __device__ void core_attention(const CoreArgs& c, int idx, float* sm) {
     const long tstride = (long)a.HN * 2;
     const long tbase = ((long)b * a.n_done * a.HN + hn) * 2;
     auto chosen = [&](int u, int end) -> bool { return u < end && ldw(a.types, a.types_f32, tbase + (long)(u / upb) * tstride) > 0.5f; };
-    // Which units are this split's.  Up to 128 (8192 tokens) every split reads all selection bits and takes every S-th selected unit,
-    // then every S-th unit of the current block: equal shares, where a range of its own holds none of them or all (4 rows of 32
-    // heads, 16 units over 5 splits: the last CTA had twice the mean).  Beyond, a range of its own, 32 units at a time.
-    constexpr int FEW = 4;
-    const bool few = n_units <= FEW * 32;
-    unsigned mask = 0, more[FEW - 1] = {0, 0, 0};       // units base .. base + 31 that are left, and the words behind
+    // Which units are this split's.  Up to 32 (2048 tokens), and up to 64 where a range would be less than four, every split reads all
+    // selection bits and takes every S-th selected unit, then every S-th unit of the current block: equal shares, where a range of
+    // its own holds none of them or all (4 rows of 32 heads, 16 units over 5 splits: the last CTA had twice the mean).  Otherwise, a
+    // range of its own, 32 units at a time, whose shares even out (whole tokens, ranges / shares, us: 16 heads of 64, 1 row,
+    // 2000 tokens 16.1 / 15.2, 3300 tokens 16.8 / 16.3, 8 rows, 2600 tokens 23.8 / 25.2, 4 rows, 5500 tokens 23.6 / 25.4, 8000
+    // tokens 28.5 / 31.1).
+    const bool few = n_units <= 32 || (n_units <= 64 && n_units < 4 * c.S);
+    unsigned mask = 0, more = 0;                        // units base .. base + 31 that are left; of few, the ones behind
     int base = 0, end = 0, own_unit = last ? 0 : 1 << 20, own_step = 1;
     if (few) {
-        bool sel[FEW];
-#pragma unroll
-        for (int i = 0; i < FEW; ++i) sel[i] = chosen(i * 32 + lane, n_units);
-        int rank = 0;                                   // selected units so far, modulo S
-#pragma unroll
-        for (int i = 0; i < FEW; ++i) {
-            const unsigned all = __ballot_sync(0xffffffffu, sel[i]);
-            const unsigned m = __ballot_sync(0xffffffffu, sel[i] && (rank + __popc(all & ((1u << lane) - 1))) % c.S == s);
-            rank = (rank + __popc(all)) % c.S;
-            if (i == 0) mask = m;
-            else more[i - 1] = m;
-        }
+        const unsigned all = __ballot_sync(0xffffffffu, chosen(lane, n_units)), behind = __ballot_sync(0xffffffffu, chosen(32 + lane, n_units));
+        const unsigned below = (1u << lane) - 1;
+        mask = __ballot_sync(0xffffffffu, (all >> lane & 1) && __popc(all & below) % c.S == s);
+        more = __ballot_sync(0xffffffffu, (behind >> lane & 1) && (__popc(all) + __popc(behind & below)) % c.S == s);
+        const int rank = (__popc(all) + __popc(behind)) % c.S;             // of the units of the current block
         own_unit = s - rank + (s < rank ? c.S : 0);
         own_step = c.S;
-        end = n_units;
     } else {
         end = (int)((long)n_units * (s + 1) / c.S);
         base = (int)((long)n_units * s / c.S) - 32;
     }
     auto next = [&](int& key0) -> int {                 // keys of the warp's next step, 0 at the end
+        if (mask == 0 && more) {
+            mask = more;
+            more = 0;
+            base = 32;
+        }
         while (mask == 0 && base + 32 < end) {
             base += 32;
-            if (few) {
-                mask = more[0];
-#pragma unroll
-                for (int i = 0; i + 2 < FEW; ++i) more[i] = more[i + 1];
-                more[FEW - 2] = 0;
-            } else {
-                mask = __ballot_sync(0xffffffffu, chosen(base + lane, end));
-            }
+            mask = __ballot_sync(0xffffffffu, chosen(base + lane, end));
         }
         if (mask) {
             key0 = (base + __ffs(mask) - 1) * 64 + warp * 16;

@@ -89,10 +89,14 @@ def test_token_kernel_matches_the_general_path(make, args, B, T0):
 @pytest.mark.parametrize("make,args,B,T0", [
     (_gdn, dict(hidden=256, heads=4, head_dim=64, expand_v=1, attn_heads=4), 1, 8200),
     (_mamba, dict(hidden=256, heads=4, head_dim=128, expand_v=0.5, attn_heads=4, nats_block_size=256), 2, 1270),
+    (_gdn, dict(hidden=256, heads=2, head_dim=128, expand_v=1, attn_heads=2), 3, 2090),
+    (_gdn, dict(hidden=256, heads=16, head_dim=64, expand_v=1, attn_heads=16), 3, 3300),
+    (_mamba, dict(hidden=256, heads=4, head_dim=128, expand_v=0.5, attn_heads=4, nats_block_size=128), 1, 4160),
+    (_gdn, dict(hidden=256, heads=2, head_dim=128, expand_v=1, attn_heads=2), 1, 8230),
 ])
 def test_token_kernel_over_many_units(make, args, B, T0):
-    """Splits that take every S-th selected unit and unit of the current block (up to 128 units), and ranges of units (beyond);
-    the tokens cross the line, and the end of a block of several units."""
+    """Splits that take every S-th selected unit and unit of the current block (up to 32 units, and up to 64 over many splits),
+    and ranges of units (beyond); the tokens cross the lines, and the end of a block of several units."""
     test_token_kernel_matches_the_general_path(make, args, B, T0)
 
 
