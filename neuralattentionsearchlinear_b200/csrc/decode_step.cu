@@ -364,12 +364,13 @@ __device__ __forceinline__ void copy_first(uint32_t dst, const void* src, uint64
     asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "l"(policy) : "memory");
 }
 
-// Ring of a warp of the attention: steps of 16 keys; three of them where four CTAs then still share an SM, else two.
-template <int DK, int DV> struct Ring {
-    static constexpr int step = 16 * (DK + DV) * 2, D = DK + DV == 128 ? 3 : 2, bytes = 4 * D * step;
+// Ring of a warp of the attention: steps of 16 keys; three of them where four CTAs then still share an SM, else two (at 128/128
+// three CTAs), or one (launch_core).
+template <int DK, int DV, bool DEEP> struct Ring {
+    static constexpr int step = 16 * (DK + DV) * 2, D = !DEEP ? 1 : DK + DV == 128 ? 3 : 2, bytes = 4 * D * step;
 };
 
-template <int DK, int DV>
+template <int DK, int DV, bool DEEP>
 __device__ void core_attention(const CoreArgs& c, int idx, float* sm) {
     const Args& a = c.a;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -391,7 +392,7 @@ __device__ void core_attention(const CoreArgs& c, int idx, float* sm) {
     // then of the current block.  Keys and values come through the warp's own ring in shared memory, D steps deep: the first D are
     // on their way before the wait for the projections, and a split of few units is no chain of loads (one step ahead in
     // registers, 8 keys at head dims 128, it was: 4 rows of 32 heads, 1030 tokens: attention 14.5 us behind the wait).
-    using R = Ring<DK, DV>;
+    using R = Ring<DK, DV, DEEP>;
     constexpr int D = R::D, KS = 16, NK = KS / KG, NV = KS / VG;
     static_assert(LK >= NK && NV >= 1, "lanes per row");
     extern __shared__ __align__(16) unsigned char ring_all[];
@@ -675,7 +676,7 @@ __device__ void core_mix_logits(const CoreArgs& c, int idx, float* sm) {
     }
 }
 
-template <int DK, int DV>
+template <int DK, int DV, bool DEEP>
 __global__ void __launch_bounds__(DS_THREADS, 4) decode_core_kernel(const CoreArgs c) {
     __shared__ __align__(16) float sm[2 * DS_MAXK + 64 + 8 + 2 * DS_THREADS * 4];
     static_assert(2 * DK + DV + 16 + 4 * DV <= 2 * DS_MAXK + 64 + 8 + 2 * DS_THREADS * 4, "attention scratch");
@@ -684,7 +685,7 @@ __global__ void __launch_bounds__(DS_THREADS, 4) decode_core_kernel(const CoreAr
     // tokens of 32 rows, 2048 tokens, 47.1 -> 49.8 us, 16 rows of 128 / 128 61 -> 65 us; the recurrence first: 50.8 and 65 us.)
     const int idx = blockIdx.x;
     if (idx < c.n_mix) core_mix_logits(c, idx, sm);
-    else if (idx < c.n_mix + c.n_attn) core_attention<DK, DV>(c, idx - c.n_mix, sm);
+    else if (idx < c.n_mix + c.n_attn) core_attention<DK, DV, DEEP>(c, idx - c.n_mix, sm);
     else if (c.vs == 64) core_recurrence<64>(c, idx - c.n_mix - c.n_attn, sm);
     else core_recurrence<32>(c, idx - c.n_mix - c.n_attn, sm);
 }
@@ -834,10 +835,22 @@ cudaError_t launch_pdl(void (*kern)(const Arg), unsigned grid, unsigned block, c
 
 template <int DK, int DV>
 cudaError_t launch_core(const CoreArgs& c, cudaStream_t st) {
-    auto kern = decode_core_kernel<DK, DV>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Ring<DK, DV>::bytes);
+    // One slot per warp where the CTAs do not fit the SMs at once and a split has few steps, which other CTAs' loads hide: the
+    // recurrence and the mixing logits, which need no ring, then share an SM four at a time at 128/128 too, and the first-level cache
+    // keeps something.  At 128/128 (three CTAs per SM with two slots) also where the recurrence's CTAs are most of the grid.  Whole
+    // tokens, deep / one slot, us: 16 heads of 128, 64 rows, 40 tokens 170 / 157, 1000 tokens 202 / 192, 32 rows, 600 tokens 65.6 /
+    // 60.1, 16 rows, 300 tokens 35.7 / 32.8, but 16 rows, 3000 tokens 61.4 / 64.1; 16 heads of 64, 32 rows, 40 tokens 22.7 / 22.0, but
+    // 2000 tokens 42 / 47.
+    constexpr int FIT = DK + DV == 256 ? 3 : 4;
+    const int units = c.a.n_done * (c.a.nbs / 64) + (c.a.own_chunk ? c.a.pos % c.a.nbs + 63 : 0) / 64;
+    const int per = (units + c.S - 1) / c.S;
+    const bool one_slot = c.n_mix + c.n_rec + c.n_attn > 148 * FIT &&
+                          (per <= 4 || (FIT == 3 && (long)per * c.n_attn <= 11l * c.n_rec));
+    auto kern = one_slot ? decode_core_kernel<DK, DV, false> : decode_core_kernel<DK, DV, true>;
+    const int bytes = one_slot ? Ring<DK, DV, false>::bytes : Ring<DK, DV, true>::bytes;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return e;
-    return launch_pdl(kern, c.n_mix + c.n_rec + c.n_attn, DS_THREADS, st, c, true, Ring<DK, DV>::bytes);
+    return launch_pdl(kern, c.n_mix + c.n_rec + c.n_attn, DS_THREADS, st, c, true, bytes);
 }
 
 // Row tiles of every segment, then the launch.  Up to 32 batch rows all eight warps share the contraction of 16 weight rows
@@ -857,7 +870,9 @@ cudaError_t launch_skinny(SkinnyArgs& a, cudaStream_t st, bool overlap) {
     return launch_pdl(skinny_kernel<8, 4, 2>, tiles, 256, st, a, overlap);
 }
 
-// Splits of the finished keys of one (batch, head) over CTAs: enough CTAs for four per SM, at least two 64-key units each.
+// Splits of the finished keys of one (batch, head) over CTAs: enough CTAs for four per SM, at least two 64-key units each.  At
+// 128/128, where three fit with the deep ring, three per SM are better up to a few rows and worse beyond (16 heads, four / three, us a
+// token: 2 rows, 2700 tokens 26.0 / 23.8, 8 rows, 2000 33.5 / 31.4, 5500 53.3 / 56.7, 16 rows, 5500 85.6 / 96.1).
 int attn_splits(int B, int HQ, int units) {
     const int want = (148 * 4 + B * HQ - 1) / (B * HQ), most = units / 2;
     const int s = want < most ? want : most;

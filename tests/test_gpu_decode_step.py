@@ -100,6 +100,17 @@ def test_token_kernel_over_many_units(make, args, B, T0):
     test_token_kernel_matches_the_general_path(make, args, B, T0)
 
 
+@pytest.mark.parametrize("make,args,B,T0", [
+    (_gdn, dict(hidden=256, heads=16, head_dim=128, expand_v=1, attn_heads=16), 17, 40),
+    (_gdn, dict(hidden=256, heads=16, head_dim=128, expand_v=1, attn_heads=16), 17, 1500),
+    (_gdn, dict(hidden=256, heads=16, head_dim=64, expand_v=1, attn_heads=16), 17, 700),
+    (_mamba, dict(hidden=256, heads=16, head_dim=128, expand_v=0.5, attn_heads=16, nats_block_size=256), 17, 200),
+])
+def test_token_kernel_with_one_ring_slot(make, args, B, T0):
+    """Grids of more CTAs than fit the SMs and few steps per split: none, one and several steps through a ring of one slot."""
+    test_token_kernel_matches_the_general_path(make, args, B, T0)
+
+
 def test_copied_cache_continues_on_its_own():
     from neuralattentionsearchlinear_b200 import NAtSCache
     torch.manual_seed(1)
