@@ -99,6 +99,26 @@ def test_walk_without_the_trailing_quirk(nat):
     assert_close(ht, ht2, 2 * TOL, "final state (no trailing quirk)")
 
 
+def test_initial_state_between_vector_loads(nat):
+    """An initial state that starts on 4 bytes is read like any other: the same bits."""
+    from neuralattentionsearchlinear_b200 import _lib
+    B, T, H, K, V, nbs = 2, 200, 3, 128, 64, 64
+    q, k, v, g, h0 = synth_mamba_inputs(B, T, H, K, V, seed=3)
+    tb = nat.build_selection_tables(otab.synth_types(B, -(-T // nbs), H, 0.5, seed=4).cuda(), T, nbs)
+    q, k, v, g, h0 = (x.cuda().contiguous() for x in (q, k, v, g.float(), h0.float()))
+    gcs = torch.cat([x.cumsum(1) for x in g.split(64, 1)], 1).contiguous()
+    shifted = torch.empty(h0.numel() + 1, device="cuda")[1:].view_as(h0).copy_(h0)
+    assert shifted.data_ptr() % 16 == 4
+    got = []
+    for s in (h0, shifted):
+        o, ht = torch.empty_like(v), torch.empty_like(h0)
+        _lib.call("natsl_mamba_walk_fused", q.data_ptr(), k.data_ptr(), v.data_ptr(), gcs.data_ptr(), tb.types_i.data_ptr(),
+                  tb.indices.data_ptr(), tb.n_blocks.data_ptr(), s.data_ptr(), o.data_ptr(), ht.data_ptr(), B, T, H, H, K, V, nbs, 1.0,
+                  _lib.FLAG_DECAY_SKIPPED, torch.cuda.current_stream().cuda_stream)
+        got.append((o, ht))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
 def test_walk_refuses_other_head_dims():
     from neuralattentionsearchlinear_b200 import _lib
     z = torch.zeros(1, 64, 1, 128, dtype=torch.bfloat16, device="cuda")
