@@ -218,7 +218,7 @@ int natsl_gdn_walk_fused_vsplit(const void* q, const void* k, const void* w, con
  * gcs = chunk-local cumsum of the log decay (natsl_chunk_local_cumsum), outputs o [B,T,H,V] bf16 and ht [B,H,K,V]
  * fp32.  o == NULL (q may then be NULL): only the recurrence runs and ht is required.  Built for K = 128, V = 64
  * and any nats_block_size that is a multiple of 64 (an unselected block's chunks update a temporary state which is
- * rolled back at the end of the block); T <= 65536.
+ * rolled back at the end of the block); T <= 65536.  ht and hstart start on 16 bytes here and in the natsl_gdn_walk_fused entries.
  * Replaces: chunk_mamba_fwd_h + chunk_fwd_o of the Mamba2 branch (src/nats/ops/mamba/chunk_h.py:139-218,
  * src/nats/ops/mamba/chunk_o.py:137-198) and chunk_cumsum_non_gated_chunks (src/nats/ops/utils/cumsum.py:136-180);
  * same results as natsl_linear_fwd_h + natsl_linear_fwd_o with rule NATSL_RULE_MAMBA. */

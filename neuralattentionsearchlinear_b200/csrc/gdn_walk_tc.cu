@@ -473,6 +473,7 @@ extern "C" int natsl_gdn_walk_fused_ex(const void* q, const void* k, const void*
                   "natsl_linear_fwd_h + natsl_linear_fwd_o", K, V, nbs);
     NATSL_REQUIRE((T + 63) / 64 <= WK_MAX_NT, NATSL_ERR_TOO_LARGE, "natsl_gdn_walk_fused: T <= 65536");
     NATSL_REQUIRE(H <= 65535 && B <= 65535, NATSL_ERR_TOO_LARGE, "natsl_gdn_walk_fused: B, H <= 65535");
+    NATSL_REQUIRE(aligned_to(16, ht, hstart), NATSL_ERR_UNSUPPORTED, "natsl_gdn_walk_fused: ht and hstart must start on 16 bytes");
     NATSL_REQUIRE(!hstart || T % nbs != 0 || (last_types && (last_dtype == NATSL_DT_F32 || last_dtype == NATSL_DT_BF16)),
                   NATSL_ERR_NULL, "natsl_gdn_walk_fused: the block-start state of a complete last block needs that block's types");
     auto kern = gdn_walk_tc_kernel;

@@ -444,6 +444,7 @@ extern "C" int natsl_gdn_walk_fused_vsplit(const void* q, const void* k, const v
     NATSL_REQUIRE(K == 128 && V == 128 && nbs == 64, NATSL_ERR_UNSUPPORTED,
                   "natsl_gdn_walk_fused_vsplit: built for K = V = 128 and nats_block_size = 64 (got K=%d V=%d nbs=%d); use "
                   "natsl_linear_fwd_h + natsl_linear_fwd_o", K, V, nbs);
+    NATSL_REQUIRE(aligned_to(16, ht), NATSL_ERR_UNSUPPORTED, "natsl_gdn_walk_fused_vsplit: ht must start on 16 bytes");
     NATSL_REQUIRE((T + 63) / 64 <= WH_MAX_NT, NATSL_ERR_TOO_LARGE, "natsl_gdn_walk_fused_vsplit: T <= 8192 (use natsl_gdn_walk_fused)");
     NATSL_REQUIRE(2L * H <= 2147483647L && B <= 65535, NATSL_ERR_TOO_LARGE, "natsl_gdn_walk_fused_vsplit: B <= 65535");
     auto kern = gdn_walk_half_kernel<true>;

@@ -41,6 +41,19 @@ def test_abi_version_and_error_string():
     assert st == -3
 
 
+def test_walks_refuse_states_between_vector_stores():
+    """Final and block-start states leave as 16-byte stores: an address between them is an error code, before any CUDA call."""
+    lib = _lib.load()
+    p, odd = 1 << 20, (1 << 20) + 4
+    gdn, mamba = [p] * 11 + [None, p], [p] * 7 + [None, p]                # inputs, no initial state, output
+    shape = lambda K, V: [1, 64, 1, 1, K, V, 64, 1.0, 0, None]
+    for ht, hstart in ((odd, None), (None, odd)):
+        for st in (lib.natsl_gdn_walk_fused_ex(*gdn, ht, hstart, p, 1, 2, *shape(128, 128)),
+                   lib.natsl_mamba_walk_fused_ex(*mamba, ht, hstart, p, 1, 2, *shape(128, 64))):
+            assert st == -2 and b"16 bytes" in lib.natsl_last_error()
+    assert lib.natsl_gdn_walk_fused_vsplit(*gdn, odd, *shape(128, 128)) == -2
+
+
 def test_op_wrappers_reject_inconsistent_shapes_before_any_launch():
     """The kernels take shapes on trust; the Python wrappers check them first (no GPU needed to see the errors)."""
     from types import SimpleNamespace
