@@ -12,7 +12,8 @@
 // What bounds it: the chain w S -> v'' -> k^T v'' -> copy of an update, one CTA per SM, and HBM: at B = 8, T = 4096, H = 16 it writes 268 MB
 // of copies and reads the updating chunks' 48 KB.  Alone (us; before: linear_scan.cu, mma.sync, four CTAs of 32 columns per pair): that
 // size with 75 % of the chunks updating 194 -> 116 (4.9 TB/s), 25 % 112 -> 75; B = 16, T = 2048, 50 % 149 -> 97; 64 heads, T = 4096, 75 %
-// 135 -> 110.  The states are the same bits.  linear_scan.cu says where the line to it lies.
+// 135 -> 110.  The states are the same bits (tests/test_gpu_states.py): roundings and sums lie where the scan has them.  linear_scan.cu
+// says where the line to it lies.
 #include "tc_common.cuh"
 #include "../../include/natsl_b200.h"
 

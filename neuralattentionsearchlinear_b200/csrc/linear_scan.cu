@@ -25,8 +25,14 @@ constexpr int SCAN_THREADS = 128;
 // (batch, head) pairs and tokens from which the gated delta rule's states at 128/128, block 64, come from gdn_states_tc.cu: one CTA per
 // pair there, four here, whose steps take longer only when they share SMs.  This kernel / that one (us): 32 pairs 37 / 40 at T = 2048, 49 / 55
 // and 109 / 109 at T = 4096 (25 and 90 % selected); 48 pairs 19 / 22 at T = 1000, 60 / 60 and 117 / 101 at T = 4096 (25 and 75 %); 64 pairs
-// 27 / 24 at T = 1000, 51 / 44 at T = 2048, 135 / 110 at T = 4096; 192 pairs of 256 tokens 21 / 18, 256 of 64 tokens 9.7 / 10.4.
-constexpr int STATES_TC_PAIRS = 64, STATES_TC_TOKENS = 256;
+// 27 / 24 at T = 1000, 51 / 44 at T = 2048, 135 / 110 at T = 4096; 256 pairs of 64 tokens 9.7 / 10.4.  Short sequences, 40 and 75 % selected:
+// 64 pairs 10.7 / 12.8 and 13.2 / 13.7 at T = 256, 14.6 / 14.6 and 16.7 / 16.5 at T = 384; 80 pairs 12.5 / 12.5 and 14.6 / 12.6 at T = 256.  A second wave that
+// is nearly empty costs that form less than the scan's third: 149 pairs 15.8 / 16.6 and 17.5 / 15.6 at T = 256, 16.7 / 14.6 at T = 320, 41 / 37 at T = 1024,
+// 158 / 120 at T = 4096; 176 pairs 163 / 119 at T = 4096 (25 %); 192 pairs 21 / 18.7 at T = 256 (50 %).  With a tenth of the chunks selected, when
+// little but the copies is left, the scan would be up to 4.6 us ahead at 64 to 72 and 149 to 164 pairs (64 pairs, T = 2048 27 / 31).  Both give the same
+// bits, so that a sequence's gradients do not depend on the batch around it.
+constexpr int STATES_TC_PAIRS = 64;
+static int states_tc_tokens(int pairs) { return pairs < 80 ? 384 : pairs > 148 && pairs < 192 ? 320 : 256; }
 
 template <int K, int BV, bool GDN>
 struct ScanSmem {
@@ -359,7 +365,7 @@ extern "C" int natsl_linear_fwd_h(int rule, const void* k, const void* w, const 
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
 #define NATSL_SCAN_ARGS k, w, u, gcs, k_rstd, types_i, indices, n_blocks, h0, h, carry, ht, B, T, H, HN, V, nbs, decay, quirk, st
     if (rule == NATSL_RULE_GDN) {
-        if (K == 128 && V == 128 && nbs == 64 && h && !ht && k_rstd && T >= STATES_TC_TOKENS && T <= 65536 && B * H >= STATES_TC_PAIRS &&
+        if (K == 128 && V == 128 && nbs == 64 && h && !ht && k_rstd && T <= 65536 && B * H >= STATES_TC_PAIRS && T >= states_tc_tokens(B * H) &&
             (long)B * ((T + 63) / 64) * H <= INT32_MAX && aligned_to(16, k, w, u, h))
             return gdn_states_tc(k, w, u, gcs, k_rstd, types_i, indices, n_blocks, h0, h, carry, B, T, H, HN, decay, quirk, st);
         if (K == 64) return launch_scan<64, 32, true>(NATSL_SCAN_ARGS);
