@@ -40,20 +40,6 @@
 
 namespace natsl {
 
-#ifdef NATSL_MW_TIMING
-// scratch build only: cycles spent per role of CTA (0, 0), summed over the chunks
-__device__ long long mw_t[32];
-#define MW_T0() long long t__ = clock64()
-#define MW_ACC(i)                                                  \
-    do {                                                           \
-        const long long n__ = clock64();                           \
-        if (lane == 0 && blockIdx.x == 0 && blockIdx.y == 0) mw_t[i] += n__ - t__; \
-        t__ = n__;                                                 \
-    } while (0)
-#else
-#define MW_T0()
-#define MW_ACC(i)
-#endif
 
 constexpr int mw_threads(bool out) { return out ? 640 : 320; }       // 20 or 10 warps
 constexpr uint32_t mw_tmem_cols(bool out) { return out ? 512 : 128; }
@@ -257,12 +243,9 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             const int stg = c % L::nstage;
             const uint32_t base = sbase + stg * L::stage;
             const int fl = m_fl[c];
-            MW_T0();
             ok = warp_wait(bar_full + stg * 8, (c / L::nstage) & 1);
             if (ok) ok = warp_wait(bar_sready, c & 1);
-            MW_ACC(0);
             if (ok) ok = warp_wait(bar_pv, c & 1);
-            MW_ACC(1);
             if (!ok) break;
             {
                 // the update of the last chunk of an unselected block would be thrown away: it is not issued
@@ -274,7 +257,6 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 umma_commit(bar_s3);
             }
             __syncwarp();
-            MW_ACC(2);
         }
     } else if (OUT && warp == 16) {
         // ------------------------------------------------------------ issuer of the output products
@@ -299,15 +281,12 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 const uint32_t base = sbase + stg * L::stage;
                 const int fl = m_fl[c];
                 const int cp = ncopy & 1;
-                MW_T0();
                 if (fresh) ok = warp_wait(bar_cfull + cp * 8, (ncopy >> 1) & 1);
                 fresh = false;
-                MW_ACC(3);
                 // q k^T of the next chunk goes to the other buffer: its last reader was P of chunk c - 1, waited for
                 // before MMA 2 of that chunk
                 const bool ahead = c + 1 < NT;
                 if (ok && ahead) ok = warp_wait(bar_full + nstg * 8, ((c + 1) / L::nstage) & 1);
-                MW_ACC(4);
                 if (ok) {
                     // q S of this chunk and q k^T of the next one, half by half in turn
                     tc_fence_after();
@@ -327,10 +306,8 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                     ++ncopy;
                     fresh = true;
                 }
-                MW_ACC(5);
                 if (ok) ok = warp_wait(bar_pfull + (c & 1) * 8, (c >> 1) & 1);   // P of this chunk
                 if (ok && c > 0) ok = warp_wait(bar_odone, (c - 1) & 1);   // D2 is free
-                MW_ACC(6);
                 if (!ok) break;
                 {
                     tc_fence_after();
@@ -338,7 +315,6 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                     umma_commit(bar_d2 + (c & 1) * 8);
                 }
                 __syncwarp();
-                MW_ACC(7);
             }
         }
     } else if (warp < 6) {
@@ -419,14 +395,12 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             const int fl = m_fl[c];
             const float mul = m_mul[c];
             const bool restore = (fl & MW_RESTORE) != 0, save = !restore && c + 1 < NT && (m_fl[c + 1] & MW_SAVE) != 0;
-            MW_T0();
             // copy pubs & 1: MMA 1 of the chunks that read its previous content must be complete
             if (OUT && (fl & MW_ACTIVE) && pubs >= 2) ok = warp_wait(bar_cempty + (pubs & 1) * 8, ((pubs >> 1) - 1) & 1);
             // once the update of this chunk is complete, publish the state for the next chunk (and pre-apply the next
             // update's decay); after a failed (bounded) wait the remaining work is skipped
             if (ok) ok = warp_wait(bar_s3, c & 1);
             if (!ok) break;
-            if (warp == 2) MW_ACC(8);
             tc_fence_after();
             if (lane == 0) mbar_arrive(bar_empty + (c % L::nstage) * 8);       // MMA 3 is done with the k tile
             if (fl & MW_ACTIVE) {
@@ -439,7 +413,6 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 tc_fence_before();
                 arrive(bar_sready);
             }
-            if (warp == 2) MW_ACC(9);
         }
         // every update's decay was pre-applied except after the last one: TMEM holds the final state.  A complete last
         // block: the decoder continues from it if that block's own type is linear, else from the state in front of the
@@ -504,12 +477,9 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             if (c + 2 < NT) g_n2 = load_g(c + 2, tr);                     // consumed in the next iteration
             // The tile of the NEXT chunk, off the serial chain.  Its arrival waits until the update of this chunk is
             // complete: the MMA warp has then consumed this chunk's phase of the barrier.
-            MW_T0();
             if (ok && c + 1 < NT) stage_v(c + 1, g_n1);
-            if (warp == 8) MW_ACC(10);
             if (ok) ok = warp_wait(bar_s3, c & 1);
             if (ok && c + 1 < NT) arrive(bar_pv);
-            if (warp == 8) MW_ACC(11);
         }
     } else if (warp == 17) {
         // ------------------------------------------------------------ stores of the outputs
@@ -535,13 +505,10 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         // P = tril(q k^T e^{g_i - g_j}) of chunk c as the bf16 A operand of P v, from TMEM to TMEM; gg: g of the row's token, gk: of
         // key cb + lane, which the warp hands around through shared memory.
         auto build_p = [&](int c, float gg, float gk) {
-            MW_T0();
             __syncwarp();
             sg[lane] = gk;
             __syncwarp();
-            if (warp == 6) MW_ACC(12);
             ok = warp_wait(bar_dp + (c & 1) * 8, (c >> 1) & 1);
-            if (warp == 6) MW_ACC(13);
             if (!ok) return;
             tc_fence_after();
             uint32_t w[16];
@@ -571,7 +538,6 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             tmem_st_wait();
             tc_fence_before();
             arrive(bar_pfull + (c & 1) * 8);
-            if (warp == 6) MW_ACC(14);
         };
         // one set of warps takes the even chunks, one the odd ones
         float g_cur = set < NT ? load_g(set, tr) : 0.f, k_cur = set < NT ? load_g(set, cb + lane) : 0.f, g_n = 0.f, k_n = 0.f;
@@ -585,11 +551,9 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             build_p(c, g_cur, k_cur);
             const float fq = __expf(g_cur + m_carry[c]);
             const bool active = (m_fl[c] & MW_ACTIVE) != 0;
-            MW_T0();
             // o = scale (e^{g+carry} q S + P v): MMA 2 complete means MMA 1 of the chunk is complete as well
             if (ok) ok = warp_wait(bar_d2 + (c & 1) * 8, (c >> 1) & 1);
             if (!ok) break;
-            if (warp == 6) MW_ACC(15);
             tc_fence_after();
             uint32_t r1[32], r2[32];
             tmem_ld32(t_lane + ((c & 1) ? MW_D1B : MW_D1), r1);
@@ -619,7 +583,6 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             }
             fence_async_smem();
             arrive(bar_ofull + (c & 1) * 8);
-            if (warp == 6) MW_ACC(16);
             if (active) ++ncopy;
             if (c + 1 < NT && (m_fl[c + 1] & MW_ACTIVE)) ++ncopy;
             g_cur = g_n;
@@ -635,14 +598,6 @@ mamba_walk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
 
 }  // namespace natsl
 
-#ifdef NATSL_MW_TIMING
-extern "C" int natsl_mw_timing(long long* out, int reset) {
-    long long z[32] = {0};
-    if (out && cudaMemcpyFromSymbol(out, natsl::mw_t, sizeof(z)) != cudaSuccess) return -1;
-    if (reset && cudaMemcpyToSymbol(natsl::mw_t, z, sizeof(z)) != cudaSuccess) return -1;
-    return 0;
-}
-#endif
 
 extern "C" int natsl_mamba_walk_fused_ex(const void* q, const void* k, const void* v, const float* gcs,
                                       const int32_t* types_i, const int32_t* indices, const int32_t* n_blocks,
