@@ -41,7 +41,7 @@ constexpr float kLog2e = 1.4426950408889634f;
 // Alone (us; before: 128 x 64 score tiles, two CTAs per SM, one block each), block 64:
 //   128/128, B = 8, T = 4096, H = 16: 25 % selected 323 -> 265, 50 % 508 -> 410, 2 % 175 -> 141;  64/64, 30 %: 286 -> 239
 //   128/64, B = 4, T = 1000, H = 16, 50 %: 38 -> 30;  128/128, B = 1, T = 2048, H = 16, 30 %: 25.6 -> 23.5
-//   64/128, B = 2, T = 2048, 12 heads over 6, block 128, 40 %: 36 -> 30;  the smallest, B = 2, T = 64, H = 4: 6.3 -> 6.6
+//   64/128, B = 2, T = 2048, 12 heads over 6, block 128, 40 %: 36 -> 30;  the smallest, 64/64, B = 2, T = 64, H = 4: 5.3 -> 5.6
 // Of that the rows asked into L2 ahead are 8 us at 25 % and 9 us at 2 %.  Eight threads per row for delta, in whole lines: 275 us.
 constexpr int BDQ_THREADS = 384;                              // TMA, MMA, planner, (no work), 8 softmax warps
 constexpr int BDQ_STEPS = 2;                                  // steps that the planner is ahead
@@ -569,7 +569,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
 // Alone (us; before: 128 x 64 score tiles, p and ds through shared memory, one CTA per pair of tiles), block 64:
 //   128/128, B = 8, T = 4096, H = 16: 25 % selected 678 -> 355, 50 % 1069 -> 545, 2 % 338 -> 182;  64/64, 30 %: 630 -> 336
 //   128/64, B = 4, T = 1000, H = 16, 50 %: 72 -> 41;  128/128, B = 1, T = 2048, H = 16, 30 %: 65 -> 36
-//   64/128, B = 2, T = 2048, 12 heads over 6, block 128, 40 %: 113 -> 56;  the smallest, B = 2, T = 64, H = 4: 8.5 -> 8.7
+//   64/128, B = 2, T = 2048, 12 heads over 6, block 128, 40 %: 113 -> 56;  the smallest, 64/64, B = 2, T = 64, H = 4: 7.5 -> 7.9, and at T = 100 7.5 -> 8.6: one step per CTA, of which the 64 keys
+//   of a single tile fill half of the lanes
 constexpr int BKV_THREADS = 384;                              // TMA, MMA, planner, (no work), 8 softmax warps
 constexpr int BKV_MAXG = 16;
 constexpr int BKV_DESCS = 2;                                  // steps that the planner is ahead

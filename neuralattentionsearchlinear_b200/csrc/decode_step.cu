@@ -17,10 +17,10 @@
 //     the first keys and values) before it waits for them.  The recurrence reads the state once: S^T k and S^T q are formed
 //     together (o = e^g S^T q + (q.k) v').  Attention splits the 64-key units of the finished blocks over CTAs; a warp
 //     takes 16 keys of a unit, several units on their way through shared memory.
-//     On the device, from the first projection to the output (us, by time stamps; before: one step of 8 or 16 keys ahead in
-//     registers, ranges of units per split, all mixing rows in one CTA): 32 rows, 2048 tokens, 16 heads of 64 50.0 -> 42.6; 4 rows,
-//     1030 tokens, 32 heads of 128 / 64 37.9 -> 29.3; 16 rows, 2048 tokens, 16 heads of 128 59.6 -> 51.7; 1 row, 300 tokens, 6 heads of
-//     128 / 256 17.5 -> 16.7.
+//     On the device, tokens back to back (us; before: one step of 8 or 16 keys ahead in registers, ranges of units per split, all
+//     mixing rows in one CTA): 32 rows, 2000 tokens, 16 heads of 64 51.3 -> 41.0; 4 rows, 1000 tokens, 32 heads of 128 / 64 36.7 -> 26.6; 16
+//     rows, 2000 tokens, 16 heads of 128 61.4 -> 50.4; 64 rows, 40 tokens 157 -> 155; 1 row, 300 tokens, 6 heads of 128 / 256 14.8 -> 15.2,
+//     1000 tokens 16.8 -> 15.9.
 //   * merge: combines the splits, both RMS norms, mixing weights and gate; extra CTAs shift the convolution tails.
 // All state (recurrent state, tails, decay sums, pooled input, key/value rows) is updated in place.
 #include "common.cuh"

@@ -29,8 +29,9 @@
 // What bounded it: the load/store unit.  Every thread's own arrival on nine barriers (960 a chunk) and output rows stored 16 bytes per
 // lane cost more than the chunk's products; the waits of all the other warps' shared loads and stores were the sum.  Now a warp
 // arrives once, outputs leave as tiles, the scalars of a chunk are worked out by all threads at the start, and what a step needs is
-// read in front of its wait.  Alone (us, outputs / state only): 64 sub-segments of 1024 tokens, H = 32 563 / 360 -> 387 / 210; 32 of
-// 2048 492 / 288 -> 329 / 175 (4.9 / 4.6 TB/s); B = 8, T = 4096, H = 16 134 / 70 -> 81 / 52; B = 4, T = 1030, H = 32 45 / 26 -> 33 / 18.
+// read in front of its wait.  Alone in a graph (us, outputs / state only), H = 32, 10 % of the blocks softmax: 64 sub-segments of 1024 tokens
+// 563 / 303 -> 381 / 198; 32 of 2048 491 / 266 -> 334 / 170 (4.8 / 4.7 TB/s); 4 of 16384, what one sequence of 65536 is cut into, 486 / 255 ->
+// 313 / 186 (5.1 / 4.3 TB/s); B = 8, T = 4096, H = 16 132 / 70 -> 86 / 54.
 // Tried and not kept: four stages, the first loads in front of the tables, no L2 prefetch (all +- 3 %, three loads at once at the start
 // 5 to 10 % slower).
 // All mbarrier waits are bounded (status word + clean teardown on expiry); every barrier is waited for in every one

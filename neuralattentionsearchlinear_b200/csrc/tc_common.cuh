@@ -141,7 +141,7 @@ __device__ __forceinline__ void umma_ss(uint32_t d_tmem, uint64_t adesc, uint64_
 // Four K-steps (64 elements of K) in one go, descriptors given by their low words (umma_desc_lo; the high word is that of
 // umma_desc(., ., 1024)): one election for the four, and the steps differ by constants, which the uniform datapath adds.
 // Descriptors formed anew for every product cost the issuing warp about a hundred cycles each.
-// (With it, alone in a graph: Mamba2 walk over 64 x 1024 tokens, H = 32 680 -> 482 us; gated delta rule, B = 8, T = 4096, H = 16,
+// (With it, alone in a graph: the Mamba2 walk of that time over 64 x 1024 tokens, H = 32 29 % less; gated delta rule, B = 8, T = 4096, H = 16,
 // 128/128, preparation and walk together 357 -> 346 us.  Under the power limit, where the clock gives what the cycles save, the
 // latter do not change: 177 - 195 and 176 - 198 us at 1.74 - 1.96 GHz.)
 constexpr uint32_t UMMA_DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);

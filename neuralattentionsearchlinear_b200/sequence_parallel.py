@@ -193,8 +193,9 @@ def one_rank_splits(L: int, nbs: int, units: int) -> int:
     """The same for one rank, which walks ``units`` = batch x heads sequences and has no exchange to hide, at the fused walk's head
     dims (K = 128, V = 64): the number of sub-segments with the least time for both passes, from what that walk takes on the device:
     1.3 us a chunk and 8 us a CTA, waves of 148 CTAs, a first pass of 0.6 of the second, 35 us of folding around them; an uncut
-    sequence needs one pass.  Mostly that is one wave of CTAs.  Op captured in a graph (us), sub-segments of 1024 tokens against it:
-    T = 4096 H = 16 86 / 76, T = 8192 H = 32 185 / 174, T = 16384 H = 16 207 / 192, H = 32 377 / 324, T = 32768 H = 32 965 / 871,
+    sequence needs one pass.  Mostly that is one wave of CTAs.  (The first pass fits two CTAs on an SM, which the model leaves out.
+    The cut, and with it the order of sums, follows the batch: a sequence's last bits may.)  Op captured in a graph (us),
+    sub-segments of 1024 tokens against it: T = 4096 H = 16 86 / 76, T = 8192 H = 32 185 / 174, T = 16384 H = 16 207 / 192, H = 32 377 / 324, T = 32768 H = 32 965 / 871,
     T = 65536 H = 32 3069 / 3006 (2 % of the blocks softmax instead of 8 %: 1411 / 1170).  An uncut sequence beside a long attention
     would save the first pass (T = 65536 H = 32, 10 %: 3401 / 3518) but is what the op waits for where few blocks are selected (2 %:
     1597 / 1170).  At other head dims the recurrence is a scan of 32 value columns per CTA, several to an SM, which wants more and
